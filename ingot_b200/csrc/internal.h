@@ -107,13 +107,10 @@ int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
 struct QmmCall {
     int32_t fmt = 0;
     int epi = 0;   // 0 store, 1 gate/up + activation
-    int bn = 256;  // token rows per tile (MMA N): 128 or 256
+    int bn = 0;    // token rows per tile: the largest tile of the list; plain formats: 32..256; dense quantized: chosen by the launch
     const void* x16 = nullptr;
     int64_t ldx = 0;
     int64_t x_rows = 0;
-    // gathered activation rows (grouped gate/up): row r of a tile is row gather_map[tile.start + r] / gather_div of x16
-    const uint32_t* gather_map = nullptr;
-    uint32_t gather_div = 1;
     const void* w[2] = {nullptr, nullptr};
     const void* s[2] = {nullptr, nullptr};
     const void* b[2] = {nullptr, nullptr};

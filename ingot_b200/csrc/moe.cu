@@ -52,7 +52,7 @@ int decode_tile_rows(const iq_moe* l, int tokens) {
     return pairs <= (int64_t)l->d.experts * 6 ? 8 : 16;
 }
 constexpr int kPrefillTileRows = 128;      // token rows per tensor-core tile while experts see few rows
-constexpr int kPrefillTileRowsBig = 256;   // ... and once they see many: every weight tile is dequantised half as often
+constexpr int kPrefillTileRowsBig = 192;   // ... and once they see many: every weight tile is dequantised less often
 constexpr int kTensorPathRowsPerExpert = 24;
 constexpr int kBigTileRowsPerExpert = 96;
 constexpr int kRouterSmemMax = 200 * 1024;
@@ -227,16 +227,13 @@ int tensor_tile_rows(int64_t rows, int64_t expert_slots) {
     return rows >= expert_slots * kBigTileRowsPerExpert ? kPrefillTileRowsBig : kPrefillTileRows;
 }
 
-// rows16: fp16 rows [n_rows, ld16] in tile order, or (gather_map given) the tokens' rows in place, fetched through
-// gather_map[sorted position] / gather_div.
+// rows16: fp16 rows [n_rows, d_model] in tile order
 int32_t run_gateup_tc(iq_moe* l, cudaStream_t cs, const __half* rows16, int64_t n_rows, const Tile* tiles,
-                      const uint32_t* ntiles, __half* h, int bn, const uint32_t* gather_map = nullptr, uint32_t gather_div = 1,
-                      int64_t ld16 = 0, int64_t x_rows = 0) {
+                      const uint32_t* ntiles, __half* h, int bn) {
     const iq_moe_desc& d = l->d;
     QmmCall c;
     c.fmt = l->fmt; c.epi = 1; c.bn = bn;
-    c.x16 = rows16; c.ldx = ld16 > 0 ? ld16 : d.d_model; c.x_rows = x_rows > 0 ? x_rows : n_rows;
-    c.gather_map = gather_map; c.gather_div = gather_div;
+    c.x16 = rows16; c.ldx = d.d_model; c.x_rows = n_rows;
     c.w[0] = d.gate.w; c.w[1] = d.up.w;
     c.s[0] = d.gate.scales; c.s[1] = d.up.scales;
     c.b[0] = d.gate.biases; c.b[1] = d.up.biases;
@@ -409,7 +406,7 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
         if (st != kOk) return st;
         return iq_qmv(ctx, stream, h, IQ_F16, d_ff, down, out, out_dtype, ldo, rows, flags, 0);
     }
-    if (fmt == kFmtAffine4 || fmt == kFmtMxfp4) {
+    if (fmt != kFmtTernary && fmt != kFmtAffine6) {
         // GEMM path, fused: the gate and the up rows of the concatenated matrix are the two weight tiles of one stage of
         // the tcgen05 kernel, whose epilogue applies the activation and writes h = half(act(gate x, up x)) directly
         // (dswiglu_hh of the reference, Shaders/yy_model.metal:187-227, without the fp32 gate|up round trip: at
@@ -434,7 +431,7 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
         const size_t row_groups = (size_t)gate_up->k / gate_up->group;
         const size_t sbytes = fmt == kFmtMxfp4 ? 1 : 2;
         QmmCall c;
-        c.fmt = fmt; c.epi = 1; c.bn = rows >= 256 ? 256 : 128;
+        c.fmt = fmt; c.epi = 1;
         c.x16 = x16; c.ldx = ld16; c.x_rows = rows;
         c.w[0] = gate_up->w;
         c.w[1] = static_cast<const uint32_t*>(gate_up->w) + (size_t)d_ff * row_words;
@@ -451,7 +448,7 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
         if (st != kOk) return st;
         return iq_qmm(ctx, stream, h, IQ_F16, d_ff, down, out, out_dtype, ldo, rows, flags, nullptr, 0);
     }
-    // other formats (8-bit, 4-bit g32): gate|up GEMM -> activation -> down GEMM
+    // ternary gate/up rows: gate|up GEMM -> activation -> down GEMM
     char* p = static_cast<char*>(workspace) + round_up_sz((size_t)rows * d_ff * 2, 256);
     float* gu = reinterpret_cast<float*>(p);
     p += round_up_sz((size_t)rows * 2 * d_ff * 4, 256);
@@ -709,22 +706,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     const bool tc = use_tensor_path(P, d.expert_count);
     if (pieces & IQ_PIECE_GATEUP) {
         if (tc) {
-            // The GEMM's producer fetches each tile's token rows through row_map (the reference gathers through rowMap
-            // too, Shaders/qmm_nax_moe.metal:512-586): nothing is packed in expert order. It needs fp16 rows: fp16
-            // activations are used in place, others are converted once per token (not once per routed pair).
-            const __half* x16 = static_cast<const __half*>(x);
-            int64_t ld16 = ldx;
-            st = kOk;
-            if (x_dtype != kF16) {
-                const size_t units = (size_t)tokens * d.d_model / 8;
-                rows_to_f16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, cs>>>(x, x_dtype, ldx, w.xs, tokens, d.d_model);
-                st = check_cuda(ctx, cudaGetLastError(), "rows_to_f16 launch");
-                x16 = w.xs;
-                ld16 = d.d_model;
-            }
-            if (st == kOk)
-                st = run_gateup_tc(l, cs, x16, P, w.tiles_b, w.ntiles + 1, w.h, tensor_tile_rows(P, d.expert_count), w.row_map,
-                                   (uint32_t)d.top_k, ld16, tokens);
+            moe_pack_tokens_kernel<<<tokens, 256, 0, cs>>>(x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k);
+            st = check_cuda(ctx, cudaGetLastError(), "moe_pack_tokens launch");
+            if (st == kOk) st = run_gateup_tc(l, cs, w.xs, P, w.tiles_b, w.ntiles + 1, w.h, tensor_tile_rows(P, d.expert_count));
         } else {
             st = run_gateup(l, cs, x, x_dtype, ldx, w.row_map, w.tiles_a, w.ntiles, max_tiles, bm, w.h);
         }
@@ -778,6 +762,7 @@ struct ExpertsWs {
     Tile* tiles;
     uint32_t* ntiles;
     __half* h;
+    __half* xs;  // rows fetched through an index, in tile order (tensor-core path)
     size_t bytes;
 };
 ExpertsWs carve_experts(const iq_moe* l, void* base, int max_rows, int sources) {
@@ -791,6 +776,7 @@ ExpertsWs carve_experts(const iq_moe* l, void* base, int max_rows, int sources) 
     w.tiles = static_cast<Tile*>(take(((size_t)max_rows / 8 + (size_t)sources * l->d.expert_count + 1) * sizeof(Tile)));
     w.ntiles = static_cast<uint32_t*>(take(16));
     w.h = static_cast<__half*>(take((size_t)max_rows * l->d.d_ff * 2));
+    w.xs = static_cast<__half*>(take((size_t)max_rows * l->d.d_model * 2));
     w.bytes = off;
     return w;
 }
@@ -848,9 +834,13 @@ int32_t moe_experts_impl(iq_moe* l, void* stream, const void* rows_f16, const ui
                                            w.ntiles);
         int32_t st2 = check_cuda(ctx, cudaGetLastError(), "ep_tiles launch");
         // the row count is only known on the device: bounds come from the capacity, total_rows picks the kernels
-        if (st2 == kOk)
-            st2 = run_gateup_tc(l, cs, static_cast<const __half*>(rows_f16), max_rows, w.tiles, w.ntiles, w.h, bn, row_index, 1,
-                                d.d_model, max_rows);
+        const __half* rows = static_cast<const __half*>(rows_f16);
+        if (st2 == kOk && row_index != nullptr) {
+            moe_gather_rows_kernel<<<ctx->sms * 8, 256, 0, cs>>>(rows, row_index, w.tiles, w.ntiles, bn, w.xs, d.d_model);
+            st2 = check_cuda(ctx, cudaGetLastError(), "moe_gather_rows launch");
+            rows = w.xs;
+        }
+        if (st2 == kOk) st2 = run_gateup_tc(l, cs, rows, max_rows, w.tiles, w.ntiles, w.h, bn);
         if (st2 == kOk) st2 = run_down_tc(l, cs, w.h, max_rows, w.tiles, w.ntiles, yd, yd_dtype, bn);
         if (st2 == kOk && yd_rows != nullptr) st2 = scatter_rows(ctx, cs, yd, yd_rows, max_rows, d.d_model, yd_dtype);
         return st2;

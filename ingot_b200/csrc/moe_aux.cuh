@@ -813,6 +813,43 @@ __global__ void __launch_bounds__(256) moe_pack_rows_kernel(const void* __restri
     }
 }
 
+// The same for the tensor-core GEMM, a block per token: its row is read and converted once and stored at the top_k places
+// its experts take it from. The GEMM reads every row once per 64 output features, so the rows have to be where tensor copies
+// fetch them in one piece: fetching them by index inside the GEMM (16-byte asynchronous copies) ran at 19 bytes per cycle
+// and SM, a third of what the tensor cores consume. 4096 tokens x 8 x 2048: 23 us.
+__global__ void __launch_bounds__(256) moe_pack_tokens_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx,
+                                                             const uint32_t* __restrict__ pos, __half* __restrict__ rows,
+                                                             int D, int topk) {
+    pdl_launch_dependents();
+    __shared__ uint32_t sp[32];
+    const int t = blockIdx.x;
+    if ((int)threadIdx.x < topk) sp[threadIdx.x] = pos[(size_t)t * topk + threadIdx.x];
+    __syncthreads();
+    for (int u = threadIdx.x; u < D / 8; u += 256) {
+        float v[8];
+        load_x8(x, x_dtype, (size_t)t * ldx + u * 8, v);
+        uint4 o;
+        o.x = pack_half2(v[0], v[1]); o.y = pack_half2(v[2], v[3]); o.z = pack_half2(v[4], v[5]); o.w = pack_half2(v[6], v[7]);
+        for (int k = 0; k < topk; k++) *reinterpret_cast<uint4*>(rows + (size_t)sp[k] * D + u * 8) = o;
+    }
+}
+
+// fp16 rows gathered through an index into the order of a tile list: rows[i] = src[index[i]] for every row i of a tile.
+__global__ void __launch_bounds__(256) moe_gather_rows_kernel(const __half* __restrict__ src, const uint32_t* __restrict__ index,
+                                                             const Tile* __restrict__ tiles, const uint32_t* __restrict__ ntiles,
+                                                             int bn, __half* __restrict__ rows, int D) {
+    pdl_launch_dependents();
+    const int per = (bn + 7) / 8, total = (int)*ntiles * per;  // eight rows per item, a warp each
+    for (int it = blockIdx.x; it < total; it += gridDim.x) {
+        const Tile t = tiles[it / per];
+        const uint32_t r = (it % per) * 8 + (threadIdx.x >> 5);
+        if (r >= t.count) continue;
+        const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)index[t.start + r] * D);
+        uint4* d = reinterpret_cast<uint4*>(rows + (size_t)(t.start + r) * D);
+        for (int u = threadIdx.x & 31; u < D / 8; u += 32) d[u] = ldg_nc_u4(s + u);
+    }
+}
+
 // Tile list of the rows a rank received, by source then by local expert; counts[s * E + e] rows from source s for
 // expert e. region_rows == 0: the sources' rows follow each other (packed); region_rows > 0: the rows of source s start
 // at s * region_rows (every source owns a fixed region of the receive buffer). One block; at most 4096 entries.

@@ -8,6 +8,15 @@ namespace iq {
 
 constexpr uint64_t kWaitCycles = 4000000000ull;  // bound of every device-side wait: about two seconds
 
+// One lane of a converged warp. Tensor copies and tcgen05 instructions take their operands from uniform registers: under
+// `if (lane == 0)` the compiler cannot know that one lane is active and wraps every one of them in a loop over the active
+// lanes (125 cycles per tcgen05.mma measured, whatever its size); under this predicate it issues them directly (30).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0;
+}
+
 // ---- PTX wrappers ---------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -122,6 +131,12 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
 __device__ __forceinline__ void sts128(uint32_t a, const uint4& v) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t r;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
     unsigned short r;
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(a));
@@ -141,10 +156,12 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  : "memory");
 }
 
-// 16-byte asynchronous copy global -> shared memory (bypassing L1), and the arrival that an mbarrier receives once all
-// of this thread's copies issued so far have landed (.noinc: it counts as one of the barrier's expected arrivals).
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// Asynchronous copy of 4, 8 or 16 bytes global -> shared memory through L1 (neighbouring pieces of the line follow), and the
+// arrival that an mbarrier receives once all of this thread's copies issued so far have landed (.noinc: it counts as one
+// of the barrier's expected arrivals).
+template <int BYTES>
+__device__ __forceinline__ void cp_async_ca(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
 }
 __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");

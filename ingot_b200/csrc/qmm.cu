@@ -1,12 +1,15 @@
 // Host side of the tcgen05 GEMM: tensor maps, kernel selection, the iq_qmm entry point.
+#include <string.h>
+
 #include "internal.h"
+#include "qmm_ta.cuh"
 #include "qmm_tc.cuh"
 
 namespace iq {
 
 namespace {
 
-typedef void (*QmmKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const QmmParams);
+typedef void (*QmmKernel)(const CUtensorMap, const CUtensorMap, const QmmParams);
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -15,74 +18,74 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 struct KernelEntry {
     int32_t fmt;
     int bn;
-    int epi;
-    int act;
-    bool gather;
     QmmKernel fn;
     int smem;
 };
 
-template <int FMT, int BN, int EPI, int ACT = kActSilu, bool GATHER = false>
+template <int FMT, int BN>
 KernelEntry entry() {
-    return KernelEntry{FMT, BN, EPI, ACT, GATHER, qmm_tc_kernel<FMT, BN, EPI, ACT, GATHER>, QmmSmem<FMT, BN, EPI>::TOTAL};
-}
-// gate/up with the activation rows gathered by row index, both tile heights
-template <int FMT, int ACT>
-void gather_entries(KernelEntry* t, int* n) {
-    t[(*n)++] = entry<FMT, 128, kEpiGateUp, ACT, true>();
-    t[(*n)++] = entry<FMT, 256, kEpiGateUp, ACT, true>();
+    return KernelEntry{FMT, BN, qmm_tc_kernel<FMT, BN>, QmmSmem<FMT, BN>::TOTAL};
 }
 
 const KernelEntry* table(int* n) {
-    static const KernelEntry fixed[] = {
-        entry<kFmtAffine4, 256, kEpiStore>(), entry<kFmtAffine4, 128, kEpiStore>(),
-        entry<kFmtAffine8, 256, kEpiStore>(), entry<kFmtAffine8, 128, kEpiStore>(),
-        entry<kFmtMxfp4, 256, kEpiStore>(),   entry<kFmtMxfp4, 128, kEpiStore>(),
-        entry<kFmtAffine4G32, 256, kEpiStore>(), entry<kFmtAffine4G32, 128, kEpiStore>(),
-        entry<kFmtAffine4, 128, kEpiGateUp>(), entry<kFmtMxfp4, 128, kEpiGateUp>(),
-        entry<kFmtAffine4, 256, kEpiGateUp>(), entry<kFmtMxfp4, 256, kEpiGateUp>(),
-        entry<kFmtAffine4, 128, kEpiGateUp, kActSwigluOai>(), entry<kFmtMxfp4, 128, kEpiGateUp, kActSwigluOai>(),
-        entry<kFmtAffine4, 256, kEpiGateUp, kActSwigluOai>(), entry<kFmtMxfp4, 256, kEpiGateUp, kActSwigluOai>(),
-        entry<kFmtAffine4, 128, kEpiGateUp, kActGelu>(), entry<kFmtAffine4, 256, kEpiGateUp, kActGelu>(),
-        entry<kFmtAffine4, 128, kEpiGateUp, kActRelu2>(), entry<kFmtAffine4, 256, kEpiGateUp, kActRelu2>(),
-        entry<kFmtMxfp4, 128, kEpiGateUp, kActGelu>(), entry<kFmtMxfp4, 256, kEpiGateUp, kActGelu>(),
-        entry<kFmtMxfp4, 128, kEpiGateUp, kActRelu2>(), entry<kFmtMxfp4, 256, kEpiGateUp, kActRelu2>(),
+    static const KernelEntry t[] = {
         // bf16 x bf16 (the router's approximate logits); the small token tiles spread few experts over many CTAs
-        entry<kFmtBf16Plain, 128, kEpiStore>(), entry<kFmtBf16Plain, 64, kEpiStore>(), entry<kFmtBf16Plain, 32, kEpiStore>(),
-        entry<kFmtTernary, 256, kEpiStore>(), entry<kFmtTernary, 128, kEpiStore>(),
-        entry<kFmtInt8Plain, 256, kEpiStore>(), entry<kFmtInt8Plain, 128, kEpiStore>(),  // rotated W8A8
+        entry<kFmtBf16Plain, 128>(), entry<kFmtBf16Plain, 64>(), entry<kFmtBf16Plain, 32>(),
+        entry<kFmtInt8Plain, 256>(), entry<kFmtInt8Plain, 128>(),  // rotated W8A8
     };
-    constexpr int kFixed = (int)(sizeof(fixed) / sizeof(fixed[0]));
-    static KernelEntry t[kFixed + 16];
-    static int count = 0;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        for (int i = 0; i < kFixed; i++) t[count++] = fixed[i];
-        gather_entries<kFmtAffine4, kActSilu>(t, &count);
-        gather_entries<kFmtAffine4, kActGelu>(t, &count);
-        gather_entries<kFmtAffine4, kActSwigluOai>(t, &count);
-        gather_entries<kFmtAffine4, kActRelu2>(t, &count);
-        gather_entries<kFmtMxfp4, kActSilu>(t, &count);
-        gather_entries<kFmtMxfp4, kActGelu>(t, &count);
-        gather_entries<kFmtMxfp4, kActSwigluOai>(t, &count);
-        gather_entries<kFmtMxfp4, kActRelu2>(t, &count);
-    });
-    *n = count;
+    *n = (int)(sizeof(t) / sizeof(t[0]));
     return t;
 }
 
-const KernelEntry* find(int32_t fmt, int bn, int epi, int act, bool gather) {
+const KernelEntry* find(int32_t fmt, int bn) {
     int n;
     const KernelEntry* t = table(&n);
-    if (epi != kEpiGateUp) act = kActSilu;
     for (int i = 0; i < n; i++)
-        if (t[i].fmt == fmt && t[i].bn == bn && t[i].epi == epi && t[i].act == act && t[i].gather == gather) return &t[i];
+        if (t[i].fmt == fmt && t[i].bn == bn) return &t[i];
     return nullptr;
+}
+
+typedef void (*TaKernel)(const TaMaps, const TaParams);
+
+// gate/up: the formats of experts and of dense FFNs
+TaKernel ta_pick(int32_t fmt, int epi) {
+    switch (fmt) {
+        case kFmtAffine4: return epi ? qmm_ta_kernel<kFmtAffine4, 1> : qmm_ta_kernel<kFmtAffine4, 0>;
+        case kFmtMxfp4: return epi ? qmm_ta_kernel<kFmtMxfp4, 1> : qmm_ta_kernel<kFmtMxfp4, 0>;
+        case kFmtAffine8: return epi ? qmm_ta_kernel<kFmtAffine8, 1> : qmm_ta_kernel<kFmtAffine8, 0>;
+        case kFmtAffine4G32: return epi ? qmm_ta_kernel<kFmtAffine4G32, 1> : qmm_ta_kernel<kFmtAffine4G32, 0>;
+        case kFmtTernary: return epi ? nullptr : qmm_ta_kernel<kFmtTernary, 0>;
+        default: return nullptr;
+    }
+}
+
+// Token rows per tile of a dense GEMM: the height (a multiple of 16, at most 192) with the least (waves over the SMs) x
+// (time of a tile). A K step costs the MMA in proportion to the height, and the conversion of its 128 x 64 weights about as
+// much as 128 tokens whatever the height. 512 tokens x 14336 features: five tiles of 112 rows are 560 work items in
+// four waves of cost 128, three of 176 would be 336 items in three waves of 176.
+int ta_tile_rows(int m, int n_tiles, int sms) {
+    int best = 16;
+    long long best_cost = -1;
+    for (int tiles = (m + kTaMaxRows - 1) / kTaMaxRows; tiles <= (m + 15) / 16; tiles++) {
+        const int h = round_up((m + tiles - 1) / tiles, 16);
+        const long long waves = ((long long)((m + h - 1) / h) * n_tiles + sms - 1) / sms;
+        const long long cost = waves * (h > 128 ? h : 128);
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = h; }
+        if (h <= 64) break;
+    }
+    return best;
 }
 
 }  // namespace
 
 int32_t qmm_init(iq_ctx* ctx) {
+    for (int fmt = 0; fmt <= kFmtTernary; fmt++)
+        for (int epi = 0; epi < 2; epi++) {
+            const TaKernel k = ta_pick(fmt, epi);
+            if (k == nullptr) continue;
+            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k), cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemMax);
+            if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmm_ta)");
+        }
     int n;
     const KernelEntry* t = table(&n);
     for (int i = 0; i < n; i++) {
@@ -111,6 +114,23 @@ int32_t make_map_2d(iq_ctx* ctx, CUtensorMap* map, const void* base, int elem, u
         swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ctx, kErrCuda, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return kOk;
+}
+
+// X as the TMA of qmm_ta.cuh sees it: [K / 64][rows][64 fp16], box = xk K steps of box_rows rows, 128-byte swizzle.
+static int32_t make_map_ksteps(iq_ctx* ctx, CUtensorMap* map, const void* base, uint64_t rows, uint64_t ksteps, uint64_t row_bytes,
+                               uint32_t box_rows, uint32_t xk) {
+    if (ctx->encode_tiled == nullptr) return fail(ctx, kErrCuda, "cuTensorMapEncodeTiled is not available");
+    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || row_bytes % 16 != 0)
+        return fail(ctx, kErrInvalidArg, "qmm: TMA needs a 16-byte aligned base and row pitch");
+    const cuuint64_t dims[3] = {64, rows, ksteps};
+    const cuuint64_t strides[2] = {row_bytes, 128};
+    const cuuint32_t box[3] = {64, box_rows, xk};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled)(
+        map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(ctx, kErrCuda, "cuTensorMapEncodeTiled (K steps) failed (%d)", (int)r);
     return kOk;
 }
 
@@ -147,64 +167,99 @@ int32_t cached_rowblock_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t
     return kOk;
 }
 
-int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
-    const KernelEntry* ke = find(c.fmt, c.bn, c.epi, c.act, c.gather_map != nullptr);
-    if (ke == nullptr) return fail(ctx, kErrNoKernel, "qmm: no kernel for format %d, tile %d, epilogue %d", c.fmt, c.bn, c.epi);
-    const bool i8 = c.fmt == kFmtInt8Plain;     // int8 rows on both sides, 128 inputs per K step
-    const bool plain = c.fmt == kFmtBf16Plain;  // bf16 activations and bf16 weights, both copied as they are
-    if (i8) {
-        CUtensorMap ax, aw;
-        int32_t ri = make_map_2d(ctx, &ax, c.x16, 0, (uint64_t)c.K, (uint64_t)c.x_rows, (uint64_t)c.ldx, 128, c.bn, true);
-        if (ri == kOk) ri = make_map_2d(ctx, &aw, c.w[0], 0, (uint64_t)c.K, (uint64_t)c.N, (uint64_t)c.K, 128, kWRows, true);
-        if (ri != kOk) return ri;
-        QmmParams q = {};
-        q.s[0] = q.s[1] = c.s[0]; q.b[0] = q.b[1] = c.b[0];
-        q.N = c.N; q.K = c.K; q.M = c.M;
-        q.y = c.y; q.y_dtype = c.y_dtype; q.ldy = c.ldy; q.accumulate = c.accumulate;
-        q.limit = c.limit;
-        q.status = ctx->d_status;
-        const int work = ((c.M + c.bn - 1) / c.bn) * ((c.N + kWRows - 1) / kWRows);
-        ke->fn<<<work < ctx->sms ? work : ctx->sms, kQmmThreads, ke->smem, st>>>(ax, aw, aw, q);
-        return check_cuda(ctx, cudaGetLastError(), "qmm_i8 launch");
-    }
-    const int pack_row = c.fmt == kFmtAffine8 ? 64 : (c.fmt == kFmtTernary ? 16 : 32);
-    const uint64_t row_bytes = (uint64_t)c.K / kBK * pack_row;
-    CUtensorMap mx, mw0, mw1;
-    int32_t r = make_map_2d(ctx, &mx, c.x16, plain ? 2 : 1, (uint64_t)c.K, (uint64_t)c.x_rows, (uint64_t)c.ldx * 2, kBK, c.bn, true);
+// The quantized formats: weights through tensor memory (csrc/qmm_ta.cuh). c.bn: the largest tile of the list (grouped).
+static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
+    const TaKernel k = ta_pick(c.fmt, c.epi);
+    if (k == nullptr) return fail(ctx, kErrNoKernel, "qmm: no kernel for format %d, epilogue %d", c.fmt, c.epi);
+    TaParams p;
+    memset(&p, 0, sizeof(p));
+    const int n_tiles = (c.N + (c.epi ? 63 : 127)) / (c.epi ? 64 : 128);
+    const int rows = c.tiles == nullptr ? ta_tile_rows(c.M, n_tiles, ctx->sms) : c.bn;
+    p.tile_rows = rows;
+    // Boxes of X: dense tiles have one height; tiles of a list have up to `rows`, a box of the nearest quarter of that. Two K
+    // steps per copy, four where that is still small.
+    p.xbox = c.tiles == nullptr || rows <= 16 ? rows : round_up(rows / 4, 16);
+    p.nbox = rows / p.xbox;
+    p.xk = rows <= 96 ? 4 : 2;
+    p.x_stage = rows * 128 * p.xk;
+    p.dcols = rows <= 128 ? 128 : kTaMaxRows;
+    // stages: at least three of codes, then up to eight of X, then as many of codes as fit
+    const int room = kTaSmemMax - kTaSmemFixed;
+    const int c_stage = ta_code_stage(c.fmt);
+    p.nx = (room - 3 * c_stage) / p.x_stage;
+    if (p.nx > 8) p.nx = 8;
+    p.nc = (room - p.nx * p.x_stage) / c_stage;
+    if (p.nc > kTaMaxStages) p.nc = kTaMaxStages;
+    const int smem = kTaSmemFixed + p.nx * p.x_stage + p.nc * c_stage;
+
+    const int bps = c.fmt == kFmtAffine8 ? 64 : (c.fmt == kFmtTernary ? 16 : 32);
+    const uint64_t row_bytes = (uint64_t)c.K / 64 * bps;
+    TaMaps maps;
+    int32_t r = kOk;
+    for (int i = 0; i < p.nbox && r == kOk; i++)
+        r = make_map_ksteps(ctx, &maps.x[i], c.x16, (uint64_t)c.x_rows, (uint64_t)c.K / 64, (uint64_t)c.ldx * 2, p.xbox * (i + 1), p.xk);
+    const uint32_t wbox = c.epi ? 64 : 128;
+    for (int i = 0; i <= c.epi && r == kOk; i++)
+        r = make_map_2d(ctx, &maps.w[i], c.w[i], 0, row_bytes, (uint64_t)c.experts * c.N, row_bytes, 128, wbox, true);
     if (r != kOk) return r;
-    if (plain) {
-        r = make_map_2d(ctx, &mw0, c.w[0], 2, (uint64_t)c.K, (uint64_t)c.experts * c.N, (uint64_t)c.K * 2, kBK, kWRows, true);
-        mw1 = mw0;
-    } else {
-        r = make_map_2d(ctx, &mw0, c.w[0], 0, row_bytes, (uint64_t)c.experts * c.N, row_bytes, pack_row, kWRows, false);
-        if (r != kOk) return r;
-        r = make_map_2d(ctx, &mw1, c.w[1] ? c.w[1] : c.w[0], 0, row_bytes, (uint64_t)c.experts * c.N, row_bytes, pack_row,
-                        kWRows, false);
-    }
-    if (r != kOk) return r;
-    QmmParams p;
+    uintptr_t align = 0;
     for (int i = 0; i < 2; i++) {
         p.s[i] = c.s[i] ? c.s[i] : c.s[0];
         p.b[i] = c.b[i] ? c.b[i] : c.b[0];
         p.ebias[i] = c.ebias[i];
+        align |= reinterpret_cast<uintptr_t>(p.s[i]) | reinterpret_cast<uintptr_t>(p.b[i]);
     }
+    // scale bytes of a weight row, and of it per stage of codes: asynchronous copies of that size need the row pitch and the
+    // base to be multiples of it
+    const int srow = c.fmt == kFmtMxfp4 ? c.K / 32 : (c.fmt == kFmtTernary ? c.K / 64 : (c.fmt == kFmtAffine4G32 ? c.K / 16 : c.K / 32));
+    const int spb = c.fmt == kFmtAffine8 ? 4 : (c.fmt == kFmtAffine4G32 ? 16 : 8);
+    p.vec = srow % spb == 0 && (align & (uintptr_t)(spb - 1)) == 0 ? 1 : 0;
     p.expert_lo = c.expert_lo;
     p.N = c.N; p.K = c.K; p.M = c.M;
     p.tiles = c.tiles; p.ntiles = c.ntiles;
     p.y = c.y; p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
     p.limit = c.limit;
-    p.xg = c.gather_map != nullptr ? static_cast<const __half*>(c.x16) : nullptr;
-    p.gather_map = c.gather_map;
-    p.ldxg = c.ldx;
-    p.gather_div = c.gather_div;
+    p.act = c.act;
     p.status = ctx->d_status;
-    p.reserved = 0;
     int grid = ctx->sms;
     if (c.tiles == nullptr) {
-        const int work = ((c.M + c.bn - 1) / c.bn) * ((c.N + kWRows - 1) / kWRows);
+        const int work = ((c.M + rows - 1) / rows) * n_tiles;
         if (work < grid) grid = work;
     }
-    ke->fn<<<grid, c.gather_map != nullptr ? kQmmGatherThreads : kQmmThreads, ke->smem, st>>>(mx, mw0, mw1, p);
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(kTaThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, k, maps, p), "qmm launch");
+}
+
+int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
+    if (c.fmt != kFmtBf16Plain && c.fmt != kFmtInt8Plain) return launch_qmm_ta(ctx, st, c);
+    // bf16 activations and weights, or int8 rows on both sides, copied as they are
+    const KernelEntry* ke = find(c.fmt, c.bn);
+    if (ke == nullptr || c.epi != 0 || c.tiles != nullptr)
+        return fail(ctx, kErrNoKernel, "qmm: no kernel for format %d, tile %d, epilogue %d", c.fmt, c.bn, c.epi);
+    const bool i8 = c.fmt == kFmtInt8Plain;
+    const int elem = i8 ? 0 : 2, es = i8 ? 1 : 2, bke = i8 ? 128 : 64;
+    CUtensorMap mx, mw;
+    int32_t r = make_map_2d(ctx, &mx, c.x16, elem, (uint64_t)c.K, (uint64_t)c.x_rows, (uint64_t)c.ldx * es, bke, c.bn, true);
+    if (r == kOk) r = make_map_2d(ctx, &mw, c.w[0], elem, (uint64_t)c.K, (uint64_t)c.N, (uint64_t)c.K * es, bke, kWRows, true);
+    if (r != kOk) return r;
+    QmmParams p = {};
+    p.s = c.s[0]; p.b = c.b[0];
+    p.N = c.N; p.K = c.K; p.M = c.M;
+    p.y = c.y; p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
+    p.limit = c.limit;
+    p.status = ctx->d_status;
+    const int work = ((c.M + c.bn - 1) / c.bn) * ((c.N + kWRows - 1) / kWRows);
+    ke->fn<<<work < ctx->sms ? work : ctx->sms, kQmmThreads, ke->smem, st>>>(mx, mw, p);
     return check_cuda(ctx, cudaGetLastError(), "qmm launch");
 }
 
@@ -259,8 +314,7 @@ extern "C" int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dt
     }
     QmmCall c;
     c.fmt = fmt;
-    c.epi = kEpiStore;
-    c.bn = rows >= 256 ? 256 : 128;
+    c.epi = 0;
     c.x16 = x16; c.ldx = ld16; c.x_rows = rows;
     c.w[0] = m->w; c.s[0] = m->scales; c.b[0] = m->biases;
     c.experts = 1;

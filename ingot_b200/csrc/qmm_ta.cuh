@@ -1,0 +1,571 @@
+// Quantized GEMM on the 5th-generation tensor cores with the dequantised weights in tensor memory, dense and grouped
+// (MoE):
+//
+//   D[128 weight rows, up to 192 tokens] += Wd[128, 64] * X[tokens, 64]^T      per K step of 64 inputs
+//
+// Why tensor memory. With the fp16 weight tile in shared memory the K step moved 104 KB through the shared-memory port
+// (tile stores 16, MMA reads of the tile 16 and of X 32, TMA writes of X 32, codes 8: 832 cycles at 128 B per cycle) for 512
+// cycles of MMA, and ran at that port's rate. tcgen05.mma takes its A operand from tensor memory: the dequantisers write
+// there with tcgen05.st, a thread per weight row and 64 weights at a time, and what is left for the port is X (written
+// and read once) and the packed codes. The MMA itself gains as well: a step of 64 inputs with N tokens takes 2 N + 40
+// cycles with A in tensor memory and 2 N + 172 with A in shared memory (measured, operands resident).
+//
+// Tensor memory (512 columns): two accumulators of up to 192 columns and four A stages of 32 columns (64 fp16 inputs per
+// lane), or two of up to 128 columns and eight A stages. Two accumulators always: the epilogue of a tile runs under the
+// next tile's main loop, which one accumulator of 256 columns could not offer beside the A stages.
+//
+// Warp roles of one persistent CTA (768 threads):
+//   warp 0       producer of X tiles: one tensor copy brings two or four K steps of the tile (128-byte swizzle). A step of its
+//                own per copy does not do: the wait, the expected bytes and the copy's issue are a chain of 500 cycles in one
+//                thread, whatever the box
+//   warp 1       allocates tensor memory, issues tcgen05.mma (one lane), commits stages and accumulators
+//   warp 2       producer of the packed codes: a stage is 128 bytes of 128 weight rows (two to eight K steps), so that DRAM
+//                and L2 see whole lines; 128-byte swizzle, so that the dequantisers' row-wise 16-byte loads are free of bank
+//                conflicts
+//   warp 3       producer of the stage's scales and biases (asynchronous copies of a row's 4-16 bytes)
+//   warps 4-7    epilogue
+//   warps 8-23   dequantisers, four groups of four warps on every fourth K step
+// The gate/up form takes 64 gate rows and the matching 64 up rows as one tile of 128: lanes 0-15 of every warp's quadrant
+// hold gate rows, lanes 16-31 the same rows of up, so that the activation needs one shuffle per two tokens and
+// everything else is the plain form.
+// Every wait is bounded: on a timeout the kernel writes a status word, all roles drain and tensor memory is released.
+//
+// Replaces qmm_t_nax3* (Shaders/qmm_nax_v3.metal:107-256) and, with a tile list, moe_gateup_swiglu2* / moe_down2*
+// (Shaders/qmm_nax_moe.metal:442-717) of the reference.
+#pragma once
+
+#include <cuda.h>
+
+#include <type_traits>
+
+#include "common.cuh"
+#include "gqmv.cuh"
+#include "ptx.cuh"
+
+namespace iq {
+
+constexpr int kTaThreads = 768;
+constexpr int kTaGroups = 4;               // dequantiser groups of four warps
+constexpr int kTaMaxRows = 192;            // token rows per tile
+constexpr int kTaCodeStage = 128 * 128;    // bytes of a stage of packed codes
+constexpr int kTaMaxStages = 12;
+constexpr int kTaSmemMax = 232448;
+constexpr int kTaSmemFixed = 1024 + 1024;  // alignment, barriers
+
+struct TaParams {
+    const void* s[2];
+    const void* b[2];
+    int32_t expert_lo;       // first expert held here: tile.expert - expert_lo indexes the stacked tensors
+    int32_t N, K;            // weight rows per expert (gate/up: of each matrix), inputs
+    int32_t M;               // token rows (dense)
+    int32_t tile_rows;       // dense tiling: token rows per tile
+    const Tile* tiles;       // work list; null: dense tiling
+    const uint32_t* ntiles;
+    void* y;
+    int32_t y_dtype;
+    int64_t ldy;
+    int32_t accumulate;
+    const float* ebias[2];   // fp32 [E, N] or null
+    float limit;
+    int32_t act;
+    // X copies: a tile of r rows takes the smallest box of xbox * (i + 1) rows, i < nbox, that holds it, xk K steps at a time
+    int32_t xbox, nbox, xk;
+    int32_t nx, nc;          // stages of X and of codes
+    int32_t x_stage;         // bytes of an X stage
+    int32_t dcols;           // columns per accumulator: 128 or 192
+    int32_t vec;             // the row pitch of the scales allows asynchronous copies
+    int32_t* status;
+};
+
+struct TaMaps {
+    CUtensorMap x[4], w[2];
+};
+
+// Shared-memory and instruction descriptors: K-major B tile with 128-byte swizzle (rows of 128 bytes, 8-row groups 1024
+// bytes apart), fp16 operands, fp32 accumulator, M = 128.
+__device__ __forceinline__ uint64_t ta_desc_sw128(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)2 << 61);
+}
+__device__ __forceinline__ uint32_t ta_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
+
+// D[128, N] (+)= A[128, 16] (tensor memory: lane = row, two inputs per column) * B[N, 16]^T (shared memory)
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,"
+        "%31,%32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
+        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
+        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// ---- formats ----------------------------------------------------------------------------------------------------------
+// KPS: K steps of 64 inputs per stage of codes (128 bytes of a row); BPS: code bytes of a row per step.
+template <int FMT>
+struct TaFmt {
+    static constexpr int BPS = FMT == kFmtAffine8 ? 64 : (FMT == kFmtTernary ? 16 : 32);
+    static constexpr int KPS = 128 / BPS;
+    static constexpr int GROUP = (FMT == kFmtMxfp4 || FMT == kFmtAffine4G32) ? 32 : (FMT == kFmtTernary ? 128 : 64);
+    static constexpr bool BIAS = FMT == kFmtAffine4 || FMT == kFmtAffine8 || FMT == kFmtAffine4G32;
+    static constexpr int ES = FMT == kFmtMxfp4 ? 1 : 2;           // bytes of a scale
+    static constexpr int SPB = 64 * KPS / GROUP * ES;             // scale bytes of a row per stage of codes: 4, 8 or 16
+    static constexpr int STAGE = kTaCodeStage + 128 * SPB * (BIAS ? 2 : 1);
+};
+inline int ta_code_stage(int32_t fmt) {
+    switch (fmt) {
+        case kFmtAffine4: return TaFmt<kFmtAffine4>::STAGE;
+        case kFmtAffine8: return TaFmt<kFmtAffine8>::STAGE;
+        case kFmtMxfp4: return TaFmt<kFmtMxfp4>::STAGE;
+        case kFmtAffine4G32: return TaFmt<kFmtAffine4G32>::STAGE;
+        default: return TaFmt<kFmtTernary>::STAGE;
+    }
+}
+
+// 64 consecutive inputs of one weight row -> 32 registers of two fp16 weights each, in input order. codes: the row's
+// 128-byte line in the stage (sw = row % 8: the swizzle), unit: the step's first 16-byte piece of it. sc / bi: the step's
+// scale and bias bits (group of 32: two of each, the later one in the upper half).
+template <int FMT>
+__device__ __forceinline__ void ta_dequant64(uint32_t codes, uint32_t unit, uint32_t sw, uint32_t sc, uint32_t bi, uint32_t (&o)[32]) {
+    if (FMT == kFmtAffine4 || FMT == kFmtAffine4G32) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint4 v = lds128(codes + (((unit + h) ^ sw) << 4));
+            const uint32_t sb = FMT == kFmtAffine4G32 ? (h ? sc >> 16 : sc & 0xFFFFu) : sc;
+            const uint32_t bb = FMT == kFmtAffine4G32 ? (h ? bi >> 16 : bi & 0xFFFFu) : bi;
+            const float s = bf16_bits_to_f32(sb), b = bf16_bits_to_f32(bb);
+            const uint32_t s2 = pack_half2(s, s), b2 = pack_half2(b, b);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    // byte j of the word holds inputs 2j (low nibble) and 2j + 1: (1024 + q_lo, 1024 + 16 q_hi), brought to
+                    // (q_lo, q_hi) by one exact fma, then w = fma(q, s, b) rounded once
+                    const uint32_t t = (__byte_perm(w[i], 0u, 0x4040 + 0x0101 * j) & 0x00F0000Fu) | 0x64006400u;
+                    o[h * 16 + i * 4 + j] = hfma2_u32(hfma2_u32(t, 0x2C003C00u, 0xD400E400u), s2, b2);
+                }
+        }
+    } else if (FMT == kFmtAffine8) {
+        const float s = bf16_bits_to_f32(sc), b = bf16_bits_to_f32(bi);
+        const uint32_t s2 = pack_half2(s, s), b2 = pack_half2(b, b);
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            const uint4 v = lds128(codes + (((unit + h) ^ sw) << 4));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const uint32_t t = __byte_perm(w[i], 0x64646464u, j ? 0x4342 : 0x4140);  // 1024 + q
+                    o[h * 8 + i * 2 + j] = dq_pair(t, s2, b2);
+                }
+        }
+    } else if (FMT == kFmtTernary) {
+        // 64 codes of two bits in 16 bytes; w = (q - 1) * s with the fp16 scale as it is stored: exact in fp16
+        const uint4 v = lds128(codes + ((unit ^ sw) << 4));
+        const uint32_t s2 = (sc & 0xFFFFu) | (sc << 16);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                // inputs 2j and 2j + 1 are the bits 4j..4j+1 and 4j+2..4j+3: multiplying by 1 + 2^14 puts the second pair
+                // at bit 16; 1024 + q, then (q - 1) * s
+                const uint32_t n = (w[i] >> (4 * j)) & 0xFu;
+                const uint32_t t = ((n * 0x4001u) & 0x00030003u) | 0x64006400u;
+                __half2 q = __hsub2(*reinterpret_cast<const __half2*>(&t), __half2half2(__ushort_as_half(0x6401)));
+                o[i * 8 + j] = hmul2_u32(*reinterpret_cast<uint32_t*>(&q), s2);
+            }
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint4 v = lds128(codes + (((unit + h) ^ sw) << 4));
+            const DqConst d = make_dq<kFmtMxfp4>((sc >> (8 * h)) & 0xFFu);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                uint32_t q[4];
+                cvt_e2m1x8(w[i], q);
+#pragma unroll
+                for (int j = 0; j < 4; j++) o[h * 16 + i * 4 + j] = hmul2_u32(q[j], d.s2);
+            }
+        }
+    }
+}
+
+// EPI: 0 store, 1 gate + up + activation.
+template <int FMT, int EPI>
+__global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_constant__ TaMaps maps, const TaParams p) {
+    using F = TaFmt<FMT>;
+    constexpr int KPS = F::KPS;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t codes0 = smem_u32(smem), x0 = codes0 + p.nc * kTaCodeStage;  // codes, X, scales
+    const uint32_t scales0 = x0 + p.nx * p.x_stage;
+    constexpr int SSTAGE = F::STAGE - kTaCodeStage;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)p.nc * F::STAGE + (size_t)p.nx * p.x_stage);
+    const uint32_t bar_cfull = smem_u32(bars), bar_cempty = bar_cfull + 8 * kTaMaxStages, bar_xfull = bar_cempty + 8 * kTaMaxStages;
+    const uint32_t bar_xempty = bar_xfull + 8 * kTaMaxStages, bar_aready = bar_xempty + 8 * kTaMaxStages;
+    const uint32_t bar_aempty = bar_aready + 64, bar_tfull = bar_aempty + 64, bar_tempty = bar_tfull + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * kTaMaxStages + 20);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < p.nc; i++) {
+            mbar_init(bar_cfull + 8 * i, 1 + 32);  // the codes' copy, the scale producer's lanes
+            mbar_init(bar_cempty + 8 * i, 4 * (KPS < kTaGroups ? KPS : kTaGroups));
+        }
+        for (int i = 0; i < p.nx; i++) {
+            mbar_init(bar_xfull + 8 * i, 1);
+            mbar_init(bar_xempty + 8 * i, 1);
+        }
+        for (int i = 0; i < 8; i++) {
+            mbar_init(bar_aready + 8 * i, 4);
+            mbar_init(bar_aempty + 8 * i, 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(bar_tfull + 8 * i, 1);
+            mbar_init(bar_tempty + 8 * i, 4);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
+    // The weights do not depend on the previous kernel of the stream: with dense tiling their producers and the dequantisers
+    // start at once; a tile list, the activations and y do.
+    if (p.tiles != nullptr || !(warp == 2 || warp == 3 || warp >= 8)) pdl_wait();
+
+    // ---- work list --------------------------------------------------------------------------------------------------
+    constexpr int NROWS = EPI ? 64 : 128;  // output features per tile
+    const int n_tiles = (p.N + NROWS - 1) / NROWS;
+    const int m_tiles = p.tiles != nullptr ? (int)(*p.ntiles) : (p.M + p.tile_rows - 1) / p.tile_rows;
+    const int total = m_tiles * n_tiles;
+    const int ksteps = p.K / 64, chunks = (ksteps + KPS - 1) / KPS;
+    const int na = p.dcols == 128 ? 8 : 4;
+    const uint32_t tmem_a = tmem + 2 * p.dcols;
+    auto decode = [&](int wi, int& expert, int& row0, int& rows, int& n0) {
+        if (p.tiles != nullptr) {
+            const Tile t = p.tiles[wi / n_tiles];
+            expert = (int)t.expert - p.expert_lo; row0 = (int)t.start; rows = (int)t.count;
+            n0 = (wi % n_tiles) * NROWS;
+        } else {
+            expert = 0; row0 = (wi % m_tiles) * p.tile_rows; rows = min(p.tile_rows, p.M - row0);
+            n0 = (wi / m_tiles) * NROWS;
+        }
+    };
+
+    if (warp == 0) {
+        // ================= X producer =================
+        if (elect_one()) {
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
+                int expert, row0, rows, n0;
+                decode(wi, expert, row0, rows, n0);
+                const int bi = (rows - 1) / p.xbox;
+                const CUtensorMap* const map = &maps.x[bi];
+                const uint32_t bytes = (uint32_t)(p.xbox * (bi + 1) * p.xk * 128);
+                for (int ks = 0; ks < ksteps; ks += p.xk) {
+                    if (!(ok = mbar_wait(bar_xempty + 8 * s, ph ^ 1, abort_flag))) break;
+                    mbar_arrive_expect_tx(bar_xfull + 8 * s, bytes);
+                    tma_load_3d(x0 + s * p.x_stage, map, bar_xfull + 8 * s, 0, row0, ks);
+                    if (++s == p.nx) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 2) {
+        // ================= producer of the packed codes =================
+        if (elect_one()) {
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
+                int expert, row0, rows, n0;
+                decode(wi, expert, row0, rows, n0);
+                const int wrow = expert * p.N + n0;
+                for (int ch = 0; ch < chunks; ch++) {
+                    if (!(ok = mbar_wait(bar_cempty + 8 * s, ph ^ 1, abort_flag))) break;
+                    mbar_arrive_expect_tx(bar_cfull + 8 * s, kTaCodeStage);
+                    const uint32_t dst = codes0 + s * kTaCodeStage;
+                    tma_load_2d(dst, &maps.w[0], bar_cfull + 8 * s, ch * 128, wrow);
+                    if (EPI) tma_load_2d(dst + kTaCodeStage / 2, &maps.w[1], bar_cfull + 8 * s, ch * 128, wrow);
+                    if (++s == p.nc) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 3) {
+        // ================= producer of the scales and biases =================
+        // Per stage of codes the SPB scale bytes of each of the 128 rows: lane l takes rows l, l + 32, ... Row pitches that
+        // allow it go by asynchronous copies, others (an odd number of groups) by two-byte loads. Rows beyond the matrix
+        // are left out: their weights only feed rows of D that are not stored.
+        constexpr int SPB = F::SPB, NT = F::BIAS ? 2 : 1;
+        const size_t pitch = (size_t)p.K / F::GROUP * F::ES;
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
+            int expert, row0, rows, n0;
+            decode(wi, expert, row0, rows, n0);
+            const char* src[4][NT];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int row = lane + 32 * i, mi = EPI ? i >> 1 : 0, n = n0 + (EPI ? row & 63 : row);
+                const size_t o = ((size_t)expert * p.N + n) * pitch;
+                src[i][0] = n < p.N ? static_cast<const char*>(p.s[mi]) + o : nullptr;
+                if (NT == 2) src[i][NT - 1] = n < p.N ? static_cast<const char*>(p.b[mi]) + o : nullptr;
+            }
+            for (int ch = 0; ch < chunks; ch++) {
+                ok = mbar_wait(bar_cempty + 8 * s, ph ^ 1, abort_flag);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                const uint32_t dst = scales0 + s * SSTAGE;
+                const int left = (int)pitch - ch * SPB;  // scale bytes of a row from this stage on
+                if (p.vec) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int t = 0; t < NT; t++)
+                            if (src[i][t] != nullptr) cp_async_ca<SPB>(dst + t * 128 * SPB + (lane + 32 * i) * SPB, src[i][t] + ch * SPB);
+                } else {
+                    uint32_t v[4][NT][SPB / 2];
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int t = 0; t < NT; t++)
+#pragma unroll
+                            for (int e = 0; e < SPB / 2; e++)
+                                v[i][t][e] = src[i][t] != nullptr && 2 * e < left ? ldg_nc_u16(src[i][t] + ch * SPB + 2 * e) : 0u;
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int t = 0; t < NT; t++)
+#pragma unroll
+                            for (int e = 0; e < SPB / 4; e++)
+                                sts32(dst + t * 128 * SPB + (lane + 32 * i) * SPB + 4 * e, v[i][t][2 * e] | (v[i][t][2 * e + 1] << 16));
+                }
+                cp_async_arrive_noinc(bar_cfull + 8 * s);
+                if (++s == p.nc) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // ================= MMA issuer =================
+        if (elect_one()) {
+            int xs = 0, as = 0, acc = 0;
+            uint32_t xph = 0, aph = 0, tph = 0;
+            bool ok = true;
+            for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
+                int expert, row0, rows, n0;
+                decode(wi, expert, row0, rows, n0);
+                const uint32_t idesc = ta_idesc((rows + 15) & ~15);
+                if (!(ok = mbar_wait(bar_tempty + 8 * acc, tph ^ 1, abort_flag))) break;
+                tc_fence_after();
+                const uint32_t td = tmem + acc * p.dcols;
+                const uint32_t kbytes = (uint32_t)(p.xbox * ((rows - 1) / p.xbox + 1) * 128);  // from one K step of a stage to the next
+                for (int ks0 = 0; ks0 < ksteps && ok; ks0 += p.xk) {
+                    if (!(ok = mbar_wait(bar_xfull + 8 * xs, xph, abort_flag))) break;
+                    const int ks1 = min(ksteps, ks0 + p.xk);
+                    uint32_t xa = x0 + xs * p.x_stage;
+                    for (int ks = ks0; ks < ks1; ks++, xa += kbytes) {
+                        if (!(ok = mbar_wait(bar_aready + 8 * as, aph, abort_flag))) break;
+                        tc_fence_after();
+                        const uint64_t bdesc = ta_desc_sw128(xa);
+                        const uint32_t ta = tmem_a + as * 32;
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(td, ta + 8 * kk, bdesc + 2 * kk, idesc, (ks | kk) ? 1u : 0u);
+                        umma_commit(bar_aempty + 8 * as);
+                        if (++as == na) { as = 0; aph ^= 1; }
+                    }
+                    umma_commit(bar_xempty + 8 * xs);
+                    if (++xs == p.nx) { xs = 0; xph ^= 1; }
+                }
+                if (ok) umma_commit(bar_tfull + 8 * acc);
+                acc ^= 1;
+                if (acc == 0) tph ^= 1;
+            }
+        }
+    } else if (warp >= 8) {
+        // ================= dequantisers =================
+        // Group g converts the steps whose number, counted over all tiles of the CTA, is g modulo 4, a thread per weight row
+        // (never by the step's number in its tile: a group that skips the end of a tile would wait on an A stage more than
+        // one round ahead, which a phase bit cannot tell from this round). One warp's step is a chain of latencies
+        // (barrier, shared-memory round trip, conversion, tensor-memory store and its completion, about 1000 cycles); four
+        // groups keep four of them under way.
+        const int grp = (warp - 8) >> 2, q = warp & 3;
+        const int row = EPI ? (lane >> 4) * 64 + q * 16 + (lane & 15) : q * 32 + lane;  // row of the stage
+        const uint32_t sw = row & 7;
+        const uint32_t my_a = tmem_a + ((uint32_t)(32 * q) << 16);
+        constexpr int SPB = F::SPB;
+        const int nash = na == 8 ? 3 : 2;
+        uint32_t it0 = 0;     // steps of the tiles before
+        int cs = 0;           // stage of codes
+        uint32_t cph = 0;
+        bool ok = true;
+        for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
+            for (int ch = 0; ch < chunks; ch++) {
+                const int j0 = (grp - (int)it0 - ch * KPS) & (kTaGroups - 1);  // this group's first step of the stage
+                if (j0 < KPS) {  // (8-bit codes have two steps per stage: two groups take it)
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_cfull + 8 * cs, cph, abort_flag));
+                    if (!ok) break;
+                    const uint32_t codes = codes0 + cs * kTaCodeStage + row * 128, scales = scales0 + cs * SSTAGE + row * SPB;
+#pragma unroll
+                    for (int i = 0; i < (KPS + kTaGroups - 1) / kTaGroups; i++) {
+                        const int j = j0 + kTaGroups * i;
+                        const int ks = ch * KPS + j;
+                        if (ks >= ksteps) break;
+                        uint32_t sc, bi = 0;
+                        if (FMT == kFmtAffine4G32) {
+                            sc = lds32(scales + 4 * j);
+                            bi = lds32(scales + 128 * SPB + 4 * j);
+                        } else {
+                            sc = lds_u16(scales + 2 * (FMT == kFmtTernary ? j >> 1 : j));
+                            if (F::BIAS) bi = lds_u16(scales + 128 * SPB + 2 * j);
+                        }
+                        uint32_t o[32];
+                        ta_dequant64<FMT>(codes, (uint32_t)(j * (F::BPS / 16)), sw, sc, bi, o);
+                        const uint32_t it = it0 + ks, as = it & (na - 1), aph = (it >> nash) & 1;
+                        ok = __all_sync(0xffffffffu, mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
+                        if (!ok) break;
+                        tc_fence_after();
+                        tmem_st32(my_a + as * 32, o);
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_aready + 8 * as);
+                    }
+                    if (!ok) break;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_cempty + 8 * cs);
+                }
+                if (++cs == p.nc) { cs = 0; cph ^= 1; }
+            }
+            it0 += ksteps;
+        }
+    } else {
+        // ================= epilogue (warps 4-7) =================
+        const int q = warp & 3;
+        const int mi = EPI ? lane >> 4 : 0;
+        const int nl = EPI ? q * 16 + (lane & 15) : q * 32 + lane;
+        int acc = 0;
+        uint32_t tph = 0;
+        for (int wi = blockIdx.x; wi < total; wi += gridDim.x) {
+            int expert, row0, rows, n0;
+            decode(wi, expert, row0, rows, n0);
+            const int n = n0 + nl;
+            const bool n_ok = n < p.N;
+            const float* eb = mi ? p.ebias[1] : p.ebias[0];
+            const float bias = eb != nullptr && n_ok ? eb[(size_t)expert * p.N + n] : 0.f;
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * acc, tph, abort_flag))) break;
+            tc_fence_after();
+            const uint32_t td = tmem + acc * p.dcols + ((uint32_t)(32 * q) << 16);
+            constexpr int CW = 16;  // token columns at a time
+            for (int c0 = 0; c0 < rows; c0 += CW) {
+                uint32_t r[CW];
+                tmem_ld16(td + c0, r);
+                tmem_ld_wait();
+                const int live = rows - c0;  // columns j < live exist
+                if (EPI) {
+                    // lanes l and l + 16 hold gate and up of one feature: the lower lane finishes token j, the upper token j + 1
+                    float g[CW / 2], u[CW / 2];
+#pragma unroll
+                    for (int j = 0; j < CW / 2; j++) {
+                        const float a = __uint_as_float(r[2 * j]) + bias, b = __uint_as_float(r[2 * j + 1]) + bias;
+                        const float other = __shfl_xor_sync(0xffffffffu, mi ? a : b, 16);
+                        g[j] = mi ? other : a;
+                        u[j] = mi ? b : other;
+                    }
+                    auto act = [&](auto tag) {
+#pragma unroll
+                        for (int j = 0; j < CW / 2; j++) g[j] = glu<decltype(tag)::value>(g[j], u[j], p.limit);
+                    };
+                    if (p.act == kActSilu) act(std::integral_constant<int, kActSilu>{});
+                    else if (p.act == kActSwigluOai) act(std::integral_constant<int, kActSwigluOai>{});
+                    else if (p.act == kActGelu) act(std::integral_constant<int, kActGelu>{});
+                    else act(std::integral_constant<int, kActRelu2>{});
+                    __half* yp = reinterpret_cast<__half*>(p.y) + (size_t)(row0 + c0 + mi) * p.ldy + n;
+#pragma unroll
+                    for (int j = 0; j < CW / 2; j++)
+                        if (n_ok && 2 * j + mi < live) yp[(size_t)(2 * j) * p.ldy] = __float2half_rn(g[j]);
+                } else {
+                    const size_t o0 = (size_t)(row0 + c0) * p.ldy + n;
+                    auto store = [&](auto load_f, auto store_f) {
+                        float v[CW];
+#pragma unroll
+                        for (int j = 0; j < CW; j++) v[j] = __uint_as_float(r[j]) + bias;
+                        if (p.accumulate) {  // all loads before the first store
+                            float old[CW];
+#pragma unroll
+                            for (int j = 0; j < CW; j++) old[j] = n_ok && j < live ? load_f(o0 + (size_t)j * p.ldy) : 0.f;
+#pragma unroll
+                            for (int j = 0; j < CW; j++) v[j] = old[j] + v[j];
+                        }
+#pragma unroll
+                        for (int j = 0; j < CW; j++)
+                            if (n_ok && j < live) store_f(o0 + (size_t)j * p.ldy, v[j]);
+                    };
+                    if (p.y_dtype == kF32) {
+                        float* y = reinterpret_cast<float*>(p.y);
+                        store([&](size_t o) { return y[o]; }, [&](size_t o, float f) { y[o] = f; });
+                    } else if (p.y_dtype == kF16) {
+                        __half* y = reinterpret_cast<__half*>(p.y);
+                        store([&](size_t o) { return __half2float(y[o]); }, [&](size_t o, float f) { y[o] = __float2half_rn(f); });
+                    } else {
+                        uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
+                        store([&](size_t o) { return bf16_bits_to_f32(y[o]); },
+                              [&](size_t o, float f) { y[o] = (uint16_t)f32_to_bf16_bits(f); });
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+            acc ^= 1;
+            if (acc == 0) tph ^= 1;
+        }
+    }
+
+    __syncwarp();
+    // ---- teardown ---------------------------------------------------------------------------------------------------
+    if (*abort_flag && (warp == 0 || warp == 2)) {  // copies in flight land before the shared memory is given back
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) {}
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag && threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, kErrTimeout);
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+}  // namespace iq
