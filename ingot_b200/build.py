@@ -13,11 +13,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libingot_qmm.so")
+PYCALL = os.path.join(LIBDIR, "_iqcall.so")
 SOURCES = ["api.cu", "qmv.cu", "moe.cu", "qmm.cu", "ep.cu", "colsplit.cu", "loader.cu", "sample.cu", "embed.cu", "tern.cu", "w8a8.cu"]
 
 NVCC_FLAGS = [
@@ -62,8 +64,19 @@ def _compile(src: str, force: bool, verbose: bool) -> str:
     return obj
 
 
+def _build_pycall(force: bool):
+    """The CPython extension through which the hot entry points are called (csrc/pycall.c)."""
+    src = os.path.join(CSRC, "pycall.c")
+    if force or _deps_newer(PYCALL, [src, os.path.join(HERE, "..", "include", "ingot_qmm.h")]):
+        cmd = [shutil.which("gcc") or "cc", "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], src, "-o", PYCALL]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"the call extension failed to build:\n{r.stdout}\n{r.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIBDIR, exist_ok=True)
+    _build_pycall(force)
     srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
         objs = list(ex.map(lambda s: _compile(s, force, verbose), srcs))

@@ -2,10 +2,13 @@
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libingot_qmm.so")
+CALL_PATH = os.path.join(HERE, "lib", "_iqcall.so")
 
 IQ_F32, IQ_F16, IQ_BF16 = 0, 1, 2
 IQ_MODE_AFFINE, IQ_MODE_MXFP4 = 0, 1
@@ -181,6 +184,27 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_call = None
+
+
+def call():
+    """The hot entry points as plain functions of integers (csrc/pycall.c), bound to the loaded library: what a launch costs
+    on the host without ctypes' argument conversion."""
+    global _call
+    if _call is None:
+        l = lib()
+        if not os.path.exists(CALL_PATH):
+            raise RuntimeError(f"{CALL_PATH} is missing: build it with `python -m ingot_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_iqcall", CALL_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_iqcall", CALL_PATH, loader=loader))
+        loader.exec_module(mod)
+        for name in ("iq_qmv", "iq_qmm", "iq_dense_ffn", "iq_moe_forward", "iq_rmsnorm", "iq_had_rows", "iq_embed_rows",
+                     "iq_argmax_rows", "iq_topk64"):
+            mod.bind(name, C.cast(getattr(l, name), C.c_void_p).value)
+        _call = mod
+    return _call
+
+
 class Context:
     """One device context (iq_ctx). Mirrors the reference's MetalContext role: device + kernel configuration."""
 
@@ -190,6 +214,7 @@ class Context:
         if st != 0:
             raise IngotError(st, lib().iq_strerror(st).decode() + f" (iq_ctx_create on device {device})")
         self.device = device
+        self.address = self._h.value  # the handle as an integer, for call()
 
     @property
     def handle(self):
@@ -213,6 +238,7 @@ class Context:
         if self._h:
             lib().iq_ctx_destroy(self._h)
             self._h = C.c_void_p()
+            self.address = 0
 
     def __del__(self):
         try:
@@ -225,6 +251,7 @@ _contexts = {}
 
 
 def context(device: int = 0) -> Context:
-    if device not in _contexts:
-        _contexts[device] = Context(device)
-    return _contexts[device]
+    ctx = _contexts.get(device)
+    if ctx is None:
+        ctx = _contexts[device] = Context(device)
+    return ctx

@@ -53,6 +53,32 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         }
     }
 }
+// A look at a barrier without waiting, for software pipelining: asked early, its latency (about 100 cycles) passes under the
+// instructions that follow, and mbar_wait_hint only waits when the answer was no. The wait spins on test_wait: a try_wait
+// that finds the phase open sleeps in steps of about 250 cycles.
+__device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok;
+}
+__device__ __forceinline__ bool mbar_wait_hint(uint32_t hint, uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (hint) return true;
+    const long long t0 = clock64();
+    while (true) {
+        if (mbar_test(bar, parity)) return true;
+        if (*abort_flag) return false;
+        if ((unsigned long long)(clock64() - t0) > kWaitCycles) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+}
 // The same wait for roles that are far from the critical path (a whole main loop away): sleeps between polls so that
 // the polling does not take issue slots from the warps doing the work.
 __device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, volatile int* abort_flag) {

@@ -60,16 +60,15 @@ TaKernel ta_pick(int32_t fmt, int epi) {
 }
 
 // Token rows per tile of a dense GEMM: the height (a multiple of 16, at most 192) with the least (waves over the SMs) x
-// (time of a tile). A K step costs the MMA in proportion to the height, and the conversion of its 128 x 64 weights about as
-// much as 128 tokens whatever the height. 512 tokens x 14336 features: five tiles of 112 rows are 560 work items in
-// four waves of cost 128, three of 176 would be 336 items in three waves of 176.
+// (time of a tile). A K step takes the MMA 2 h + 40 cycles for h tokens, and its issue and hand-overs about 400 whatever the
+// height, so lower tiles than 176 rows only pay when they save a wave.
 int ta_tile_rows(int m, int n_tiles, int sms) {
     int best = 16;
     long long best_cost = -1;
     for (int tiles = (m + kTaMaxRows - 1) / kTaMaxRows; tiles <= (m + 15) / 16; tiles++) {
         const int h = round_up((m + tiles - 1) / tiles, 16);
         const long long waves = ((long long)((m + h - 1) / h) * n_tiles + sms - 1) / sms;
-        const long long cost = waves * (h > 128 ? h : 128);
+        const long long cost = waves * (h > 176 ? h : 176);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = h; }
         if (h <= 64) break;
     }
@@ -180,7 +179,7 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     // steps per copy, four where that is still small.
     p.xbox = c.tiles == nullptr || rows <= 16 ? rows : round_up(rows / 4, 16);
     p.nbox = rows / p.xbox;
-    p.xk = rows <= 96 ? 4 : 2;
+    p.xk = rows <= 128 ? 4 : 2;
     p.x_stage = rows * 128 * p.xk;
     p.dcols = rows <= 128 ? 128 : kTaMaxRows;
     // stages: at least three of codes, then up to eight of X, then as many of codes as fit

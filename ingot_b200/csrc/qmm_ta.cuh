@@ -82,11 +82,8 @@ struct TaMaps {
 };
 
 // Shared-memory and instruction descriptors: K-major B tile with 128-byte swizzle (rows of 128 bytes, 8-row groups 1024
-// bytes apart), fp16 operands, fp32 accumulator, M = 128.
-__device__ __forceinline__ uint64_t ta_desc_sw128(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
-}
+// bytes apart; the low 14 bits take the address in units of 16 bytes), fp16 operands, fp32 accumulator, M = 128.
+constexpr uint64_t kTaDescHi = ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 __device__ __forceinline__ uint32_t ta_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
 
 // D[128, N] (+)= A[128, 16] (tensor memory: lane = row, two inputs per column) * B[N, 16]^T (shared memory)
@@ -97,15 +94,11 @@ __device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, ui
         ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,"
-        "%31,%32};"
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -140,52 +133,48 @@ inline int ta_code_stage(int32_t fmt) {
     }
 }
 
-// 64 consecutive inputs of one weight row -> 32 registers of two fp16 weights each, in input order. codes: the row's
-// 128-byte line in the stage (sw = row % 8: the swizzle), unit: the step's first 16-byte piece of it. sc / bi: the step's
-// scale and bias bits (group of 32: two of each, the later one in the upper half).
+// 32 consecutive inputs of one weight row -> 16 registers of two fp16 weights each, in input order. codes: the row's
+// 128-byte line in the stage (sw = row % 8: the swizzle), unit: the first 16-byte piece of them in it (ternary: of the 64
+// inputs, half h). sc / bi: the scale and bias bits.
 template <int FMT>
-__device__ __forceinline__ void ta_dequant64(uint32_t codes, uint32_t unit, uint32_t sw, uint32_t sc, uint32_t bi, uint32_t (&o)[32]) {
+__device__ __forceinline__ void ta_dequant32(uint32_t codes, uint32_t unit, int h, uint32_t sw, uint32_t sc, uint32_t bi,
+                                             uint32_t (&o)[16]) {
     if (FMT == kFmtAffine4 || FMT == kFmtAffine4G32) {
+        const uint4 v = lds128(codes + ((unit ^ sw) << 4));
+        const float s = bf16_bits_to_f32(sc), b = bf16_bits_to_f32(bi);
+        const uint32_t s2 = pack_half2(s, s), b2 = pack_half2(b, b);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint4 v = lds128(codes + (((unit + h) ^ sw) << 4));
-            const uint32_t sb = FMT == kFmtAffine4G32 ? (h ? sc >> 16 : sc & 0xFFFFu) : sc;
-            const uint32_t bb = FMT == kFmtAffine4G32 ? (h ? bi >> 16 : bi & 0xFFFFu) : bi;
-            const float s = bf16_bits_to_f32(sb), b = bf16_bits_to_f32(bb);
-            const uint32_t s2 = pack_half2(s, s), b2 = pack_half2(b, b);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        for (int i = 0; i < 4; i++)
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    // byte j of the word holds inputs 2j (low nibble) and 2j + 1: (1024 + q_lo, 1024 + 16 q_hi), brought to
-                    // (q_lo, q_hi) by one exact fma, then w = fma(q, s, b) rounded once
-                    const uint32_t t = (__byte_perm(w[i], 0u, 0x4040 + 0x0101 * j) & 0x00F0000Fu) | 0x64006400u;
-                    o[h * 16 + i * 4 + j] = hfma2_u32(hfma2_u32(t, 0x2C003C00u, 0xD400E400u), s2, b2);
-                }
-        }
+            for (int j = 0; j < 4; j++) {
+                // byte j of the word holds inputs 2j (low nibble) and 2j + 1: (1024 + q_lo, 1024 + 16 q_hi), brought to
+                // (q_lo, q_hi) by one exact fma, then w = fma(q, s, b) rounded once
+                const uint32_t t = (__byte_perm(w[i], 0u, 0x4040 + 0x0101 * j) & 0x00F0000Fu) | 0x64006400u;
+                o[i * 4 + j] = hfma2_u32(hfma2_u32(t, 0x2C003C00u, 0xD400E400u), s2, b2);
+            }
     } else if (FMT == kFmtAffine8) {
         const float s = bf16_bits_to_f32(sc), b = bf16_bits_to_f32(bi);
         const uint32_t s2 = pack_half2(s, s), b2 = pack_half2(b, b);
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-            const uint4 v = lds128(codes + (((unit + h) ^ sw) << 4));
+        for (int q = 0; q < 2; q++) {
+            const uint4 v = lds128(codes + (((unit + q) ^ sw) << 4));
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
                     const uint32_t t = __byte_perm(w[i], 0x64646464u, j ? 0x4342 : 0x4140);  // 1024 + q
-                    o[h * 8 + i * 2 + j] = dq_pair(t, s2, b2);
+                    o[q * 8 + i * 2 + j] = dq_pair(t, s2, b2);
                 }
         }
     } else if (FMT == kFmtTernary) {
-        // 64 codes of two bits in 16 bytes; w = (q - 1) * s with the fp16 scale as it is stored: exact in fp16
-        const uint4 v = lds128(codes + ((unit ^ sw) << 4));
+        // 32 codes of two bits in eight bytes; w = (q - 1) * s with the fp16 scale as it is stored: exact in fp16
+        const uint2 v = lds64(codes + ((unit ^ sw) << 4) + 8 * h);
         const uint32_t s2 = (sc & 0xFFFFu) | (sc << 16);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        const uint32_t w[2] = {v.x, v.y};
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < 2; i++)
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 // inputs 2j and 2j + 1 are the bits 4j..4j+1 and 4j+2..4j+3: multiplying by 1 + 2^14 puts the second pair
@@ -196,18 +185,15 @@ __device__ __forceinline__ void ta_dequant64(uint32_t codes, uint32_t unit, uint
                 o[i * 8 + j] = hmul2_u32(*reinterpret_cast<uint32_t*>(&q), s2);
             }
     } else {
+        const uint4 v = lds128(codes + ((unit ^ sw) << 4));
+        const DqConst d = make_dq<kFmtMxfp4>(sc);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint4 v = lds128(codes + (((unit + h) ^ sw) << 4));
-            const DqConst d = make_dq<kFmtMxfp4>((sc >> (8 * h)) & 0xFFu);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        for (int i = 0; i < 4; i++) {
+            uint32_t q[4];
+            cvt_e2m1x8(w[i], q);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                uint32_t q[4];
-                cvt_e2m1x8(w[i], q);
-#pragma unroll
-                for (int j = 0; j < 4; j++) o[h * 16 + i * 4 + j] = hmul2_u32(q[j], d.s2);
-            }
+            for (int j = 0; j < 4; j++) o[i * 4 + j] = hmul2_u32(q[j], d.s2);
         }
     }
 }
@@ -379,34 +365,41 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
+        // Every barrier is asked one step ahead, before the MMAs of the current step are issued: three waits in a row per two
+        // steps, each a round trip of 100 cycles and more, cost 5 %. What is left, some 400 cycles of this one thread per step,
+        // is the bound of tiles with fewer than about 180 tokens (more state in the loop, such as answers asked two steps
+        // ahead or pairs of steps on one barrier, measured slower).
         if (elect_one()) {
             int xs = 0, as = 0, acc = 0;
             uint32_t xph = 0, aph = 0, tph = 0;
+            uint32_t a_hint = 0, x_hint = 0;
+            const uint32_t xdesc0 = (x0 & 0x3FFFFu) >> 4;
             bool ok = true;
             for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
                 int expert, row0, rows, n0;
                 decode(wi, expert, row0, rows, n0);
                 const uint32_t idesc = ta_idesc((rows + 15) & ~15);
-                if (!(ok = mbar_wait(bar_tempty + 8 * acc, tph ^ 1, abort_flag))) break;
-                tc_fence_after();
+                if (!(ok = mbar_wait_hint(0, bar_tempty + 8 * acc, tph ^ 1, abort_flag))) break;
                 const uint32_t td = tmem + acc * p.dcols;
-                const uint32_t kbytes = (uint32_t)(p.xbox * ((rows - 1) / p.xbox + 1) * 128);  // from one K step of a stage to the next
+                const uint32_t kunits = (uint32_t)(p.xbox * ((rows - 1) / p.xbox + 1) * 8);
                 for (int ks0 = 0; ks0 < ksteps && ok; ks0 += p.xk) {
-                    if (!(ok = mbar_wait(bar_xfull + 8 * xs, xph, abort_flag))) break;
+                    if (!(ok = mbar_wait_hint(x_hint, bar_xfull + 8 * xs, xph, abort_flag))) break;
                     const int ks1 = min(ksteps, ks0 + p.xk);
-                    uint32_t xa = x0 + xs * p.x_stage;
-                    for (int ks = ks0; ks < ks1; ks++, xa += kbytes) {
-                        if (!(ok = mbar_wait(bar_aready + 8 * as, aph, abort_flag))) break;
-                        tc_fence_after();
-                        const uint64_t bdesc = ta_desc_sw128(xa);
-                        const uint32_t ta = tmem_a + as * 32;
-#pragma unroll
-                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(td, ta + 8 * kk, bdesc + 2 * kk, idesc, (ks | kk) ? 1u : 0u);
-                        umma_commit(bar_aempty + 8 * as);
-                        if (++as == na) { as = 0; aph ^= 1; }
-                    }
-                    umma_commit(bar_xempty + 8 * xs);
+                    uint32_t xdesc = xdesc0 + xs * ((uint32_t)p.x_stage >> 4);
+                    const uint32_t xdone = bar_xempty + 8 * xs;
                     if (++xs == p.nx) { xs = 0; xph ^= 1; }
+                    for (int ks = ks0; ks < ks1; ks++, xdesc += kunits) {
+                        if (!(ok = mbar_wait_hint(a_hint, bar_aready + 8 * as, aph, abort_flag))) break;
+                        const uint32_t ta = tmem_a + as * 32, done = bar_aempty + 8 * as;
+                        if (++as == na) { as = 0; aph ^= 1; }
+                        a_hint = mbar_test(bar_aready + 8 * as, aph);
+                        if (ks + 1 == ks1) x_hint = mbar_test(bar_xfull + 8 * xs, xph);
+                        tc_fence_after();
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, (ks | kk) ? 1u : 0u);
+                        umma_commit(done);
+                    }
+                    umma_commit(xdone);
                 }
                 if (ok) umma_commit(bar_tfull + 8 * acc);
                 acc ^= 1;
@@ -442,6 +435,8 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
                         const int j = j0 + kTaGroups * i;
                         const int ks = ch * KPS + j;
                         if (ks >= ksteps) break;
+                        const uint32_t it = it0 + ks, as = it & (na - 1), aph = (it >> nash) & 1;
+                        const uint32_t a_hint = mbar_test(bar_aempty + 8 * as, aph ^ 1);
                         uint32_t sc, bi = 0;
                         if (FMT == kFmtAffine4G32) {
                             sc = lds32(scales + 4 * j);
@@ -450,13 +445,20 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
                             sc = lds_u16(scales + 2 * (FMT == kFmtTernary ? j >> 1 : j));
                             if (F::BIAS) bi = lds_u16(scales + 128 * SPB + 2 * j);
                         }
-                        uint32_t o[32];
-                        ta_dequant64<FMT>(codes, (uint32_t)(j * (F::BPS / 16)), sw, sc, bi, o);
-                        const uint32_t it = it0 + ks, as = it & (na - 1), aph = (it >> nash) & 1;
-                        ok = __all_sync(0xffffffffu, mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
+                        ok = __all_sync(0xffffffffu, a_hint || mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
                         if (!ok) break;
                         tc_fence_after();
-                        tmem_st32(my_a + as * 32, o);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            uint32_t o[16];
+                            // groups of 32 (g32: 16 bits each; mxfp4: 8 bits each) have a scale per half
+                            const uint32_t sch = FMT == kFmtAffine4G32 ? sc & 0xFFFFu : (FMT == kFmtMxfp4 ? sc & 0xFFu : sc);
+                            ta_dequant32<FMT>(codes, (uint32_t)(j * (F::BPS / 16) + (FMT == kFmtTernary ? 0 : h * (F::BPS / 32))), h, sw, sch,
+                                              FMT == kFmtAffine4G32 ? bi & 0xFFFFu : bi, o);
+                            tmem_st16(my_a + as * 32 + h * 16, o);
+                            if (FMT == kFmtAffine4G32) { sc >>= 16; bi >>= 16; }
+                            if (FMT == kFmtMxfp4) sc >>= 8;
+                        }
                         tmem_st_wait();
                         tc_fence_before();
                         __syncwarp();
