@@ -19,7 +19,7 @@ import torch
 import torch.distributed as dist
 
 from . import capi
-from .linear import DenseQ, VQMV, _dtype_id, _stream_ptr
+from .linear import DenseQ, VQMV, _DT, _dtype_id, _stream_ptr
 from .moe import MoELayer
 
 
@@ -258,9 +258,8 @@ class DeviceExchange:
 def rmsnorm(x: torch.Tensor, out: torch.Tensor, rows: int, eps: float = 1e-6, stream=None):
     """out = x / sqrt(mean(x²) + eps), fp32 in, bf16/fp16/fp32 out (unit weight)."""
     ctx = capi.context(x.device.index or 0)
-    dt = {torch.float32: capi.IQ_F32, torch.float16: capi.IQ_F16, torch.bfloat16: capi.IQ_BF16}[out.dtype]
-    ctx.check(capi.lib().iq_rmsnorm(ctx.handle, _stream_ptr(stream), x.data_ptr(), x.stride(0), out.data_ptr(), dt,
-                                    out.stride(0), rows, x.shape[1], eps))
+    ctx.check(capi.call().rmsnorm(ctx.address, _stream_ptr(stream), x.data_ptr(), x.stride(0), out.data_ptr(), _DT[out.dtype],
+                                  out.stride(0), rows, x.shape[1], eps))
 
 
 class MoEStack:

@@ -25,13 +25,18 @@ def _dtype_id(t: torch.Tensor) -> int:
 
 
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> int:
-    return (stream or torch.cuda.current_stream()).cuda_stream
+    # the current stream of the current device, without building a Stream object around it
+    return stream.cuda_stream if stream is not None else torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _no_cpu():
+    raise ValueError("tensors must live on a CUDA device: the operators have no CPU path")
 
 
 def _need_cuda(*ts: torch.Tensor):
     for t in ts:
         if t is not None and not t.is_cuda:
-            raise ValueError("tensors must live on a CUDA device: the operators have no CPU path")
+            _no_cpu()
 
 
 class DenseQ:
@@ -82,6 +87,29 @@ class DenseQ:
         self.w, self.s, self.b = w.contiguous(), scales.contiguous(), None if biases is None else biases.contiguous()
         self.N, self.K, self.bits, self.gs, self.mode, self.experts = N, K, bits, gs, mode, experts
 
+    # what the C description of the matrix is made of: assigning one of these drops the cached description
+    _DESCRIBED = frozenset(("w", "s", "b", "N", "K", "bits", "gs", "mode", "experts"))
+    _ql, _ql_address, _ctx = None, 0, None
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name in self._DESCRIBED and self._ql is not None:
+            object.__setattr__(self, "_ql", None)
+
+    def _described(self) -> int:
+        """Address of the matrix's C description, built once (a decode step passes the same matrices over and over)."""
+        q = self._ql
+        if q is None or q.w != self.w.data_ptr():  # (the storage may have been exchanged under the tensor)
+            q = self._ql = self.qlinear()
+            self._ql_address = C.addressof(q)
+        return self._ql_address
+
+    def _context(self) -> capi.Context:
+        ctx = self._ctx
+        if ctx is None or ctx.address == 0:
+            ctx = self._ctx = capi.context(self.device_index)
+        return ctx
+
     def qlinear(self) -> capi.QLinear:
         return capi.QLinear(self.w.data_ptr(), 0 if self.s is None else self.s.data_ptr(),
                             0 if self.b is None else self.b.data_ptr(), self.N,
@@ -109,9 +137,9 @@ class DenseQ:
         """x[rows, K] rotated into a float16 scratch (grown on demand, like the reference's rotation buffer)."""
         if self._rot is None or self._rot.shape[0] < rows:
             self._rot = torch.empty(max(rows, 16), self.K, dtype=torch.float16, device=self.w.device)
-        ctx = capi.context(self.device_index)
-        ctx.check(capi.lib().iq_had_rows(ctx.handle, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
-                                         self.had.data_ptr(), self._rot.data_ptr(), self.K, rows, self.K))
+        ctx = self._context()
+        ctx.check(capi.call().had_rows(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
+                                       self.had.data_ptr(), self._rot.data_ptr(), self.K, rows, self.K))
         return self._rot
 
     # ---- embedding (Linear.swift:65-93) -------------------------------------------------------------------------
@@ -129,18 +157,18 @@ class DenseQ:
         if out_f is not None and out_h is not None and out_f.stride(0) != out_h.stride(0):
             raise ValueError("out_f and out_h share one row stride")
         o = out_f if out_f is not None else out_h
-        ctx = capi.context(self.device_index)
-        q = self.qlinear()
+        ctx = self._context()
         if self.bits == 2:  # ternary table: dequantise, then the inverse rotation (embed_rows_t, xc_tern.metal:44-65)
             if self.had is None:
                 raise ValueError("a ternary table needs the rotation's signs (set_hadamard)")
+            q = self.qlinear()
             ctx.check(capi.lib().iq_embed_rows_ternary(ctx.handle, _stream_ptr(stream), C.byref(q), self.had.data_ptr(),
                                                        tok.data_ptr(), rows, 0 if out_f is None else out_f.data_ptr(),
                                                        0 if out_h is None else out_h.data_ptr(), o.stride(0)))
             return
-        ctx.check(capi.lib().iq_embed_rows(ctx.handle, _stream_ptr(stream), C.byref(q), tok.data_ptr(), rows,
-                                           0 if out_f is None else out_f.data_ptr(),
-                                           0 if out_h is None else out_h.data_ptr(), o.stride(0)))
+        ctx.check(capi.call().embed_rows(ctx.address, _stream_ptr(stream), self._described(), tok.data_ptr(), rows,
+                                         0 if out_f is None else out_f.data_ptr(),
+                                         0 if out_h is None else out_h.data_ptr(), o.stride(0)))
 
     # ---- prefill GEMM (Linear.swift:688-713) --------------------------------------------------------------------
     def qmm_workspace_bytes(self, rows: int, x_dtype: torch.dtype) -> int:
@@ -154,15 +182,16 @@ class DenseQ:
                        workspace: Optional[torch.Tensor] = None, stream: Optional[torch.cuda.Stream] = None):
         """Y[rows, N] (+)= X[rows, K] · Wᵀ on the tensor cores. y may be float32 (the reference's default), float16
         (`halfOut`) or bfloat16. rows must be a multiple of 64 (Linear.swift:695)."""
-        _need_cuda(x, y)
-        ctx = capi.context(self.device_index)
-        ql = self.qlinear()
+        if not (x.is_cuda and y.is_cuda):
+            _no_cpu()
+        ctx = self._context()
         if self.had is not None:  # rotated basis: the rotation runs first, as in the reference's launcher
             x = self.encode_rotate(x, rows, stream)
         ws_ptr, ws_bytes = (0, 0) if workspace is None else (workspace.data_ptr(), workspace.numel() * workspace.element_size())
-        ctx.check(capi.lib().iq_qmm(ctx.handle, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), C.byref(ql),
-                                    y.data_ptr(), _dtype_id(y), y.stride(0), rows,
-                                    capi.IQ_FLAG_ACCUMULATE if accumulate else 0, ws_ptr, ws_bytes))
+        st = capi.call().qmm(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), self._described(), y.data_ptr(),
+                             _dtype_id(y), y.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, ws_ptr, ws_bytes)
+        if st:
+            ctx.check(st)
 
     def encode_qmm_i8(self, x: torch.Tensor, y: torch.Tensor, rows: int, accumulate: bool = False,
                       scratch: Optional[torch.Tensor] = None, stream: Optional[torch.cuda.Stream] = None):
@@ -215,16 +244,22 @@ class VQMV:
                stream: Optional[torch.cuda.Stream] = None):
         """Y[rows, N] (+)= X[rows, K] · Wᵀ, rows ≤ 16. `ldx`/`ldy` are row strides in elements (default: the tensors'),
         `n_prefix` computes only the first rows of W (Linear.swift:350-366)."""
-        _need_cuda(x, y)
-        ctx = capi.context(m.device_index)
-        ql = m.qlinear()
+        if not (x.is_cuda and y.is_cuda):
+            _no_cpu()
+        ctx = m._ctx
+        if ctx is None or ctx.address == 0:
+            ctx = m._context()
         if m.had is not None:  # Linear.swift:292-297: the input rotation first, then the kernel on the rotated rows
             x, ldx = m.encode_rotate(x, rows, stream), m.K
-        ctx.check(capi.lib().iq_qmv(ctx.handle, _stream_ptr(stream), x.data_ptr(), _dtype_id(x),
-                                    ldx if ldx is not None else (x.stride(0) if x.dim() > 1 else m.K), C.byref(ql),
-                                    y.data_ptr(), _dtype_id(y),
-                                    ldy if ldy is not None else (y.stride(0) if y.dim() > 1 else m.N), rows,
-                                    capi.IQ_FLAG_ACCUMULATE if accumulate else 0, n_prefix or 0))
+        if ldx is None:
+            ldx = x.stride(0) if x.dim() > 1 else m.K
+        if ldy is None:
+            ldy = y.stride(0) if y.dim() > 1 else m.N
+        st = capi.call().qmv(ctx.address, _stream_ptr(stream), x.data_ptr(), _DT.get(x.dtype, -1), ldx, m._described(), y.data_ptr(),
+                             _DT.get(y.dtype, -1), ldy, rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, n_prefix or 0)
+        if st:
+            _dtype_id(x), _dtype_id(y)  # a type the library does not know is a TypeError
+            ctx.check(st)
 
 
 class DenseMLP:
@@ -237,26 +272,30 @@ class DenseMLP:
         self.act = {"silu": capi.IQ_ACT_SILU, "gelu": capi.IQ_ACT_GELU, "swiglu_oai": capi.IQ_ACT_SWIGLU_OAI,
                     "relu2": capi.IQ_ACT_RELU2}[act]
         self.limit = limit
-        self._ws = None
+        self._ws, self._sized = None, None  # scratch, and the (rows, dtype, matrices) it was last checked for
 
     def _workspace(self, rows: int, x_dtype: torch.dtype) -> torch.Tensor:
+        key = (rows, x_dtype, self.gate_up, self.down)
+        if self._sized == key:
+            return self._ws
         ctx = capi.context(self.gate_up.device_index)
         n = C.c_size_t()
         a, b = self.gate_up.qlinear(), self.down.qlinear()
         ctx.check(capi.lib().iq_dense_ffn_workspace_bytes(ctx.handle, C.byref(a), C.byref(b), rows, _DT[x_dtype], C.byref(n)))
         if self._ws is None or self._ws.numel() < n.value:
             self._ws = torch.empty(max(n.value, 256), dtype=torch.uint8, device=self.gate_up.w.device)
+        self._sized = key
         return self._ws
 
     def encode(self, x: torch.Tensor, out: torch.Tensor, rows: int, accumulate: bool = False,
                stream: Optional[torch.cuda.Stream] = None):
         """out[rows, D] (+)= down(act(gate x)·up x) (Dense.swift:56-96). rows ≤ 16 runs the GEMV kernels, larger
         multiples of 64 the GEMM kernels. Scratch is sized on first use and reused."""
-        _need_cuda(x, out)
-        ctx = capi.context(self.gate_up.device_index)
+        if not (x.is_cuda and out.is_cuda):
+            _no_cpu()
+        ctx = self.gate_up._context()
         ws = self._workspace(rows, x.dtype)
-        a, b = self.gate_up.qlinear(), self.down.qlinear()
-        ctx.check(capi.lib().iq_dense_ffn(ctx.handle, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
-                                          C.byref(a), C.byref(b), self.act, self.limit, out.data_ptr(), _dtype_id(out),
-                                          out.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0,
-                                          ws.data_ptr(), ws.numel()))
+        ctx.check(capi.call().dense_ffn(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
+                                        self.gate_up._described(), self.down._described(), self.act, self.limit, out.data_ptr(),
+                                        _dtype_id(out), out.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0,
+                                        ws.data_ptr(), ws.numel()))

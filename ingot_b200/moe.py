@@ -13,7 +13,7 @@ from typing import Iterable, Optional
 import torch
 
 from . import capi
-from .linear import DenseQ, _dtype_id, _need_cuda, _stream_ptr
+from .linear import DenseQ, _dtype_id, _need_cuda, _no_cpu, _stream_ptr
 
 PIECES = {
     "router": capi.IQ_PIECE_ROUTER, "route": capi.IQ_PIECE_ROUTE, "group": capi.IQ_PIECE_GROUP,
@@ -111,7 +111,8 @@ class MoELayer:
                only: Optional[Iterable[str]] = None, stream: Optional[torch.cuda.Stream] = None):
         """out[rows, D] (+)= MoE(x[rows, D]) (MoELayer.encode MoE.swift:346-428; PrefillMoE.encodeAll
         MoEPrefill.swift:274). `only`: piece names to run, in the reference's vocabulary."""
-        _need_cuda(x, out)
+        if not (x.is_cuda and out.is_cuda):
+            _no_cpu()
         if rows > self.max_tokens:
             raise ValueError(f"rows = {rows} exceeds the scratch reserved at construction ({self.max_tokens})")
         mask = capi.IQ_PIECE_ALL
@@ -119,8 +120,8 @@ class MoELayer:
             mask = 0
             for p in ([only] if isinstance(only, str) else only):
                 mask |= PIECES[p]
-        self.ctx.check(capi.lib().iq_moe_forward(
-            self._h, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), out.data_ptr(), _dtype_id(out),
+        self.ctx.check(capi.call().moe_forward(
+            self._h.value, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), out.data_ptr(), _dtype_id(out),
             out.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, mask, self.workspace.data_ptr(),
             self.workspace.numel()))
 

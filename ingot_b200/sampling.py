@@ -8,20 +8,21 @@ from typing import Optional, Sequence
 import torch
 
 from . import capi
-from .linear import _need_cuda, _stream_ptr
+from .linear import _no_cpu, _stream_ptr
 
 CANDIDATES = 64
 
 
 def argmax_rows(x: torch.Tensor, rows: int, stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
     """Index of the largest logit of each of the first `rows` rows of x (fp32 [*, n]); ties go to the lower index."""
-    _need_cuda(x)
+    if not x.is_cuda:
+        _no_cpu()
     if x.dtype != torch.float32:
         raise TypeError("logits are float32")
     ctx = capi.context(x.device.index or 0)
     out = torch.empty(rows, dtype=torch.int32, device=x.device)
-    ctx.check(capi.lib().iq_argmax_rows(ctx.handle, _stream_ptr(stream), x.data_ptr(), x.stride(0), rows, x.shape[1],
-                                        out.data_ptr()))
+    ctx.check(capi.call().argmax_rows(ctx.address, _stream_ptr(stream), x.data_ptr(), x.stride(0), rows, x.shape[1],
+                                      out.data_ptr()))
     return out
 
 
@@ -38,14 +39,15 @@ class TopK64:
 
     def encode(self, x: torch.Tensor, rows: int, temperatures: Sequence[float], stream: Optional[torch.cuda.Stream] = None):
         """Returns (idx int32 [rows, 64], val float32 [rows, 64], z float32 [rows, 2] = (max, sum exp((x - max) / T)))."""
-        _need_cuda(x)
+        if not x.is_cuda:
+            _no_cpu()
         if x.dtype != torch.float32 or rows > self.max_rows or x.shape[1] != self.vocab:
             raise ValueError("TopK64: float32 logits [rows <= max_rows, vocab]")
         idx = torch.empty(rows, CANDIDATES, dtype=torch.int32, device=x.device)
         val = torch.empty(rows, CANDIDATES, dtype=torch.float32, device=x.device)
         z = torch.empty(rows, 2, dtype=torch.float32, device=x.device)
         t = (C.c_float * len(temperatures))(*temperatures)
-        self.ctx.check(capi.lib().iq_topk64(self.ctx.handle, _stream_ptr(stream), x.data_ptr(), x.stride(0), rows, self.vocab, t,
-                                            len(temperatures), idx.data_ptr(), val.data_ptr(), z.data_ptr(),
-                                            self.scratch.data_ptr(), self.scratch.numel()))
+        self.ctx.check(capi.call().topk64(self.ctx.address, _stream_ptr(stream), x.data_ptr(), x.stride(0), rows, self.vocab,
+                                          C.addressof(t), len(temperatures), idx.data_ptr(), val.data_ptr(), z.data_ptr(),
+                                          self.scratch.data_ptr(), self.scratch.numel()))
         return idx, val, z
