@@ -124,19 +124,16 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// (volatile: without it the compiler may move the load above the condition that guards its address)
 __device__ __forceinline__ uint4 ldg_nc_u4(const void* p) {
     uint4 r;
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                  : "l"(p));
     return r;
 }
 
-__device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) {
-    unsigned short r;
-    asm("ld.global.nc.u16 %0, [%1];" : "=h"(r) : "l"(p));
-    return r;
-}
+__device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) { return __ldg(static_cast<const unsigned short*>(p)); }
 
 // Prefetching variants: volatile, so the compiler keeps them where they are written (ahead of a barrier wait) instead
 // of sinking them to the first use.
@@ -151,10 +148,6 @@ __device__ __forceinline__ uint32_t ldg_nc_u8_early(const void* p) {
     return r;
 }
 
-__device__ __forceinline__ uint32_t ldg_nc_u8(const void* p) {
-    uint32_t r;
-    asm("ld.global.nc.u8 %0, [%1];" : "=r"(r) : "l"(p));
-    return r;
-}
+__device__ __forceinline__ uint32_t ldg_nc_u8(const void* p) { return __ldg(static_cast<const unsigned char*>(p)); }
 
 }  // namespace iq

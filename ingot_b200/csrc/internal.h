@@ -57,6 +57,23 @@ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 inline size_t round_up_sz(size_t v, size_t m) { return (v + m - 1) / m * m; }
 inline int dtype_size(int32_t dt) { return dt == kF32 ? 4 : 2; }
 
+// A launch that may start before its predecessor in the stream has ended; the kernel calls pdl_wait() before it touches
+// anything the predecessor may still write or read.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // format id from (bits, group, mode) or -1
 int32_t format_of(const iq_qlinear* m);
 
@@ -130,7 +147,6 @@ struct QmmCall {
 int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c);
 int32_t launch_tern_qmv(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
                         int32_t y_dtype, int64_t ldy, int32_t rows, int32_t n, int32_t accumulate);
-int32_t tern_init(iq_ctx* ctx);
 int32_t w8a8_init(iq_ctx* ctx);
 int32_t gqmv_init(iq_ctx* ctx);
 int32_t qmm_init(iq_ctx* ctx);

@@ -213,4 +213,11 @@ __device__ __forceinline__ double ld_dsmem_f64(const double* p, uint32_t cta) {
     return v;
 }
 
+// a word stored at the same shared-memory offset as `p` in the block with rank `cta` of this cluster
+__device__ __forceinline__ void st_dsmem_u32(uint32_t* p, uint32_t cta, uint32_t v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(cta));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(v) : "memory");
+}
+
 }  // namespace iq

@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
         // ================= producer of the scales and biases =================
         // Per stage of codes the SPB scale bytes of each of the 128 rows: lane l takes rows l, l + 32, ... Row pitches that
         // allow it go by asynchronous copies, others (an odd number of groups) by two-byte loads. Rows beyond the matrix
-        // are left out: their weights only feed rows of D that are not stored.
+        // take the last row's: their weights only feed rows of D that are not stored.
         constexpr int SPB = F::SPB, NT = F::BIAS ? 2 : 1;
         const size_t pitch = (size_t)p.K / F::GROUP * F::ES;
         int s = 0;
@@ -326,10 +326,10 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
             const char* src[4][NT];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int row = lane + 32 * i, mi = EPI ? i >> 1 : 0, n = n0 + (EPI ? row & 63 : row);
+                const int row = lane + 32 * i, mi = EPI ? i >> 1 : 0, n = min(n0 + (EPI ? row & 63 : row), p.N - 1);
                 const size_t o = ((size_t)expert * p.N + n) * pitch;
-                src[i][0] = n < p.N ? static_cast<const char*>(p.s[mi]) + o : nullptr;
-                if (NT == 2) src[i][NT - 1] = n < p.N ? static_cast<const char*>(p.b[mi]) + o : nullptr;
+                src[i][0] = static_cast<const char*>(p.s[mi]) + o;
+                if (NT == 2) src[i][NT - 1] = static_cast<const char*>(p.b[mi]) + o;
             }
             for (int ch = 0; ch < chunks; ch++) {
                 ok = mbar_wait(bar_cempty + 8 * s, ph ^ 1, abort_flag);
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
                     for (int i = 0; i < 4; i++)
 #pragma unroll
                         for (int t = 0; t < NT; t++)
-                            if (src[i][t] != nullptr) cp_async_ca<SPB>(dst + t * 128 * SPB + (lane + 32 * i) * SPB, src[i][t] + ch * SPB);
+                            cp_async_ca<SPB>(dst + t * 128 * SPB + (lane + 32 * i) * SPB, src[i][t] + ch * SPB);
                 } else {
                     uint32_t v[4][NT][SPB / 2];
 #pragma unroll
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
                         for (int t = 0; t < NT; t++)
 #pragma unroll
                             for (int e = 0; e < SPB / 2; e++)
-                                v[i][t][e] = src[i][t] != nullptr && 2 * e < left ? ldg_nc_u16(src[i][t] + ch * SPB + 2 * e) : 0u;
+                                v[i][t][e] = ldg_nc_u16(src[i][t] + ch * SPB + min(2 * e, left - 2));
 #pragma unroll
                     for (int i = 0; i < 4; i++)
 #pragma unroll

@@ -7,6 +7,7 @@
 
 #include "gqmv.cuh"
 #include "internal.h"
+#include "qmv_direct.cuh"
 #include "qmv_imma.cuh"
 #include "qmv_imma_grouped.cuh"
 #include "qmv_stream.cuh"
@@ -288,6 +289,63 @@ int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     return kOk;
 }
 
+// ---- int8 tensor-core path with the weights loaded straight into registers: the plain GEMVs the staged kernel refuses, and the
+// dense FFN's gate + up ---------------------------------------------------------------------------------------------
+typedef void (*QdKernel)(const QdParams);
+template <int FMT, int NW>
+QdKernel qd_pick_mv(int ms, bool vec) {
+    if (ms == 2) return vec ? qmv_direct_kernel<FMT, 2, NW, true> : qmv_direct_kernel<FMT, 2, NW, false>;
+    return vec ? qmv_direct_kernel<FMT, 1, NW, true> : qmv_direct_kernel<FMT, 1, NW, false>;
+}
+QdKernel qd_pick(int32_t fmt, int nw, int ms, bool vec) {
+    switch (fmt) {
+        case kFmtAffine4: return nw == 2 ? qd_pick_mv<kFmtAffine4, 2>(ms, vec) : qd_pick_mv<kFmtAffine4, 1>(ms, vec);
+        case kFmtAffine4G32: return nw == 2 ? qd_pick_mv<kFmtAffine4G32, 2>(ms, vec) : qd_pick_mv<kFmtAffine4G32, 1>(ms, vec);
+        case kFmtAffine8:
+            if (nw == 2) return ms == 2 ? qmv_direct_kernel<kFmtAffine8, 2, 2, false> : qmv_direct_kernel<kFmtAffine8, 1, 2, false>;
+            return qd_pick_mv<kFmtAffine8, 1>(ms, vec);
+        default: return nullptr;
+    }
+}
+// Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error. The choice looks
+// at the matrix alone, not at the row count.
+int32_t launch_qmv_direct(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
+    if (c.tiles != nullptr || c.mode == kModeDown || c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0) return 1;
+    if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;
+    const int nw = c.mode == kModeGateUp ? 2 : 1, gs = c.fmt == kFmtAffine4G32 ? 32 : 64, G = c.K / gs;
+    const int per = qd_batch(c.fmt == kFmtAffine8, nw);  // groups per batch
+    bool vec = per > 1 && G % per == 0;
+    QdParams p;
+    memset(&p, 0, sizeof(p));
+    for (int i = 0; i < 2; i++) {
+        p.w[i] = reinterpret_cast<const unsigned char*>(c.w[i] ? c.w[i] : c.w[0]);
+        p.s[i] = reinterpret_cast<const unsigned char*>(c.s[i] ? c.s[i] : c.s[0]);
+        p.b[i] = reinterpret_cast<const unsigned char*>(c.b[i] ? c.b[i] : c.b[0]);
+        if (reinterpret_cast<uintptr_t>(p.w[i]) & 15) return 1;
+        if ((reinterpret_cast<uintptr_t>(p.s[i]) | reinterpret_cast<uintptr_t>(p.b[i])) & (uintptr_t)(2 * per - 1)) vec = false;
+    }
+    auto smem_for = [&](int ms) { return G * ms * 32 * (gs / 4) + G * ms * 32 + 2 * kQdWarps * nw * ms * 256; };
+    if (smem_for(1) > kQsSmemMax) return 1;
+    const bool wide = smem_for(2) <= kQsSmemMax;  // eight rows per launch; else four
+    p.N = c.N; p.K = c.K;
+    p.x_dtype = c.x_dtype; p.ldx = c.ldx;
+    p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
+    p.act = c.act; p.limit = c.limit;
+    const size_t xes = c.x_dtype == kF32 ? 4 : 2, yes = c.y_dtype == kF32 ? 4 : 2;
+    for (int m0 = 0; m0 < c.rows;) {
+        const int left = c.rows - m0, ms = left > 4 && wide ? 2 : 1, m = left < 4 * ms ? left : 4 * ms;
+        p.M = m;
+        p.x = static_cast<const char*>(c.x) + (size_t)m0 * c.ldx * xes;
+        p.y = static_cast<char*>(c.y) + (size_t)m0 * c.ldy * yes;
+        const int smem = smem_for(ms), slots = ctx->sms * (ms == 1 && smem <= kQsSmemMax / 2 - 1024 ? 2 : 1);
+        const int32_t r = check_cuda(ctx, launch_dependent(qd_pick(c.fmt, nw, ms, vec), dim3(c.N / 16 < slots ? c.N / 16 : slots), kQdThreads,
+                                                           smem, st, p), "qmv_direct launch");
+        if (r != kOk) return r;
+        m0 += m;
+    }
+    return kOk;
+}
+
 // ---- int8 tensor-core path for the MoE decode tiles (gate/up + activation, down; affine 4-bit experts) ---------------
 typedef void (*QgKernel)(const CUtensorMap, const CUtensorMap, const QgParams);
 // gw4: each consumer warp's K slice is four groups, its activation fragments stay in registers (8-row tiles only)
@@ -410,6 +468,12 @@ int32_t gqmv_init(iq_ctx* ctx) {
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
         }
+    const int32_t qd_fmts[3] = {kFmtAffine4, kFmtAffine4G32, kFmtAffine8};
+    for (int v = 0; v < 24; v++) {
+        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qd_pick(qd_fmts[v % 3], 1 + v / 3 % 2, 1 + v / 6 % 2, v >= 12)),
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
+        if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_direct)");
+    }
     for (int fmt = 0; fmt < 4; fmt++)
         for (int mh = 1; mh <= 2; mh++)
             for (int mode = 0; mode < 3; mode++)
@@ -430,10 +494,12 @@ int32_t gqmv_init(iq_ctx* ctx) {
 }
 
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
-    // One kernel per (format, shape), chosen from the matrix alone: the int8 tensor-core kernels for affine codes whose
-    // K fits their staging, the streaming fp16 kernel for MXFP4 and the remaining affine shapes, the register-staged
-    // fp16 kernel where a 16-row block over the whole K does not fit a stage.
+    // One kernel per (format, shape), chosen from the matrix alone: for affine codes the int8 tensor-core kernels (staged
+    // where K fits the staging, else with the weights in registers), the streaming fp16 kernel for MXFP4 and the remaining
+    // expert tiles, the register-staged fp16 kernel where a 16-row block over the whole K does not fit a stage.
     int32_t r = launch_qmv_imma(ctx, st, c);
+    if (r != 1) return r;
+    r = launch_qmv_direct(ctx, st, c);
     if (r != 1) return r;
     r = launch_qmv_imma_grouped(ctx, st, c);
     if (r != 1) return r;

@@ -8,6 +8,7 @@
 // dequantiser (csrc/qmm_tc.cuh). The kernels here are small: a 4096 x 4096 ternary matrix is 4 MB.
 #include "common.cuh"
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace iq {
 namespace {
@@ -34,6 +35,7 @@ __device__ __forceinline__ void fwht1024(float* sh, int tid) {
 __global__ void __launch_bounds__(256) had_rows_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx,
                                                       const float* __restrict__ signs, __half* __restrict__ y, int64_t ldy) {
     __shared__ float sh[1024];
+    pdl_launch_dependents();
     const int tid = threadIdx.x, k0 = blockIdx.x * 1024;
     if (tid < 128) {
         float v[8];
@@ -74,11 +76,17 @@ __global__ void __launch_bounds__(256) embed_rows_tern_kernel(const uint32_t* __
 }
 
 // Decode GEMV: Y[m, n] (+)= sum_k x[m, k] * (q[n, k] - 1) * s[n, k / 128] for up to 16 rows of (already rotated) fp16
-// activations. One warp per output feature; a lane takes 16-byte pieces of the row (64 codes, half a scale group): the
-// weights are -s, 0, +s, so a piece contributes s * sum_k (q_k - 1) x_k, the inner sum with exact products. The
-// activations sit in shared memory as floats, the rows of one input side by side and four floats of padding after every
-// 64 inputs, so that the 32 lanes' 16-byte loads (64 inputs apart) fall into different banks. A row's bits do not
-// depend on the other rows.
+// activations, on m16n8k16 fp16 tensor-core MMAs: the weights -1, 0, +1 are exact in fp16, so every product is exact, and
+// the scale multiplies the fp32 sum of a group of 128.
+//
+// A block is 16 output features, its eight warps take the groups of 128 inputs round robin, and their sums meet in shared
+// memory in warp order. Lane (g, t) of a warp holds rows g and g + 8 and inputs 32 t .. 32 t + 31 of the group: eight
+// bytes of codes per row, 64 bytes of each activation row. The order of the inputs inside an MMA is free as long as both
+// operands agree: inputs k and k + 4 make a pair, because their codes are one byte apart, so that one shift and one mask
+// turn them into the selector of the byte permutation that looks both weights up.
+//
+// Bound: HBM (12 MB for 9216 x 5120: 2 us); the kernel before expanded codes to floats one by one against activations in
+// shared memory and took 127 us there.
 constexpr int kTernWarps = 8;
 struct TernParams {
     const __half* x;
@@ -89,77 +97,115 @@ struct TernParams {
     int32_t y_dtype;
     int64_t ldy;
     int32_t M, N, K, accumulate;
-    int32_t kt;  // inputs staged at a time (a multiple of 64)
 };
 
-template <int MH>  // activation rows handled per pass: 8 * MH >= M
+template <int MH>  // sets of eight activation rows
 __global__ void __launch_bounds__(kTernWarps * 32) tern_qmv_kernel(const TernParams p) {
-    extern __shared__ __align__(16) float xs[];  // input k, row m at k * MR + (k / 64) * 4 + m
-    constexpr int MR = 8 * MH;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = blockIdx.x * kTernWarps + warp;
-    const bool n_ok = n < p.N;
-    const uint4* wr = reinterpret_cast<const uint4*>(p.w + (size_t)(n_ok ? n : 0) * (p.K / 16));
-    const __half* sr = p.s + (size_t)(n_ok ? n : 0) * (p.K / 128);
-    float acc[MR];
+    __shared__ float red[kTernWarps][MH][16][8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    pdl_launch_dependents();
+    const int G = p.K / 128;
+    const unsigned char* w0 = reinterpret_cast<const unsigned char*>(p.w) + (size_t)(blockIdx.x * 16 + g) * (p.K / 4) + t * 8;
+    const unsigned char* w1 = w0 + (size_t)8 * (p.K / 4);
+    const uint16_t* s0 = reinterpret_cast<const uint16_t*>(p.s) + (size_t)(blockIdx.x * 16 + g) * G;
+    const uint16_t* s1 = s0 + (size_t)8 * G;
+    constexpr int PF = 4;  // groups of codes and scales on their way ahead of the one being used
+    uint2 q[PF][2];
+    uint32_t sc[PF][2];
+    auto fetch = [&](int i, int grp) {  // (no condition around the loads: groups past the end read the last one again)
+        grp = min(grp, G - 1);
+        q[i][0] = *reinterpret_cast<const uint2*>(w0 + grp * 32);
+        q[i][1] = *reinterpret_cast<const uint2*>(w1 + grp * 32);
+        sc[i][0] = ldg_nc_u16(s0 + grp);
+        sc[i][1] = ldg_nc_u16(s1 + grp);
+    };
 #pragma unroll
-    for (int m = 0; m < MR; m++) acc[m] = 0.f;
-    for (int k0 = 0; k0 < p.K; k0 += p.kt) {  // K in tiles that fit shared memory
-    const int klen = min(p.kt, p.K - k0);
-    __syncthreads();
-    for (int i = tid; i < klen * MR; i += kTernWarps * 32) {
-        const int k = i / MR, m = i % MR;
-        xs[k * MR + (k >> 6) * 4 + m] = m < p.M ? __half2float(p.x[(size_t)m * p.ldx + k0 + k]) : 0.f;
-    }
-    __syncthreads();
-    if (!n_ok) continue;
-    for (int cl = lane; cl < klen / 64; cl += 32) {
-        const int c = k0 / 64 + cl;
-        const uint4 q4 = ldg_nc_u4(wr + c);
-        const float sc = __half2float(sr[c >> 1]);
-        const uint32_t words[4] = {q4.x, q4.y, q4.z, q4.w};
-        float part[MR];
+    for (int i = 0; i < PF; i++) fetch(i, warp + i * kTernWarps);
+    pdl_wait();  // the activations are the rotation's output
+    float acc[MH][4];
 #pragma unroll
-        for (int m = 0; m < MR; m++) part[m] = 0.f;
+    for (int h = 0; h < MH; h++)
 #pragma unroll
-        for (int wi = 0; wi < 4; wi++) {
+        for (int j = 0; j < 4; j++) acc[h][j] = 0.f;
+    for (int g0 = warp; g0 < G; g0 += PF * kTernWarps) {
 #pragma unroll
-            for (int e = 0; e < 16; e++) {
-                const float sgn = (float)((words[wi] >> (2 * e)) & 3u) - 1.0f;  // -1, 0, +1
-                const float* xk = xs + (size_t)(cl * 64 + wi * 16 + e) * MR + cl * 4;
+        for (int i = 0; i < PF; i++) {
+            const int grp = g0 + i * kTernWarps;
+            if (grp >= G) break;
+            uint4 xv[MH][4];  // inputs 8 j .. 8 j + 7 of the lane's 32
 #pragma unroll
-                for (int m = 0; m < MR; m += 4) {
-                    const float4 xv = *reinterpret_cast<const float4*>(xk + m);
-                    part[m] = fmaf(sgn, xv.x, part[m]);
-                    part[m + 1] = fmaf(sgn, xv.y, part[m + 1]);
-                    part[m + 2] = fmaf(sgn, xv.z, part[m + 2]);
-                    part[m + 3] = fmaf(sgn, xv.w, part[m + 3]);
+            for (int h = 0; h < MH; h++) {
+                const bool live = 8 * h + g < p.M;
+                const uint4* xp = reinterpret_cast<const uint4*>(p.x + (size_t)(live ? 8 * h + g : 0) * p.ldx + grp * 128 + t * 32);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    xv[h][j] = xp[j];
+                    if (!live) xv[h][j] = make_uint4(0, 0, 0, 0);
                 }
             }
-        }
+            float d[MH][4];
 #pragma unroll
-        for (int m = 0; m < MR; m++) acc[m] = fmaf(sc, part[m], acc[m]);
-    }
-    }
-    if (!n_ok) return;
+            for (int h = 0; h < MH; h++)
 #pragma unroll
-    for (int m = 0; m < MR; m++) {
-        float v = acc[m];
+                for (int j = 0; j < 4; j++) d[h][j] = 0.f;
+            const uint32_t words[2][2] = {{q[i][0].x, q[i][0].y}, {q[i][1].x, q[i][1].y}};
+            const float f0 = __half2float(__ushort_as_half((unsigned short)sc[i][0])), f1 = __half2float(__ushort_as_half((unsigned short)sc[i][1]));
+            fetch(i, grp + PF * kTernWarps);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && m < p.M) {
-            const size_t o = (size_t)m * p.ldy + n;
-            if (p.y_dtype == kF32) {
-                float* yp = reinterpret_cast<float*>(p.y) + o;
-                *yp = p.accumulate ? *yp + v : v;
-            } else if (p.y_dtype == kF16) {
-                __half* yp = reinterpret_cast<__half*>(p.y) + o;
-                *yp = __float2half_rn(p.accumulate ? __half2float(*yp) + v : v);
-            } else {
-                uint16_t* yp = reinterpret_cast<uint16_t*>(p.y) + o;
-                *yp = (uint16_t)f32_to_bf16_bits(p.accumulate ? bf16_bits_to_f32(*yp) + v : v);
+            for (int j = 0; j < 4; j++) {  // eight inputs: two MMAs
+                uint32_t a[2][4];
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const uint32_t c8 = j & 1 ? words[r][j >> 1] >> 16 : words[r][j >> 1];  // eight codes in the low 16 bits
+#pragma unroll
+                    for (int pr = 0; pr < 4; pr++) {
+                        // codes pr and pr + 4 to bits 4-5 and 12-13: selectors of the high bytes of -1, 0, 1, 2 as fp16
+                        const uint32_t sel = ((pr < 2 ? c8 << (4 - 2 * pr) : c8 >> (2 * pr - 4)) & 0x3030u) | 0x0404u;
+                        a[r][pr] = __byte_perm(0x403C00BCu, 0u, sel);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < MH; h++) {
+                    const uint4 v = xv[h][j];
+                    const uint32_t x04 = __byte_perm(v.x, v.z, 0x5410), x15 = __byte_perm(v.x, v.z, 0x7632);
+                    const uint32_t x26 = __byte_perm(v.y, v.w, 0x5410), x37 = __byte_perm(v.y, v.w, 0x7632);
+                    mma16816(d[h], a[0][0], a[1][0], a[0][1], a[1][1], x04, x15);
+                    mma16816(d[h], a[0][2], a[1][2], a[0][3], a[1][3], x26, x37);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < MH; h++) {
+                acc[h][0] = fmaf(f0, d[h][0], acc[h][0]);
+                acc[h][1] = fmaf(f0, d[h][1], acc[h][1]);
+                acc[h][2] = fmaf(f1, d[h][2], acc[h][2]);
+                acc[h][3] = fmaf(f1, d[h][3], acc[h][3]);
             }
         }
+    }
+#pragma unroll
+    for (int h = 0; h < MH; h++) {
+        red[warp][h][g][2 * t] = acc[h][0];
+        red[warp][h][g][2 * t + 1] = acc[h][1];
+        red[warp][h][g + 8][2 * t] = acc[h][2];
+        red[warp][h][g + 8][2 * t + 1] = acc[h][3];
+    }
+    __syncthreads();
+    if (tid >= 128 * MH) return;
+    const int n = tid & 15, m8 = (tid >> 4) & 7, h = tid >> 7, m = 8 * h + m8;
+    if (m >= p.M) return;
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < kTernWarps; k++) v += red[k][h][n][m8];
+    const size_t o = (size_t)m * p.ldy + blockIdx.x * 16 + n;
+    if (p.y_dtype == kF32) {
+        float* yp = reinterpret_cast<float*>(p.y) + o;
+        *yp = p.accumulate ? *yp + v : v;
+    } else if (p.y_dtype == kF16) {
+        __half* yp = reinterpret_cast<__half*>(p.y) + o;
+        *yp = __float2half_rn(p.accumulate ? __half2float(*yp) + v : v);
+    } else {
+        uint16_t* yp = reinterpret_cast<uint16_t*>(p.y) + o;
+        *yp = (uint16_t)f32_to_bf16_bits(p.accumulate ? bf16_bits_to_f32(*yp) + v : v);
     }
 }
 
@@ -177,22 +223,8 @@ int32_t launch_tern_qmv(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_d
     p.w = static_cast<const uint32_t*>(m->w); p.s = static_cast<const __half*>(m->scales);
     p.y = y; p.y_dtype = y_dtype; p.ldy = ldy;
     p.M = rows; p.N = n; p.K = m->k; p.accumulate = accumulate;
-    const int mh = rows > 8 ? 2 : 1;
-    p.kt = m->k < 4096 / mh ? m->k : 4096 / mh;  // 128 KB of staged activations at most (K is a multiple of 128)
-    const size_t smem = ((size_t)p.kt * 8 * mh + (size_t)p.kt / 64 * 4) * sizeof(float);
-    const unsigned grid = (unsigned)((n + kTernWarps - 1) / kTernWarps);
-    if (mh == 1) tern_qmv_kernel<1><<<grid, kTernWarps * 32, smem, st>>>(p);
-    else tern_qmv_kernel<2><<<grid, kTernWarps * 32, smem, st>>>(p);
-    return check_cuda(ctx, cudaGetLastError(), "tern_qmv launch");
-}
-
-int32_t tern_init(iq_ctx* ctx) {
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(tern_qmv_kernel<1>),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(tern_qmv_kernel<2>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 200 * 1024);
-    return check_cuda(ctx, e, "cudaFuncSetAttribute(tern_qmv)");
+    return check_cuda(ctx, launch_dependent(rows > 8 ? tern_qmv_kernel<2> : tern_qmv_kernel<1>, dim3((unsigned)(n / 16)), kTernWarps * 32, 0, st, p),
+                      "tern_qmv launch");
 }
 
 }  // namespace iq

@@ -194,3 +194,21 @@ def test_embed_rows_bf16_table(cuda_device):
     torch.cuda.synchronize()
     want = t[tok.long()].float()
     assert torch.equal(of, want) and torch.equal(oh, want.to(torch.float16))
+
+
+@pytest.mark.parametrize("bits,group", [(8, 64), (4, 32), (4, 64)])
+@pytest.mark.parametrize("rows,D,F", [(6, 832, 4800), (64, 192, 320), (576, 832, 448)])
+def test_dense_ffn_ragged(cuda_device, bits, group, rows, D, F):
+    """Widths that are no multiple of the tiles: 300 row blocks per matrix and an odd number of groups on the decode kernels,
+    half tiles of output features, odd numbers of K steps and several token tiles on the GEMM."""
+    rng = np.random.default_rng(60 + rows + D + F + bits + group)
+    gu, hgu = affine_case(rng, 2 * F, D, bits, cuda_device, group=group)
+    dn, hdn = affine_case(rng, D, F, bits, cuda_device, group=group)
+    xh = synth.activations_np(rng, rows, D)
+    wgu = deq(hgu, bits, group=group)
+    h = qref.round_f16(qref.silu_glu(qref.matmul_t(xh, wgu[:F]), qref.matmul_t(xh, wgu[F:])))
+    ref = qref.matmul_t(h, deq(hdn, bits, group=group))
+    out = torch.zeros(rows, D, dtype=torch.float32, device=cuda_device)
+    DenseMLP(gu, dn).encode(x_tensor(xh, cuda_device), out, rows)
+    assert capi.context(0).device_status() == 0
+    assert qref.max_rel(out.cpu().numpy(), ref) <= 2 * TOL  # h is rounded to fp16 on both sides, from sums in other orders

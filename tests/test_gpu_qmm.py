@@ -98,3 +98,19 @@ def test_qmm_rejects_what_the_reference_rejects(cuda_device):
     with pytest.raises(capi.IngotError) as e:
         m.encode_qmm_f32(xb, y, 64)  # bf16 activations need the conversion workspace
     assert e.value.status == -4
+
+
+@pytest.mark.parametrize("fmt", ["q4", "q8", "mxfp4"])
+@pytest.mark.parametrize("M,N,K", [(64, 64, 64), (192, 64, 192), (448, 192, 832), (1088, 2112, 320), (2048, 128, 1088)])
+def test_qmm_tile_edges(cuda_device, fmt, M, N, K):
+    """Odd numbers of K steps (1, 3, 5, 13, 17: stages of codes that end early, scales whose row pitch allows no vector copy),
+    half tiles of output features, token tiles of other heights; accumulation onto an existing result."""
+    rng = np.random.default_rng(M + N + K)
+    m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, int(fmt[1]), cuda_device)
+    x = synth.activations_np(rng, M, K)
+    ref = qref.matmul_t(x, deq(host, 4 if fmt == "mxfp4" else int(fmt[1])))
+    xt = x_tensor(x, cuda_device)
+    y = run_qmm(m, xt, M)
+    assert qref.max_rel(y.cpu().numpy(), ref) <= TOL
+    y2 = run_qmm(m, xt, M, accumulate=True, y=y.clone())
+    assert torch.equal(y2, 2 * y)

@@ -235,3 +235,17 @@ def test_qmv_non_finite_activations_propagate(cuda_device, bad, K):
     ref = qref.matmul_t(x[[0, 2]], deq(host, 4))
     assert not np.isfinite(y[1]).any()
     assert qref.max_rel(y[[0, 2]], ref) <= TOL
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("N,K,rows", [(16, 832, 4), (4784, 192, 5), (4752, 7680, 3), (32, 14336, 8), (9488, 1024, 1)])
+def test_qmv_weights_in_registers(cuda_device, bits, N, K, rows):
+    """Input widths the staged kernel does not take: an odd number of groups (832 = 13 of 64), several 16-row blocks per CTA
+    with a remainder (4784 = 299 blocks, 9488 = 593), fewer groups than K slices (192), rows longer than a stage."""
+    rng = np.random.default_rng(700 + bits + N + K + rows)
+    m, host = affine_case(rng, N, K, bits, cuda_device)
+    x = synth.activations_np(rng, rows, K)
+    y = run(m, x_tensor(x, cuda_device), rows)
+    assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(x, deq(host, bits))) <= TOL
+    alone = run(m, x_tensor(x[rows - 1:], cuda_device), 1)
+    assert torch.equal(alone[0], y[rows - 1])

@@ -80,3 +80,17 @@ def test_lm_head_then_argmax(cuda_device):
     assert np.array_equal(am.cpu().numpy().astype(np.uint32), qref.argmax_rows(y.cpu().numpy()))
     ref = qref.matmul_t(x, qref.dequant_affine(w[0], s[0], b[0], 4))
     assert qref.max_rel(y.cpu().numpy(), ref) <= 1e-3
+
+
+@pytest.mark.parametrize("V", [63, 64, 65, 1024, 4095, 4096, 4097, 8192])
+def test_candidates_at_the_edges_of_a_part(cuda_device, V):
+    """Fewer, exactly and more than 64 logits, parts that end on a boundary, and rows whose logits are all equal, equal but
+    one, or all but 64 far below."""
+    x = logits("random", V, 5, V)
+    x[1] = 2.5
+    x[2] = 2.5
+    x[2, V - 1] = 3.0
+    x[3] = -1e30
+    x[3, :: max(1, V // 64)] = 1.0
+    x[4] = np.float32(1.0) + np.arange(V, dtype=np.float32) * np.float32(2 ** -23)  # neighbouring floats
+    check(x, [0.7])

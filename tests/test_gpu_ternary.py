@@ -135,3 +135,20 @@ def test_ternary_guards(cuda_device):
     with pytest.raises(capi.IngotError) as e:  # the kernel takes the rotation's fp16 output
         VQMV.encode(x, m, y, 2)
     assert e.value.status == -1
+
+
+@pytest.mark.parametrize("N,K,rows", [(16, 1024, 8), (48, 5120, 9), (2400, 5120, 5), (16, 14336, 16)])
+def test_ternary_qmv_edges(cuda_device, N, K, rows):
+    """One block, group counts that the warps do not share evenly (40, 112), the step from eight to nine rows; a row alone has
+    the same bits."""
+    rng = np.random.default_rng(N + K + rows)
+    m, wf, signs, _ = case(rng, N, K, cuda_device)
+    x = half_activations(rng, rows, K)
+    xt = x_tensor(x, cuda_device, torch.float16)
+    y = torch.zeros(rows, N, dtype=torch.float32, device=cuda_device)
+    VQMV.encode(xt, m, y, rows)
+    alone = torch.zeros(1, N, dtype=torch.float32, device=cuda_device)
+    VQMV.encode(xt[rows - 1:].contiguous(), m, alone, 1)
+    torch.cuda.synchronize()
+    assert torch.equal(alone[0], y[rows - 1])
+    assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(qref.rotate_input(x, signs), wf)) <= TERN_TOL
