@@ -5,6 +5,7 @@
 
 #include "internal.h"
 #include "moe_aux.cuh"
+#include "moe_small.cuh"
 
 struct iq_moe {
     iq_ctx* ctx = nullptr;
@@ -36,6 +37,7 @@ struct MoeWs {
     __half* h;
     void* yd;
     __half* xs;  // activations in expert order, fp16 [P, d_model] (tensor-core path)
+    FixedRows fx, fh;  // calls of few tokens: the activations and h as block fixed point
     // shared expert (only when the layer has one): fp16 copy of x, h, output, per-token weight, tile list
     __half* s_x16;
     __half* s_h;
@@ -87,6 +89,11 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     w.h = static_cast<__half*>(take(P * d.d_ff * 2));
     w.yd = take(P * d.d_model * (yd_dtype_of(l) == kF16 ? 2 : 4));
     w.xs = static_cast<__half*>(take(P * d.d_model * 2));
+    const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens;
+    w.fx.digits = static_cast<unsigned char*>(take(few * (d.d_model / 64) * 128));
+    w.fx.scale = static_cast<float2*>(take(few * (d.d_model / 64) * 8));
+    w.fh.digits = static_cast<unsigned char*>(take(few * d.top_k * (d.d_ff / 64) * 128));
+    w.fh.scale = static_cast<float2*>(take(few * d.top_k * (d.d_ff / 64) * 8));
     w.s_x16 = nullptr; w.s_h = nullptr; w.s_yd = nullptr; w.s_w = nullptr; w.s_tiles = nullptr; w.s_ntiles = nullptr;
     if (d.shared != IQ_SHARED_NONE) {
         const size_t T = (size_t)tokens;
@@ -136,13 +143,12 @@ bool tensor_router(const iq_moe* l, int tokens, int32_t x_dtype) {
 }
 float router_err_coef(const iq_moe* l) { return (float)l->d.d_model * 4.76837158e-7f * 1.05f * l->router_wnorm_max; }
 
-int32_t launch_route(iq_moe* l, cudaStream_t st, const float* logits, int ld, int tokens, uint32_t* inds, float* wts,
-                     const void* refine_x = nullptr, int64_t ldx = 0) {
+RouteParams route_params(const iq_moe* l, const float* logits, int ld, int tokens, uint32_t* inds, float* wts) {
     RouteParams rp;
     rp.logits = logits;
     rp.logits_rw = const_cast<float*>(logits);
-    rp.x = static_cast<const uint16_t*>(refine_x);
-    rp.ldx = ldx;
+    rp.x = nullptr;
+    rp.ldx = 0;
     rp.wr = static_cast<const uint16_t*>(l->d.router_w);
     rp.D = l->d.d_model;
     rp.err_coef = router_err_coef(l);
@@ -155,6 +161,14 @@ int32_t launch_route(iq_moe* l, cudaStream_t st, const float* logits, int ld, in
     rp.sigmoid = l->d.router_score == IQ_SCORE_SIGMOID ? 1 : 0;
     rp.select_bias = l->d.router_select_bias;
     rp.eps = l->d.route_eps;
+    return rp;
+}
+
+int32_t launch_route(iq_moe* l, cudaStream_t st, const float* logits, int ld, int tokens, uint32_t* inds, float* wts,
+                     const void* refine_x = nullptr, int64_t ldx = 0) {
+    RouteParams rp = route_params(l, logits, ld, tokens, inds, wts);
+    rp.x = static_cast<const uint16_t*>(refine_x);
+    rp.ldx = ldx;
     const bool wide = refine_x != nullptr && tokens <= kRouteWideMaxTokens;
     route_kernel_for(l->d.experts, refine_x != nullptr, wide)<<<wide ? tokens : (tokens + 3) / 4, 128, 0, st>>>(rp);
     return check_cuda(l->ctx, cudaGetLastError(), "route_topk launch");
@@ -262,6 +276,87 @@ int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows,
     return launch_qmm(l->ctx, cs, c);
 }
 
+// ---- few tokens (csrc/moe_small.cuh) ----
+typedef void (*RouteSmallKernel)(const RouteSmallParams);
+template <int WFMT, int TT>
+RouteSmallKernel route_small_vpl(int experts) {
+    return experts <= 128 ? moe_route_small_kernel<WFMT, TT, 4> : moe_route_small_kernel<WFMT, TT, 16>;
+}
+template <int WFMT>
+RouteSmallKernel route_small_of(int tt, int experts) {
+    return tt == 1 ? route_small_vpl<WFMT, 1>(experts) : tt == 2 ? route_small_vpl<WFMT, 2>(experts)
+         : tt == 4 ? route_small_vpl<WFMT, 4>(experts) : route_small_vpl<WFMT, 8>(experts);
+}
+RouteSmallKernel route_small_pick(bool q8, int tt, int experts) { return q8 ? route_small_of<1>(tt, experts) : route_small_of<0>(tt, experts); }
+constexpr size_t kRouteSmallSmemMax = 200 * 1024;
+
+// Router, top-k and permutation in one cluster: up to eight tokens, while the float64 products of a block (a cluster has
+// eight) stay at a few microseconds and the tokens fit its shared memory. 128 experts x 2048 inputs: all eight tokens.
+int route_small_tokens(int tokens) { return tokens <= 1 ? 1 : tokens <= 2 ? 2 : tokens <= 4 ? 4 : 8; }
+bool use_route_small(const iq_moe* l, int tokens) {
+    const iq_moe_desc& d = l->d;
+    const int tt = route_small_tokens(tokens);
+    return tokens <= kSmallTokens && l->ext_inds == nullptr && d.expert_lo == 0 && d.expert_count == d.experts &&
+           (int64_t)d.experts * d.d_model * tt <= (1 << 21) && route_small_smem(tt, d.d_model, d.experts) <= kRouteSmallSmemMax;
+}
+// The experts' kernels for few tokens: affine 4-bit weights, 16-byte aligned
+bool use_experts_small(const iq_moe* l) {
+    const iq_moe_desc& d = l->d;
+    uintptr_t a = 0;
+    for (const iq_qlinear* m : {&d.gate, &d.up, &d.down})
+        a |= reinterpret_cast<uintptr_t>(m->w) | (reinterpret_cast<uintptr_t>(m->scales) << 2) | (reinterpret_cast<uintptr_t>(m->biases) << 2);
+    return l->fmt == kFmtAffine4 && (a & 15) == 0;
+}
+
+int32_t run_route_small(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, int64_t ldx, int tokens, const MoeWs& w, bool fixed) {
+    const iq_moe_desc& d = l->d;
+    RouteSmallParams p;
+    p.r = route_params(l, w.logits, l->ld, tokens, w.inds, w.wts);
+    p.x = x; p.x_dtype = x_dtype; p.ldx = ldx;
+    p.wr = d.router_w; p.ws = d.router_scales; p.wb = d.router_biases;
+    p.counts = w.counts; p.offsets = w.offsets; p.row_map = w.row_map; p.pos = w.pos; p.ntiles = w.ntiles;
+    p.tiles_a = w.tiles_a; p.tiles_b = w.tiles_b;
+    p.fx = fixed ? w.fx : FixedRows{nullptr, nullptr};
+    const int tt = route_small_tokens(tokens);
+    return check_cuda(l->ctx, launch_dependent(route_small_pick(d.router_kind != IQ_ROUTER_BF16, tt, d.experts), dim3(kSmallCluster), kSmallThreads,
+                                               route_small_smem(tt, d.d_model, d.experts), cs, p), "moe_route_small launch");
+}
+
+int32_t run_experts_small(iq_moe* l, cudaStream_t cs, int tokens, const MoeWs& w, void* out, int32_t out_dtype, int64_t ldo, int accumulate) {
+    const iq_moe_desc& d = l->d;
+    iq_ctx* ctx = l->ctx;
+    GateUpSmallParams g;
+    const iq_qlinear* m[2] = {&d.gate, &d.up};
+    for (int i = 0; i < 2; i++) {
+        g.w[i] = static_cast<const unsigned char*>(m[i]->w);
+        g.s[i] = static_cast<const unsigned char*>(m[i]->scales);
+        g.b[i] = static_cast<const unsigned char*>(m[i]->biases);
+        g.ebias[i] = i ? d.up_bias : d.gate_bias;
+    }
+    g.D = d.d_model; g.I = d.d_ff; g.topk = d.top_k;
+    g.x = w.fx; g.row_map = w.row_map; g.tiles = w.tiles_a; g.ntiles = w.ntiles;
+    g.act = d.act; g.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
+    g.h = w.h; g.fh = w.fh;
+    const int64_t items = (int64_t)tokens * d.top_k * (d.d_ff / 64);
+    int32_t st = check_cuda(ctx, launch_dependent(moe_gateup_small_kernel, dim3((unsigned)(items < ctx->sms ? items : ctx->sms)), kSmallThreads, 0, cs, g),
+                            "moe_gateup_small launch");
+    if (st != kOk) return st;
+    DownSmallParams p;
+    p.w = static_cast<const unsigned char*>(d.down.w);
+    p.s = static_cast<const unsigned char*>(d.down.scales);
+    p.b = static_cast<const unsigned char*>(d.down.biases);
+    p.D = d.d_model; p.I = d.d_ff; p.topk = d.top_k; p.T = tokens;
+    p.fh = w.fh; p.inds = w.inds; p.pos = w.pos; p.wts = w.wts;
+    p.ebias = d.down_bias;
+    p.yd = static_cast<__half*>(w.yd);
+    p.out = out; p.out_dtype = out_dtype; p.ldo = ldo; p.accumulate = accumulate;
+    p.slices = 1;
+    while (p.slices * 2 * d.top_k <= 16) p.slices *= 2;
+    const int ditems = tokens * (d.d_model / 16);
+    return check_cuda(ctx, launch_dependent(moe_down_small_kernel, dim3(ditems < ctx->sms ? ditems : ctx->sms), kSmallThreads, 0, cs, p),
+                      "moe_down_small launch");
+}
+
 // The shared expert (MoE.swift:140-154; the reference runs it as expert id E of the same kernels): one more FFN over all
 // tokens, rows in place, through the same tile kernels with a copy of the layer whose expert tensors are the shared
 // expert's; out += w_s * y_s with w_s = sigmoid(x . shared_gate) or 1.
@@ -290,6 +385,35 @@ int32_t run_shared_expert(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_d
         st = check_cuda(ctx, cudaGetLastError(), "shared tiles launch");
         if (st == kOk) st = run_gateup_tc(&tmp, cs, w.s_x16, tokens, w.s_tiles, w.s_ntiles, w.s_h, bn);
         if (st == kOk) st = run_down_tc(&tmp, cs, w.s_h, tokens, w.s_tiles, w.s_ntiles, w.s_yd, ydt, bn);
+    } else if (tokens <= 16) {  // a dense FFN on the decode kernels, no tile list
+        GqmvCall c;
+        c.mode = kModeGateUp;
+        c.fmt = kFmtAffine4;
+        const iq_qlinear* m[2] = {&d.shared_gate_proj, &d.shared_up};
+        for (int i = 0; i < 2; i++) {
+            c.w[i] = static_cast<const uint32_t*>(m[i]->w);
+            c.s[i] = m[i]->scales;
+            c.b[i] = m[i]->biases;
+        }
+        c.N = d.shared_up.n; c.K = d.d_model;
+        c.x = x; c.x_dtype = x_dtype; c.ldx = ldx;
+        c.rows = tokens; c.max_rows = tokens;
+        c.y = w.s_h; c.y_dtype = kF16; c.ldy = d.shared_up.n;
+        c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
+        c.act = d.act;
+        st = launch_gqmv(ctx, cs, c);
+        if (st != kOk) return st;
+        GqmvCall q;
+        q.mode = kModePlain;
+        q.fmt = kFmtAffine4;
+        q.w[0] = static_cast<const uint32_t*>(d.shared_down.w);
+        q.s[0] = d.shared_down.scales;
+        q.b[0] = d.shared_down.biases;
+        q.N = q.n_full = d.d_model; q.K = d.shared_up.n;
+        q.x = w.s_h; q.x_dtype = kF16; q.ldx = d.shared_up.n;
+        q.rows = tokens; q.max_rows = tokens;
+        q.y = w.s_yd; q.y_dtype = ydt; q.ldy = d.d_model;
+        st = launch_gqmv(ctx, cs, q);
     } else {
         const int bm = 16;
         shared_tiles_kernel<<<1, 128, 0, cs>>>(tokens, bm, 0u, w.s_tiles, w.s_ntiles);
@@ -324,6 +448,9 @@ int32_t moe_init(iq_ctx* ctx) {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(router_logits_kernel<1>),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kRouterSmemMax);
+    for (int v = 0; v < 16 && e == cudaSuccess; v++)
+        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(route_small_pick(v & 1, 1 << (v >> 1 & 3), v >> 3 ? 256 : 32)),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouteSmallSmemMax);
     return check_cuda(ctx, e, "cudaFuncSetAttribute(router)");
 }
 
@@ -610,6 +737,16 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     const float* wts = l->ext_wts ? l->ext_wts : w.wts;
     int32_t st;
 
+    const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l);
+    if (small) {
+        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, small_experts);
+        if (st == kOk && small_experts)
+            st = run_experts_small(l, cs, tokens, w, out, out_dtype, ldo, (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0);
+        if (st != kOk) return st;
+        if (small_experts)
+            return d.shared != IQ_SHARED_NONE ? run_shared_expert(l, cs, x, x_dtype, ldx, tokens, w, out, out_dtype, ldo) : kOk;
+        pieces &= ~(uint32_t)(IQ_PIECE_ROUTER | IQ_PIECE_ROUTE | IQ_PIECE_GROUP);
+    }
     const bool fast_router = tensor_router(l, tokens, x_dtype);
     if ((pieces & IQ_PIECE_ROUTER) && fast_router) {
         QmmCall c;
@@ -888,6 +1025,6 @@ extern "C" int32_t iq_rmsnorm(iq_ctx* ctx, void* stream, const float* x, int64_t
     if (x == nullptr || out == nullptr || rows < 1 || d < 4 || d % 4 != 0 || ldx < d || ldo < d || ldx % 4 != 0 ||
         ldo % 4 != 0 || out_dtype < 0 || out_dtype > 2)
         return fail(ctx, kErrInvalidArg, "rmsnorm: arguments");
-    rmsnorm_kernel<<<rows, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(x, ldx, out, out_dtype, ldo, d, eps);
-    return check_cuda(ctx, cudaGetLastError(), "rmsnorm launch");
+    return check_cuda(ctx, launch_dependent(rmsnorm_kernel, dim3(rows), 256, 0, reinterpret_cast<cudaStream_t>(stream), x, ldx, out, out_dtype, ldo, d, eps),
+                      "rmsnorm launch");
 }

@@ -350,6 +350,54 @@ __device__ __forceinline__ float exact_dot_bf16(const uint16_t* __restrict__ xro
     return (float)acc;
 }
 
+// A float as an unsigned that orders like it (-0 as +0, so that they tie; -inf above 0, which stands for "not a candidate").
+__device__ __forceinline__ uint32_t route_key(float f) {
+    const uint32_t u = __float_as_uint(f == 0.f ? 0.f : f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// The selection rule and the weights, by one warp for one token: lane l holds the scores v[j] of experts 32 j + l (pv[j]: the
+// unbiased sigmoid score), `taken` marks experts out of the running. Writes inds / wts when `store`; lane k returns the k-th
+// expert (k < topk). Two warp reductions per pick (maximum, then the lowest index that holds it) on integer keys.
+template <int VPL>
+__device__ __forceinline__ uint32_t route_select(const float (&v)[VPL], const float (&pv)[VPL], uint32_t taken, int topk, int lane,
+                                                 bool sigmoid, float eps, float scale, const float* pes, uint32_t* inds, float* wts,
+                                                 bool store) {
+    uint32_t key[VPL];
+#pragma unroll
+    for (int j = 0; j < VPL; j++) key[j] = ((taken >> j) & 1u) ? 0u : route_key(v[j]);
+    float myv = -INFINITY, myp = 0.f;
+    uint32_t myi = 0;
+    for (int k = 0; k < topk; k++) {
+        uint32_t bk = 0, bj = 0;
+        float bv = 0.f, bp = 0.f;
+#pragma unroll
+        for (int j = 0; j < VPL; j++)
+            if (key[j] > bk) { bk = key[j]; bj = j; bv = v[j]; bp = pv[j]; }
+        const uint32_t top = __reduce_max_sync(0xffffffffu, bk);
+        const uint32_t gi = __reduce_min_sync(0xffffffffu, bk == top ? bj * 32 + lane : 0xFFFFFFFFu);
+        const float gv = __shfl_sync(0xffffffffu, bv, gi & 31u), gp = sigmoid ? __shfl_sync(0xffffffffu, bp, gi & 31u) : 0.f;
+#pragma unroll
+        for (int j = 0; j < VPL; j++)
+            if ((uint32_t)(j * 32 + lane) == gi) key[j] = 0;
+        if (lane == k) { myv = gv; myi = gi; myp = gp; }
+    }
+    float num = myp, sum = 0.f;
+    if (!sigmoid) {
+        const float top1 = __shfl_sync(0xffffffffu, myv, 0);
+        num = lane < topk ? expf(myv - top1) : 0.f;
+    }
+    for (int k = 0; k < topk; k++) sum += __shfl_sync(0xffffffffu, num, k);
+    if (sigmoid) sum += eps;
+    if (lane < topk && store) {
+        float w = num / sum * scale;
+        if (pes != nullptr) w *= pes[myi];
+        inds[lane] = myi;
+        wts[lane] = w;
+    }
+    return myi;
+}
+
 // WPT: warps per token. 1: a block takes four tokens. 4 (refinement only): a block takes one token and its warps share
 // the exact dot products (candidate c goes to warp c % 4, results meet in shared memory); everything else runs in all
 // four warps alike. With few tokens per GPU the refinement is one dependent chain per warp, so four warps per token
@@ -385,23 +433,24 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
         // ---- which experts can still be among the k largest? Those within 2 eps of the k-th largest approximate value:
         // with |approx - exact| <= eps everywhere, at least k experts have an exact value >= kth - eps, so a true member of
         // the top k has exact >= kth - eps and approx >= kth - 2 eps. The exact values of these candidates decide.
-        uint32_t tk = taken;
-        float kth = -INFINITY;
+        uint32_t key[VPL], kth_key = 0;
+#pragma unroll
+        for (int j = 0; j < VPL; j++) key[j] = ((taken >> j) & 1u) ? 0u : route_key(v[j]);
         for (int k = 0; k < p.topk; k++) {
-            float bv = -INFINITY;
-            int bj = -1;
+            uint32_t bk = 0, bj = 0;
 #pragma unroll
             for (int j = 0; j < VPL; j++)
-                if (!((tk >> j) & 1u) && (bj < 0 || v[j] > bv)) { bv = v[j]; bj = j; }
-            float gv = bj >= 0 ? bv : -INFINITY;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) gv = fmaxf(gv, __shfl_xor_sync(0xffffffffu, gv, o));
+                if (key[j] > bk) { bk = key[j]; bj = j; }
+            kth_key = __reduce_max_sync(0xffffffffu, bk);
             // one holder of the maximum drops out (the lowest lane; which one is irrelevant for the k-th value)
-            const uint32_t holders = __ballot_sync(0xffffffffu, bj >= 0 && bv == gv);
-            if (holders == 0u) { gv = -INFINITY; }
-            else if (lane == __ffs(holders) - 1) tk |= 1u << bj;
-            kth = gv;
+            const uint32_t holders = __ballot_sync(0xffffffffu, bk == kth_key);
+            if (lane == __ffs(holders) - 1) {
+#pragma unroll
+                for (int j = 0; j < VPL; j++)
+                    if ((uint32_t)j == bj) key[j] = 0;
+            }
         }
+        const float kth = __uint_as_float((kth_key & 0x80000000u) ? (kth_key & 0x7FFFFFFFu) : ~kth_key);
         const uint16_t* xrow = p.x + (size_t)t * p.ldx;
         float ss = 0.f;
         for (int u = lane; u < p.D / 8; u += 32) {
@@ -459,63 +508,8 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
             }
         }
     }
-    float myv = -INFINITY, myp = 0.f;
-    uint32_t myi = 0;
-    for (int k = 0; k < p.topk; k++) {
-        float bv = -INFINITY;
-        uint32_t bi = 0xFFFFFFFFu;
-#pragma unroll
-        for (int j = 0; j < VPL; j++) {
-            if (!((taken >> j) & 1u) && (bi == 0xFFFFFFFFu || v[j] > bv)) {
-                bv = v[j];
-                bi = j * 32 + lane;
-            }
-        }
-        // warp maximum over the lanes that still have a candidate, then the lowest index among the equal ones
-        float gv = bv;
-        uint32_t any = bi != 0xFFFFFFFFu;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, gv, o);
-            const uint32_t oa = __shfl_xor_sync(0xffffffffu, any, o);
-            if (oa && (!any || ov > gv)) gv = ov;
-            any |= oa;
-        }
-        uint32_t gi = (bi != 0xFFFFFFFFu && bv == gv) ? bi : 0xFFFFFFFFu;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) gi = min(gi, __shfl_xor_sync(0xffffffffu, gi, o));
-        float gp = 0.f;  // the chosen expert's unbiased score, from the lane that holds it
-#pragma unroll
-        for (int j = 0; j < VPL; j++)
-            if ((uint32_t)(j * 32 + lane) == gi) {
-                taken |= 1u << j;
-                gp = pv[j];
-            }
-        gp = __shfl_sync(0xffffffffu, gp, gi & 31u);
-        if (lane == k) { myv = gv; myi = gi; myp = gp; }
-    }
-    if (p.sigmoid) {
-        float sum = 0.f;
-        for (int k = 0; k < p.topk; k++) sum += __shfl_sync(0xffffffffu, myp, k);
-        sum += p.eps;
-        if (lane < p.topk && (WPT == 1 || wib == 0)) {
-            float w = myp / sum * p.scale;
-            if (p.pes != nullptr) w *= p.pes[myi];
-            p.inds[(size_t)t * p.topk + lane] = myi;
-            p.wts[(size_t)t * p.topk + lane] = w;
-        }
-        return;
-    }
-    const float top1 = __shfl_sync(0xffffffffu, myv, 0);
-    const float ex = lane < p.topk ? expf(myv - top1) : 0.f;
-    float sum = 0.f;
-    for (int k = 0; k < p.topk; k++) sum += __shfl_sync(0xffffffffu, ex, k);
-    if (lane < p.topk && (WPT == 1 || wib == 0)) {
-        float w = ex / sum * p.scale;
-        if (p.pes != nullptr) w *= p.pes[myi];
-        p.inds[(size_t)t * p.topk + lane] = myi;
-        p.wts[(size_t)t * p.topk + lane] = w;
-    }
+    route_select<VPL>(v, pv, taken, p.topk, lane, p.sigmoid != 0, p.eps, p.scale, p.pes, p.inds + (size_t)t * p.topk,
+                      p.wts + (size_t)t * p.topk, WPT == 1 || wib == 0);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -984,6 +978,8 @@ __global__ void __launch_bounds__(256) shared_add_kernel(const void* __restrict_
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ x, int64_t ldx, void* __restrict__ out,
                                                      int32_t out_dtype, int64_t ldo, int d, float eps) {
     __shared__ float wsum[8];
+    pdl_launch_dependents();
+    pdl_wait();
     const float* xr = x + (size_t)blockIdx.x * ldx;
     float s = 0.f;
     for (int i = threadIdx.x * 4; i < d; i += 1024) {

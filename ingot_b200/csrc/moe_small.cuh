@@ -1,0 +1,555 @@
+// The MoE block for up to eight tokens in three kernels, where a decode step of few tokens is a chain of latencies and not
+// of bytes (one token of the 128-expert layer reads 21 MB, 3 us, and took 59 us in eight kernels):
+//
+//   moe_route_small_kernel   router logits, top-k and the permutation in one cluster of eight blocks; also the activations as
+//                            block fixed point (the int8 kernels' operand, see qmv_imma.cuh), once per token
+//   moe_gateup_small_kernel  h = act(gate x, up x) per (expert tile, 64 features): weights straight from global memory into
+//                            registers, and h leaves as fp16 and as the down projection's block fixed point, group by group
+//   moe_down_small_kernel    per (token, 16 features) the down projections of all the token's experts side by side in the
+//                            block's warps, then their weighted sum: the combine needs no kernel and no round trip
+//
+// Each starts while its predecessor runs (programmatic dependent launch); the down kernel has its first weights on the way
+// before h exists. Affine 4-bit experts, all of them on this GPU. The results are those of the separate kernels: exact
+// float64 logits, the same quantisation, sums in fixed orders.
+#pragma once
+
+#include "common.cuh"
+#include "gqmv.cuh"
+#include "moe_aux.cuh"
+#include "ptx.cuh"
+#include "qmv_imma.cuh"
+
+namespace iq {
+
+constexpr int kSmallTokens = 8;
+constexpr int kSmallThreads = 512;
+constexpr int kSmallCluster = 8;
+
+// Row r of an activation matrix as block fixed point: per group of 64 inputs 128 bytes, the high digits' fragments of the
+// four lanes of a quad (16 bytes each: two MMAs) and the low digits', and {2^(e-13), sum}.
+struct FixedRows {
+    unsigned char* digits;  // [rows][groups][2][4][16]
+    float2* scale;          // [rows][groups]
+};
+
+// Eight consecutive inputs (word w8 of the group's eight) of a row's group: the eight threads of a group are eight
+// neighbouring lanes. See qmv_imma.cuh for the arithmetic.
+__device__ __forceinline__ void fixed_point_unit(const float (&v)[8], int w8, unsigned char* digits, float2* scale) {
+    float amax = 0.f, sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        amax = fmaxf(amax, fabsf(v[k]));
+        sum += v[k];
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    }
+    float sc, inv;
+    qi_group_scale(amax, sum, sc, inv);
+    if (digits == nullptr) return;
+    if (w8 == 0) *scale = make_float2(sc, sum);
+    uint32_t hi_w[2] = {0, 0}, lo_w[2] = {0, 0};
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int X = __float2int_rn(v[k] * inv);
+        const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
+        hi_w[k & 1] |= (uint32_t)(hi_d & 0xFF) << (8 * (k >> 1));
+        lo_w[k & 1] |= (uint32_t)(lo_d & 0xFF) << (8 * (k >> 1));
+    }
+    unsigned char* f = digits + (w8 >> 1) * 16 + (w8 & 1) * 8;
+    *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
+    *reinterpret_cast<uint2*>(f + 64) = make_uint2(lo_w[0], lo_w[1]);
+}
+
+struct RouteSmallParams {
+    RouteParams r;               // logits_rw, inds, wts, T, E, ld, topk, D and the scoring rule
+    const void* x;
+    int32_t x_dtype;
+    int64_t ldx;
+    const void* wr;
+    const void* ws;              // 8-bit router: scales and biases
+    const void* wb;
+    uint32_t *counts, *offsets, *row_map, *pos, *ntiles;
+    Tile *tiles_a, *tiles_b;
+    FixedRows fx;                // the activations as block fixed point, or null
+};
+constexpr size_t route_small_smem(int tt, int D, int E) {
+    return (size_t)tt * D * 8 + (size_t)4 * (E / kSmallCluster) * tt * 8 + (size_t)tt * E * 4 + 16 * kSmallTokens * 4 + 64 * 4;
+}
+
+// WFMT: 0 bf16 router, 1 8-bit affine. TT: tokens rounded up to 1, 2, 4, 8. VPL: experts per lane of the selection.
+// A block of the cluster takes E / 8 experts; its sixteen warps are (four experts, a quarter of the inputs) each, products
+// and sums in float64 (exact at fp32 resolution: the logits are the other router kernels' bits). The logits meet in the
+// first block's shared memory, which then selects (a warp per token) and groups.
+template <int WFMT, int TT, int VPL>
+__global__ void __launch_bounds__(kSmallThreads, 1) __cluster_dims__(kSmallCluster, 1, 1) moe_route_small_kernel(const RouteSmallParams p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int T = p.r.T, E = p.r.E, D = p.r.D, topk = p.r.topk, units = D / 8, epc = E / kSmallCluster;
+    double2* xs = reinterpret_cast<double2*>(smem);                               // [TT][4][units]: inputs 2j, 2j + 1 of a unit
+    double* part = reinterpret_cast<double*>(smem + (size_t)TT * D * 8);          // [4][epc][TT]
+    float* lg = reinterpret_cast<float*>(part + (size_t)4 * epc * TT);            // [TT][E], the first block's
+    uint32_t* sinds = reinterpret_cast<uint32_t*>(lg + (size_t)TT * E);           // [16 * 8]
+    uint32_t* wsum = sinds + 16 * kSmallTokens;                                   // [2][32]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x, e0 = rank * epc;
+    pdl_launch_dependents();
+
+    // one unit of eight router weights of four experts: bf16 words, or codes with scale and bias
+    auto fetch = [&](uint4 (&w)[4], int pr, int u) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const size_t e = e0 + (pr >> 2) * 4 + i;
+            if (WFMT == 0) {
+                w[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.wr) + e * D) + u);
+            } else {
+                const uint2 q = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint32_t*>(p.wr) + e * (D / 4)) + u);
+                const size_t gi = e * (D / 64) + u / 8;
+                w[i] = make_uint4(q.x, q.y, __ldg(reinterpret_cast<const uint16_t*>(p.ws) + gi), __ldg(reinterpret_cast<const uint16_t*>(p.wb) + gi));
+            }
+        }
+    };
+    const int uq = (units + 3) / 4;  // units per quarter of the inputs
+    uint4 w[4], wn[4];
+    {
+        const int u0 = (warp & 3) * uq + lane;  // the router does not depend on the previous kernel
+        fetch(w, warp < epc ? warp : 0, min(u0, units - 1));
+    }
+    pdl_wait();
+    for (int i = tid; i < TT * units; i += kSmallThreads) {
+        const int t = i / units, u = i % units;
+        float v[8];
+        if (t < T) load_x8(p.x, p.x_dtype, (size_t)t * p.ldx + u * 8, v);
+        else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) xs[(t * 4 + j) * units + u] = make_double2((double)v[2 * j], (double)v[2 * j + 1]);
+    }
+    __syncthreads();
+    for (int pr = warp; pr < epc; pr += kSmallThreads / 32) {
+        double acc[4 * TT];
+#pragma unroll
+        for (int i = 0; i < 4 * TT; i++) acc[i] = 0.0;
+        const int u_end = min(units, ((pr & 3) + 1) * uq);
+        int u = (pr & 3) * uq + lane;
+        if (pr != warp && u < u_end) fetch(w, pr, u);
+        for (; u < u_end; u += 32) {
+            fetch(wn, pr, min(u + 32, units - 1));
+            float sc[4], bi[4];
+            if (WFMT == 1) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) { sc[i] = bf16_bits_to_f32(w[i].z); bi[i] = bf16_bits_to_f32(w[i].w); }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                double wd[4][2];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (WFMT == 0) {
+                        const uint32_t q = j == 0 ? w[i].x : (j == 1 ? w[i].y : (j == 2 ? w[i].z : w[i].w));
+                        wd[i][0] = (double)__uint_as_float(q << 16);
+                        wd[i][1] = (double)__uint_as_float(q & 0xFFFF0000u);
+                    } else {  // the fp32 s*q + b of the reference's CPU dequantisation
+                        const uint32_t q = (j < 2 ? w[i].x : w[i].y) >> (16 * (j & 1));
+                        wd[i][0] = (double)__fadd_rn(__fmul_rn(sc[i], (float)(q & 0xFFu)), bi[i]);
+                        wd[i][1] = (double)__fadd_rn(__fmul_rn(sc[i], (float)((q >> 8) & 0xFFu)), bi[i]);
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < TT; t++) {
+                    const double2 xv = xs[(t * 4 + j) * units + u];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        acc[i * TT + t] = fma(xv.x, wd[i][0], acc[i * TT + t]);
+                        acc[i * TT + t] = fma(xv.y, wd[i][1], acc[i * TT + t]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = wn[i];
+        }
+        // the lanes' sums: while there are several values left, a lane keeps half of them and hands over the other half
+        int n = 4 * TT, idx = 0, dup = 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            if (n > 1) {
+                const int half = n / 2;
+                const bool up = lane & o;
+#pragma unroll
+                for (int i = 0; i < 2 * TT; i++) {
+                    if (i >= half) break;
+                    const double send = up ? acc[i] : acc[i + half], keep = up ? acc[i + half] : acc[i];
+                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+                if (up) idx += half;
+                n = half;
+            } else {
+                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+                dup |= lane & o;
+            }
+        }
+        if (dup == 0) part[((pr & 3) * epc + (pr >> 2) * 4 + idx / TT) * TT + idx % TT] = acc[0];
+    }
+    __syncthreads();
+    cluster_sync_all();  // (every block of the cluster runs: the first one's shared memory may be written)
+    for (int i = tid; i < epc * TT; i += kSmallThreads) {
+        const int e = i / TT, t = i % TT;
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) s += part[(k * epc + e) * TT + t];
+        const float f = (float)s;
+        st_dsmem_u32(reinterpret_cast<uint32_t*>(lg + (size_t)t * E + e0 + e), 0, __float_as_uint(f));
+        if (t < T) p.r.logits_rw[(size_t)t * p.r.ld + e0 + e] = f;
+    }
+    if (rank == kSmallCluster - 1)
+        for (int i = tid; i < T * (p.r.ld - E); i += kSmallThreads) p.r.logits_rw[(size_t)(i / (p.r.ld - E)) * p.r.ld + E + i % (p.r.ld - E)] = 0.f;
+    cluster_sync_all();
+    // the other blocks turn the activations into fixed point (tokens rank - 1, rank + 6)
+    if (rank != 0) {
+        if (p.fx.digits == nullptr) return;
+        for (int t = rank - 1; t < T; t += kSmallCluster - 1) {
+            const int G = D / 64, upad = (units + 31) / 32 * 32;
+            for (int u = tid; u < upad; u += kSmallThreads) {
+                const bool live = u < units;
+                float v[8];
+                load_x8(p.x, p.x_dtype, (size_t)t * p.ldx + (live ? u : 0) * 8, v);
+                const size_t g = (size_t)t * G + u / 8;
+                fixed_point_unit(v, u & 7, live ? p.fx.digits + g * 128 : nullptr, p.fx.scale + (live ? g : 0));
+            }
+        }
+        return;
+    }
+    if (warp < T) {
+        const int t = warp;
+        float v[VPL], pv[VPL];
+        uint32_t taken = 0;
+#pragma unroll
+        for (int j = 0; j < VPL; j++) {
+            const int e = j * 32 + lane;
+            float f = e < E ? lg[(size_t)t * E + e] : -INFINITY;
+            if (e < E && p.r.logit_bias != nullptr) f += p.r.logit_bias[e];
+            pv[j] = 0.f;
+            if (p.r.sigmoid) {
+                f = (float)(1.0 / (1.0 + exp(-(double)f)));
+                pv[j] = f;
+                if (e < E && p.r.select_bias != nullptr) f += p.r.select_bias[e];
+            }
+            if (f != f) f = -INFINITY;
+            v[j] = f;
+            if (e >= E) taken |= 1u << j;
+        }
+        const uint32_t mine = route_select<VPL>(v, pv, taken, topk, lane, p.r.sigmoid != 0, p.r.eps, p.r.scale, p.r.pes,
+                                                p.r.inds + (size_t)t * topk, p.r.wts + (size_t)t * topk, true);
+        if (lane < topk) sinds[t * topk + lane] = mine;
+    }
+    __syncthreads();
+    // ---- the permutation: a thread per expert counts and places, a thread per pair finds its position --------------------
+    const int P = T * topk;
+    uint32_t c = 0;
+    if (tid < E)
+        for (int i = 0; i < P; i++) c += sinds[i] == (uint32_t)tid;
+    uint32_t off = c, til = c > 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xffffffffu, off, o), b = __shfl_up_sync(0xffffffffu, til, o);
+        if (lane >= o) { off += a; til += b; }
+    }
+    if (lane == 31) { wsum[warp] = off; wsum[32 + warp] = til; }
+    __syncthreads();
+    for (int k = 0; k < warp; k++) { off += wsum[k]; til += wsum[32 + k]; }
+    uint32_t* soff = reinterpret_cast<uint32_t*>(part);  // exclusive offsets
+    __syncthreads();
+    if (tid < E) {
+        soff[tid] = off - c;
+        p.counts[tid] = c;
+        p.offsets[tid] = off - c;
+        if (c > 0) p.tiles_a[til - 1] = p.tiles_b[til - 1] = Tile{(uint32_t)tid, off - c, c, 0};  // (c <= T: one tile)
+        if (tid == E - 1) {
+            p.offsets[E] = off;
+            p.ntiles[0] = p.ntiles[1] = til;
+        }
+    }
+    __syncthreads();
+    if (tid < P) {
+        const uint32_t e = sinds[tid];
+        uint32_t r = soff[e];
+        for (int j = 0; j < tid; j++) r += sinds[j] == e;
+        p.row_map[r] = (uint32_t)tid;
+        p.pos[tid] = r;
+    }
+}
+
+struct GateUpSmallParams {
+    const unsigned char *w[2], *s[2], *b[2];  // stacked gate and up
+    int32_t D, I, topk;
+    FixedRows x;               // the tokens
+    const uint32_t* row_map;
+    const Tile* tiles;
+    const uint32_t* ntiles;
+    const float* ebias[2];     // [E, I] or null
+    int32_t act;
+    float limit;
+    __half* h;                 // [P, I]
+    FixedRows fh;              // h as block fixed point
+};
+
+// Codes, scales and biases of two neighbouring groups of 64 inputs of weight rows g and g + 8 (a lane's share), straight from
+// global memory. Groups past the end read the last one again. even: the pair's scales are one aligned word.
+struct SmallBatch {
+    uint2 q[2][2];         // [group][row]
+    uint32_t s[2], b[2];   // [row]: two bf16
+};
+__device__ __forceinline__ void small_load(SmallBatch& v, const unsigned char* w, const unsigned char* s, const unsigned char* b, int64_t row,
+                                           int G, int g0, bool even, int t) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int64_t r = row + 8 * h;
+        const int ga = min(g0, G - 1), gb = min(g0 + 1, G - 1);
+        v.q[0][h] = __ldg(reinterpret_cast<const uint2*>(w + (r * G + ga) * 32 + t * 8));
+        v.q[1][h] = __ldg(reinterpret_cast<const uint2*>(w + (r * G + gb) * 32 + t * 8));
+        const uint16_t* sp = reinterpret_cast<const uint16_t*>(s) + r * G;
+        const uint16_t* bp = reinterpret_cast<const uint16_t*>(b) + r * G;
+        if (even) {
+            v.s[h] = __ldg(reinterpret_cast<const uint32_t*>(sp + ga));
+            v.b[h] = __ldg(reinterpret_cast<const uint32_t*>(bp + ga));
+        } else {
+            v.s[h] = (uint32_t)__ldg(sp + ga) | ((uint32_t)__ldg(sp + gb) << 16);
+            v.b[h] = (uint32_t)__ldg(bp + ga) | ((uint32_t)__ldg(bp + gb) << 16);
+        }
+    }
+}
+// One group of the batch against one set of four activation rows: xb the lane's digits, xs its row's {2^(e-13), sum}.
+__device__ __forceinline__ void small_mma(float (&acc)[2], const SmallBatch& v, int u, const uint4& xb, const float2& xs) {
+    constexpr uint32_t MSK = 0x0F0F0F0Fu;
+    const int z[4] = {0, 0, 0, 0};
+    int d[4];
+    const uint2 w0 = v.q[u][0], w1 = v.q[u][1];
+    imma16832_u8s8(d, w0.x & MSK, w1.x & MSK, (w0.x >> 4) & MSK, (w1.x >> 4) & MSK, xb.x, xb.y, z);
+    imma16832_u8s8(d, w0.y & MSK, w1.y & MSK, (w0.y >> 4) & MSK, (w1.y >> 4) & MSK, xb.z, xb.w, d);
+    const float v0 = (float)(d[0] * 128 + d[1]), v1 = (float)(d[2] * 128 + d[3]);
+    const float s0 = __uint_as_float(u ? (v.s[0] & 0xFFFF0000u) : (v.s[0] << 16)), s1 = __uint_as_float(u ? (v.s[1] & 0xFFFF0000u) : (v.s[1] << 16));
+    const float b0 = __uint_as_float(u ? (v.b[0] & 0xFFFF0000u) : (v.b[0] << 16)), b1 = __uint_as_float(u ? (v.b[1] & 0xFFFF0000u) : (v.b[1] << 16));
+    acc[0] = fmaf(v0, s0 * xs.x, acc[0]);
+    acc[0] = fmaf(b0, xs.y, acc[0]);
+    acc[1] = fmaf(v1, s1 * xs.x, acc[1]);
+    acc[1] = fmaf(b1, xs.y, acc[1]);
+}
+
+// A block's item: 64 features (gate and up) of one tile of up to eight rows; its sixteen warps are four blocks of 16 rows x
+// four slices of the inputs.
+__global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(const GateUpSmallParams p) {
+    constexpr int RS = 72;  // floats between activation rows of the slices' sums (the lanes of a store in different banks)
+    __shared__ float red[4][2][8][RS];
+    __shared__ float gmax[16], gsum[16];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int rb = warp & 3, ks = warp >> 2;
+    const int G = p.D / 64, NB = p.I / 64;
+    const int pairs = (G + 1) / 2, p0 = pairs * ks / 4, p1 = pairs * (ks + 1) / 4;  // this slice, in pairs of groups
+    const bool even = (G & 1) == 0;
+    pdl_wait();
+    pdl_launch_dependents();  // (after the wait: what the down kernel reads early is then complete)
+    const int total = (int)__ldcg(p.ntiles) * NB;
+    for (int it = blockIdx.x; it < total; it += gridDim.x) {
+        const uint4 tw = __ldcg(reinterpret_cast<const uint4*>(p.tiles) + it / NB);
+        const Tile tile = Tile{tw.x, tw.y, tw.z, tw.w};
+        const int n0 = (it % NB) * 64, M = (int)tile.count, sets = M > 4 ? 2 : 1;
+        const int64_t row = (int64_t)tile.expert * p.I + n0 + rb * 16 + g;
+        SmallBatch cur[2], nxt[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) small_load(cur[i], p.w[i], p.s[i], p.b[i], row, G, 2 * min(p0, pairs - 1), even, t);
+        // fragments: lane (g, t) holds digit g % 2 of row g / 2 of the set; scales: of row t of the set
+        const unsigned char* xd[2];
+        const float2* xs[2];
+        bool xl[2];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const int m = 4 * c + (g >> 1), ms = 4 * c + t;
+            xl[c] = m < M;
+            const uint32_t tok = __ldcg(p.row_map + tile.start + min(m, M - 1)) / (uint32_t)p.topk;
+            const uint32_t tks = __ldcg(p.row_map + tile.start + min(ms, M - 1)) / (uint32_t)p.topk;
+            xd[c] = p.x.digits + (size_t)tok * G * 128 + (g & 1) * 64 + t * 16;
+            xs[c] = p.x.scale + (size_t)tks * G;
+        }
+        float acc[2][2][2];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int c = 0; c < 2; c++) acc[i][c][0] = acc[i][c][1] = 0.f;
+        auto compute = [&](const SmallBatch (&v)[2], int pr) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int grp = 2 * pr + u;
+                if (grp >= G) break;
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    if (c >= sets) break;
+                    uint4 xb = *reinterpret_cast<const uint4*>(xd[c] + grp * 128);
+                    if (!xl[c]) xb = make_uint4(0, 0, 0, 0);
+                    const float2 sv = xs[c][grp];
+                    small_mma(acc[0][c], v[0], u, xb, sv);
+                    small_mma(acc[1][c], v[1], u, xb, sv);
+                }
+            }
+        };
+        int pr = p0;
+        for (; pr + 1 < p1; pr += 2) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) small_load(nxt[i], p.w[i], p.s[i], p.b[i], row, G, 2 * (pr + 1), even, t);
+            compute(cur, pr);
+#pragma unroll
+            for (int i = 0; i < 2; i++) small_load(cur[i], p.w[i], p.s[i], p.b[i], row, G, 2 * min(pr + 2, pairs - 1), even, t);
+            compute(nxt, pr + 1);
+        }
+        if (pr < p1) compute(cur, pr);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                red[ks][i][4 * c + t][rb * 16 + g] = acc[i][c][0];
+                red[ks][i][4 * c + t][rb * 16 + 8 + g] = acc[i][c][1];
+            }
+        __syncthreads();
+        // a thread per (feature, row): the slices in order, the activation, and the group of 64 features as block fixed point
+        const int f = tid & 63, m = tid >> 6;
+        float gv = 0.f, uv = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            gv += red[k][0][m][f];
+            uv += red[k][1][m][f];
+        }
+        if (p.ebias[0] != nullptr) {
+            gv += p.ebias[0][(size_t)tile.expert * p.I + n0 + f];
+            uv += p.ebias[1][(size_t)tile.expert * p.I + n0 + f];
+        }
+        const __half h16 = __float2half_rn(glu_rt(p.act, gv, uv, p.limit));
+        const float hv = m < M ? __half2float(h16) : 0.f;
+        float amax = fabsf(hv), sum = hv;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        }
+        if (lane == 0) { gmax[warp] = amax; gsum[warp] = sum; }
+        __syncthreads();  // (also: every sum of this item has been read)
+        if (m < M) {
+            const size_t pos = tile.start + m;
+            amax = fmaxf(gmax[warp & ~1], gmax[warp | 1]);
+            sum = gsum[warp & ~1] + gsum[warp | 1];
+            float sc, inv;
+            qi_group_scale(amax, sum, sc, inv);
+            const size_t rec = pos * NB + n0 / 64;
+            if (f == 0) p.fh.scale[rec] = make_float2(sc, sum);
+            const int X = __float2int_rn(hv * inv);
+            const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
+            unsigned char* d = p.fh.digits + rec * 128 + ((f >> 4) & 3) * 16 + ((f >> 3) & 1) * 8 + (f & 1) * 4 + ((f & 7) >> 1);
+            d[0] = (unsigned char)(hi_d & 0xFF);
+            d[64] = (unsigned char)(lo_d & 0xFF);
+            p.h[pos * p.I + n0 + f] = h16;
+        }
+    }
+}
+
+struct DownSmallParams {
+    const unsigned char *w, *s, *b;
+    int32_t D, I, topk, T;
+    FixedRows fh;
+    const uint32_t *inds, *pos;
+    const float* wts;
+    const float* ebias;        // [E, D] or null
+    __half* yd;                // [P, D]
+    void* out;
+    int32_t out_dtype;
+    int64_t ldo;
+    int32_t accumulate;
+    int32_t slices;            // of the inputs per pair: 16 warps / pairs
+};
+
+// A block's item: 16 features of one token; warp j * slices + k is slice k of the token's j-th expert.
+__global__ void __launch_bounds__(kSmallThreads, 1) moe_down_small_kernel(const DownSmallParams p) {
+    __shared__ float part[2][16][16];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int j = warp / p.slices, ks = warp % p.slices;
+    const int G = p.I / 64, NB = p.D / 16, total = p.T * NB;
+    const int pairs = (G + 1) / 2, p0 = pairs * ks / p.slices, p1 = pairs * (ks + 1) / p.slices;
+    const bool even = (G & 1) == 0, mine = j < p.topk;
+    pdl_launch_dependents();
+    // the routing was complete before the gate/up kernel let this one start (it is read past the L1 cache), and the weights
+    // depend on nothing else
+    auto row_of = [&](int it) {
+        return (int64_t)__ldcg(p.inds + (it / NB) * p.topk + (mine ? j : 0)) * p.D + (it % NB) * 16 + g;
+    };
+    SmallBatch cur, nxt;
+    int it = blockIdx.x;
+    int64_t row = it < total ? row_of(it) : 0;
+    if (it >= total) row = g;
+    small_load(cur, p.w, p.s, p.b, row, G, 2 * min(p0, pairs - 1), even, t);
+    pdl_wait();
+    for (int n = 0; it < total; it += gridDim.x, n++) {
+        const int tok = it / NB, next = it + gridDim.x;
+        const int64_t next_row = row_of(next < total ? next : it);
+        float acc[2] = {0.f, 0.f};
+        if (mine) {
+            const uint32_t pos = __ldcg(p.pos + tok * p.topk + j);
+            // one activation row: its high digits are column 0, the low ones column 1, the other columns zero
+            const unsigned char* hd = p.fh.digits + (size_t)pos * G * 128 + (g & 1) * 64 + t * 16;
+            const float2* hs = p.fh.scale + (size_t)pos * G;
+            auto compute = [&](const SmallBatch& v, int pr) {
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int grp = 2 * pr + u;
+                    if (grp >= G) break;
+                    uint4 xb = *reinterpret_cast<const uint4*>(hd + grp * 128);
+                    if (g > 1) xb = make_uint4(0, 0, 0, 0);
+                    small_mma(acc, v, u, xb, hs[grp]);
+                }
+            };
+            int pr = p0;
+            for (; pr + 1 < p1; pr += 2) {
+                small_load(nxt, p.w, p.s, p.b, row, G, 2 * (pr + 1), even, t);
+                compute(cur, pr);
+                const bool same = pr + 2 < p1;
+                small_load(cur, p.w, p.s, p.b, same ? row : next_row, G, 2 * (same ? pr + 2 : min(p0, pairs - 1)), even, t);
+                compute(nxt, pr + 1);
+            }
+            if (pr < p1) {
+                small_load(nxt, p.w, p.s, p.b, next_row, G, 2 * min(p0, pairs - 1), even, t);
+                compute(cur, pr);
+                cur = nxt;
+            }
+        }
+        row = next_row;
+        if (t == 0) {  // row 0 of the set
+            part[n & 1][warp][g] = acc[0];
+            part[n & 1][warp][g + 8] = acc[1];
+        }
+        __syncthreads();
+        if (tid < 16) {
+            const int d = (it % NB) * 16 + tid;
+            float sum = 0.f;
+            for (int k = 0; k < p.topk; k++) {
+                const uint32_t pos = __ldcg(p.pos + tok * p.topk + k);
+                float y = 0.f;
+                for (int q = 0; q < p.slices; q++) y += part[n & 1][k * p.slices + q][tid];
+                if (p.ebias != nullptr) y += p.ebias[(size_t)__ldcg(p.inds + tok * p.topk + k) * p.D + d];
+                const __half y16 = __float2half_rn(y);
+                p.yd[(size_t)pos * p.D + d] = y16;
+                sum = fmaf(__ldcg(p.wts + tok * p.topk + k), __half2float(y16), sum);
+            }
+            const size_t o = (size_t)tok * p.ldo + d;
+            if (p.out_dtype == kF32) {
+                float* op = reinterpret_cast<float*>(p.out) + o;
+                *op = p.accumulate ? sum + *op : sum;
+            } else if (p.out_dtype == kBF16) {
+                uint16_t* op = reinterpret_cast<uint16_t*>(p.out) + o;
+                *op = (uint16_t)f32_to_bf16_bits(p.accumulate ? bf16_bits_to_f32(*op) + sum : sum);
+            } else {
+                __half* op = reinterpret_cast<__half*>(p.out) + o;
+                *op = __float2half_rn(p.accumulate ? __half2float(*op) + sum : sum);
+            }
+        }
+    }
+}
+
+}  // namespace iq
