@@ -86,6 +86,7 @@ int32_t make_map_rowblock(iq_ctx* ctx, CUtensorMap* map, const void* base, uint6
 int32_t cached_rowblock_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, int32_t box_rows, CUtensorMap* out);
 
 struct Tile;
+struct FixedRows;
 // One launch of the gqmv family. mode: 0 plain, 1 gate/up, 2 down. `max_rows` bounds the rows of any tile (<= 16).
 // tiles == nullptr means a single tile of `rows` rows. grid_tiles = upper bound of the tile count for the launch.
 struct GqmvCall {
@@ -116,6 +117,7 @@ struct GqmvCall {
     const float* ebias[2] = {nullptr, nullptr};
     float limit = 0.f;
     int32_t act = 0;  // gate/up mode: activation (kAct*)
+    const FixedRows* fx = nullptr;  // grouped gate/up: the token rows as block fixed point, when the caller has them
 };
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
 

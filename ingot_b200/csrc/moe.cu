@@ -37,7 +37,7 @@ struct MoeWs {
     __half* h;
     void* yd;
     __half* xs;  // activations in expert order, fp16 [P, d_model] (tensor-core path)
-    FixedRows fx, fh;  // calls of few tokens: the activations and h as block fixed point
+    FixedRows fx, fh;  // the activations as block fixed point (up to kFixedTokens); h likewise (up to kSmallTokens)
     // shared expert (only when the layer has one): fp16 copy of x, h, output, per-token weight, tile list
     __half* s_x16;
     __half* s_h;
@@ -59,6 +59,7 @@ constexpr int kTensorPathRowsPerExpert = 24;
 constexpr int kBigTileRowsPerExpert = 96;
 constexpr int kRouterSmemMax = 200 * 1024;
 constexpr int kGroupChunkedMinPairs = 4096;  // from here on the permutation runs as a chunked counting sort
+constexpr int kFixedTokens = 512;  // calls that run on the decode tile kernels have at most this many (24 rows per expert)
 constexpr int kRouterTiledMinTokens = 64;  // above this the router runs as a tiled float64 GEMM
 
 // Expert outputs between the down projection and the combine: fp16 for affine experts, fp32 for MXFP4 ones, whose
@@ -89,9 +90,9 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     w.h = static_cast<__half*>(take(P * d.d_ff * 2));
     w.yd = take(P * d.d_model * (yd_dtype_of(l) == kF16 ? 2 : 4));
     w.xs = static_cast<__half*>(take(P * d.d_model * 2));
-    const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens;
-    w.fx.digits = static_cast<unsigned char*>(take(few * (d.d_model / 64) * 128));
-    w.fx.scale = static_cast<float2*>(take(few * (d.d_model / 64) * 8));
+    const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens, fixed = tokens < kFixedTokens ? tokens : kFixedTokens;
+    w.fx.digits = static_cast<unsigned char*>(take(fixed * (d.d_model / 64) * 128));
+    w.fx.scale = static_cast<float2*>(take(fixed * (d.d_model / 64) * 8));
     w.fh.digits = static_cast<unsigned char*>(take(few * d.top_k * (d.d_ff / 64) * 128));
     w.fh.scale = static_cast<float2*>(take(few * d.top_k * (d.d_ff / 64) * 8));
     w.s_x16 = nullptr; w.s_h = nullptr; w.s_yd = nullptr; w.s_w = nullptr; w.s_tiles = nullptr; w.s_ntiles = nullptr;
@@ -170,14 +171,15 @@ int32_t launch_route(iq_moe* l, cudaStream_t st, const float* logits, int ld, in
     rp.x = static_cast<const uint16_t*>(refine_x);
     rp.ldx = ldx;
     const bool wide = refine_x != nullptr && tokens <= kRouteWideMaxTokens;
-    route_kernel_for(l->d.experts, refine_x != nullptr, wide)<<<wide ? tokens : (tokens + 3) / 4, 128, 0, st>>>(rp);
-    return check_cuda(l->ctx, cudaGetLastError(), "route_topk launch");
+    return check_cuda(l->ctx, launch_dependent(route_kernel_for(l->d.experts, refine_x != nullptr, wide), dim3(wide ? tokens : (tokens + 3) / 4), 128, 0, st, rp),
+                      "route_topk launch");
 }
 
 // Gate + up + activation of every tile: h[row, :] = half(act(x W_gate^T + b_g, x W_up^T + b_u)). Expert e's weights live
 // at local slot e - expert_lo: the offset is folded into the base pointers. row_map == nullptr: x rows are in place.
 int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, int64_t ldx, const uint32_t* row_map,
-                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, int bm, __half* h, int row_map_div = 0) {
+                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, int bm, __half* h, int row_map_div = 0,
+                   const FixedRows* fx = nullptr) {
     const iq_moe_desc& d = l->d;
     const int64_t lo = d.expert_lo;
     GqmvCall c;
@@ -207,6 +209,7 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
     }
     c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
     c.act = d.act;
+    c.fx = fx;
     return launch_gqmv(l->ctx, cs, c);
 }
 
@@ -277,6 +280,13 @@ int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows,
 }
 
 // ---- few tokens (csrc/moe_small.cuh) ----
+int router_tokens(int tokens) { return tokens <= 1 ? 1 : tokens <= 2 ? 2 : tokens <= 4 ? 4 : 8; }
+typedef void (*RouterKernel)(const RouterIn, float*, int, int, int, int);
+template <int WFMT>
+RouterKernel router_kernel_of(int tt) {
+    return tt == 1 ? router_logits_kernel<WFMT, 1> : tt == 2 ? router_logits_kernel<WFMT, 2> : tt == 4 ? router_logits_kernel<WFMT, 4> : router_logits_kernel<WFMT, 8>;
+}
+RouterKernel router_kernel_pick(bool q8, int tt) { return q8 ? router_kernel_of<1>(tt) : router_kernel_of<0>(tt); }
 typedef void (*RouteSmallKernel)(const RouteSmallParams);
 template <int WFMT, int TT>
 RouteSmallKernel route_small_vpl(int experts) {
@@ -292,10 +302,9 @@ constexpr size_t kRouteSmallSmemMax = 200 * 1024;
 
 // Router, top-k and permutation in one cluster: up to eight tokens, while the float64 products of a block (a cluster has
 // eight) stay at a few microseconds and the tokens fit its shared memory. 128 experts x 2048 inputs: all eight tokens.
-int route_small_tokens(int tokens) { return tokens <= 1 ? 1 : tokens <= 2 ? 2 : tokens <= 4 ? 4 : 8; }
 bool use_route_small(const iq_moe* l, int tokens) {
     const iq_moe_desc& d = l->d;
-    const int tt = route_small_tokens(tokens);
+    const int tt = router_tokens(tokens);
     return tokens <= kSmallTokens && l->ext_inds == nullptr && d.expert_lo == 0 && d.expert_count == d.experts &&
            (int64_t)d.experts * d.d_model * tt <= (1 << 21) && route_small_smem(tt, d.d_model, d.experts) <= kRouteSmallSmemMax;
 }
@@ -312,12 +321,11 @@ int32_t run_route_small(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dty
     const iq_moe_desc& d = l->d;
     RouteSmallParams p;
     p.r = route_params(l, w.logits, l->ld, tokens, w.inds, w.wts);
-    p.x = x; p.x_dtype = x_dtype; p.ldx = ldx;
-    p.wr = d.router_w; p.ws = d.router_scales; p.wb = d.router_biases;
+    p.in = RouterIn{x, x_dtype, ldx, d.router_w, d.router_scales, d.router_biases, d.d_model};
     p.counts = w.counts; p.offsets = w.offsets; p.row_map = w.row_map; p.pos = w.pos; p.ntiles = w.ntiles;
     p.tiles_a = w.tiles_a; p.tiles_b = w.tiles_b;
     p.fx = fixed ? w.fx : FixedRows{nullptr, nullptr};
-    const int tt = route_small_tokens(tokens);
+    const int tt = router_tokens(tokens);
     return check_cuda(l->ctx, launch_dependent(route_small_pick(d.router_kind != IQ_ROUTER_BF16, tt, d.experts), dim3(kSmallCluster), kSmallThreads,
                                                route_small_smem(tt, d.d_model, d.experts), cs, p), "moe_route_small launch");
 }
@@ -443,10 +451,9 @@ int32_t moe_init(iq_ctx* ctx) {
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)router_tiled_smem(64));
     cudaFuncSetAttribute(reinterpret_cast<const void*>(router_logits_tiled_kernel<1, 64>),
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)router_tiled_smem(64));
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(router_logits_kernel<0>),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kRouterSmemMax);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(router_logits_kernel<1>),
+    cudaError_t e = cudaSuccess;
+    for (int v = 0; v < 8 && e == cudaSuccess; v++)
+        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(router_kernel_pick(v & 1, 1 << (v >> 1))),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kRouterSmemMax);
     for (int v = 0; v < 16 && e == cudaSuccess; v++)
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(route_small_pick(v & 1, 1 << (v >> 1 & 3), v >> 3 ? 256 : 32)),
@@ -791,21 +798,17 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
                             "router_logits_tiled launch");
             if (st != kOk) return st;
         } else {
-        // experts per block: small ranges for few tokens (more blocks, shorter dot products per thread)
-        int eb = d.experts < 256 ? d.experts : 256;
-        if (tokens <= 64) eb = 8;  // a decode batch: 256 blocks of 8 experts x 32 K slices fill the GPU (20 -> 10 us at 64 tokens)
-        else if (tokens <= 256 && eb > 32) eb = 32;
-        while (d.experts % eb != 0) eb /= 2;
-        const size_t smem = (size_t)kRouterTT * d.d_model * 8 + (size_t)256 * kRouterTT * 8;
+        // eight experts per block (fewer where that leaves the GPU empty) and as many tokens as fit shared memory
+        int tt = router_tokens(tokens);
+        while (tt > 1 && router_block_smem(tt, d.d_model, 8) > (size_t)kRouterSmemMax) tt /= 2;
+        const int groups = (tokens + tt - 1) / tt;
+        const int epc = d.experts / 8 * groups * 2 <= ctx->sms ? 4 : 8;
+        const size_t smem = router_block_smem(tt, d.d_model, epc);
         if (smem > (size_t)kRouterSmemMax) return fail(ctx, kErrUnsupported, "moe: d_model = %d is too wide for the router kernel", d.d_model);
-        const dim3 grid((tokens + kRouterTT - 1) / kRouterTT, d.experts / eb);
-        if (d.router_kind == IQ_ROUTER_BF16)
-            router_logits_kernel<0><<<grid, 256, smem, cs>>>(x, x_dtype, ldx, d.router_w, nullptr, nullptr, w.logits,
-                                                              tokens, d.experts, d.d_model, l->ld, eb);
-        else
-            router_logits_kernel<1><<<grid, 256, smem, cs>>>(x, x_dtype, ldx, d.router_w, d.router_scales,
-                                                              d.router_biases, w.logits, tokens, d.experts, d.d_model,
-                                                              l->ld, eb);
+        const RouterIn in = {x, x_dtype, ldx, d.router_w, d.router_scales, d.router_biases, d.d_model};
+        st = check_cuda(ctx, launch_dependent(router_kernel_pick(d.router_kind != IQ_ROUTER_BF16, tt), dim3(groups, d.experts / epc), kRouterThreads, smem, cs,
+                                              in, w.logits, tokens, d.experts, l->ld, epc), "router_logits launch");
+        if (st != kOk) return st;
         }
         st = check_cuda(ctx, cudaGetLastError(), "router_logits launch");
         if (st != kOk) return st;
@@ -816,6 +819,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st != kOk) return st;
     }
     const int bm = decode_tile_rows(l, tokens);
+    // whole calls on the decode tile kernels: the counting kernel leaves the activations as fixed point for the gate/up one
+    const bool fixed = (pieces & (IQ_PIECE_GROUP | IQ_PIECE_GATEUP)) == (IQ_PIECE_GROUP | IQ_PIECE_GATEUP) && l->fmt == kFmtAffine4 &&
+                       tokens <= kFixedTokens && P < kGroupChunkedMinPairs && !use_tensor_path(P, d.expert_count) && bm == 8;
     if (pieces & IQ_PIECE_GROUP) {
         GroupParams gp;
         gp.inds = inds; gp.counts = w.counts; gp.offsets = w.offsets; gp.row_map = w.row_map; gp.pos = w.pos;
@@ -824,16 +830,20 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         gp.e_lo = d.expert_lo; gp.e_hi = d.expert_lo + d.expert_count;
         gp.chunk_hist = w.chunk_hist;
         gp.chunks = (P + kGroupChunk - 1) / kGroupChunk;
+        gp.fx = FixedRows{nullptr, nullptr};
+        st = kOk;
         if (P >= kGroupChunkedMinPairs && d.experts * 8 * 4 <= 48 * 1024) {
             // many pairs: a chunked counting sort touches each pair once per kernel instead of once per expert
             moe_hist_kernel<<<gp.chunks, 256, d.experts * 4, cs>>>(gp);
             moe_scan_kernel<<<1, 256, 0, cs>>>(gp);
             moe_place_kernel<<<gp.chunks, 256, d.experts * 8 * 4, cs>>>(gp);
         } else {
-            moe_count_kernel<<<d.experts, 256, 0, cs>>>(gp);
-            moe_scatter_kernel<<<d.experts, 256, 0, cs>>>(gp);
+            if (fixed) { gp.fx = w.fx; gp.x = x; gp.x_dtype = x_dtype; gp.ldx = ldx; gp.T = tokens; gp.D = d.d_model; }
+            st = check_cuda(ctx, launch_dependent(moe_count_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_count launch");
+            if (st != kOk) return st;
+            st = check_cuda(ctx, launch_dependent(moe_scatter_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_scatter launch");
         }
-        st = check_cuda(ctx, cudaGetLastError(), "moe_group launch");
+        if (st == kOk) st = check_cuda(ctx, cudaGetLastError(), "moe_group launch");
         if (st != kOk) return st;
     }
     const int64_t max_tiles64 = (int64_t)d.expert_count + P / bm;
@@ -847,7 +857,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
             st = check_cuda(ctx, cudaGetLastError(), "moe_pack_tokens launch");
             if (st == kOk) st = run_gateup_tc(l, cs, w.xs, P, w.tiles_b, w.ntiles + 1, w.h, tensor_tile_rows(P, d.expert_count));
         } else {
-            st = run_gateup(l, cs, x, x_dtype, ldx, w.row_map, w.tiles_a, w.ntiles, max_tiles, bm, w.h);
+            st = run_gateup(l, cs, x, x_dtype, ldx, w.row_map, w.tiles_a, w.ntiles, max_tiles, bm, w.h, 0, fixed ? &w.fx : nullptr);
         }
         if (st != kOk) return st;
     }
@@ -862,8 +872,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         cp.out = out; cp.out_dtype = out_dtype; cp.ldo = ldo;
         cp.T = tokens; cp.D = d.d_model; cp.topk = d.top_k;
         cp.accumulate = (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0;
-        moe_combine_kernel<<<tokens, 256, 0, cs>>>(cp);
-        st = check_cuda(ctx, cudaGetLastError(), "moe_combine launch");
+        st = check_cuda(ctx, launch_dependent(moe_combine_kernel, dim3(tokens), 256, 0, cs, cp), "moe_combine launch");
         if (st != kOk) return st;
         if (d.shared != IQ_SHARED_NONE) {
             st = run_shared_expert(l, cs, x, x_dtype, ldx, tokens, w, out, out_dtype, ldo);

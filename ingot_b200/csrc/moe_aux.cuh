@@ -8,6 +8,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fixed_rows.cuh"
 #include "gqmv.cuh"
 #include "ptx.cuh"
 
@@ -21,108 +22,142 @@ namespace iq {
 // size or the number of GPUs. Columns E..ld-1 of the output are written as zero (the reference pads the router to a
 // multiple of 64 rows, MoE.swift:258-273).
 //
-// Block: TT tokens (x staged in shared memory as doubles), thread = (expert, k-slice).
-constexpr int kRouterTT = 4;
+// Few tokens: a block of sixteen warps takes TT tokens (inputs converted to float64 once, in shared memory) and epc experts;
+// a warp takes four experts and one of NQ slices of the inputs, so that an input read from shared memory feeds four
+// products, and the next weights are on their way while the current ones are used.
+constexpr int kRouterThreads = 512;
+__host__ __device__ constexpr int router_slices(int epc) { return epc >= 64 ? 1 : 16 / (epc / 4); }
+__host__ __device__ constexpr size_t router_block_smem(int tt, int D, int epc) {
+    return (size_t)tt * D * 8 + (size_t)router_slices(epc) * epc * tt * 8;
+}
 
-template <int WFMT>  // 0: bf16 dense router; 1: 8-bit affine g64 router
-__global__ void __launch_bounds__(256) router_logits_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx,
-                                                            const void* __restrict__ wr, const void* __restrict__ ws,
-                                                            const void* __restrict__ wb, float* __restrict__ logits,
-                                                            int T, int E, int D, int ld, int eb) {
-    // eb: experts per block (a power of two, at most 256); blockIdx.y picks the expert range. Few tokens take small
-    // ranges so that the dot products spread over many blocks and K slices.
-    extern __shared__ __align__(16) unsigned char smem[];
-    double* xs = reinterpret_cast<double*>(smem);                      // [TT][D]
-    double* part = xs + (size_t)kRouterTT * D;                         // [slices][TT][ee]
-    const int tid = threadIdx.x;
-    const int t0 = blockIdx.x * kRouterTT;
-    const int nt = min(kRouterTT, T - t0);
-    const int ee = eb;                          // experts handled by this block
-    const int slices = 256 / ee;                // k-slices per expert
-    for (int i = tid; i < kRouterTT * D / 8; i += 256) {
-        const int tt = i / (D / 8), ku = i % (D / 8);
-        float v[8];
-        if (tt < nt) load_x8(x, x_dtype, (size_t)(t0 + tt) * ldx + ku * 8, v);
-        else {
+struct RouterIn {
+    const void* x;
+    int32_t x_dtype;
+    int64_t ldx;
+    const void* wr;  // bf16 [E, D], or 8-bit codes with scales and biases
+    const void* ws;
+    const void* wb;
+    int32_t D;
+};
+
+// Experts e0 .. e0 + epc - 1, tokens t0 .. t0 + T - 1 (T <= TT): done(e, t, logit) for every pair, by one thread each, after a
+// block barrier. xs: [TT][4][units] pairs of inputs, part: [NQ][epc][TT].
+template <int WFMT, int TT, class Done>
+__device__ __forceinline__ void router_block(const RouterIn& p, double2* xs, double* part, int t0, int T, int e0, int epc, Done done) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int D = p.D, units = D / 8, NQ = router_slices(epc), jobs = epc / 4 * NQ, uq = (units + NQ - 1) / NQ;
+    // one unit of eight router weights of four experts: bf16 words, or codes with scale and bias
+    auto fetch = [&](uint4 (&w)[4], int job, int u) {
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = 0.f;
+        for (int i = 0; i < 4; i++) {
+            const size_t e = e0 + job / NQ * 4 + i;
+            if (WFMT == 0) {
+                w[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.wr) + e * D) + u);
+            } else {
+                const uint2 q = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint32_t*>(p.wr) + e * (D / 4)) + u);
+                const size_t gi = e * (D / 64) + u / 8;
+                w[i] = make_uint4(q.x, q.y, __ldg(reinterpret_cast<const uint16_t*>(p.ws) + gi), __ldg(reinterpret_cast<const uint16_t*>(p.wb) + gi));
+            }
         }
+    };
+    uint4 w[4], wn[4];
+    fetch(w, warp < jobs ? warp : 0, min(warp % NQ * uq + lane, units - 1));  // the router does not depend on the previous kernel
+    pdl_wait();
+    for (int i = tid; i < TT * units; i += kRouterThreads) {
+        const int t = i / units, u = i % units;
+        float v[8];
+        load_x8(p.x, p.x_dtype, (size_t)(t0 + min(t, T - 1)) * p.ldx + u * 8, v);
 #pragma unroll
-        for (int e = 0; e < 8; e++) xs[(size_t)tt * D + ku * 8 + e] = (double)v[e];
+        for (int j = 0; j < 4; j++) xs[(t * 4 + j) * units + u] = make_double2((double)v[2 * j], (double)v[2 * j + 1]);
     }
     __syncthreads();
-    const int el = tid % ee, sl = tid / ee;
-    const int units = D / 8;                                  // 8-input units per row
-    const int upw = (units + slices - 1) / slices;            // units per slice
-    {
-        const int e = blockIdx.y * ee + el;
-        double acc[kRouterTT];
+    for (int job = warp; job < jobs; job += kRouterThreads / 32) {
+        const int kq = job % NQ;
+        double acc[4 * TT];
 #pragma unroll
-        for (int tt = 0; tt < kRouterTT; tt++) acc[tt] = 0.0;
-        if (e < E && sl < slices) {
-            for (int u = sl * upw; u < min(units, (sl + 1) * upw); u++) {
-                double w[8];
-                if (WFMT == 0) {
-                    const uint4 r = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(wr) +
-                                                                    (size_t)e * D + u * 8);
-                    const uint32_t q[4] = {r.x, r.y, r.z, r.w};
+        for (int i = 0; i < 4 * TT; i++) acc[i] = 0.0;
+        const int u_end = min(units, (kq + 1) * uq);
+        int u = kq * uq + lane;
+        if (job != warp && u < u_end) fetch(w, job, u);
+        for (; u < u_end; u += 32) {
+            fetch(wn, job, min(u + 32, units - 1));
+            float sc[4], bi[4];
+            if (WFMT == 1) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        w[2 * j] = (double)__uint_as_float(q[j] << 16);
-                        w[2 * j + 1] = (double)__uint_as_float(q[j] & 0xFFFF0000u);
-                    }
-                } else {
-                    const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint32_t*>(wr) +
-                                                                    (size_t)e * (D / 4) + u * 2);
-                    const int gi = e * (D / 64) + u / 8;
-                    // the weight value is the fp32 s*q + b of the reference's CPU dequantisation
-                    const float sc = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(ws)[gi]);
-                    const float bi = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(wb)[gi]);
+                for (int i = 0; i < 4; i++) { sc[i] = bf16_bits_to_f32(w[i].z); bi[i] = bf16_bits_to_f32(w[i].w); }
+            }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        w[j] = (double)__fadd_rn(__fmul_rn(sc, (float)((r.x >> (8 * j)) & 0xFFu)), bi);
-                        w[4 + j] = (double)__fadd_rn(__fmul_rn(sc, (float)((r.y >> (8 * j)) & 0xFFu)), bi);
+            for (int j = 0; j < 4; j++) {
+                double wd[4][2];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (WFMT == 0) {
+                        const uint32_t q = j == 0 ? w[i].x : (j == 1 ? w[i].y : (j == 2 ? w[i].z : w[i].w));
+                        wd[i][0] = (double)__uint_as_float(q << 16);
+                        wd[i][1] = (double)__uint_as_float(q & 0xFFFF0000u);
+                    } else {  // the fp32 s*q + b of the reference's CPU dequantisation
+                        const uint32_t q = (j < 2 ? w[i].x : w[i].y) >> (16 * (j & 1));
+                        wd[i][0] = (double)__fadd_rn(__fmul_rn(sc[i], (float)(q & 0xFFu)), bi[i]);
+                        wd[i][1] = (double)__fadd_rn(__fmul_rn(sc[i], (float)((q >> 8) & 0xFFu)), bi[i]);
                     }
                 }
 #pragma unroll
-                for (int tt = 0; tt < kRouterTT; tt++) {
-                    if (tt >= nt) break;
-                    const double2* xp = reinterpret_cast<const double2*>(xs + (size_t)tt * D + u * 8);
+                for (int t = 0; t < TT; t++) {
+                    const double2 xv = xs[(t * 4 + j) * units + u];
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const double2 xv = xp[j];
-                        acc[tt] = fma(xv.x, w[2 * j], acc[tt]);
-                        acc[tt] = fma(xv.y, w[2 * j + 1], acc[tt]);
+                    for (int i = 0; i < 4; i++) {
+                        acc[i * TT + t] = fma(xv.x, wd[i][0], acc[i * TT + t]);
+                        acc[i * TT + t] = fma(xv.y, wd[i][1], acc[i * TT + t]);
                     }
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = wn[i];
         }
-        if (slices > 1) {
-            __syncthreads();
+        // the lanes' sums: while there are several values left, a lane keeps half of them and hands over the other half
+        int n = 4 * TT, idx = 0, dup = 0;
 #pragma unroll
-            for (int tt = 0; tt < kRouterTT; tt++) part[((size_t)sl * kRouterTT + tt) * ee + el] = acc[tt];
-            __syncthreads();
-            if (sl == 0) {
+        for (int o = 16; o > 0; o >>= 1) {
+            if (n > 1) {
+                const int half = n / 2;
+                const bool up = lane & o;
 #pragma unroll
-                for (int tt = 0; tt < kRouterTT; tt++) {
-                    double s = 0.0;
-                    for (int k = 0; k < slices; k++) s += part[((size_t)k * kRouterTT + tt) * ee + el];
-                    acc[tt] = s;
+                for (int i = 0; i < 2 * TT; i++) {
+                    if (i >= half) break;
+                    const double send = up ? acc[i] : acc[i + half], keep = up ? acc[i + half] : acc[i];
+                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
                 }
+                if (up) idx += half;
+                n = half;
+            } else {
+                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+                dup |= lane & o;
             }
         }
-        if (sl == 0 && e < E) {
-#pragma unroll
-            for (int tt = 0; tt < kRouterTT; tt++)
-                if (tt < nt) logits[(size_t)(t0 + tt) * ld + e] = (float)acc[tt];
-        }
+        if (dup == 0) part[(kq * epc + job / NQ * 4 + idx / TT) * TT + idx % TT] = acc[0];
     }
-    if (blockIdx.y == 0) {
-        for (int i = tid; i < kRouterTT * (ld - E); i += 256) {
-            const int tt = i / (ld - E), c = E + i % (ld - E);
-            if (tt < nt) logits[(size_t)(t0 + tt) * ld + c] = 0.f;
-        }
+    __syncthreads();
+    for (int i = tid; i < epc * TT; i += kRouterThreads) {
+        const int e = i / TT, t = i % TT;
+        double s = 0.0;
+        for (int k = 0; k < NQ; k++) s += part[(k * epc + e) * TT + t];
+        if (t < T) done(e0 + e, t0 + t, (float)s);
     }
+}
+
+// Grid (token groups, expert groups of epc).
+template <int WFMT, int TT>
+__global__ void __launch_bounds__(kRouterThreads, 1) router_logits_kernel(const RouterIn p, float* __restrict__ logits, int T, int E, int ld, int epc) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    double2* xs = reinterpret_cast<double2*>(smem);
+    double* part = reinterpret_cast<double*>(smem + (size_t)TT * p.D * 8);
+    const int t0 = blockIdx.x * TT;
+    pdl_launch_dependents();
+    router_block<WFMT, TT>(p, xs, part, t0, min(TT, T - t0), blockIdx.y * epc, epc, [&](int e, int t, float f) { logits[(size_t)t * ld + e] = f; });
+    if (blockIdx.y == 0)
+        for (int i = threadIdx.x; i < TT * (ld - E); i += kRouterThreads)
+            if (t0 + i / (ld - E) < T) logits[(size_t)(t0 + i / (ld - E)) * ld + E + i % (ld - E)] = 0.f;
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -405,6 +440,8 @@ __device__ __forceinline__ uint32_t route_select(const float (&v)[VPL], const fl
 template <int VPL, bool REFINE = false, int WPT = 1>
 __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = WPT == 1 ? blockIdx.x * 4 + wib : blockIdx.x;
     if (t >= p.T) return;  // WPT = 4: the whole block leaves
     __shared__ float sx[WPT > 1 ? VPL * 32 : 1];  // WPT = 4: exact logits of the candidates
@@ -529,11 +566,21 @@ struct GroupParams {
     int32_t e_lo, e_hi;     // experts owned here (expert parallel); tiles are emitted only for these
     uint32_t* chunk_hist;   // [chunks, E] scratch of the chunked form (many pairs)
     int32_t chunks;
+    // the counting kernel also turns the activations into fixed point for the decode kernels (fx.digits null: it does not)
+    FixedRows fx;
+    const void* x;
+    int32_t x_dtype;
+    int64_t ldx;
+    int32_t T, D;
 };
 
 __global__ void __launch_bounds__(256) moe_count_kernel(const GroupParams p) {
     __shared__ uint32_t wsum[8];
     const uint32_t e = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (p.fx.digits != nullptr)
+        for (int t = blockIdx.x; t < p.T; t += gridDim.x) fixed_point_row(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
     uint32_t c = 0;
     for (int i = threadIdx.x; i < p.P; i += 256) c += p.inds[i] == e;
 #pragma unroll
@@ -550,6 +597,8 @@ __global__ void __launch_bounds__(256) moe_count_kernel(const GroupParams p) {
 __global__ void __launch_bounds__(256) moe_scatter_kernel(const GroupParams p) {
     __shared__ uint32_t sh[3][8];
     __shared__ uint32_t base[4];
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t e = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // exclusive prefixes over the experts before this one: pairs, tiles of height a, tiles of height b
@@ -741,6 +790,8 @@ struct CombineParams {
 
 __global__ void __launch_bounds__(256) moe_combine_kernel(const CombineParams p) {
     const int t = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ uint32_t spos[32];
     __shared__ float sw[32];
     if (threadIdx.x < p.topk) {

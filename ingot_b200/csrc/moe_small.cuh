@@ -14,6 +14,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fixed_rows.cuh"
 #include "gqmv.cuh"
 #include "moe_aux.cuh"
 #include "ptx.cuh"
@@ -25,200 +26,45 @@ constexpr int kSmallTokens = 8;
 constexpr int kSmallThreads = 512;
 constexpr int kSmallCluster = 8;
 
-// Row r of an activation matrix as block fixed point: per group of 64 inputs 128 bytes, the high digits' fragments of the
-// four lanes of a quad (16 bytes each: two MMAs) and the low digits', and {2^(e-13), sum}.
-struct FixedRows {
-    unsigned char* digits;  // [rows][groups][2][4][16]
-    float2* scale;          // [rows][groups]
-};
-
-// Eight consecutive inputs (word w8 of the group's eight) of a row's group: the eight threads of a group are eight
-// neighbouring lanes. See qmv_imma.cuh for the arithmetic.
-__device__ __forceinline__ void fixed_point_unit(const float (&v)[8], int w8, unsigned char* digits, float2* scale) {
-    float amax = 0.f, sum = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        amax = fmaxf(amax, fabsf(v[k]));
-        sum += v[k];
-    }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    }
-    float sc, inv;
-    qi_group_scale(amax, sum, sc, inv);
-    if (digits == nullptr) return;
-    if (w8 == 0) *scale = make_float2(sc, sum);
-    uint32_t hi_w[2] = {0, 0}, lo_w[2] = {0, 0};
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int X = __float2int_rn(v[k] * inv);
-        const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
-        hi_w[k & 1] |= (uint32_t)(hi_d & 0xFF) << (8 * (k >> 1));
-        lo_w[k & 1] |= (uint32_t)(lo_d & 0xFF) << (8 * (k >> 1));
-    }
-    unsigned char* f = digits + (w8 >> 1) * 16 + (w8 & 1) * 8;
-    *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
-    *reinterpret_cast<uint2*>(f + 64) = make_uint2(lo_w[0], lo_w[1]);
-}
-
 struct RouteSmallParams {
     RouteParams r;               // logits_rw, inds, wts, T, E, ld, topk, D and the scoring rule
-    const void* x;
-    int32_t x_dtype;
-    int64_t ldx;
-    const void* wr;
-    const void* ws;              // 8-bit router: scales and biases
-    const void* wb;
+    RouterIn in;
     uint32_t *counts, *offsets, *row_map, *pos, *ntiles;
     Tile *tiles_a, *tiles_b;
     FixedRows fx;                // the activations as block fixed point, or null
 };
 constexpr size_t route_small_smem(int tt, int D, int E) {
-    return (size_t)tt * D * 8 + (size_t)4 * (E / kSmallCluster) * tt * 8 + (size_t)tt * E * 4 + 16 * kSmallTokens * 4 + 64 * 4;
+    return router_block_smem(tt, D, E / kSmallCluster) + (size_t)tt * E * 4 + 16 * kSmallTokens * 4 + 64 * 4 + (size_t)E * 4;
 }
 
 // WFMT: 0 bf16 router, 1 8-bit affine. TT: tokens rounded up to 1, 2, 4, 8. VPL: experts per lane of the selection.
-// A block of the cluster takes E / 8 experts; its sixteen warps are (four experts, a quarter of the inputs) each, products
-// and sums in float64 (exact at fp32 resolution: the logits are the other router kernels' bits). The logits meet in the
+// A block of the cluster takes E / 8 experts (router_block: the other router kernels' bits). The logits meet in the
 // first block's shared memory, which then selects (a warp per token) and groups.
 template <int WFMT, int TT, int VPL>
 __global__ void __launch_bounds__(kSmallThreads, 1) __cluster_dims__(kSmallCluster, 1, 1) moe_route_small_kernel(const RouteSmallParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int T = p.r.T, E = p.r.E, D = p.r.D, topk = p.r.topk, units = D / 8, epc = E / kSmallCluster;
-    double2* xs = reinterpret_cast<double2*>(smem);                               // [TT][4][units]: inputs 2j, 2j + 1 of a unit
-    double* part = reinterpret_cast<double*>(smem + (size_t)TT * D * 8);          // [4][epc][TT]
-    float* lg = reinterpret_cast<float*>(part + (size_t)4 * epc * TT);            // [TT][E], the first block's
-    uint32_t* sinds = reinterpret_cast<uint32_t*>(lg + (size_t)TT * E);           // [16 * 8]
-    uint32_t* wsum = sinds + 16 * kSmallTokens;                                   // [2][32]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x, e0 = rank * epc;
+    const int T = p.r.T, E = p.r.E, D = p.r.D, topk = p.r.topk, epc = E / kSmallCluster;
+    double2* xs = reinterpret_cast<double2*>(smem);
+    double* part = reinterpret_cast<double*>(smem + (size_t)TT * D * 8);
+    float* lg = reinterpret_cast<float*>(part + (size_t)router_slices(epc) * epc * TT);  // [TT][E], the first block's
+    uint32_t* sinds = reinterpret_cast<uint32_t*>(lg + (size_t)TT * E);                  // [16 * 8]
+    uint32_t* wsum = sinds + 16 * kSmallTokens;                                          // [2][32]
+    uint32_t* soff = wsum + 64;                                                          // [E] exclusive offsets
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x;
     pdl_launch_dependents();
-
-    // one unit of eight router weights of four experts: bf16 words, or codes with scale and bias
-    auto fetch = [&](uint4 (&w)[4], int pr, int u) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const size_t e = e0 + (pr >> 2) * 4 + i;
-            if (WFMT == 0) {
-                w[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.wr) + e * D) + u);
-            } else {
-                const uint2 q = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint32_t*>(p.wr) + e * (D / 4)) + u);
-                const size_t gi = e * (D / 64) + u / 8;
-                w[i] = make_uint4(q.x, q.y, __ldg(reinterpret_cast<const uint16_t*>(p.ws) + gi), __ldg(reinterpret_cast<const uint16_t*>(p.wb) + gi));
-            }
-        }
-    };
-    const int uq = (units + 3) / 4;  // units per quarter of the inputs
-    uint4 w[4], wn[4];
-    {
-        const int u0 = (warp & 3) * uq + lane;  // the router does not depend on the previous kernel
-        fetch(w, warp < epc ? warp : 0, min(u0, units - 1));
-    }
-    pdl_wait();
-    for (int i = tid; i < TT * units; i += kSmallThreads) {
-        const int t = i / units, u = i % units;
-        float v[8];
-        if (t < T) load_x8(p.x, p.x_dtype, (size_t)t * p.ldx + u * 8, v);
-        else {
-#pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) xs[(t * 4 + j) * units + u] = make_double2((double)v[2 * j], (double)v[2 * j + 1]);
-    }
-    __syncthreads();
-    for (int pr = warp; pr < epc; pr += kSmallThreads / 32) {
-        double acc[4 * TT];
-#pragma unroll
-        for (int i = 0; i < 4 * TT; i++) acc[i] = 0.0;
-        const int u_end = min(units, ((pr & 3) + 1) * uq);
-        int u = (pr & 3) * uq + lane;
-        if (pr != warp && u < u_end) fetch(w, pr, u);
-        for (; u < u_end; u += 32) {
-            fetch(wn, pr, min(u + 32, units - 1));
-            float sc[4], bi[4];
-            if (WFMT == 1) {
-#pragma unroll
-                for (int i = 0; i < 4; i++) { sc[i] = bf16_bits_to_f32(w[i].z); bi[i] = bf16_bits_to_f32(w[i].w); }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                double wd[4][2];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (WFMT == 0) {
-                        const uint32_t q = j == 0 ? w[i].x : (j == 1 ? w[i].y : (j == 2 ? w[i].z : w[i].w));
-                        wd[i][0] = (double)__uint_as_float(q << 16);
-                        wd[i][1] = (double)__uint_as_float(q & 0xFFFF0000u);
-                    } else {  // the fp32 s*q + b of the reference's CPU dequantisation
-                        const uint32_t q = (j < 2 ? w[i].x : w[i].y) >> (16 * (j & 1));
-                        wd[i][0] = (double)__fadd_rn(__fmul_rn(sc[i], (float)(q & 0xFFu)), bi[i]);
-                        wd[i][1] = (double)__fadd_rn(__fmul_rn(sc[i], (float)((q >> 8) & 0xFFu)), bi[i]);
-                    }
-                }
-#pragma unroll
-                for (int t = 0; t < TT; t++) {
-                    const double2 xv = xs[(t * 4 + j) * units + u];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        acc[i * TT + t] = fma(xv.x, wd[i][0], acc[i * TT + t]);
-                        acc[i * TT + t] = fma(xv.y, wd[i][1], acc[i * TT + t]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) w[i] = wn[i];
-        }
-        // the lanes' sums: while there are several values left, a lane keeps half of them and hands over the other half
-        int n = 4 * TT, idx = 0, dup = 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            if (n > 1) {
-                const int half = n / 2;
-                const bool up = lane & o;
-#pragma unroll
-                for (int i = 0; i < 2 * TT; i++) {
-                    if (i >= half) break;
-                    const double send = up ? acc[i] : acc[i + half], keep = up ? acc[i + half] : acc[i];
-                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-                }
-                if (up) idx += half;
-                n = half;
-            } else {
-                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
-                dup |= lane & o;
-            }
-        }
-        if (dup == 0) part[((pr & 3) * epc + (pr >> 2) * 4 + idx / TT) * TT + idx % TT] = acc[0];
-    }
-    __syncthreads();
-    cluster_sync_all();  // (every block of the cluster runs: the first one's shared memory may be written)
-    for (int i = tid; i < epc * TT; i += kSmallThreads) {
-        const int e = i / TT, t = i % TT;
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) s += part[(k * epc + e) * TT + t];
-        const float f = (float)s;
-        st_dsmem_u32(reinterpret_cast<uint32_t*>(lg + (size_t)t * E + e0 + e), 0, __float_as_uint(f));
-        if (t < T) p.r.logits_rw[(size_t)t * p.r.ld + e0 + e] = f;
-    }
+    cluster_sync_all();  // every block of the cluster runs: the first one's shared memory may be written
+    router_block<WFMT, TT>(p.in, xs, part, 0, T, rank * epc, epc, [&](int e, int t, float f) {
+        st_dsmem_u32(reinterpret_cast<uint32_t*>(lg + (size_t)t * E + e), 0, __float_as_uint(f));
+        p.r.logits_rw[(size_t)t * p.r.ld + e] = f;
+    });
     if (rank == kSmallCluster - 1)
         for (int i = tid; i < T * (p.r.ld - E); i += kSmallThreads) p.r.logits_rw[(size_t)(i / (p.r.ld - E)) * p.r.ld + E + i % (p.r.ld - E)] = 0.f;
     cluster_sync_all();
     // the other blocks turn the activations into fixed point (tokens rank - 1, rank + 6)
     if (rank != 0) {
         if (p.fx.digits == nullptr) return;
-        for (int t = rank - 1; t < T; t += kSmallCluster - 1) {
-            const int G = D / 64, upad = (units + 31) / 32 * 32;
-            for (int u = tid; u < upad; u += kSmallThreads) {
-                const bool live = u < units;
-                float v[8];
-                load_x8(p.x, p.x_dtype, (size_t)t * p.ldx + (live ? u : 0) * 8, v);
-                const size_t g = (size_t)t * G + u / 8;
-                fixed_point_unit(v, u & 7, live ? p.fx.digits + g * 128 : nullptr, p.fx.scale + (live ? g : 0));
-            }
-        }
+        for (int t = rank - 1; t < T; t += kSmallCluster - 1)
+            fixed_point_row(p.in.x, p.in.x_dtype, (size_t)t * p.in.ldx, D, p.fx, t, tid, kSmallThreads);
         return;
     }
     if (warp < T) {
@@ -259,8 +105,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) __cluster_dims__(kSmallClust
     if (lane == 31) { wsum[warp] = off; wsum[32 + warp] = til; }
     __syncthreads();
     for (int k = 0; k < warp; k++) { off += wsum[k]; til += wsum[32 + k]; }
-    uint32_t* soff = reinterpret_cast<uint32_t*>(part);  // exclusive offsets
-    __syncthreads();
     if (tid < E) {
         soff[tid] = off - c;
         p.counts[tid] = c;

@@ -351,10 +351,11 @@ typedef void (*QgKernel)(const CUtensorMap, const CUtensorMap, const QgParams);
 // gw4: each consumer warp's K slice is four groups, its activation fragments stay in registers (8-row tiles only)
 template <int MODE, bool TM>
 QgKernel qg_pick_mt(int ms, bool gw4) {
-    if (ms == 4) return qmv_imma_grouped_kernel<MODE, 4, TM, 0>;
-    return gw4 ? qmv_imma_grouped_kernel<MODE, 2, TM, 4> : qmv_imma_grouped_kernel<MODE, 2, TM, 0>;
+    if (ms == 4) return qmv_imma_grouped_kernel<MODE, 4, TM, 0, 8>;
+    return gw4 ? qmv_imma_grouped_kernel<MODE, 2, TM, 4, 8> : qmv_imma_grouped_kernel<MODE, 2, TM, 0, 8>;
 }
-QgKernel qg_pick(int mode, int ms, bool tm, bool gw4) {
+QgKernel qg_pick(int mode, int ms, bool tm, bool gw4, bool fx = false) {
+    if (fx) return qmv_imma_grouped_kernel<kModeGateUp, 2, true, 4, 16>;
     if (mode == kModeGateUp) return tm ? qg_pick_mt<kModeGateUp, true>(ms, gw4) : qg_pick_mt<kModeGateUp, false>(ms, gw4);
     return tm ? qg_pick_mt<kModeDown, true>(ms, gw4) : qg_pick_mt<kModeDown, false>(ms, gw4);
 }
@@ -384,15 +385,20 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     p.srow_bytes = G * 2;
     p.xq_bytes = G * ms * 512;
     p.xsc_bytes = G * ms * 32;
+    // Sixteen consumer warps with the token rows as fixed point: K slices of four groups that divide them (K = 1024, 2048,
+    // 4096), gate/up tiles of eight rows
+    const bool fx = c.fx != nullptr && c.mode == kModeGateUp && ms == 2 && tm && c.row_map != nullptr && G % 4 == 0 && G / 4 <= 16 && 16 % (G / 4) == 0;
+    const int kQgWarps = fx ? 16 : 8;
+    if (fx) { p.fx = *c.fx; p.xq_bytes = p.xsc_bytes = 0; }
     p.red_bytes = 2 * kQgWarps * nw * ms * 64 * 4;
     const int fixed = p.xq_bytes + p.xsc_bytes + p.red_bytes + 256 + (tm ? 1024 : 0);
     // K slices per block of rows. 8-row tiles: one slice of four groups per warp when K allows it (the activation
     // fragments then live in registers: 69 against 83 us on the 64-token layer); else four slices (32-row blocks: half as
     // many hand-overs per byte) when two stages of that size fit, else eight.
     int ctas = 1, nstages = 0;
-    const bool gw4 = ms == 2 && G == 4 * kQgWarps;
-    const int cand[4] = {gw4 ? kQgWarps : kQgWarps / 2, kQgWarps, kQgWarps / 4, kQgWarps / 8};
-    for (int ci = 0; ci < 4 && nstages < 2; ci++) {
+    const bool gw4 = ms == 2 && (fx || G == 4 * kQgWarps);
+    const int cand[4] = {fx ? G / 4 : (gw4 ? kQgWarps : kQgWarps / 2), kQgWarps, kQgWarps / 4, kQgWarps / 8};
+    for (int ci = 0; ci < (fx ? 1 : 4) && nstages < 2; ci++) {
         const int wk = cand[ci];
         if (G % wk != 0 || (G / wk) % 4 != 0) continue;  // a warp's K slice: runs of four groups
         const int R = 16 * (kQgWarps / wk);
@@ -402,6 +408,11 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
         p.mat_bytes = round_up(R * p.row_pitch + 2 * R * p.srow_bytes, tm ? 1024 : 16);
         p.stage_bytes = nw * p.mat_bytes;
         nstages = (kQsSmemMax - fixed) / p.stage_bytes;
+    }
+    if (nstages < 2 && fx) {
+        GqmvCall without = c;
+        without.fx = nullptr;
+        return launch_qmv_imma_grouped(ctx, st, without);
     }
     if (nstages < 2) return 1;
     if (nstages > 8) nstages = 8;
@@ -437,7 +448,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)(items < slots ? items : slots), 1, 1);
-    cfg.blockDim = dim3(kQgThreads, 1, 1);
+    cfg.blockDim = dim3(qg_threads(kQgWarps), 1, 1);
     cfg.dynamicSmemBytes = fixed + nstages * p.stage_bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -445,7 +456,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, ms, tm, gw4 && p.wk == kQgWarps), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, ms, tm, gw4 && p.wk == kQgWarps, fx), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
 }
 
 }  // namespace
@@ -461,6 +472,11 @@ int32_t gqmv_init(iq_ctx* ctx) {
     for (int i = 0; i < 14; i++) {
         cudaError_t e = cudaFuncSetAttribute(qi[i], cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma)");
+    }
+    {
+        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(kModeGateUp, 2, true, true, true)),
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
+        if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
     }
     for (int mode = kModeGateUp; mode <= kModeDown; mode++)
         for (int v = 0; v < 6; v++) {  // 4 row sets, 2, 2 with register-resident activations; bulk or tensor copies
