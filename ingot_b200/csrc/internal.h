@@ -120,6 +120,8 @@ struct GqmvCall {
     const FixedRows* fx = nullptr;  // grouped gate/up: the token rows as block fixed point, when the caller has them
 };
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
+// Tiles of up to eight rows of affine 4-bit experts on the int8 kernel; 1: the shape does not fit it
+int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
 
 // One launch of the tensor-core GEMM (csrc/qmm.cu). x16: fp16 activations [x_rows, ldx] (bf16 with the plain bf16 format); w[i]: stacked
 // [experts * N, K] codes (w[1]: the up matrix of the gate/up epilogue). tiles == nullptr: dense tiling over M x N.
@@ -136,6 +138,7 @@ struct QmmCall {
     int32_t experts = 1;
     int32_t expert_lo = 0;
     int32_t N = 0, K = 0, M = 0;
+    int32_t w_rows = 0;  // plain formats: rows of w when fewer than N, the rest counts as zeros (0: N)
     const Tile* tiles = nullptr;
     const uint32_t* ntiles = nullptr;
     void* y = nullptr;

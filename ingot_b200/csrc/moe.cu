@@ -1,6 +1,7 @@
 // MoE layer and dense gated FFN entry points.
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "internal.h"
@@ -43,24 +44,19 @@ struct MoeWs {
     __half* s_h;
     void* s_yd;
     float* s_w;
-    Tile* s_tiles;
-    uint32_t* s_ntiles;
     size_t bytes;
 };
 
-// Height of the tiles of the GEMV-style expert kernels: 8 rows while experts see few rows, else 16.
-int decode_tile_rows(const iq_moe* l, int tokens) {
-    const int64_t pairs = (int64_t)tokens * l->d.top_k;
-    return pairs <= (int64_t)l->d.experts * 6 ? 8 : 16;
-}
-constexpr int kPrefillTileRows = 128;      // token rows per tensor-core tile while experts see few rows
-constexpr int kPrefillTileRowsBig = 192;   // ... and once they see many: every weight tile is dequantised less often
-constexpr int kTensorPathRowsPerExpert = 24;
-constexpr int kBigTileRowsPerExpert = 96;
+constexpr int kDecodeTileRows = 8;  // token rows per tile of the int8 expert kernels
 constexpr int kRouterSmemMax = 200 * 1024;
 constexpr int kGroupChunkedMinPairs = 4096;  // from here on the permutation runs as a chunked counting sort
-constexpr int kFixedTokens = 512;  // calls that run on the decode tile kernels have at most this many (24 rows per expert)
-constexpr int kRouterTiledMinTokens = 64;  // above this the router runs as a tiled float64 GEMM
+constexpr int kFixedTokens = 512;  // up to here the counting kernel leaves the activations as fixed point for the int8 kernels
+// Router products (tokens x experts x inputs) up to which a block takes eight tokens against a few experts in float64 (about
+// 0.35 us per million): beyond, the tensor cores with exact refinement (22 us at 27 to 400 million) where they apply, else the
+// tiled float64 GEMM. 128 experts x 2048 inputs, router and top-k: 128 tokens 22.8 -> 14.4 us, 200 tokens 22.5 -> 20.4, 400
+// tokens 22.5 against 37.6; 32 experts x 2880 inputs, 257 tokens 30.9 -> 10.8, 1000 tokens 41.0 against 38.6.
+constexpr int64_t kRouterBlockWork = 56000000, kRouterTiledWork = 90000000;
+int64_t router_work(const iq_moe* l, int tokens) { return (int64_t)tokens * l->d.experts * l->d.d_model; }
 
 // Expert outputs between the down projection and the combine: fp16 for affine experts, fp32 for MXFP4 ones, whose
 // outputs can pass half's range (the reference makes the same choice, MoEPrefill.swift:159-160).
@@ -86,7 +82,7 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     w.ntiles = static_cast<uint32_t*>(take(16));
     w.chunk_hist = static_cast<uint32_t*>(take((P / kGroupChunk + 1) * (size_t)d.experts * 4));
     w.tiles_a = static_cast<Tile*>(take((d.experts + P / 8 + 1) * sizeof(Tile)));
-    w.tiles_b = static_cast<Tile*>(take((d.experts + P / kPrefillTileRows + 1) * sizeof(Tile)));
+    w.tiles_b = static_cast<Tile*>(take((d.experts + P / 32 + 1) * sizeof(Tile)));
     w.h = static_cast<__half*>(take(P * d.d_ff * 2));
     w.yd = take(P * d.d_model * (yd_dtype_of(l) == kF16 ? 2 : 4));
     w.xs = static_cast<__half*>(take(P * d.d_model * 2));
@@ -95,15 +91,13 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     w.fx.scale = static_cast<float2*>(take(fixed * (d.d_model / 64) * 8));
     w.fh.digits = static_cast<unsigned char*>(take(few * d.top_k * (d.d_ff / 64) * 128));
     w.fh.scale = static_cast<float2*>(take(few * d.top_k * (d.d_ff / 64) * 8));
-    w.s_x16 = nullptr; w.s_h = nullptr; w.s_yd = nullptr; w.s_w = nullptr; w.s_tiles = nullptr; w.s_ntiles = nullptr;
+    w.s_x16 = nullptr; w.s_h = nullptr; w.s_yd = nullptr; w.s_w = nullptr;
     if (d.shared != IQ_SHARED_NONE) {
         const size_t T = (size_t)tokens;
         w.s_x16 = static_cast<__half*>(take(T * d.d_model * 2));
         w.s_h = static_cast<__half*>(take(T * d.shared_up.n * 2));
         w.s_yd = take(T * d.d_model * 4);
         w.s_w = static_cast<float*>(take(T * 4));
-        w.s_tiles = static_cast<Tile*>(take((T / 16 + 2) * sizeof(Tile)));
-        w.s_ntiles = static_cast<uint32_t*>(take(16));
     }
     w.bytes = off;
     return w;
@@ -139,8 +133,7 @@ constexpr int kRouteWideMaxTokens = 2048;
 bool tensor_router(const iq_moe* l, int tokens, int32_t x_dtype) {
     const iq_moe_desc& d = l->d;
     return l->router_wnorm_max > 0.f && l->ext_inds == nullptr && d.router_kind == IQ_ROUTER_BF16 &&
-           d.router_score == IQ_SCORE_SOFTMAX && x_dtype == kBF16 && tokens > kRouterTiledMinTokens && d.experts % 64 == 0 &&
-           d.d_model % 64 == 0;
+           d.router_score == IQ_SCORE_SOFTMAX && x_dtype == kBF16 && router_work(l, tokens) > kRouterBlockWork;
 }
 float router_err_coef(const iq_moe* l) { return (float)l->d.d_model * 4.76837158e-7f * 1.05f * l->router_wnorm_max; }
 
@@ -175,10 +168,10 @@ int32_t launch_route(iq_moe* l, cudaStream_t st, const float* logits, int ld, in
                       "route_topk launch");
 }
 
-// Gate + up + activation of every tile: h[row, :] = half(act(x W_gate^T + b_g, x W_up^T + b_u)). Expert e's weights live
+// On the int8 kernels; 1: the shape does not fit them. Gate + up + activation of every tile: h[row, :] = half(act(x W_gate^T + b_g, x W_up^T + b_u)). Expert e's weights live
 // at local slot e - expert_lo: the offset is folded into the base pointers. row_map == nullptr: x rows are in place.
 int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, int64_t ldx, const uint32_t* row_map,
-                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, int bm, __half* h, int row_map_div = 0,
+                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, __half* h, int row_map_div = 0,
                    const FixedRows* fx = nullptr) {
     const iq_moe_desc& d = l->d;
     const int64_t lo = d.expert_lo;
@@ -201,7 +194,7 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
     c.x = x; c.x_dtype = x_dtype; c.ldx = ldx;
     c.row_map = row_map; c.topk = row_map_div > 0 ? row_map_div : d.top_k;  // x row = row_map[sorted position] / divisor
     c.tiles = tiles; c.ntiles = ntiles; c.grid_tiles = max_tiles;
-    c.rows = 0; c.max_rows = bm;
+    c.rows = 0; c.max_rows = kDecodeTileRows;
     c.y = h; c.y_dtype = kF16; c.ldy = d.d_ff;
     if (d.gate_bias) {
         c.ebias[0] = d.gate_bias - lo * d.d_ff;
@@ -210,12 +203,12 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
     c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
     c.act = d.act;
     c.fx = fx;
-    return launch_gqmv(l->ctx, cs, c);
+    return launch_qmv_imma_grouped(l->ctx, cs, c);
 }
 
-// Down projection of every tile: yd[row, :] = h[row, :] W_down^T + b_d.
-int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles, const uint32_t* ntiles, int max_tiles,
-                 int bm, void* yd, int32_t yd_dtype) {
+// Likewise the down projection of every tile: yd[row, :] = h[row, :] W_down^T + b_d.
+int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles, const uint32_t* ntiles, int max_tiles, void* yd,
+                 int32_t yd_dtype) {
     const iq_moe_desc& d = l->d;
     const int64_t lo = d.expert_lo;
     GqmvCall c;
@@ -231,17 +224,22 @@ int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles,
     c.N = d.d_model; c.K = d.d_ff;
     c.x = h; c.x_dtype = kF16; c.ldx = d.d_ff;
     c.tiles = tiles; c.ntiles = ntiles; c.grid_tiles = max_tiles;
-    c.rows = 0; c.max_rows = bm;
+    c.rows = 0; c.max_rows = kDecodeTileRows;
     c.y = yd; c.y_dtype = yd_dtype; c.ldy = d.d_model;
     if (d.down_bias) c.ebias[0] = d.down_bias - lo * d.d_model;
-    return launch_gqmv(l->ctx, cs, c);
+    return launch_qmv_imma_grouped(l->ctx, cs, c);
 }
 
-// The experts run on the tcgen05 grouped GEMM once they see enough rows each for 128-row MMA tiles to pay; below
-// that the layer is bandwidth-bound and the GEMV-style tile kernels read each touched expert once.
-bool use_tensor_path(int64_t rows, int64_t expert_slots) { return rows >= expert_slots * kTensorPathRowsPerExpert; }
+// The affine experts run on the int8 kernels while they see up to six rows each on average; those need no dequantisation but
+// work through a tile four rows at a time. 128 experts of 2048 x 768, 8 of them per token, gate/up and down together: 64 tokens
+// (4 rows) 124 us against 139 on the grouped GEMM, 128 tokens (8 rows) 168 against 145. Everything else, MXFP4 experts
+// at any number of rows, runs on the grouped GEMM (MXFP4 at 4 tokens 132 -> 87 us for the layer, at 64 tokens 406 -> 145).
+constexpr int kInt8RowsPerExpert = 6;
+bool use_int8_path(const iq_moe* l, int64_t rows, int64_t expert_slots) { return l->fmt == kFmtAffine4 && rows <= expert_slots * kInt8RowsPerExpert; }
+// Token rows per tile of the grouped GEMM, by the average rows per expert. Up to 64 rows two CTAs share an SM (and 32 hold two
+// stages of activations more than 64); from 96 rows on every weight tile is dequantised less often at 192.
 int tensor_tile_rows(int64_t rows, int64_t expert_slots) {
-    return rows >= expert_slots * kBigTileRowsPerExpert ? kPrefillTileRowsBig : kPrefillTileRows;
+    return rows <= expert_slots * 8 ? 32 : rows <= expert_slots * 48 ? 64 : rows < expert_slots * 96 ? 128 : 192;
 }
 
 // rows16: fp16 rows [n_rows, d_model] in tile order
@@ -294,14 +292,13 @@ RouteSmallKernel route_small_vpl(int experts) {
 }
 template <int WFMT>
 RouteSmallKernel route_small_of(int tt, int experts) {
-    return tt == 1 ? route_small_vpl<WFMT, 1>(experts) : tt == 2 ? route_small_vpl<WFMT, 2>(experts)
-         : tt == 4 ? route_small_vpl<WFMT, 4>(experts) : route_small_vpl<WFMT, 8>(experts);
+    return tt == 1 ? route_small_vpl<WFMT, 1>(experts) : tt == 2 ? route_small_vpl<WFMT, 2>(experts) : route_small_vpl<WFMT, 4>(experts);
 }
 RouteSmallKernel route_small_pick(bool q8, int tt, int experts) { return q8 ? route_small_of<1>(tt, experts) : route_small_of<0>(tt, experts); }
 constexpr size_t kRouteSmallSmemMax = 200 * 1024;
 
-// Router, top-k and permutation in one cluster: up to eight tokens, while the float64 products of a block (a cluster has
-// eight) stay at a few microseconds and the tokens fit its shared memory. 128 experts x 2048 inputs: all eight tokens.
+// Router, top-k and permutation in one cluster: while the float64 products of a block (a cluster has eight) stay at a few
+// microseconds and the tokens fit its shared memory.
 bool use_route_small(const iq_moe* l, int tokens) {
     const iq_moe_desc& d = l->d;
     const int tt = router_tokens(tokens);
@@ -385,15 +382,7 @@ int32_t run_shared_expert(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_d
     int32_t st = check_cuda(ctx, cudaGetLastError(), "shared_gate launch");
     if (st != kOk) return st;
     const int32_t ydt = yd_dtype_of(l);
-    if (use_tensor_path(tokens, 1)) {
-        const int bn = tensor_tile_rows(tokens, 1);
-        const size_t units = (size_t)tokens * d.d_model / 8;
-        rows_to_f16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, cs>>>(x, x_dtype, ldx, w.s_x16, tokens, d.d_model);
-        shared_tiles_kernel<<<1, 128, 0, cs>>>(tokens, bn, 0u, w.s_tiles, w.s_ntiles);
-        st = check_cuda(ctx, cudaGetLastError(), "shared tiles launch");
-        if (st == kOk) st = run_gateup_tc(&tmp, cs, w.s_x16, tokens, w.s_tiles, w.s_ntiles, w.s_h, bn);
-        if (st == kOk) st = run_down_tc(&tmp, cs, w.s_h, tokens, w.s_tiles, w.s_ntiles, w.s_yd, ydt, bn);
-    } else if (tokens <= 16) {  // a dense FFN on the decode kernels, no tile list
+    if (tokens <= 16) {  // a dense FFN on the decode kernels
         GqmvCall c;
         c.mode = kModeGateUp;
         c.fmt = kFmtAffine4;
@@ -422,13 +411,12 @@ int32_t run_shared_expert(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_d
         q.rows = tokens; q.max_rows = tokens;
         q.y = w.s_yd; q.y_dtype = ydt; q.ldy = d.d_model;
         st = launch_gqmv(ctx, cs, q);
-    } else {
-        const int bm = 16;
-        shared_tiles_kernel<<<1, 128, 0, cs>>>(tokens, bm, 0u, w.s_tiles, w.s_ntiles);
-        st = check_cuda(ctx, cudaGetLastError(), "shared tiles launch");
-        const int max_tiles = (tokens + bm - 1) / bm;
-        if (st == kOk) st = run_gateup(&tmp, cs, x, x_dtype, ldx, nullptr, w.s_tiles, w.s_ntiles, max_tiles, bm, w.s_h);
-        if (st == kOk) st = run_down(&tmp, cs, w.s_h, w.s_tiles, w.s_ntiles, max_tiles, bm, w.s_yd, ydt);
+    } else {  // ... or on the GEMM
+        const size_t units = (size_t)tokens * d.d_model / 8;
+        rows_to_f16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, cs>>>(x, x_dtype, ldx, w.s_x16, tokens, d.d_model);
+        st = check_cuda(ctx, cudaGetLastError(), "rows_to_f16 launch");
+        if (st == kOk) st = run_gateup_tc(&tmp, cs, w.s_x16, tokens, nullptr, nullptr, w.s_h, 0);
+        if (st == kOk) st = run_down_tc(&tmp, cs, w.s_h, tokens, nullptr, nullptr, w.s_yd, ydt, 0);
     }
     if (st != kOk) return st;
     shared_add_kernel<<<tokens, 256, 0, cs>>>(w.s_yd, ydt, w.s_w, out, out_dtype, ldo, tokens, d.d_model);
@@ -746,7 +734,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
 
     const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l);
     if (small) {
-        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, small_experts);
+        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, l->fmt == kFmtAffine4);
         if (st == kOk && small_experts)
             st = run_experts_small(l, cs, tokens, w, out, out_dtype, ldo, (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0);
         if (st != kOk) return st;
@@ -764,12 +752,16 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         c.x16 = x; c.ldx = ldx; c.x_rows = tokens;
         c.w[0] = d.router_w;
         c.experts = 1;
-        c.N = d.experts; c.K = d.d_model; c.M = tokens;
+        c.N = l->ld; c.w_rows = d.experts; c.K = d.d_model; c.M = tokens;  // (the columns past the experts become zeros)
         c.y = w.logits; c.y_dtype = kF32; c.ldy = l->ld;
         st = launch_qmm(ctx, cs, c);
         if (st != kOk) return st;
     } else if ((pieces & IQ_PIECE_ROUTER) && l->ext_inds == nullptr) {
-        if (tokens > kRouterTiledMinTokens && d.d_model % 64 == 0) {
+        // eight experts per block (fewer where that leaves the GPU empty) and as many tokens as fit shared memory
+        int tt = router_tokens(tokens);
+        while (tt > 1 && router_block_smem(tt, d.d_model, 8) > (size_t)kRouterSmemMax) tt /= 2;
+        const bool fits = router_block_smem(tt, d.d_model, 8) <= (size_t)kRouterSmemMax;
+        if (tokens > 64 && (router_work(l, tokens) > kRouterTiledWork || !fits)) {
             // register-tiled float64 GEMM; the K range is split over a cluster until the grid fills the GPU several
             // times over (the blocks of one SM share its float64 pipe, so balance comes from many small blocks)
             const int bm = tokens >= 1024 ? 64 : 32;
@@ -798,13 +790,10 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
                             "router_logits_tiled launch");
             if (st != kOk) return st;
         } else {
-        // eight experts per block (fewer where that leaves the GPU empty) and as many tokens as fit shared memory
-        int tt = router_tokens(tokens);
-        while (tt > 1 && router_block_smem(tt, d.d_model, 8) > (size_t)kRouterSmemMax) tt /= 2;
         const int groups = (tokens + tt - 1) / tt;
         const int epc = d.experts / 8 * groups * 2 <= ctx->sms ? 4 : 8;
         const size_t smem = router_block_smem(tt, d.d_model, epc);
-        if (smem > (size_t)kRouterSmemMax) return fail(ctx, kErrUnsupported, "moe: d_model = %d is too wide for the router kernel", d.d_model);
+        if (!fits) return fail(ctx, kErrUnsupported, "moe: d_model = %d is too wide for the router kernel", d.d_model);
         const RouterIn in = {x, x_dtype, ldx, d.router_w, d.router_scales, d.router_biases, d.d_model};
         st = check_cuda(ctx, launch_dependent(router_kernel_pick(d.router_kind != IQ_ROUTER_BF16, tt), dim3(groups, d.experts / epc), kRouterThreads, smem, cs,
                                               in, w.logits, tokens, d.experts, l->ld, epc), "router_logits launch");
@@ -818,15 +807,15 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         st = launch_route(l, cs, w.logits, l->ld, tokens, w.inds, w.wts, fast_router ? x : nullptr, ldx);
         if (st != kOk) return st;
     }
-    const int bm = decode_tile_rows(l, tokens);
-    // whole calls on the decode tile kernels: the counting kernel leaves the activations as fixed point for the gate/up one
-    const bool fixed = (pieces & (IQ_PIECE_GROUP | IQ_PIECE_GATEUP)) == (IQ_PIECE_GROUP | IQ_PIECE_GATEUP) && l->fmt == kFmtAffine4 &&
-                       tokens <= kFixedTokens && P < kGroupChunkedMinPairs && !use_tensor_path(P, d.expert_count) && bm == 8;
+    const bool int8 = use_int8_path(l, P, d.expert_count);
+    const int bn = tensor_tile_rows(P, d.expert_count);
+    // whole calls on the int8 kernels: the counting kernel leaves the activations as fixed point for the gate/up one
+    const bool fixed = int8 && (pieces & IQ_PIECE_GATEUP) && (small || ((pieces & IQ_PIECE_GROUP) && tokens <= kFixedTokens && P < kGroupChunkedMinPairs));
     if (pieces & IQ_PIECE_GROUP) {
         GroupParams gp;
         gp.inds = inds; gp.counts = w.counts; gp.offsets = w.offsets; gp.row_map = w.row_map; gp.pos = w.pos;
         gp.tiles_a = w.tiles_a; gp.tiles_b = w.tiles_b; gp.ntiles = w.ntiles;
-        gp.P = P; gp.E = d.experts; gp.bm_a = bm; gp.bm_b = tensor_tile_rows(P, d.expert_count);
+        gp.P = P; gp.E = d.experts; gp.bm_a = kDecodeTileRows; gp.bm_b = bn;
         gp.e_lo = d.expert_lo; gp.e_hi = d.expert_lo + d.expert_count;
         gp.chunk_hist = w.chunk_hist;
         gp.chunks = (P + kGroupChunk - 1) / kGroupChunk;
@@ -846,24 +835,19 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st == kOk) st = check_cuda(ctx, cudaGetLastError(), "moe_group launch");
         if (st != kOk) return st;
     }
-    const int64_t max_tiles64 = (int64_t)d.expert_count + P / bm;
-    const int max_tiles = (int)(max_tiles64 < P ? max_tiles64 : P);
-    if (max_tiles > 65535 && !use_tensor_path(P, d.expert_count))
-        return fail(ctx, kErrInvalidArg, "moe: %d tokens give too many tiles for one launch", tokens);
-    const bool tc = use_tensor_path(P, d.expert_count);
+    const int max_tiles = (int)std::min<int64_t>((int64_t)d.expert_count + P / kDecodeTileRows, P);
     if (pieces & IQ_PIECE_GATEUP) {
-        if (tc) {
+        st = int8 ? run_gateup(l, cs, x, x_dtype, ldx, w.row_map, w.tiles_a, w.ntiles, max_tiles, w.h, 0, fixed ? &w.fx : nullptr) : 1;
+        if (st == 1) {
             moe_pack_tokens_kernel<<<tokens, 256, 0, cs>>>(x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k);
             st = check_cuda(ctx, cudaGetLastError(), "moe_pack_tokens launch");
-            if (st == kOk) st = run_gateup_tc(l, cs, w.xs, P, w.tiles_b, w.ntiles + 1, w.h, tensor_tile_rows(P, d.expert_count));
-        } else {
-            st = run_gateup(l, cs, x, x_dtype, ldx, w.row_map, w.tiles_a, w.ntiles, max_tiles, bm, w.h, 0, fixed ? &w.fx : nullptr);
+            if (st == kOk) st = run_gateup_tc(l, cs, w.xs, P, w.tiles_b, w.ntiles + 1, w.h, bn);
         }
         if (st != kOk) return st;
     }
     if (pieces & IQ_PIECE_DOWN) {
-        st = tc ? run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), tensor_tile_rows(P, d.expert_count))
-                : run_down(l, cs, w.h, w.tiles_a, w.ntiles, max_tiles, bm, w.yd, yd_dtype_of(l));
+        st = int8 ? run_down(l, cs, w.h, w.tiles_a, w.ntiles, max_tiles, w.yd, yd_dtype_of(l)) : 1;
+        if (st == 1) st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn);
         if (st != kOk) return st;
     }
     if (pieces & IQ_PIECE_COMBINE) {
@@ -974,34 +958,28 @@ int32_t moe_experts_impl(iq_moe* l, void* stream, const void* rows_f16, const ui
         return fail(ctx, kErrWorkspace, "moe_experts: workspace %zu < %zu", workspace_bytes, w.bytes);
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
     const int64_t slots = (int64_t)sources * d.expert_count;
-    if (use_tensor_path(total_rows, slots)) {
-        const int bn = tensor_tile_rows(total_rows, slots);
-        ep_tiles_kernel<<<1, 512, 0, cs>>>(counts, sources, d.experts, d.expert_lo, d.expert_count, bn, (uint32_t)region_rows, w.tiles,
-                                           w.ntiles);
-        int32_t st2 = check_cuda(ctx, cudaGetLastError(), "ep_tiles launch");
-        // the row count is only known on the device: bounds come from the capacity, total_rows picks the kernels
-        const __half* rows = static_cast<const __half*>(rows_f16);
-        if (st2 == kOk && row_index != nullptr) {
-            moe_gather_rows_kernel<<<ctx->sms * 8, 256, 0, cs>>>(rows, row_index, w.tiles, w.ntiles, bn, w.xs, d.d_model);
-            st2 = check_cuda(ctx, cudaGetLastError(), "moe_gather_rows launch");
-            rows = w.xs;
-        }
-        if (st2 == kOk) st2 = run_gateup_tc(l, cs, rows, max_rows, w.tiles, w.ntiles, w.h, bn);
-        if (st2 == kOk) st2 = run_down_tc(l, cs, w.h, max_rows, w.tiles, w.ntiles, yd, yd_dtype, bn);
-        if (st2 == kOk && yd_rows != nullptr) st2 = scatter_rows(ctx, cs, yd, yd_rows, max_rows, d.d_model, yd_dtype);
-        return st2;
-    }
-    const int bm = total_rows <= slots * 6 ? 8 : 16;
-    ep_tiles_kernel<<<1, 512, 0, cs>>>(counts, sources, d.experts, d.expert_lo, d.expert_count, bm, (uint32_t)region_rows, w.tiles,
-                                       w.ntiles);
+    // the row count is only known on the device: bounds come from the capacity, total_rows picks the kernels
+    const bool int8 = use_int8_path(l, total_rows, slots);
+    const int bn = int8 ? 16 : tensor_tile_rows(total_rows, slots);  // (where a shape does not fit the int8 kernels the GEMM takes their tiles)
+    ep_tiles_kernel<<<1, 512, 0, cs>>>(counts, sources, d.experts, d.expert_lo, d.expert_count, int8 ? kDecodeTileRows : bn,
+                                       (uint32_t)region_rows, w.tiles, w.ntiles);
     int32_t st = check_cuda(ctx, cudaGetLastError(), "ep_tiles launch");
     if (st != kOk) return st;
-    const int64_t mt = max_rows / bm + slots;
-    const int max_tiles = (int)(mt < max_rows ? mt : max_rows);
-    if (max_tiles > 65535) return fail(ctx, kErrInvalidArg, "moe_experts: too many tiles for one launch");
-    st = run_gateup(l, cs, rows_f16, kF16, d.d_model, row_index, w.tiles, w.ntiles, max_tiles, bm, w.h, 1);
+    const int max_tiles = (int)std::min<int64_t>(max_rows / kDecodeTileRows + slots, max_rows);
+    st = int8 ? run_gateup(l, cs, rows_f16, kF16, d.d_model, row_index, w.tiles, w.ntiles, max_tiles, w.h, 1) : 1;
+    if (st == 1) {
+        const __half* rows = static_cast<const __half*>(rows_f16);
+        if (row_index != nullptr) {
+            moe_gather_rows_kernel<<<ctx->sms * 8, 256, 0, cs>>>(rows, row_index, w.tiles, w.ntiles, bn, w.xs, d.d_model);
+            st = check_cuda(ctx, cudaGetLastError(), "moe_gather_rows launch");
+            if (st != kOk) return st;
+            rows = w.xs;
+        }
+        st = run_gateup_tc(l, cs, rows, max_rows, w.tiles, w.ntiles, w.h, bn);
+    }
     if (st != kOk) return st;
-    st = run_down(l, cs, w.h, w.tiles, w.ntiles, max_tiles, bm, yd, yd_dtype);
+    st = int8 ? run_down(l, cs, w.h, w.tiles, w.ntiles, max_tiles, yd, yd_dtype) : 1;
+    if (st == 1) st = run_down_tc(l, cs, w.h, max_rows, w.tiles, w.ntiles, yd, yd_dtype, bn);
     if (st != kOk || yd_rows == nullptr) return st;
     return scatter_rows(ctx, cs, yd, yd_rows, max_rows, d.d_model, yd_dtype);
 }

@@ -1001,14 +1001,6 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const void* __restrict
     *reinterpret_cast<uint4*>(out + i) = o;
 }
 
-// Tile list of the shared expert: all T rows in place, tiles of bm rows, expert id `expert`.
-__global__ void shared_tiles_kernel(int T, int bm, uint32_t expert, Tile* __restrict__ tiles, uint32_t* __restrict__ ntiles) {
-    const int n = (T + bm - 1) / bm;
-    for (int j = threadIdx.x; j < n; j += blockDim.x)
-        tiles[j] = Tile{expert, (uint32_t)(j * bm), (uint32_t)min(bm, T - j * bm), 0};
-    if (threadIdx.x == 0) ntiles[0] = (uint32_t)n;
-}
-
 // out[t, :] += sg[t] * ys[t, :] (the shared expert's contribution)
 __global__ void __launch_bounds__(256) shared_add_kernel(const void* __restrict__ ys, int32_t ys_dtype, const float* __restrict__ sg,
                                                         void* __restrict__ out, int32_t out_dtype, int64_t ldo, int T, int D) {

@@ -1,5 +1,6 @@
-// The MoE block for up to eight tokens in three kernels, where a decode step of few tokens is a chain of latencies and not
-// of bytes (one token of the 128-expert layer reads 21 MB, 3 us, and took 59 us in eight kernels):
+// The MoE block for up to three tokens in three kernels, where a decode step of few tokens is a chain of latencies and not
+// of bytes (one token of the 128-expert layer reads 21 MB, 3 us, and took 59 us in eight kernels, 25 in three; three tokens
+// 52 us against 57. From four on, 67 against 61, the separate kernels, which stage the weights, win):
 //
 //   moe_route_small_kernel   router logits, top-k and the permutation in one cluster of eight blocks; also the activations as
 //                            block fixed point (the int8 kernels' operand, see qmv_imma.cuh), once per token
@@ -22,7 +23,7 @@
 
 namespace iq {
 
-constexpr int kSmallTokens = 8;
+constexpr int kSmallTokens = 3;
 constexpr int kSmallThreads = 512;
 constexpr int kSmallCluster = 8;
 
@@ -37,7 +38,7 @@ constexpr size_t route_small_smem(int tt, int D, int E) {
     return router_block_smem(tt, D, E / kSmallCluster) + (size_t)tt * E * 4 + 16 * kSmallTokens * 4 + 64 * 4 + (size_t)E * 4;
 }
 
-// WFMT: 0 bf16 router, 1 8-bit affine. TT: tokens rounded up to 1, 2, 4, 8. VPL: experts per lane of the selection.
+// WFMT: 0 bf16 router, 1 8-bit affine. TT: tokens rounded up to 1, 2, 4. VPL: experts per lane of the selection.
 // A block of the cluster takes E / 8 experts (router_block: the other router kernels' bits). The logits meet in the
 // first block's shared memory, which then selects (a warp per token) and groups.
 template <int WFMT, int TT, int VPL>
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) __cluster_dims__(kSmallClust
     double2* xs = reinterpret_cast<double2*>(smem);
     double* part = reinterpret_cast<double*>(smem + (size_t)TT * D * 8);
     float* lg = reinterpret_cast<float*>(part + (size_t)router_slices(epc) * epc * TT);  // [TT][E], the first block's
-    uint32_t* sinds = reinterpret_cast<uint32_t*>(lg + (size_t)TT * E);                  // [16 * 8]
+    uint32_t* sinds = reinterpret_cast<uint32_t*>(lg + (size_t)TT * E);                  // [16 * kSmallTokens]
     uint32_t* wsum = sinds + 16 * kSmallTokens;                                          // [2][32]
     uint32_t* soff = wsum + 64;                                                          // [E] exclusive offsets
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x;
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) __cluster_dims__(kSmallClust
     if (rank == kSmallCluster - 1)
         for (int i = tid; i < T * (p.r.ld - E); i += kSmallThreads) p.r.logits_rw[(size_t)(i / (p.r.ld - E)) * p.r.ld + E + i % (p.r.ld - E)] = 0.f;
     cluster_sync_all();
-    // the other blocks turn the activations into fixed point (tokens rank - 1, rank + 6)
+    // the other blocks turn the activations into fixed point
     if (rank != 0) {
         if (p.fx.digits == nullptr) return;
         for (int t = rank - 1; t < T; t += kSmallCluster - 1)
@@ -181,11 +182,11 @@ __device__ __forceinline__ void small_mma(float (&acc)[2], const SmallBatch& v, 
     acc[1] = fmaf(b1, xs.y, acc[1]);
 }
 
-// A block's item: 64 features (gate and up) of one tile of up to eight rows; its sixteen warps are four blocks of 16 rows x
+// A block's item: 64 features (gate and up) of one tile of up to four rows; its sixteen warps are four blocks of 16 rows x
 // four slices of the inputs.
 __global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(const GateUpSmallParams p) {
     constexpr int RS = 72;  // floats between activation rows of the slices' sums (the lanes of a store in different banks)
-    __shared__ float red[4][2][8][RS];
+    __shared__ float red[4][2][4][RS];
     __shared__ float gmax[16], gsum[16];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int rb = warp & 3, ks = warp >> 2;
@@ -198,43 +199,28 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(cons
     for (int it = blockIdx.x; it < total; it += gridDim.x) {
         const uint4 tw = __ldcg(reinterpret_cast<const uint4*>(p.tiles) + it / NB);
         const Tile tile = Tile{tw.x, tw.y, tw.z, tw.w};
-        const int n0 = (it % NB) * 64, M = (int)tile.count, sets = M > 4 ? 2 : 1;
+        const int n0 = (it % NB) * 64, M = (int)tile.count;
         const int64_t row = (int64_t)tile.expert * p.I + n0 + rb * 16 + g;
         SmallBatch cur[2], nxt[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) small_load(cur[i], p.w[i], p.s[i], p.b[i], row, G, 2 * min(p0, pairs - 1), even, t);
         // fragments: lane (g, t) holds digit g % 2 of row g / 2 of the set; scales: of row t of the set
-        const unsigned char* xd[2];
-        const float2* xs[2];
-        bool xl[2];
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-            const int m = 4 * c + (g >> 1), ms = 4 * c + t;
-            xl[c] = m < M;
-            const uint32_t tok = __ldcg(p.row_map + tile.start + min(m, M - 1)) / (uint32_t)p.topk;
-            const uint32_t tks = __ldcg(p.row_map + tile.start + min(ms, M - 1)) / (uint32_t)p.topk;
-            xd[c] = p.x.digits + (size_t)tok * G * 128 + (g & 1) * 64 + t * 16;
-            xs[c] = p.x.scale + (size_t)tks * G;
-        }
-        float acc[2][2][2];
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int c = 0; c < 2; c++) acc[i][c][0] = acc[i][c][1] = 0.f;
+        const bool live = (g >> 1) < M;
+        const uint32_t tok = __ldcg(p.row_map + tile.start + min(g >> 1, M - 1)) / (uint32_t)p.topk;
+        const uint32_t tks = __ldcg(p.row_map + tile.start + min(t, M - 1)) / (uint32_t)p.topk;
+        const unsigned char* xd = p.x.digits + (size_t)tok * G * 128 + (g & 1) * 64 + t * 16;
+        const float2* xs = p.x.scale + (size_t)tks * G;
+        float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
         auto compute = [&](const SmallBatch (&v)[2], int pr) {
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 const int grp = 2 * pr + u;
                 if (grp >= G) break;
-#pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    if (c >= sets) break;
-                    uint4 xb = *reinterpret_cast<const uint4*>(xd[c] + grp * 128);
-                    if (!xl[c]) xb = make_uint4(0, 0, 0, 0);
-                    const float2 sv = xs[c][grp];
-                    small_mma(acc[0][c], v[0], u, xb, sv);
-                    small_mma(acc[1][c], v[1], u, xb, sv);
-                }
+                uint4 xb = *reinterpret_cast<const uint4*>(xd + grp * 128);
+                if (!live) xb = make_uint4(0, 0, 0, 0);
+                const float2 sv = xs[grp];
+                small_mma(acc[0], v[0], u, xb, sv);
+                small_mma(acc[1], v[1], u, xb, sv);
             }
         };
         int pr = p0;
@@ -248,20 +234,18 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(cons
         }
         if (pr < p1) compute(cur, pr);
 #pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                red[ks][i][4 * c + t][rb * 16 + g] = acc[i][c][0];
-                red[ks][i][4 * c + t][rb * 16 + 8 + g] = acc[i][c][1];
-            }
+        for (int i = 0; i < 2; i++) {
+            red[ks][i][t][rb * 16 + g] = acc[i][0];
+            red[ks][i][t][rb * 16 + 8 + g] = acc[i][1];
+        }
         __syncthreads();
         // a thread per (feature, row): the slices in order, the activation, and the group of 64 features as block fixed point
         const int f = tid & 63, m = tid >> 6;
         float gv = 0.f, uv = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            gv += red[k][0][m][f];
-            uv += red[k][1][m][f];
+            gv += red[k][0][m & 3][f];  // (rows past the fourth: nothing is stored)
+            uv += red[k][1][m & 3][f];
         }
         if (p.ebias[0] != nullptr) {
             gv += p.ebias[0][(size_t)tile.expert * p.I + n0 + f];

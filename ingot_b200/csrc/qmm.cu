@@ -48,13 +48,14 @@ const KernelEntry* find(int32_t fmt, int bn) {
 typedef void (*TaKernel)(const TaMaps, const TaParams);
 
 // gate/up: the formats of experts and of dense FFNs
+template <int GROUPS>
 TaKernel ta_pick(int32_t fmt, int epi) {
     switch (fmt) {
-        case kFmtAffine4: return epi ? qmm_ta_kernel<kFmtAffine4, 1> : qmm_ta_kernel<kFmtAffine4, 0>;
-        case kFmtMxfp4: return epi ? qmm_ta_kernel<kFmtMxfp4, 1> : qmm_ta_kernel<kFmtMxfp4, 0>;
-        case kFmtAffine8: return epi ? qmm_ta_kernel<kFmtAffine8, 1> : qmm_ta_kernel<kFmtAffine8, 0>;
-        case kFmtAffine4G32: return epi ? qmm_ta_kernel<kFmtAffine4G32, 1> : qmm_ta_kernel<kFmtAffine4G32, 0>;
-        case kFmtTernary: return epi ? nullptr : qmm_ta_kernel<kFmtTernary, 0>;
+        case kFmtAffine4: return epi ? qmm_ta_kernel<kFmtAffine4, 1, GROUPS> : qmm_ta_kernel<kFmtAffine4, 0, GROUPS>;
+        case kFmtMxfp4: return epi ? qmm_ta_kernel<kFmtMxfp4, 1, GROUPS> : qmm_ta_kernel<kFmtMxfp4, 0, GROUPS>;
+        case kFmtAffine8: return epi ? qmm_ta_kernel<kFmtAffine8, 1, GROUPS> : qmm_ta_kernel<kFmtAffine8, 0, GROUPS>;
+        case kFmtAffine4G32: return epi ? qmm_ta_kernel<kFmtAffine4G32, 1, GROUPS> : qmm_ta_kernel<kFmtAffine4G32, 0, GROUPS>;
+        case kFmtTernary: return epi ? nullptr : qmm_ta_kernel<kFmtTernary, 0, GROUPS>;
         default: return nullptr;
     }
 }
@@ -80,9 +81,10 @@ int ta_tile_rows(int m, int n_tiles, int sms) {
 int32_t qmm_init(iq_ctx* ctx) {
     for (int fmt = 0; fmt <= kFmtTernary; fmt++)
         for (int epi = 0; epi < 2; epi++) {
-            const TaKernel k = ta_pick(fmt, epi);
+            const TaKernel k = ta_pick<kTaGroups>(fmt, epi), low = ta_pick<kTaGroupsLow>(fmt, epi);
             if (k == nullptr) continue;
             cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k), cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemMax);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(low), cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemLow);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmm_ta)");
         }
     int n;
@@ -168,7 +170,8 @@ int32_t cached_rowblock_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t
 
 // The quantized formats: weights through tensor memory (csrc/qmm_ta.cuh). c.bn: the largest tile of the list (grouped).
 static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
-    const TaKernel k = ta_pick(c.fmt, c.epi);
+    const bool low = c.tiles != nullptr && c.bn <= kTaLowRows;  // two CTAs per SM
+    const TaKernel k = low ? ta_pick<kTaGroupsLow>(c.fmt, c.epi) : ta_pick<kTaGroups>(c.fmt, c.epi);
     if (k == nullptr) return fail(ctx, kErrNoKernel, "qmm: no kernel for format %d, epilogue %d", c.fmt, c.epi);
     TaParams p;
     memset(&p, 0, sizeof(p));
@@ -179,11 +182,11 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     // steps per copy, four where that is still small.
     p.xbox = c.tiles == nullptr || rows <= 16 ? rows : round_up(rows / 4, 16);
     p.nbox = rows / p.xbox;
-    p.xk = rows <= 128 ? 4 : 2;
+    p.xk = low ? (rows <= 32 ? 4 : 2) : (rows <= 128 ? 4 : 2);
     p.x_stage = rows * 128 * p.xk;
-    p.dcols = rows <= 128 ? 128 : kTaMaxRows;
+    p.dcols = low ? kTaLowRows : (rows <= 128 ? 128 : kTaMaxRows);
     // stages: at least three of codes, then up to eight of X, then as many of codes as fit
-    const int room = kTaSmemMax - kTaSmemFixed;
+    const int room = (low ? kTaSmemLow : kTaSmemMax) - kTaSmemFixed;
     const int c_stage = ta_code_stage(c.fmt);
     p.nx = (room - 3 * c_stage) / p.x_stage;
     if (p.nx > 8) p.nx = 8;
@@ -220,7 +223,7 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     p.limit = c.limit;
     p.act = c.act;
     p.status = ctx->d_status;
-    int grid = ctx->sms;
+    int grid = low ? 2 * ctx->sms : ctx->sms;
     if (c.tiles == nullptr) {
         const int work = ((c.M + rows - 1) / rows) * n_tiles;
         if (work < grid) grid = work;
@@ -228,7 +231,7 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(kTaThreads, 1, 1);
+    cfg.blockDim = dim3(ta_threads(low ? kTaGroupsLow : kTaGroups), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -249,7 +252,7 @@ int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     const int elem = i8 ? 0 : 2, es = i8 ? 1 : 2, bke = i8 ? 128 : 64;
     CUtensorMap mx, mw;
     int32_t r = make_map_2d(ctx, &mx, c.x16, elem, (uint64_t)c.K, (uint64_t)c.x_rows, (uint64_t)c.ldx * es, bke, c.bn, true);
-    if (r == kOk) r = make_map_2d(ctx, &mw, c.w[0], elem, (uint64_t)c.K, (uint64_t)c.N, (uint64_t)c.K * es, bke, kWRows, true);
+    if (r == kOk) r = make_map_2d(ctx, &mw, c.w[0], elem, (uint64_t)c.K, (uint64_t)(c.w_rows ? c.w_rows : c.N), (uint64_t)c.K * es, bke, kWRows, true);
     if (r != kOk) return r;
     QmmParams p = {};
     p.s = c.s[0]; p.b = c.b[0];

@@ -24,10 +24,16 @@
 //                conflicts
 //   warp 3       producer of the stage's scales and biases (asynchronous copies of a row's 4-16 bytes)
 //   warps 4-7    epilogue
-//   warps 8-23   dequantisers, four groups of four warps on every fourth K step
+//   warps 8-23   dequantisers, four groups of four warps on every fourth K step (two CTAs per SM: two groups)
 // The gate/up form takes 64 gate rows and the matching 64 up rows as one tile of 128: lanes 0-15 of every warp's quadrant
 // hold gate rows, lanes 16-31 the same rows of up, so that the activation needs one shuffle per two tokens and
 // everything else is the plain form.
+// Tiles of a list that hold up to 64 tokens (MoE decode and short prefills) leave the MMA idle: a step of 16 tokens is 72 cycles
+// of it, and the 400 cycles of the issuing thread and of its hand-overs are the time. Two CTAs per SM, each with two
+// dequantiser groups, half of the shared memory and 256 columns (two accumulators of 64, four A stages), run two such
+// chains side by side: 32 experts of 2880 x 2880 (MXFP4) at 64 tokens, gate/up 102 -> 78 us (3.6 TB/s) and down 53 -> 45;
+// 128 experts of 2048 x 768 (4 bits) at 200 tokens 100 -> 90 and 51 -> 46. Three groups per CTA were slower (48 registers).
+// What bounds it now is issue slots: 70 % busy, two thirds of them the conversion of the codes.
 // Every wait is bounded: on a timeout the kernel writes a status word, all roles drain and tensor memory is released.
 //
 // Replaces qmm_t_nax3* (Shaders/qmm_nax_v3.metal:107-256) and, with a tile list, moe_gateup_swiglu2* / moe_down2*
@@ -44,12 +50,15 @@
 
 namespace iq {
 
-constexpr int kTaThreads = 768;
-constexpr int kTaGroups = 4;               // dequantiser groups of four warps
+constexpr int kTaGroups = 4;               // dequantiser groups of four warps: one CTA per SM
+constexpr int kTaGroupsLow = 2;            // ... two CTAs per SM (tiles of up to 64 tokens)
+constexpr int kTaLowRows = 64;
+constexpr int ta_threads(int groups) { return 256 + 128 * groups; }
 constexpr int kTaMaxRows = 192;            // token rows per tile
 constexpr int kTaCodeStage = 128 * 128;    // bytes of a stage of packed codes
 constexpr int kTaMaxStages = 12;
 constexpr int kTaSmemMax = 232448;
+constexpr int kTaSmemLow = 115712;         // two CTAs per SM: half of 228 KB each, less the system's KB
 constexpr int kTaSmemFixed = 1024 + 1024;  // alignment, barriers
 
 struct TaParams {
@@ -72,7 +81,7 @@ struct TaParams {
     int32_t xbox, nbox, xk;
     int32_t nx, nc;          // stages of X and of codes
     int32_t x_stage;         // bytes of an X stage
-    int32_t dcols;           // columns per accumulator: 128 or 192
+    int32_t dcols;           // columns per accumulator: 64, 128 or 192
     int32_t vec;             // the row pitch of the scales allows asynchronous copies
     int32_t* status;
 };
@@ -199,10 +208,11 @@ __device__ __forceinline__ void ta_dequant32(uint32_t codes, uint32_t unit, int 
 }
 
 // EPI: 0 store, 1 gate + up + activation.
-template <int FMT, int EPI>
-__global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_constant__ TaMaps maps, const TaParams p) {
+template <int FMT, int EPI, int GROUPS>
+__global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 2) qmm_ta_kernel(const __grid_constant__ TaMaps maps, const TaParams p) {
     using F = TaFmt<FMT>;
     constexpr int KPS = F::KPS;
+    constexpr uint32_t TCOLS = GROUPS == kTaGroups ? 512 : 256;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t codes0 = smem_u32(smem), x0 = codes0 + p.nc * kTaCodeStage;  // codes, X, scales
@@ -219,7 +229,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.nc; i++) {
             mbar_init(bar_cfull + 8 * i, 1 + 32);  // the codes' copy, the scale producer's lanes
-            mbar_init(bar_cempty + 8 * i, 4 * (KPS < kTaGroups ? KPS : kTaGroups));
+            mbar_init(bar_cempty + 8 * i, 4 * (KPS < GROUPS ? KPS : GROUPS));
         }
         for (int i = 0; i < p.nx; i++) {
             mbar_init(bar_xfull + 8 * i, 1);
@@ -238,7 +248,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
         fence_async_smem();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TCOLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -408,7 +418,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
         }
     } else if (warp >= 8) {
         // ================= dequantisers =================
-        // Group g converts the steps whose number, counted over all tiles of the CTA, is g modulo 4, a thread per weight row
+        // Group g converts the steps whose number, counted over all tiles of the CTA, is g modulo GROUPS, a thread per weight row
         // (never by the step's number in its tile: a group that skips the end of a tile would wait on an A stage more than
         // one round ahead, which a phase bit cannot tell from this round). One warp's step is a chain of latencies
         // (barrier, shared-memory round trip, conversion, tensor-memory store and its completion, about 1000 cycles); four
@@ -425,14 +435,14 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
         bool ok = true;
         for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
             for (int ch = 0; ch < chunks; ch++) {
-                const int j0 = (grp - (int)it0 - ch * KPS) & (kTaGroups - 1);  // this group's first step of the stage
+                const int j0 = (grp - (int)it0 - ch * KPS) & (GROUPS - 1);  // this group's first step of the stage
                 if (j0 < KPS) {  // (8-bit codes have two steps per stage: two groups take it)
                     ok = __all_sync(0xffffffffu, mbar_wait(bar_cfull + 8 * cs, cph, abort_flag));
                     if (!ok) break;
                     const uint32_t codes = codes0 + cs * kTaCodeStage + row * 128, scales = scales0 + cs * SSTAGE + row * SPB;
 #pragma unroll
-                    for (int i = 0; i < (KPS + kTaGroups - 1) / kTaGroups; i++) {
-                        const int j = j0 + kTaGroups * i;
+                    for (int i = 0; i < (KPS + GROUPS - 1) / GROUPS; i++) {
+                        const int j = j0 + GROUPS * i;
                         const int ks = ch * KPS + j;
                         if (ks >= ksteps) break;
                         const uint32_t it = it0 + ks, as = it & (na - 1), aph = (it >> nash) & 1;
@@ -566,7 +576,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) qmm_ta_kernel(const __grid_cons
     if (*abort_flag && threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, kErrTimeout);
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
     }
 }
 

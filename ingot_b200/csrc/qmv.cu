@@ -359,6 +359,8 @@ QgKernel qg_pick(int mode, int ms, bool tm, bool gw4, bool fx = false) {
     if (mode == kModeGateUp) return tm ? qg_pick_mt<kModeGateUp, true>(ms, gw4) : qg_pick_mt<kModeGateUp, false>(ms, gw4);
     return tm ? qg_pick_mt<kModeDown, true>(ms, gw4) : qg_pick_mt<kModeDown, false>(ms, gw4);
 }
+}  // namespace
+
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     if ((c.mode != kModeGateUp && c.mode != kModeDown) || c.tiles == nullptr || c.fmt != kFmtAffine4) return 1;
@@ -459,8 +461,6 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, ms, tm, gw4 && p.wk == kQgWarps, fx), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
 }
 
-}  // namespace
-
 int32_t gqmv_init(iq_ctx* ctx) {
 #define IQ_QI_ALL(F)                                                                                           \
     reinterpret_cast<const void*>(qmv_imma_kernel<F, 1, 0>), reinterpret_cast<const void*>(qmv_imma_kernel<F, 1, 4>), \
@@ -516,8 +516,6 @@ int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     int32_t r = launch_qmv_imma(ctx, st, c);
     if (r != 1) return r;
     r = launch_qmv_direct(ctx, st, c);
-    if (r != 1) return r;
-    r = launch_qmv_imma_grouped(ctx, st, c);
     if (r != 1) return r;
     r = launch_qmv_stream(ctx, st, c);
     if (r != 1) return r;
