@@ -1,4 +1,4 @@
-// Bandwidth-bound quantized GEMV family ("qmv" / decode "gather_qmv"): Y[M<=16, N] = X[M, K] * W^T with W in MLX affine
+// Bandwidth-bound quantized GEMV family ("qmv"): Y[M<=16, N] = X[M, K] * W^T with W in MLX affine
 // 4/8-bit (group 64) or MXFP4 (group 32) format, read once from HBM with 128-bit loads and dequantised in registers.
 //
 // One warp owns 16 consecutive output rows of W and a slice of K. Each lane streams 16-byte pieces ("chunks") of two
@@ -13,9 +13,8 @@
 // fixed warp order, which makes a row's bits independent of the other rows (the reference's row-invariance property,
 // Tests/IngotTests/KernelCaseTests.swift:68-86).
 //
-// Replaces the reference's decode kernels vnax_qmv_nf1_sg32 / fn_qmv8_nf1 / vqmv_* (Shaders/verify_nax.metal:105-209,
-// Shaders/verify.metal:89-155) and, through the tile list, vnax_moe_gateup* / vnax_moe_down_split*
-// (Shaders/verify_nax.metal:258-509).
+// Runs where the inputs are too wide for the other kernels of the family (affine: beyond some 25000). Replaces the reference's
+// decode kernels vnax_qmv_nf1_sg32 / fn_qmv8_nf1 / vqmv_* (Shaders/verify_nax.metal:105-209, Shaders/verify.metal:89-155).
 #pragma once
 
 #include "common.cuh"
@@ -31,29 +30,21 @@ struct Tile {
 enum : int { kModePlain = 0, kModeGateUp = 1, kModeDown = 2 };
 
 struct GqmvParams {
-    // weights: [0] = the matrix (plain / down) or gate; [1] = up (gate/up mode only)
+    // weights: [0] = the matrix (plain) or gate; [1] = up (gate/up mode only)
     const uint32_t* w[2];
     const void* s[2];
     const void* b[2];
-    int64_t w_estride;  // uint32 words between experts
-    int64_t s_estride;  // scale elements between experts
-    int32_t N, K;       // output rows per expert, inputs
+    int32_t N, K;       // output rows, inputs
     // activations
     const void* x;
     int32_t x_dtype;
     int64_t ldx;
-    const uint32_t* row_map;  // gate/up: sorted position -> pair id (token = pair / topk); null: rows are in place
-    int32_t topk;
-    // work list
-    const Tile* tiles;       // null: one tile {0, 0, M}
-    const uint32_t* ntiles;  // device count of valid tiles
     int32_t M;
     // outputs
     void* y;
     int32_t y_dtype;
     int64_t ldy;
     int32_t accumulate;
-    const float* ebias[2];  // expert biases fp32 [E, N] (gate/up: gate and up; down: [0]) or null
     float limit;            // swiglu_oai clamp
     int32_t act;            // gate/up mode: activation (kAct*)
     // K tiling (host-chosen): K is walked in tiles of `kt` inputs, kt a multiple of 512
@@ -171,16 +162,8 @@ __global__ void __launch_bounds__(RG* WK * 32) gqmv_kernel(const GqmvParams p) {
     constexpr int U = NW == 2 ? 1 : 2;  // steps per register batch
     extern __shared__ __align__(16) unsigned char smem[];
 
-    // ---- which tile ------------------------------------------------------------------------------------------
-    Tile tile;
-    if (p.tiles != nullptr) {
-        if (blockIdx.y >= *p.ntiles) return;
-        tile = p.tiles[blockIdx.y];
-    } else {
-        tile.expert = 0; tile.start = 0; tile.count = (uint32_t)p.M; tile.pad = 0;
-    }
-    const int M = (int)tile.count;  // live activation rows (1 .. 8 * MH)
-    const int MR = M;               // rows of the staged x block
+    const int M = p.M;   // live activation rows (1 .. 8 * MH)
+    const int MR = M;    // rows of the staged x block
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rg = warp / WK, wk = warp % WK;
@@ -202,12 +185,12 @@ __global__ void __launch_bounds__(RG* WK * 32) gqmv_kernel(const GqmvParams p) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int64_t r = rows_ok ? (n0 + g + 8 * h) : 0;
-            wrow[i][h] = reinterpret_cast<const uint4*>(p.w[i] + tile.expert * p.w_estride + r * row_words);
+            wrow[i][h] = reinterpret_cast<const uint4*>(p.w[i] + r * row_words);
             srow[i][h] = reinterpret_cast<const unsigned char*>(p.s[i]) +
-                         (tile.expert * p.s_estride + r * row_groups) * (FMT == kFmtMxfp4 ? 1 : 2);
+                         r * row_groups * (FMT == kFmtMxfp4 ? 1 : 2);
             brow[i][h] = FMT == kFmtMxfp4 ? srow[i][h]
                                           : reinterpret_cast<const unsigned char*>(p.b[i]) +
-                                                (tile.expert * p.s_estride + r * row_groups) * 2;
+                                                r * row_groups * 2;
         }
 
     float acc[NW][MH][4];
@@ -310,10 +293,7 @@ __global__ void __launch_bounds__(RG* WK * 32) gqmv_kernel(const GqmvParams p) {
                 float v[8];
                 const bool live = uidx < total;
                 if (live) {
-                    size_t row;
-                    if (MODE == kModeGateUp && p.row_map != nullptr) row = p.row_map[tile.start + m] / (uint32_t)p.topk;
-                    else row = (size_t)tile.start + m;
-                    load_x8(p.x, p.x_dtype, row * p.ldx + k0 + ku * 8, v);
+                    load_x8(p.x, p.x_dtype, (size_t)m * p.ldx + k0 + ku * 8, v);
                 } else {
 #pragma unroll
                     for (int e = 0; e < 8; e++) v[e] = 0.f;
@@ -383,16 +363,9 @@ __global__ void __launch_bounds__(RG* WK * 32) gqmv_kernel(const GqmvParams p) {
             if (m >= M) continue;
             float v = acc[0][h][e];
             if (MODE == kModeGateUp) {
-                float u = acc[NW - 1][h][e];
-                if (p.ebias[0] != nullptr) {
-                    v += p.ebias[0][(size_t)tile.expert * p.N + n];
-                    u += p.ebias[1][(size_t)tile.expert * p.N + n];
-                }
-                v = glu_rt(p.act, v, u, p.limit);
-            } else if (MODE == kModeDown) {
-                if (p.ebias[0] != nullptr) v += p.ebias[0][(size_t)tile.expert * p.N + n];
+                v = glu_rt(p.act, v, acc[NW - 1][h][e], p.limit);
             }
-            const size_t o = (size_t)(tile.start + m) * p.ldy + n;
+            const size_t o = (size_t)m * p.ldy + n;
             if (p.y_dtype == kF32) {
                 float* yp = reinterpret_cast<float*>(p.y) + o;
                 *yp = p.accumulate ? *yp + v : v;

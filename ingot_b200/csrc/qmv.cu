@@ -37,7 +37,6 @@ template <int FMT, int MH>
 GqmvKernel pick_mode(int mode, int wk) {
     switch (mode) {
         case kModeGateUp: return pick_cfg<FMT, MH, kModeGateUp>(wk);
-        case kModeDown: return pick_cfg<FMT, MH, kModeDown>(wk);
         default: return pick_cfg<FMT, MH, kModePlain>(wk);
     }
 }
@@ -62,21 +61,9 @@ constexpr int kSmemBudget = 200 * 1024;
 // ---- streaming (TMA ring) path --------------------------------------------------------------------------------------
 typedef void (*QsKernel)(const QsParams);
 
-template <int FMT, int MH>
-QsKernel qs_pick_mode(int mode) {
-    switch (mode) {
-        case kModeGateUp: return qmv_stream_kernel<FMT, MH, kModeGateUp>;
-        case kModeDown: return qmv_stream_kernel<FMT, MH, kModeDown>;
-        default: return qmv_stream_kernel<FMT, MH, kModePlain>;
-    }
-}
-QsKernel qs_pick(int32_t fmt, int mh, int mode) {
-    switch (fmt) {
-        case kFmtAffine4: return mh == 2 ? qs_pick_mode<kFmtAffine4, 2>(mode) : qs_pick_mode<kFmtAffine4, 1>(mode);
-        case kFmtAffine8: return mh == 2 ? qs_pick_mode<kFmtAffine8, 2>(mode) : qs_pick_mode<kFmtAffine8, 1>(mode);
-        case kFmtMxfp4: return mh == 2 ? qs_pick_mode<kFmtMxfp4, 2>(mode) : qs_pick_mode<kFmtMxfp4, 1>(mode);
-        default: return nullptr;
-    }
+QsKernel qs_pick(int mh, int mode) {
+    if (mode == kModeGateUp) return mh == 2 ? qmv_stream_kernel<2, kModeGateUp> : qmv_stream_kernel<1, kModeGateUp>;
+    return mh == 2 ? qmv_stream_kernel<2, kModePlain> : qmv_stream_kernel<1, kModePlain>;
 }
 constexpr int kQsSmemMax = 226 * 1024;
 
@@ -84,27 +71,19 @@ constexpr int kQiCtasPerSm = 2;  // up to four rows: two CTAs per SM (one CTA wi
 
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_stream(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
-    if (c.fmt == kFmtAffine4G32 || c.fmt == kFmtAffine6) return 1;  // not this kernel's formats
-    const bool has_bias = c.fmt != kFmtMxfp4;
+    if (c.fmt != kFmtMxfp4) return 1;
     const int nw = c.mode == kModeGateUp ? 2 : 1;
     const int mh = c.max_rows > 8 ? 2 : 1;
-    const int ck = c.fmt == kFmtAffine8 ? 16 : 32;
-    const int qu = ck == 32 ? 4 : 2;
-    const int row_bytes = c.fmt == kFmtAffine8 ? c.K : c.K / 2;
-    const int srow_bytes = c.fmt == kFmtMxfp4 ? c.K / 32 : c.K / 64 * 2;
-    const int per_row = row_bytes + srow_bytes * (has_bias ? 2 : 1);
-    for (int i = 0; i < nw; i++) {
-        if ((reinterpret_cast<uintptr_t>(c.w[i] ? c.w[i] : c.w[0]) & 15) || (reinterpret_cast<uintptr_t>(c.s[i] ? c.s[i] : c.s[0]) & 15) ||
-            (has_bias && (reinterpret_cast<uintptr_t>(c.b[i] ? c.b[i] : c.b[0]) & 15)))
-            return 1;
-    }
+    const int row_bytes = c.K / 2, srow_bytes = c.K / 32, per_row = row_bytes + srow_bytes;
+    for (int i = 0; i < nw; i++)
+        if ((reinterpret_cast<uintptr_t>(c.w[i]) & 15) || (reinterpret_cast<uintptr_t>(c.s[i]) & 15)) return 1;
     int rgs = 1;
     while (rgs < 8 && 16 * rgs * per_row * nw < 24 * 1024 && 16 * rgs * 2 <= c.N) rgs *= 2;
     const int R = 16 * rgs;
     const int mat_bytes = round_up(R * per_row, 128);
     const int stage_bytes = nw * mat_bytes;
     const int nsteps = (row_bytes / 16 + 3) / 4;
-    const int xs_bytes = round_up(nsteps * qu * c.max_rows * 4 * 16, 128);
+    const int xs_bytes = round_up(nsteps * 4 * c.max_rows * 4 * 16, 128);
     const int red_bytes = 2 * 8 * nw * mh * 4 * 32 * 4;
     const int fixed = xs_bytes + red_bytes + 256;  // + barriers, abort flag, zero block
     if (stage_bytes > 80 * 1024) return 1;
@@ -117,23 +96,16 @@ int32_t launch_qmv_stream(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     }
     if (nstages < 2) return 1;
     if (nstages > 8) nstages = 8;
-    QsKernel k = qs_pick(c.fmt, mh, c.mode);
-    if (k == nullptr) return 1;
 
     QsParams p;
     memset(&p, 0, sizeof(p));
     for (int i = 0; i < 2; i++) {
         p.w[i] = reinterpret_cast<const unsigned char*>(c.w[i] ? c.w[i] : c.w[0]);
         p.s[i] = reinterpret_cast<const unsigned char*>(c.s[i] ? c.s[i] : c.s[0]);
-        p.b[i] = reinterpret_cast<const unsigned char*>(c.b[i] ? c.b[i] : c.b[0]);
-        p.ebias[i] = c.ebias[i];
     }
-    p.w_ebytes = c.w_estride * 4;
-    p.s_ebytes = c.s_estride * (c.fmt == kFmtMxfp4 ? 1 : 2);
     p.N = c.N; p.K = c.K;
     p.x = c.x; p.x_dtype = c.x_dtype; p.ldx = c.ldx;
-    p.row_map = c.row_map; p.topk = c.topk;
-    p.tiles = c.tiles; p.ntiles = c.ntiles; p.M = c.rows;
+    p.M = c.rows;
     p.y = c.y; p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
     p.limit = c.limit;
     p.act = c.act;
@@ -143,21 +115,9 @@ int32_t launch_qmv_stream(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     p.xs_bytes = xs_bytes; p.red_bytes = red_bytes;
     p.status = ctx->d_status;
 
-    const int64_t items = (int64_t)p.NB * c.grid_tiles;
-    const int64_t slots = (int64_t)ctx->sms * ctas_per_sm;
-    const int grid = (int)(items < slots ? items : slots);
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(kQsThreads, 1, 1);
-    cfg.dynamicSmemBytes = fixed + nstages * stage_bytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, k, p), "qmv_stream launch");
+    const int slots = ctx->sms * ctas_per_sm;
+    return check_cuda(ctx, launch_dependent(qs_pick(mh, c.mode), dim3(p.NB < slots ? p.NB : slots), kQsThreads,
+                                            (size_t)(fixed + nstages * stage_bytes), st, p), "qmv_stream launch");
 }
 
 // The tail split's scratch slot of a stream: launches of one stream run in series (a dependent launch waits for its
@@ -175,7 +135,7 @@ int tail_slot_of(iq_ctx* ctx, cudaStream_t st) {
 // ---- int8 tensor-core path (decode, up to four rows, affine codes) -----------------------------------------------
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
-    if (c.mode != kModePlain || c.tiles != nullptr || c.rows > 16 || c.rows < 1) return 1;
+    if (c.mode != kModePlain || c.rows > 16 || c.rows < 1) return 1;
     if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine8 && c.fmt != kFmtAffine6) return 1;
     if (c.K % 2048 != 0 || c.N < kQiRows) return 1;
     if ((reinterpret_cast<uintptr_t>(c.w[0]) & 15) || (reinterpret_cast<uintptr_t>(c.s[0]) & 15) ||
@@ -310,7 +270,7 @@ QdKernel qd_pick(int32_t fmt, int nw, int ms, bool vec) {
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error. The choice looks
 // at the matrix alone, not at the row count.
 int32_t launch_qmv_direct(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
-    if (c.tiles != nullptr || c.mode == kModeDown || c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0) return 1;
+    if (c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0) return 1;
     if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;
     const int nw = c.mode == kModeGateUp ? 2 : 1, gs = c.fmt == kFmtAffine4G32 ? 32 : 64, G = c.K / gs;
     const int per = qd_batch(c.fmt == kFmtAffine8, nw);  // groups per batch
@@ -348,23 +308,22 @@ int32_t launch_qmv_direct(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
 
 // ---- int8 tensor-core path for the MoE decode tiles (gate/up + activation, down; affine 4-bit experts) ---------------
 typedef void (*QgKernel)(const CUtensorMap, const CUtensorMap, const QgParams);
-// gw4: each consumer warp's K slice is four groups, its activation fragments stay in registers (8-row tiles only)
+// gw4: each consumer warp's K slice is four groups, its activation fragments stay in registers
 template <int MODE, bool TM>
-QgKernel qg_pick_mt(int ms, bool gw4) {
-    if (ms == 4) return qmv_imma_grouped_kernel<MODE, 4, TM, 0, 8>;
-    return gw4 ? qmv_imma_grouped_kernel<MODE, 2, TM, 4, 8> : qmv_imma_grouped_kernel<MODE, 2, TM, 0, 8>;
+QgKernel qg_pick_mt(bool gw4) {
+    return gw4 ? qmv_imma_grouped_kernel<MODE, TM, 4, 8> : qmv_imma_grouped_kernel<MODE, TM, 0, 8>;
 }
-QgKernel qg_pick(int mode, int ms, bool tm, bool gw4, bool fx = false) {
-    if (fx) return qmv_imma_grouped_kernel<kModeGateUp, 2, true, 4, 16>;
-    if (mode == kModeGateUp) return tm ? qg_pick_mt<kModeGateUp, true>(ms, gw4) : qg_pick_mt<kModeGateUp, false>(ms, gw4);
-    return tm ? qg_pick_mt<kModeDown, true>(ms, gw4) : qg_pick_mt<kModeDown, false>(ms, gw4);
+QgKernel qg_pick(int mode, bool tm, bool gw4, bool fx = false) {
+    if (fx) return qmv_imma_grouped_kernel<kModeGateUp, true, 4, 16>;
+    if (mode == kModeGateUp) return tm ? qg_pick_mt<kModeGateUp, true>(gw4) : qg_pick_mt<kModeGateUp, false>(gw4);
+    return tm ? qg_pick_mt<kModeDown, true>(gw4) : qg_pick_mt<kModeDown, false>(gw4);
 }
 }  // namespace
 
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     if ((c.mode != kModeGateUp && c.mode != kModeDown) || c.tiles == nullptr || c.fmt != kFmtAffine4) return 1;
-    if (c.K % 64 != 0 || c.N % 16 != 0 || c.max_rows > 16 || c.accumulate) return 1;
+    if (c.K % 64 != 0 || c.N % 16 != 0 || c.max_rows > 8 || c.accumulate) return 1;
     const int nw = c.mode == kModeGateUp ? 2 : 1;
     for (int i = 0; i < nw; i++)
         if ((reinterpret_cast<uintptr_t>(c.w[i]) & 15) || (reinterpret_cast<uintptr_t>(c.s[i]) & 15) ||
@@ -382,23 +341,23 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     const bool tm = ctx->encode_tiled != nullptr && c.expert_count > 0 && p.row_bytes % 128 == 0 && p.row_bytes / 128 <= 256 &&
                     c.w_estride * 4 == (int64_t)c.N * p.row_bytes;
     if (c.K < 2048 && !tm) return 1;
-    const int ms = c.max_rows > 8 ? 4 : 2;
+    constexpr int ms = 2;  // sets of four activation rows per tile
     p.row_pitch = tm ? p.row_bytes : p.row_bytes + 32;
     p.srow_bytes = G * 2;
     p.xq_bytes = G * ms * 512;
     p.xsc_bytes = G * ms * 32;
     // Sixteen consumer warps with the token rows as fixed point: K slices of four groups that divide them (K = 1024, 2048,
     // 4096), gate/up tiles of eight rows
-    const bool fx = c.fx != nullptr && c.mode == kModeGateUp && ms == 2 && tm && c.row_map != nullptr && G % 4 == 0 && G / 4 <= 16 && 16 % (G / 4) == 0;
+    const bool fx = c.fx != nullptr && c.mode == kModeGateUp && tm && c.row_map != nullptr && G % 4 == 0 && G / 4 <= 16 && 16 % (G / 4) == 0;
     const int kQgWarps = fx ? 16 : 8;
     if (fx) { p.fx = *c.fx; p.xq_bytes = p.xsc_bytes = 0; }
     p.red_bytes = 2 * kQgWarps * nw * ms * 64 * 4;
     const int fixed = p.xq_bytes + p.xsc_bytes + p.red_bytes + 256 + (tm ? 1024 : 0);
-    // K slices per block of rows. 8-row tiles: one slice of four groups per warp when K allows it (the activation
+    // K slices per block of rows: one slice of four groups per warp when K allows it (the activation
     // fragments then live in registers: 69 against 83 us on the 64-token layer); else four slices (32-row blocks: half as
     // many hand-overs per byte) when two stages of that size fit, else eight.
     int ctas = 1, nstages = 0;
-    const bool gw4 = ms == 2 && (fx || G == 4 * kQgWarps);
+    const bool gw4 = fx || G == 4 * kQgWarps;
     const int cand[4] = {fx ? G / 4 : (gw4 ? kQgWarps : kQgWarps / 2), kQgWarps, kQgWarps / 4, kQgWarps / 8};
     for (int ci = 0; ci < (fx ? 1 : 4) && nstages < 2; ci++) {
         const int wk = cand[ci];
@@ -458,7 +417,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, ms, tm, gw4 && p.wk == kQgWarps, fx), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, gw4 && p.wk == kQgWarps, fx), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
 }
 
 int32_t gqmv_init(iq_ctx* ctx) {
@@ -474,13 +433,13 @@ int32_t gqmv_init(iq_ctx* ctx) {
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma)");
     }
     {
-        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(kModeGateUp, 2, true, true, true)),
+        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(kModeGateUp, true, true, true)),
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
     }
     for (int mode = kModeGateUp; mode <= kModeDown; mode++)
-        for (int v = 0; v < 6; v++) {  // 4 row sets, 2, 2 with register-resident activations; bulk or tensor copies
-            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(mode, v % 3 == 0 ? 4 : 2, v >= 3, v % 3 == 2)),
+        for (int v = 0; v < 4; v++) {  // bulk or tensor copies; activations in registers or not
+            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(mode, v >= 2, v % 2 == 1)),
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
         }
@@ -492,27 +451,26 @@ int32_t gqmv_init(iq_ctx* ctx) {
     }
     for (int fmt = 0; fmt < 4; fmt++)
         for (int mh = 1; mh <= 2; mh++)
-            for (int mode = 0; mode < 3; mode++)
+            for (int mode = kModePlain; mode <= kModeGateUp; mode++)
                 for (int wk = 2; wk <= 8; wk *= 2) {
                     GqmvKernel k = pick(fmt, mh, mode, wk);
                     cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k),
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 20480);
                     if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(gqmv)");
                 }
-    for (int fmt = 0; fmt < 3; fmt++)
-        for (int mh = 1; mh <= 2; mh++)
-            for (int mode = 0; mode < 3; mode++) {
-                cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qs_pick(fmt, mh, mode)),
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
-                if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_stream)");
-            }
+    for (int mh = 1; mh <= 2; mh++)
+        for (int mode = kModePlain; mode <= kModeGateUp; mode++) {
+            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qs_pick(mh, mode)),
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
+            if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_stream)");
+        }
     return kOk;
 }
 
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     // One kernel per (format, shape), chosen from the matrix alone: for affine codes the int8 tensor-core kernels (staged
-    // where K fits the staging, else with the weights in registers), the streaming fp16 kernel for MXFP4 and the remaining
-    // expert tiles, the register-staged fp16 kernel where a 16-row block over the whole K does not fit a stage.
+    // where K fits the staging, else with the weights in registers), the streaming fp16 kernel for MXFP4, the register-staged
+    // fp16 kernel where K is too wide for either.
     int32_t r = launch_qmv_imma(ctx, st, c);
     if (r != 1) return r;
     r = launch_qmv_direct(ctx, st, c);
@@ -542,7 +500,7 @@ int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
 
     // K slices per CTA: the fewest that still fill the GPU, keeping at least two steps per warp
     const int nsteps = (kt / ck + 3) / 4;
-    const int64_t row_groups = (int64_t)(c.N / 16) * c.grid_tiles;
+    const int64_t row_groups = c.N / 16;
     const int64_t target = (int64_t)ctx->sms * 24;
     int wk = 2;
     while (wk < 8 && row_groups * wk < target && nsteps / (wk * 2) >= 2) wk *= 2;
@@ -556,19 +514,16 @@ int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
         p.w[i] = c.w[i] ? c.w[i] : c.w[0];
         p.s[i] = c.s[i] ? c.s[i] : c.s[0];
         p.b[i] = c.b[i] ? c.b[i] : c.b[0];
-        p.ebias[i] = c.ebias[i];
     }
-    p.w_estride = c.w_estride; p.s_estride = c.s_estride;
     p.N = c.N; p.K = c.K;
     p.x = c.x; p.x_dtype = c.x_dtype; p.ldx = c.ldx;
-    p.row_map = c.row_map; p.topk = c.topk;
-    p.tiles = c.tiles; p.ntiles = c.ntiles; p.M = c.rows;
+    p.M = c.rows;
     p.y = c.y; p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
     p.limit = c.limit;
     p.act = c.act;
     p.kt = kt; p.xs_bytes = xs_bytes;
 
-    dim3 grid((c.N / 16 + rg - 1) / rg, c.grid_tiles, 1);
+    dim3 grid((c.N / 16 + rg - 1) / rg);
     k<<<grid, 256, smem, st>>>(p);
     return check_cuda(ctx, cudaGetLastError(), "gqmv launch");
 }

@@ -1,5 +1,5 @@
 // MoE decode on the int8 tensor-core path: the expert tiles' gate + up + activation and down projections for tiles of
-// up to 16 routed rows (affine 4-bit experts). Same arithmetic as qmv_imma.cuh: codes enter m16n8k32 u8 x s8 MMAs
+// up to eight routed rows (affine 4-bit experts). Same arithmetic as qmv_imma.cuh: codes enter m16n8k32 u8 x s8 MMAs
 // unconverted, the tile's activation rows are converted once per tile to block fixed point (two signed 7-bit digits per
 // group of 64 inputs), per group y += s * 2^(e-13) * (128 * acc_hi + acc_lo) + b * sum(x); a row's bits do not depend on
 // the other rows of its tile.
@@ -11,8 +11,8 @@
 // next item, and four epilogue warps add them up, apply the activation and store, one item behind (hand-over through
 // named barriers: buffer full, buffer free), so that no item waits for a barrier of the whole CTA.
 //
-// Replaces the reference's vnax_moe_gateup* / vnax_moe_down_split* decode kernels (Shaders/verify_nax.metal:258-509)
-// where the fp16 tile kernels of qmv_stream.cuh ran before; those still serve MXFP4 experts and odd shapes. The down
+// Replaces the reference's vnax_moe_gateup* / vnax_moe_down_split* decode kernels (Shaders/verify_nax.metal:258-509).
+// MXFP4 experts and shapes that do not fit run on the grouped GEMM. The down
 // projection of a narrow expert (K = 768) runs here as 128-row blocks without a K split.
 #pragma once
 
@@ -64,7 +64,7 @@ struct QgParams {
     int32_t* status;
 };
 
-// MODE: kModeGateUp (two matrices, h = act(gate, up)) or kModeDown; MS: sets of four activation rows per tile (2 or 4).
+// MODE: kModeGateUp (two matrices, h = act(gate, up)) or kModeDown.
 // TM: a block of R rows of a matrix arrives as one swizzled tensor copy, laid out [128-byte column][row][128] (see
 // qmv_imma.cuh), instead of one bulk copy per row: expert rows are 384 to 1024 bytes, and copies that short are bound by
 // their issue rate (one producer warp sustains about one per 60 ns), not by their bytes.
@@ -75,10 +75,11 @@ struct QgParams {
 // of converting them per CTA and tile: the conversion's shared memory goes to the ring, its instructions away, and with
 // twice the warps per scheduler the latencies of a warp's chain (shared-memory loads, shuffles, MMAs, the hand-over) hide
 // behind one another: eight warps issued 0.43 instructions per cycle and scheduler.
-template <int MODE, int MS, bool TM, int GW, int NCW>
+template <int MODE, bool TM, int GW, int NCW>
 __global__ void __launch_bounds__(qg_threads(NCW), 1)
     qmv_imma_grouped_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, const QgParams p) {
     constexpr int NW = MODE == kModeGateUp ? 2 : 1;
+    constexpr int MS = 2;   // sets of four activation rows per tile
     constexpr int GB = 32;  // code bytes per group of 64 inputs (4-bit)
     constexpr int kQgWarps = NCW;
     constexpr bool FX = NCW == 16;
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
                 w[j] = 0;
                 if (j < tpl && ti < ntl) {
                     const int sets = (min((int)p.tiles[ti].count, 4 * MS) + 3) >> 2;
-                    w[j] = 3 + (sets > 2 ? 4 : sets);
+                    w[j] = 3 + sets;
                 }
                 mine += w[j];
             }
@@ -445,8 +446,7 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
                 }
             };
             if (ok && rows_ok) {
-                if (MS == 4 && sets > 2) body(std::integral_constant<int, MS>{});
-                else if (sets > 1) body(std::integral_constant<int, 2>{});
+                if (sets > 1) body(std::integral_constant<int, 2>{});
                 else body(std::integral_constant<int, 1>{});
             }
             __syncwarp();
