@@ -84,6 +84,7 @@ int32_t make_map_rowblock(iq_ctx* ctx, CUtensorMap* map, const void* base, uint6
                           uint32_t box_rows);
 // The same through the context's cache, copied into *out; an error code (with the message recorded) when the encoding fails.
 int32_t cached_rowblock_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, int32_t box_rows, CUtensorMap* out);
+int32_t cached_rows16_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, CUtensorMap* out);
 
 struct Tile;
 struct FixedRows;

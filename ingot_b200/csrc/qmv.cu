@@ -5,11 +5,13 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "gqmv.cuh"
 #include "internal.h"
-#include "qmv_direct.cuh"
 #include "qmv_imma.cuh"
 #include "qmv_imma_grouped.cuh"
+#include "qmv_ring.cuh"
 #include "qmv_stream.cuh"
 
 namespace iq {
@@ -249,59 +251,86 @@ int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     return kOk;
 }
 
-// ---- int8 tensor-core path with the weights loaded straight into registers: the plain GEMVs the staged kernel refuses, and the
-// dense FFN's gate + up ---------------------------------------------------------------------------------------------
-typedef void (*QdKernel)(const QdParams);
+// ---- int8 tensor-core path with a ring of weights per warp: the plain GEMVs the staged kernel refuses, and the dense FFN's
+// gate + up ---------------------------------------------------------------------------------------------------------
+typedef void (*QrKernel)(const QrMaps, const QrParams);
 template <int FMT, int NW>
-QdKernel qd_pick_mv(int ms, bool vec) {
-    if (ms == 2) return vec ? qmv_direct_kernel<FMT, 2, NW, true> : qmv_direct_kernel<FMT, 2, NW, false>;
-    return vec ? qmv_direct_kernel<FMT, 1, NW, true> : qmv_direct_kernel<FMT, 1, NW, false>;
+QrKernel qr_pick_mv(int ms, bool vec) {
+    if (ms == 4) return vec ? qmv_ring_kernel<FMT, 4, NW, true> : qmv_ring_kernel<FMT, 4, NW, false>;
+    if (ms == 2) return vec ? qmv_ring_kernel<FMT, 2, NW, true> : qmv_ring_kernel<FMT, 2, NW, false>;
+    return vec ? qmv_ring_kernel<FMT, 1, NW, true> : qmv_ring_kernel<FMT, 1, NW, false>;
 }
-QdKernel qd_pick(int32_t fmt, int nw, int ms, bool vec) {
-    switch (fmt) {
-        case kFmtAffine4: return nw == 2 ? qd_pick_mv<kFmtAffine4, 2>(ms, vec) : qd_pick_mv<kFmtAffine4, 1>(ms, vec);
-        case kFmtAffine4G32: return nw == 2 ? qd_pick_mv<kFmtAffine4G32, 2>(ms, vec) : qd_pick_mv<kFmtAffine4G32, 1>(ms, vec);
-        case kFmtAffine8:
-            if (nw == 2) return ms == 2 ? qmv_direct_kernel<kFmtAffine8, 2, 2, false> : qmv_direct_kernel<kFmtAffine8, 1, 2, false>;
-            return qd_pick_mv<kFmtAffine8, 1>(ms, vec);
-        default: return nullptr;
+template <int FMT>
+QrKernel qr_pick_f(int nw, int ms, bool vec) { return nw == 2 ? qr_pick_mv<FMT, 2>(ms, vec) : qr_pick_mv<FMT, 1>(ms, vec); }
+QrKernel qr_pick(int32_t fmt, int nw, int ms, bool vec) {
+    return fmt == kFmtAffine8 ? qr_pick_f<kFmtAffine8>(nw, ms, vec)
+         : fmt == kFmtAffine4G32 ? qr_pick_f<kFmtAffine4G32>(nw, ms, vec) : qr_pick_f<kFmtAffine4>(nw, ms, vec);
+}
+// How a matrix is split, whatever the rows of the call (a row's bits must not depend on them).
+struct QrPlan {
+    int ms;      // sets of four rows a launch can take
+    int warps, wk;
+};
+QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms) {
+    QrPlan best = {0, 0, 0};
+    // as many row sets as fit beside at least two slots per warp, then as many warps
+    for (int ms = 4; ms >= 1 && best.ms == 0; ms /= 2)
+        for (int w = kQrMaxWarps; w >= (ms > 1 ? 8 : 4); w -= 4)
+            if (qr_smem(fmt, K, nw, ms, vec, w, 2) <= (size_t)kQsSmemMax) { best.ms = ms; best.warps = w; break; }
+    if (best.ms == 0) return best;
+    // K slices: the least (rounds of a CTA) x (columns of a warp in a round + the round's own cost, about one column's)
+    const int gpc = qr_groups(fmt), G = K / (fmt == kFmtAffine4G32 ? 32 : 64), ncol = (G + gpc - 1) / gpc, nblk = N / 16;
+    long long cost = -1;
+    for (int wk = best.warps; wk >= 1; wk--) {
+        if (best.warps % wk != 0 || wk > ncol) continue;
+        const long long per = (long long)(best.warps / wk) * sms, rounds = (nblk + per - 1) / per, c = rounds * ((ncol + wk - 1) / wk + 1);
+        if (cost < 0 || c < cost) { cost = c; best.wk = wk; }
     }
+    return best;
 }
-// Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error. The choice looks
-// at the matrix alone, not at the row count.
-int32_t launch_qmv_direct(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
-    if (c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0) return 1;
+// Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
+int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
+    if (c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0 || ctx->encode_tiled == nullptr) return 1;
     if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;
-    const int nw = c.mode == kModeGateUp ? 2 : 1, gs = c.fmt == kFmtAffine4G32 ? 32 : 64, G = c.K / gs;
-    const int per = qd_batch(c.fmt == kFmtAffine8, nw);  // groups per batch
-    bool vec = per > 1 && G % per == 0;
-    QdParams p;
+    const int nw = c.mode == kModeGateUp ? 2 : 1, gpc = qr_groups(c.fmt), G = c.K / (c.fmt == kFmtAffine4G32 ? 32 : 64);
+    bool vec = G % gpc == 0;
+    QrParams p;
     memset(&p, 0, sizeof(p));
-    for (int i = 0; i < 2; i++) {
-        p.w[i] = reinterpret_cast<const unsigned char*>(c.w[i] ? c.w[i] : c.w[0]);
-        p.s[i] = reinterpret_cast<const unsigned char*>(c.s[i] ? c.s[i] : c.s[0]);
-        p.b[i] = reinterpret_cast<const unsigned char*>(c.b[i] ? c.b[i] : c.b[0]);
-        if (reinterpret_cast<uintptr_t>(p.w[i]) & 15) return 1;
-        if ((reinterpret_cast<uintptr_t>(p.s[i]) | reinterpret_cast<uintptr_t>(p.b[i])) & (uintptr_t)(2 * per - 1)) vec = false;
+    for (int i = 0; i < nw; i++) {
+        p.s[i] = static_cast<const unsigned char*>(c.s[i]);
+        p.b[i] = static_cast<const unsigned char*>(c.b[i]);
+        const uintptr_t sb = reinterpret_cast<uintptr_t>(p.s[i]) | reinterpret_cast<uintptr_t>(p.b[i]);
+        if ((reinterpret_cast<uintptr_t>(c.w[i]) & 15) || (sb & 3)) return 1;
+        if (sb & (uintptr_t)(2 * gpc - 1)) vec = false;
     }
-    auto smem_for = [&](int ms) { return G * ms * 32 * (gs / 4) + G * ms * 32 + 2 * kQdWarps * nw * ms * 256; };
-    if (smem_for(1) > kQsSmemMax) return 1;
-    const bool wide = smem_for(2) <= kQsSmemMax;  // eight rows per launch; else four
+    const QrPlan plan = qr_plan(c.fmt, c.n_full > 0 ? c.n_full : c.N, c.K, nw, vec, ctx->sms);
+    if (plan.ms == 0) return 1;
+    const int row_bytes = c.fmt == kFmtAffine8 ? c.K : c.K / 2;
+    QrMaps maps = {};
+    for (int i = 0; i < nw; i++) {
+        const int32_t r = cached_rows16_map(ctx, c.w[i], c.N, row_bytes, &maps.w[i]);
+        if (r != kOk) return r;
+    }
     p.N = c.N; p.K = c.K;
     p.x_dtype = c.x_dtype; p.ldx = c.ldx;
     p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
     p.act = c.act; p.limit = c.limit;
+    p.wk = plan.wk;
+    p.status = ctx->d_status;
     const size_t xes = c.x_dtype == kF32 ? 4 : 2, yes = c.y_dtype == kF32 ? 4 : 2;
+    const int nsup = (c.N / 16 + plan.warps / plan.wk - 1) / (plan.warps / plan.wk);
     for (int m0 = 0; m0 < c.rows;) {
-        const int left = c.rows - m0, ms = left > 4 && wide ? 2 : 1, m = left < 4 * ms ? left : 4 * ms;
-        p.M = m;
+        int ms = 1;
+        while (ms < plan.ms && 4 * ms < c.rows - m0) ms *= 2;
+        p.M = std::min(c.rows - m0, 4 * ms);
         p.x = static_cast<const char*>(c.x) + (size_t)m0 * c.ldx * xes;
         p.y = static_cast<char*>(c.y) + (size_t)m0 * c.ldy * yes;
-        const int smem = smem_for(ms), slots = ctx->sms * (ms == 1 && smem <= kQsSmemMax / 2 - 1024 ? 2 : 1);
-        const int32_t r = check_cuda(ctx, launch_dependent(qd_pick(c.fmt, nw, ms, vec), dim3(c.N / 16 < slots ? c.N / 16 : slots), kQdThreads,
-                                                           smem, st, p), "qmv_direct launch");
+        p.depth = 2;
+        while (p.depth < 6 && qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth + 1) <= (size_t)kQsSmemMax) p.depth++;
+        const int32_t r = check_cuda(ctx, launch_dependent(qr_pick(c.fmt, nw, ms, vec), dim3(std::min(nsup, ctx->sms)), plan.warps * 32,
+                                                           qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth), st, maps, p), "qmv_ring launch");
         if (r != kOk) return r;
-        m0 += m;
+        m0 += p.M;
     }
     return kOk;
 }
@@ -443,11 +472,11 @@ int32_t gqmv_init(iq_ctx* ctx) {
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
         }
-    const int32_t qd_fmts[3] = {kFmtAffine4, kFmtAffine4G32, kFmtAffine8};
-    for (int v = 0; v < 24; v++) {
-        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qd_pick(qd_fmts[v % 3], 1 + v / 3 % 2, 1 + v / 6 % 2, v >= 12)),
+    const int32_t qr_fmts[3] = {kFmtAffine4, kFmtAffine4G32, kFmtAffine8};
+    for (int v = 0; v < 36; v++) {
+        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qr_pick(qr_fmts[v % 3], 1 + v / 3 % 2, 1 << (v / 6 % 3), v >= 18)),
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
-        if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_direct)");
+        if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_ring)");
     }
     for (int fmt = 0; fmt < 4; fmt++)
         for (int mh = 1; mh <= 2; mh++)
@@ -469,11 +498,11 @@ int32_t gqmv_init(iq_ctx* ctx) {
 
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     // One kernel per (format, shape), chosen from the matrix alone: for affine codes the int8 tensor-core kernels (staged
-    // where K fits the staging, else with the weights in registers), the streaming fp16 kernel for MXFP4, the register-staged
+    // where K fits the staging, else with a ring per warp), the streaming fp16 kernel for MXFP4, the register-staged
     // fp16 kernel where K is too wide for either.
     int32_t r = launch_qmv_imma(ctx, st, c);
     if (r != 1) return r;
-    r = launch_qmv_direct(ctx, st, c);
+    r = launch_qmv_ring(ctx, st, c);
     if (r != 1) return r;
     r = launch_qmv_stream(ctx, st, c);
     if (r != 1) return r;
