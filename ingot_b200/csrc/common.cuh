@@ -87,6 +87,33 @@ __device__ __forceinline__ void load_x8(const void* x, int32_t dtype, size_t i, 
     }
 }
 
+// The same in two steps, for loops that want several loads under way: the loads (volatile: they stay where they are written,
+// and one instruction sequence for every type, no branch between them), then the conversion.
+struct RawX8 {
+    uint4 a, b;
+};
+__device__ __forceinline__ RawX8 load_raw_x8(const void* x, int32_t dtype, size_t i) {
+    const char* p = static_cast<const char*>(x) + i * (dtype == kF32 ? 4 : 2);
+    RawX8 r;
+    asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.a.x), "=r"(r.a.y), "=r"(r.a.z), "=r"(r.a.w) : "l"(p));
+    asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.b.x), "=r"(r.b.y), "=r"(r.b.z), "=r"(r.b.w) : "l"(p + (dtype == kF32 ? 16 : 0)));
+    return r;
+}
+__device__ __forceinline__ void unpack_x8(const RawX8& r, int32_t dtype, float (&v)[8]) {
+    const uint32_t w[8] = {r.a.x, r.a.y, r.a.z, r.a.w, r.b.x, r.b.y, r.b.z, r.b.w};
+    if (dtype == kF32) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = __uint_as_float(w[j]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+            v[2 * j] = dtype == kBF16 ? __uint_as_float(w[j] << 16) : f.x;
+            v[2 * j + 1] = dtype == kBF16 ? __uint_as_float(w[j] & 0xFFFF0000u) : f.y;
+        }
+    }
+}
+
 // Gated FFN activation on fp32 values.
 template <int ACT>
 __device__ __forceinline__ float glu(float g, float u, float limit) {

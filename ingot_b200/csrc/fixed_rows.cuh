@@ -32,14 +32,8 @@ __device__ __forceinline__ void fixed_point_unit(const float (&v)[8], int w8, un
     qi_group_scale(amax, sum, sc, inv);
     if (digits == nullptr) return;
     if (w8 == 0) *scale = make_float2(sc, sum);
-    uint32_t hi_w[2] = {0, 0}, lo_w[2] = {0, 0};
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int X = __float2int_rn(v[k] * inv);
-        const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
-        hi_w[k & 1] |= (uint32_t)(hi_d & 0xFF) << (8 * (k >> 1));
-        lo_w[k & 1] |= (uint32_t)(lo_d & 0xFF) << (8 * (k >> 1));
-    }
+    uint32_t hi_w[2], lo_w[2];
+    qi_digits8<false>(v, inv, hi_w, lo_w);
     unsigned char* f = digits + (w8 >> 1) * 16 + (w8 & 1) * 8;
     *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
     *reinterpret_cast<uint2*>(f + 64) = make_uint2(lo_w[0], lo_w[1]);

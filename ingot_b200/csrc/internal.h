@@ -118,9 +118,13 @@ struct GqmvCall {
     const float* ebias[2] = {nullptr, nullptr};
     float limit = 0.f;
     int32_t act = 0;  // gate/up mode: activation (kAct*)
+    void* scratch = nullptr;  // device memory of rows * K * 9 / 4 bytes that the call may use (256-byte aligned), or null
     const FixedRows* fx = nullptr;  // grouped gate/up: the token rows as block fixed point, when the caller has them
 };
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
+// iq_qmv with scratch (see GqmvCall)
+int32_t qmv_with_scratch(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y, int32_t y_dtype,
+                         int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix, void* scratch);
 // Tiles of up to eight rows of affine 4-bit experts on the int8 kernel; 1: the shape does not fit it
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
 

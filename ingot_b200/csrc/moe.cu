@@ -476,7 +476,9 @@ extern "C" int32_t iq_dense_ffn_workspace_bytes(iq_ctx* ctx, const iq_qlinear* g
                     gate_up->k, down->n, down->k);
     const size_t d_ff = down->k;
     size_t total = round_up_sz((size_t)rows * d_ff * 2, 256);  // h fp16
-    if (rows > 16) {
+    if (rows <= 16) {
+        total += round_up_sz((size_t)rows * std::max(d_ff, (size_t)gate_up->k) / 4 * 9, 256);  // x, then h, as block fixed point
+    } else {
         size_t q = 0;
         int32_t st = iq_qmm_workspace_bytes(ctx, gate_up, rows, x_dtype, &q);
         if (st != kOk) return st;
@@ -524,9 +526,10 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
         c.y = h; c.y_dtype = kF16; c.ldy = d_ff;
         c.limit = act == IQ_ACT_SWIGLU_OAI ? act_limit : 0.f;
         c.act = act;
+        c.scratch = static_cast<char*>(workspace) + round_up_sz((size_t)rows * d_ff * 2, 256);
         st = launch_gqmv(ctx, cs, c);
         if (st != kOk) return st;
-        return iq_qmv(ctx, stream, h, IQ_F16, d_ff, down, out, out_dtype, ldo, rows, flags, 0);
+        return qmv_with_scratch(ctx, stream, h, IQ_F16, d_ff, down, out, out_dtype, ldo, rows, flags, 0, c.scratch);
     }
     if (fmt != kFmtTernary && fmt != kFmtAffine6) {
         // GEMM path, fused: the gate and the up rows of the concatenated matrix are the two weight tiles of one stage of

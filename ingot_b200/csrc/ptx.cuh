@@ -189,6 +189,9 @@ template <int BYTES>
 __device__ __forceinline__ void cp_async_ca(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
 }
+__device__ __forceinline__ void cp_async_cg16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 // four bytes of which the first n are copied, the others zero
 __device__ __forceinline__ void cp_async4_zfill(uint32_t dst, const void* src, int n) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");

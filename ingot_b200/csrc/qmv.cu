@@ -134,6 +134,108 @@ int tail_slot_of(iq_ctx* ctx, cudaStream_t st) {
     return ctx->qmv_tail_stream_count++;
 }
 
+// ---- int8 tensor-core path with a ring of weights per warp: the plain GEMVs the staged kernel refuses, and the dense FFN's
+// gate + up ---------------------------------------------------------------------------------------------------------
+typedef void (*QrKernel)(const QrMaps, const QrParams);
+template <int FMT, int NW>
+QrKernel qr_pick_mv(int ms, bool vec) {
+    if (ms == 4) return vec ? qmv_ring_kernel<FMT, 4, NW, true> : qmv_ring_kernel<FMT, 4, NW, false>;
+    if (ms == 2) return vec ? qmv_ring_kernel<FMT, 2, NW, true> : qmv_ring_kernel<FMT, 2, NW, false>;
+    return vec ? qmv_ring_kernel<FMT, 1, NW, true> : qmv_ring_kernel<FMT, 1, NW, false>;
+}
+template <int FMT>
+QrKernel qr_pick_f(int nw, int ms, bool vec) { return nw == 2 ? qr_pick_mv<FMT, 2>(ms, vec) : qr_pick_mv<FMT, 1>(ms, vec); }
+QrKernel qr_pick(int32_t fmt, int nw, int ms, bool vec) {
+    return fmt == kFmtAffine8 ? qr_pick_f<kFmtAffine8>(nw, ms, vec)
+         : fmt == kFmtAffine4G32 ? qr_pick_f<kFmtAffine4G32>(nw, ms, vec) : qr_pick_f<kFmtAffine4>(nw, ms, vec);
+}
+constexpr int kQrPreUnits = 1000;
+// How a matrix is split, whatever the rows of the call (a row's bits must not depend on them).
+struct QrPlan {
+    int ms;      // sets of four rows a launch can take
+    int warps, wk;
+};
+// wk8: eight slices of equal length, the sums of the staged kernel.
+QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms, bool wk8) {
+    QrPlan best = {0, 0, 0};
+    // as many row sets as fit beside at least two slots per warp, then as many warps
+    for (int ms = 4; ms >= 1 && best.ms == 0; ms /= 2)
+        for (int w = kQrMaxWarps; w >= (ms > 1 ? 8 : 4); w -= wk8 ? 8 : 4)
+            if (qr_smem(fmt, K, nw, ms, vec, w, 2) <= (size_t)kQsSmemMax) { best.ms = ms; best.warps = w; break; }
+    if (best.ms == 0) return best;
+    // K slices: the least (rounds of a CTA) x (columns of a warp in a round + the round's own cost, about one column's)
+    const int gpc = qr_groups(fmt), G = K / (fmt == kFmtAffine4G32 ? 32 : 64), ncol = (G + gpc - 1) / gpc, nblk = N / 16;
+    long long cost = -1;
+    for (int wk = best.warps; wk >= 1; wk--) {
+        if (best.warps % wk != 0 || wk > ncol || (wk8 && wk != 8)) continue;
+        const long long per = (long long)(best.warps / wk) * sms, rounds = (nblk + per - 1) / per, c = rounds * ((ncol + wk - 1) / wk + 1);
+        if (cost < 0 || c < cost) { cost = c; best.wk = wk; }
+    }
+    return best;
+}
+// Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
+int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk8 = false) {
+    if (c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0 || ctx->encode_tiled == nullptr) return 1;
+    if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;
+    const int nw = c.mode == kModeGateUp ? 2 : 1, gpc = qr_groups(c.fmt), G = c.K / (c.fmt == kFmtAffine4G32 ? 32 : 64);
+    bool vec = G % gpc == 0;
+    QrParams p;
+    memset(&p, 0, sizeof(p));
+    for (int i = 0; i < nw; i++) {
+        p.s[i] = static_cast<const unsigned char*>(c.s[i]);
+        p.b[i] = static_cast<const unsigned char*>(c.b[i]);
+        const uintptr_t sb = reinterpret_cast<uintptr_t>(p.s[i]) | reinterpret_cast<uintptr_t>(p.b[i]);
+        if ((reinterpret_cast<uintptr_t>(c.w[i]) & 15) || (sb & 3)) return 1;
+        if (sb & (uintptr_t)(2 * gpc - 1)) vec = false;
+    }
+    const QrPlan plan = qr_plan(c.fmt, c.n_full > 0 ? c.n_full : c.N, c.K, nw, vec, ctx->sms, wk8);
+    if (plan.ms == 0 || plan.wk == 0) return 1;
+    const int row_bytes = c.fmt == kFmtAffine8 ? c.K : c.K / 2;
+    QrMaps maps = {};
+    for (int i = 0; i < nw; i++) {
+        const int32_t r = cached_rows16_map(ctx, c.w[i], c.N, row_bytes, &maps.w[i]);
+        if (r != kOk) return r;
+    }
+    p.N = c.N; p.K = c.K;
+    p.x_dtype = c.x_dtype; p.ldx = c.ldx;
+    p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
+    p.act = c.act; p.limit = c.limit;
+    p.wk = plan.wk;
+    p.runs = wk8 ? 1 : 0;
+    p.status = ctx->d_status;
+    const size_t xes = c.x_dtype == kF32 ? 4 : 2, yes = c.y_dtype == kF32 ? 4 : 2;
+    // The activations: every CTA converts them, or one more kernel does it for all where that is shorter (a CTA takes about
+    // 1 us per 2000 units of eight inputs, the kernel 1.5 us)
+    const int units = c.rows * (c.K / 8);
+    const bool pre = c.scratch != nullptr && units > kQrPreUnits;
+    const size_t rec = (size_t)G * (c.fmt == kFmtAffine4G32 ? 64 : 128);  // bytes of a row's digits
+    if (pre) {
+        unsigned char* digits = static_cast<unsigned char*>(c.scratch);
+        float2* scale = reinterpret_cast<float2*>(digits + c.rows * rec);
+        auto k = c.fmt == kFmtAffine8 ? qr_convert_kernel<true, false> : c.fmt == kFmtAffine4G32 ? qr_convert_kernel<false, true> : qr_convert_kernel<false, false>;
+        const int32_t r = check_cuda(ctx, launch_dependent(k, dim3((units + 255) / 256), 256, 0, st, c.x, c.x_dtype, c.ldx, c.K, c.rows, digits, scale), "qr_convert launch");
+        if (r != kOk) return r;
+        p.xd = digits;
+        p.xs = scale;
+    }
+    const int nsup = (c.N / 16 + plan.warps / plan.wk - 1) / (plan.warps / plan.wk);
+    for (int m0 = 0; m0 < c.rows;) {
+        int ms = 1;
+        while (ms < plan.ms && 4 * ms < c.rows - m0) ms *= 2;
+        p.M = std::min(c.rows - m0, 4 * ms);
+        p.x = static_cast<const char*>(c.x) + (size_t)m0 * c.ldx * xes;
+        p.y = static_cast<char*>(c.y) + (size_t)m0 * c.ldy * yes;
+        p.depth = 2;
+        while (p.depth < 6 && qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth + 1) <= (size_t)kQsSmemMax) p.depth++;
+        const int32_t r = check_cuda(ctx, launch_dependent(qr_pick(c.fmt, nw, ms, vec), dim3(std::min(nsup, ctx->sms)), plan.warps * 32,
+                                                           qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth), st, maps, p), "qmv_ring launch");
+        if (r != kOk) return r;
+        if (pre) { p.xd += p.M * rec; p.xs += (size_t)p.M * G; }
+        m0 += p.M;
+    }
+    return kOk;
+}
+
 // ---- int8 tensor-core path (decode, up to four rows, affine codes) -----------------------------------------------
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
@@ -189,6 +291,13 @@ int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
         tail_slices = 1;
         while (tail_slices * 2 * tail <= slots && tail_slices * 2 <= 32 && G % (tail_slices * 2) == 0) tail_slices *= 2;
         if (tail_slices < 8 || tail * tail_slices > kQmvTailPieces) tail_slices = 0;
+    }
+    // Nine to sixteen rows: the ring kernel reads the weights once, with the same K slices and order of sums (14336 x 4096 at 4
+    // bits and 16 rows 50.1 -> 33.5 us, 8 bits 56.0 -> 40.7); up to eight this kernel's deeper staging is level or ahead (one
+    // row 9.2 against 13.2). Left-over blocks are summed by pieces, so a matrix that has them stays here.
+    if (c.rows > 8 && tail_slices == 0 && !w6) {
+        const int32_t r = launch_qmv_ring(ctx, st, c, true);
+        if (r != 1) return r;
     }
     const size_t xes = c.x_dtype == kF32 ? 4 : 2, yes = c.y_dtype == kF32 ? 4 : 2;
     for (int m0 = 0; m0 < c.rows; m0 += 8) {  // nine to sixteen rows: two launches of up to eight
@@ -247,90 +356,6 @@ int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
 #undef IQ_QI_LAUNCH
         const int32_t r = check_cuda(ctx, e, "qmv_imma launch");
         if (r != kOk) return r;
-    }
-    return kOk;
-}
-
-// ---- int8 tensor-core path with a ring of weights per warp: the plain GEMVs the staged kernel refuses, and the dense FFN's
-// gate + up ---------------------------------------------------------------------------------------------------------
-typedef void (*QrKernel)(const QrMaps, const QrParams);
-template <int FMT, int NW>
-QrKernel qr_pick_mv(int ms, bool vec) {
-    if (ms == 4) return vec ? qmv_ring_kernel<FMT, 4, NW, true> : qmv_ring_kernel<FMT, 4, NW, false>;
-    if (ms == 2) return vec ? qmv_ring_kernel<FMT, 2, NW, true> : qmv_ring_kernel<FMT, 2, NW, false>;
-    return vec ? qmv_ring_kernel<FMT, 1, NW, true> : qmv_ring_kernel<FMT, 1, NW, false>;
-}
-template <int FMT>
-QrKernel qr_pick_f(int nw, int ms, bool vec) { return nw == 2 ? qr_pick_mv<FMT, 2>(ms, vec) : qr_pick_mv<FMT, 1>(ms, vec); }
-QrKernel qr_pick(int32_t fmt, int nw, int ms, bool vec) {
-    return fmt == kFmtAffine8 ? qr_pick_f<kFmtAffine8>(nw, ms, vec)
-         : fmt == kFmtAffine4G32 ? qr_pick_f<kFmtAffine4G32>(nw, ms, vec) : qr_pick_f<kFmtAffine4>(nw, ms, vec);
-}
-// How a matrix is split, whatever the rows of the call (a row's bits must not depend on them).
-struct QrPlan {
-    int ms;      // sets of four rows a launch can take
-    int warps, wk;
-};
-QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms) {
-    QrPlan best = {0, 0, 0};
-    // as many row sets as fit beside at least two slots per warp, then as many warps
-    for (int ms = 4; ms >= 1 && best.ms == 0; ms /= 2)
-        for (int w = kQrMaxWarps; w >= (ms > 1 ? 8 : 4); w -= 4)
-            if (qr_smem(fmt, K, nw, ms, vec, w, 2) <= (size_t)kQsSmemMax) { best.ms = ms; best.warps = w; break; }
-    if (best.ms == 0) return best;
-    // K slices: the least (rounds of a CTA) x (columns of a warp in a round + the round's own cost, about one column's)
-    const int gpc = qr_groups(fmt), G = K / (fmt == kFmtAffine4G32 ? 32 : 64), ncol = (G + gpc - 1) / gpc, nblk = N / 16;
-    long long cost = -1;
-    for (int wk = best.warps; wk >= 1; wk--) {
-        if (best.warps % wk != 0 || wk > ncol) continue;
-        const long long per = (long long)(best.warps / wk) * sms, rounds = (nblk + per - 1) / per, c = rounds * ((ncol + wk - 1) / wk + 1);
-        if (cost < 0 || c < cost) { cost = c; best.wk = wk; }
-    }
-    return best;
-}
-// Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
-int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
-    if (c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0 || ctx->encode_tiled == nullptr) return 1;
-    if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;
-    const int nw = c.mode == kModeGateUp ? 2 : 1, gpc = qr_groups(c.fmt), G = c.K / (c.fmt == kFmtAffine4G32 ? 32 : 64);
-    bool vec = G % gpc == 0;
-    QrParams p;
-    memset(&p, 0, sizeof(p));
-    for (int i = 0; i < nw; i++) {
-        p.s[i] = static_cast<const unsigned char*>(c.s[i]);
-        p.b[i] = static_cast<const unsigned char*>(c.b[i]);
-        const uintptr_t sb = reinterpret_cast<uintptr_t>(p.s[i]) | reinterpret_cast<uintptr_t>(p.b[i]);
-        if ((reinterpret_cast<uintptr_t>(c.w[i]) & 15) || (sb & 3)) return 1;
-        if (sb & (uintptr_t)(2 * gpc - 1)) vec = false;
-    }
-    const QrPlan plan = qr_plan(c.fmt, c.n_full > 0 ? c.n_full : c.N, c.K, nw, vec, ctx->sms);
-    if (plan.ms == 0) return 1;
-    const int row_bytes = c.fmt == kFmtAffine8 ? c.K : c.K / 2;
-    QrMaps maps = {};
-    for (int i = 0; i < nw; i++) {
-        const int32_t r = cached_rows16_map(ctx, c.w[i], c.N, row_bytes, &maps.w[i]);
-        if (r != kOk) return r;
-    }
-    p.N = c.N; p.K = c.K;
-    p.x_dtype = c.x_dtype; p.ldx = c.ldx;
-    p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;
-    p.act = c.act; p.limit = c.limit;
-    p.wk = plan.wk;
-    p.status = ctx->d_status;
-    const size_t xes = c.x_dtype == kF32 ? 4 : 2, yes = c.y_dtype == kF32 ? 4 : 2;
-    const int nsup = (c.N / 16 + plan.warps / plan.wk - 1) / (plan.warps / plan.wk);
-    for (int m0 = 0; m0 < c.rows;) {
-        int ms = 1;
-        while (ms < plan.ms && 4 * ms < c.rows - m0) ms *= 2;
-        p.M = std::min(c.rows - m0, 4 * ms);
-        p.x = static_cast<const char*>(c.x) + (size_t)m0 * c.ldx * xes;
-        p.y = static_cast<char*>(c.y) + (size_t)m0 * c.ldy * yes;
-        p.depth = 2;
-        while (p.depth < 6 && qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth + 1) <= (size_t)kQsSmemMax) p.depth++;
-        const int32_t r = check_cuda(ctx, launch_dependent(qr_pick(c.fmt, nw, ms, vec), dim3(std::min(nsup, ctx->sms)), plan.warps * 32,
-                                                           qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth), st, maps, p), "qmv_ring launch");
-        if (r != kOk) return r;
-        m0 += p.M;
     }
     return kOk;
 }
@@ -573,8 +598,8 @@ int32_t format_of(const iq_qlinear* m) {
 
 using namespace iq;
 
-extern "C" int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m,
-                          void* y, int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix) {
+int32_t iq::qmv_with_scratch(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
+                             int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix, void* scratch) {
     if (ctx == nullptr) return kErrInvalidArg;
     if (x == nullptr || y == nullptr || m == nullptr || m->w == nullptr || m->scales == nullptr)
         return fail(ctx, kErrInvalidArg, "qmv: null pointer");
@@ -612,5 +637,11 @@ extern "C" int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dt
     c.rows = rows; c.max_rows = rows; c.grid_tiles = 1;
     c.y = y; c.y_dtype = y_dtype; c.ldy = ldy;
     c.accumulate = (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0;
+    c.scratch = scratch;
     return launch_gqmv(ctx, reinterpret_cast<cudaStream_t>(stream), c);
+}
+
+extern "C" int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m,
+                          void* y, int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix) {
+    return qmv_with_scratch(ctx, stream, x, x_dtype, ldx, m, y, y_dtype, ldy, rows, flags, n_prefix, nullptr);
 }

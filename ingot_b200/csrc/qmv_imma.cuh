@@ -112,6 +112,25 @@ __device__ __forceinline__ void unpack6x16(uint32_t w0, uint32_t w1, uint32_t w2
     o[3] = spread6(w2 >> 8);
 }
 
+// Eight activations as two signed 7-bit digits each: X = round(v * inv), |X| <= 8192, hi = (X + 64) >> 7, lo = X - 128 hi; words
+// of four digits, [b0 / b1 half]: 4-bit codes put even k in the low nibbles (b0) and odd k in the high ones (b1), 8-bit codes
+// put k 0-3 in one word and k 4-7 in the next. The rounding is the addition of 1.5 * 2^23 (+ 64), which leaves X + 64 in the
+// low bits, and four digits go through the shifts and masks at a time: 26 instructions, not 80 (the conversion is every CTA's
+// prologue and was a third of all instructions of a launch of four rows and 14336 inputs).
+template <bool W8>
+__device__ __forceinline__ void qi_digits8(const float (&v)[8], float inv, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        uint32_t f[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) f[i] = __float_as_uint(fmaf(v[W8 ? 4 * h + i : 2 * i + h], inv, 12582976.0f));
+        const uint32_t p0 = __byte_perm(f[0], f[1], 0x5410), p1 = __byte_perm(f[2], f[3], 0x5410);
+        hi[h] = __byte_perm(p0 >> 7, p1 >> 7, 0x6420);
+        const uint32_t l = (__byte_perm(p0, p1, 0x6420) & 0x7F7F7F7Fu) ^ 0x40404040u;  // seven bits, sign flipped back ...
+        lo[h] = l + ((l & 0x40404040u) << 1);                                           // ... and extended
+    }
+}
+
 // Block fixed point of one group of 64 activations: from the group's largest magnitude and its sum, the power of two
 // 2^(e-13) the digits are counted in (2^e > amax >= 2^(e-1)) and its inverse. A group that holds a NaN or an infinity
 // (amax or the sum not finite; fmaxf drops a NaN, the sum keeps it) gets a NaN scale and a NaN sum, so that every output
@@ -385,10 +404,8 @@ __global__ void __launch_bounds__(kQiMaxThreads, MS == 1 ? 2 : 1)
             *reinterpret_cast<uint2*>(xq + fb + 64) = make_uint2(0, 0);
             if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(0.f, 0.f);
         }
-        for (int u = tid; u < G * 8 * p.M; u += nct) {
+        auto convert = [&](const float (&v)[8], int u) {
             const int m = u / (G * 8), j = (u >> 3) % G, w8 = u & 7;
-            float v[8];
-            load_x8(p.x, p.x_dtype, (size_t)m * p.ldx + j * 64 + w8 * 8, v);
             float amax = 0.f, sum = 0.f;
 #pragma unroll
             for (int k = 0; k < 8; k++) {
@@ -403,23 +420,38 @@ __global__ void __launch_bounds__(kQiMaxThreads, MS == 1 ? 2 : 1)
             float scale, inv;
             qi_group_scale(amax, sum, scale, inv);
             if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(scale, sum);
-            uint32_t hi_w[2] = {0, 0}, lo_w[2] = {0, 0};  // [b0 / b1 half] bytes i = 0..3
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int X = __float2int_rn(v[k] * inv);       // |X| <= 8192
-                const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
-                // input k of the span: 4-bit codes put even k in the low nibbles (b0) and odd k in the high ones (b1);
-                // 8-bit codes put k 0-3 in one word (b0) and k 4-7 in the next (b1)
-                const int half = W8 ? (k >> 2) : (k & 1), i = W8 ? (k & 3) : (k >> 1);
-                hi_w[half] |= (uint32_t)(hi_d & 0xFF) << (8 * i);
-                lo_w[half] |= (uint32_t)(lo_d & 0xFF) << (8 * i);
-            }
+            uint32_t hi_w[2], lo_w[2];
+            qi_digits8<W8>(v, inv, hi_w, lo_w);
             // the span is word w8 of the group's eight (4-bit: lane t = w8 / 2, MMA w8 % 2) or words 2 w8, 2 w8 + 1 of
             // its sixteen (8-bit: lane t = w8 / 2, MMA w8 % 2): the same slot either way
             const int t = w8 >> 1, mm = w8 & 1;
             const int fb = ((j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * 16 + mm * 8;  // the row's hi-digit column, lane 0
             *reinterpret_cast<uint2*>(xq + fb + t * 16) = make_uint2(hi_w[0], hi_w[1]);
             *reinterpret_cast<uint2*>(xq + fb + (4 + t) * 16) = make_uint2(lo_w[0], lo_w[1]);
+        };
+        const int units = G * 8 * p.M;  // (a multiple of 32: whole warps leave the loops together)
+        if (units <= 2 * nct) {
+            for (int u = tid; u < units; u += nct) {
+                float v[8];
+                load_x8(p.x, p.x_dtype, (size_t)(u / (G * 8)) * p.ldx + (u % (G * 8)) * 8, v);
+                convert(v, u);
+            }
+        } else {  // four loads under way per thread
+            for (int u0 = tid; u0 < units; u0 += 4 * nct) {
+                RawX8 raw[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int u = min(u0 + q * nct, units - 1);
+                    raw[q] = load_raw_x8(p.x, p.x_dtype, (size_t)(u / (G * 8)) * p.ldx + (u % (G * 8)) * 8);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (u0 + q * nct >= units) break;
+                    float v[8];
+                    unpack_x8(raw[q], p.x_dtype, v);
+                    convert(v, u0 + q * nct);
+                }
+            }
         }
         const uint32_t xtok = qi_consumer_barrier(nct);
         if (p.tail_blocks > 0) asm volatile("bar.arrive 2, %0;" ::"r"(nct + 32) : "memory");  // the producer may read xq

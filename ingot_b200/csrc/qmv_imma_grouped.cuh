@@ -328,15 +328,8 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
                         qi_group_scale(amax, sum, scale, inv);
                         if (!live) continue;
                         if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(scale, sum);
-                        uint32_t hi_w[2] = {0, 0}, lo_w[2] = {0, 0};
-#pragma unroll
-                        for (int k = 0; k < 8; k++) {
-                            const int X = __float2int_rn(v[k4][k] * inv);
-                            const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
-                            const int half = k & 1, i = k >> 1;  // even inputs: low nibbles (b0), odd: high nibbles (b1)
-                            hi_w[half] |= (uint32_t)(hi_d & 0xFF) << (8 * i);
-                            lo_w[half] |= (uint32_t)(lo_d & 0xFF) << (8 * i);
-                        }
+                        uint32_t hi_w[2], lo_w[2];
+                        qi_digits8<false>(v[k4], inv, hi_w, lo_w);
                         const int tt = w8 >> 1, mm = w8 & 1;
                         const int fb = ((j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * 16 + mm * 8;
                         *reinterpret_cast<uint2*>(xq + fb + tt * 16) = make_uint2(hi_w[0], hi_w[1]);

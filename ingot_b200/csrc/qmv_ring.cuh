@@ -10,7 +10,7 @@
 // 128 bytes of 16 weight rows (of each matrix), one tensor copy with the 128-byte swizzle, and those rows' scales and biases
 // by asynchronous copies of 4 to 16 bytes per lane; the warp issues them itself, `depth` slots ahead and across the blocks of
 // rows, and waits on its own barriers, so that the only synchronisation of the CTA is where the K slices of a block of 16 rows
-// meet. Warps are wk K slices (every wk-th 128-byte column) x row blocks; the host picks the split (csrc/qmv.cu). Against the
+// meet. Warps are wk K slices (every wk-th 128-byte column, or runs of them) x row blocks; the host picks the split (csrc/qmv.cu). Against the
 // register batches: 8-bit FFN 2048 -> 7680 -> 2048 at 3 rows 27.2 -> 21.2 us, at 12 rows 72.6 -> 46.9; 4-bit 4096 -> 14336 at
 // one row 42.9 -> 36.2, at 8 rows 105 -> 72.
 #pragma once
@@ -25,6 +25,47 @@ namespace iq {
 
 constexpr int kQrMaxWarps = 16;
 constexpr int kQrBox = 2048;  // bytes of a slot's codes per matrix
+
+// Eight inputs (unit w8 of a group, its threads neighbouring lanes) as block fixed point, in B-fragment order: the high digits
+// at f, the low ones four lanes' fragments on.
+template <bool W8, bool G32>
+__device__ __forceinline__ void qr_convert(const float (&v)[8], int w8, bool live, unsigned char* rec, float2* scale_out) {
+    constexpr int TPG = G32 ? 4 : 8, XL = G32 ? 8 : 16;
+    float amax = 0.f, sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        amax = fmaxf(amax, fabsf(v[k]));
+        sum += v[k];
+    }
+#pragma unroll
+    for (int o = 1; o < TPG; o <<= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    }
+    float scale, inv;
+    qi_group_scale(amax, sum, scale, inv);
+    if (!live) return;
+    if (w8 == 0) *scale_out = make_float2(scale, sum);
+    uint32_t hi_w[2], lo_w[2];
+    qi_digits8<W8>(v, inv, hi_w, lo_w);
+    unsigned char* f = rec + (G32 ? w8 * 8 : (w8 >> 1) * 16 + (w8 & 1) * 8);
+    *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
+    *reinterpret_cast<uint2*>(f + 4 * XL) = make_uint2(lo_w[0], lo_w[1]);
+}
+
+// The rows of a call converted once, for CTAs that would each spend longer on it: [rows][groups] records of the digits (128
+// bytes; groups of 32: 64) and of {scale, sum}. 256 threads, a unit of eight inputs each.
+template <bool W8, bool G32>
+__global__ void __launch_bounds__(256) qr_convert_kernel(const void* x, int32_t x_dtype, int64_t ldx, int K, int M, unsigned char* digits, float2* scale) {
+    constexpr int TPG = G32 ? 4 : 8, REC = G32 ? 64 : 128;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int units = M * (K / 8), u = blockIdx.x * 256 + threadIdx.x, uc = min(u, units - 1);
+    float v[8];
+    load_x8(x, x_dtype, (size_t)(uc / (K / 8)) * ldx + (uc % (K / 8)) * 8, v);
+    const size_t rec = uc / TPG;  // (K is a multiple of the group)
+    qr_convert<W8, G32>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
+}
 
 struct QrMaps {
     CUtensorMap w[2];
@@ -43,6 +84,9 @@ struct QrParams {
     int32_t act;           // gate/up form: activation
     float limit;
     int32_t wk, depth;     // K slices; slots per warp
+    int32_t runs;          // slices are runs of columns (else every wk-th column: 5 % faster)
+    const unsigned char* xd;  // the rows as qr_convert_kernel left them, or null: converted here, from x
+    const float2* xs;
     int32_t* status;
 };
 
@@ -89,12 +133,13 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
     __syncwarp();
     pdl_launch_dependents();
 
-    // ---- this warp's items: its column of blocks of 16 rows, every wk-th 128 bytes of them --------------------------------
+    // ---- this warp's items: its column of blocks of 16 rows, its share of their 128-byte columns --------------------------
     const int rbs = nwarps / p.wk, rb = warp / p.wk, ks = warp % p.wk;
     const int nblk = p.N / 16, nsup = (nblk + rbs - 1) / rbs;
     const int lo = (int)((int64_t)nsup * blockIdx.x / gridDim.x), hi = (int)((int64_t)nsup * (blockIdx.x + 1) / gridDim.x);
     auto block_of = [&](int sb) { return sb * rbs + rb; };
-    int psb = lo, pcol = ks, pslot = 0;  // the next item to ask for
+    const int step = p.runs ? 1 : p.wk, col0 = p.runs ? ncol * ks / p.wk : ks, col1 = p.runs ? ncol * (ks + 1) / p.wk : ncol;
+    int psb = lo, pcol = col0, pslot = 0;  // the next item to ask for
     const bool odd_rows = (G & 1) != 0;
     auto issue = [&]() {
         const int blk = block_of(psb);
@@ -126,7 +171,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
         }
         cp_async_arrive_noinc(full);
         if (++pslot == depth) pslot = 0;
-        if ((pcol += p.wk) >= ncol) { pcol = ks; psb++; }
+        if ((pcol += step) >= col1) { pcol = col0; psb++; }
     };
     for (int i = 0; i < depth; i++) issue();  // the weights do not depend on the previous kernel of the stream
     pdl_wait();
@@ -140,39 +185,44 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
         *reinterpret_cast<uint2*>(f + 4 * XL) = make_uint2(0, 0);
         if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(0.f, 0.f);
     }
-    const int units = G * TPG * p.M, upad = (units + 31) / 32 * 32;  // whole warps: the groups' shuffles need their threads
-    for (int u = tid; u < upad; u += nthreads) {
-        const bool live = u < units;
-        const int m = live ? u / (G * TPG) : 0, j = (u / TPG) % G, w8 = u % TPG;
-        float v[8];
-        load_x8(p.x, p.x_dtype, (size_t)m * p.ldx + j * GS + w8 * 8, v);
-        float amax = 0.f, sum = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            amax = fmaxf(amax, fabsf(v[k]));
-            sum += v[k];
+    if (p.xd != nullptr) {
+        constexpr int PC = XL / 2;  // 16-byte pieces of a record
+        for (int m = 0; m < p.M; m++) {
+            const uint32_t d = smem_u32(xq) + ((m >> 2) * 32 + 8 * (m & 3)) * XL, sd = smem_u32(xsc) + m * 8;
+            const unsigned char* src = p.xd + (size_t)m * G * PC * 16;
+            for (int j = tid; j < G * PC; j += nthreads) cp_async_cg16(d + (j / PC) * (MS * 32 * XL) + (j % PC) * 16, src + (size_t)j * 16);
+            for (int j = tid; j < G; j += nthreads) cp_async_ca<8>(sd + j * (4 * MS * 8), p.xs + (size_t)m * G + j);
         }
-#pragma unroll
-        for (int o = 1; o < TPG; o <<= 1) {
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    const int units = p.xd != nullptr ? 0 : G * TPG * p.M, upad = (units + 31) / 32 * 32;  // whole warps: the groups' shuffles need their threads
+    auto convert = [&](const float (&v)[8], int u) {
+        const int m = u / (G * TPG), j = (u / TPG) % G;
+        qr_convert<W8, G32>(v, u % TPG, u < units, xq + ((size_t)(j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * XL, xsc + j * 4 * MS + m);
+    };
+    if (units <= 2 * nthreads) {
+        for (int u = tid; u < upad; u += nthreads) {
+            const int uc = min(u, units - 1);
+            float v[8];
+            load_x8(p.x, p.x_dtype, (size_t)(uc / (G * TPG)) * p.ldx + (uc % (G * TPG)) * 8, v);
+            convert(v, u);
         }
-        float scale, inv;
-        qi_group_scale(amax, sum, scale, inv);
-        if (!live) continue;
-        if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(scale, sum);
-        uint32_t hi_w[2] = {0, 0}, lo_w[2] = {0, 0};
+    } else {  // four loads under way per thread
+        for (int u0 = tid; u0 < upad; u0 += 4 * nthreads) {
+            RawX8 raw[4];
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int X = __float2int_rn(v[k] * inv);
-            const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
-            const int half = W8 ? (k >> 2) : (k & 1), i = W8 ? (k & 3) : (k >> 1);
-            hi_w[half] |= (uint32_t)(hi_d & 0xFF) << (8 * i);
-            lo_w[half] |= (uint32_t)(lo_d & 0xFF) << (8 * i);
+            for (int q = 0; q < 4; q++) {
+                const int u = min(u0 + q * nthreads, units - 1);
+                raw[q] = load_raw_x8(p.x, p.x_dtype, (size_t)(u / (G * TPG)) * p.ldx + (u % (G * TPG)) * 8);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (u0 + q * nthreads >= upad) break;  // (whole warps)
+                float v[8];
+                unpack_x8(raw[q], p.x_dtype, v);
+                convert(v, u0 + q * nthreads);
+            }
         }
-        unsigned char* f = xq + ((size_t)(j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * XL + (G32 ? w8 * 8 : (w8 >> 1) * 16 + (w8 & 1) * 8);
-        *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
-        *reinterpret_cast<uint2*>(f + 4 * XL) = make_uint2(lo_w[0], lo_w[1]);
     }
     __syncthreads();
 
@@ -188,7 +238,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
         for (int i = 0; i < NW; i++)
 #pragma unroll
             for (int c = 0; c < MS; c++) acc[i][c][0] = acc[i][c][1] = 0.f;
-        for (int col = block_of(sb) < nblk ? ks : ncol; col < ncol; col += p.wk) {
+        for (int col = block_of(sb) < nblk ? col0 : col1; col < col1; col += step) {
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar + 8 * slot, ph, abort_flag));
             if (ok) {
                 uint32_t sc[NW][2][GPC / 2], bi[NW][2][GPC / 2];

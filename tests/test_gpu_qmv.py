@@ -238,10 +238,11 @@ def test_qmv_non_finite_activations_propagate(cuda_device, bad, K):
 
 
 @pytest.mark.parametrize("bits", [4, 8])
-@pytest.mark.parametrize("N,K,rows", [(16, 832, 4), (4784, 192, 5), (4752, 7680, 3), (32, 14336, 8), (9488, 1024, 1)])
-def test_qmv_weights_in_registers(cuda_device, bits, N, K, rows):
+@pytest.mark.parametrize("N,K,rows", [(16, 832, 4), (4784, 192, 5), (4752, 7680, 3), (32, 14336, 8), (9488, 1024, 1), (1040, 1600, 13), (4096, 2048, 16), (1040, 4096, 9)])
+def test_qmv_ring_edges(cuda_device, bits, N, K, rows):
     """Input widths the staged kernel does not take: an odd number of groups (832 = 13 of 64), several 16-row blocks per CTA
-    with a remainder (4784 = 299 blocks, 9488 = 593), fewer groups than K slices (192), rows longer than a stage."""
+    with a remainder (4784 = 299 blocks, 9488 = 593), fewer groups than K slices (192), rows longer than a stage; and widths it
+    takes up to eight rows, where a row alone runs there and has to have the same bits."""
     rng = np.random.default_rng(700 + bits + N + K + rows)
     m, host = affine_case(rng, N, K, bits, cuda_device)
     x = synth.activations_np(rng, rows, K)
