@@ -118,6 +118,7 @@ struct GqmvCall {
     const float* ebias[2] = {nullptr, nullptr};
     float limit = 0.f;
     int32_t act = 0;  // gate/up mode: activation (kAct*)
+    bool early = false;  // tiles: the list is complete when the launch's predecessor lets it start (a launch of the same kind did)
     void* scratch = nullptr;  // device memory of rows * K * 9 / 4 bytes that the call may use (256-byte aligned), or null
     const FixedRows* fx = nullptr;  // grouped gate/up: the token rows as block fixed point, when the caller has them
 };
@@ -146,6 +147,7 @@ struct QmmCall {
     int32_t w_rows = 0;  // plain formats: rows of w when fewer than N, the rest counts as zeros (0: N)
     const Tile* tiles = nullptr;
     const uint32_t* ntiles = nullptr;
+    bool early = false;  // see GqmvCall
     void* y = nullptr;
     int32_t y_dtype = 0;
     int64_t ldy = 0;

@@ -208,7 +208,7 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
 
 // Likewise the down projection of every tile: yd[row, :] = h[row, :] W_down^T + b_d.
 int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles, const uint32_t* ntiles, int max_tiles, void* yd,
-                 int32_t yd_dtype) {
+                 int32_t yd_dtype, bool early = false) {
     const iq_moe_desc& d = l->d;
     const int64_t lo = d.expert_lo;
     GqmvCall c;
@@ -227,6 +227,7 @@ int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles,
     c.rows = 0; c.max_rows = kDecodeTileRows;
     c.y = yd; c.y_dtype = yd_dtype; c.ldy = d.d_model;
     if (d.down_bias) c.ebias[0] = d.down_bias - lo * d.d_model;
+    c.early = early;
     return launch_qmv_imma_grouped(l->ctx, cs, c);
 }
 
@@ -263,7 +264,7 @@ int32_t run_gateup_tc(iq_moe* l, cudaStream_t cs, const __half* rows16, int64_t 
 }
 
 int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows, const Tile* tiles, const uint32_t* ntiles,
-                    void* yd, int32_t yd_dtype, int bn) {
+                    void* yd, int32_t yd_dtype, int bn, bool early = false) {
     const iq_moe_desc& d = l->d;
     QmmCall c;
     c.fmt = l->fmt; c.epi = 0; c.bn = bn;
@@ -274,6 +275,7 @@ int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows,
     c.tiles = tiles; c.ntiles = ntiles;
     c.y = yd; c.y_dtype = yd_dtype; c.ldy = d.d_model;
     c.ebias[0] = d.down_bias;
+    c.early = early;
     return launch_qmm(l->ctx, cs, c);
 }
 
@@ -839,9 +841,13 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st != kOk) return st;
     }
     const int max_tiles = (int)std::min<int64_t>((int64_t)d.expert_count + P / kDecodeTileRows, P);
+    // which kernel made h: a down projection on the same one may start on the tile list and its weights before h is there
+    bool after_int8 = false, after_gemm = false;
     if (pieces & IQ_PIECE_GATEUP) {
         st = int8 ? run_gateup(l, cs, x, x_dtype, ldx, w.row_map, w.tiles_a, w.ntiles, max_tiles, w.h, 0, fixed ? &w.fx : nullptr) : 1;
+        after_int8 = st == kOk;
         if (st == 1) {
+            after_gemm = true;
             moe_pack_tokens_kernel<<<tokens, 256, 0, cs>>>(x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k);
             st = check_cuda(ctx, cudaGetLastError(), "moe_pack_tokens launch");
             if (st == kOk) st = run_gateup_tc(l, cs, w.xs, P, w.tiles_b, w.ntiles + 1, w.h, bn);
@@ -849,8 +855,8 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st != kOk) return st;
     }
     if (pieces & IQ_PIECE_DOWN) {
-        st = int8 ? run_down(l, cs, w.h, w.tiles_a, w.ntiles, max_tiles, w.yd, yd_dtype_of(l)) : 1;
-        if (st == 1) st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn);
+        st = int8 ? run_down(l, cs, w.h, w.tiles_a, w.ntiles, max_tiles, w.yd, yd_dtype_of(l), after_int8) : 1;
+        if (st == 1) st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn, after_gemm);
         if (st != kOk) return st;
     }
     if (pieces & IQ_PIECE_COMBINE) {

@@ -233,6 +233,7 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     const int spb = c.fmt == kFmtAffine8 ? 4 : (c.fmt == kFmtAffine4G32 ? 16 : 8);
     p.vec = srow % spb == 0 && (align & (uintptr_t)(spb - 1)) == 0 ? 1 : 0;
     p.expert_lo = c.expert_lo;
+    p.early = c.early ? 1 : 0;
     p.N = c.N; p.K = c.K; p.M = c.M;
     p.tiles = c.tiles; p.ntiles = c.ntiles;
     p.y = c.y; p.y_dtype = c.y_dtype; p.ldy = c.ldy; p.accumulate = c.accumulate;

@@ -82,6 +82,7 @@ struct TaParams {
     int32_t nx, nc;          // stages of X and of codes
     int32_t x_stage;         // bytes of an X stage
     int32_t dcols;           // columns per accumulator: 64, 128 or 192
+    int32_t early;           // the tile list is complete when the kernel starts
     int32_t vec;             // the row pitch of the scales allows asynchronous copies
     int32_t* status;
 };
@@ -256,10 +257,12 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pdl_launch_dependents();
-    // The weights do not depend on the previous kernel of the stream: with dense tiling their producers and the dequantisers
-    // start at once; a tile list, the activations and y do.
-    if (p.tiles != nullptr || !(warp == 2 || warp == 3 || warp >= 8)) pdl_wait();
+    // The weights do not depend on the previous kernel of the stream: with dense tiling, or behind a launch over the same tile
+    // list (p.early: that one lets its dependents start after its own wait, so the list is complete), their producers and
+    // the dequantisers start at once; a tile list, the activations and y do.
+    if (p.tiles == nullptr) pdl_launch_dependents();
+    if ((p.tiles != nullptr && !p.early) || !(warp == 2 || warp == 3 || warp >= 8)) pdl_wait();
+    if (p.tiles != nullptr) pdl_launch_dependents();
 
     // ---- work list --------------------------------------------------------------------------------------------------
     constexpr int NROWS = EPI ? 64 : 128;  // output features per tile

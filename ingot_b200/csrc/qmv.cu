@@ -441,6 +441,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     p.w_ebytes = c.w_estride * 4;
     p.s_ebytes = c.s_estride * 2;
     p.expert_lo = c.expert_lo;
+    p.early = c.early ? 1 : 0;
     CUtensorMap wmaps[2] = {};
     const CUtensorMap* maps[2] = {&wmaps[0], &wmaps[1]};
     if (tm) {

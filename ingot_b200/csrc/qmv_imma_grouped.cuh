@@ -54,6 +54,7 @@ struct QgParams {
     const float* ebias[2];
     float limit;
     int32_t act;
+    int32_t early;               // the tile list is complete when this kernel starts
     FixedRows fx;                // sixteen consumer warps: the token rows as block fixed point
     int32_t rgs, wk;             // row blocks of 16 per item x K slices = consumer warps
     int32_t NB;                  // items per tile
@@ -113,8 +114,11 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
         fence_async_smem();
     }
     __syncthreads();
+    // The tile list, the activations and y come from earlier kernels of the stream. A down projection behind this kernel's own
+    // gate/up (p.early) may read the list at once and stream weights: the gate/up lets its dependents start only after its
+    // own wait, so that the list is complete by then.
+    if (!p.early) pdl_wait();
     pdl_launch_dependents();
-    pdl_wait();  // the tile list, the activations and y come from earlier kernels of the stream
 
     const int R = 16 * p.rgs;
     const int G = p.K / 64;
@@ -241,6 +245,7 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
         }
     } else if (warp < kQgWarps) {
         // ================= consumers =================
+        if (p.early) pdl_wait();
         const int g = lane >> 2, t = lane & 3;
         const int rb = warp / p.wk, ks = warp % p.wk;
         const int gw = GW > 0 ? GW : G / p.wk, g0 = ks * gw;
@@ -485,6 +490,7 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
         }
     } else {
         // ================= epilogue =================
+        if (p.early) pdl_wait();
         const int et = tid - (kQgWarps + 1) * 32;
         const int rsh = 31 - __clz(R);  // R is a power of two
         int ti = lo / p.NB, blk = lo % p.NB, cur_tile = -1, M = 0;
