@@ -245,7 +245,7 @@ int tensor_tile_rows(int64_t rows, int64_t expert_slots) {
 
 // rows16: fp16 rows [n_rows, d_model] in tile order
 int32_t run_gateup_tc(iq_moe* l, cudaStream_t cs, const __half* rows16, int64_t n_rows, const Tile* tiles,
-                      const uint32_t* ntiles, __half* h, int bn) {
+                      const uint32_t* ntiles, __half* h, int bn, bool early = false) {
     const iq_moe_desc& d = l->d;
     QmmCall c;
     c.fmt = l->fmt; c.epi = 1; c.bn = bn;
@@ -258,6 +258,7 @@ int32_t run_gateup_tc(iq_moe* l, cudaStream_t cs, const __half* rows16, int64_t 
     c.tiles = tiles; c.ntiles = ntiles;
     c.y = h; c.y_dtype = kF16; c.ldy = d.d_ff;
     c.ebias[0] = d.gate_bias; c.ebias[1] = d.up_bias;
+    c.early = early;
     c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
     c.act = d.act;
     return launch_qmm(l->ctx, cs, c);
@@ -828,9 +829,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         st = kOk;
         if (P >= kGroupChunkedMinPairs && d.experts * 8 * 4 <= 48 * 1024) {
             // many pairs: a chunked counting sort touches each pair once per kernel instead of once per expert
-            moe_hist_kernel<<<gp.chunks, 256, d.experts * 4, cs>>>(gp);
-            moe_scan_kernel<<<1, 256, 0, cs>>>(gp);
-            moe_place_kernel<<<gp.chunks, 256, d.experts * 8 * 4, cs>>>(gp);
+            st = check_cuda(ctx, launch_dependent(moe_hist_kernel, dim3(gp.chunks), 256, d.experts * 4, cs, gp), "moe_hist launch");
+            if (st == kOk) st = check_cuda(ctx, launch_dependent(moe_scan_kernel, dim3(1), 256, 0, cs, gp), "moe_scan launch");
+            if (st == kOk) st = check_cuda(ctx, launch_dependent(moe_place_kernel, dim3(gp.chunks), 256, d.experts * 8 * 4, cs, gp), "moe_place launch");
         } else {
             if (fixed) { gp.fx = w.fx; gp.x = x; gp.x_dtype = x_dtype; gp.ldx = ldx; gp.T = tokens; gp.D = d.d_model; }
             st = check_cuda(ctx, launch_dependent(moe_count_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_count launch");
@@ -848,9 +849,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         after_int8 = st == kOk;
         if (st == 1) {
             after_gemm = true;
-            moe_pack_tokens_kernel<<<tokens, 256, 0, cs>>>(x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k);
-            st = check_cuda(ctx, cudaGetLastError(), "moe_pack_tokens launch");
-            if (st == kOk) st = run_gateup_tc(l, cs, w.xs, P, w.tiles_b, w.ntiles + 1, w.h, bn);
+            st = check_cuda(ctx, launch_dependent(moe_pack_tokens_kernel, dim3(tokens), 256, 0, cs, x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k),
+                            "moe_pack_tokens launch");
+            if (st == kOk) st = run_gateup_tc(l, cs, w.xs, P, w.tiles_b, w.ntiles + 1, w.h, bn, true);
         }
         if (st != kOk) return st;
     }

@@ -675,6 +675,8 @@ constexpr int kGroupChunk = 1024;
 
 __global__ void __launch_bounds__(256) moe_hist_kernel(const GroupParams p) {
     extern __shared__ uint32_t hist[];
+    pdl_launch_dependents();
+    pdl_wait();
     for (int e = threadIdx.x; e < p.E; e += 256) hist[e] = 0;
     __syncthreads();
     const int i0 = blockIdx.x * kGroupChunk, i1 = min(p.P, i0 + kGroupChunk);
@@ -684,8 +686,10 @@ __global__ void __launch_bounds__(256) moe_hist_kernel(const GroupParams p) {
 }
 
 __global__ void __launch_bounds__(256) moe_scan_kernel(const GroupParams p) {
-    __shared__ uint32_t sc[256], sa[256], sb[256];
-    const int tid = threadIdx.x;
+    __shared__ uint32_t wsum[3][8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
     // experts handled by this thread: a contiguous run, so that a block-wide scan over threads orders the experts
     const int per = (p.E + 255) / 256;
     const int e0 = tid * per, e1 = min(p.E, e0 + per);
@@ -709,10 +713,16 @@ __global__ void __launch_bounds__(256) moe_scan_kernel(const GroupParams p) {
             b_sum += (run + p.bm_b - 1) / p.bm_b;
         }
     }
-    sc[tid] = c_sum; sa[tid] = a_sum; sb[tid] = b_sum;
+    uint32_t off = c_sum, ta = a_sum, tb = b_sum;  // inclusive over the warp, then exclusive over the block
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, off, o), y = __shfl_up_sync(0xffffffffu, ta, o), z = __shfl_up_sync(0xffffffffu, tb, o);
+        if (lane >= o) { off += x; ta += y; tb += z; }
+    }
+    if (lane == 31) { wsum[0][warp] = off; wsum[1][warp] = ta; wsum[2][warp] = tb; }
     __syncthreads();
-    uint32_t off = 0, ta = 0, tb = 0;
-    for (int i = 0; i < tid; i++) { off += sc[i]; ta += sa[i]; tb += sb[i]; }
+    off -= c_sum; ta -= a_sum; tb -= b_sum;
+    for (int w = 0; w < warp; w++) { off += wsum[0][w]; ta += wsum[1][w]; tb += wsum[2][w]; }
     for (int e = e0; e < e1; e++) {
         const uint32_t cnt = p.counts[e];
         p.offsets[e] = off;
@@ -734,6 +744,8 @@ __global__ void __launch_bounds__(256) moe_scan_kernel(const GroupParams p) {
 __global__ void __launch_bounds__(256) moe_place_kernel(const GroupParams p) {
     extern __shared__ uint32_t sm[];  // [8 warps][E] pairs of each expert in each warp's share, then running counts
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
     for (int i = tid; i < 8 * p.E; i += 256) sm[i] = 0;
     __syncthreads();
     // warp w walks pairs [i0 + 128 w, i0 + 128 w + 128) of the chunk, 32 at a time
@@ -865,7 +877,8 @@ __global__ void __launch_bounds__(256) moe_pack_rows_kernel(const void* __restri
 __global__ void __launch_bounds__(256) moe_pack_tokens_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx,
                                                              const uint32_t* __restrict__ pos, __half* __restrict__ rows,
                                                              int D, int topk) {
-    pdl_launch_dependents();
+    pdl_wait();
+    pdl_launch_dependents();  // (after the wait: the GEMM behind it may start on the tile list and the weights)
     __shared__ uint32_t sp[32];
     const int t = blockIdx.x;
     if ((int)threadIdx.x < topk) sp[threadIdx.x] = pos[(size_t)t * topk + threadIdx.x];
