@@ -657,7 +657,7 @@ extern "C" int32_t iq_moe_create(iq_ctx* ctx, const iq_moe_desc* d, iq_moe** out
     l->d = *d;
     l->fmt = fg;
     l->ld = round_up(d->experts, 64);
-    if (d->router_kind == IQ_ROUTER_BF16 && d->router_score == IQ_SCORE_SOFTMAX && d->experts % 64 == 0) {
+    if (d->router_kind == IQ_ROUTER_BF16 && d->router_score == IQ_SCORE_SOFTMAX) {
         // set-up time (this call takes no stream): the largest row norm of the router, for the error bound of the
         // tensor-core logits. The router tensor must be complete on the device when the layer is created.
         uint32_t* dmax = nullptr;

@@ -317,6 +317,46 @@ def test_moe_other_activations(cuda_device, act, T):
     check_layer(layer, host, synth.activations_np(rng, T, 2048), T, act)
 
 
+@pytest.mark.parametrize("E,K,D,I,T", [
+    (32, 4, 192, 64, 1), (32, 4, 192, 64, 3), (96, 16, 320, 192, 2), (512, 10, 1024, 64, 3),  # the three-kernel path: odd
+    (32, 4, 192, 64, 4),             # group counts, one slice per expert, experts beyond a warp's four; and past its end
+    (32, 4, 832, 128, 5),            # few rows, a width the int8 kernels do not take
+    (32, 4, 256, 128, 48), (32, 4, 256, 128, 49),     # six rows per expert: the last on the int8 kernels, the first beyond
+    (32, 4, 256, 128, 65), (32, 4, 256, 128, 385), (32, 4, 256, 128, 767), (32, 4, 256, 128, 768)])  # GEMM tile heights
+def test_moe_edges_of_the_paths(cuda_device, E, K, D, I, T):
+    rng = np.random.default_rng(800 + E + D + T)
+    layer, host = build_layer(rng, cuda_device, E, K, D, I, max_tokens=T)
+    check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
+
+
+@pytest.mark.parametrize("T", [3, 33, 257])
+def test_moe_mxfp4_low_tiles(cuda_device, T):
+    """MXFP4 experts on tiles of 32 and 64 rows, two CTAs per SM: an odd number of K steps (9), a last tile of features that is
+    not full in the down projection (576 = 4.5 x 128)."""
+    rng = np.random.default_rng(900 + T)
+    layer, host = build_layer(rng, cuda_device, 32, 4, 576, 192, fmt="mxfp4", act="swiglu_oai", biases=True, max_tokens=T)
+    check_layer(layer, host, synth.activations_np(rng, T, 576), T, "swiglu_oai")
+
+
+def test_router_tensor_logits_of_96_experts(cuda_device):
+    """The tensor-core logits with exact refinement where the experts do not fill the tile (96 of 128 columns)."""
+    rng = np.random.default_rng(950)
+    E, K, D, T = 96, 6, 1024, 600
+    layer, host = build_layer(rng, cuda_device, E, K, D, 64, max_tokens=T)
+    x = synth.activations_np(rng, T, D)
+    out = torch.zeros(T, D, dtype=torch.float32, device=cuda_device)
+    layer.encode(x_tensor(x, cuda_device), out, T)
+    v = layer.views(T)
+    logits = qref.router_logits(x, host["router"])
+    inds, wts = qref.route(logits, K)
+    got = v["logits"].cpu().numpy()
+    pick = inds.astype(np.int64)
+    assert np.array_equal(np.take_along_axis(got, pick, axis=1), np.take_along_axis(logits, pick, axis=1))
+    assert np.array_equal(v["inds"].cpu().numpy().astype(np.uint32), inds)
+    assert not got[:, E:].any()  # the columns past the experts
+    assert qref.max_rel(out.cpu().numpy(), qref.moe_ffn(x, inds, wts, host["weights"])) <= TOL
+
+
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("T", [1, 19, 300])
 def test_moe_shared_expert(cuda_device, T, gated):
