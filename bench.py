@@ -635,7 +635,7 @@ def run_ours(args):
         ms_gu = time_steps(torch, dist, 1, gateup_all, max(2, args.steps // 2), 1) / len(stack.layers)
         flops = 2.0 * t_n * TOPK * (2 * I) * D
         tf = flops / (ms_gu * 1e-3) / 1e12
-        traffic, traffic_src = profiled_traffic("qmm_tc_grouped_gateup_down_prefill4096.md") if t_n == PREFILL_TOKENS else (None, None)
+        traffic, traffic_src = profiled_traffic("qmm_ta_grouped_prefill4096.md") if t_n == PREFILL_TOKENS else (None, None)
         roof = {"kernel": "experts gate+up+SwiGLU (grouped)", "bound": "tensor", "achieved": round(tf, 2),
                 "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s", "frac": round(tf / peaks["bf16_tflops_sustained"], 4),
                 "traffic": traffic, "traffic_source": traffic_src,
