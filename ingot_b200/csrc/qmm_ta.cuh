@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.nc; i++) {
             mbar_init(bar_cfull + 8 * i, 1 + 32);  // the codes' copy, the scale producer's lanes
-            mbar_init(bar_cempty + 8 * i, 4 * (KPS < GROUPS ? KPS : GROUPS));
+            mbar_init(bar_cempty + 8 * i, 4 * GROUPS);
         }
         for (int i = 0; i < p.nx; i++) {
             mbar_init(bar_xfull + 8 * i, 1);
@@ -439,9 +439,13 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
             for (int ch = 0; ch < chunks; ch++) {
                 const int j0 = (grp - (int)it0 - ch * KPS) & (GROUPS - 1);  // this group's first step of the stage
-                if (j0 < KPS) {  // (8-bit codes have two steps per stage: two groups take it)
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar_cfull + 8 * cs, cph, abort_flag));
-                    if (!ok) break;
+                // Every group waits for every stage and hands it back, also those that hold no step of its own (8-bit codes have
+                // two steps per stage, for two of the four groups). A group that passed stages over could ask for the next round
+                // of one whose first codes had not arrived yet, which a phase bit answers with yes: with an odd number of
+                // stages it then converted a stage in flight and counted as its reader one round early.
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_cfull + 8 * cs, cph, abort_flag));
+                if (!ok) break;
+                if (j0 < KPS) {
                     const uint32_t codes = codes0 + cs * kTaCodeStage + row * 128, scales = scales0 + cs * SSTAGE + row * SPB;
 #pragma unroll
                     for (int i = 0; i < (KPS + GROUPS - 1) / GROUPS; i++) {
@@ -478,9 +482,9 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                         if (lane == 0) mbar_arrive(bar_aready + 8 * as);
                     }
                     if (!ok) break;
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_cempty + 8 * cs);
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_cempty + 8 * cs);
                 if (++cs == p.nc) { cs = 0; cph ^= 1; }
             }
             it0 += ksteps;

@@ -114,3 +114,19 @@ def test_qmm_tile_edges(cuda_device, fmt, M, N, K):
     assert qref.max_rel(y.cpu().numpy(), ref) <= TOL
     y2 = run_qmm(m, xt, M, accumulate=True, y=y.clone())
     assert torch.equal(y2, 2 * y)
+
+
+def test_qmm_8bit_stages_of_odd_number(cuda_device):
+    """64 rows at 8 bits: three stages of codes, each converted by two of the four groups; launches with the weights out of
+    L2 give the same bits every time."""
+    rng = np.random.default_rng(65)
+    M, N, K = 64, 2048, 4096
+    m, host = affine_case(rng, N, K, 8, cuda_device)
+    x = synth.activations_np(rng, M, K)
+    xt = x_tensor(x, cuda_device)
+    y = run_qmm(m, xt, M)
+    assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(x, deq(host, 8))) <= TOL
+    flush = torch.empty(160 << 20, dtype=torch.uint8, device=cuda_device)
+    for _ in range(20):
+        flush.zero_()
+        assert torch.equal(run_qmm(m, xt, M), y)
