@@ -101,10 +101,10 @@ def test_qmm_rejects_what_the_reference_rejects(cuda_device):
 
 
 @pytest.mark.parametrize("fmt", ["q4", "q8", "mxfp4"])
-@pytest.mark.parametrize("M,N,K", [(64, 64, 64), (192, 64, 192), (448, 192, 832), (1088, 2112, 320), (2048, 128, 1088)])
+@pytest.mark.parametrize("M,N,K", [(64, 64, 64), (192, 64, 192), (448, 192, 832), (1088, 2112, 320), (2048, 128, 1088), (64, 19008, 192)])
 def test_qmm_tile_edges(cuda_device, fmt, M, N, K):
     """Odd numbers of K steps (1, 3, 5, 13, 17: stages of codes that end early, scales whose row pitch allows no vector copy),
-    half tiles of output features, token tiles of other heights; accumulation onto an existing result."""
+    half tiles of output features, token tiles of other heights, more low tiles than SMs; accumulation onto an existing result."""
     rng = np.random.default_rng(M + N + K)
     m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, int(fmt[1]), cuda_device)
     x = synth.activations_np(rng, M, K)
