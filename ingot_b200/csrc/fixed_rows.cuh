@@ -8,7 +8,7 @@
 namespace iq {
 
 // Row r of an activation matrix as block fixed point: per group of 64 inputs 128 bytes, the high digits' fragments of the
-// four lanes of a quad (16 bytes each: two MMAs) and the low digits', and {2^(e-13), sum}.
+// four lanes of a quad (16 bytes each: two MMAs) and the low digits', and {2^(e-15), sum}.
 struct FixedRows {
     unsigned char* digits;  // [rows][groups][2][4][16]
     float2* scale;          // [rows][groups]
@@ -29,11 +29,11 @@ __device__ __forceinline__ void fixed_point_unit(const float (&v)[8], int w8, un
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
     }
     float sc, inv;
-    qi_group_scale(amax, sum, sc, inv);
+    qi_group_scale<8>(amax, sum, sc, inv);
     if (digits == nullptr) return;
     if (w8 == 0) *scale = make_float2(sc, sum);
     uint32_t hi_w[2], lo_w[2];
-    qi_digits8<false>(v, inv, hi_w, lo_w);
+    qi_digits8<false, 8>(v, inv, hi_w, lo_w);
     unsigned char* f = digits + (w8 >> 1) * 16 + (w8 & 1) * 8;
     *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
     *reinterpret_cast<uint2*>(f + 64) = make_uint2(lo_w[0], lo_w[1]);

@@ -165,7 +165,7 @@ __device__ __forceinline__ void small_load(SmallBatch& v, const unsigned char* w
         }
     }
 }
-// One group of the batch against one set of four activation rows: xb the lane's digits, xs its row's {2^(e-13), sum}.
+// One group of the batch against one set of four activation rows: xb the lane's digits, xs its row's {2^(e-15), sum}.
 __device__ __forceinline__ void small_mma(float (&acc)[2], const SmallBatch& v, int u, const uint4& xb, const float2& xs) {
     constexpr uint32_t MSK = 0x0F0F0F0Fu;
     const int z[4] = {0, 0, 0, 0};
@@ -173,7 +173,7 @@ __device__ __forceinline__ void small_mma(float (&acc)[2], const SmallBatch& v, 
     const uint2 w0 = v.q[u][0], w1 = v.q[u][1];
     imma16832_u8s8(d, w0.x & MSK, w1.x & MSK, (w0.x >> 4) & MSK, (w1.x >> 4) & MSK, xb.x, xb.y, z);
     imma16832_u8s8(d, w0.y & MSK, w1.y & MSK, (w0.y >> 4) & MSK, (w1.y >> 4) & MSK, xb.z, xb.w, d);
-    const float v0 = (float)(d[0] * 128 + d[1]), v1 = (float)(d[2] * 128 + d[3]);
+    const float v0 = (float)(d[0] * 256 + d[1]), v1 = (float)(d[2] * 256 + d[3]);
     const float s0 = __uint_as_float(u ? (v.s[0] & 0xFFFF0000u) : (v.s[0] << 16)), s1 = __uint_as_float(u ? (v.s[1] & 0xFFFF0000u) : (v.s[1] << 16));
     const float b0 = __uint_as_float(u ? (v.b[0] & 0xFFFF0000u) : (v.b[0] << 16)), b1 = __uint_as_float(u ? (v.b[1] & 0xFFFF0000u) : (v.b[1] << 16));
     acc[0] = fmaf(v0, s0 * xs.x, acc[0]);
@@ -266,11 +266,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(cons
             amax = fmaxf(gmax[warp & ~1], gmax[warp | 1]);
             sum = gsum[warp & ~1] + gsum[warp | 1];
             float sc, inv;
-            qi_group_scale(amax, sum, sc, inv);
+            qi_group_scale<8>(amax, sum, sc, inv);
             const size_t rec = pos * NB + n0 / 64;
             if (f == 0) p.fh.scale[rec] = make_float2(sc, sum);
             const int X = __float2int_rn(hv * inv);
-            const int hi_d = (X + 64) >> 7, lo_d = X - (hi_d << 7);
+            const int hi_d = (X + 128) >> 8, lo_d = X - (hi_d << 8);
             unsigned char* d = p.fh.digits + rec * 128 + ((f >> 4) & 3) * 16 + ((f >> 3) & 1) * 8 + (f & 1) * 4 + ((f & 7) >> 1);
             d[0] = (unsigned char)(hi_d & 0xFF);
             d[64] = (unsigned char)(lo_d & 0xFF);

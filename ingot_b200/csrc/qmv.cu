@@ -213,7 +213,7 @@ int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk
         unsigned char* digits = static_cast<unsigned char*>(c.scratch);
         float2* scale = reinterpret_cast<float2*>(digits + c.rows * rec);
         auto k = c.fmt == kFmtAffine8 ? qr_convert_kernel<true, false> : c.fmt == kFmtAffine4G32 ? qr_convert_kernel<false, true> : qr_convert_kernel<false, false>;
-        const int32_t r = check_cuda(ctx, launch_dependent(k, dim3((units + 255) / 256), 256, 0, st, c.x, c.x_dtype, c.ldx, c.K, c.rows, digits, scale), "qr_convert launch");
+        const int32_t r = check_cuda(ctx, launch_dependent(k, dim3((units + 255) / 256), 256, 0, st, c.x, c.x_dtype, c.ldx, c.K, c.rows, wk8 ? 7 : 8, digits, scale), "qr_convert launch");
         if (r != kOk) return r;
         p.xd = digits;
         p.xs = scale;

@@ -112,30 +112,40 @@ __device__ __forceinline__ void unpack6x16(uint32_t w0, uint32_t w1, uint32_t w2
     o[3] = spread6(w2 >> 8);
 }
 
-// Eight activations as two signed 7-bit digits each: X = round(v * inv), |X| <= 8192, hi = (X + 64) >> 7, lo = X - 128 hi; words
-// of four digits, [b0 / b1 half]: 4-bit codes put even k in the low nibbles (b0) and odd k in the high ones (b1), 8-bit codes
-// put k 0-3 in one word and k 4-7 in the next. The rounding is the addition of 1.5 * 2^23 (+ 64), which leaves X + 64 in the
-// low bits, and four digits go through the shifts and masks at a time: 26 instructions, not 80 (the conversion is every CTA's
-// prologue and was a third of all instructions of a launch of four rows and 14336 inputs).
-template <bool W8>
+// Eight activations as two signed digits of BITS bits each: X = round(v * inv), hi = (X + 2^(BITS-1)) >> BITS, lo = X - 2^BITS hi;
+// words of four digits, [b0 / b1 half]: 4-bit codes put even k in the low nibbles (b0) and odd k in the high ones (b1), 8-bit
+// codes put k 0-3 in one word and k 4-7 in the next. The rounding is the addition of 1.5 * 2^23 (+ 2^(BITS-1)), which leaves
+// X + 2^(BITS-1) in the low bits, and four digits go through the shifts and masks at a time. The conversion is every CTA's
+// prologue and was a third of all instructions of a launch of four rows and 14336 inputs at 80 per eight inputs.
+// 7 bits: this file's kernel and the ring kernel where it stands in for it. 8 bits: the kernels that took over from fp16 MMAs,
+// whose activations had 11 bits of their own: a gated h has groups whose largest value is ten times the usual one, and 14 bits
+// of that were 1.0e-3 of an FFN's output off the fp16 kernels', 16 bits are 4e-4 (the fp16 weights' rounding).
+template <bool W8, int BITS>
 __device__ __forceinline__ void qi_digits8(const float (&v)[8], float inv, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         uint32_t f[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) f[i] = __float_as_uint(fmaf(v[W8 ? 4 * h + i : 2 * i + h], inv, 12582976.0f));
-        const uint32_t p0 = __byte_perm(f[0], f[1], 0x5410), p1 = __byte_perm(f[2], f[3], 0x5410);
-        hi[h] = __byte_perm(p0 >> 7, p1 >> 7, 0x6420);
-        const uint32_t l = (__byte_perm(p0, p1, 0x6420) & 0x7F7F7F7Fu) ^ 0x40404040u;  // seven bits, sign flipped back ...
-        lo[h] = l + ((l & 0x40404040u) << 1);                                           // ... and extended
+        for (int i = 0; i < 4; i++) f[i] = __float_as_uint(fmaf(v[W8 ? 4 * h + i : 2 * i + h], inv, 12582912.0f + (1 << (BITS - 1))));
+        if (BITS == 8) {
+            const uint32_t p0 = __byte_perm(f[0], f[1], 0x5140), p1 = __byte_perm(f[2], f[3], 0x5140);  // first bytes, second bytes
+            hi[h] = __byte_perm(p0, p1, 0x7632);
+            lo[h] = __byte_perm(p0, p1, 0x5410) ^ 0x80808080u;
+        } else {
+            const uint32_t p0 = __byte_perm(f[0], f[1], 0x5410), p1 = __byte_perm(f[2], f[3], 0x5410);
+            hi[h] = __byte_perm(p0 >> 7, p1 >> 7, 0x6420);
+            const uint32_t l = (__byte_perm(p0, p1, 0x6420) & 0x7F7F7F7Fu) ^ 0x40404040u;  // seven bits, sign flipped back ...
+            lo[h] = l + ((l & 0x40404040u) << 1);                                           // ... and extended
+        }
     }
 }
 
 // Block fixed point of one group of 64 activations: from the group's largest magnitude and its sum, the power of two
-// 2^(e-13) the digits are counted in (2^e > amax >= 2^(e-1)) and its inverse. A group that holds a NaN or an infinity
+// 2^(e-2*BITS+1) the digits are counted in (2^e > amax >= 2^(e-1)) and its inverse. A group that holds a NaN or an infinity
 // (amax or the sum not finite; fmaxf drops a NaN, the sum keeps it) gets a NaN scale and a NaN sum, so that every output
 // it feeds comes out NaN, where the fp16 kernels and an fp32 matrix product give NaN or an infinity: a non-finite input
 // must not turn into a finite output. Groups whose largest magnitude is below 2^-100 count as zero.
+template <int BITS>
 __device__ __forceinline__ void qi_group_scale(float amax, float& sum, float& scale, float& inv) {
     scale = 0.f;
     inv = 0.f;
@@ -145,10 +155,12 @@ __device__ __forceinline__ void qi_group_scale(float amax, float& sum, float& sc
         return;
     }
     if (amax > 0.f) {
-        const int e = (int)((__float_as_uint(amax) >> 23) & 0xFF) - 126;
+        int e = (int)((__float_as_uint(amax) >> 23) & 0xFF) - 126;
+        // (8 bits: the last 0.4 % below a power of two would leave the high digit's range)
+        if (BITS == 8 && (__float_as_uint(amax) & 0x7FFFFFu) >= 0x7EFF00u) e++;
         if (e > -100) {
-            scale = __uint_as_float((uint32_t)(e - 13 + 127) << 23);
-            inv = __uint_as_float((uint32_t)(13 - e + 127) << 23);
+            scale = __uint_as_float((uint32_t)(e - 2 * BITS + 1 + 127) << 23);
+            inv = __uint_as_float((uint32_t)(2 * BITS - 1 - e + 127) << 23);
         }
     }
 }
@@ -418,10 +430,10 @@ __global__ void __launch_bounds__(kQiMaxThreads, MS == 1 ? 2 : 1)
                 sum += __shfl_xor_sync(0xffffffffu, sum, o);
             }
             float scale, inv;
-            qi_group_scale(amax, sum, scale, inv);
+            qi_group_scale<7>(amax, sum, scale, inv);
             if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(scale, sum);
             uint32_t hi_w[2], lo_w[2];
-            qi_digits8<W8>(v, inv, hi_w, lo_w);
+            qi_digits8<W8, 7>(v, inv, hi_w, lo_w);
             // the span is word w8 of the group's eight (4-bit: lane t = w8 / 2, MMA w8 % 2) or words 2 w8, 2 w8 + 1 of
             // its sixteen (8-bit: lane t = w8 / 2, MMA w8 % 2): the same slot either way
             const int t = w8 >> 1, mm = w8 & 1;

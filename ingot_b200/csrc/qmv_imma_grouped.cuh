@@ -1,7 +1,7 @@
 // MoE decode on the int8 tensor-core path: the expert tiles' gate + up + activation and down projections for tiles of
 // up to eight routed rows (affine 4-bit experts). Same arithmetic as qmv_imma.cuh: codes enter m16n8k32 u8 x s8 MMAs
-// unconverted, the tile's activation rows are converted once per tile to block fixed point (two signed 7-bit digits per
-// group of 64 inputs), per group y += s * 2^(e-13) * (128 * acc_hi + acc_lo) + b * sum(x); a row's bits do not depend on
+// unconverted, the tile's activation rows are converted once per tile to block fixed point (two signed 8-bit digits per
+// group of 64 inputs), per group y += s * 2^(e-15) * (256 * acc_hi + acc_lo) + b * sum(x); a row's bits do not depend on
 // the other rows of its tile.
 //
 // Work items are (tile, block of R = 16 * rgs weight rows); a CTA takes a contiguous range of items, so a tile's
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
     static_assert(!FX || (GW > 0 && TM && MODE == kModeGateUp), "sixteen consumer warps: the gate/up form with fragments in registers");
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char* xq = smem;                                            // [groups][MS][32 lanes] uint4: B fragments
-    float2* xsc = reinterpret_cast<float2*>(smem + p.xq_bytes);          // [groups][MS * 4 rows] {2^(e-13), sum x}
+    float2* xsc = reinterpret_cast<float2*>(smem + p.xq_bytes);          // [groups][MS * 4 rows] {2^(e-15), sum x}
     float* red = reinterpret_cast<float*>(smem + p.xq_bytes + p.xsc_bytes);  // [2][kQgWarps][NW * MS][32 lanes][2]
     unsigned char* stages = smem + p.xq_bytes + p.xsc_bytes + p.red_bytes;
     if (TM) stages += (1024u - (smem_u32(stages) & 1023u)) & 1023u;  // the swizzle pattern is a function of the address
@@ -330,11 +330,11 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
                             sum += __shfl_xor_sync(0xffffffffu, sum, o);
                         }
                         float scale, inv;
-                        qi_group_scale(amax, sum, scale, inv);
+                        qi_group_scale<8>(amax, sum, scale, inv);
                         if (!live) continue;
                         if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(scale, sum);
                         uint32_t hi_w[2], lo_w[2];
-                        qi_digits8<false>(v[k4], inv, hi_w, lo_w);
+                        qi_digits8<false, 8>(v[k4], inv, hi_w, lo_w);
                         const int tt = w8 >> 1, mm = w8 & 1;
                         const int fb = ((j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * 16 + mm * 8;
                         *reinterpret_cast<uint2*>(xq + fb + tt * 16) = make_uint2(hi_w[0], hi_w[1]);
@@ -431,8 +431,8 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
                                 const float bi1 = __uint_as_float(q1 ? (b1w[i] & 0xFFFF0000u) : (b1w[i] << 16));
 #pragma unroll
                                 for (int c = 0; c < NS; c++) {
-                                    const float v0 = (float)(d[i][c][0] * 128 + d[i][c][1]);
-                                    const float v1 = (float)(d[i][c][2] * 128 + d[i][c][3]);
+                                    const float v0 = (float)(d[i][c][0] * 256 + d[i][c][1]);
+                                    const float v1 = (float)(d[i][c][2] * 256 + d[i][c][3]);
                                     acc[i][c][0] = fmaf(v0, sc0 * xs[c].x, acc[i][c][0]);
                                     acc[i][c][0] = fmaf(bi0, xs[c].y, acc[i][c][0]);
                                     acc[i][c][1] = fmaf(v1, sc1 * xs[c].x, acc[i][c][1]);

@@ -2,7 +2,7 @@
 // multiple of 64, groups of 32, rows longer than its stages, and the gate + up + activation form of the dense FFN.
 //
 // Same arithmetic: codes enter m16n8k32 u8 x s8 unconverted, the activations are converted once per CTA to block fixed
-// point per group (two signed 7-bit digits, see qmv_imma.cuh), per group y += s * 2^(e-13) * (128 * acc_hi + acc_lo) +
+// point per group (two signed 8-bit digits, see qmv_imma.cuh), per group y += s * 2^(e-15) * (256 * acc_hi + acc_lo) +
 // b * sum(x); a row's bits do not depend on the other rows of the call.
 //
 // Bound: HBM, which wants 45 KB and more under way per SM all the time. Weights loaded into registers a batch ahead came to 16
@@ -28,7 +28,7 @@ constexpr int kQrBox = 2048;  // bytes of a slot's codes per matrix
 
 // Eight inputs (unit w8 of a group, its threads neighbouring lanes) as block fixed point, in B-fragment order: the high digits
 // at f, the low ones four lanes' fragments on.
-template <bool W8, bool G32>
+template <bool W8, bool G32, int BITS>
 __device__ __forceinline__ void qr_convert(const float (&v)[8], int w8, bool live, unsigned char* rec, float2* scale_out) {
     constexpr int TPG = G32 ? 4 : 8, XL = G32 ? 8 : 16;
     float amax = 0.f, sum = 0.f;
@@ -43,11 +43,11 @@ __device__ __forceinline__ void qr_convert(const float (&v)[8], int w8, bool liv
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
     }
     float scale, inv;
-    qi_group_scale(amax, sum, scale, inv);
+    qi_group_scale<BITS>(amax, sum, scale, inv);
     if (!live) return;
     if (w8 == 0) *scale_out = make_float2(scale, sum);
     uint32_t hi_w[2], lo_w[2];
-    qi_digits8<W8>(v, inv, hi_w, lo_w);
+    qi_digits8<W8, BITS>(v, inv, hi_w, lo_w);
     unsigned char* f = rec + (G32 ? w8 * 8 : (w8 >> 1) * 16 + (w8 & 1) * 8);
     *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
     *reinterpret_cast<uint2*>(f + 4 * XL) = make_uint2(lo_w[0], lo_w[1]);
@@ -56,7 +56,7 @@ __device__ __forceinline__ void qr_convert(const float (&v)[8], int w8, bool liv
 // The rows of a call converted once, for CTAs that would each spend longer on it: [rows][groups] records of the digits (128
 // bytes; groups of 32: 64) and of {scale, sum}. 256 threads, a unit of eight inputs each.
 template <bool W8, bool G32>
-__global__ void __launch_bounds__(256) qr_convert_kernel(const void* x, int32_t x_dtype, int64_t ldx, int K, int M, unsigned char* digits, float2* scale) {
+__global__ void __launch_bounds__(256) qr_convert_kernel(const void* x, int32_t x_dtype, int64_t ldx, int K, int M, int bits, unsigned char* digits, float2* scale) {
     constexpr int TPG = G32 ? 4 : 8, REC = G32 ? 64 : 128;
     pdl_launch_dependents();
     pdl_wait();
@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(256) qr_convert_kernel(const void* x, int32_t 
     float v[8];
     load_x8(x, x_dtype, (size_t)(uc / (K / 8)) * ldx + (uc % (K / 8)) * 8, v);
     const size_t rec = uc / TPG;  // (K is a multiple of the group)
-    qr_convert<W8, G32>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
+    if (bits == 7) qr_convert<W8, G32, 7>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
+    else qr_convert<W8, G32, 8>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
 }
 
 struct QrMaps {
@@ -84,7 +85,7 @@ struct QrParams {
     int32_t act;           // gate/up form: activation
     float limit;
     int32_t wk, depth;     // K slices; slots per warp
-    int32_t runs;          // slices are runs of columns (else every wk-th column: 5 % faster)
+    int32_t runs;          // as the staged kernel: 7-bit digits, slices are runs of columns (else every wk-th column: 5 % faster)
     const unsigned char* xd;  // the rows as qr_convert_kernel left them, or null: converted here, from x
     const float2* xs;
     int32_t* status;
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
     const int nwarps = blockDim.x >> 5, depth = p.depth;
     const int G = p.K / GS, ncol = (G + GPC - 1) / GPC;
     unsigned char* xq = smem + (size_t)nwarps * depth * NW * kQrBox;               // [groups][MS][32 lanes] XL bytes
-    float2* xsc = reinterpret_cast<float2*>(xq + (size_t)G * MS * 32 * XL);        // [groups][MS * 4 rows] {2^(e-13), sum x}
+    float2* xsc = reinterpret_cast<float2*>(xq + (size_t)G * MS * 32 * XL);        // [groups][MS * 4 rows] {2^(e-15), sum x}
     float* red = reinterpret_cast<float*>(xsc + (size_t)G * MS * 4);               // [2][warps][NW * MS * 64]
     uint32_t* srings = reinterpret_cast<uint32_t*>(red + (size_t)2 * nwarps * NW * MS * 64);
     uint64_t* bars = reinterpret_cast<uint64_t*>(srings + (size_t)nwarps * depth * NW * 2 * 16 * SPW);
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
     for (int i = 0; i < depth; i++) issue();  // the weights do not depend on the previous kernel of the stream
     pdl_wait();
 
-    // ---- activations -> block fixed point, two 7-bit digits, in B-fragment order (see qmv_imma.cuh) ---------------------
+    // ---- activations -> block fixed point, two 8-bit digits, in B-fragment order (see qmv_imma.cuh) ---------------------
     const int nthreads = nwarps * 32;
     for (int u = tid; u < G * TPG * (4 * MS - p.M); u += nthreads) {  // rows the call does not have: zero digits and scale
         const int m = p.M + u / (G * TPG), j = (u / TPG) % G, w8 = u % TPG;
@@ -198,7 +199,9 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
     const int units = p.xd != nullptr ? 0 : G * TPG * p.M, upad = (units + 31) / 32 * 32;  // whole warps: the groups' shuffles need their threads
     auto convert = [&](const float (&v)[8], int u) {
         const int m = u / (G * TPG), j = (u / TPG) % G;
-        qr_convert<W8, G32>(v, u % TPG, u < units, xq + ((size_t)(j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * XL, xsc + j * 4 * MS + m);
+        unsigned char* rec = xq + ((size_t)(j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * XL;
+        if (p.runs) qr_convert<W8, G32, 7>(v, u % TPG, u < units, rec, xsc + j * 4 * MS + m);
+        else qr_convert<W8, G32, 8>(v, u % TPG, u < units, rec, xsc + j * 4 * MS + m);
     };
     if (units <= 2 * nthreads) {
         for (int u = tid; u < upad; u += nthreads) {
@@ -228,6 +231,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
 
     const uint32_t xq32 = smem_u32(xq) + lane * XL, xsc32 = smem_u32(xsc) + t * 8;
     auto bf = [](uint32_t w, int hi_half) { return __uint_as_float(hi_half ? (w & 0xFFFF0000u) : (w << 16)); };
+    const int radix = p.runs ? 128 : 256;
     const bool shifted = odd_rows && (g & 1);  // rows g and g + 8 start in the middle of a word
     int slot = 0;
     uint32_t ph = 0;
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
                         }
 #pragma unroll
                         for (int c = 0; c < MS; c++) {
-                            const float v0 = (float)(d[c][0] * 128 + d[c][1]), v1 = (float)(d[c][2] * 128 + d[c][3]);
+                            const float v0 = (float)(d[c][0] * radix + d[c][1]), v1 = (float)(d[c][2] * radix + d[c][3]);
                             acc[i][c][0] = fmaf(v0, sc0 * xs[c].x, acc[i][c][0]);
                             acc[i][c][0] = fmaf(bi0, xs[c].y, acc[i][c][0]);
                             acc[i][c][1] = fmaf(v1, sc1 * xs[c].x, acc[i][c][1]);
