@@ -87,22 +87,26 @@ class DenseQ:
         self.w, self.s, self.b = w.contiguous(), scales.contiguous(), None if biases is None else biases.contiguous()
         self.N, self.K, self.bits, self.gs, self.mode, self.experts = N, K, bits, gs, mode, experts
 
-    # what the C description of the matrix is made of: assigning one of these drops the cached description
+    # What the C description of the matrix is made of: assigning one of these starts another generation, and a description is
+    # used in the generation it was built in only.
     _DESCRIBED = frozenset(("w", "s", "b", "N", "K", "bits", "gs", "mode", "experts"))
-    _ql, _ql_address, _ctx = None, 0, None
+    _ql, _ctx, _generation = None, None, None
 
     def __setattr__(self, name, value):
         object.__setattr__(self, name, value)
-        if name in self._DESCRIBED and self._ql is not None:
-            object.__setattr__(self, "_ql", None)
+        if name in self._DESCRIBED:
+            object.__setattr__(self, "_generation", object())
 
-    def _described(self) -> int:
-        """Address of the matrix's C description, built once (a decode step passes the same matrices over and over)."""
-        q = self._ql
-        if q is None or q.w != self.w.data_ptr():  # (the storage may have been exchanged under the tensor)
-            q = self._ql = self.qlinear()
-            self._ql_address = C.addressof(q)
-        return self._ql_address
+    def _described(self) -> tuple:
+        """(address of the matrix's C description, the description, its generation), built once: a decode step passes the same
+        matrices over and over. The caller holds the tuple over its call: the address is the description's as long as somebody
+        holds it, and another thread may assign to the matrix while a launch runs without the interpreter lock. One attribute
+        for all of it: a thread that finds it finds a whole description."""
+        d, generation = self._ql, self._generation
+        if d is None or d[2] is not generation or d[1].w != self.w.data_ptr():  # (the storage may have been exchanged under the tensor)
+            q = self.qlinear()
+            d = self._ql = (C.addressof(q), q, generation)
+        return d
 
     def _context(self) -> capi.Context:
         ctx = self._ctx
@@ -166,7 +170,8 @@ class DenseQ:
                                                        tok.data_ptr(), rows, 0 if out_f is None else out_f.data_ptr(),
                                                        0 if out_h is None else out_h.data_ptr(), o.stride(0)))
             return
-        ctx.check(capi.call().embed_rows(ctx.address, _stream_ptr(stream), self._described(), tok.data_ptr(), rows,
+        d = self._described()
+        ctx.check(capi.call().embed_rows(ctx.address, _stream_ptr(stream), d[0], tok.data_ptr(), rows,
                                          0 if out_f is None else out_f.data_ptr(),
                                          0 if out_h is None else out_h.data_ptr(), o.stride(0)))
 
@@ -188,7 +193,8 @@ class DenseQ:
         if self.had is not None:  # rotated basis: the rotation runs first, as in the reference's launcher
             x = self.encode_rotate(x, rows, stream)
         ws_ptr, ws_bytes = (0, 0) if workspace is None else (workspace.data_ptr(), workspace.numel() * workspace.element_size())
-        st = capi.call().qmm(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), self._described(), y.data_ptr(),
+        d = self._described()
+        st = capi.call().qmm(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), d[0], y.data_ptr(),
                              _dtype_id(y), y.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, ws_ptr, ws_bytes)
         if st:
             ctx.check(st)
@@ -255,7 +261,8 @@ class VQMV:
             ldx = x.stride(0) if x.dim() > 1 else m.K
         if ldy is None:
             ldy = y.stride(0) if y.dim() > 1 else m.N
-        st = capi.call().qmv(ctx.address, _stream_ptr(stream), x.data_ptr(), _DT.get(x.dtype, -1), ldx, m._described(), y.data_ptr(),
+        d = m._described()
+        st = capi.call().qmv(ctx.address, _stream_ptr(stream), x.data_ptr(), _DT.get(x.dtype, -1), ldx, d[0], y.data_ptr(),
                              _DT.get(y.dtype, -1), ldy, rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, n_prefix or 0)
         if st:
             _dtype_id(x), _dtype_id(y)  # a type the library does not know is a TypeError
@@ -295,7 +302,8 @@ class DenseMLP:
             _no_cpu()
         ctx = self.gate_up._context()
         ws = self._workspace(rows, x.dtype)
+        a, b = self.gate_up._described(), self.down._described()
         ctx.check(capi.call().dense_ffn(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
-                                        self.gate_up._described(), self.down._described(), self.act, self.limit, out.data_ptr(),
+                                        a[0], b[0], self.act, self.limit, out.data_ptr(),
                                         _dtype_id(out), out.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0,
                                         ws.data_ptr(), ws.numel()))

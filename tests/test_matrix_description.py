@@ -1,0 +1,93 @@
+"""The C description of a matrix that the hot calls keep (DenseQ._described), with stand-ins for the library and for device
+tensors: what it says, how long it lives and when it is built again."""
+import types
+
+import pytest
+import torch
+
+from ingot_b200 import capi, linear
+from ingot_b200.linear import DenseQ, VQMV
+
+
+def bare_matrix(N=16, K=64):
+    m = DenseQ.__new__(DenseQ)  # (the constructor refuses CPU tensors)
+    m.had, m._rot = None, None
+    m.w, m.s, m.b = torch.zeros(N, K // 8, dtype=torch.int32), torch.zeros(N, 1, dtype=torch.bfloat16), torch.zeros(N, 1, dtype=torch.bfloat16)
+    m.N, m.K, m.bits, m.gs, m.mode, m.experts = N, K, 4, 64, "affine", 1
+    return m
+
+
+def rows(n, k, dtype=torch.float32):
+    t = torch.zeros(n, k, dtype=dtype)
+    return types.SimpleNamespace(is_cuda=True, dtype=dtype, dim=t.dim, stride=t.stride, data_ptr=t.data_ptr, keep=t)
+
+
+@pytest.fixture
+def fake(monkeypatch):
+    """capi with a context and calls that record what they are given."""
+    f = types.SimpleNamespace(seen=[], during=lambda: None)
+
+    def qmv(ctx, stream, x, xd, ldx, q, *rest):
+        f.during()
+        d = capi.QLinear.from_address(q)
+        f.seen.append((d.w, d.scales, d.biases, d.n, d.k))
+        return 0
+
+    monkeypatch.setattr(capi, "context", lambda device=0: types.SimpleNamespace(address=1, check=lambda st: None, device=device))
+    monkeypatch.setattr(capi, "call", lambda: types.SimpleNamespace(qmv=qmv))
+    return f
+
+
+def encode(m):
+    VQMV.encode(rows(1, m.K), m, rows(1, m.N), 1, stream=types.SimpleNamespace(cuda_stream=0))
+
+
+def test_description_outlives_an_assignment_during_the_call(fake, monkeypatch):
+    """Another thread may assign to the matrix while a launch runs without the interpreter lock: what the call reads stays."""
+    freed = []
+
+    class Tracked(capi.QLinear):
+        def __del__(self):
+            freed.append(True)
+
+    monkeypatch.setattr(linear.capi, "QLinear", Tracked)
+    m = bare_matrix()
+    w0 = m.w
+
+    def during():
+        m.w = torch.ones_like(w0)
+        assert not freed
+
+    fake.during = during
+    encode(m)
+    assert fake.seen[0][0] == w0.data_ptr()
+
+
+def test_description_is_whole_for_a_second_thread(fake):
+    """A thread that finds the cached description finds its address too: the second thread is let in wherever the first one
+    stores something."""
+    inner = []
+
+    class Interleaved(DenseQ):
+        def __setattr__(self, name, value):
+            super().__setattr__(name, value)
+            if name == "_ql" and value is not None:
+                encode(self)
+                inner.append(fake.seen[-1])
+
+    m = bare_matrix()
+    m.__class__ = Interleaved
+    encode(m)
+    want = (m.w.data_ptr(), m.s.data_ptr(), m.b.data_ptr(), m.N, m.K)
+    assert inner == [want] and fake.seen[-1] == want
+
+
+def test_description_follows_assignments(fake):
+    m = bare_matrix()
+    encode(m)
+    first = m._described()
+    assert m._described() is first  # built once
+    m.w, m.N = torch.zeros(32, 8, dtype=torch.int32), 32
+    m.s, m.b = torch.zeros(32, 1, dtype=torch.bfloat16), torch.zeros(32, 1, dtype=torch.bfloat16)
+    encode(m)
+    assert fake.seen[-1] == (m.w.data_ptr(), m.s.data_ptr(), m.b.data_ptr(), 32, 64)
