@@ -98,14 +98,16 @@ class DenseQ:
             object.__setattr__(self, "_generation", object())
 
     def _described(self) -> tuple:
-        """(address of the matrix's C description, the description, its generation), built once: a decode step passes the same
-        matrices over and over. The caller holds the tuple over its call: the address is the description's as long as somebody
+        """(address of the matrix's C description, the description, its generation, its three pointers), built once: a decode step
+        passes the same matrices over and over. The caller holds the tuple over its call: the address is the description's as long as somebody
         holds it, and another thread may assign to the matrix while a launch runs without the interpreter lock. One attribute
         for all of it: a thread that finds it finds a whole description."""
-        d, generation = self._ql, self._generation
-        if d is None or d[2] is not generation or d[1].w != self.w.data_ptr():  # (the storage may have been exchanged under the tensor)
+        d, generation, s, b = self._ql, self._generation, self.s, self.b
+        w, s, b = self.w.data_ptr(), 0 if s is None else s.data_ptr(), 0 if b is None else b.data_ptr()
+        # (the storages may have been exchanged under the tensors)
+        if d is None or d[2] is not generation or d[3] != w or d[4] != s or d[5] != b:
             q = self.qlinear()
-            d = self._ql = (C.addressof(q), q, generation)
+            d = self._ql = (C.addressof(q), q, generation, q.w or 0, q.scales or 0, q.biases or 0)
         return d
 
     def _context(self) -> capi.Context:

@@ -91,3 +91,13 @@ def test_description_follows_assignments(fake):
     m.s, m.b = torch.zeros(32, 1, dtype=torch.bfloat16), torch.zeros(32, 1, dtype=torch.bfloat16)
     encode(m)
     assert fake.seen[-1] == (m.w.data_ptr(), m.s.data_ptr(), m.b.data_ptr(), 32, 64)
+
+
+@pytest.mark.parametrize("name", ["w", "s", "b"])
+def test_description_follows_an_exchanged_storage(fake, name):
+    """t.data = ... exchanges the memory under a tensor without an assignment to the matrix."""
+    m = bare_matrix()
+    encode(m)
+    getattr(m, name).data = torch.ones_like(getattr(m, name))
+    encode(m)
+    assert fake.seen[-1] == (m.w.data_ptr(), m.s.data_ptr(), m.b.data_ptr(), m.N, m.K)
