@@ -97,6 +97,10 @@ class DenseQ:
         if name in self._DESCRIBED:
             object.__setattr__(self, "_generation", object())
 
+    def __getstate__(self):
+        # copies and pickles take the matrix, not the addresses and handles kept beside it
+        return {k: v for k, v in self.__dict__.items() if k not in ("_ql", "_ctx", "_generation")}
+
     def _described(self) -> tuple:
         """(address of the matrix's C description, the description, its generation, its three pointers), built once: a decode step
         passes the same matrices over and over. The caller holds the tuple over its call: the address is the description's as long as somebody

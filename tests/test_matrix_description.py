@@ -1,5 +1,7 @@
 """The C description of a matrix that the hot calls keep (DenseQ._described), with stand-ins for the library and for device
 tensors: what it says, how long it lives and when it is built again."""
+import copy
+import pickle
 import types
 
 import pytest
@@ -101,3 +103,14 @@ def test_description_follows_an_exchanged_storage(fake, name):
     getattr(m, name).data = torch.ones_like(getattr(m, name))
     encode(m)
     assert fake.seen[-1] == (m.w.data_ptr(), m.s.data_ptr(), m.b.data_ptr(), m.N, m.K)
+
+
+def test_a_used_matrix_copies_and_pickles(fake):
+    m = bare_matrix()
+    encode(m)
+    m._ctx = capi.Context.__new__(capi.Context)  # (a context holds a C pointer: neither copies nor pickles)
+    m._ctx._h = capi.C.c_void_p()
+    for c in (copy.copy(m), copy.deepcopy(m), pickle.loads(pickle.dumps(m))):
+        encode(c)
+        assert fake.seen[-1] == (c.w.data_ptr(), c.s.data_ptr(), c.b.data_ptr(), m.N, m.K)
+    assert copy.deepcopy(m).w.data_ptr() != m.w.data_ptr()
