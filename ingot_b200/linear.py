@@ -90,7 +90,7 @@ class DenseQ:
     # What the C description of the matrix is made of: assigning one of these starts another generation, and a description is
     # used in the generation it was built in only.
     _DESCRIBED = frozenset(("w", "s", "b", "N", "K", "bits", "gs", "mode", "experts"))
-    _ql, _ctx, _generation = None, None, None
+    _ql, _generation = None, None
 
     def __setattr__(self, name, value):
         object.__setattr__(self, name, value)
@@ -99,26 +99,20 @@ class DenseQ:
 
     def __getstate__(self):
         # copies and pickles take the matrix, not the addresses and handles kept beside it
-        return {k: v for k, v in self.__dict__.items() if k not in ("_ql", "_ctx", "_generation")}
+        return {k: v for k, v in self.__dict__.items() if k not in ("_ql", "_generation")}
 
     def _described(self) -> tuple:
-        """(address of the matrix's C description, the description, its generation, its three pointers), built once: a decode step
-        passes the same matrices over and over. The caller holds the tuple over its call: the address is the description's as long as somebody
-        holds it, and another thread may assign to the matrix while a launch runs without the interpreter lock. One attribute
-        for all of it: a thread that finds it finds a whole description."""
+        """(address of the matrix's C description, the description, its generation, its three pointers, the context of its device),
+        built once: a decode step passes the same matrices over and over. The caller holds the tuple over its call: the
+        address is good as long as somebody holds the description, and another thread may assign to the matrix while a launch
+        runs without the interpreter lock. One attribute for all of it: a thread that finds it finds a whole description."""
         d, generation, s, b = self._ql, self._generation, self.s, self.b
         w, s, b = self.w.data_ptr(), 0 if s is None else s.data_ptr(), 0 if b is None else b.data_ptr()
         # (the storages may have been exchanged under the tensors)
-        if d is None or d[2] is not generation or d[3] != w or d[4] != s or d[5] != b:
+        if d is None or d[2] is not generation or d[3] != w or d[4] != s or d[5] != b or d[6].address == 0:
             q = self.qlinear()
-            d = self._ql = (C.addressof(q), q, generation, q.w or 0, q.scales or 0, q.biases or 0)
+            d = self._ql = (C.addressof(q), q, generation, q.w or 0, q.scales or 0, q.biases or 0, capi.context(self.device_index))
         return d
-
-    def _context(self) -> capi.Context:
-        ctx = self._ctx
-        if ctx is None or ctx.address == 0:
-            ctx = self._ctx = capi.context(self.device_index)
-        return ctx
 
     def qlinear(self) -> capi.QLinear:
         return capi.QLinear(self.w.data_ptr(), 0 if self.s is None else self.s.data_ptr(),
@@ -147,7 +141,7 @@ class DenseQ:
         """x[rows, K] rotated into a float16 scratch (grown on demand, like the reference's rotation buffer)."""
         if self._rot is None or self._rot.shape[0] < rows:
             self._rot = torch.empty(max(rows, 16), self.K, dtype=torch.float16, device=self.w.device)
-        ctx = self._context()
+        ctx = self._described()[6]
         ctx.check(capi.call().had_rows(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
                                        self.had.data_ptr(), self._rot.data_ptr(), self.K, rows, self.K))
         return self._rot
@@ -167,7 +161,8 @@ class DenseQ:
         if out_f is not None and out_h is not None and out_f.stride(0) != out_h.stride(0):
             raise ValueError("out_f and out_h share one row stride")
         o = out_f if out_f is not None else out_h
-        ctx = self._context()
+        d = self._described()
+        ctx = d[6]
         if self.bits == 2:  # ternary table: dequantise, then the inverse rotation (embed_rows_t, xc_tern.metal:44-65)
             if self.had is None:
                 raise ValueError("a ternary table needs the rotation's signs (set_hadamard)")
@@ -176,7 +171,6 @@ class DenseQ:
                                                        tok.data_ptr(), rows, 0 if out_f is None else out_f.data_ptr(),
                                                        0 if out_h is None else out_h.data_ptr(), o.stride(0)))
             return
-        d = self._described()
         ctx.check(capi.call().embed_rows(ctx.address, _stream_ptr(stream), d[0], tok.data_ptr(), rows,
                                          0 if out_f is None else out_f.data_ptr(),
                                          0 if out_h is None else out_h.data_ptr(), o.stride(0)))
@@ -195,11 +189,11 @@ class DenseQ:
         (`halfOut`) or bfloat16. rows must be a multiple of 64 (Linear.swift:695)."""
         if not (x.is_cuda and y.is_cuda):
             _no_cpu()
-        ctx = self._context()
+        d = self._described()
+        ctx = d[6]
         if self.had is not None:  # rotated basis: the rotation runs first, as in the reference's launcher
             x = self.encode_rotate(x, rows, stream)
         ws_ptr, ws_bytes = (0, 0) if workspace is None else (workspace.data_ptr(), workspace.numel() * workspace.element_size())
-        d = self._described()
         st = capi.call().qmm(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), d[0], y.data_ptr(),
                              _dtype_id(y), y.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, ws_ptr, ws_bytes)
         if st:
@@ -258,16 +252,14 @@ class VQMV:
         `n_prefix` computes only the first rows of W (Linear.swift:350-366)."""
         if not (x.is_cuda and y.is_cuda):
             _no_cpu()
-        ctx = m._ctx
-        if ctx is None or ctx.address == 0:
-            ctx = m._context()
+        d = m._described()
+        ctx = d[6]
         if m.had is not None:  # Linear.swift:292-297: the input rotation first, then the kernel on the rotated rows
             x, ldx = m.encode_rotate(x, rows, stream), m.K
         if ldx is None:
             ldx = x.stride(0) if x.dim() > 1 else m.K
         if ldy is None:
             ldy = y.stride(0) if y.dim() > 1 else m.N
-        d = m._described()
         st = capi.call().qmv(ctx.address, _stream_ptr(stream), x.data_ptr(), _DT.get(x.dtype, -1), ldx, d[0], y.data_ptr(),
                              _DT.get(y.dtype, -1), ldy, rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, n_prefix or 0)
         if st:
@@ -306,9 +298,9 @@ class DenseMLP:
         multiples of 64 the GEMM kernels. Scratch is sized on first use and reused."""
         if not (x.is_cuda and out.is_cuda):
             _no_cpu()
-        ctx = self.gate_up._context()
-        ws = self._workspace(rows, x.dtype)
         a, b = self.gate_up._described(), self.down._described()
+        ctx = a[6]
+        ws = self._workspace(rows, x.dtype)
         ctx.check(capi.call().dense_ffn(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
                                         a[0], b[0], self.act, self.limit, out.data_ptr(),
                                         _dtype_id(out), out.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0,

@@ -27,15 +27,16 @@ def rows(n, k, dtype=torch.float32):
 @pytest.fixture
 def fake(monkeypatch):
     """capi with a context and calls that record what they are given."""
-    f = types.SimpleNamespace(seen=[], during=lambda: None)
+    f = types.SimpleNamespace(seen=[], contexts=[], during=lambda: None)
 
     def qmv(ctx, stream, x, xd, ldx, q, *rest):
         f.during()
         d = capi.QLinear.from_address(q)
+        f.contexts.append(ctx)
         f.seen.append((d.w, d.scales, d.biases, d.n, d.k))
         return 0
 
-    monkeypatch.setattr(capi, "context", lambda device=0: types.SimpleNamespace(address=1, check=lambda st: None, device=device))
+    monkeypatch.setattr(capi, "context", lambda device=0: types.SimpleNamespace(address=device + 1, check=lambda st: None, device=device))
     monkeypatch.setattr(capi, "call", lambda: types.SimpleNamespace(qmv=qmv))
     return f
 
@@ -108,9 +109,18 @@ def test_description_follows_an_exchanged_storage(fake, name):
 def test_a_used_matrix_copies_and_pickles(fake):
     m = bare_matrix()
     encode(m)
-    m._ctx = capi.Context.__new__(capi.Context)  # (a context holds a C pointer: neither copies nor pickles)
-    m._ctx._h = capi.C.c_void_p()
     for c in (copy.copy(m), copy.deepcopy(m), pickle.loads(pickle.dumps(m))):
         encode(c)
         assert fake.seen[-1] == (c.w.data_ptr(), c.s.data_ptr(), c.b.data_ptr(), m.N, m.K)
     assert copy.deepcopy(m).w.data_ptr() != m.w.data_ptr()
+
+
+def test_context_follows_the_matrix_to_another_device(fake, monkeypatch):
+    """A matrix whose codes are assigned from another GPU is launched with that GPU's context."""
+    m = bare_matrix()
+    where = [0]
+    monkeypatch.setattr(DenseQ, "device_index", property(lambda self: where[0]))
+    encode(m)
+    where[0], m.w = 1, m.w.clone()
+    encode(m)
+    assert fake.contexts == [1, 2]
