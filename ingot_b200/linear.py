@@ -277,18 +277,18 @@ class DenseMLP:
         self.act = {"silu": capi.IQ_ACT_SILU, "gelu": capi.IQ_ACT_GELU, "swiglu_oai": capi.IQ_ACT_SWIGLU_OAI,
                     "relu2": capi.IQ_ACT_RELU2}[act]
         self.limit = limit
-        self._ws, self._sized = None, None  # scratch, and the (rows, dtype, matrices) it was last checked for
+        self._ws, self._sized = None, None  # scratch, and what it was last sized for: rows, dtype, device, widths
 
-    def _workspace(self, rows: int, x_dtype: torch.dtype) -> torch.Tensor:
-        key = (rows, x_dtype, self.gate_up, self.down)
+    def _workspace(self, ctx: capi.Context, rows: int, x_dtype: torch.dtype) -> torch.Tensor:
+        gu, dn = self.gate_up, self.down
+        key = (rows, x_dtype, ctx.device, gu.N, gu.K, dn.N, dn.K)
         if self._sized == key:
             return self._ws
-        ctx = capi.context(self.gate_up.device_index)
         n = C.c_size_t()
-        a, b = self.gate_up.qlinear(), self.down.qlinear()
+        a, b = gu.qlinear(), dn.qlinear()
         ctx.check(capi.lib().iq_dense_ffn_workspace_bytes(ctx.handle, C.byref(a), C.byref(b), rows, _DT[x_dtype], C.byref(n)))
-        if self._ws is None or self._ws.numel() < n.value:
-            self._ws = torch.empty(max(n.value, 256), dtype=torch.uint8, device=self.gate_up.w.device)
+        if self._ws is None or self._ws.numel() < n.value or self._ws.device != gu.w.device:
+            self._ws = torch.empty(max(n.value, 256), dtype=torch.uint8, device=gu.w.device)
         self._sized = key
         return self._ws
 
@@ -300,7 +300,7 @@ class DenseMLP:
             _no_cpu()
         a, b = self.gate_up._described(), self.down._described()
         ctx = a[6]
-        ws = self._workspace(rows, x.dtype)
+        ws = self._workspace(ctx, rows, x.dtype)
         ctx.check(capi.call().dense_ffn(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
                                         a[0], b[0], self.act, self.limit, out.data_ptr(),
                                         _dtype_id(out), out.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0,

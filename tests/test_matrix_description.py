@@ -36,7 +36,7 @@ def fake(monkeypatch):
         f.seen.append((d.w, d.scales, d.biases, d.n, d.k))
         return 0
 
-    monkeypatch.setattr(capi, "context", lambda device=0: types.SimpleNamespace(address=device + 1, check=lambda st: None, device=device))
+    monkeypatch.setattr(capi, "context", lambda device=0: types.SimpleNamespace(address=device + 1, check=lambda st: None, device=device, handle=None))
     monkeypatch.setattr(capi, "call", lambda: types.SimpleNamespace(qmv=qmv))
     return f
 
@@ -124,3 +124,22 @@ def test_context_follows_the_matrix_to_another_device(fake, monkeypatch):
     where[0], m.w = 1, m.w.clone()
     encode(m)
     assert fake.contexts == [1, 2]
+
+
+def test_ffn_scratch_follows_the_matrices(fake, monkeypatch):
+    """The scratch of a dense FFN is sized for the widths its matrices have at the call, also when their fields were assigned."""
+    def bytes_of(ctx, gu, dn, rows, x_dtype, n):
+        n._obj.value = 1000 * rows * dn._obj.k
+        return 0
+
+    given = []
+    monkeypatch.setattr(capi, "lib", lambda: types.SimpleNamespace(iq_dense_ffn_workspace_bytes=bytes_of))
+    monkeypatch.setattr(capi, "call", lambda: types.SimpleNamespace(dense_ffn=lambda *a: given.append(a[15]) or 0))
+    mlp = linear.DenseMLP(bare_matrix(128, 64), bare_matrix(64, 64))
+    step = lambda: mlp.encode(rows(2, 64), rows(2, 64), 2, stream=types.SimpleNamespace(cuda_stream=0))
+    step()
+    step()
+    for m, n, k in ((mlp.gate_up, 256, 64), (mlp.down, 64, 128)):
+        m.w, m.N, m.K = torch.zeros(n, k // 8, dtype=torch.int32), n, k
+    step()
+    assert given == [1000 * 2 * 64] * 2 + [1000 * 2 * 128]
