@@ -119,7 +119,7 @@ struct GqmvCall {
     float limit = 0.f;
     int32_t act = 0;  // gate/up mode: activation (kAct*)
     bool early = false;  // tiles: the list is complete when the launch's predecessor lets it start (a launch of the same kind did)
-    void* scratch = nullptr;  // device memory of rows * K * 9 / 4 bytes that the call may use (256-byte aligned), or null
+    void* scratch = nullptr;  // device memory of rows * K * 7 / 2 bytes that the call may use (256-byte aligned), or null
     const FixedRows* fx = nullptr;  // grouped gate/up: the token rows as block fixed point, when the caller has them
 };
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);

@@ -480,7 +480,7 @@ extern "C" int32_t iq_dense_ffn_workspace_bytes(iq_ctx* ctx, const iq_qlinear* g
     const size_t d_ff = down->k;
     size_t total = round_up_sz((size_t)rows * d_ff * 2, 256);  // h fp16
     if (rows <= 16) {
-        total += round_up_sz((size_t)rows * std::max(d_ff, (size_t)gate_up->k) / 4 * 9, 256);  // x, then h, as block fixed point
+        total += round_up_sz((size_t)rows * std::max(d_ff, (size_t)gate_up->k) / 2 * 7, 256);  // x, then h, as block fixed point
     } else {
         size_t q = 0;
         int32_t st = iq_qmm_workspace_bytes(ctx, gate_up, rows, x_dtype, &q);

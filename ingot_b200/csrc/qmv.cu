@@ -137,32 +137,47 @@ int tail_slot_of(iq_ctx* ctx, cudaStream_t st) {
 // ---- int8 tensor-core path with a ring of weights per warp: the plain GEMVs the staged kernel refuses, and the dense FFN's
 // gate + up ---------------------------------------------------------------------------------------------------------
 typedef void (*QrKernel)(const QrMaps, const QrParams);
+template <int FMT, int NW, int MS, int LAY>
+QrKernel qr_pick_v(bool vec) { return vec ? qmv_ring_kernel<FMT, MS, NW, true, LAY> : qmv_ring_kernel<FMT, MS, NW, false, LAY>; }
 template <int FMT, int NW>
-QrKernel qr_pick_mv(int ms, bool vec) {
-    if (ms == 4) return vec ? qmv_ring_kernel<FMT, 4, NW, true> : qmv_ring_kernel<FMT, 4, NW, false>;
-    if (ms == 2) return vec ? qmv_ring_kernel<FMT, 2, NW, true> : qmv_ring_kernel<FMT, 2, NW, false>;
-    return vec ? qmv_ring_kernel<FMT, 1, NW, true> : qmv_ring_kernel<FMT, 1, NW, false>;
+QrKernel qr_pick_16(int ms, bool vec) { return ms == 4 ? qr_pick_v<FMT, NW, 4, kQr16>(vec) : ms == 2 ? qr_pick_v<FMT, NW, 2, kQr16>(vec) : qr_pick_v<FMT, NW, 1, kQr16>(vec); }
+template <int FMT, int NW>
+QrKernel qr_pick_23(int lay, int ms, bool vec) {
+    if (lay == kQr23Tall) return ms == 2 ? qr_pick_v<FMT, NW, 2, kQr23Tall>(vec) : qr_pick_v<FMT, NW, 1, kQr23Tall>(vec);
+    return ms == 2 ? qr_pick_v<FMT, NW, 2, kQr23>(vec) : qr_pick_v<FMT, NW, 1, kQr23>(vec);
 }
-template <int FMT>
-QrKernel qr_pick_f(int nw, int ms, bool vec) { return nw == 2 ? qr_pick_mv<FMT, 2>(ms, vec) : qr_pick_mv<FMT, 1>(ms, vec); }
-QrKernel qr_pick(int32_t fmt, int nw, int ms, bool vec) {
-    return fmt == kFmtAffine8 ? qr_pick_f<kFmtAffine8>(nw, ms, vec)
-         : fmt == kFmtAffine4G32 ? qr_pick_f<kFmtAffine4G32>(nw, ms, vec) : qr_pick_f<kFmtAffine4>(nw, ms, vec);
+QrKernel qr_pick(int32_t fmt, int nw, int lay, int ms, bool vec) {
+    if (fmt == kFmtAffine8) return nw == 2 ? qr_pick_16<kFmtAffine8, 2>(ms, vec) : qr_pick_16<kFmtAffine8, 1>(ms, vec);
+    if (fmt == kFmtAffine4G32) return nw == 2 ? qr_pick_23<kFmtAffine4G32, 2>(lay, ms, vec) : qr_pick_23<kFmtAffine4G32, 1>(lay, ms, vec);
+    if (lay == kQr16) return qr_pick_16<kFmtAffine4, 1>(ms, vec);
+    return nw == 2 ? qr_pick_23<kFmtAffine4, 2>(lay, ms, vec) : qr_pick_23<kFmtAffine4, 1>(lay, ms, vec);
 }
 constexpr int kQrPreUnits = 1000;
+// Shapes of a launch, by the rows it takes
+struct QrShape { int lay, ms; };
+constexpr QrShape kQrShapes16[3] = {{kQr16, 1}, {kQr16, 2}, {kQr16, 4}};
+constexpr QrShape kQrShapes23[4] = {{kQr23, 1}, {kQr23, 2}, {kQr23Tall, 1}, {kQr23Tall, 2}};
+int qr_shape_rows(QrShape h) { return h.ms * qr_rows(h.lay); }
 // How a matrix is split, whatever the rows of the call (a row's bits must not depend on them).
 struct QrPlan {
-    int ms;      // sets of four rows a launch can take
+    int max_rows;  // rows a launch can take
     int warps, wk;
 };
-// wk8: eight slices of equal length, the sums of the staged kernel.
-QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms, bool wk8) {
+// wk8: eight slices of equal length, the sums of the staged kernel. wide: 23-bit digits.
+QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms, bool wk8, bool wide) {
     QrPlan best = {0, 0, 0};
-    // as many row sets as fit beside at least two slots per warp, then as many warps
-    for (int ms = 4; ms >= 1 && best.ms == 0; ms /= 2)
-        for (int w = kQrMaxWarps; w >= (ms > 1 ? 8 : 4); w -= wk8 ? 8 : 4)
-            if (qr_smem(fmt, K, nw, ms, vec, w, 2) <= (size_t)kQsSmemMax) { best.ms = ms; best.warps = w; break; }
-    if (best.ms == 0) return best;
+    auto fits = [&](QrShape h, int warps) { return qr_smem(fmt, K, nw, h.lay, h.ms, vec, warps, 2) <= (size_t)kQsSmemMax; };
+    if (wide) {
+        // as many warps as fit beside two rows; a launch with more rows takes fewer where it has to
+        for (int w = kQrMaxWarps; w >= 4 && best.warps == 0; w -= 4)
+            if (fits(kQrShapes23[0], w)) best.warps = w;
+    } else {
+        // as many row sets as fit beside at least two slots per warp, then as many warps
+        for (int v = 2; v >= 0 && best.warps == 0; v--)
+            for (int w = kQrMaxWarps; w >= (v > 0 ? 8 : 4); w -= wk8 ? 8 : 4)
+                if (fits(kQrShapes16[v], w)) { best.max_rows = qr_shape_rows(kQrShapes16[v]); best.warps = w; break; }
+    }
+    if (best.warps == 0) return best;
     // K slices: the least (rounds of a CTA) x (columns of a warp in a round + the round's own cost, about one column's)
     const int gpc = qr_groups(fmt), G = K / (fmt == kFmtAffine4G32 ? 32 : 64), ncol = (G + gpc - 1) / gpc, nblk = N / 16;
     long long cost = -1;
@@ -171,6 +186,10 @@ QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms, bool wk8) {
         const long long per = (long long)(best.warps / wk) * sms, rounds = (nblk + per - 1) / per, c = rounds * ((ncol + wk - 1) / wk + 1);
         if (cost < 0 || c < cost) { cost = c; best.wk = wk; }
     }
+    if (wide && best.wk > 0)
+        for (int v = 0; v < 4; v++)
+            for (int w = best.warps; w >= 8 || w == best.warps; w -= best.wk)
+                if (fits(kQrShapes23[v], w)) { best.max_rows = qr_shape_rows(kQrShapes23[v]); break; }
     return best;
 }
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
@@ -178,6 +197,7 @@ int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk
     if (c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0 || ctx->encode_tiled == nullptr) return 1;
     if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;
     const int nw = c.mode == kModeGateUp ? 2 : 1, gpc = qr_groups(c.fmt), G = c.K / (c.fmt == kFmtAffine4G32 ? 32 : 64);
+    const bool wide = c.fmt != kFmtAffine8 && !wk8;
     bool vec = G % gpc == 0;
     QrParams p;
     memset(&p, 0, sizeof(p));
@@ -188,8 +208,8 @@ int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk
         if ((reinterpret_cast<uintptr_t>(c.w[i]) & 15) || (sb & 3)) return 1;
         if (sb & (uintptr_t)(2 * gpc - 1)) vec = false;
     }
-    const QrPlan plan = qr_plan(c.fmt, c.n_full > 0 ? c.n_full : c.N, c.K, nw, vec, ctx->sms, wk8);
-    if (plan.ms == 0 || plan.wk == 0) return 1;
+    const QrPlan plan = qr_plan(c.fmt, c.n_full > 0 ? c.n_full : c.N, c.K, nw, vec, ctx->sms, wk8, wide);
+    if (plan.max_rows == 0 || plan.wk == 0) return 1;
     const int row_bytes = c.fmt == kFmtAffine8 ? c.K : c.K / 2;
     QrMaps maps = {};
     for (int i = 0; i < nw; i++) {
@@ -208,29 +228,33 @@ int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk
     // 1 us per 2000 units of eight inputs, the kernel 1.5 us)
     const int units = c.rows * (c.K / 8);
     const bool pre = c.scratch != nullptr && units > kQrPreUnits;
-    const size_t rec = (size_t)G * (c.fmt == kFmtAffine4G32 ? 64 : 128);  // bytes of a row's digits
+    const size_t rec = (size_t)G * qr_record(c.fmt == kFmtAffine4G32, wide ? kQr23 : kQr16);  // bytes of a row's digits
     if (pre) {
         unsigned char* digits = static_cast<unsigned char*>(c.scratch);
         float2* scale = reinterpret_cast<float2*>(digits + c.rows * rec);
-        auto k = c.fmt == kFmtAffine8 ? qr_convert_kernel<true, false> : c.fmt == kFmtAffine4G32 ? qr_convert_kernel<false, true> : qr_convert_kernel<false, false>;
+        auto k = c.fmt == kFmtAffine8 ? qr_convert_kernel<true, false, false> : c.fmt == kFmtAffine4G32 ? qr_convert_kernel<false, true, true>
+               : wide ? qr_convert_kernel<false, false, true> : qr_convert_kernel<false, false, false>;
         const int32_t r = check_cuda(ctx, launch_dependent(k, dim3((units + 255) / 256), 256, 0, st, c.x, c.x_dtype, c.ldx, c.K, c.rows, wk8 ? 7 : 8, digits, scale), "qr_convert launch");
         if (r != kOk) return r;
         p.xd = digits;
         p.xs = scale;
     }
-    const int nsup = (c.N / 16 + plan.warps / plan.wk - 1) / (plan.warps / plan.wk);
     for (int m0 = 0; m0 < c.rows;) {
-        int ms = 1;
-        while (ms < plan.ms && 4 * ms < c.rows - m0) ms *= 2;
-        p.M = std::min(c.rows - m0, 4 * ms);
+        const QrShape* h = wide ? kQrShapes23 : kQrShapes16;
+        while (qr_shape_rows(*h) < plan.max_rows && qr_shape_rows(*h) < c.rows - m0) h++;
+        auto smem = [&](int warps, int depth) { return qr_smem(c.fmt, c.K, nw, h->lay, h->ms, vec, warps, depth); };
+        int warps = plan.warps;
+        while (smem(warps, 2) > (size_t)kQsSmemMax) warps -= plan.wk;  // (23 bits: a multiple of the slices that fits, the plan saw to it)
+        p.M = std::min(c.rows - m0, qr_shape_rows(*h));
         p.x = static_cast<const char*>(c.x) + (size_t)m0 * c.ldx * xes;
         p.y = static_cast<char*>(c.y) + (size_t)m0 * c.ldy * yes;
         p.depth = 2;
-        while (p.depth < 6 && qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth + 1) <= (size_t)kQsSmemMax) p.depth++;
-        const int32_t r = check_cuda(ctx, launch_dependent(qr_pick(c.fmt, nw, ms, vec), dim3(std::min(nsup, ctx->sms)), plan.warps * 32,
-                                                           qr_smem(c.fmt, c.K, nw, ms, vec, plan.warps, p.depth), st, maps, p), "qmv_ring launch");
+        while (p.depth < 6 && smem(warps, p.depth + 1) <= (size_t)kQsSmemMax) p.depth++;
+        const int nsup = (c.N / 16 + warps / plan.wk - 1) / (warps / plan.wk);
+        const int32_t r = check_cuda(ctx, launch_dependent(qr_pick(c.fmt, nw, h->lay, h->ms, vec), dim3(std::min(nsup, ctx->sms)), warps * 32,
+                                                           smem(warps, p.depth), st, maps, p), "qmv_ring launch");
         if (r != kOk) return r;
-        if (pre) { p.xd += p.M * rec; p.xs += (size_t)p.M * G; }
+        if (pre) { p.xd += p.M * rec; p.xs += (size_t)p.M * G * (wide ? 2 : 1); }
         m0 += p.M;
     }
     return kOk;
@@ -498,10 +522,15 @@ int32_t gqmv_init(iq_ctx* ctx) {
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
         }
-    const int32_t qr_fmts[3] = {kFmtAffine4, kFmtAffine4G32, kFmtAffine8};
-    for (int v = 0; v < 36; v++) {
-        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qr_pick(qr_fmts[v % 3], 1 + v / 3 % 2, 1 << (v / 6 % 3), v >= 18)),
+    for (int v = 0; v < 44; v++) {  // formats and shapes, one and two matrices, scales in one piece or not
+        const int i = v >> 2;
+        const int32_t fmt = i < 3 ? kFmtAffine8 : i < 7 ? kFmtAffine4G32 : kFmtAffine4;
+        const QrShape h = i < 3 ? kQrShapes16[i] : kQrShapes23[(i - 3) % 4];
+        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qr_pick(fmt, 1 + (v & 1), h.lay, h.ms, (v & 2) != 0)),
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
+        if (e == cudaSuccess && i < 3)  // 4 bits in the staged kernel's place
+            e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qr_pick(kFmtAffine4, 1, h.lay, h.ms, (v & 2) != 0)),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_ring)");
     }
     for (int fmt = 0; fmt < 4; fmt++)

@@ -118,8 +118,7 @@ __device__ __forceinline__ void unpack6x16(uint32_t w0, uint32_t w1, uint32_t w2
 // X + 2^(BITS-1) in the low bits, and four digits go through the shifts and masks at a time. The conversion is every CTA's
 // prologue and was a third of all instructions of a launch of four rows and 14336 inputs at 80 per eight inputs.
 // 7 bits: this file's kernel and the ring kernel where it stands in for it. 8 bits: the kernels that took over from fp16 MMAs,
-// whose activations had 11 bits of their own: a gated h has groups whose largest value is ten times the usual one, and 14 bits
-// of that were 1.0e-3 of an FFN's output off the fp16 kernels', 16 bits are 4e-4 (the fp16 weights' rounding).
+// whose activations had 11 bits of their own (the ring kernel's 4-bit formats with a third digit, see there).
 template <bool W8, int BITS>
 __device__ __forceinline__ void qi_digits8(const float (&v)[8], float inv, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
 #pragma unroll

@@ -2,8 +2,18 @@
 // multiple of 64, groups of 32, rows longer than its stages, and the gate + up + activation form of the dense FFN.
 //
 // Same arithmetic: codes enter m16n8k32 u8 x s8 unconverted, the activations are converted once per CTA to block fixed
-// point per group (two signed 8-bit digits, see qmv_imma.cuh), per group y += s * 2^(e-15) * (256 * acc_hi + acc_lo) +
-// b * sum(x); a row's bits do not depend on the other rows of the call.
+// point per group (see qmv_imma.cuh), per group y += s * 2^(e-15) * (256 * acc_hi + acc_lo) + b * sum(x); a row's bits do not
+// depend on the other rows of the call.
+//
+// Digits. 4-bit codes times bf16 scales, plus bf16 biases, are exact in fp16 but for a few, and the fp16 MMAs that ran these
+// shapes took bf16 and fp16 activations as they are: 2e-7 off the 64-bit product (2880 inputs). 16 bits relative to a group's
+// largest value are 8e-6 off it, and 2e-4 where a few inputs are 100 times the rest. So the 4-bit formats take 23 bits, which
+// hold every bf16 value down to 2^-15 of the group's largest, in three digits. Up to four rows: the eight columns of an MMA are
+// two rows of (high, middle), (low, low), so that a lane's two accumulators are digits of one product, and the row's two lanes
+// meet with the K slices. From five rows on: three MMAs per eight rows, one per digit, and the lane adds the two parts itself: the
+// same sums. 8-bit codes were rounded in fp16 weights (2e-4): 16 bits, four rows of (high, low) per MMA. What the third digit
+// costs: 14336 x 4160 at one row nothing (15.6 -> 14.6 us), at 4 rows 17.2 -> 18.8, at 16 rows (two launches) 32 -> 42; the fp16
+// kernel took 18.1, 23.8 and 40.6.
 //
 // Bound: HBM, which wants 45 KB and more under way per SM all the time. Weights loaded into registers a batch ahead came to 16
 // to 32 KB (2.3 TB/s with eight rows' state beside them). Here every warp runs a ring of its own in shared memory: a slot is
@@ -12,7 +22,7 @@
 // rows, and waits on its own barriers, so that the only synchronisation of the CTA is where the K slices of a block of 16 rows
 // meet. Warps are wk K slices (every wk-th 128-byte column, or runs of them) x row blocks; the host picks the split (csrc/qmv.cu). Against the
 // register batches: 8-bit FFN 2048 -> 7680 -> 2048 at 3 rows 27.2 -> 21.2 us, at 12 rows 72.6 -> 46.9; 4-bit 4096 -> 14336 at
-// one row 42.9 -> 36.2, at 8 rows 105 -> 72.
+// one row 42.9 -> 36.0, at 8 rows 105 -> 82 (16-bit digits 72).
 #pragma once
 
 #include <cuda.h>
@@ -26,11 +36,39 @@ namespace iq {
 constexpr int kQrMaxWarps = 16;
 constexpr int kQrBox = 2048;  // bytes of a slot's codes per matrix
 
-// Eight inputs (unit w8 of a group, its threads neighbouring lanes) as block fixed point, in B-fragment order: the high digits
-// at f, the low ones four lanes' fragments on.
-template <bool W8, bool G32, int BITS>
+// How the activations' digits lie in shared memory, per group of inputs and set of rows: 16 bits, sets of four rows; 24 bits,
+// sets of two rows; 23 bits, sets of eight (each digit of all rows together).
+enum : int { kQr16 = 0, kQr23 = 1, kQr23Tall = 2 };
+__host__ __device__ constexpr int qr_rows(int lay) { return lay == kQr16 ? 4 : (lay == kQr23 ? 2 : 8); }
+__host__ __device__ constexpr int qr_record(bool g32, int lay) { return (lay == kQr16 ? 2 : 3) * (g32 ? 32 : 64); }  // digits of a group and row
+__host__ __device__ constexpr int qr_scales(int lay) { return lay == kQr23Tall ? 8 : 4; }   // float2 {2^(e-15), sum x} of a group and set
+__host__ __device__ constexpr int qr_sums(int lay) { return lay == kQr23Tall ? 128 : 64; }  // sums of a set and 16 weight rows
+
+// Eight activations as 2^8 d[0] + d[1] + 2^-7 d[2] in units of 1 / inv, signed bytes, words of four: the 16 bits of qi_digits8, and
+// what their rounding left over in units of 2^-7 (-64 .. 64).
+template <bool W8>
+__device__ __forceinline__ void qr_digits23(const float (&v)[8], float inv, uint32_t (&d)[3][2]) {
+    constexpr float kInt = 12582912.0f;  // 1.5 * 2^23
+    qi_digits8<W8, 8>(v, inv, d[0], d[1]);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        uint32_t l[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float x = v[W8 ? 4 * h + i : 2 * i + h];
+            const float whole = fmaf(x, inv, kInt + 128.f) - (kInt + 128.f);
+            l[i] = __float_as_uint(fmaf(fmaf(x, inv, -whole), 128.f, kInt));
+        }
+        d[2][h] = __byte_perm(__byte_perm(l[0], l[1], 0x0040), __byte_perm(l[2], l[3], 0x0040), 0x5410);
+    }
+}
+
+// Eight inputs (unit w8 of a group, its threads neighbouring lanes) as block fixed point, in B-fragment order: the digits from
+// the highest down, four lanes' fragments each, STEP bytes from digit to digit. BITS: of a digit; 23: three digits, and SE
+// scale entries (two: for the lane with the high and middle digits, with the sum, and for the one with the low digit).
+template <bool W8, bool G32, int BITS, int STEP, int SE>
 __device__ __forceinline__ void qr_convert(const float (&v)[8], int w8, bool live, unsigned char* rec, float2* scale_out) {
-    constexpr int TPG = G32 ? 4 : 8, XL = G32 ? 8 : 16;
+    constexpr int TPG = G32 ? 4 : 8;
     float amax = 0.f, sum = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
@@ -43,29 +81,41 @@ __device__ __forceinline__ void qr_convert(const float (&v)[8], int w8, bool liv
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
     }
     float scale, inv;
-    qi_group_scale<BITS>(amax, sum, scale, inv);
+    qi_group_scale<BITS == 23 ? 8 : BITS>(amax, sum, scale, inv);
     if (!live) return;
-    if (w8 == 0) *scale_out = make_float2(scale, sum);
-    uint32_t hi_w[2], lo_w[2];
-    qi_digits8<W8, BITS>(v, inv, hi_w, lo_w);
     unsigned char* f = rec + (G32 ? w8 * 8 : (w8 >> 1) * 16 + (w8 & 1) * 8);
-    *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
-    *reinterpret_cast<uint2*>(f + 4 * XL) = make_uint2(lo_w[0], lo_w[1]);
+    if (BITS == 23) {
+        if (w8 == 0) {
+            scale_out[0] = make_float2(scale, sum);
+            if (SE == 2) scale_out[SE - 1] = make_float2(scale * 0.0078125f, 0.f);
+        }
+        uint32_t d[3][2];
+        qr_digits23<W8>(v, inv, d);
+#pragma unroll
+        for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(f + i * STEP) = make_uint2(d[i][0], d[i][1]);
+    } else {
+        if (w8 == 0) *scale_out = make_float2(scale, sum);
+        uint32_t hi_w[2], lo_w[2];
+        qi_digits8<W8, BITS == 23 ? 8 : BITS>(v, inv, hi_w, lo_w);
+        *reinterpret_cast<uint2*>(f) = make_uint2(hi_w[0], hi_w[1]);
+        *reinterpret_cast<uint2*>(f + STEP) = make_uint2(lo_w[0], lo_w[1]);
+    }
 }
 
-// The rows of a call converted once, for CTAs that would each spend longer on it: [rows][groups] records of the digits (128
-// bytes; groups of 32: 64) and of {scale, sum}. 256 threads, a unit of eight inputs each.
-template <bool W8, bool G32>
+// The rows of a call converted once, for CTAs that would each spend longer on it: [rows][groups] records of the digits and of
+// {scale, sum} (two entries with 23 bits). 256 threads, a unit of eight inputs each.
+template <bool W8, bool G32, bool WIDE>
 __global__ void __launch_bounds__(256) qr_convert_kernel(const void* x, int32_t x_dtype, int64_t ldx, int K, int M, int bits, unsigned char* digits, float2* scale) {
-    constexpr int TPG = G32 ? 4 : 8, REC = G32 ? 64 : 128;
+    constexpr int TPG = G32 ? 4 : 8, REC = qr_record(G32, WIDE ? kQr23 : kQr16), STEP = G32 ? 32 : 64;
     pdl_launch_dependents();
     pdl_wait();
     const int units = M * (K / 8), u = blockIdx.x * 256 + threadIdx.x, uc = min(u, units - 1);
     float v[8];
     load_x8(x, x_dtype, (size_t)(uc / (K / 8)) * ldx + (uc % (K / 8)) * 8, v);
     const size_t rec = uc / TPG;  // (K is a multiple of the group)
-    if (bits == 7) qr_convert<W8, G32, 7>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
-    else qr_convert<W8, G32, 8>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
+    if (WIDE) qr_convert<W8, G32, 23, STEP, 2>(v, uc % TPG, u < units, digits + rec * REC, scale + 2 * rec);
+    else if (bits == 7) qr_convert<W8, G32, 7, STEP, 1>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
+    else qr_convert<W8, G32, 8, STEP, 1>(v, uc % TPG, u < units, digits + rec * REC, scale + rec);
 }
 
 struct QrMaps {
@@ -74,7 +124,7 @@ struct QrMaps {
 struct QrParams {
     const unsigned char* s[2];
     const unsigned char* b[2];
-    int32_t N, K, M;       // weight rows (of each matrix), inputs, activation rows (<= 4 * MS)
+    int32_t N, K, M;       // weight rows (of each matrix), inputs, activation rows (<= MS sets)
     const void* x;
     int32_t x_dtype;
     int64_t ldx;
@@ -95,15 +145,15 @@ struct QrParams {
 __host__ __device__ constexpr int qr_groups(int32_t fmt) { return fmt == kFmtAffine8 ? 2 : (fmt == kFmtAffine4G32 ? 8 : 4); }  // groups per 128 bytes
 __host__ __device__ constexpr int qr_swords(int32_t fmt, bool vec) { return qr_groups(fmt) / 2 + (vec ? 0 : 1); }
 // Shared memory of a CTA: rings, fragments and scales of the activations, two buffers of partial sums, barriers, flag.
-inline size_t qr_smem(int32_t fmt, int K, int nw, int ms, bool vec, int warps, int depth) {
+inline size_t qr_smem(int32_t fmt, int K, int nw, int lay, int ms, bool vec, int warps, int depth) {
     const size_t gs = fmt == kFmtAffine4G32 ? 32 : 64, G = K / gs;
-    return 1024 + (size_t)warps * depth * nw * (kQrBox + 2 * 16 * qr_swords(fmt, vec) * 4) + G * ms * (32 * (gs / 4) + 32) +
-           (size_t)2 * warps * nw * ms * 256 + (size_t)warps * depth * 8 + 16;
+    return 1024 + (size_t)warps * depth * nw * (kQrBox + 2 * 16 * qr_swords(fmt, vec) * 4) + G * ms * (qr_rows(lay) * qr_record(gs == 32, lay) + qr_scales(lay) * 8) +
+           (size_t)2 * warps * nw * ms * qr_sums(lay) * 4 + (size_t)warps * depth * 8 + 16;
 }
 
-// FMT: kFmtAffine4, kFmtAffine4G32 or kFmtAffine8; MS: sets of four activation rows; NW: matrices (2: gate and up); VEC: the
-// scales of a slot's row can be copied as one aligned piece (K a multiple of 256, at 8 bits of 128).
-template <int FMT, int MS, int NW, bool VEC>
+// FMT: kFmtAffine4, kFmtAffine4G32 or kFmtAffine8; MS: sets of activation rows; NW: matrices (2: gate and up); VEC: the
+// scales of a slot's row can be copied as one aligned piece (K a multiple of 256, at 8 bits of 128); LAY: kQr16, kQr23, kQr23Tall.
+template <int FMT, int MS, int NW, bool VEC, int LAY>
 __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __grid_constant__ QrMaps maps, const QrParams p) {
     constexpr bool W8 = FMT == kFmtAffine8, G32 = FMT == kFmtAffine4G32;
     constexpr int GS = G32 ? 32 : 64;                  // inputs per group
@@ -111,15 +161,20 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
     constexpr int SPW = qr_swords(FMT, VEC);
     constexpr int XL = GS / 4;                         // bytes of a lane's B fragment per group and row set: 8 or 16
     constexpr int TPG = GS / 8;                        // threads per group in the conversion
+    constexpr bool WIDE = LAY != kQr16, TALL = LAY == kQr23Tall;
+    constexpr int RPS = qr_rows(LAY), SPS = qr_scales(LAY), SE = SPS / RPS;  // rows, scale entries of a set; entries of a row
+    constexpr int REC = qr_record(G32, LAY), SETB = RPS * REC;               // digits of a group: of a row, of a set
+    constexpr int DSTEP = (TALL ? 8 : 1) * 4 * XL, RSTEP = TALL ? 4 * XL : REC;  // from digit to digit, from row to row of a set
+    constexpr int FPS = qr_sums(LAY), AC = TALL ? 8 : 2;                     // sums of a set: of a warp, of a lane
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int nwarps = blockDim.x >> 5, depth = p.depth;
     const int G = p.K / GS, ncol = (G + GPC - 1) / GPC;
-    unsigned char* xq = smem + (size_t)nwarps * depth * NW * kQrBox;               // [groups][MS][32 lanes] XL bytes
-    float2* xsc = reinterpret_cast<float2*>(xq + (size_t)G * MS * 32 * XL);        // [groups][MS * 4 rows] {2^(e-15), sum x}
-    float* red = reinterpret_cast<float*>(xsc + (size_t)G * MS * 4);               // [2][warps][NW * MS * 64]
-    uint32_t* srings = reinterpret_cast<uint32_t*>(red + (size_t)2 * nwarps * NW * MS * 64);
+    unsigned char* xq = smem + (size_t)nwarps * depth * NW * kQrBox;               // [groups][MS][rows][digits][4 lanes] XL bytes (tall: [digits][rows])
+    float2* xsc = reinterpret_cast<float2*>(xq + (size_t)G * MS * SETB);           // [groups][MS][SPS] {2^(e-15), sum x}
+    float* red = reinterpret_cast<float*>(xsc + (size_t)G * MS * SPS);             // [2][warps][NW * MS * FPS]
+    uint32_t* srings = reinterpret_cast<uint32_t*>(red + (size_t)2 * nwarps * NW * MS * FPS);
     uint64_t* bars = reinterpret_cast<uint64_t*>(srings + (size_t)nwarps * depth * NW * 2 * 16 * SPW);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + nwarps * depth);
     const uint32_t ring = smem_u32(smem) + warp * depth * NW * kQrBox;
@@ -179,29 +234,31 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
 
     // ---- activations -> block fixed point, two 8-bit digits, in B-fragment order (see qmv_imma.cuh) ---------------------
     const int nthreads = nwarps * 32;
-    for (int u = tid; u < G * TPG * (4 * MS - p.M); u += nthreads) {  // rows the call does not have: zero digits and scale
+    for (int u = tid; u < G * TPG * (RPS * MS - p.M); u += nthreads) {  // rows the call does not have: zero digits and scale
         const int m = p.M + u / (G * TPG), j = (u / TPG) % G, w8 = u % TPG;
-        unsigned char* f = xq + ((size_t)(j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * XL + (G32 ? w8 * 8 : (w8 >> 1) * 16 + (w8 & 1) * 8);
-        *reinterpret_cast<uint2*>(f) = make_uint2(0, 0);
-        *reinterpret_cast<uint2*>(f + 4 * XL) = make_uint2(0, 0);
-        if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(0.f, 0.f);
+        unsigned char* f = xq + (size_t)(j * MS + m / RPS) * SETB + (m % RPS) * RSTEP + (G32 ? w8 * 8 : (w8 >> 1) * 16 + (w8 & 1) * 8);
+#pragma unroll
+        for (int i = 0; i < REC / (4 * XL); i++) *reinterpret_cast<uint2*>(f + i * DSTEP) = make_uint2(0, 0);
+        if (w8 < SE) xsc[j * SPS * MS + m * SE + w8] = make_float2(0.f, 0.f);
     }
     if (p.xd != nullptr) {
-        constexpr int PC = XL / 2;  // 16-byte pieces of a record
+        constexpr int PC = REC / 16, PD = XL / 4;  // 16-byte pieces of a record, of a digit
         for (int m = 0; m < p.M; m++) {
-            const uint32_t d = smem_u32(xq) + ((m >> 2) * 32 + 8 * (m & 3)) * XL, sd = smem_u32(xsc) + m * 8;
-            const unsigned char* src = p.xd + (size_t)m * G * PC * 16;
-            for (int j = tid; j < G * PC; j += nthreads) cp_async_cg16(d + (j / PC) * (MS * 32 * XL) + (j % PC) * 16, src + (size_t)j * 16);
-            for (int j = tid; j < G; j += nthreads) cp_async_ca<8>(sd + j * (4 * MS * 8), p.xs + (size_t)m * G + j);
+            const uint32_t d = smem_u32(xq) + (m / RPS) * SETB + (m % RPS) * RSTEP, sd = smem_u32(xsc) + m * SE * 8;
+            const unsigned char* src = p.xd + (size_t)m * G * REC;
+            for (int j = tid; j < G * PC; j += nthreads) cp_async_cg16(d + (j / PC) * (MS * SETB) + (j % PC) / PD * DSTEP + (j % PD) * 16, src + (size_t)j * 16);
+            for (int j = tid; j < G; j += nthreads) cp_async_ca<SE * 8>(sd + j * (SPS * MS * 8), p.xs + ((size_t)m * G + j) * (WIDE ? 2 : 1));
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
     const int units = p.xd != nullptr ? 0 : G * TPG * p.M, upad = (units + 31) / 32 * 32;  // whole warps: the groups' shuffles need their threads
     auto convert = [&](const float (&v)[8], int u) {
         const int m = u / (G * TPG), j = (u / TPG) % G;
-        unsigned char* rec = xq + ((size_t)(j * MS + (m >> 2)) * 32 + 8 * (m & 3)) * XL;
-        if (p.runs) qr_convert<W8, G32, 7>(v, u % TPG, u < units, rec, xsc + j * 4 * MS + m);
-        else qr_convert<W8, G32, 8>(v, u % TPG, u < units, rec, xsc + j * 4 * MS + m);
+        unsigned char* rec = xq + (size_t)(j * MS + m / RPS) * SETB + (m % RPS) * RSTEP;
+        float2* sc = xsc + j * SPS * MS + m * SE;
+        if (WIDE) qr_convert<W8, G32, 23, DSTEP, SE>(v, u % TPG, u < units, rec, sc);
+        else if (p.runs) qr_convert<W8, G32, 7, DSTEP, SE>(v, u % TPG, u < units, rec, sc);
+        else qr_convert<W8, G32, 8, DSTEP, SE>(v, u % TPG, u < units, rec, sc);
     };
     if (units <= 2 * nthreads) {
         for (int u = tid; u < upad; u += nthreads) {
@@ -229,19 +286,24 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
     }
     __syncthreads();
 
-    const uint32_t xq32 = smem_u32(xq) + lane * XL, xsc32 = smem_u32(xsc) + t * 8;
+    // lane (g, t) feeds column g: its digit of its row (kQr23: the row's fourth column takes the low digit as well)
+    const uint32_t xq32 = smem_u32(xq) + (LAY == kQr23 ? ((g >> 2) * 3 + min(g & 3, 2)) * 4 * XL + t * XL : lane * XL);
+    const uint32_t xsc32 = smem_u32(xsc) + t * (TALL ? 16 : 8);
     auto bf = [](uint32_t w, int hi_half) { return __uint_as_float(hi_half ? (w & 0xFFFF0000u) : (w << 16)); };
-    const int radix = p.runs ? 128 : 256;
+    // a lane's two accumulators are the columns 2t and 2t + 1 (kQr23, odd t: twice the low digit, of which one counts)
+    const int radix = TALL ? 256 : WIDE ? (t & 1 ? 0 : 256) : (p.runs ? 128 : 256);
     const bool shifted = odd_rows && (g & 1);  // rows g and g + 8 start in the middle of a word
     int slot = 0;
     uint32_t ph = 0;
     bool ok = true;
     for (int sb = lo, it = 0; sb < hi; sb++, it++) {
-        float acc[NW][MS][2];
+        float acc[NW][MS][AC];
 #pragma unroll
         for (int i = 0; i < NW; i++)
 #pragma unroll
-            for (int c = 0; c < MS; c++) acc[i][c][0] = acc[i][c][1] = 0.f;
+            for (int c = 0; c < MS; c++)
+#pragma unroll
+                for (int q = 0; q < AC; q++) acc[i][c][q] = 0.f;
         for (int col = block_of(sb) < nblk ? col0 : col1; col < col1; col += step) {
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar + 8 * slot, ph, abort_flag));
             if (ok) {
@@ -276,19 +338,31 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
                     const int grp = col * GPC + u;
                     if (!VEC && grp >= G) break;
                     const int z[4] = {0, 0, 0, 0};
-                    uint2 xb[MS][2];
-                    float2 xs[MS];
+                    constexpr int DB = TALL ? 3 : 1, XS = TALL ? 2 : 1;  // B fragments of a set, rows of a lane's accumulators
+                    uint2 xb[MS][DB][2];
+                    float2 xs[MS][XS];
 #pragma unroll
                     for (int c = 0; c < MS; c++) {
-                        if (G32) {
-                            xb[c][0] = lds64(xq32 + (grp * MS + c) * 32 * XL);
-                        } else {
-                            const uint4 r = lds128(xq32 + (grp * MS + c) * 32 * XL);
-                            xb[c][0] = make_uint2(r.x, r.y);
-                            xb[c][1] = make_uint2(r.z, r.w);
+#pragma unroll
+                        for (int i = 0; i < DB; i++) {
+                            const uint32_t a = xq32 + (grp * MS + c) * SETB + i * DSTEP;
+                            if (G32) {
+                                xb[c][i][0] = lds64(a);
+                            } else {
+                                const uint4 r = lds128(a);
+                                xb[c][i][0] = make_uint2(r.x, r.y);
+                                xb[c][i][1] = make_uint2(r.z, r.w);
+                            }
                         }
-                        const uint2 sr = lds64(xsc32 + (grp * MS + c) * 32);
-                        xs[c] = make_float2(__uint_as_float(sr.x), __uint_as_float(sr.y));
+                        const uint32_t a = xsc32 + (grp * MS + c) * SPS * 8;
+                        if (TALL) {
+                            const uint4 sr = lds128(a);
+                            xs[c][0] = make_float2(__uint_as_float(sr.x), __uint_as_float(sr.y));
+                            xs[c][XS - 1] = make_float2(__uint_as_float(sr.z), __uint_as_float(sr.w));
+                        } else {
+                            const uint2 sr = lds64(a);
+                            xs[c][0] = make_float2(__uint_as_float(sr.x), __uint_as_float(sr.y));
+                        }
                     }
 #pragma unroll
                     for (int i = 0; i < NW; i++) {
@@ -320,20 +394,35 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
                         }
                         const float sc0 = bf(sc[i][0][u / 2], u & 1), sc1 = bf(sc[i][1][u / 2], u & 1);
                         const float bi0 = bf(bi[i][0][u / 2], u & 1), bi1 = bf(bi[i][1][u / 2], u & 1);
-                        int d[MS][4];
+                        int d[MS][DB][4];
 #pragma unroll
-                        for (int c = 0; c < MS; c++) imma16832_u8s8(d[c], a[0][0], a[0][1], a[0][2], a[0][3], xb[c][0].x, xb[c][0].y, z);
+                        for (int c = 0; c < MS; c++)
+#pragma unroll
+                            for (int q = 0; q < DB; q++) imma16832_u8s8(d[c][q], a[0][0], a[0][1], a[0][2], a[0][3], xb[c][q][0].x, xb[c][q][0].y, z);
                         if (!G32) {
 #pragma unroll
-                            for (int c = 0; c < MS; c++) imma16832_u8s8(d[c], a[1][0], a[1][1], a[1][2], a[1][3], xb[c][1].x, xb[c][1].y, d[c]);
+                            for (int c = 0; c < MS; c++)
+#pragma unroll
+                                for (int q = 0; q < DB; q++) imma16832_u8s8(d[c][q], a[1][0], a[1][1], a[1][2], a[1][3], xb[c][q][1].x, xb[c][q][1].y, d[c][q]);
                         }
 #pragma unroll
                         for (int c = 0; c < MS; c++) {
-                            const float v0 = (float)(d[c][0] * radix + d[c][1]), v1 = (float)(d[c][2] * radix + d[c][3]);
-                            acc[i][c][0] = fmaf(v0, sc0 * xs[c].x, acc[i][c][0]);
-                            acc[i][c][0] = fmaf(bi0, xs[c].y, acc[i][c][0]);
-                            acc[i][c][1] = fmaf(v1, sc1 * xs[c].x, acc[i][c][1]);
-                            acc[i][c][1] = fmaf(bi1, xs[c].y, acc[i][c][1]);
+                            if (TALL) {  // accumulator q: activation row 2 t + q % 2 of the set, weight row g + 8 (q / 2)
+#pragma unroll
+                                for (int q = 0; q < 4; q++) {
+                                    const float s = q < 2 ? sc0 : sc1, x = xs[c][q % XS].x;
+                                    float &hi = acc[i][c][q % AC], &lo = acc[i][c][(4 + q) % AC];
+                                    hi = fmaf((float)(d[c][0][q] * radix + d[c][DB / 2][q]), s * x, hi);
+                                    hi = fmaf(q < 2 ? bi0 : bi1, xs[c][q % XS].y, hi);
+                                    lo = fmaf((float)d[c][DB - 1][q], s * (x * 0.0078125f), lo);
+                                }
+                            } else {
+                                const float v0 = (float)(d[c][0][0] * radix + d[c][0][1]), v1 = (float)(d[c][0][2] * radix + d[c][0][3]);
+                                acc[i][c][0] = fmaf(v0, sc0 * xs[c][0].x, acc[i][c][0]);
+                                acc[i][c][0] = fmaf(bi0, xs[c][0].y, acc[i][c][0]);
+                                acc[i][c][1] = fmaf(v1, sc1 * xs[c][0].x, acc[i][c][1]);
+                                acc[i][c][1] = fmaf(bi1, xs[c][0].y, acc[i][c][1]);
+                            }
                         }
                     }
                 }
@@ -343,22 +432,31 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
             if (++slot == depth) { slot = 0; ph ^= 1; }
         }
         // ---- the K slices meet in shared memory (two buffers: one barrier per round) -------------------------------------
-        float* mine = red + ((it & 1) * nwarps + warp) * (NW * MS * 64);
+        float* mine = red + ((it & 1) * nwarps + warp) * (NW * MS * FPS);
 #pragma unroll
         for (int i = 0; i < NW; i++)
 #pragma unroll
-            for (int c = 0; c < MS; c++) *reinterpret_cast<float2*>(mine + (i * MS + c) * 64 + lane * 2) = make_float2(acc[i][c][0], acc[i][c][1]);
+            for (int c = 0; c < MS; c++) {
+                if (TALL)
+                    *reinterpret_cast<float4*>(mine + (i * MS + c) * FPS + lane * 4) =
+                        make_float4(acc[i][c][0] + acc[i][c][4 % AC], acc[i][c][1] + acc[i][c][5 % AC], acc[i][c][2 % AC] + acc[i][c][6 % AC], acc[i][c][3 % AC] + acc[i][c][7 % AC]);
+                else *reinterpret_cast<float2*>(mine + (i * MS + c) * FPS + lane * 2) = make_float2(acc[i][c][0], acc[i][c][1]);
+            }
         __syncthreads();
-        for (int o = tid; o < rbs * 64 * MS; o += nthreads) {
-            const int rbi = o / (64 * MS), c = (o >> 6) % MS, mm = (o >> 4) & 3, r = o & 15, m = 4 * c + mm, blk = sb * rbs + rbi;
+        for (int o = tid; o < rbs * 16 * RPS * MS; o += nthreads) {
+            const int rbi = o / (16 * RPS * MS), c = o / (16 * RPS) % MS, mm = (o >> 4) % RPS, r = o & 15, m = RPS * c + mm, blk = sb * rbs + rbi;
             if (m >= p.M || blk >= nblk) continue;
-            const float* part = red + ((it & 1) * nwarps + rbi * p.wk) * (NW * MS * 64) + c * 64 + (4 * (r & 7) + mm) * 2 + (r >> 3);
+            const float* part = red + ((it & 1) * nwarps + rbi * p.wk) * (NW * MS * FPS) + c * FPS +
+                                (TALL ? (4 * (r & 7) + (mm >> 1)) * 4 + (r >> 3) * 2 + (mm & 1) : (4 * (r & 7) + mm * SE) * 2 + (r >> 3));
             float v[NW];
 #pragma unroll
             for (int i = 0; i < NW; i++) v[i] = 0.f;
             for (int k = 0; k < p.wk; k++)
 #pragma unroll
-                for (int i = 0; i < NW; i++) v[i] += part[(k * NW + i) * MS * 64];
+                for (int i = 0; i < NW; i++) {
+                    const float* q = part + (k * NW + i) * MS * FPS;
+                    v[i] += LAY == kQr23 ? q[0] + q[2] : q[0];
+                }
             const float f = NW == 2 ? glu_rt(p.act, v[0], v[NW - 1], p.limit) : v[0];
             const size_t y = (size_t)m * p.ldy + (size_t)blk * 16 + r;
             if (p.y_dtype == kF32) {

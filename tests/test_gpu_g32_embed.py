@@ -212,3 +212,28 @@ def test_dense_ffn_ragged(cuda_device, bits, group, rows, D, F):
     DenseMLP(gu, dn).encode(x_tensor(xh, cuda_device), out, rows)
     assert capi.context(0).device_status() == 0
     assert qref.max_rel(out.cpu().numpy(), ref) <= 2 * TOL  # h is rounded to fp16 on both sides, from sums in other orders
+
+
+@pytest.mark.parametrize("bits,group", [(4, 64), (8, 64), (4, 32)])
+@pytest.mark.parametrize("D,F", [(1600, 2880), (2048, 2048), (832, 6144), (2048, 320)])
+def test_dense_ffn_row_invariance(cuda_device, bits, group, D, F):
+    """A row of a decode FFN has the same bits alone and among others, whichever kernel makes the activations' digits (from 1000
+    units of eight inputs on one of its own: 5 rows of 1600, 3 of 2880), whatever layout of them the number of rows picks,
+    and with nine and more rows of a width the staged kernel takes (2048, 6144)."""
+    rng = np.random.default_rng(70 + bits + group + D + F)
+    gu, _ = affine_case(rng, 2 * F, D, bits, cuda_device, group=group)
+    dn, _ = affine_case(rng, D, F, bits, cuda_device, group=group)
+    mlp = DenseMLP(gu, dn)
+    x = x_tensor(synth.activations_np(rng, 16, D), cuda_device)
+
+    def ffn(xr):
+        out = torch.zeros(xr.shape[0], D, dtype=torch.float32, device=cuda_device)
+        mlp.encode(xr.contiguous(), out, xr.shape[0])
+        return out
+
+    full = ffn(x)
+    for rows in (1, 2, 3, 4, 5, 8, 9, 12):
+        assert torch.equal(ffn(x[:rows]), full[:rows]), rows
+    for i in (3, 8, 15):
+        assert torch.equal(ffn(x[i:i + 1])[0], full[i]), i
+    assert capi.context(0).device_status() == 0

@@ -250,3 +250,27 @@ def test_qmv_ring_edges(cuda_device, bits, N, K, rows):
     assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(x, deq(host, bits))) <= TOL
     alone = run(m, x_tensor(x[rows - 1:], cuda_device), 1)
     assert torch.equal(alone[0], y[rows - 1])
+
+
+@pytest.mark.parametrize("dist", ["normal", "channels", "group"])
+@pytest.mark.parametrize("N,K,rows,group", [(256, 2880, 1, 64), (256, 1600, 5, 64), (128, 14336, 3, 64), (256, 2880, 16, 64), (256, 1536, 7, 32), (64, 4096, 12, 32)])
+def test_qmv_ring_keeps_16_bit_activations_whole(cuda_device, N, K, rows, group, dist):
+    """4-bit weights are all but exact and bf16 and fp16 activations go into the sums whole, also where a few input channels, or one
+    input of every group, are 100 times the rest: against the 64-bit product what is left is the sums' 32 bits. Digits of 23 bits add
+    at most 2^-23 of a group's largest input per input, K / group + 16 sums in fp32 round to 2^-24 each, and code and bias terms
+    are some four times their difference: 1e-5 of the largest output. (16-bit digits: 1e-4 to 8e-4 with the outliers.)"""
+    rng = np.random.default_rng(N + K + rows)
+    m, host = affine_case(rng, N, K, 4, cuda_device, group=group)
+    x = rng.normal(0, 1, size=(rows, K)).astype(np.float32)
+    if dist == "channels":
+        x[:, rng.choice(K, 4, replace=False)] *= 100
+    elif dist == "group":
+        x[:, np.arange(0, K, 64) + rng.integers(0, 64, size=K // 64)] *= 100
+    for dt in (torch.bfloat16, torch.float16):
+        xt = torch.from_numpy(x).to(cuda_device).to(dt)
+        y = run(m, xt, rows)
+        w = host[0][0].astype(np.uint32)
+        q = ((w[:, :, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15).reshape(N, K).astype(np.float64)
+        s, b = (np.repeat(synth.bf16_bits_to_f32(t[0]).astype(np.float64), group, axis=1) for t in host[1:])
+        ref = xt.double().cpu().numpy() @ (q * s + b).T
+        assert np.abs(y.double().cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
