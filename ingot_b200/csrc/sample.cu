@@ -9,6 +9,8 @@
 #include <float.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -233,7 +235,8 @@ __global__ void __launch_bounds__(1024) __cluster_dims__(kArgmaxBlocks, 1, 1)
     __shared__ uint32_t bi[32];
     __shared__ float cv[kArgmaxBlocks];
     __shared__ uint32_t ci[kArgmaxBlocks];
-    const int row = blockIdx.y, tid = threadIdx.x;
+    // (rows on the x dimension: the others end at 65,535)
+    const int row = blockIdx.x / kArgmaxBlocks, part = blockIdx.x % kArgmaxBlocks, tid = threadIdx.x;
     pdl_launch_dependents();
     cluster_sync_all();  // the first block runs: its shared memory may be written
     pdl_wait();
@@ -241,16 +244,16 @@ __global__ void __launch_bounds__(1024) __cluster_dims__(kArgmaxBlocks, 1, 1)
     float m = -INFINITY;
     uint32_t mi = 0;
     constexpr int U = 8;  // loads in flight per thread
-    for (int i = blockIdx.x * 1024 + tid; i < N; i += U * kArgmaxBlocks * 1024) {
+    for (uint32_t i = part * 1024 + tid; i < (uint32_t)N; i += U * kArgmaxBlocks * 1024) {  // (unsigned: i and j pass N)
         float v[U];
 #pragma unroll
         for (int k = 0; k < U; k++) {
-            const int j = i + k * kArgmaxBlocks * 1024;
-            v[k] = j < N ? xr[j] : -INFINITY;
+            const uint32_t j = i + k * kArgmaxBlocks * 1024;
+            v[k] = j < (uint32_t)N ? xr[j] : -INFINITY;
         }
 #pragma unroll
         for (int k = 0; k < U; k++)
-            if (v[k] > m) { m = v[k]; mi = (uint32_t)(i + k * kArgmaxBlocks * 1024); }
+            if (v[k] > m) { m = v[k]; mi = i + k * kArgmaxBlocks * 1024; }
     }
     float sm = m;
     for (int o = 16; o > 0; o >>= 1) sm = fmaxf(sm, __shfl_xor_sync(0xffffffffu, sm, o));
@@ -263,11 +266,11 @@ __global__ void __launch_bounds__(1024) __cluster_dims__(kArgmaxBlocks, 1, 1)
         uint32_t ix = bi[0];
         for (int i = 1; i < 32; i++)
             if (bv[i] > b || (bv[i] == b && bi[i] < ix)) { b = bv[i]; ix = bi[i]; }
-        st_dsmem_u32(reinterpret_cast<uint32_t*>(&cv[blockIdx.x]), 0, __float_as_uint(b));
-        st_dsmem_u32(&ci[blockIdx.x], 0, ix);
+        st_dsmem_u32(reinterpret_cast<uint32_t*>(&cv[part]), 0, __float_as_uint(b));
+        st_dsmem_u32(&ci[part], 0, ix);
     }
     cluster_sync_all();
-    if (blockIdx.x == 0 && tid == 0) {
+    if (part == 0 && tid == 0) {
         float b = cv[0];
         uint32_t ix = ci[0];
         for (int i = 1; i < kArgmaxBlocks; i++)
@@ -285,9 +288,13 @@ extern "C" int32_t iq_argmax_rows(iq_ctx* ctx, void* stream, const float* x, int
                                   uint32_t* out) {
     if (ctx == nullptr) return kErrInvalidArg;
     if (x == nullptr || out == nullptr || rows < 1 || n < 1 || ldx < n) return fail(ctx, kErrInvalidArg, "argmax_rows: arguments");
-    return check_cuda(ctx, launch_dependent(argmax_rows_kernel, dim3(kArgmaxBlocks, rows), 1024, 0,
-                                           reinterpret_cast<cudaStream_t>(stream), x, ldx, out, n),
-                      "argmax_rows launch");
+    constexpr int32_t kRows = 1 << 27;  // of one launch: kArgmaxBlocks blocks each
+    int32_t st = kOk;
+    for (int64_t r = 0; r < rows && st == kOk; r += kRows)
+        st = check_cuda(ctx, launch_dependent(argmax_rows_kernel, dim3((unsigned)std::min<int64_t>(rows - r, kRows) * kArgmaxBlocks), 1024, 0,
+                                              reinterpret_cast<cudaStream_t>(stream), x + r * ldx, ldx, out + r, n),
+                        "argmax_rows launch");
+    return st;
 }
 
 extern "C" int32_t iq_topk64_scratch_bytes(int32_t rows, int32_t vocab, size_t* bytes) {

@@ -94,3 +94,10 @@ def test_candidates_at_the_edges_of_a_part(cuda_device, V):
     x[3, :: max(1, V // 64)] = 1.0
     x[4] = np.float32(1.0) + np.arange(V, dtype=np.float32) * np.float32(2 ** -23)  # neighbouring floats
     check(x, [0.7])
+
+
+@pytest.mark.parametrize("rows,n", [(65535, 5), (65536, 5), (70001, 3)])
+def test_argmax_of_more_rows_than_a_grid_dimension(cuda_device, rows, n):
+    x = logits("ties", n, rows, rows + n)
+    got = sampling.argmax_rows(torch.from_numpy(x).to(cuda_device), rows)
+    assert np.array_equal(got.cpu().numpy().astype(np.uint32), qref.argmax_rows(x))
