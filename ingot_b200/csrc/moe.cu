@@ -87,9 +87,9 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     w.yd = take(P * d.d_model * (yd_dtype_of(l) == kF16 ? 2 : 4));
     w.xs = static_cast<__half*>(take(P * d.d_model * 2));
     const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens, fixed = tokens < kFixedTokens ? tokens : kFixedTokens;
-    w.fx.digits = static_cast<unsigned char*>(take(fixed * (d.d_model / 64) * 128));
+    w.fx.digits = static_cast<unsigned char*>(take((fixed * 128 + few * 64) * (d.d_model / 64)));  // (few tokens: the wide form)
     w.fx.scale = static_cast<float2*>(take(fixed * (d.d_model / 64) * 8));
-    w.fh.digits = static_cast<unsigned char*>(take(few * d.top_k * (d.d_ff / 64) * 128));
+    w.fh.digits = static_cast<unsigned char*>(take(few * d.top_k * (d.d_ff / 64) * 192));
     w.fh.scale = static_cast<float2*>(take(few * d.top_k * (d.d_ff / 64) * 8));
     w.s_x16 = nullptr; w.s_h = nullptr; w.s_yd = nullptr; w.s_w = nullptr;
     if (d.shared != IQ_SHARED_NONE) {
@@ -317,7 +317,7 @@ bool use_experts_small(const iq_moe* l) {
     return l->fmt == kFmtAffine4 && (a & 15) == 0;
 }
 
-int32_t run_route_small(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, int64_t ldx, int tokens, const MoeWs& w, bool fixed) {
+int32_t run_route_small(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, int64_t ldx, int tokens, const MoeWs& w, bool fixed, bool wide) {
     const iq_moe_desc& d = l->d;
     RouteSmallParams p;
     p.r = route_params(l, w.logits, l->ld, tokens, w.inds, w.wts);
@@ -325,6 +325,7 @@ int32_t run_route_small(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dty
     p.counts = w.counts; p.offsets = w.offsets; p.row_map = w.row_map; p.pos = w.pos; p.ntiles = w.ntiles;
     p.tiles_a = w.tiles_a; p.tiles_b = w.tiles_b;
     p.fx = fixed ? w.fx : FixedRows{nullptr, nullptr};
+    p.wide = wide ? 1 : 0;
     const int tt = router_tokens(tokens);
     return check_cuda(l->ctx, launch_dependent(route_small_pick(d.router_kind != IQ_ROUTER_BF16, tt, d.experts), dim3(kSmallCluster), kSmallThreads,
                                                route_small_smem(tt, d.d_model, d.experts), cs, p), "moe_route_small launch");
@@ -740,7 +741,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
 
     const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l);
     if (small) {
-        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, l->fmt == kFmtAffine4);
+        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, l->fmt == kFmtAffine4, small_experts);
         if (st == kOk && small_experts)
             st = run_experts_small(l, cs, tokens, w, out, out_dtype, ldo, (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0);
         if (st != kOk) return st;

@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(256) moe_count_kernel(const GroupParams p) {
     pdl_launch_dependents();
     pdl_wait();
     if (p.fx.digits != nullptr)
-        for (int t = blockIdx.x; t < p.T; t += gridDim.x) fixed_point_row(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
+        for (int t = blockIdx.x; t < p.T; t += gridDim.x) fixed_point_row<false>(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
     uint32_t c = 0;
     for (int i = threadIdx.x; i < p.P; i += 256) c += p.inds[i] == e;
 #pragma unroll

@@ -11,8 +11,13 @@
 //
 // Each starts while its predecessor runs (programmatic dependent launch); the down kernel has its first weights on the way
 // before h exists. Affine 4-bit experts, all of them on this GPU. The results are those of the separate kernels: exact
-// float64 logits, the same quantisation, sums in fixed orders.
+// float64 logits, sums in fixed orders. The activations and h are fixed point of 23 bits (three digits: the columns of an MMA are two
+// rows of (high, middle), (low, low), as in qmv_ring.cuh), which keeps bf16 activations whole as the fp16 kernels did that ran the
+// widths the staged kernels do not take: with 16 bits a layer of 2880 x 768 with input channels 100 times the rest was 8.5e-4 off
+// the 64-bit result instead of 4.9e-4.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "fixed_rows.cuh"
@@ -33,6 +38,7 @@ struct RouteSmallParams {
     uint32_t *counts, *offsets, *row_map, *pos, *ntiles;
     Tile *tiles_a, *tiles_b;
     FixedRows fx;                // the activations as block fixed point, or null
+    int32_t wide;                // its form: 23 bits (moe_gateup_small_kernel's), or 16
 };
 constexpr size_t route_small_smem(int tt, int D, int E) {
     return router_block_smem(tt, D, E / kSmallCluster) + (size_t)tt * E * 4 + 16 * kSmallTokens * 4 + 64 * 4 + (size_t)E * 4;
@@ -64,8 +70,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) __cluster_dims__(kSmallClust
     // the other blocks turn the activations into fixed point
     if (rank != 0) {
         if (p.fx.digits == nullptr) return;
-        for (int t = rank - 1; t < T; t += kSmallCluster - 1)
-            fixed_point_row(p.in.x, p.in.x_dtype, (size_t)t * p.in.ldx, D, p.fx, t, tid, kSmallThreads);
+        for (int t = rank - 1; t < T; t += kSmallCluster - 1) {
+            if (p.wide) fixed_point_row<true>(p.in.x, p.in.x_dtype, (size_t)t * p.in.ldx, D, p.fx, t, tid, kSmallThreads);
+            else fixed_point_row<false>(p.in.x, p.in.x_dtype, (size_t)t * p.in.ldx, D, p.fx, t, tid, kSmallThreads);
+        }
         return;
     }
     if (warp < T) {
@@ -165,15 +173,18 @@ __device__ __forceinline__ void small_load(SmallBatch& v, const unsigned char* w
         }
     }
 }
-// One group of the batch against one set of four activation rows: xb the lane's digits, xs its row's {2^(e-15), sum}.
-__device__ __forceinline__ void small_mma(float (&acc)[2], const SmallBatch& v, int u, const uint4& xb, const float2& xs) {
+// One group of the batch against one set of two activation rows: xb the lane's digits (column g: digit g % 4 of row g / 4, the last
+// digit twice), xs its part's scale and sum: lanes of even t hold the high and middle digits' sums of row t / 2, those of odd t the
+// low one's (radix 0: one of the two).
+__device__ __forceinline__ float2 small_part(const float2& row, int t) { return t & 1 ? make_float2(row.x * 0.0078125f, 0.f) : row; }
+__device__ __forceinline__ void small_mma(float (&acc)[2], const SmallBatch& v, int u, const uint4& xb, const float2& xs, int radix) {
     constexpr uint32_t MSK = 0x0F0F0F0Fu;
     const int z[4] = {0, 0, 0, 0};
     int d[4];
     const uint2 w0 = v.q[u][0], w1 = v.q[u][1];
     imma16832_u8s8(d, w0.x & MSK, w1.x & MSK, (w0.x >> 4) & MSK, (w1.x >> 4) & MSK, xb.x, xb.y, z);
     imma16832_u8s8(d, w0.y & MSK, w1.y & MSK, (w0.y >> 4) & MSK, (w1.y >> 4) & MSK, xb.z, xb.w, d);
-    const float v0 = (float)(d[0] * 256 + d[1]), v1 = (float)(d[2] * 256 + d[3]);
+    const float v0 = (float)(d[0] * radix + d[1]), v1 = (float)(d[2] * radix + d[3]);
     const float s0 = __uint_as_float(u ? (v.s[0] & 0xFFFF0000u) : (v.s[0] << 16)), s1 = __uint_as_float(u ? (v.s[1] & 0xFFFF0000u) : (v.s[1] << 16));
     const float b0 = __uint_as_float(u ? (v.b[0] & 0xFFFF0000u) : (v.b[0] << 16)), b1 = __uint_as_float(u ? (v.b[1] & 0xFFFF0000u) : (v.b[1] << 16));
     acc[0] = fmaf(v0, s0 * xs.x, acc[0]);
@@ -182,17 +193,18 @@ __device__ __forceinline__ void small_mma(float (&acc)[2], const SmallBatch& v, 
     acc[1] = fmaf(b1, xs.y, acc[1]);
 }
 
-// A block's item: 64 features (gate and up) of one tile of up to four rows; its sixteen warps are four blocks of 16 rows x
-// four slices of the inputs.
+// A block's item: 64 features (gate and up) of one tile of up to three rows, in sets of two; its sixteen warps are four blocks of
+// 16 rows x four slices of the inputs.
 __global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(const GateUpSmallParams p) {
     constexpr int RS = 72;  // floats between activation rows of the slices' sums (the lanes of a store in different banks)
-    __shared__ float red[4][2][4][RS];
+    __shared__ float red[4][2][8][RS];  // [slice][matrix][row, part]
     __shared__ float gmax[16], gsum[16];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int rb = warp & 3, ks = warp >> 2;
     const int G = p.D / 64, NB = p.I / 64;
     const int pairs = (G + 1) / 2, p0 = pairs * ks / 4, p1 = pairs * (ks + 1) / 4;  // this slice, in pairs of groups
     const bool even = (G & 1) == 0;
+    const int radix = t & 1 ? 0 : 256;
     pdl_wait();
     pdl_launch_dependents();  // (after the wait: what the down kernel reads early is then complete)
     const int total = (int)__ldcg(p.ntiles) * NB;
@@ -204,48 +216,63 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(cons
         SmallBatch cur[2], nxt[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) small_load(cur[i], p.w[i], p.s[i], p.b[i], row, G, 2 * min(p0, pairs - 1), even, t);
-        // fragments: lane (g, t) holds digit g % 2 of row g / 2 of the set; scales: of row t of the set
-        const bool live = (g >> 1) < M;
-        const uint32_t tok = __ldcg(p.row_map + tile.start + min(g >> 1, M - 1)) / (uint32_t)p.topk;
-        const uint32_t tks = __ldcg(p.row_map + tile.start + min(t, M - 1)) / (uint32_t)p.topk;
-        const unsigned char* xd = p.x.digits + (size_t)tok * G * 128 + (g & 1) * 64 + t * 16;
-        const float2* xs = p.x.scale + (size_t)tks * G;
-        float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-        auto compute = [&](const SmallBatch (&v)[2], int pr) {
+        const unsigned char* xd[2];
+        const float2* xs[2];
+        bool live[2];
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int grp = 2 * pr + u;
-                if (grp >= G) break;
-                uint4 xb = *reinterpret_cast<const uint4*>(xd + grp * 128);
-                if (!live) xb = make_uint4(0, 0, 0, 0);
-                const float2 sv = xs[grp];
-                small_mma(acc[0], v[0], u, xb, sv);
-                small_mma(acc[1], v[1], u, xb, sv);
+        for (int c = 0; c < 2; c++) {
+            const int m = 2 * c + (g >> 2), mt = 2 * c + (t >> 1);
+            live[c] = m < M;
+            const uint32_t tok = __ldcg(p.row_map + tile.start + min(m, M - 1)) / (uint32_t)p.topk;
+            const uint32_t tks = __ldcg(p.row_map + tile.start + min(mt, M - 1)) / (uint32_t)p.topk;
+            xd[c] = p.x.digits + (size_t)tok * G * 192 + min(g & 3, 2) * 64 + t * 16;
+            xs[c] = p.x.scale + (size_t)tks * G;
+        }
+        float acc[2][2][2] = {{{0.f, 0.f}, {0.f, 0.f}}, {{0.f, 0.f}, {0.f, 0.f}}};  // [matrix][set]
+        auto slice = [&](auto sets) {  // (their number outside the loop: no branch between the groups' loads)
+            auto compute = [&](const SmallBatch (&v)[2], int pr) {
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int grp = 2 * pr + u;
+                    if (grp >= G) break;
+#pragma unroll
+                    for (int c = 0; c < decltype(sets)::value; c++) {
+                        uint4 xb = *reinterpret_cast<const uint4*>(xd[c] + grp * 192);
+                        if (!live[c]) xb = make_uint4(0, 0, 0, 0);
+                        const float2 sv = small_part(xs[c][grp], t);
+                        small_mma(acc[0][c], v[0], u, xb, sv, radix);
+                        small_mma(acc[1][c], v[1], u, xb, sv, radix);
+                    }
+                }
+            };
+            int pr = p0;
+            for (; pr + 1 < p1; pr += 2) {
+#pragma unroll
+                for (int i = 0; i < 2; i++) small_load(nxt[i], p.w[i], p.s[i], p.b[i], row, G, 2 * (pr + 1), even, t);
+                compute(cur, pr);
+#pragma unroll
+                for (int i = 0; i < 2; i++) small_load(cur[i], p.w[i], p.s[i], p.b[i], row, G, 2 * min(pr + 2, pairs - 1), even, t);
+                compute(nxt, pr + 1);
             }
+            if (pr < p1) compute(cur, pr);
         };
-        int pr = p0;
-        for (; pr + 1 < p1; pr += 2) {
+        if (M > 2) slice(std::integral_constant<int, 2>{});
+        else slice(std::integral_constant<int, 1>{});
 #pragma unroll
-            for (int i = 0; i < 2; i++) small_load(nxt[i], p.w[i], p.s[i], p.b[i], row, G, 2 * (pr + 1), even, t);
-            compute(cur, pr);
+        for (int i = 0; i < 2; i++)
 #pragma unroll
-            for (int i = 0; i < 2; i++) small_load(cur[i], p.w[i], p.s[i], p.b[i], row, G, 2 * min(pr + 2, pairs - 1), even, t);
-            compute(nxt, pr + 1);
-        }
-        if (pr < p1) compute(cur, pr);
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            red[ks][i][t][rb * 16 + g] = acc[i][0];
-            red[ks][i][t][rb * 16 + 8 + g] = acc[i][1];
-        }
+            for (int c = 0; c < 2; c++) {
+                red[ks][i][4 * c + t][rb * 16 + g] = acc[i][c][0];
+                red[ks][i][4 * c + t][rb * 16 + 8 + g] = acc[i][c][1];
+            }
         __syncthreads();
         // a thread per (feature, row): the slices in order, the activation, and the group of 64 features as block fixed point
         const int f = tid & 63, m = tid >> 6;
         float gv = 0.f, uv = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            gv += red[k][0][m & 3][f];  // (rows past the fourth: nothing is stored)
-            uv += red[k][1][m & 3][f];
+            gv += red[k][0][2 * m & 7][f] + red[k][0][(2 * m & 7) + 1][f];  // (rows past the fourth: nothing is stored)
+            uv += red[k][1][2 * m & 7][f] + red[k][1][(2 * m & 7) + 1][f];
         }
         if (p.ebias[0] != nullptr) {
             gv += p.ebias[0][(size_t)tile.expert * p.I + n0 + f];
@@ -271,9 +298,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_gateup_small_kernel(cons
             if (f == 0) p.fh.scale[rec] = make_float2(sc, sum);
             const int X = __float2int_rn(hv * inv);
             const int hi_d = (X + 128) >> 8, lo_d = X - (hi_d << 8);
-            unsigned char* d = p.fh.digits + rec * 128 + ((f >> 4) & 3) * 16 + ((f >> 3) & 1) * 8 + (f & 1) * 4 + ((f & 7) >> 1);
+            const int lo7 = __float2int_rn(fmaf(hv, inv, -(float)X) * 128.f);
+            unsigned char* d = p.fh.digits + rec * 192 + ((f >> 4) & 3) * 16 + ((f >> 3) & 1) * 8 + (f & 1) * 4 + ((f & 7) >> 1);
             d[0] = (unsigned char)(hi_d & 0xFF);
             d[64] = (unsigned char)(lo_d & 0xFF);
+            d[128] = (unsigned char)(lo7 & 0xFF);
             p.h[pos * p.I + n0 + f] = h16;
         }
     }
@@ -296,12 +325,13 @@ struct DownSmallParams {
 
 // A block's item: 16 features of one token; warp j * slices + k is slice k of the token's j-th expert.
 __global__ void __launch_bounds__(kSmallThreads, 1) moe_down_small_kernel(const DownSmallParams p) {
-    __shared__ float part[2][16][16];
+    __shared__ float part[2][16][2][16];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int j = warp / p.slices, ks = warp % p.slices;
     const int G = p.I / 64, NB = p.D / 16, total = p.T * NB;
     const int pairs = (G + 1) / 2, p0 = pairs * ks / p.slices, p1 = pairs * (ks + 1) / p.slices;
     const bool even = (G & 1) == 0, mine = j < p.topk;
+    const int radix = t & 1 ? 0 : 256;
     pdl_launch_dependents();
     // the routing was complete before the gate/up kernel let this one start (it is read past the L1 cache), and the weights
     // depend on nothing else
@@ -320,17 +350,17 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_down_small_kernel(const 
         float acc[2] = {0.f, 0.f};
         if (mine) {
             const uint32_t pos = __ldcg(p.pos + tok * p.topk + j);
-            // one activation row: its high digits are column 0, the low ones column 1, the other columns zero
-            const unsigned char* hd = p.fh.digits + (size_t)pos * G * 128 + (g & 1) * 64 + t * 16;
+            // one activation row: its digits are the first four columns, the others zero
+            const unsigned char* hd = p.fh.digits + (size_t)pos * G * 192 + min(g & 3, 2) * 64 + t * 16;
             const float2* hs = p.fh.scale + (size_t)pos * G;
             auto compute = [&](const SmallBatch& v, int pr) {
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     const int grp = 2 * pr + u;
                     if (grp >= G) break;
-                    uint4 xb = *reinterpret_cast<const uint4*>(hd + grp * 128);
-                    if (g > 1) xb = make_uint4(0, 0, 0, 0);
-                    small_mma(acc, v, u, xb, hs[grp]);
+                    uint4 xb = *reinterpret_cast<const uint4*>(hd + grp * 192);
+                    if (g > 3) xb = make_uint4(0, 0, 0, 0);
+                    small_mma(acc, v, u, xb, small_part(hs[grp], t), radix);
                 }
             };
             int pr = p0;
@@ -348,9 +378,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_down_small_kernel(const 
             }
         }
         row = next_row;
-        if (t == 0) {  // row 0 of the set
-            part[n & 1][warp][g] = acc[0];
-            part[n & 1][warp][g + 8] = acc[1];
+        if (t < 2) {  // row 0 of the set
+            part[n & 1][warp][t][g] = acc[0];
+            part[n & 1][warp][t][g + 8] = acc[1];
         }
         __syncthreads();
         if (tid < 16) {
@@ -359,7 +389,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) moe_down_small_kernel(const 
             for (int k = 0; k < p.topk; k++) {
                 const uint32_t pos = __ldcg(p.pos + tok * p.topk + k);
                 float y = 0.f;
-                for (int q = 0; q < p.slices; q++) y += part[n & 1][k * p.slices + q][tid];
+                for (int q = 0; q < p.slices; q++) y += part[n & 1][k * p.slices + q][0][tid] + part[n & 1][k * p.slices + q][1][tid];
                 if (p.ebias != nullptr) y += p.ebias[(size_t)__ldcg(p.inds + tok * p.topk + k) * p.D + d];
                 const __half y16 = __float2half_rn(y);
                 p.yd[(size_t)pos * p.D + d] = y16;

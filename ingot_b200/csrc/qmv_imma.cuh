@@ -118,7 +118,7 @@ __device__ __forceinline__ void unpack6x16(uint32_t w0, uint32_t w1, uint32_t w2
 // X + 2^(BITS-1) in the low bits, and four digits go through the shifts and masks at a time. The conversion is every CTA's
 // prologue and was a third of all instructions of a launch of four rows and 14336 inputs at 80 per eight inputs.
 // 7 bits: this file's kernel and the ring kernel where it stands in for it. 8 bits: the kernels that took over from fp16 MMAs,
-// whose activations had 11 bits of their own (the ring kernel's 4-bit formats with a third digit, see there).
+// whose activations had 11 bits of their own (the ring kernel's 4-bit formats and the MoE block of few tokens with a third digit, see there).
 template <bool W8, int BITS>
 __device__ __forceinline__ void qi_digits8(const float (&v)[8], float inv, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
 #pragma unroll
@@ -136,6 +136,25 @@ __device__ __forceinline__ void qi_digits8(const float (&v)[8], float inv, uint3
             const uint32_t l = (__byte_perm(p0, p1, 0x6420) & 0x7F7F7F7Fu) ^ 0x40404040u;  // seven bits, sign flipped back ...
             lo[h] = l + ((l & 0x40404040u) << 1);                                           // ... and extended
         }
+    }
+}
+
+// Eight activations as 2^8 d[0] + d[1] + 2^-7 d[2] in units of 1 / inv, signed bytes, words of four: the 16 bits of qi_digits8, and
+// what their rounding left over in units of 2^-7 (-64 .. 64).
+template <bool W8>
+__device__ __forceinline__ void qi_digits23(const float (&v)[8], float inv, uint32_t (&d)[3][2]) {
+    constexpr float kInt = 12582912.0f;  // 1.5 * 2^23
+    qi_digits8<W8, 8>(v, inv, d[0], d[1]);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        uint32_t l[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float x = v[W8 ? 4 * h + i : 2 * i + h];
+            const float whole = fmaf(x, inv, kInt + 128.f) - (kInt + 128.f);
+            l[i] = __float_as_uint(fmaf(fmaf(x, inv, -whole), 128.f, kInt));
+        }
+        d[2][h] = __byte_perm(__byte_perm(l[0], l[1], 0x0040), __byte_perm(l[2], l[3], 0x0040), 0x5410);
     }
 }
 

@@ -44,25 +44,6 @@ __host__ __device__ constexpr int qr_record(bool g32, int lay) { return (lay == 
 __host__ __device__ constexpr int qr_scales(int lay) { return lay == kQr23Tall ? 8 : 4; }   // float2 {2^(e-15), sum x} of a group and set
 __host__ __device__ constexpr int qr_sums(int lay) { return lay == kQr23Tall ? 128 : 64; }  // sums of a set and 16 weight rows
 
-// Eight activations as 2^8 d[0] + d[1] + 2^-7 d[2] in units of 1 / inv, signed bytes, words of four: the 16 bits of qi_digits8, and
-// what their rounding left over in units of 2^-7 (-64 .. 64).
-template <bool W8>
-__device__ __forceinline__ void qr_digits23(const float (&v)[8], float inv, uint32_t (&d)[3][2]) {
-    constexpr float kInt = 12582912.0f;  // 1.5 * 2^23
-    qi_digits8<W8, 8>(v, inv, d[0], d[1]);
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        uint32_t l[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float x = v[W8 ? 4 * h + i : 2 * i + h];
-            const float whole = fmaf(x, inv, kInt + 128.f) - (kInt + 128.f);
-            l[i] = __float_as_uint(fmaf(fmaf(x, inv, -whole), 128.f, kInt));
-        }
-        d[2][h] = __byte_perm(__byte_perm(l[0], l[1], 0x0040), __byte_perm(l[2], l[3], 0x0040), 0x5410);
-    }
-}
-
 // Eight inputs (unit w8 of a group, its threads neighbouring lanes) as block fixed point, in B-fragment order: the digits from
 // the highest down, four lanes' fragments each, STEP bytes from digit to digit. BITS: of a digit; 23: three digits, and SE
 // scale entries (two: for the lane with the high and middle digits, with the sum, and for the one with the low digit).
@@ -90,7 +71,7 @@ __device__ __forceinline__ void qr_convert(const float (&v)[8], int w8, bool liv
             if (SE == 2) scale_out[SE - 1] = make_float2(scale * 0.0078125f, 0.f);
         }
         uint32_t d[3][2];
-        qr_digits23<W8>(v, inv, d);
+        qi_digits23<W8>(v, inv, d);
 #pragma unroll
         for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(f + i * STEP) = make_uint2(d[i][0], d[i][1]);
     } else {

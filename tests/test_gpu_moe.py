@@ -422,3 +422,30 @@ def test_moe_pieces_and_external_routing(cuda_device):
     layer.set_external_routing(None, None)
     ref = qref.moe_ffn(x, inds.cpu().numpy().astype(np.uint32), wts.cpu().numpy(), host["weights"])
     assert qref.max_rel(out.cpu().numpy(), ref) <= TOL
+
+
+@pytest.mark.parametrize("D,I,T", [(2880, 192, 1), (1600, 320, 2), (2880, 768, 3), (128, 64, 3)])
+def test_moe_few_tokens_keep_activations_whole(cuda_device, D, I, T):
+    """Up to three tokens, input channels 100 times the rest: h is the fp16 rounding of the 64-bit gated product but for the values
+    that lie within the fp32 sums' error of a rounding boundary: some 3e-6 of a value either way, of 2^-11: about 1 %. (16-bit
+    digits: a third to a half of all h.)"""
+    rng = np.random.default_rng(960 + D + I + T)
+    E, K = 32, 4
+    layer, host = build_layer(rng, cuda_device, E, K, D, I, max_tokens=T)
+    x = rng.normal(0, 0.2, size=(T, D)).astype(np.float32)
+    x[:, rng.choice(D, 3, replace=False)] *= 100
+    xt = torch.from_numpy(x).to(cuda_device).to(torch.bfloat16)
+    out = torch.zeros(T, D, dtype=torch.float32, device=cuda_device)
+    layer.encode(xt, out, T)
+    assert capi.context(0).device_status() == 0
+    v = layer.views(T)
+    x64 = xt.double().cpu().numpy()
+    inds, row_map, h = (v[k].cpu().numpy() for k in ("inds", "row_map", "h"))
+    off = total = 0
+    for r, pair in enumerate(row_map.astype(np.int64)):
+        g, u, _ = (w.astype(np.float64) for w in host["weights"](int(inds.reshape(-1)[pair])))
+        xg, xu = g @ x64[pair // K], u @ x64[pair // K]
+        want = (xg / (1 + np.exp(-xg)) * xu).astype(np.float16)
+        off += int((want.view(np.uint16) != h[r].view(np.uint16)).sum())
+        total += I
+    assert off <= 0.03 * total, (off, total)
