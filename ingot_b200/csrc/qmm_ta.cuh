@@ -372,7 +372,9 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                             for (int e = 0; e < SPB / 4; e++)
                                 sts32(dst + t * 128 * SPB + (lane + 32 * i) * SPB + 4 * e, v[i][t][2 * e] | (v[i][t][2 * e + 1] << 16));
                 }
-                cp_async_arrive_noinc(bar_cfull + 8 * s);
+                // (the copies' arrival orders copies only: plain stores are published by an arrival that releases them)
+                if (p.vec) cp_async_arrive_noinc(bar_cfull + 8 * s);
+                else mbar_arrive(bar_cfull + 8 * s);
                 if (++s == p.nc) { s = 0; ph ^= 1; }
             }
         }

@@ -130,3 +130,23 @@ def test_qmm_8bit_stages_of_odd_number(cuda_device):
     for _ in range(20):
         flush.zero_()
         assert torch.equal(run_qmm(m, xt, M), y)
+
+
+@pytest.mark.parametrize("fmt,group", [("q4", 64), ("q8", 64), ("q4", 32), ("mxfp4", 32)])
+@pytest.mark.parametrize("M", [64, 320])
+def test_qmm_scales_by_plain_loads(cuda_device, fmt, group, M):
+    """2880 inputs: the rows of scales are no multiple of the pieces that asynchronous copies take, so they go through plain loads
+    and stores. Launches with everything out of L2, and with it in L2, give the same bits every time."""
+    rng = np.random.default_rng(66 + M + group)
+    N, K = 1152, 2880
+    bits = 8 if fmt == "q8" else 4
+    m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, bits, cuda_device, group=group)
+    x = synth.activations_np(rng, M, K)
+    xt = x_tensor(x, cuda_device)
+    y = run_qmm(m, xt, M)
+    assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(x, deq(host, bits, group=group))) <= TOL
+    flush = torch.empty(160 << 20, dtype=torch.uint8, device=cuda_device)
+    for i in range(20):
+        if i % 2 == 0:
+            flush.zero_()
+        assert torch.equal(run_qmm(m, xt, M), y)
