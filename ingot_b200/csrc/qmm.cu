@@ -233,7 +233,8 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     // base to be multiples of it
     const int srow = c.fmt == kFmtMxfp4 ? c.K / 32 : (c.fmt == kFmtTernary ? c.K / 64 : (c.fmt == kFmtAffine4G32 ? c.K / 16 : c.K / 32));
     const int spb = c.fmt == kFmtAffine8 ? 4 : (c.fmt == kFmtAffine4G32 ? 16 : 8);
-    p.vec = srow % spb == 0 && (align & (uintptr_t)(spb - 1)) == 0 ? 1 : 0;
+    p.vec = srow % spb == 0 && (align & (uintptr_t)(spb - 1)) == 0 ? 1 : (align & 1) ? -1 : 0;
+    if (p.vec < 0 && c.fmt != kFmtMxfp4) return fail(ctx, kErrInvalidArg, "qmm: scales and biases must be 2-byte aligned");
     p.expert_lo = c.expert_lo;
     p.early = c.early ? 1 : 0;
     p.N = c.N; p.K = c.K; p.M = c.M;

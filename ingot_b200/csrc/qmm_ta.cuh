@@ -83,7 +83,7 @@ struct TaParams {
     int32_t x_stage;         // bytes of an X stage
     int32_t dcols;           // columns per accumulator: 64, 128 or 192
     int32_t early;           // the tile list is complete when the kernel starts
-    int32_t vec;             // the row pitch of the scales allows asynchronous copies
+    int32_t vec;             // how scales are read: 1 by asynchronous copies, 0 in pairs of bytes, -1 (MXFP4) byte by byte
     int32_t* status;
 };
 
@@ -326,7 +326,8 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     } else if (warp == 3) {
         // ================= producer of the scales and biases =================
         // Per stage of codes the SPB scale bytes of each of the 128 rows: lane l takes rows l, l + 32, ... Row pitches that
-        // allow it go by asynchronous copies, others (an odd number of groups) by two-byte loads. Rows beyond the matrix
+        // allow it go by asynchronous copies, others (an odd number of groups) by two-byte loads, MXFP4 scales at an odd address
+        // (a tensor inside a mapped file) by bytes. Rows beyond the matrix
         // take the last row's: their weights only feed rows of D that are not stored.
         constexpr int SPB = F::SPB, NT = F::BIAS ? 2 : 1;
         const size_t pitch = (size_t)p.K / F::GROUP * F::ES;
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                 if (!(ok = __all_sync(0xffffffffu, ok))) break;
                 const uint32_t dst = scales0 + s * SSTAGE;
                 const int left = (int)pitch - ch * SPB;  // scale bytes of a row from this stage on
-                if (p.vec) {
+                if (p.vec > 0) {
 #pragma unroll
                     for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -362,8 +363,10 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
 #pragma unroll
                         for (int t = 0; t < NT; t++)
 #pragma unroll
-                            for (int e = 0; e < SPB / 2; e++)
-                                v[i][t][e] = ldg_nc_u16(src[i][t] + ch * SPB + min(2 * e, left - 2));
+                            for (int e = 0; e < SPB / 2; e++) {
+                                const char* a = src[i][t] + ch * SPB + min(2 * e, left - 2);
+                                v[i][t][e] = FMT == kFmtMxfp4 && p.vec < 0 ? ldg_nc_u8(a) | (ldg_nc_u8(a + 1) << 8) : ldg_nc_u16(a);
+                            }
 #pragma unroll
                     for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -373,7 +376,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                                 sts32(dst + t * 128 * SPB + (lane + 32 * i) * SPB + 4 * e, v[i][t][2 * e] | (v[i][t][2 * e + 1] << 16));
                 }
                 // (the copies' arrival orders copies only: plain stores are published by an arrival that releases them)
-                if (p.vec) cp_async_arrive_noinc(bar_cfull + 8 * s);
+                if (p.vec > 0) cp_async_arrive_noinc(bar_cfull + 8 * s);
                 else mbar_arrive(bar_cfull + 8 * s);
                 if (++s == p.nc) { s = 0; ph ^= 1; }
             }

@@ -449,3 +449,28 @@ def test_moe_few_tokens_keep_activations_whole(cuda_device, D, I, T):
         off += int((want.view(np.uint16) != h[r].view(np.uint16)).sum())
         total += I
     assert off <= 0.03 * total, (off, total)
+
+
+@pytest.mark.parametrize("T", [2, 70])
+def test_moe_mxfp4_scales_at_odd_addresses(cuda_device, T):
+    """Expert scales one byte into a larger tensor: the same bits as from an aligned one."""
+    rng = np.random.default_rng(970 + T)
+    E, K, D, I = 32, 4, 576, 192
+    w = [synth.mxfp4_np(rng, n, k, E) for n, k in ((I, D), (I, D), (D, I))]
+    wr = synth.bf16_values_tensor(synth.router_np(rng, E, D), cuda_device)
+    xt = x_tensor(synth.activations_np(rng, T, D), cuda_device)
+    outs = []
+    for by in (0, 1):
+        mats = []
+        for codes, scales in w:
+            m = synth.dense_q_mxfp4(codes, scales, cuda_device)
+            buf = torch.full((m.s.numel() + 16,), 255, dtype=torch.uint8, device=cuda_device)
+            m.s = buf[by: by + m.s.numel()].view_as(m.s).copy_(m.s)
+            assert m.s.data_ptr() % 2 == by
+            mats.append(m)
+        layer = MoELayer(RouterSpec(E, K), wr, *mats, max_tokens=T)
+        out = torch.zeros(T, D, dtype=torch.float32, device=cuda_device)
+        layer.encode(xt, out, T)
+        assert capi.context(0).device_status() == 0
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])

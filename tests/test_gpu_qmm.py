@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from ingot_b200 import capi, synth
-from ingot_b200.linear import VQMV
+from ingot_b200.linear import DenseMLP, DenseQ, VQMV
 from oracle import qref
 from gpu_util import TOL, affine_case, deq, mxfp4_case, x_tensor
 
@@ -150,3 +150,38 @@ def test_qmm_scales_by_plain_loads(cuda_device, fmt, group, M):
         if i % 2 == 0:
             flush.zero_()
         assert torch.equal(run_qmm(m, xt, M), y)
+
+
+def shifted_scales(m, by):
+    """The matrix with its MXFP4 scales `by` bytes into a larger tensor, as views of a mapped file have them."""
+    buf = torch.full((m.s.numel() + 16,), 255, dtype=torch.uint8, device=m.s.device)  # (255 is NaN: a scale read beside its place shows)
+    s = buf[by: by + m.s.numel()].view_as(m.s)
+    s.copy_(m.s)
+    assert s.data_ptr() % 16 == by
+    return DenseQ(m.w, s, None, m.N, m.K, 4, 32, "mxfp4", m.experts)
+
+
+@pytest.mark.parametrize("by", [1, 2, 4, 8, 9])
+@pytest.mark.parametrize("K", [64, 576, 1024])
+def test_mxfp4_scales_at_any_address(cuda_device, K, by):
+    """MXFP4 scales are bytes: any address will do, in the GEMM, the GEMV and the dense FFN of few and of many rows."""
+    rng = np.random.default_rng(67 + K + by)
+    N = 192
+    m, host = mxfp4_case(rng, N, K, cuda_device)
+    o = shifted_scales(m, by)
+    for M in (64, 320):
+        x = synth.activations_np(rng, M, K)
+        assert qref.max_rel(run_qmm(o, x_tensor(x, cuda_device), M).cpu().numpy(), qref.matmul_t(x, deq(host))) <= TOL
+    dn, _ = mxfp4_case(rng, K, 64, cuda_device)
+    gu, _ = mxfp4_case(rng, 128, K, cuda_device)
+    for rows in (1, 7, 64):
+        xt = x_tensor(synth.activations_np(rng, rows, K), cuda_device)
+        a, b = (torch.zeros(rows, K, dtype=torch.float32, device=cuda_device) for _ in range(2))
+        DenseMLP(gu, dn).encode(xt, a, rows)
+        DenseMLP(shifted_scales(gu, by), shifted_scales(dn, by)).encode(xt, b, rows)
+        assert qref.max_rel(b.cpu().numpy(), a.cpu().numpy()) <= TOL  # (other kernels where the address rules the first out)
+        if rows <= 16:
+            y = torch.zeros(rows, N, dtype=torch.float32, device=cuda_device)
+            VQMV.encode(xt, o, y, rows)
+            assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(xt.float().cpu().numpy(), deq(host))) <= TOL
+    assert capi.context(0).device_status() == 0
