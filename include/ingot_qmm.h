@@ -165,7 +165,8 @@ int32_t iq_qmm_w8a8(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, i
 /* ---- dense gated FFN ------------------------------------------------------------------------------------------------
  * out[rows, d] (+)= down( act(gate x) * up x ) with gate|up concatenated by rows as one [2*d_ff, d] matrix (gate rows
  * first). Replaces DenseMLP.encode / encodePrefill (Sources/Ingot/Layers/Dense.swift:56-96) and dswiglu*
- * (Shaders/yy_model.metal:187-227). rows <= 16 takes the GEMV path, larger multiples of 64 the GEMM path. */
+ * (Shaders/yy_model.metal:187-227). rows <= 16 takes the GEMV path, larger multiples of 64 the GEMM path. The workspace is
+ * 16-byte aligned. */
 int32_t iq_dense_ffn_workspace_bytes(iq_ctx* ctx, const iq_qlinear* gate_up, const iq_qlinear* down, int32_t rows,
                                      int32_t x_dtype, size_t* bytes);
 int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* gate_up,

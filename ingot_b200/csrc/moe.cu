@@ -499,8 +499,8 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
     size_t need = 0;
     int32_t st = iq_dense_ffn_workspace_bytes(ctx, gate_up, down, rows, x_dtype, &need);
     if (st != kOk) return st;
-    if (workspace == nullptr || workspace_bytes < need)
-        return fail(ctx, kErrWorkspace, "dense_ffn: workspace %zu < %zu", workspace_bytes, need);
+    if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0)
+        return fail(ctx, kErrWorkspace, "dense_ffn: workspace %zu < %zu (16-byte aligned)", workspace_bytes, need);
     if (act < IQ_ACT_SILU || act > IQ_ACT_RELU2) return fail(ctx, kErrUnsupported, "dense_ffn: activation %d", act);
     const int32_t fmt = format_of(gate_up);
     if (fmt < 0 || format_of(down) < 0) return fail(ctx, kErrUnsupported, "dense_ffn: weight format");

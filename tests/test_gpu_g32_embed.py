@@ -237,3 +237,22 @@ def test_dense_ffn_row_invariance(cuda_device, bits, group, D, F):
     for i in (3, 8, 15):
         assert torch.equal(ffn(x[i:i + 1])[0], full[i]), i
     assert capi.context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("rows", [2, 16, 64])
+def test_dense_ffn_refuses_an_unaligned_workspace(cuda_device, rows):
+    """Its parts are written 8 and 16 bytes at a time."""
+    rng = np.random.default_rng(80)
+    gu, _ = affine_case(rng, 2 * 1024, 1024, 4, cuda_device)
+    dn, _ = affine_case(rng, 1024, 1024, 4, cuda_device)
+    x = torch.zeros(rows, 1024, dtype=torch.bfloat16, device=cuda_device)
+    out = torch.zeros(rows, 1024, dtype=torch.float32, device=cuda_device)
+    ctx, n = capi.context(0), capi.C.c_size_t()
+    a, b = gu.qlinear(), dn.qlinear()
+    ctx.check(capi.lib().iq_dense_ffn_workspace_bytes(ctx.handle, capi.C.byref(a), capi.C.byref(b), rows, capi.IQ_BF16, capi.C.byref(n)))
+    ws = torch.empty(n.value + 16, dtype=torch.uint8, device=cuda_device)
+    for off, want in ((8, -4), (4, -4), (2, -4), (0, 0)):
+        st = capi.lib().iq_dense_ffn(ctx.handle, torch.cuda.current_stream().cuda_stream, x.data_ptr(), capi.IQ_BF16, 1024, capi.C.byref(a),
+                                     capi.C.byref(b), capi.IQ_ACT_SILU, 0.0, out.data_ptr(), capi.IQ_F32, 1024, rows, 0, ws.data_ptr() + off, n.value)
+        assert st == want, (off, st)
+    assert ctx.device_status() == 0
