@@ -128,6 +128,8 @@ int32_t qmv_with_scratch(iq_ctx* ctx, void* stream, const void* x, int32_t x_dty
                          int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix, void* scratch);
 // Tiles of up to eight rows of affine 4-bit experts on the int8 kernel; 1: the shape does not fit it
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
+// Whether its gate/up form takes the token rows as fixed point (GqmvCall::fx) for K inputs; for others it converts them itself
+bool qmv_grouped_takes_fixed(const iq_ctx* ctx, int K);
 
 // One launch of the tensor-core GEMM (csrc/qmm.cu). x16: fp16 activations [x_rows, ldx] (bf16 with the plain bf16 format); w[i]: stacked
 // [experts * N, K] codes (w[1]: the up matrix of the gate/up epilogue). tiles == nullptr: dense tiling over M x N.

@@ -740,8 +740,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     int32_t st;
 
     const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l);
+    const bool takes_fixed = l->fmt == kFmtAffine4 && qmv_grouped_takes_fixed(ctx, d.d_model);
     if (small) {
-        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, l->fmt == kFmtAffine4, small_experts);
+        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, small_experts || takes_fixed, small_experts);
         if (st == kOk && small_experts)
             st = run_experts_small(l, cs, tokens, w, out, out_dtype, ldo, (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0);
         if (st != kOk) return st;
@@ -816,8 +817,8 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     }
     const bool int8 = use_int8_path(l, P, d.expert_count);
     const int bn = tensor_tile_rows(P, d.expert_count);
-    // whole calls on the int8 kernels: the counting kernel leaves the activations as fixed point for the gate/up one
-    const bool fixed = int8 && (pieces & IQ_PIECE_GATEUP) && (small || ((pieces & IQ_PIECE_GROUP) && tokens <= kFixedTokens && P < kGroupChunkedMinPairs));
+    // whole calls on the int8 kernels: the counting kernel leaves the activations as fixed point for the gate/up one, where that takes them
+    const bool fixed = int8 && takes_fixed && (pieces & IQ_PIECE_GATEUP) && (small || ((pieces & IQ_PIECE_GROUP) && tokens <= kFixedTokens && P < kGroupChunkedMinPairs));
     if (pieces & IQ_PIECE_GROUP) {
         GroupParams gp;
         gp.inds = inds; gp.counts = w.counts; gp.offsets = w.offsets; gp.row_map = w.row_map; gp.pos = w.pos;

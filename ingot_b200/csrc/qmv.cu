@@ -398,6 +398,9 @@ QgKernel qg_pick(int mode, bool tm, bool gw4, bool fx = false) {
 }
 }  // namespace
 
+// Sixteen consumer warps: K slices of four groups that divide them (K = 256, 512, 1024, 2048, 4096)
+bool qmv_grouped_takes_fixed(const iq_ctx* ctx, int K) { return ctx->encode_tiled != nullptr && K % 256 == 0 && K <= 4096 && 16 % (K / 256) == 0; }
+
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     if ((c.mode != kModeGateUp && c.mode != kModeDown) || c.tiles == nullptr || c.fmt != kFmtAffine4) return 1;
@@ -424,9 +427,8 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     p.srow_bytes = G * 2;
     p.xq_bytes = G * ms * 512;
     p.xsc_bytes = G * ms * 32;
-    // Sixteen consumer warps with the token rows as fixed point: K slices of four groups that divide them (K = 1024, 2048,
-    // 4096), gate/up tiles of eight rows
-    const bool fx = c.fx != nullptr && c.mode == kModeGateUp && tm && c.row_map != nullptr && G % 4 == 0 && G / 4 <= 16 && 16 % (G / 4) == 0;
+    // Sixteen consumer warps with the token rows as fixed point: gate/up tiles of eight rows
+    const bool fx = c.fx != nullptr && c.mode == kModeGateUp && tm && c.row_map != nullptr && qmv_grouped_takes_fixed(ctx, c.K);
     const int kQgWarps = fx ? 16 : 8;
     if (fx) { p.fx = *c.fx; p.xq_bytes = p.xsc_bytes = 0; }
     p.red_bytes = 2 * kQgWarps * nw * ms * 64 * 4;

@@ -474,3 +474,12 @@ def test_moe_mxfp4_scales_at_odd_addresses(cuda_device, T):
         assert capi.context(0).device_status() == 0
         outs.append(out)
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("D,I", [(1536, 128), (3072, 64), (5120, 64), (768, 1536)])
+@pytest.mark.parametrize("T", [4, 40])
+def test_moe_decode_widths_that_are_no_power_of_two(cuda_device, D, I, T):
+    """Widths whose K slices do not divide the sixteen warps: the int8 kernels convert the token rows themselves, gate/up as down."""
+    rng = np.random.default_rng(980 + D + T)
+    layer, host = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
+    check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
