@@ -371,7 +371,7 @@ __device__ __forceinline__ float exact_dot_bf16(const uint16_t* __restrict__ xro
     double a4[4] = {0.0, 0.0, 0.0, 0.0};  // four independent chains (the float64 adds would otherwise wait for each other)
     for (int u = lane; u < D / 8; u += 32) {
         const uint4 xv = *reinterpret_cast<const uint4*>(xrow + u * 8);
-        const uint4 wv = ldg_nc_u4(wrow + u * 8);
+        const uint4 wv = __ldg(reinterpret_cast<const uint4*>(wrow + u * 8));
         const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {

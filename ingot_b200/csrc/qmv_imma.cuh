@@ -434,8 +434,10 @@ __global__ void __launch_bounds__(kQiMaxThreads, MS == 1 ? 2 : 1)
             *reinterpret_cast<uint2*>(xq + fb + 64) = make_uint2(0, 0);
             if (w8 == 0) xsc[j * 4 * MS + m] = make_float2(0.f, 0.f);
         }
-        auto convert = [&](const float (&v)[8], int u) {
-            const int m = u / (G * 8), j = (u >> 3) % G, w8 = u & 7;
+        // row of unit u (no division for a single row: it is a fair part of that call's prologue)
+        auto row_of = [&](int u) { return p.M == 1 ? 0 : u / (G * 8); };
+        auto convert = [&](const float (&v)[8], int u, int m) {
+            const int j = (u - m * (G * 8)) >> 3, w8 = u & 7;
             float amax = 0.f, sum = 0.f;
 #pragma unroll
             for (int k = 0; k < 8; k++) {
@@ -462,9 +464,10 @@ __global__ void __launch_bounds__(kQiMaxThreads, MS == 1 ? 2 : 1)
         const int units = G * 8 * p.M;  // (a multiple of 32: whole warps leave the loops together)
         if (units <= 2 * nct) {
             for (int u = tid; u < units; u += nct) {
+                const int m = row_of(u);
                 float v[8];
-                load_x8(p.x, p.x_dtype, (size_t)(u / (G * 8)) * p.ldx + (u % (G * 8)) * 8, v);
-                convert(v, u);
+                load_x8(p.x, p.x_dtype, (size_t)m * p.ldx + (u - m * (G * 8)) * 8, v);
+                convert(v, u, m);
             }
         } else {  // four loads under way per thread
             for (int u0 = tid; u0 < units; u0 += 4 * nct) {
@@ -479,7 +482,7 @@ __global__ void __launch_bounds__(kQiMaxThreads, MS == 1 ? 2 : 1)
                     if (u0 + q * nct >= units) break;
                     float v[8];
                     unpack_x8(raw[q], p.x_dtype, v);
-                    convert(v, u0 + q * nct);
+                    convert(v, u0 + q * nct, (u0 + q * nct) / (G * 8));
                 }
             }
         }

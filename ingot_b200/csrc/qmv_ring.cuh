@@ -215,13 +215,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
 
     // ---- activations -> block fixed point, two 8-bit digits, in B-fragment order (see qmv_imma.cuh) ---------------------
     const int nthreads = nwarps * 32;
-    for (int u = tid; u < G * TPG * (RPS * MS - p.M); u += nthreads) {  // rows the call does not have: zero digits and scale
-        const int m = p.M + u / (G * TPG), j = (u / TPG) % G, w8 = u % TPG;
-        unsigned char* f = xq + (size_t)(j * MS + m / RPS) * SETB + (m % RPS) * RSTEP + (G32 ? w8 * 8 : (w8 >> 1) * 16 + (w8 & 1) * 8);
-#pragma unroll
-        for (int i = 0; i < REC / (4 * XL); i++) *reinterpret_cast<uint2*>(f + i * DSTEP) = make_uint2(0, 0);
-        if (w8 < SE) xsc[j * SPS * MS + m * SE + w8] = make_float2(0.f, 0.f);
-    }
+    // (rows the call does not have keep what the memory held: a column of B feeds its own column of D, which nobody reads)
     if (p.xd != nullptr) {
         constexpr int PC = REC / 16, PD = XL / 4;  // 16-byte pieces of a record, of a digit
         for (int m = 0; m < p.M; m++) {
@@ -233,8 +227,10 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
     const int units = p.xd != nullptr ? 0 : G * TPG * p.M, upad = (units + 31) / 32 * 32;  // whole warps: the groups' shuffles need their threads
-    auto convert = [&](const float (&v)[8], int u) {
-        const int m = u / (G * TPG), j = (u / TPG) % G;
+    // row of unit u (no division for a single row: it is a fair part of that call's prologue)
+    auto row_of = [&](int u) { return p.M == 1 ? 0 : u / (G * TPG); };
+    auto convert = [&](const float (&v)[8], int u, int m) {
+        const int j = (u - m * (G * TPG)) / TPG;
         unsigned char* rec = xq + (size_t)(j * MS + m / RPS) * SETB + (m % RPS) * RSTEP;
         float2* sc = xsc + j * SPS * MS + m * SE;
         if (WIDE) qr_convert<W8, G32, 23, DSTEP, SE>(v, u % TPG, u < units, rec, sc);
@@ -243,10 +239,10 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
     };
     if (units <= 2 * nthreads) {
         for (int u = tid; u < upad; u += nthreads) {
-            const int uc = min(u, units - 1);
+            const int uc = min(u, units - 1), m = row_of(uc);
             float v[8];
-            load_x8(p.x, p.x_dtype, (size_t)(uc / (G * TPG)) * p.ldx + (uc % (G * TPG)) * 8, v);
-            convert(v, u);
+            load_x8(p.x, p.x_dtype, (size_t)m * p.ldx + (uc - m * (G * TPG)) * 8, v);
+            convert(v, u, m);
         }
     } else {  // four loads under way per thread
         for (int u0 = tid; u0 < upad; u0 += 4 * nthreads) {
@@ -261,7 +257,7 @@ __global__ void __launch_bounds__(kQrMaxWarps * 32, 1) qmv_ring_kernel(const __g
                 if (u0 + q * nthreads >= upad) break;  // (whole warps)
                 float v[8];
                 unpack_x8(raw[q], p.x_dtype, v);
-                convert(v, u0 + q * nthreads);
+                convert(v, u0 + q * nthreads, (u0 + q * nthreads) / (G * TPG));
             }
         }
     }
