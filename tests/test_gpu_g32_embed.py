@@ -256,3 +256,24 @@ def test_dense_ffn_refuses_an_unaligned_workspace(cuda_device, rows):
                                      capi.C.byref(b), capi.IQ_ACT_SILU, 0.0, out.data_ptr(), capi.IQ_F32, 1024, rows, 0, ws.data_ptr() + off, n.value)
         assert st == want, (off, st)
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("bits,group", [(4, 64), (8, 64), (4, 32)])
+def test_dense_ffn_inputs_too_wide_for_the_other_kernels(cuda_device, bits, group):
+    """Gate + up + activation on the register-staged fp16 kernel."""
+    rng = np.random.default_rng(75 + bits + group)
+    D, F, rows = 40960, 64, 9
+    gu, hgu = affine_case(rng, 2 * F, D, bits, cuda_device, group=group)
+    dn, hdn = affine_case(rng, D, F, bits, cuda_device, group=group)
+    xh = synth.activations_np(rng, rows, D)
+    wgu = deq(hgu, bits, group=group)
+    h = qref.round_f16(qref.silu_glu(qref.matmul_t(xh, wgu[:F]), qref.matmul_t(xh, wgu[F:])))
+    ref = qref.matmul_t(h, deq(hdn, bits, group=group))
+    x = x_tensor(xh, cuda_device)
+    out, one = (torch.zeros(n, D, dtype=torch.float32, device=cuda_device) for n in (rows, 1))
+    mlp = DenseMLP(gu, dn)
+    mlp.encode(x, out, rows)
+    mlp.encode(x[4:5].contiguous(), one, 1)
+    assert capi.context(0).device_status() == 0
+    assert qref.max_rel(out.cpu().numpy(), ref) <= 2 * TOL  # h is rounded to fp16 on both sides, from sums in other orders
+    assert torch.equal(one[0], out[4])

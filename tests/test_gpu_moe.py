@@ -104,8 +104,8 @@ def test_moe_small_mxfp4_gptoss_style(cuda_device, T):
 @pytest.mark.parametrize("T", [1, 8, 16, 64, 100, 256, 512])
 def test_moe_c2_configuration(cuda_device, T):
     """128 experts, top-8, d_model 2048, d_ff 768, 4-bit g64, bf16 router ~ N(0, 0.02), x ~ N(0, 1), seed 0. The token
-    counts walk the decode tile kernels (8-row tiles with one and two live row sets, 16-row tiles) and the first size of
-    the grouped GEMM."""
+    counts walk the three-kernel path, the decode tile kernels (8-row tiles with one and two live row sets) and the grouped GEMM
+    (from 100 tokens on)."""
     rng = np.random.default_rng(0)
     layer, host = build_layer(rng, cuda_device, 128, 8, 2048, 768, max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, 2048), T, "silu")
@@ -113,7 +113,7 @@ def test_moe_c2_configuration(cuda_device, T):
 
 def test_moe_c2_layer_at_the_benchmarked_size(cuda_device):
     """The layer the 48-layer stack is made of, at the benchmark's 4096 prefill tokens (32,768 routed rows: the chunked
-    counting sort, 256-row tiles, the single-accumulator gate/up path): logits, indices, weights and the whole permutation
+    counting sort, tiles of 192 and 64 rows): logits, indices, weights and the whole permutation
     against the oracle in full, the outputs on 32 sampled tokens."""
     rng = np.random.default_rng(4096)
     T, E, K, D, I = 4096, 128, 8, 2048, 768
@@ -285,7 +285,8 @@ def test_tensor_router_near_ties_at_the_boundary(cuda_device):
 @pytest.mark.parametrize("T", [3, 200])
 def test_router_8bit_affine(cuda_device, T):
     """A router stored as 8-bit affine codes (MoE.swift:258-273 keeps the router quantized when the checkpoint does): the
-    logits are the float64 dot products with the fp32 weights s*q + b, bit for bit, through both router kernels."""
+    logits are the float64 dot products with the fp32 weights s*q + b, bit for bit, in the cluster that routes a few tokens
+    and in the kernel for more (the tiled GEMM for many: test_router_tiled_float64_gemm)."""
     rng = np.random.default_rng(70 + T)
     E, K, D, I = 64, 4, 256, 128
     g, u, d = synth.affine_np(rng, I, D, 4, E), synth.affine_np(rng, I, D, 4, E), synth.affine_np(rng, D, I, 4, E)
@@ -310,8 +311,8 @@ def test_router_8bit_affine(cuda_device, T):
 @pytest.mark.parametrize("act", ["gelu", "relu2"])
 @pytest.mark.parametrize("T", [3, 40, 700])
 def test_moe_other_activations(cuda_device, act, T):
-    """GELU (tanh form) gate and relu^2 without gate (qmm.metal:9-31 ACT 1 and 3) through the decode tiles (int8 and fp16
-    GEMV kernels) and the tcgen05 grouped GEMM."""
+    """GELU (tanh form) gate and relu^2 without gate (qmm.metal:9-31 ACT 1 and 3) through the three-kernel path, the decode tiles and
+    the tcgen05 grouped GEMM."""
     rng = np.random.default_rng(90 + T)
     layer, host = build_layer(rng, cuda_device, 32, 2, 2048, 128, act=act, max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, 2048), T, act)
@@ -483,3 +484,39 @@ def test_moe_decode_widths_that_are_no_power_of_two(cuda_device, D, I, T):
     rng = np.random.default_rng(980 + D + T)
     layer, host = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
+
+
+@pytest.mark.parametrize("kind,E,D,T", [("q8", 512, 2048, 100), ("q8", 64, 1408, 1030), ("sigmoid", 256, 4096, 101), ("f16", 96, 2880, 333),
+                                       ("f32", 32, 4096, 1025)])
+def test_router_tiled_float64_gemm(cuda_device, kind, E, D, T):
+    """More than 90 million products and no tensor-core route (an 8-bit router, sigmoid scores, activations that are not bf16): the
+    register-tiled float64 GEMM, both tile heights, token and expert tiles that are not full, the K range over a cluster or not.
+    The logits are the correctly rounded float64 dot products."""
+    assert T * E * D > 90_000_000 and T > 64
+    rng = np.random.default_rng(990 + E + T)
+    K, I = 4, 64
+    g, u, d = synth.affine_np(rng, I, D, 4, E), synth.affine_np(rng, I, D, 4, E), synth.affine_np(rng, D, I, 4, E)
+    mk = lambda t: synth.dense_q_affine(t[0], t[1], t[2], 4, cuda_device)
+    extra, spec = {}, RouterSpec(E, K)
+    if kind == "q8":
+        rw, rs, rb = synth.affine_np(rng, E, D, 8)
+        dev_t = lambda a, dt: torch.from_numpy(a[0].view(dt).copy()).to(cuda_device)
+        w, wr = dev_t(rw, np.int32), qref.dequant_affine(rw[0], rs[0], rb[0], 8)
+        extra = {"router_scales": dev_t(rs, np.int16).view(torch.bfloat16), "router_biases": dev_t(rb, np.int16).view(torch.bfloat16)}
+    else:
+        wr = synth.router_np(rng, E, D)
+        w = synth.bf16_values_tensor(wr, cuda_device)
+        if kind == "sigmoid":
+            spec = RouterSpec(E, K, score="sigmoid")
+    layer = MoELayer(spec, w, mk(g), mk(u), mk(d), max_tokens=T, **extra)
+    dt = {"f16": torch.float16, "f32": torch.float32}.get(kind, torch.bfloat16)
+    xt = torch.from_numpy(rng.normal(0, 1, size=(T, D)).astype(np.float32)).to(cuda_device).to(dt)
+    out = torch.zeros(T, D, dtype=torch.float32, device=cuda_device)
+    layer.encode(xt, out, T, only=("router", "route"))
+    assert capi.context(0).device_status() == 0
+    v = layer.views(T)
+    logits = qref.router_logits(xt.float().cpu().numpy(), wr)
+    got = v["logits"].cpu().numpy()
+    assert np.array_equal(got[:, :E], logits) and not got[:, E:].any()
+    inds, _ = qref.route(logits, K, sigmoid=kind == "sigmoid")
+    assert np.array_equal(v["inds"].cpu().numpy().astype(np.uint32), inds)

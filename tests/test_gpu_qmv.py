@@ -274,3 +274,19 @@ def test_qmv_ring_keeps_16_bit_activations_whole(cuda_device, N, K, rows, group,
         s, b = (np.repeat(synth.bf16_bits_to_f32(t[0]).astype(np.float64), group, axis=1) for t in host[1:])
         ref = xt.double().cpu().numpy() @ (q * s + b).T
         assert np.abs(y.double().cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("fmt,N,K", [("q4", 48, 40960), ("q8", 48, 28672), ("g32", 48, 40960), ("mxfp4", 48, 14336), ("q4", 16, 65600)])
+def test_qmv_inputs_too_wide_for_the_other_kernels(cuda_device, fmt, N, K):
+    """The register-staged fp16 kernel, K walked in tiles that fit shared memory: against the oracle, and the same bits for a row
+    alone, among 8 and among 16."""
+    rng = np.random.default_rng(900 + N + K)
+    bits, group = (8, 64) if fmt == "q8" else (4, 32 if fmt in ("g32", "mxfp4") else 64)
+    m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, bits, cuda_device, group=group)
+    x = synth.activations_np(rng, 16, K)
+    xt = x_tensor(x, cuda_device)
+    full = run(m, xt, 16)
+    assert qref.max_rel(full.cpu().numpy(), qref.matmul_t(x, deq(host, bits, group=group))) <= TOL
+    for rows in (1, 8, 9):
+        assert torch.equal(run(m, xt[:rows].contiguous(), rows), full[:rows]), rows
+    assert torch.equal(run(m, xt[11:12].contiguous(), 1)[0], full[11])
