@@ -120,8 +120,8 @@ int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_
                int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix);
 
 /* ---- prefill GEMM --------------------------------------------------------------------------------------------------
- * Y[rows, n] (+)= X[rows, k] * W^T on the tcgen05 tensor cores (weights dequantised to fp16 in shared memory, fp32
- * accumulation in tensor memory). Replaces DenseQ.encodeQmmF32(ctx, enc, x:, xOffset:, y:, rows:, accumulate:, halfOut:)
+ * Y[rows, n] (+)= X[rows, k] * W^T on the tcgen05 tensor cores (weights dequantised to fp16 and fp32 accumulation,
+ * both in tensor memory). Replaces DenseQ.encodeQmmF32(ctx, enc, x:, xOffset:, y:, rows:, accumulate:, halfOut:)
  * (Sources/Ingot/Layers/Linear.swift:688-713) and qmm_t_nax3* (Shaders/qmm_nax_v3.metal:107-256).
  * Requires rows % 64 == 0 and n % 64 == 0 like the reference (Linear.swift:695), k % 64 == 0.
  * x of dtype bf16/f32 is converted to fp16 into the workspace first; fp16 x is used in place. */
@@ -288,8 +288,8 @@ int32_t iq_moe_experts(iq_moe* layer, void* stream, const void* rows_f16, int32_
                        const uint32_t* counts, int32_t sources, int32_t region_rows, void* yd, int32_t yd_dtype,
                        void* const* yd_rows, void* workspace, size_t workspace_bytes);
 /* The same for rows left where they arrived: row i of the expert-major order (sum(counts) rows, experts ascending) is
- * row row_index[i] of rows_f16 (device array of max_rows entries, e.g. from iq_ep_index); the kernels fetch the rows
- * through the index, so nothing is gathered first. counts: device uint32 [experts] (one source). */
+ * row row_index[i] of rows_f16 (device array of max_rows entries, e.g. from iq_ep_index); the int8 kernels (few
+ * rows per expert) fetch the rows through the index, for the GEMM they are gathered into the workspace first. counts: device uint32 [experts] (one source). */
 int32_t iq_moe_experts_indexed(iq_moe* layer, void* stream, const void* rows_f16, const uint32_t* row_index, int32_t total_rows,
                                int32_t max_rows, const uint32_t* counts, void* yd, int32_t yd_dtype, void* const* yd_rows,
                                void* workspace, size_t workspace_bytes);
@@ -306,8 +306,9 @@ int32_t iq_moe_combine_rows(iq_moe* layer, void* stream, const void* yd_rows, in
  *   iq_moe_forward(ROUTER|ROUTE|GROUP); iq_ep_pack_push; iq_ep_barrier(then_plan = 1);
  *   iq_moe_experts(recv, counts = own counts matrix, region_rows); iq_ep_return_push; iq_ep_barrier(0);
  *   (or, faster: iq_ep_index, then iq_moe_experts_indexed(recv, row_index, merged counts, yd_rows = table), and no
- *   iq_ep_return_push: the experts fetch the rows through the index and their outputs go from yd straight into the
- *   sources' return buffers through the table; iq_ep_compact gathers the rows first instead)
+ *   iq_ep_return_push: the experts take the rows through the index (the int8 kernels of few rows directly, the GEMM after
+ *   gathering them) and their outputs go from yd straight into the sources' return buffers through the table;
+ *   iq_ep_compact gathers the rows before that call instead)
  *   iq_moe_combine_rows(back).
  * Rows move with plain 16-byte peer stores (no TMA, no multicast). Every rank must run the same sequence; the barrier's
  * wait is bounded (IQ_ERR_TIMEOUT in iq_ctx_status when a peer never arrives). At most 8 ranks. */
@@ -341,7 +342,7 @@ int32_t iq_ep_compact(iq_ep* ep, void* stream, const void* recv_rows, int32_t d_
                       void** table, const uint32_t** merged_counts);
 /* The same order without moving the rows: row_index[i] = the receive-buffer row at position i of the expert-major order
  * (device array of world * region_rows entries), table and merged_counts as in iq_ep_compact; for
- * iq_moe_experts_indexed(recv, row_index, ...). Faster: the rows are read once, by the experts' kernels. */
+ * iq_moe_experts_indexed(recv, row_index, ...), whose int8 kernels (few rows per expert) read the rows in place. */
 int32_t iq_ep_index(iq_ep* ep, void* stream, int32_t d_model, int32_t yd_dtype, uint32_t* row_index, void** table,
                     const uint32_t** merged_counts);
 /* The dispatch with every token row sent once per destination rank, however many of its experts live there (top-8

@@ -162,19 +162,6 @@ __device__ __forceinline__ uint4 ldg_nc_u4(const void* p) {
 
 __device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) { return __ldg(static_cast<const unsigned short*>(p)); }
 
-// Prefetching variants: volatile, so the compiler keeps them where they are written (ahead of a barrier wait) instead
-// of sinking them to the first use.
-__device__ __forceinline__ uint32_t ldg_nc_u16_early(const void* p) {
-    unsigned short r;
-    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(r) : "l"(p));
-    return r;
-}
-__device__ __forceinline__ uint32_t ldg_nc_u8_early(const void* p) {
-    uint32_t r;
-    asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(r) : "l"(p));
-    return r;
-}
-
 __device__ __forceinline__ uint32_t ldg_nc_u8(const void* p) { return __ldg(static_cast<const unsigned char*>(p)); }
 
 }  // namespace iq

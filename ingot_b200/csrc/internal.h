@@ -52,7 +52,6 @@ constexpr int kQmvTailBlocks = 64;        // ... over at most this many 16-row b
 int32_t fail(iq_ctx* ctx, int32_t code, const char* fmt, ...);
 int32_t check_cuda(iq_ctx* ctx, cudaError_t e, const char* what);
 
-inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 inline size_t round_up_sz(size_t v, size_t m) { return (v + m - 1) / m * m; }
 inline int dtype_size(int32_t dt) { return dt == kF32 ? 4 : 2; }

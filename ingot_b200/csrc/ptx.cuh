@@ -79,21 +79,6 @@ __device__ __forceinline__ bool mbar_wait_hint(uint32_t hint, uint32_t bar, uint
         }
     }
 }
-// The same wait for roles that are far from the critical path (a whole main loop away): sleeps between polls so that
-// the polling does not take issue slots from the warps doing the work.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (true) {
-        __nanosleep(200);
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if ((unsigned long long)(clock64() - t0) > kWaitCycles) {
-            *abort_flag = 1;
-            return false;
-        }
-    }
-}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -153,9 +138,6 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 r;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a));
     return r;
-}
-__device__ __forceinline__ void sts128(uint32_t a, const uint4& v) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
     uint32_t r;

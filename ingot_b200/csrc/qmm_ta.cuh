@@ -257,9 +257,11 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // The weights do not depend on the previous kernel of the stream: with dense tiling, or behind a launch over the same tile
-    // list (p.early: that one lets its dependents start after its own wait, so the list is complete), their producers and
-    // the dequantisers start at once; a tile list, the activations and y do.
+    // The weights do not depend on the previous kernel of the stream, a tile list, the activations and y do. With dense tiling the
+    // weights' producers and the dequantisers start at once. With p.early as well: the tile list is complete then, because the
+    // first kernel of the chain (packing, gate/up, down) waited in every thread before it let the next one start. An early kernel
+    // of the chain lets its own successor start without having waited; that one may read the list on the strength of the first
+    // kernel's wait alone, and nothing else of what its predecessors wrote before its own.
     if (p.tiles == nullptr) pdl_launch_dependents();
     if ((p.tiles != nullptr && !p.early) || !(warp == 2 || warp == 3 || warp >= 8)) pdl_wait();
     if (p.tiles != nullptr) pdl_launch_dependents();

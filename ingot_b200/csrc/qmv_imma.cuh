@@ -1,5 +1,6 @@
 // Decode GEMV on the int8 tensor-core path: y[m, n] = sum_k x[m, k] * (s[n, g] * q[n, k] + b[n, g]) for up to eight
-// activation rows per launch (the host cuts 9..16 rows into two launches) and affine 4-, 6- or 8-bit weights.
+// activation rows per launch and affine 4-, 6- or 8-bit weights. Nine to sixteen rows go to the ring kernel (qmv_ring.cuh), which
+// reads the weights once and gives the same bits, or, at 6 bits and where blocks are left over, as two launches.
 //
 // Why integers. The fp16 formulation converts every code to a half (several ALU instructions per code) before the MMA
 // and ends up bound by instruction issue at a third of the memory roofline. Here the codes go into the MMA as they
@@ -22,7 +23,7 @@
 //
 // Same operator as the reference's vnax_qmv* kernels (Shaders/verify_nax.metal:105-230); taken when K is a multiple
 // of 2048 and the activations of eight rows plus two stages fit shared memory (a choice that does not look at the row
-// count), the fp16 kernels serve the rest.
+// count); the ring kernel serves the rest, the register-staged fp16 kernel (gqmv.cuh) what is too wide for both.
 #pragma once
 
 #include "common.cuh"
@@ -86,11 +87,6 @@ __device__ __forceinline__ uint4 lds128_after(uint32_t addr, uint32_t token) {
 __device__ __forceinline__ uint32_t lds32_after(uint32_t addr, uint32_t token) {
     uint32_t v;
     asm("ld.shared.u32 %0, [%1]; // %2" : "=r"(v) : "r"(addr), "r"(token));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds_u16_after(uint32_t addr, uint32_t token) {
-    uint32_t v;
-    asm("ld.shared.u16 %0, [%1]; // %2" : "=r"(v) : "r"(addr), "r"(token));
     return v;
 }
 __device__ __forceinline__ float2 lds64f_after(uint32_t addr, uint32_t token) {

@@ -5,7 +5,7 @@
 //
 // Replaces, on sm_100a, had_rows_h, embed_rows_t and vnax_qmvt* of the reference (Shaders/xc_tern.metal:29-65, 110-230;
 // launcher Layers/Linear.swift:298-349). The prefill GEMM of the format is the tcgen05 kernel with a ternary
-// dequantiser (csrc/qmm_tc.cuh). The kernels here are small: a 4096 x 4096 ternary matrix is 4 MB.
+// dequantiser (csrc/qmm_ta.cuh). The kernels here are small: a 4096 x 4096 ternary matrix is 4 MB.
 #include "common.cuh"
 #include "internal.h"
 #include "ptx.cuh"
