@@ -486,7 +486,9 @@ extern "C" int32_t iq_dense_ffn_workspace_bytes(iq_ctx* ctx, const iq_qlinear* g
         size_t q = 0;
         int32_t st = iq_qmm_workspace_bytes(ctx, gate_up, rows, x_dtype, &q);
         if (st != kOk) return st;
-        total += round_up_sz((size_t)rows * 2 * d_ff * 4, 256) + round_up_sz(q, 256);  // gate|up fp32 + qmm scratch
+        total += round_up_sz(q, 256);  // qmm scratch
+        const int32_t fmt = format_of(gate_up);
+        if (fmt == kFmtTernary || fmt == kFmtAffine6) total += round_up_sz((size_t)rows * 2 * d_ff * 4, 256);  // gate|up fp32 (no fused form)
     }
     *bytes = total;
     return kOk;
