@@ -108,7 +108,7 @@ class ExpertParallelMoE:
             merged = dx.compact(b["xc_dx"], b["rows_dx"])
             L.experts(b["xc_dx"], min(rows * k, dx.max_rows), merged, 1, b["yd_dx"], b["ws_dx"], yd_rows=b["rows_dx"])
         elif dx.fused_return:
-            # the same order as an index into the receive buffer: the experts' kernels fetch the rows themselves
+            # the same order as an index into the receive buffer: the experts' call takes the rows through it
             merged = (dx.index_tokens if by_token else dx.index)(b["index_dx"], b["rows_dx"])
             L.experts_indexed(dx.recv, b["index_dx"], min(rows * k, dx.max_rows), merged, b["yd_dx"], b["ws_dx"],
                               yd_rows=b["rows_dx"])
