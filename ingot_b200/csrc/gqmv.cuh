@@ -13,8 +13,8 @@
 // fixed warp order, which makes a row's bits independent of the other rows (the reference's row-invariance property,
 // Tests/IngotTests/KernelCaseTests.swift:68-86).
 //
-// Runs where the inputs are too wide for the other kernels of the family (8 bits: beyond some 24,000, 4 bits 32,000; MXFP4: where 16
-// rows of weights exceed 80 KB, 9,600, or sixteen rows of activations leave no room for two such stages) and where scales are not
+// Runs where the inputs are too wide for the other kernels of the family (8 bits: beyond some 24,000, 4 bits 32,000; MXFP4: beyond
+// 9,600, where 16 rows of weights exceed 80 KB) and where scales are not
 // aligned for them. Replaces the reference's decode kernels vnax_qmv_nf1_sg32 / fn_qmv8_nf1 / vqmv_* (Shaders/verify_nax.metal:105-209, Shaders/verify.metal:89-155).
 #pragma once
 

@@ -568,21 +568,22 @@ int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     const int ck = c.fmt == kFmtAffine8 ? 16 : 32;  // inputs per 16-byte chunk
     const int mh = c.max_rows > 8 ? 2 : 1;
     const int nw = c.mode == kModeGateUp ? 2 : 1;
-    // K tile: everything at once when the staged activations fit, else the largest multiple of 1024 that does
+    // K tile: everything at once when the staged activations of sixteen rows fit, else the largest multiple of 1024 that does
+    // (whatever the rows of this call: the tiles, and the slices inside them, set the order of a row's sums)
     int kt = c.K;
-    auto smem_for = [&](int ktile, int* xs_bytes) {
+    auto smem_for = [&](int ktile, int rows, int* xs_bytes) {
         const int nsteps = (ktile / ck + 3) / 4;
         const int qu = ck == 32 ? 4 : 2;
-        *xs_bytes = nsteps * qu * c.max_rows * 4 * 16;
-        const int red_bytes = 8 * nw * mh * 4 * 32 * 4;
+        *xs_bytes = nsteps * qu * rows * 4 * 16;
+        const int red_bytes = 8 * nw * (rows > 8 ? 2 : 1) * 4 * 32 * 4;
         return *xs_bytes + red_bytes;
     };
     int xs_bytes;
-    while (smem_for(kt, &xs_bytes) > kSmemBudget) {
+    while (smem_for(kt, 16, &xs_bytes) > kSmemBudget) {
         kt = kt > 1024 ? (kt - 1) / 1024 * 1024 : 0;
         if (kt == 0) return fail(ctx, kErrInvalidArg, "qmv: activations do not fit shared memory");
     }
-    const int smem = smem_for(kt, &xs_bytes);
+    const int smem = smem_for(kt, c.max_rows, &xs_bytes);
 
     // K slices per CTA: the fewest that still fill the GPU, keeping at least two steps per warp
     const int nsteps = (kt / ck + 3) / 4;

@@ -276,7 +276,7 @@ def test_qmv_ring_keeps_16_bit_activations_whole(cuda_device, N, K, rows, group,
         assert np.abs(y.double().cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
-@pytest.mark.parametrize("fmt,N,K", [("q4", 48, 40960), ("q8", 48, 28672), ("g32", 48, 40960), ("mxfp4", 48, 14336), ("q4", 16, 65600)])
+@pytest.mark.parametrize("fmt,N,K", [("q4", 48, 40960), ("q8", 48, 28672), ("g32", 48, 40960), ("mxfp4", 48, 14336), ("q4", 16, 65600), ("g32", 1024, 36928)])
 def test_qmv_inputs_too_wide_for_the_other_kernels(cuda_device, fmt, N, K):
     """The register-staged fp16 kernel, K walked in tiles that fit shared memory: against the oracle, and the same bits for a row
     alone, among 8 and among 16."""
