@@ -96,6 +96,18 @@ int32_t launch_qmv_stream(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
         ctas_per_sm = 2;
         nstages = (kQsSmemMax / 2 - 1024 - fixed) / stage_bytes;
     }
+    if (nstages < 2 && c.rows > 1) {
+        // the rows' activations leave no room for two stages: two launches of half the rows, so that a row stays on this kernel
+        // (and keeps its bits) whatever the rows of the call
+        GqmvCall half = c;
+        half.rows = half.max_rows = c.rows / 2;
+        const int32_t r = launch_qmv_stream(ctx, st, half);
+        if (r != kOk) return r;
+        half.x = static_cast<const char*>(c.x) + (size_t)half.rows * c.ldx * dtype_size(c.x_dtype);
+        half.y = static_cast<char*>(c.y) + (size_t)half.rows * c.ldy * dtype_size(c.y_dtype);
+        half.rows = half.max_rows = c.rows - half.rows;
+        return launch_qmv_stream(ctx, st, half);
+    }
     if (nstages < 2) return 1;
     if (nstages > 8) nstages = 8;
 

@@ -290,3 +290,18 @@ def test_qmv_inputs_too_wide_for_the_other_kernels(cuda_device, fmt, N, K):
     for rows in (1, 8, 9):
         assert torch.equal(run(m, xt[:rows].contiguous(), rows), full[:rows]), rows
     assert torch.equal(run(m, xt[11:12].contiguous(), 1)[0], full[11])
+
+
+@pytest.mark.parametrize("N,K", [(96, 2880), (208, 5760), (64, 7168), (48, 9600)])
+def test_qmv_mxfp4_row_invariance(cuda_device, N, K):
+    """A row has the same bits alone and among others, also where the activations of all of them leave no room for the weights'
+    stages and the call is cut (5760 inputs: sixteen rows; 9600: more than a few). Among eight and among nine the MMAs differ."""
+    rng = np.random.default_rng(910 + N + K)
+    m, host = mxfp4_case(rng, N, K, cuda_device)
+    x = synth.activations_np(rng, 16, K)
+    xt = x_tensor(x, cuda_device)
+    full = run(m, xt, 16)
+    assert qref.max_rel(full.cpu().numpy(), qref.matmul_t(x, deq(host))) <= TOL
+    for rows in (1, 5, 8, 9, 13):
+        assert torch.equal(run(m, xt[:rows].contiguous(), rows), full[:rows]), rows
+    assert torch.equal(run(m, xt[11:12].contiguous(), 1)[0], full[11])
