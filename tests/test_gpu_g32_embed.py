@@ -260,12 +260,13 @@ def test_dense_ffn_refuses_an_unaligned_workspace(cuda_device, rows):
 
 @pytest.mark.parametrize("bits,group", [(4, 64), (8, 64), (4, 32)])
 def test_dense_ffn_inputs_too_wide_for_the_other_kernels(cuda_device, bits, group):
-    """Gate + up + activation on the register-staged fp16 kernel."""
+    """Gate + up + activation on the register-staged fp16 kernel. (Activations of 1/16: 8-bit weights have a deviation of 0.9, 40960 of
+    them against N(0, 1) give gates of 180 and products of their squares, beyond half's 65504; so they stay below 700.)"""
     rng = np.random.default_rng(75 + bits + group)
     D, F, rows = 40960, 64, 9
     gu, hgu = affine_case(rng, 2 * F, D, bits, cuda_device, group=group)
     dn, hdn = affine_case(rng, D, F, bits, cuda_device, group=group)
-    xh = synth.activations_np(rng, rows, D)
+    xh = synth.activations_np(rng, rows, D) / 16
     wgu = deq(hgu, bits, group=group)
     h = qref.round_f16(qref.silu_glu(qref.matmul_t(xh, wgu[:F]), qref.matmul_t(xh, wgu[F:])))
     ref = qref.matmul_t(h, deq(hdn, bits, group=group))
