@@ -24,9 +24,12 @@ def _dtype_id(t: torch.Tensor) -> int:
     return _DT[t.dtype]
 
 
+# the current stream of the current device, without building a Stream object around it (absent where torch has no CUDA)
+_device, _raw_stream = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> int:
-    # the current stream of the current device, without building a Stream object around it
-    return stream.cuda_stream if stream is not None else torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return stream.cuda_stream if stream is not None else _raw_stream(_device())
 
 
 def _no_cpu():
@@ -102,8 +105,8 @@ class DenseQ:
         return {k: v for k, v in self.__dict__.items() if k not in ("_ql", "_generation")}
 
     def _described(self) -> tuple:
-        """(address of the matrix's C description, the description, its generation, its three pointers, the context of its device),
-        built once: a decode step passes the same matrices over and over. The caller holds the tuple over its call: the
+        """(address of the matrix's C description, the description, its generation, its three pointers, the context of its device,
+        the C entry points), built once: a decode step passes the same matrices over and over. The caller holds the tuple over its call: the
         address is good as long as somebody holds the description, and another thread may assign to the matrix while a launch
         runs without the interpreter lock. One attribute for all of it: a thread that finds it finds a whole description."""
         d, generation, s, b = self._ql, self._generation, self.s, self.b
@@ -111,7 +114,8 @@ class DenseQ:
         # (the storages may have been exchanged under the tensors)
         if d is None or d[2] is not generation or d[3] != w or d[4] != s or d[5] != b or d[6].address == 0:
             q = self.qlinear()
-            d = self._ql = (C.addressof(q), q, generation, q.w or 0, q.scales or 0, q.biases or 0, capi.context(self.device_index))
+            d = self._ql = (C.addressof(q), q, generation, q.w or 0, q.scales or 0, q.biases or 0, capi.context(self.device_index),
+                            capi.call())
         return d
 
     def qlinear(self) -> capi.QLinear:
@@ -141,8 +145,9 @@ class DenseQ:
         """x[rows, K] rotated into a float16 scratch (grown on demand, like the reference's rotation buffer)."""
         if self._rot is None or self._rot.shape[0] < rows:
             self._rot = torch.empty(max(rows, 16), self.K, dtype=torch.float16, device=self.w.device)
-        ctx = self._described()[6]
-        ctx.check(capi.call().had_rows(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
+        d = self._described()
+        ctx = d[6]
+        ctx.check(d[7].had_rows(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
                                        self.had.data_ptr(), self._rot.data_ptr(), self.K, rows, self.K))
         return self._rot
 
@@ -171,7 +176,7 @@ class DenseQ:
                                                        tok.data_ptr(), rows, 0 if out_f is None else out_f.data_ptr(),
                                                        0 if out_h is None else out_h.data_ptr(), o.stride(0)))
             return
-        ctx.check(capi.call().embed_rows(ctx.address, _stream_ptr(stream), d[0], tok.data_ptr(), rows,
+        ctx.check(d[7].embed_rows(ctx.address, _stream_ptr(stream), d[0], tok.data_ptr(), rows,
                                          0 if out_f is None else out_f.data_ptr(),
                                          0 if out_h is None else out_h.data_ptr(), o.stride(0)))
 
@@ -194,7 +199,7 @@ class DenseQ:
         if self.had is not None:  # rotated basis: the rotation runs first, as in the reference's launcher
             x = self.encode_rotate(x, rows, stream)
         ws_ptr, ws_bytes = (0, 0) if workspace is None else (workspace.data_ptr(), workspace.numel() * workspace.element_size())
-        st = capi.call().qmm(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0), d[0], y.data_ptr(),
+        st = d[7].qmm(ctx.address, stream.cuda_stream if stream is not None else _raw_stream(_device()), x.data_ptr(), _dtype_id(x), x.stride(0), d[0], y.data_ptr(),
                              _dtype_id(y), y.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, ws_ptr, ws_bytes)
         if st:
             ctx.check(st)
@@ -260,7 +265,7 @@ class VQMV:
             ldx = x.stride(0) if x.dim() > 1 else m.K
         if ldy is None:
             ldy = y.stride(0) if y.dim() > 1 else m.N
-        st = capi.call().qmv(ctx.address, _stream_ptr(stream), x.data_ptr(), _DT.get(x.dtype, -1), ldx, d[0], y.data_ptr(),
+        st = d[7].qmv(ctx.address, stream.cuda_stream if stream is not None else _raw_stream(_device()), x.data_ptr(), _DT.get(x.dtype, -1), ldx, d[0], y.data_ptr(),
                              _DT.get(y.dtype, -1), ldy, rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0, n_prefix or 0)
         if st:
             _dtype_id(x), _dtype_id(y)  # a type the library does not know is a TypeError
@@ -301,7 +306,7 @@ class DenseMLP:
         a, b = self.gate_up._described(), self.down._described()
         ctx = a[6]
         ws = self._workspace(ctx, rows, x.dtype)
-        ctx.check(capi.call().dense_ffn(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
+        ctx.check(a[7].dense_ffn(ctx.address, _stream_ptr(stream), x.data_ptr(), _dtype_id(x), x.stride(0),
                                         a[0], b[0], self.act, self.limit, out.data_ptr(),
                                         _dtype_id(out), out.stride(0), rows, capi.IQ_FLAG_ACCUMULATE if accumulate else 0,
                                         ws.data_ptr(), ws.numel()))
