@@ -360,15 +360,19 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                             cp_async_ca<SPB>(dst + t * 128 * SPB + (lane + 32 * i) * SPB, src[i][t] + ch * SPB);
                 } else {
                     uint32_t v[4][NT][SPB / 2];
+                    auto load = [&](auto bytes) {  // (the choice outside: the loads of a stage go out together)
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
+                        for (int i = 0; i < 4; i++)
 #pragma unroll
-                        for (int t = 0; t < NT; t++)
+                            for (int t = 0; t < NT; t++)
 #pragma unroll
-                            for (int e = 0; e < SPB / 2; e++) {
-                                const char* a = src[i][t] + ch * SPB + min(2 * e, left - 2);
-                                v[i][t][e] = FMT == kFmtMxfp4 && p.vec < 0 ? ldg_nc_u8(a) | (ldg_nc_u8(a + 1) << 8) : ldg_nc_u16(a);
-                            }
+                                for (int e = 0; e < SPB / 2; e++) {
+                                    const char* a = src[i][t] + ch * SPB + min(2 * e, left - 2);
+                                    v[i][t][e] = decltype(bytes)::value ? ldg_nc_u8(a) | (ldg_nc_u8(a + 1) << 8) : ldg_nc_u16(a);
+                                }
+                    };
+                    if (FMT == kFmtMxfp4 && p.vec < 0) load(std::true_type{});
+                    else load(std::false_type{});
 #pragma unroll
                     for (int i = 0; i < 4; i++)
 #pragma unroll
