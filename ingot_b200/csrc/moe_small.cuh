@@ -1,5 +1,5 @@
 // The MoE block for up to three tokens in three kernels, where a decode step of few tokens is a chain of latencies and not
-// of bytes (one token of the 128-expert layer reads 21 MB, 3 us, and took 59 us in eight kernels, 25 in three; three tokens
+// of bytes (one token of the 128-expert layer reads 21 MB, 3 us, and took 59 us in eight kernels, 26 in three; three tokens
 // 52 us against 57. From four on, 67 against 61, the separate kernels, which stage the weights, win):
 //
 //   moe_route_small_kernel   router logits, top-k and the permutation in one cluster of eight blocks; also the activations as
