@@ -124,7 +124,10 @@ int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_
  * both in tensor memory). Replaces DenseQ.encodeQmmF32(ctx, enc, x:, xOffset:, y:, rows:, accumulate:, halfOut:)
  * (Sources/Ingot/Layers/Linear.swift:688-713) and qmm_t_nax3* (Shaders/qmm_nax_v3.metal:107-256).
  * Requires rows % 64 == 0 and n % 64 == 0 like the reference (Linear.swift:695), k % 64 == 0.
- * x of dtype bf16/f32 is converted to fp16 into the workspace first; fp16 x is used in place. */
+ * x of dtype bf16/f32 is converted to fp16 into the workspace first; fp16 x is used in place. Where the tiles fill the GPU's SMs
+ * badly, some are divided along k and their partial sums go through the workspace, behind the converted rows (round(rows * k * 2,
+ * 256) bytes, none for fp16): iq_qmm_workspace_bytes asks for both, and a workspace that holds the converted rows only is
+ * accepted as well (the same products, summed in another order). */
 int32_t iq_qmm_workspace_bytes(iq_ctx* ctx, const iq_qlinear* m, int32_t rows, int32_t x_dtype, size_t* bytes);
 int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
                int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, void* workspace, size_t workspace_bytes);
@@ -133,8 +136,8 @@ int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_
  * ordinary Metal buffers made at construction). Meant for hosts where cudaMalloc is off limits at the call site: a
  * plugin inside an engine whose pool owns all device memory, a path that runs after the pool is sealed, a sandbox or
  * real-time loop with a "no allocation" rule. Same operation and results as iq_qmm, but the fp16 copy of bf16/fp32
- * activations goes to an 8 MiB array built into the library (held by every GPU that loads it until the process
- * exits) instead of a caller workspace. Limits and rules:
+ * activations goes to an array built into the library (8 MiB, and 40 MiB for partial sums, held by every GPU that loads it
+ * until the process exits) instead of a caller workspace. Limits and rules:
  *   - rows * k <= 4,194,304 (8 MiB of fp16); larger calls return IQ_ERR_WORKSPACE and should use iq_qmm;
  *   - the first call on a device looks up the array's device address (cudaGetSymbolAddress) with that device current;
  *     make that first call outside any stream capture;

@@ -130,6 +130,22 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
 // Whether its gate/up form takes the token rows as fixed point (GqmvCall::fx) for K inputs; for others it converts them itself
 bool qmv_grouped_takes_fixed(const iq_ctx* ctx, int K);
 
+// Scratch of the GEMM's K split (csrc/qmm_ta.cuh). bytes: what the split of a dense GEMM takes (0: it is not split); part: null where
+// the scratch does not hold that.
+struct QmmSplit {
+    float* part = nullptr;
+    size_t bytes = 0;
+};
+QmmSplit qmm_split(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K, void* scratch, size_t bytes);
+size_t qmm_split_max_bytes(iq_ctx* ctx);  // of any dense GEMM
+int32_t launch_convert_x(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, void* out, int rows, int k);
+size_t qmm_convert_bytes(int rows, int k, int32_t x_dtype);
+// iq_qmm's preconditions, and its GEMM on fp16 rows
+int32_t qmm_check(iq_ctx* ctx, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, const void* y, int32_t y_dtype, int64_t ldy,
+                  int32_t rows);
+int32_t qmm_f16(iq_ctx* ctx, cudaStream_t st, const void* x, int64_t ldx, const iq_qlinear* m, void* y, int32_t y_dtype, int64_t ldy, int32_t rows,
+                uint32_t flags, const QmmSplit& split);
+
 // One launch of the tensor-core GEMM (csrc/qmm.cu). x16: fp16 activations [x_rows, ldx] (bf16 with the plain bf16 format); w[i]: stacked
 // [experts * N, K] codes (w[1]: the up matrix of the gate/up epilogue). tiles == nullptr: dense tiling over M x N.
 struct QmmCall {
@@ -156,6 +172,7 @@ struct QmmCall {
     const float* ebias[2] = {nullptr, nullptr};
     float limit = 0.f;
     int32_t act = 0;  // gate/up epilogue: activation (kAct*)
+    QmmSplit split;   // quantized formats: scratch of the K split, or none
 };
 int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c);
 int32_t launch_tern_qmv(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,

@@ -44,6 +44,7 @@ struct MoeWs {
     __half* s_h;
     void* s_yd;
     float* s_w;
+    QmmSplit split;  // what the workspace holds beyond `bytes`: partial sums of the shared expert's GEMMs
     size_t bytes;
 };
 
@@ -245,7 +246,7 @@ int tensor_tile_rows(int64_t rows, int64_t expert_slots) {
 
 // rows16: fp16 rows [n_rows, d_model] in tile order
 int32_t run_gateup_tc(iq_moe* l, cudaStream_t cs, const __half* rows16, int64_t n_rows, const Tile* tiles,
-                      const uint32_t* ntiles, __half* h, int bn, bool early = false) {
+                      const uint32_t* ntiles, __half* h, int bn, bool early = false, const QmmSplit& split = QmmSplit()) {
     const iq_moe_desc& d = l->d;
     QmmCall c;
     c.fmt = l->fmt; c.epi = 1; c.bn = bn;
@@ -259,13 +260,14 @@ int32_t run_gateup_tc(iq_moe* l, cudaStream_t cs, const __half* rows16, int64_t 
     c.y = h; c.y_dtype = kF16; c.ldy = d.d_ff;
     c.ebias[0] = d.gate_bias; c.ebias[1] = d.up_bias;
     c.early = early;
+    c.split = split;
     c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
     c.act = d.act;
     return launch_qmm(l->ctx, cs, c);
 }
 
 int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows, const Tile* tiles, const uint32_t* ntiles,
-                    void* yd, int32_t yd_dtype, int bn, bool early = false) {
+                    void* yd, int32_t yd_dtype, int bn, bool early = false, const QmmSplit& split = QmmSplit()) {
     const iq_moe_desc& d = l->d;
     QmmCall c;
     c.fmt = l->fmt; c.epi = 0; c.bn = bn;
@@ -277,6 +279,7 @@ int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows,
     c.y = yd; c.y_dtype = yd_dtype; c.ldy = d.d_model;
     c.ebias[0] = d.down_bias;
     c.early = early;
+    c.split = split;
     return launch_qmm(l->ctx, cs, c);
 }
 
@@ -416,11 +419,11 @@ int32_t run_shared_expert(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_d
         q.y = w.s_yd; q.y_dtype = ydt; q.ldy = d.d_model;
         st = launch_gqmv(ctx, cs, q);
     } else {  // ... or on the GEMM
-        const size_t units = (size_t)tokens * d.d_model / 8;
-        rows_to_f16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, cs>>>(x, x_dtype, ldx, w.s_x16, tokens, d.d_model);
-        st = check_cuda(ctx, cudaGetLastError(), "rows_to_f16 launch");
-        if (st == kOk) st = run_gateup_tc(&tmp, cs, w.s_x16, tokens, nullptr, nullptr, w.s_h, 0);
-        if (st == kOk) st = run_down_tc(&tmp, cs, w.s_h, tokens, nullptr, nullptr, w.s_yd, ydt, 0);
+        const QmmSplit gu = qmm_split(ctx, kFmtAffine4, 1, tokens, d.shared_up.n, d.d_model, w.split.part, w.split.bytes);
+        const QmmSplit dn = qmm_split(ctx, kFmtAffine4, 0, tokens, d.d_model, d.shared_up.n, w.split.part, w.split.bytes);
+        st = launch_convert_x(ctx, cs, x, x_dtype, ldx, w.s_x16, tokens, d.d_model);
+        if (st == kOk) st = run_gateup_tc(&tmp, cs, w.s_x16, tokens, nullptr, nullptr, w.s_h, 0, false, gu);
+        if (st == kOk) st = run_down_tc(&tmp, cs, w.s_h, tokens, nullptr, nullptr, w.s_yd, ydt, 0, false, dn);
     }
     if (st != kOk) return st;
     shared_add_kernel<<<tokens, 256, 0, cs>>>(w.s_yd, ydt, w.s_w, out, out_dtype, ldo, tokens, d.d_model);
@@ -472,25 +475,38 @@ using namespace iq;
 // ---------------------------------------------------------------------------------------------------------------------
 // dense FFN
 
+namespace {
+// Scratch of the GEMM path: h fp16 | converted x | (ternary: gate|up fp32) | partial sums of the GEMMs' K splits
+struct FfnWs {
+    size_t convert, need, bytes;  // offset of the converted x; without the partial sums (their offset); with them
+};
+FfnWs ffn_ws(iq_ctx* ctx, const iq_qlinear* gate_up, const iq_qlinear* down, int rows, int32_t x_dtype) {
+    FfnWs w;
+    const int32_t fmt = format_of(gate_up);
+    const size_t d_ff = down->k;
+    w.convert = round_up_sz((size_t)rows * d_ff * 2, 256);
+    w.need = w.convert + round_up_sz(qmm_convert_bytes(rows, gate_up->k, x_dtype), 256);
+    const bool fused = fmt != kFmtTernary && fmt != kFmtAffine6;
+    if (!fused) w.need += round_up_sz((size_t)rows * 2 * d_ff * 4, 256);
+    w.bytes = w.need + std::max(qmm_split(ctx, fmt, fused, rows, fused ? (int)d_ff : gate_up->n, gate_up->k, nullptr, 0).bytes,
+                                qmm_split(ctx, format_of(down), 0, rows, down->n, down->k, nullptr, 0).bytes);
+    return w;
+}
+}  // namespace
+
 extern "C" int32_t iq_dense_ffn_workspace_bytes(iq_ctx* ctx, const iq_qlinear* gate_up, const iq_qlinear* down,
                                                 int32_t rows, int32_t x_dtype, size_t* bytes) {
     if (ctx == nullptr || gate_up == nullptr || down == nullptr || bytes == nullptr) return kErrInvalidArg;
     if (gate_up->n % 2 != 0 || gate_up->n / 2 != down->k || gate_up->k != down->n)
         return fail(ctx, kErrInvalidArg, "dense_ffn: gate|up [%d, %d] and down [%d, %d] do not chain", gate_up->n,
                     gate_up->k, down->n, down->k);
-    const size_t d_ff = down->k;
-    size_t total = round_up_sz((size_t)rows * d_ff * 2, 256);  // h fp16
     if (rows <= 16) {
-        total += round_up_sz((size_t)rows * std::max(d_ff, (size_t)gate_up->k) / 2 * 7, 256);  // x, then h, as block fixed point
+        const size_t d_ff = down->k;
+        *bytes = round_up_sz((size_t)rows * d_ff * 2, 256) +                                     // h fp16
+                 round_up_sz((size_t)rows * std::max(d_ff, (size_t)gate_up->k) / 2 * 7, 256);  // x, then h, as block fixed point
     } else {
-        size_t q = 0;
-        int32_t st = iq_qmm_workspace_bytes(ctx, gate_up, rows, x_dtype, &q);
-        if (st != kOk) return st;
-        total += round_up_sz(q, 256);  // qmm scratch
-        const int32_t fmt = format_of(gate_up);
-        if (fmt == kFmtTernary || fmt == kFmtAffine6) total += round_up_sz((size_t)rows * 2 * d_ff * 4, 256);  // gate|up fp32 (no fused form)
+        *bytes = ffn_ws(ctx, gate_up, down, rows, x_dtype).bytes;
     }
-    *bytes = total;
     return kOk;
 }
 
@@ -501,6 +517,11 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
     size_t need = 0;
     int32_t st = iq_dense_ffn_workspace_bytes(ctx, gate_up, down, rows, x_dtype, &need);
     if (st != kOk) return st;
+    FfnWs ws = {};
+    if (rows > 16) {
+        ws = ffn_ws(ctx, gate_up, down, rows, x_dtype);
+        need = ws.need;  // (a workspace without room for the K splits is good as well: every tile is one item then)
+    }
     if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0)
         return fail(ctx, kErrWorkspace, "dense_ffn: workspace %zu < %zu (16-byte aligned)", workspace_bytes, need);
     if (act < IQ_ACT_SILU || act > IQ_ACT_RELU2) return fail(ctx, kErrUnsupported, "dense_ffn: activation %d", act);
@@ -544,18 +565,22 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
         // rows = 2048, d_ff = 14336 that is 235 MB not written and read back); then the down GEMM.
         if (rows % 64 != 0 || d_ff % 64 != 0 || gate_up->k % 64 != 0)
             return fail(ctx, kErrInvalidArg, "dense_ffn: rows = %d, d_ff = %d, d = %d must be multiples of 64", rows, d_ff, gate_up->k);
-        char* q = static_cast<char*>(workspace) + round_up_sz((size_t)rows * d_ff * 2, 256);
+        st = qmm_check(ctx, h, IQ_F16, d_ff, down, out, out_dtype, ldo, rows);
+        if (st != kOk) return st;
+        char* base = static_cast<char*>(workspace);
         const void* x16 = x;
         int64_t ld16 = ldx;
+        QmmSplit gu, dn;
+        if (workspace_bytes >= ws.bytes) {
+            gu = qmm_split(ctx, fmt, 1, rows, d_ff, gate_up->k, base + ws.need, ws.bytes - ws.need);
+            dn = qmm_split(ctx, format_of(down), 0, rows, down->n, down->k, base + ws.need, ws.bytes - ws.need);
+        }
         if (x_dtype != IQ_F16) {
             if (ldx < gate_up->k || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
                 return fail(ctx, kErrInvalidArg, "dense_ffn: x must be 16-byte aligned with ldx >= d and ldx %% 8 == 0");
-            const size_t units = (size_t)rows * gate_up->k / 8;
-            rows_to_f16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, cs>>>(x, x_dtype, ldx, reinterpret_cast<__half*>(q), rows,
-                                                                               gate_up->k);
-            st = check_cuda(ctx, cudaGetLastError(), "rows_to_f16 launch");
+            st = launch_convert_x(ctx, cs, x, x_dtype, ldx, base + ws.convert, rows, gate_up->k);
             if (st != kOk) return st;
-            x16 = q;
+            x16 = base + ws.convert;
             ld16 = gate_up->k;
         }
         const size_t row_words = (size_t)gate_up->k / 32 * gate_up->bits;
@@ -575,9 +600,10 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
         c.y = h; c.y_dtype = kF16; c.ldy = d_ff;
         c.limit = act == IQ_ACT_SWIGLU_OAI ? act_limit : 0.f;
         c.act = act;
+        c.split = gu;
         st = launch_qmm(ctx, cs, c);
         if (st != kOk) return st;
-        return iq_qmm(ctx, stream, h, IQ_F16, d_ff, down, out, out_dtype, ldo, rows, flags, nullptr, 0);
+        return qmm_f16(ctx, cs, h, d_ff, down, out, out_dtype, ldo, rows, flags, dn);
     }
     // ternary gate/up rows: gate|up GEMM -> activation -> down GEMM
     char* p = static_cast<char*>(workspace) + round_up_sz((size_t)rows * d_ff * 2, 256);
@@ -689,7 +715,7 @@ extern "C" void iq_moe_destroy(iq_moe* l) { delete l; }
 
 extern "C" int32_t iq_moe_workspace_bytes(const iq_moe* l, int32_t max_tokens, size_t* bytes) {
     if (l == nullptr || bytes == nullptr || max_tokens < 1) return kErrInvalidArg;
-    *bytes = carve(l, nullptr, max_tokens).bytes;
+    *bytes = carve(l, nullptr, max_tokens).bytes + (l->d.shared != IQ_SHARED_NONE && max_tokens > 16 ? qmm_split_max_bytes(l->ctx) : 0);
     return kOk;
 }
 
@@ -735,6 +761,8 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     MoeWs w = carve(l, workspace, tokens);
     if (workspace == nullptr || workspace_bytes < w.bytes)
         return fail(ctx, kErrWorkspace, "moe: workspace %zu < %zu", workspace_bytes, w.bytes);
+    w.split.part = reinterpret_cast<float*>(static_cast<char*>(workspace) + w.bytes);
+    w.split.bytes = workspace_bytes - w.bytes;
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
     const int P = tokens * d.top_k;
     const uint32_t* inds = l->ext_inds ? l->ext_inds : w.inds;

@@ -1001,19 +1001,6 @@ __global__ void __launch_bounds__(128) shared_gate_kernel(const void* __restrict
     if (lane == 0) sg[t] = w;
 }
 
-// fp16 copy of x [T, D] (rows in place), the tensor-core GEMM's operand type
-__global__ void __launch_bounds__(256) rows_to_f16_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx,
-                                                         __half* __restrict__ out, int T, int D) {
-    const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 8;
-    if (i >= (size_t)T * D) return;
-    const size_t r = i / D, c = i % D;
-    float v[8];
-    load_x8(x, x_dtype, r * ldx + c, v);
-    uint4 o;
-    o.x = pack_half2(v[0], v[1]); o.y = pack_half2(v[2], v[3]); o.z = pack_half2(v[4], v[5]); o.w = pack_half2(v[6], v[7]);
-    *reinterpret_cast<uint4*>(out + i) = o;
-}
-
 // out[t, :] += sg[t] * ys[t, :] (the shared expert's contribution)
 __global__ void __launch_bounds__(256) shared_add_kernel(const void* __restrict__ ys, int32_t ys_dtype, const float* __restrict__ sg,
                                                         void* __restrict__ out, int32_t out_dtype, int64_t ldo, int T, int D) {

@@ -1,6 +1,8 @@
 // Host side of the tcgen05 GEMM: tensor maps, kernel selection, the iq_qmm entry point.
 #include <string.h>
 
+#include <algorithm>
+
 #include "internal.h"
 #include "qmm_ta.cuh"
 #include "qmm_tc.cuh"
@@ -45,6 +47,8 @@ const KernelEntry* find(int32_t fmt, int bn) {
     return nullptr;
 }
 
+int ta_step_bytes(int32_t fmt) { return fmt == kFmtAffine8 ? 64 : (fmt == kFmtTernary ? 16 : 32); }  // code bytes of a row per K step
+
 typedef void (*TaKernel)(const TaMaps, const TaParams);
 
 // gate/up: the formats of experts and of dense FFNs
@@ -60,18 +64,38 @@ TaKernel ta_pick(int32_t fmt, int epi) {
     }
 }
 
-// Token rows per tile of a dense GEMM: the height (a multiple of 16, at most 192) with the least (waves over the SMs) x
-// (time of a tile). A K step takes the MMA 2 h + 40 cycles for h tokens, and its issue and hand-overs about 400 whatever the
-// height, so lower tiles than 176 rows only pay when they save a wave.
-int ta_tile_rows(int m, int n_tiles, int sms) {
-    int best = 16;
-    long long best_cost = -1;
-    for (int tiles = (m + kTaMaxRows - 1) / kTaMaxRows; tiles <= (m + 15) / 16; tiles++) {
-        const int h = round_up((m + tiles - 1) / tiles, 16);
-        const long long waves = ((long long)((m + h - 1) / h) * n_tiles + sms - 1) / sms;
-        const long long cost = waves * (h > 176 ? h : 176);
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = h; }
-        if (h <= 64) break;
+// Tiling of a dense GEMM: token rows per tile (a multiple of 16, at most 192), K split of the tiles beyond the whole rounds.
+struct TaPlan {
+    int rows, n_tiles, ustep, grid;
+    TaSplit split;
+    bool low;  // two CTAs per SM
+};
+int ta_xk(bool low, int rows) { return low ? (rows <= 32 ? 4 : 2) : (rows <= 128 ? 4 : 2); }  // K steps per copy of X
+int ta_ustep(int32_t fmt, int xk) { return std::max(128 / ta_step_bytes(fmt), xk); }  // whole stages of codes and of X
+
+// The height with the least time: whole rounds over the SMs, or with the split the share of the split tiles and what the split costs.
+TaPlan ta_plan(int32_t fmt, int epi, int M, int N, int K, int sms, bool may_split) {
+    TaPlan best = {};
+    double best_cost = -1;
+    const int n_tiles = (N + (epi ? 63 : 127)) / (epi ? 64 : 128), ksteps = K / 64;
+    for (int tiles = (M + kTaMaxRows - 1) / kTaMaxRows; tiles <= (M + 15) / 16; tiles++) {
+        TaPlan p;
+        p.rows = round_up((M + tiles - 1) / tiles, 16);
+        p.n_tiles = n_tiles;
+        const int total = (M + p.rows - 1) / p.rows * n_tiles;
+        // Two CTAs per SM for low tiles; with a tile per SM or less the one with four dequantiser groups (MXFP4 24576 x 2048 at 64
+        // rows 21.0 -> 18.5 us)
+        p.low = p.rows <= kTaLowRows && total > sms;
+        const int ctas = p.low ? 2 * sms : sms;
+        p.ustep = ta_ustep(fmt, ta_xk(p.low, p.rows));
+        p.split = may_split ? ta_split(total, ctas, ksteps, p.ustep, p.rows, p.low) : TaSplit{0, 0, 0};
+        const double step = ta_step_cycles(p.rows, p.low);
+        double cost = (double)((total - p.split.tiles + ctas - 1) / ctas) * ksteps * step;
+        if (p.split.tiles)
+            cost += (p.split.tiles * p.split.units + p.split.ctas - 1) / p.split.ctas * p.ustep * step + (double)ta_split_cycles(p.split, p.rows);
+        p.grid = total < ctas && p.split.tiles == 0 ? total : ctas;
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = p; }
+        if (p.rows <= 64) break;
     }
     return best;
 }
@@ -189,18 +213,27 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     if (ta_pick<kTaGroups>(c.fmt, c.epi) == nullptr) return fail(ctx, kErrNoKernel, "qmm: no kernel for format %d, epilogue %d", c.fmt, c.epi);
     TaParams p;
     memset(&p, 0, sizeof(p));
-    const int n_tiles = (c.N + (c.epi ? 63 : 127)) / (c.epi ? 64 : 128);
-    const int rows = c.tiles == nullptr ? ta_tile_rows(c.M, n_tiles, ctx->sms) : c.bn;
-    // Two CTAs per SM for low tiles; a dense matrix with a tile per SM or less keeps the one with four dequantiser groups (MXFP4
-    // 24576 x 2048 at 64 rows 21.0 -> 18.5 us)
-    const bool low = rows <= kTaLowRows && (c.tiles != nullptr || n_tiles * ((c.M + rows - 1) / rows) > ctx->sms);
+    TaPlan plan = {};
+    if (c.tiles == nullptr) {
+        plan = ta_plan(c.fmt, c.epi, c.M, c.N, c.K, ctx->sms, c.split.part != nullptr);
+    } else {
+        plan.rows = c.bn;
+        plan.low = plan.rows <= kTaLowRows;
+        plan.grid = plan.low ? 2 * ctx->sms : ctx->sms;
+        plan.ustep = ta_ustep(c.fmt, ta_xk(plan.low, plan.rows));
+    }
+    const int rows = plan.rows;
+    const bool low = plan.low;
     const TaKernel k = low ? ta_pick<kTaGroupsLow>(c.fmt, c.epi) : ta_pick<kTaGroups>(c.fmt, c.epi);
+    p.ustep = plan.ustep;
+    p.split = plan.split;
+    p.part = c.split.part;
     p.tile_rows = rows;
     // Boxes of X: dense tiles have one height; tiles of a list have up to `rows`, a box of the nearest quarter of that. Two K
     // steps per copy, four where that is still small.
     p.xbox = c.tiles == nullptr || rows <= 16 ? rows : round_up(rows / 4, 16);
     p.nbox = rows / p.xbox;
-    p.xk = low ? (rows <= 32 ? 4 : 2) : (rows <= 128 ? 4 : 2);
+    p.xk = ta_xk(low, rows);
     p.x_stage = rows * 128 * p.xk;
     p.dcols = low ? kTaLowRows : (rows <= 128 ? 128 : kTaMaxRows);
     // stages: at least three of codes, then up to eight of X, then as many of codes as fit
@@ -212,8 +245,7 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     if (p.nc > kTaMaxStages) p.nc = kTaMaxStages;
     const int smem = kTaSmemFixed + p.nx * p.x_stage + p.nc * c_stage;
 
-    const int bps = c.fmt == kFmtAffine8 ? 64 : (c.fmt == kFmtTernary ? 16 : 32);
-    const uint64_t row_bytes = (uint64_t)c.K / 64 * bps;
+    const uint64_t row_bytes = (uint64_t)c.K / 64 * ta_step_bytes(c.fmt);
     TaMaps maps;
     int32_t r = kOk;
     for (int i = 0; i < p.nbox && r == kOk; i++)
@@ -243,14 +275,9 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     p.limit = c.limit;
     p.act = c.act;
     p.status = ctx->d_status;
-    int grid = low ? 2 * ctx->sms : ctx->sms;
-    if (c.tiles == nullptr) {
-        const int work = ((c.M + rows - 1) / rows) * n_tiles;
-        if (work < grid) grid = work;
-    }
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.gridDim = dim3(plan.grid, 1, 1);
     cfg.blockDim = dim3(ta_threads(low ? kTaGroupsLow : kTaGroups), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -259,7 +286,11 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, k, maps, p), "qmm launch");
+    r = check_cuda(ctx, cudaLaunchKernelEx(&cfg, k, maps, p), "qmm launch");
+    if (r != kOk || p.split.tiles == 0) return r;
+    const int warps = plan.split.tiles * ((rows + 3) / 4) * 4, blocks = (warps + 7) / 8;
+    return check_cuda(ctx, launch_dependent(c.epi ? ta_sum_kernel<1> : ta_sum_kernel<0>, dim3(std::min(blocks, 8 * ctx->sms)), 256, 0, st, p),
+                      "qmm sums launch");
 }
 
 int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
@@ -289,18 +320,31 @@ int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
 
 using namespace iq;
 
+namespace iq {
+QmmSplit qmm_split(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K, void* scratch, size_t bytes) {
+    QmmSplit r;
+    if (fmt < 0 || fmt == kFmtAffine6 || fmt > kFmtTernary) return r;
+    const TaPlan p = ta_plan(fmt, epi, M, N, K, ctx->sms, true);
+    r.bytes = round_up_sz(ta_split_bytes(p.split, p.rows), 256);
+    if (r.bytes != 0 && bytes >= r.bytes && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0) r.part = static_cast<float*>(scratch);
+    return r;
+}
+size_t qmm_split_max_bytes(iq_ctx* ctx) { return (size_t)2 * ctx->sms * ta_slot(kTaMaxRows) * 4; }  // (two CTAs per SM: slots of a third)
+size_t qmm_convert_bytes(int rows, int k, int32_t x_dtype) { return x_dtype == IQ_F16 ? 0 : round_up_sz((size_t)rows * k * 2, 256); }
+
+}  // namespace iq
+
 extern "C" int32_t iq_qmm_workspace_bytes(iq_ctx* ctx, const iq_qlinear* m, int32_t rows, int32_t x_dtype, size_t* bytes) {
     if (ctx == nullptr || m == nullptr || bytes == nullptr || rows < 1) return kErrInvalidArg;
     // The MMA takes fp16 weights with fp16 activations only (a bf16 B operand beside an fp16 A operand is an illegal
     // instruction on sm_100a: kind::f16 wants both operands of one type), so bf16 and fp32 activations are converted
-    *bytes = x_dtype == IQ_F16 ? 0 : round_up_sz((size_t)rows * m->k * 2, 256);
+    *bytes = qmm_convert_bytes(rows, m->k, x_dtype) + qmm_split(ctx, format_of(m), 0, rows, m->n, m->k, nullptr, 0).bytes;
     return kOk;
 }
 
-extern "C" int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m,
-                          void* y, int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, void* workspace,
-                          size_t workspace_bytes) {
-    if (ctx == nullptr) return kErrInvalidArg;
+namespace iq {
+int32_t qmm_check(iq_ctx* ctx, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, const void* y, int32_t y_dtype, int64_t ldy,
+                  int32_t rows) {
     if (x == nullptr || y == nullptr || m == nullptr || m->w == nullptr || m->scales == nullptr)
         return fail(ctx, kErrInvalidArg, "qmm: null pointer");
     const int32_t fmt = format_of(m);
@@ -318,32 +362,47 @@ extern "C" int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dt
     if (x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 2) return fail(ctx, kErrInvalidArg, "qmm: dtype");
     if (ldx < m->k || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0 || ldy < m->n)
         return fail(ctx, kErrInvalidArg, "qmm: x must be 16-byte aligned with ldx >= k, ldx %% 8 == 0; ldy >= n");
-    cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
-    const void* x16 = x;
-    int64_t ld16 = ldx;
-    if (x_dtype != IQ_F16) {
-        size_t need = 0;
-        iq_qmm_workspace_bytes(ctx, m, rows, x_dtype, &need);
-        if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0)
-            return fail(ctx, kErrWorkspace, "qmm: workspace %zu < %zu (256-byte aligned)", workspace_bytes, need);
-        const size_t units = (size_t)rows * m->k / 8;
-        convert_x_f16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, cs>>>(x, x_dtype, ldx, static_cast<__half*>(workspace),
-                                                                             rows, m->k);
-        int32_t st = check_cuda(ctx, cudaGetLastError(), "convert_x launch");
-        if (st != kOk) return st;
-        x16 = workspace;
-        ld16 = m->k;
-    }
+    return kOk;
+}
+
+int32_t launch_convert_x(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, void* out, int rows, int k) {
+    const size_t units = (size_t)rows * k / 8;
+    return check_cuda(ctx, launch_dependent(convert_x_f16_kernel, dim3((unsigned)((units + 255) / 256)), 256, 0, st, x, x_dtype, ldx,
+                                            static_cast<__half*>(out), rows, k), "convert_x launch");
+}
+
+int32_t qmm_f16(iq_ctx* ctx, cudaStream_t st, const void* x, int64_t ldx, const iq_qlinear* m, void* y, int32_t y_dtype, int64_t ldy, int32_t rows,
+                uint32_t flags, const QmmSplit& split) {
     QmmCall c;
-    c.fmt = fmt;
+    c.fmt = format_of(m);
     c.epi = 0;
-    c.x16 = x16; c.ldx = ld16; c.x_rows = rows;
+    c.x16 = x; c.ldx = ldx; c.x_rows = rows;
     c.w[0] = m->w; c.s[0] = m->scales; c.b[0] = m->biases;
     c.experts = 1;
     c.N = m->n; c.K = m->k; c.M = rows;
     c.y = y; c.y_dtype = y_dtype; c.ldy = ldy;
     c.accumulate = (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0;
-    return launch_qmm(ctx, cs, c);
+    c.split = split;
+    return launch_qmm(ctx, st, c);
+}
+}  // namespace iq
+
+extern "C" int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m,
+                          void* y, int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, void* workspace,
+                          size_t workspace_bytes) {
+    if (ctx == nullptr) return kErrInvalidArg;
+    int32_t st = qmm_check(ctx, x, x_dtype, ldx, m, y, y_dtype, ldy, rows);
+    if (st != kOk) return st;
+    cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
+    const size_t need = qmm_convert_bytes(rows, m->k, x_dtype);
+    QmmSplit split;  // (a workspace that holds the converted activations only is good as well: every tile is one item then)
+    if (workspace != nullptr && workspace_bytes > need)
+        split = qmm_split(ctx, format_of(m), 0, rows, m->n, m->k, static_cast<char*>(workspace) + need, workspace_bytes - need);
+    if (x_dtype == IQ_F16) return qmm_f16(ctx, cs, x, ldx, m, y, y_dtype, ldy, rows, flags, split);
+    if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0)
+        return fail(ctx, kErrWorkspace, "qmm: workspace %zu < %zu (256-byte aligned)", workspace_bytes, need);
+    st = launch_convert_x(ctx, cs, x, x_dtype, ldx, workspace, rows, m->k);
+    return st != kOk ? st : qmm_f16(ctx, cs, workspace, m->k, m, y, y_dtype, ldy, rows, flags, split);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -354,9 +413,10 @@ extern "C" int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dt
 // a "no allocation after start-up" rule (real-time serving paths, sandboxes that filter the allocator entry points).
 // iq_qmm needs a scratch buffer when the activations are bf16 or fp32 (they are converted to fp16 first) and expects the
 // caller to bring it. This variant brings its own: a fixed array that is part of the library image, so it exists on
-// every GPU that loads the library, from load until the process exits, and costs that GPU kNoAllocBytes of memory.
-constexpr size_t kNoAllocBytes = 8u << 20;  // 8 MiB: rows * k <= 4,194,304 activations (e.g. 1024 x 4096)
-static __device__ __align__(256) unsigned char g_qmm_noalloc_scratch[kNoAllocBytes];
+// every GPU that loads the library, from load until the process exits, and costs that GPU kNoAllocBytes + kNoAllocSplit of memory.
+constexpr size_t kNoAllocBytes = 8u << 20;   // 8 MiB: rows * k <= 4,194,304 activations (e.g. 1024 x 4096)
+constexpr size_t kNoAllocSplit = 40u << 20;  // partial sums of the K split: two slots of 192 tokens per SM (28 MiB on 148)
+static __device__ __align__(256) unsigned char g_qmm_noalloc_scratch[kNoAllocBytes + kNoAllocSplit];
 
 namespace {
 constexpr int kMaxDevices = 64;
@@ -392,5 +452,5 @@ extern "C" int32_t iq_qmm_noalloc(iq_ctx* ctx, void* stream, const void* x, int3
     }
     // Every byte the GEMM reads from the scratch is written by this call's own conversion pass first, so nothing has
     // to be cleared; what the previous call left behind is simply overwritten.
-    return iq_qmm(ctx, stream, x, x_dtype, ldx, m, y, y_dtype, ldy, rows, flags, scratch, kNoAllocBytes);
+    return iq_qmm(ctx, stream, x, x_dtype, ldx, m, y, y_dtype, ldy, rows, flags, scratch, kNoAllocBytes + kNoAllocSplit);
 }

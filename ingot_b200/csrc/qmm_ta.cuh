@@ -61,6 +61,11 @@ constexpr int kTaSmemMax = 232448;
 constexpr int kTaSmemLow = 115712;         // two CTAs per SM: half of 228 KB each, less the system's KB
 constexpr int kTaSmemFixed = 1024 + 1024;  // alignment, barriers
 
+// K split of the tiles that fill no whole round (below)
+struct TaSplit {
+    int32_t tiles, units, ctas;  // split tiles (the first ones of the list), units per tile, CTAs that share them
+};
+
 struct TaParams {
     const void* s[2];
     const void* b[2];
@@ -83,6 +88,9 @@ struct TaParams {
     int32_t x_stage;         // bytes of an X stage
     int32_t dcols;           // columns per accumulator: 64, 128 or 192
     int32_t early;           // the tile list is complete when the kernel starts
+    TaSplit split;           // dense
+    float* part;             // its partial sums
+    int32_t ustep;           // K steps per unit of the split
     int32_t vec;             // how scales are read: 1 by asynchronous copies, 0 in pairs of bytes, -1 (MXFP4) byte by byte
     int32_t* status;
 };
@@ -90,6 +98,51 @@ struct TaParams {
 struct TaMaps {
     CUtensorMap x[4], w[2];
 };
+
+// ---- split of the last round ------------------------------------------------------------------------------------------
+// T tiles over G CTAs take ceil(T / G) rounds, the last one with T % G tiles: 336 tiles on 148 CTAs spend a third of the time on
+// 40 of them, and a 64-row call has 52 tiles in all. So the R tiles beyond the whole rounds are divided along K: their
+// R x units units of `ustep` K steps are dealt to the CTAs in equal contiguous runs (a run touches two tiles at most). A piece of
+// a tile goes to a slot of fp32 sums, and ta_sum_kernel behind the GEMM adds a tile's slots in the order of K and stores.
+// Measured and taken back: sums by whichever piece ends last (four epilogue warps read 98 KB per piece at the latency of their
+// loads: 20 us for four pieces of 192 tokens, under which the next tile's accumulator waits); tile lists (a round is one of many).
+// On one B200, us: 64 rows x 4096 x 14336 (8 bits) 72.7 -> 25.9, 128 x 7744 x 11520 (4 bits) 52.8 -> 36.6, 320 x 4096 x 14336
+// 65.5 -> 44.6, 4096 x 1024 x 7680 80.4 -> 72.8, 2048 x 4096 x 14336 (8 bits, added) 248 -> 239; dense FFN of 256 rows, 2048 x 7680 81 -> 65.
+constexpr int kTaSplitPieces = 8;    // pieces per tile at most (one more where a run begins in the tile before)
+// Cycles of a K step of tiles of `rows` tokens (measured: 440 up to 64 rows, where issue and hand-overs are the time, 0.65 more per row
+// beyond), and of a split: the sums' kernel, and the partial sums that are written and read at some 1900 bytes per cycle.
+inline int ta_step_cycles(int rows, bool low) { return (440 + (rows > 64 ? (rows - 64) * 13 / 20 : 0)) * (low ? 2 : 1); }
+inline long long ta_split_cycles(const TaSplit& s, int rows) { return 7000 + (long long)(s.ctas + s.tiles) * rows * 1024 / 1900; }
+inline TaSplit ta_split(int total, int ctas, int ksteps, int ustep, int rows, bool low) {
+    TaSplit r;
+    r.units = (ksteps + ustep - 1) / ustep;
+    r.tiles = total < ctas ? total : total % ctas;
+    r.ctas = r.tiles * kTaSplitPieces < ctas ? r.tiles * kTaSplitPieces : ctas;
+    if (r.tiles * r.units < r.ctas) r.ctas = r.tiles * r.units;
+    // the round saved, less the CTA's share of it, has to be longer than what the split costs
+    if (r.tiles == 0 || (long long)(r.ctas - r.tiles) * ksteps * ta_step_cycles(rows, low) <= ta_split_cycles(r, rows) * r.ctas) r.tiles = r.ctas = 0;
+    return r;
+}
+// What a CTA does, worked out once and read from shared memory at every item (in registers it made the roles' loops spill): its
+// pieces of split tiles, then whole tiles.
+struct TaSched {
+    int32_t total, n_tiles, m_tiles, split;  // work items, tiles of features, tiles of tokens, split tiles
+    int32_t np;
+    struct Piece {
+        int32_t tile, ks0, ks1;
+        int32_t slot;  // of the partial sums, -1: the whole tile
+    } piece[2];
+};
+// The CTAs [c0, c1) share split tile t; a CTA's piece is in the slot of its number, or of ctas + t where the tile is its second
+__host__ __device__ inline void ta_split_tile(const TaSplit& s, int t, int& c0, int& c1, int& slot0) {
+    const int all = s.tiles * s.units, ua = t * s.units;
+    c0 = ((ua + 1) * s.ctas - 1) / all;  // the last CTA whose run starts at or before the tile's first unit
+    c1 = ((ua + s.units) * s.ctas - 1) / all + 1;
+    slot0 = c0 * all / s.ctas < ua ? s.ctas + t : c0;
+}
+// floats of a slot for tiles of up to `rows` tokens; slots: one per CTA, one per split tile
+__host__ __device__ inline int ta_slot(int rows) { return 128 * ((rows + 15) & ~15); }
+inline size_t ta_split_bytes(const TaSplit& s, int rows) { return (size_t)(s.ctas + s.tiles) * ta_slot(rows) * 4; }
 
 // Shared-memory and instruction descriptors: K-major B tile with 128-byte swizzle (rows of 128 bytes, 8-row groups 1024
 // bytes apart; the low 14 bits take the address in units of 16 bytes), fp16 operands, fp32 accumulator, M = 128.
@@ -208,6 +261,58 @@ __device__ __forceinline__ void ta_dequant32(uint32_t codes, uint32_t unit, int 
     }
 }
 
+// What becomes of CW token columns of a tile: v[j] is feature n of token row0 + j (gate/up: lanes l and l + 16 hold gate and up of
+// feature n) with the expert's bias, j < live.
+template <int EPI, int CW>
+__device__ __forceinline__ void ta_store(const TaParams& p, float (&v)[CW], int row0, int n, bool n_ok, int live, int mi) {
+    if (EPI) {
+        // the lower lane finishes token j, the upper token j + 1
+        float g[CW / 2], u[CW / 2];
+#pragma unroll
+        for (int j = 0; j < CW / 2; j++) {
+            const float other = __shfl_xor_sync(0xffffffffu, mi ? v[2 * j] : v[2 * j + 1], 16);
+            g[j] = mi ? other : v[2 * j];
+            u[j] = mi ? v[2 * j + 1] : other;
+        }
+        auto act = [&](auto tag) {
+#pragma unroll
+            for (int j = 0; j < CW / 2; j++) g[j] = glu<decltype(tag)::value>(g[j], u[j], p.limit);
+        };
+        if (p.act == kActSilu) act(std::integral_constant<int, kActSilu>{});
+        else if (p.act == kActSwigluOai) act(std::integral_constant<int, kActSwigluOai>{});
+        else if (p.act == kActGelu) act(std::integral_constant<int, kActGelu>{});
+        else act(std::integral_constant<int, kActRelu2>{});
+        __half* yp = reinterpret_cast<__half*>(p.y) + (size_t)(row0 + mi) * p.ldy + n;
+#pragma unroll
+        for (int j = 0; j < CW / 2; j++)
+            if (n_ok && 2 * j + mi < live) yp[(size_t)(2 * j) * p.ldy] = __float2half_rn(g[j]);
+    } else {
+        const size_t o0 = (size_t)row0 * p.ldy + n;
+        auto store = [&](auto load_f, auto store_f) {
+            if (p.accumulate) {  // all loads before the first store
+                float old[CW];
+#pragma unroll
+                for (int j = 0; j < CW; j++) old[j] = n_ok && j < live ? load_f(o0 + (size_t)j * p.ldy) : 0.f;
+#pragma unroll
+                for (int j = 0; j < CW; j++) v[j] = old[j] + v[j];
+            }
+#pragma unroll
+            for (int j = 0; j < CW; j++)
+                if (n_ok && j < live) store_f(o0 + (size_t)j * p.ldy, v[j]);
+        };
+        if (p.y_dtype == kF32) {
+            float* y = reinterpret_cast<float*>(p.y);
+            store([&](size_t o) { return y[o]; }, [&](size_t o, float f) { y[o] = f; });
+        } else if (p.y_dtype == kF16) {
+            __half* y = reinterpret_cast<__half*>(p.y);
+            store([&](size_t o) { return __half2float(y[o]); }, [&](size_t o, float f) { y[o] = __float2half_rn(f); });
+        } else {
+            uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
+            store([&](size_t o) { return bf16_bits_to_f32(y[o]); }, [&](size_t o, float f) { y[o] = (uint16_t)f32_to_bf16_bits(f); });
+        }
+    }
+}
+
 // EPI: 0 store, 1 gate + up + activation.
 template <int FMT, int EPI, int GROUPS>
 __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 2) qmm_ta_kernel(const __grid_constant__ TaMaps maps, const TaParams p) {
@@ -225,6 +330,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     const uint32_t bar_aempty = bar_aready + 64, bar_tfull = bar_aempty + 64, bar_tempty = bar_tfull + 16;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * kTaMaxStages + 20);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile TaSched* sched = reinterpret_cast<volatile TaSched*>(tmem_slot + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -247,6 +353,26 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
+        // the work list
+        if (p.tiles != nullptr && !p.early) pdl_wait();
+        constexpr int NROWS = EPI ? 64 : 128;
+        const int n_tiles = (p.N + NROWS - 1) / NROWS, m_tiles = p.tiles != nullptr ? (int)(*p.ntiles) : (p.M + p.tile_rows - 1) / p.tile_rows;
+        const int total = m_tiles * n_tiles, bid = (int)blockIdx.x;
+        const TaSplit& sp = p.split;
+        sched->total = total; sched->n_tiles = n_tiles; sched->m_tiles = m_tiles; sched->split = sp.tiles;
+        int np = 0;
+        if (bid < sp.ctas) {
+            const int all = sp.tiles * sp.units, lo = bid * all / sp.ctas, hi = (bid + 1) * all / sp.ctas;
+            for (int t = lo / sp.units; t * sp.units < hi; t++, np++) {  // (two at most)
+                const int ua = t * sp.units, ub = ua + sp.units;
+                volatile TaSched::Piece& c = sched->piece[np];
+                int c0, c1, slot0;
+                ta_split_tile(sp, t, c0, c1, slot0);
+                c.tile = t; c.ks0 = max(lo - ua, 0) * p.ustep; c.ks1 = min((min(hi, ub) - ua) * p.ustep, p.K / 64);
+                c.slot = c1 - c0 == 1 ? -1 : bid == c0 ? slot0 : bid;
+            }
+        }
+        sched->np = np;
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TCOLS)
@@ -266,23 +392,32 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     if ((p.tiles != nullptr && !p.early) || !(warp == 2 || warp == 3 || warp >= 8)) pdl_wait();
     if (p.tiles != nullptr) pdl_launch_dependents();
 
-    // ---- work list --------------------------------------------------------------------------------------------------
     constexpr int NROWS = EPI ? 64 : 128;  // output features per tile
-    const int n_tiles = (p.N + NROWS - 1) / NROWS;
-    const int m_tiles = p.tiles != nullptr ? (int)(*p.ntiles) : (p.M + p.tile_rows - 1) / p.tile_rows;
-    const int total = m_tiles * n_tiles;
-    const int ksteps = p.K / 64, chunks = (ksteps + KPS - 1) / KPS;
+    const int ksteps = p.K / 64;
     const int na = p.dcols == 128 ? 8 : 4;
     const uint32_t tmem_a = tmem + 2 * p.dcols;
-    auto decode = [&](int wi, int& expert, int& row0, int& rows, int& n0) {
-        if (p.tiles != nullptr) {
-            const Tile t = p.tiles[wi / n_tiles];
-            expert = (int)t.expert - p.expert_lo; row0 = (int)t.start; rows = (int)t.count;
-            n0 = (wi % n_tiles) * NROWS;
+    struct Item {
+        int ks0, ks1, expert, row0, rows, n0;
+    };
+    auto item = [&](int i, Item& t) -> bool {
+        int tile;
+        const int np = sched->np, n_tiles = sched->n_tiles, m_tiles = sched->m_tiles;
+        if (i < np) {
+            tile = sched->piece[i].tile; t.ks0 = sched->piece[i].ks0; t.ks1 = sched->piece[i].ks1;
         } else {
-            expert = 0; row0 = (wi % m_tiles) * p.tile_rows; rows = min(p.tile_rows, p.M - row0);
-            n0 = (wi / m_tiles) * NROWS;
+            tile = sched->split + (int)blockIdx.x + (i - np) * (int)gridDim.x;
+            t.ks0 = 0; t.ks1 = ksteps;
+            if (tile >= sched->total) return false;
         }
+        if (p.tiles != nullptr) {
+            const Tile l = p.tiles[tile / n_tiles];
+            t.expert = (int)l.expert - p.expert_lo; t.row0 = (int)l.start; t.rows = (int)l.count;
+            t.n0 = (tile % n_tiles) * NROWS;
+        } else {
+            t.expert = 0; t.row0 = (tile % m_tiles) * p.tile_rows; t.rows = min(p.tile_rows, p.M - t.row0);
+            t.n0 = (tile / m_tiles) * NROWS;
+        }
+        return true;
     };
 
     if (warp == 0) {
@@ -291,16 +426,15 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
-                int expert, row0, rows, n0;
-                decode(wi, expert, row0, rows, n0);
-                const int bi = (rows - 1) / p.xbox;
+            Item t;
+            for (int i = 0; ok && item(i, t); i++) {
+                const int bi = (t.rows - 1) / p.xbox;
                 const CUtensorMap* const map = &maps.x[bi];
                 const uint32_t bytes = (uint32_t)(p.xbox * (bi + 1) * p.xk * 128);
-                for (int ks = 0; ks < ksteps; ks += p.xk) {
+                for (int ks = t.ks0; ks < t.ks1; ks += p.xk) {
                     if (!(ok = mbar_wait(bar_xempty + 8 * s, ph ^ 1, abort_flag))) break;
                     mbar_arrive_expect_tx(bar_xfull + 8 * s, bytes);
-                    tma_load_3d(x0 + s * p.x_stage, map, bar_xfull + 8 * s, 0, row0, ks);
+                    tma_load_3d(x0 + s * p.x_stage, map, bar_xfull + 8 * s, 0, t.row0, ks);
                     if (++s == p.nx) { s = 0; ph ^= 1; }
                 }
             }
@@ -311,11 +445,10 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
-                int expert, row0, rows, n0;
-                decode(wi, expert, row0, rows, n0);
-                const int wrow = expert * p.N + n0;
-                for (int ch = 0; ch < chunks; ch++) {
+            Item t;
+            for (int i = 0; ok && item(i, t); i++) {
+                const int wrow = t.expert * p.N + t.n0;
+                for (int ch = t.ks0 / KPS; ch * KPS < t.ks1; ch++) {
                     if (!(ok = mbar_wait(bar_cempty + 8 * s, ph ^ 1, abort_flag))) break;
                     mbar_arrive_expect_tx(bar_cfull + 8 * s, kTaCodeStage);
                     const uint32_t dst = codes0 + s * kTaCodeStage;
@@ -336,18 +469,17 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         int s = 0;
         uint32_t ph = 0;
         bool ok = true;
-        for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
-            int expert, row0, rows, n0;
-            decode(wi, expert, row0, rows, n0);
+        Item t;
+        for (int it = 0; ok && item(it, t); it++) {
             const char* src[4][NT];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int row = lane + 32 * i, mi = EPI ? i >> 1 : 0, n = min(n0 + (EPI ? row & 63 : row), p.N - 1);
-                const size_t o = ((size_t)expert * p.N + n) * pitch;
+                const int row = lane + 32 * i, mi = EPI ? i >> 1 : 0, n = min(t.n0 + (EPI ? row & 63 : row), p.N - 1);
+                const size_t o = ((size_t)t.expert * p.N + n) * pitch;
                 src[i][0] = static_cast<const char*>(p.s[mi]) + o;
                 if (NT == 2) src[i][NT - 1] = static_cast<const char*>(p.b[mi]) + o;
             }
-            for (int ch = 0; ch < chunks; ch++) {
+            for (int ch = t.ks0 / KPS; ch * KPS < t.ks1; ch++) {
                 ok = mbar_wait(bar_cempty + 8 * s, ph ^ 1, abort_flag);
                 if (!(ok = __all_sync(0xffffffffu, ok))) break;
                 const uint32_t dst = scales0 + s * SSTAGE;
@@ -356,19 +488,19 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
 #pragma unroll
                     for (int i = 0; i < 4; i++)
 #pragma unroll
-                        for (int t = 0; t < NT; t++)
-                            cp_async_ca<SPB>(dst + t * 128 * SPB + (lane + 32 * i) * SPB, src[i][t] + ch * SPB);
+                        for (int m = 0; m < NT; m++)
+                            cp_async_ca<SPB>(dst + m * 128 * SPB + (lane + 32 * i) * SPB, src[i][m] + ch * SPB);
                 } else {
                     uint32_t v[4][NT][SPB / 2];
                     auto load = [&](auto bytes) {  // (the choice outside: the loads of a stage go out together)
 #pragma unroll
                         for (int i = 0; i < 4; i++)
 #pragma unroll
-                            for (int t = 0; t < NT; t++)
+                            for (int m = 0; m < NT; m++)
 #pragma unroll
                                 for (int e = 0; e < SPB / 2; e++) {
-                                    const char* a = src[i][t] + ch * SPB + min(2 * e, left - 2);
-                                    v[i][t][e] = decltype(bytes)::value ? ldg_nc_u8(a) | (ldg_nc_u8(a + 1) << 8) : ldg_nc_u16(a);
+                                    const char* a = src[i][m] + ch * SPB + min(2 * e, left - 2);
+                                    v[i][m][e] = decltype(bytes)::value ? ldg_nc_u8(a) | (ldg_nc_u8(a + 1) << 8) : ldg_nc_u16(a);
                                 }
                     };
                     if (FMT == kFmtMxfp4 && p.vec < 0) load(std::true_type{});
@@ -376,10 +508,10 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
 #pragma unroll
                     for (int i = 0; i < 4; i++)
 #pragma unroll
-                        for (int t = 0; t < NT; t++)
+                        for (int m = 0; m < NT; m++)
 #pragma unroll
                             for (int e = 0; e < SPB / 4; e++)
-                                sts32(dst + t * 128 * SPB + (lane + 32 * i) * SPB + 4 * e, v[i][t][2 * e] | (v[i][t][2 * e + 1] << 16));
+                                sts32(dst + m * 128 * SPB + (lane + 32 * i) * SPB + 4 * e, v[i][m][2 * e] | (v[i][m][2 * e + 1] << 16));
                 }
                 // (the copies' arrival orders copies only: plain stores are published by an arrival that releases them)
                 if (p.vec > 0) cp_async_arrive_noinc(bar_cfull + 8 * s);
@@ -399,16 +531,15 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             uint32_t a_hint = 0, x_hint = 0;
             const uint32_t xdesc0 = (x0 & 0x3FFFFu) >> 4;
             bool ok = true;
-            for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
-                int expert, row0, rows, n0;
-                decode(wi, expert, row0, rows, n0);
-                const uint32_t idesc = ta_idesc((rows + 15) & ~15);
+            Item t;
+            for (int i = 0; ok && item(i, t); i++) {
+                const uint32_t idesc = ta_idesc((t.rows + 15) & ~15);
                 if (!(ok = mbar_wait_hint(0, bar_tempty + 8 * acc, tph ^ 1, abort_flag))) break;
                 const uint32_t td = tmem + acc * p.dcols;
-                const uint32_t kunits = (uint32_t)(p.xbox * ((rows - 1) / p.xbox + 1) * 8);
-                for (int ks0 = 0; ks0 < ksteps && ok; ks0 += p.xk) {
+                const uint32_t kunits = (uint32_t)(p.xbox * ((t.rows - 1) / p.xbox + 1) * 8);
+                for (int ks0 = t.ks0; ks0 < t.ks1 && ok; ks0 += p.xk) {
                     if (!(ok = mbar_wait_hint(x_hint, bar_xfull + 8 * xs, xph, abort_flag))) break;
-                    const int ks1 = min(ksteps, ks0 + p.xk);
+                    const int ks1 = min(t.ks1, ks0 + p.xk);
                     uint32_t xdesc = xdesc0 + xs * ((uint32_t)p.x_stage >> 4);
                     const uint32_t xdone = bar_xempty + 8 * xs;
                     if (++xs == p.nx) { xs = 0; xph ^= 1; }
@@ -420,7 +551,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                         if (ks + 1 == ks1) x_hint = mbar_test(bar_xfull + 8 * xs, xph);
                         tc_fence_after();
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, (ks | kk) ? 1u : 0u);
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, ks != t.ks0 || kk != 0 ? 1u : 0u);
                         umma_commit(done);
                     }
                     umma_commit(xdone);
@@ -432,7 +563,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         }
     } else if (warp >= 8) {
         // ================= dequantisers =================
-        // Group g converts the steps whose number, counted over all tiles of the CTA, is g modulo GROUPS, a thread per weight row
+        // Group g converts the steps whose number, counted over all items of the CTA, is g modulo GROUPS, a thread per weight row
         // (never by the step's number in its tile: a group that skips the end of a tile would wait on an A stage more than
         // one round ahead, which a phase bit cannot tell from this round). One warp's step is a chain of latencies
         // (barrier, shared-memory round trip, conversion, tensor-memory store and its completion, about 1000 cycles); four
@@ -443,12 +574,14 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         const uint32_t my_a = tmem_a + ((uint32_t)(32 * q) << 16);
         constexpr int SPB = F::SPB;
         const int nash = na == 8 ? 3 : 2;
-        uint32_t it0 = 0;     // steps of the tiles before
+        uint32_t it0 = 0;     // steps of the items before
         int cs = 0;           // stage of codes
         uint32_t cph = 0;
         bool ok = true;
-        for (int wi = blockIdx.x; wi < total && ok; wi += gridDim.x) {
-            for (int ch = 0; ch < chunks; ch++) {
+        Item t;
+        for (int n = 0; ok && item(n, t); n++) {
+            const int steps = t.ks1 - t.ks0;  // (t.ks0 is the first step of a stage)
+            for (int ch = 0; ch * KPS < steps; ch++) {
                 const int j0 = (grp - (int)it0 - ch * KPS) & (GROUPS - 1);  // this group's first step of the stage
                 // Every group waits for every stage and hands it back, also those that hold no step of its own (8-bit codes have
                 // two steps per stage, for two of the four groups). A group that passed stages over could ask for the next round
@@ -462,7 +595,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                     for (int i = 0; i < (KPS + GROUPS - 1) / GROUPS; i++) {
                         const int j = j0 + GROUPS * i;
                         const int ks = ch * KPS + j;
-                        if (ks >= ksteps) break;
+                        if (ks >= steps) break;
                         const uint32_t it = it0 + ks, as = it & (na - 1), aph = (it >> nash) & 1;
                         const uint32_t a_hint = mbar_test(bar_aempty + 8 * as, aph ^ 1);
                         uint32_t sc, bi = 0;
@@ -498,7 +631,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                 if (lane == 0) mbar_arrive(bar_cempty + 8 * cs);
                 if (++cs == p.nc) { cs = 0; cph ^= 1; }
             }
-            it0 += ksteps;
+            it0 += steps;
         }
     } else {
         // ================= epilogue (warps 4-7) =================
@@ -507,73 +640,33 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         const int nl = EPI ? q * 16 + (lane & 15) : q * 32 + lane;
         int acc = 0;
         uint32_t tph = 0;
-        for (int wi = blockIdx.x; wi < total; wi += gridDim.x) {
-            int expert, row0, rows, n0;
-            decode(wi, expert, row0, rows, n0);
-            const int n = n0 + nl;
+        Item t;
+        for (int i = 0; item(i, t); i++) {
+            const int rows = t.rows, n = t.n0 + nl;
             const bool n_ok = n < p.N;
             const float* eb = mi ? p.ebias[1] : p.ebias[0];
-            const float bias = eb != nullptr && n_ok ? eb[(size_t)expert * p.N + n] : 0.f;
+            const float bias = eb != nullptr && n_ok ? eb[(size_t)t.expert * p.N + n] : 0.f;
             if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * acc, tph, abort_flag))) break;
             tc_fence_after();
             const uint32_t td = tmem + acc * p.dcols + ((uint32_t)(32 * q) << 16);
             constexpr int CW = 16;  // token columns at a time
+            const int slot = i < sched->np ? sched->piece[i].slot : -1;
+            float4* const part = reinterpret_cast<float4*>(p.part) + (size_t)slot * (ta_slot(p.tile_rows) / 4) + q * (ta_slot(p.tile_rows) / 16) + lane;
             for (int c0 = 0; c0 < rows; c0 += CW) {
                 uint32_t r[CW];
                 tmem_ld16(td + c0, r);
                 tmem_ld_wait();
-                const int live = rows - c0;  // columns j < live exist
-                if (EPI) {
-                    // lanes l and l + 16 hold gate and up of one feature: the lower lane finishes token j, the upper token j + 1
-                    float g[CW / 2], u[CW / 2];
+                if (slot >= 0) {  // a piece: [warp][four columns][lane], 16 bytes each
 #pragma unroll
-                    for (int j = 0; j < CW / 2; j++) {
-                        const float a = __uint_as_float(r[2 * j]) + bias, b = __uint_as_float(r[2 * j + 1]) + bias;
-                        const float other = __shfl_xor_sync(0xffffffffu, mi ? a : b, 16);
-                        g[j] = mi ? other : a;
-                        u[j] = mi ? b : other;
-                    }
-                    auto act = [&](auto tag) {
-#pragma unroll
-                        for (int j = 0; j < CW / 2; j++) g[j] = glu<decltype(tag)::value>(g[j], u[j], p.limit);
-                    };
-                    if (p.act == kActSilu) act(std::integral_constant<int, kActSilu>{});
-                    else if (p.act == kActSwigluOai) act(std::integral_constant<int, kActSwigluOai>{});
-                    else if (p.act == kActGelu) act(std::integral_constant<int, kActGelu>{});
-                    else act(std::integral_constant<int, kActRelu2>{});
-                    __half* yp = reinterpret_cast<__half*>(p.y) + (size_t)(row0 + c0 + mi) * p.ldy + n;
-#pragma unroll
-                    for (int j = 0; j < CW / 2; j++)
-                        if (n_ok && 2 * j + mi < live) yp[(size_t)(2 * j) * p.ldy] = __float2half_rn(g[j]);
-                } else {
-                    const size_t o0 = (size_t)(row0 + c0) * p.ldy + n;
-                    auto store = [&](auto load_f, auto store_f) {
-                        float v[CW];
-#pragma unroll
-                        for (int j = 0; j < CW; j++) v[j] = __uint_as_float(r[j]) + bias;
-                        if (p.accumulate) {  // all loads before the first store
-                            float old[CW];
-#pragma unroll
-                            for (int j = 0; j < CW; j++) old[j] = n_ok && j < live ? load_f(o0 + (size_t)j * p.ldy) : 0.f;
-#pragma unroll
-                            for (int j = 0; j < CW; j++) v[j] = old[j] + v[j];
-                        }
-#pragma unroll
-                        for (int j = 0; j < CW; j++)
-                            if (n_ok && j < live) store_f(o0 + (size_t)j * p.ldy, v[j]);
-                    };
-                    if (p.y_dtype == kF32) {
-                        float* y = reinterpret_cast<float*>(p.y);
-                        store([&](size_t o) { return y[o]; }, [&](size_t o, float f) { y[o] = f; });
-                    } else if (p.y_dtype == kF16) {
-                        __half* y = reinterpret_cast<__half*>(p.y);
-                        store([&](size_t o) { return __half2float(y[o]); }, [&](size_t o, float f) { y[o] = __float2half_rn(f); });
-                    } else {
-                        uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
-                        store([&](size_t o) { return bf16_bits_to_f32(y[o]); },
-                              [&](size_t o, float f) { y[o] = (uint16_t)f32_to_bf16_bits(f); });
-                    }
+                    for (int j = 0; j < CW / 4; j++)
+                        part[(c0 / 4 + j) * 32] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                              __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+                    continue;
                 }
+                float v[CW];
+#pragma unroll
+                for (int j = 0; j < CW; j++) v[j] = __uint_as_float(r[j]) + bias;
+                ta_store<EPI, CW>(p, v, t.row0 + c0, n, n_ok, rows - c0, mi);
             }
             tc_fence_before();
             __syncwarp();
@@ -595,6 +688,42 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
+    }
+}
+
+// Sums of the pieces of the split tiles, behind the GEMM: a warp takes a quarter of a tile's rows and four token columns, 16
+// bytes per lane and piece.
+template <int EPI>
+__global__ void __launch_bounds__(256) ta_sum_kernel(const TaParams p) {
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int NROWS = EPI ? 64 : 128;
+    const int m_tiles = (p.M + p.tile_rows - 1) / p.tile_rows;
+    const TaSplit& sp = p.split;
+    const int cols = (p.tile_rows + 3) / 4, lane = threadIdx.x & 31;
+    const int slot4 = ta_slot(p.tile_rows) / 4;
+    for (int w = blockIdx.x * 8 + (threadIdx.x >> 5); w < sp.tiles * cols * 4; w += gridDim.x * 8) {
+        const int q = w & 3, c4 = (w >> 2) % cols, t = (w >> 2) / cols;
+        const int row0 = (t % m_tiles) * p.tile_rows, rows = min(p.tile_rows, p.M - row0), n0 = (t / m_tiles) * NROWS;
+        int a, b, slot0;
+        ta_split_tile(sp, t, a, b, slot0);
+        if (b - a == 1 || 4 * c4 >= rows) continue;
+        const int mi = EPI ? lane >> 4 : 0, n = n0 + (EPI ? q * 16 + (lane & 15) : q * 32 + lane);
+        const bool n_ok = n < p.N;
+        const float* eb = mi ? p.ebias[1] : p.ebias[0];
+        const float bias = eb != nullptr && n_ok ? eb[n] : 0.f;
+        const float4* s = reinterpret_cast<const float4*>(p.part) + q * (slot4 / 4) + c4 * 32 + lane;
+        float4 f[kTaSplitPieces + 2];  // (a run that starts inside the tile's neighbour makes one piece more)
+#pragma unroll
+        for (int k = 0; k < kTaSplitPieces + 2; k++)
+            if (a + k < b) f[k] = s[(size_t)(k == 0 ? slot0 : a + k) * slot4];
+        float v[4] = {f[0].x, f[0].y, f[0].z, f[0].w};
+#pragma unroll
+        for (int k = 1; k < kTaSplitPieces + 2; k++)
+            if (a + k < b) { v[0] += f[k].x; v[1] += f[k].y; v[2] += f[k].z; v[3] += f[k].w; }
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] += bias;
+        ta_store<EPI, 4>(p, v, row0 + 4 * c4, n, n_ok, rows - 4 * c4, mi);
     }
 }
 

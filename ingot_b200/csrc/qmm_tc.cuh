@@ -233,9 +233,10 @@ __global__ void __launch_bounds__(kQmmThreads, 1)
 }
 
 // fp32 / bf16 activations -> fp16, row-major [rows, k] contiguous (the MMA's B operand type)
-__global__ void convert_x_f16_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx, __half* __restrict__ out,
-                                     int rows, int k) {
-    pdl_launch_dependents();
+__global__ void __launch_bounds__(256) convert_x_f16_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx, __half* __restrict__ out,
+                                                           int rows, int k) {
+    pdl_wait();
+    pdl_launch_dependents();  // (after the wait: what runs before this kernel has ended when the GEMM starts on its weights)
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (i >= (size_t)rows * k) return;
     const size_t r = i / k, c = i % k;

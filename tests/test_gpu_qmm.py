@@ -185,3 +185,52 @@ def test_mxfp4_scales_at_any_address(cuda_device, K, by):
             VQMV.encode(xt, o, y, rows)
             assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(xt.float().cpu().numpy(), deq(host))) <= TOL
     assert capi.context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("fmt,group", [("q4", 64), ("q8", 64), ("q4", 32), ("mxfp4", 32)])
+@pytest.mark.parametrize("M,N,K", [(64, 192, 14336), (64, 2112, 5824), (192, 128, 9216), (128, 7744, 2880), (320, 4096, 4160), (2048, 4096, 5120)])
+def test_qmm_split_along_k(cuda_device, fmt, group, M, N, K):
+    """Tiles that fill no whole round are divided along K: one tile in eight pieces and more, runs that end inside a tile, an odd number
+    of stages, pieces before whole tiles. Against the oracle, against the call whose workspace has no room for the sums (every tile
+    in one piece), the same bits every time, and added onto a result."""
+    rng = np.random.default_rng(71 + M + N + K + group)
+    bits = 8 if fmt == "q8" else 4
+    m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, bits, cuda_device, group=group)
+    x = synth.activations_np(rng, M, K)
+    xt = x_tensor(x, cuda_device)
+    y = run_qmm(m, xt, M)
+    sel = np.sort(rng.choice(N, size=min(N, 96), replace=False))
+    some = tuple(h[:, sel] for h in host)
+    ref = qref.matmul_t(x, deq(some, bits, group=group))
+    got = y[:, torch.from_numpy(sel).to(cuda_device)].cpu().numpy()
+    assert qref.max_rel(got, ref) <= TOL
+    whole = torch.zeros_like(y)
+    m.encode_qmm_f32(xt, whole, M, workspace=torch.empty(M * K * 2, dtype=torch.uint8, device=cuda_device))
+    # the same products in another order of sums: 14336 roundings of 2^-24, as a random walk, are 7e-6 of a sum's size
+    assert float((y - whole).abs().max() / whole.abs().max()) <= 2e-5
+    assert torch.equal(run_qmm(m, xt, M), y)
+    y0 = torch.randn(M, N, device=cuda_device)
+    assert torch.equal(run_qmm(m, xt, M, accumulate=True, y=y0.clone()), y0 + y)
+    assert torch.equal(run_qmm(m, x_tensor(x, cuda_device, torch.float16), M, torch.float16), y.to(torch.float16))
+
+
+@pytest.mark.parametrize("act", ["silu", "swiglu_oai"])
+@pytest.mark.parametrize("rows,d,d_ff", [(64, 1216, 8768), (256, 2048, 7680), (320, 4160, 1088)])
+def test_dense_ffn_split_along_k(cuda_device, rows, d, d_ff, act):
+    """The gated epilogue on the sums of pieces, and the down projection's split, against a float64 product."""
+    rng = np.random.default_rng(72 + rows)
+    gu, hg = affine_case(rng, 2 * d_ff, d, 4, cuda_device)
+    dn, hd = affine_case(rng, d, d_ff, 4, cuda_device)
+    x = x_tensor(synth.activations_np(rng, rows, d), cuda_device)
+    out = torch.zeros(rows, d, dtype=torch.float32, device=cuda_device)
+    DenseMLP(gu, dn, act).encode(x, out, rows)
+    assert capi.context(0).device_status() == 0
+    w = [torch.from_numpy(deq(h, 4)).to(cuda_device).double() for h in (hg, hd)]
+    g, u = (x.double() @ w[0].T).split(d_ff, dim=1)
+    if act == "silu":
+        h = g / (1 + torch.exp(-g)) * u
+    else:
+        g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0)
+        h = (u + 1) * g / (1 + torch.exp(-1.702 * g))
+    ref = h.to(torch.float16).double() @ w[1].T
+    assert float((out - ref).abs().max() / ref.abs().max()) <= TOL
