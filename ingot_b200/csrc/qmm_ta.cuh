@@ -282,34 +282,42 @@ __device__ __forceinline__ void ta_store(const TaParams& p, float (&v)[CW], int 
         else if (p.act == kActSwigluOai) act(std::integral_constant<int, kActSwigluOai>{});
         else if (p.act == kActGelu) act(std::integral_constant<int, kActGelu>{});
         else act(std::integral_constant<int, kActRelu2>{});
+        if (!n_ok) return;
         __half* yp = reinterpret_cast<__half*>(p.y) + (size_t)(row0 + mi) * p.ldy + n;
+        const size_t step = 2 * p.ldy;
+        if (live >= CW) {
 #pragma unroll
-        for (int j = 0; j < CW / 2; j++)
-            if (n_ok && 2 * j + mi < live) yp[(size_t)(2 * j) * p.ldy] = __float2half_rn(g[j]);
+            for (int j = 0; j < CW / 2; j++, yp += step) *yp = __float2half_rn(g[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < CW / 2; j++, yp += step)
+                if (2 * j + mi < live) *yp = __float2half_rn(g[j]);
+        }
     } else {
-        const size_t o0 = (size_t)row0 * p.ldy + n;
-        auto store = [&](auto load_f, auto store_f) {
+        if (!n_ok) return;
+        const size_t step = p.ldy;
+        auto store = [&](auto* y, auto load_f, auto round_f) {
+            y += (size_t)row0 * p.ldy + n;
             if (p.accumulate) {  // all loads before the first store
                 float old[CW];
+                auto* yp = y;
 #pragma unroll
-                for (int j = 0; j < CW; j++) old[j] = n_ok && j < live ? load_f(o0 + (size_t)j * p.ldy) : 0.f;
+                for (int j = 0; j < CW; j++, yp += step) old[j] = j < live ? load_f(*yp) : 0.f;
 #pragma unroll
                 for (int j = 0; j < CW; j++) v[j] = old[j] + v[j];
             }
+            if (live >= CW) {
 #pragma unroll
-            for (int j = 0; j < CW; j++)
-                if (n_ok && j < live) store_f(o0 + (size_t)j * p.ldy, v[j]);
+                for (int j = 0; j < CW; j++, y += step) *y = round_f(v[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < CW; j++, y += step)
+                    if (j < live) *y = round_f(v[j]);
+            }
         };
-        if (p.y_dtype == kF32) {
-            float* y = reinterpret_cast<float*>(p.y);
-            store([&](size_t o) { return y[o]; }, [&](size_t o, float f) { y[o] = f; });
-        } else if (p.y_dtype == kF16) {
-            __half* y = reinterpret_cast<__half*>(p.y);
-            store([&](size_t o) { return __half2float(y[o]); }, [&](size_t o, float f) { y[o] = __float2half_rn(f); });
-        } else {
-            uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
-            store([&](size_t o) { return bf16_bits_to_f32(y[o]); }, [&](size_t o, float f) { y[o] = (uint16_t)f32_to_bf16_bits(f); });
-        }
+        if (p.y_dtype == kF32) store(reinterpret_cast<float*>(p.y), [](float f) { return f; }, [](float f) { return f; });
+        else if (p.y_dtype == kF16) store(reinterpret_cast<__half*>(p.y), [](__half h) { return __half2float(h); }, [](float f) { return __float2half_rn(f); });
+        else store(reinterpret_cast<uint16_t*>(p.y), [](uint16_t u) { return bf16_bits_to_f32(u); }, [](float f) { return (uint16_t)f32_to_bf16_bits(f); });
     }
 }
 
