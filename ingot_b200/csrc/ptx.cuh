@@ -209,4 +209,10 @@ __device__ __forceinline__ void st_dsmem_u32(uint32_t* p, uint32_t cta, uint32_t
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void st_dsmem_u64(unsigned long long* p, uint32_t cta, unsigned long long v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(cta));
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(v) : "memory");
+}
+
 }  // namespace iq

@@ -18,9 +18,10 @@ namespace iq {
 namespace {
 
 constexpr int kTopK = 64;
-constexpr int kChunk = 4096;   // logits per part
-constexpr int kMaxParts = 64;  // parts per row: up to 262,144 logits
-constexpr int kSortThreads = 1024;
+constexpr int kMaxVocab = 262144;
+constexpr int kTopBlocks = 8;      // blocks of a cluster, which share a row
+constexpr int kTopThreads = 1024;
+constexpr int kTopList = 1024;     // keys of a block's list of candidates
 
 // Sort key of a logit: an unsigned that orders like the float (-0 taken as +0 so that it ties with it); 0 = not a candidate.
 __device__ __forceinline__ uint32_t order_key(float v) {
@@ -28,196 +29,204 @@ __device__ __forceinline__ uint32_t order_key(float v) {
     const uint32_t u = __float_as_uint(v == 0.f ? 0.f : v);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-
-constexpr int kPerThread = kChunk / kSortThreads;
-constexpr int kSteps = 16;  // two bits of the key per step
-
-struct SelectSmem {
-    uint32_t count[kSteps][3];
-    uint32_t above[kPerThread][kSortThreads / 32];  // accepted above the threshold / equal to it, per (k, warp)
-    uint32_t equal[kPerThread][kSortThreads / 32];
-};
-
-// The 64 largest of the block's kChunk keys (key k of thread t has index t + k * kSortThreads; equal keys count the lower
-// index as the larger), fewer when there are fewer candidates: emit(k, position) for each, positions in index order from 0.
-// Returns how many. The threshold is found two bits at a time by counting the keys at or above three trial values (a ballot
-// per key and value, one barrier per step), and the search stops as soon as exactly 64 are left: about 10 steps for
-// ordinary logits. A full bitonic sort of the 4096 keys took 78 barriers and 69 us for eight rows of 128,000.
-template <class Emit>
-__device__ __forceinline__ int select64(const uint32_t (&u)[kPerThread], SelectSmem& sm, int tid, Emit emit) {
-    const int lane = tid & 31, warp = tid >> 5;
-    if (tid < kSteps * 3) sm.count[tid / 3][tid % 3] = 0;
-    __syncthreads();
-    uint32_t thr = 0, n_at = 0xFFFFFFFFu;  // the keys at or above thr are at least 64, if there are that many candidates
-    for (int st = 0; st < kSteps; st++) {
-        const int sh = 30 - 2 * st;
-        uint32_t c[3] = {0, 0, 0};
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            const uint32_t trial = thr | ((uint32_t)(j + 1) << sh);
-#pragma unroll
-            for (int k = 0; k < kPerThread; k++) c[j] += __popc(__ballot_sync(0xffffffffu, u[k] >= trial));
-        }
-        if (lane < 3) {
-            const uint32_t mine = lane == 0 ? c[0] : (lane == 1 ? c[1] : c[2]);
-            if (mine != 0) atomicAdd(&sm.count[st][lane], mine);
-        }
-        __syncthreads();
-        const uint32_t n1 = sm.count[st][0], n2 = sm.count[st][1], n3 = sm.count[st][2];
-        if (n3 >= kTopK) { thr |= 3u << sh; n_at = n3; }
-        else if (n2 >= kTopK) { thr |= 2u << sh; n_at = n2; }
-        else if (n1 >= kTopK) { thr |= 1u << sh; n_at = n1; }
-        if (n_at == kTopK) break;
-    }
-    if (thr == 0) thr = 1;  // fewer than 64 candidates: all of them
-    // positions in index order: keys above the threshold all count, keys equal to it the first ones
-    uint32_t ba[kPerThread], be[kPerThread];
-#pragma unroll
-    for (int k = 0; k < kPerThread; k++) {
-        ba[k] = __ballot_sync(0xffffffffu, u[k] > thr);
-        be[k] = __ballot_sync(0xffffffffu, u[k] == thr);
-        if (lane == 0) {
-            sm.above[k][warp] = __popc(ba[k]);
-            sm.equal[k][warp] = __popc(be[k]);
-        }
-    }
-    __syncthreads();
-    uint32_t total_above = 0, total_equal = 0, above[kPerThread], equal[kPerThread];  // accepted before this (k, warp)
-#pragma unroll
-    for (int k = 0; k < kPerThread; k++) {
-        const uint32_t a = sm.above[k][lane], e = sm.equal[k][lane];
-        uint32_t pa = lane < warp ? a : 0, pe = lane < warp ? e : 0, ta = a, te = e;
-        pa = __reduce_add_sync(0xffffffffu, pa);
-        pe = __reduce_add_sync(0xffffffffu, pe);
-        ta = __reduce_add_sync(0xffffffffu, ta);
-        te = __reduce_add_sync(0xffffffffu, te);
-        above[k] = total_above + pa;
-        equal[k] = total_equal + pe;
-        total_above += ta;
-        total_equal += te;
-    }
-    // (when the search stopped early, keys between the threshold and the 64th are all above: total_above + total_equal = 64)
-    const uint32_t room = kTopK - total_above;  // equal keys that still fit
-    const uint32_t below = (1u << lane) - 1u;
-#pragma unroll
-    for (int k = 0; k < kPerThread; k++) {
-        const uint32_t na = above[k] + __popc(ba[k] & below), ne = equal[k] + __popc(be[k] & below);
-        if (u[k] > thr) emit(k, (int)(na + min(ne, room)));
-        else if (u[k] == thr && ne < room) emit(k, (int)(na + ne));
-    }
-    return (int)(total_above + min(total_equal, room));
+// With its id: keys are distinct, and of equal logits the lower id has the larger one.
+__device__ __forceinline__ unsigned long long full_key(uint32_t u, uint32_t id) {
+    return u == 0 ? 0ull : ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - id);
 }
+__device__ __forceinline__ unsigned long long max_u64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
 struct TopkParams {
     const float* x;
     int64_t ldx;
-    int32_t rows, V, parts;
+    int32_t V, span;  // logits of a row, and of a block: a multiple of kTopThreads
     float inv_t[16];
-    unsigned long long* part_keys;  // [rows, parts, 64] key << 32 | ~id, 0 where a part has fewer
-    float* part_mz;                 // [rows, parts, 2] part maximum and sum exp((x - part max) / T)
-    uint32_t* idx;                  // [rows, 64]
-    float* val;                     // [rows, 64]
-    float* z;                       // [rows, 2]
+    uint32_t* idx;    // [rows, 64]
+    float* val;       // [rows, 64]
+    float* z;         // [rows, 2]
 };
 
-__global__ void __launch_bounds__(kSortThreads) topk64_part_kernel(const TopkParams p) {
-    __shared__ SelectSmem sel;
-    __shared__ float red[32];
-    const int part = blockIdx.x, row = blockIdx.y, tid = threadIdx.x;
+// The 64 largest keys of a row, its maximum and its softmax denominator, by the eight blocks of a cluster.
+//
+// A block reads its span once (KPT logits per thread, in registers). The largest keys of 128 groups of its logits (eight lanes
+// each) are distinct, so that the 64th of them is not above the block's 64th largest key, and the keys from there on (about 90
+// of ordinary logits, whatever the span) are the list from which the block's 64 best are ranked by counting, several threads per
+// key. Where the list would not fit (orders made for it), the bound is searched by halving until it does. The first block gets
+// the eight sorted runs through distributed shared memory and ranks what is not below the smallest eighth-best.
+//
+// Bound: latency (a row of 128,000 is 0.5 MB). Two kernels of 4096-logit parts, searching the 64th key two bits and one block-wide
+// barrier at a time, took 23 us for one row of 128,000, 34 for eight and 51 for sixteen; now 11.4, 11.5 and 21.
+// KEEP: the span stays in registers; where it is long, or more than eight rows want two blocks per SM (sixteen rows of 128,000
+// 23 -> 21 us), it is read again instead.
+template <int KPT, bool KEEP>
+__global__ void __launch_bounds__(kTopThreads, KEEP ? 1 : 2) __cluster_dims__(kTopBlocks, 1, 1)
+    topk64_kernel(const __grid_constant__ TopkParams p) {
+    __shared__ unsigned long long list[kTopList], group_max[128], bound_;
+    __shared__ unsigned long long run[kTopBlocks][kTopK];  // the first block's: sorted candidates of every block
+    __shared__ double part_z[kTopBlocks];                  // likewise
+    __shared__ float part_max[kTopBlocks];
+    __shared__ float red[32], redz[32];
+    __shared__ uint32_t count[2], larger[kTopList];
+    const int row = blockIdx.x / kTopBlocks, part = blockIdx.x % kTopBlocks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_launch_dependents();
+    larger[tid] = 0;
+    if (tid < 2) count[tid] = 0;
+    if (tid == 0) bound_ = 1;  // (where fewer than 64 groups have a candidate: all that there are)
+    cluster_sync_all();  // the first block runs: its shared memory may be written
     pdl_wait();
     const float* xr = p.x + (size_t)row * p.ldx;
-    const int i0 = part * kChunk;
-    float v[kPerThread];
-    uint32_t u[kPerThread];
+    const int i0 = part * p.span + tid, end = min(p.V, (part + 1) * p.span);
+    auto read = [&](int k) {
+        const int i = i0 + k * kTopThreads;
+        return i < end ? xr[i] : -INFINITY;
+    };
+    float kept[KEEP ? KPT : 1];
+    if (KEEP) {
+#pragma unroll
+        for (int k = 0; k < KPT; k++) kept[KEEP ? k : 0] = read(k);
+    }
+    // every logit of the thread in order of id, eight loads at a time
+    auto each = [&](auto f) {
+#pragma unroll
+        for (int k0 = 0; k0 < KPT; k0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int k = k0; k < min(KPT, k0 + 8); k++) v[k - k0] = KEEP ? kept[KEEP ? k : 0] : read(k);
+#pragma unroll
+            for (int k = k0; k < min(KPT, k0 + 8); k++) f(k, v[k - k0]);
+        }
+    };
     float m = -INFINITY;
-#pragma unroll
-    for (int k = 0; k < kPerThread; k++) {
-        const int id = i0 + tid + k * kSortThreads;
-        v[k] = id < p.V ? xr[id] : -INFINITY;
-        u[k] = order_key(v[k]);
-        m = fmaxf(m, v[k]);
-    }
-    // part maximum
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((tid & 31) == 0) red[tid >> 5] = m;
-    __syncthreads();
-    m = red[tid & 31];
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __syncthreads();
-    // sum exp((x - part max) / T) in a fixed order: per thread, warp tree, then the warps in order
-    float s = 0.f;
-    if (m > -INFINITY) {
-        const float it = p.inv_t[row];
-#pragma unroll
-        for (int k = 0; k < kPerThread; k++)
-            if (i0 + tid + k * kSortThreads < p.V) s += expf((v[k] - m) * it);
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((tid & 31) == 0) red[tid >> 5] = s;
-    unsigned long long* out = p.part_keys + ((size_t)row * p.parts + part) * kTopK;
-    const int n = select64(u, sel, tid, [&](int k, int pos) {  // starts with a barrier
-        out[pos] = ((unsigned long long)u[k] << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(i0 + tid + k * kSortThreads));
+    uint32_t best = 0, best_id = 0;
+    each([&](int k, float v) {
+        const uint32_t u = order_key(v);
+        if (u > best) { best = u; best_id = i0 + k * kTopThreads; }
+        m = fmaxf(m, v);
     });
-    if (tid >= n && tid < kTopK) out[tid] = 0ull;
-    if (tid == 0) {
-        float tot = 0.f;
-        for (int i = 0; i < kSortThreads / 32; i++) tot += red[i];
-        p.part_mz[((size_t)row * p.parts + part) * 2] = m;
-        p.part_mz[((size_t)row * p.parts + part) * 2 + 1] = tot;
-    }
-}
-
-__global__ void __launch_bounds__(kSortThreads) topk64_merge_kernel(const TopkParams p) {
-    __shared__ SelectSmem sel;
-    __shared__ unsigned long long best[kTopK];
-    const int row = blockIdx.x, tid = threadIdx.x;
-    pdl_launch_dependents();
-    pdl_wait();
-    // the parts' candidates in part order, and in id order inside a part: index order is id order
-    unsigned long long key[kPerThread];
-    uint32_t u[kPerThread];
-#pragma unroll
-    for (int k = 0; k < kPerThread; k++) {
-        const int i = tid + k * kSortThreads;
-        key[k] = i < p.parts * kTopK ? p.part_keys[(size_t)row * p.parts * kTopK + i] : 0ull;
-        u[k] = (uint32_t)(key[k] >> 32);
-    }
-    if (tid < kTopK) best[tid] = 0ull;
-    const int n = select64(u, sel, tid, [&](int k, int pos) { best[pos] = key[k]; });  // starts with a barrier
+    unsigned long long gm = full_key(best, best_id);
+    for (int o = 4; o > 0; o >>= 1) gm = max_u64(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+    if ((lane & 7) == 0) group_max[4 * warp + (lane >> 3)] = gm;
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) red[warp] = m;
     __syncthreads();
-    if (tid < kTopK) {
-        // one thread per candidate: its place is the number of larger keys (the keys are distinct: they hold the id)
-        const unsigned long long k = best[tid];
-        int place = tid;
-        uint32_t id = 0xFFFFFFFFu;
-        float v = -FLT_MAX;
-        if (tid < n) {
-            place = 0;
-            for (int i = 0; i < n; i++) place += best[i] > k;
-            id = 0xFFFFFFFFu - (uint32_t)(k & 0xFFFFFFFFull);
-            v = p.x[(size_t)row * p.ldx + id];  // the logit's own bits (-0 stays -0)
-        }
-        p.idx[(size_t)row * kTopK + place] = id;
-        p.val[(size_t)row * kTopK + place] = v;
+    {  // the 64th of the groups' keys: eight threads count the larger ones of one
+        const unsigned long long mine = group_max[tid >> 3];
+        uint32_t c = 0;
+#pragma unroll
+        for (int j = 0; j < 16; j++) c += group_max[(tid & 7) + 8 * j] > mine;
+        for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        if ((tid & 7) == 0 && c == kTopK - 1 && mine != 0) bound_ = mine;
     }
-    if (tid >= kSortThreads - 32) {  // the last warp: two parts per lane
-        const int lane = tid & 31;
-        const float* mz = p.part_mz + (size_t)row * p.parts * 2;
-        float mq[kMaxParts / 32], zq[kMaxParts / 32], M = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < kMaxParts / 32; j++) {
-            const int q = lane + 32 * j;
-            mq[j] = q < p.parts ? mz[2 * q] : -INFINITY;
-            zq[j] = q < p.parts ? mz[2 * q + 1] : 0.f;
-            M = fmaxf(M, mq[j]);
+    m = red[lane];
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    __syncthreads();
+    unsigned long long bound = bound_;
+    // the keys from the bound on, in any order (few threads have one)
+    auto collect = [&](unsigned long long from, uint32_t* n) {
+        const uint32_t high = (uint32_t)(from >> 32);
+        each([&](int k, float v) {
+            const uint32_t u = order_key(v);
+            if (u >= high) {
+                const unsigned long long key = full_key(u, (uint32_t)(i0 + k * kTopThreads));
+                if (key >= from) {
+                    const uint32_t at = atomicAdd(n, 1u);
+                    if (at < kTopList) list[at] = key;
+                }
+            }
+        });
+    };
+    collect(bound, &count[0]);
+    // sum exp((x - block maximum) / T) in a fixed order: four sums per thread, trees over the warp and the warps (in float64)
+    const float inv_t = p.inv_t[row];
+    float z = 0.f;
+    if (m > -INFINITY) {
+        float e[4] = {0.f, 0.f, 0.f, 0.f};
+        each([&](int k, float v) { e[k & 3] += i0 + k * kTopThreads < end ? expf((v - m) * inv_t) : 0.f; });
+        z = (e[0] + e[1]) + (e[2] + e[3]);
+        for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    }
+    if (lane == 0) redz[warp] = z;
+    __syncthreads();
+    uint32_t n = count[0];
+    if (n > kTopList) {  // halve between the bound (too many keys) and the top (none) until the list fits; the keys are distinct
+        unsigned long long lo = bound, hi = ~0ull;
+        while (true) {
+            const unsigned long long mid = lo + (hi - lo) / 2;
+            uint32_t c = 0;
+            each([&](int k, float v) { c += full_key(order_key(v), (uint32_t)(i0 + k * kTopThreads)) >= mid; });
+            c = __reduce_add_sync(0xffffffffu, c);
+            __syncthreads();
+            if (tid == 0) count[1] = 0;
+            __syncthreads();
+            if (lane == 0) atomicAdd(&count[1], c);
+            __syncthreads();
+            n = count[1];
+            if (n > kTopList) lo = mid;
+            else if (n < kTopK) hi = mid;
+            else { bound = mid; break; }
         }
-        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        double Z = 0.0;
-        const float it = p.inv_t[row];
+        __syncthreads();
+        if (tid == 0) count[1] = 0;
+        __syncthreads();
+        collect(bound, &count[1]);
+        __syncthreads();
+    }
+    // a key's place is the number of larger ones: all threads count, several for a key
+    if (n != 0) {
+        const uint32_t per = max(1u, kTopThreads / n), c = tid % n, j = tid / n;
+        const unsigned long long mine = list[c];
+        if (j < per) {
+            uint32_t l = 0;
+            for (uint32_t i = j; i < n; i += per) l += list[i] > mine;
+            if (l != 0) atomicAdd(&larger[c], l);
+        }
+        __syncthreads();
+        if (j == 0 && larger[c] < kTopK) st_dsmem_u64(&run[part][larger[c]], 0, mine);
+    }
+    if (tid < kTopK && tid >= n) st_dsmem_u64(&run[part][tid], 0, 0ull);
+    if (warp == kTopThreads / 32 - 1) {
+        double tot = (double)redz[lane];
+        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        if (lane == 0) {
+            st_dsmem_u64(reinterpret_cast<unsigned long long*>(&part_z[part]), 0, (unsigned long long)__double_as_longlong(tot));
+            st_dsmem_u32(reinterpret_cast<uint32_t*>(&part_max[part]), 0, __float_as_uint(m));
+        }
+    }
+    cluster_sync_all();
+    if (part != 0) return;
+    // ---- the first block: two threads per key, four runs each ----------------------------------------------------------
+    unsigned long long floor8 = run[lane & 7][7];
+    for (int o = 4; o > 0; o >>= 1) {
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, floor8, o);
+        floor8 = other < floor8 ? other : floor8;
+    }
+    const unsigned long long mine = run[tid >> 7][(tid >> 1) & 63];
+    uint32_t place = 0;
+    if (mine != 0 && mine >= floor8) {
 #pragma unroll
-        for (int j = 0; j < kMaxParts / 32; j++)
-            if (mq[j] > -INFINITY) Z += (double)zq[j] * exp((double)(mq[j] - M) * (double)it);
+        for (int j = 0; j < kTopBlocks / 2; j++) {
+            const unsigned long long* r = run[(tid & 1) * (kTopBlocks / 2) + j];
+            int c = 0;
+#pragma unroll
+            for (int o = 32; o > 0; o >>= 1) c += r[c + o - 1] > mine ? o : 0;
+            place += c + (r[c] > mine);
+        }
+    }
+    place += __shfl_xor_sync(0xffffffffu, place, 1);
+    const int found = min(__syncthreads_count(mine != 0 && (tid & 1) == 0), kTopK);
+    if ((tid & 1) == 0 && mine != 0 && mine >= floor8 && place < kTopK) {
+        const uint32_t id = 0xFFFFFFFFu - (uint32_t)(mine & 0xFFFFFFFFull);
+        p.idx[(size_t)row * kTopK + place] = id;
+        p.val[(size_t)row * kTopK + place] = xr[id];  // the logit's own bits (-0 stays -0)
+    }
+    if (tid < kTopK && tid >= found) {
+        p.idx[(size_t)row * kTopK + tid] = 0xFFFFFFFFu;
+        p.val[(size_t)row * kTopK + tid] = -FLT_MAX;
+    }
+    if (warp == kTopThreads / 32 - 1) {
+        const float mq = lane < kTopBlocks ? part_max[lane] : -INFINITY;
+        float M = mq;
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        double Z = mq > -INFINITY ? part_z[lane & (kTopBlocks - 1)] * exp((double)(mq - M) * (double)inv_t) : 0.0;
         for (int o = 16; o > 0; o >>= 1) Z += __shfl_xor_sync(0xffffffffu, Z, o);
         if (lane == 0) {
             p.z[row * 2] = M;
@@ -297,9 +306,10 @@ extern "C" int32_t iq_argmax_rows(iq_ctx* ctx, void* stream, const float* x, int
     return st;
 }
 
+// (the kernel needs no scratch; what the contract asks for stays as it is)
 extern "C" int32_t iq_topk64_scratch_bytes(int32_t rows, int32_t vocab, size_t* bytes) {
-    if (bytes == nullptr || rows < 1 || rows > 16 || vocab < 1 || vocab > kChunk * kMaxParts) return kErrInvalidArg;
-    const size_t parts = (size_t)(vocab + kChunk - 1) / kChunk;
+    if (bytes == nullptr || rows < 1 || rows > 16 || vocab < 1 || vocab > kMaxVocab) return kErrInvalidArg;
+    const size_t parts = (size_t)(vocab + 4095) / 4096;
     *bytes = (size_t)rows * parts * (kTopK * 8 + 2 * 4) + 256;
     return kOk;
 }
@@ -311,23 +321,20 @@ extern "C" int32_t iq_topk64(iq_ctx* ctx, void* stream, const float* x, int64_t 
     size_t need = 0;
     if (x == nullptr || idx == nullptr || val == nullptr || z == nullptr || temperatures == nullptr || ldx < vocab ||
         (n_temperatures != 1 && n_temperatures != rows) || iq_topk64_scratch_bytes(rows, vocab, &need) != kOk)
-        return fail(ctx, kErrInvalidArg, "topk64: arguments (1..16 rows, up to %d logits, one temperature or one per row)",
-                    kChunk * kMaxParts);
+        return fail(ctx, kErrInvalidArg, "topk64: arguments (1..16 rows, up to %d logits, one temperature or one per row)", kMaxVocab);
     if (scratch == nullptr || scratch_bytes < need || (reinterpret_cast<uintptr_t>(scratch) & 7) != 0)
         return fail(ctx, kErrWorkspace, "topk64: scratch %zu < %zu (8-byte aligned)", scratch_bytes, need);
     TopkParams p;
-    p.x = x; p.ldx = ldx; p.rows = rows; p.V = vocab;
-    p.parts = (vocab + kChunk - 1) / kChunk;
+    p.x = x; p.ldx = ldx; p.V = vocab;
+    p.span = round_up((vocab + kTopBlocks - 1) / kTopBlocks, kTopThreads);
     for (int r = 0; r < 16; r++) {
         const float t = temperatures[n_temperatures == 1 ? 0 : (r < rows ? r : 0)];
         if (!(t > 0.f)) return fail(ctx, kErrInvalidArg, "topk64: temperature %g", (double)t);
         p.inv_t[r] = 1.0f / t;
     }
-    p.part_keys = static_cast<unsigned long long*>(scratch);
-    p.part_mz = reinterpret_cast<float*>(p.part_keys + (size_t)rows * p.parts * kTopK);
     p.idx = idx; p.val = val; p.z = z;
-    cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
-    cudaError_t e = launch_dependent(topk64_part_kernel, dim3(p.parts, rows), kSortThreads, 0, cs, p);
-    if (e == cudaSuccess) e = launch_dependent(topk64_merge_kernel, dim3(rows), kSortThreads, 0, cs, p);
-    return check_cuda(ctx, e, "topk64 launch");
+    const int kpt = p.span / kTopThreads;
+    auto kernel = kpt <= 4 ? topk64_kernel<4, true> : kpt <= 8 ? topk64_kernel<8, true> : kpt > 16 ? topk64_kernel<32, false>
+                  : rows <= 8 ? topk64_kernel<16, true> : topk64_kernel<16, false>;
+    return check_cuda(ctx, launch_dependent(kernel, dim3(rows * kTopBlocks), kTopThreads, 0, reinterpret_cast<cudaStream_t>(stream), p), "topk64 launch");
 }

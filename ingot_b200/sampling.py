@@ -27,7 +27,7 @@ def argmax_rows(x: torch.Tensor, rows: int, stream: Optional[torch.cuda.Stream] 
 
 
 class TopK64:
-    """Scratch sized once for (rows, vocabulary); `encode` enqueues the two kernels."""
+    """Scratch sized once for (rows, vocabulary); `encode` enqueues the kernel."""
 
     def __init__(self, max_rows: int, vocab: int, device: torch.device):
         n = C.c_size_t()

@@ -101,3 +101,16 @@ def test_argmax_of_more_rows_than_a_grid_dimension(cuda_device, rows, n):
     x = logits("ties", n, rows, rows + n)
     got = sampling.argmax_rows(torch.from_numpy(x).to(cuda_device), rows)
     assert np.array_equal(got.cpu().numpy().astype(np.uint32), qref.argmax_rows(x))
+
+
+@pytest.mark.parametrize("V,rows", [(5000, 2), (60000, 3), (131072, 8), (131072, 9), (262144, 2)])
+@pytest.mark.parametrize("rest", [-1e3, -np.inf])
+def test_candidates_of_orders_that_fill_the_list(cuda_device, V, rows, rest):
+    """63 of the 128 groups that a block takes its bound from hold all the large logits (thousands of them), so that the bound is a
+    small one and the list of keys from there on overflows; with as many distinct values as logits, and with eight values."""
+    rng = np.random.default_rng(V + rows)
+    x = (rng.random((rows, V)) * 10).astype(np.float32)
+    x[1] = np.floor(x[1])
+    x[:, (np.arange(V) % 1024) // 8 >= 63] = rest
+    x[:, 1023] = -5.0  # (one small finite logit)
+    check(x, [0.9])
