@@ -60,6 +60,27 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
     return *reinterpret_cast<uint32_t*>(&r);
 }
 
+// Four consecutive activations as floats; x + i is a multiple of 8 bytes (fp32: 16).
+__device__ __forceinline__ void load_x4(const void* x, int32_t dtype, size_t i, float (&v)[4]) {
+    if (dtype == kF32) {
+        const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + i);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        return;
+    }
+    const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(x) + i);
+    const uint32_t w[2] = {r.x, r.y};
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        if (dtype == kBF16) {
+            v[2 * j] = __uint_as_float(w[j] << 16);
+            v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
+        } else {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+            v[2 * j] = f.x; v[2 * j + 1] = f.y;
+        }
+    }
+}
+
 // Loads 8 consecutive activations starting at element index `i` (a multiple of 8) and returns them as fp32.
 __device__ __forceinline__ void load_x8(const void* x, int32_t dtype, size_t i, float (&v)[8]) {
     if (dtype == kBF16) {

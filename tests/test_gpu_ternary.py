@@ -137,10 +137,10 @@ def test_ternary_guards(cuda_device):
     assert e.value.status == -1
 
 
-@pytest.mark.parametrize("N,K,rows", [(16, 1024, 8), (48, 5120, 9), (2400, 5120, 5), (16, 14336, 16)])
+@pytest.mark.parametrize("N,K,rows", [(16, 1024, 8), (48, 5120, 9), (2400, 5120, 5), (16, 14336, 16), (7152, 1024, 3), (7120, 2048, 16), (32, 51200, 2)])
 def test_ternary_qmv_edges(cuda_device, N, K, rows):
-    """One block, group counts that the warps do not share evenly (40, 112), the step from eight to nine rows; a row alone has
-    the same bits."""
+    """One block, group counts that the warps do not share evenly (40, 112), the step from eight to nine rows, blocks of 32 features
+    with half a block at the end, scales that shared memory does not hold; a row alone has the same bits."""
     rng = np.random.default_rng(N + K + rows)
     m, wf, signs, _ = case(rng, N, K, cuda_device)
     x = half_activations(rng, rows, K)
