@@ -187,6 +187,36 @@ __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// ---- pairs of CTAs (tcgen05 with cta_group::2): the even CTA of a cluster of two issues for both -------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// arrival on the barrier at the same shared-memory offset of the cluster's CTA `cta`
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t cta) {
+    asm volatile("{\n.reg .b32 r;\nmapa.shared::cluster.u32 r, %0, %1;\nmbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n}\n" ::"r"(bar), "r"(cta)
+                 : "memory");
+}
+// Tensor copy into this CTA's shared memory whose bytes count on the barrier at this offset of the pair's even CTA
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile(
+        "{\n.reg .b32 r;\nmapa.shared::cluster.u32 r, %2, 0;\n"
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [r];\n}\n"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+// ... without the ordering of memory at cluster scope, which makes the thread wait for all it has under way: for what is complete
+// already (tensor memory behind tcgen05.wait)
+__device__ __forceinline__ void mbar_arrive_remote_done(uint32_t bar, uint32_t cta) {
+    asm volatile("{\n.reg .b32 r;\nmapa.shared::cluster.u32 r, %0, %1;\nmbarrier.arrive.shared::cluster.b64 _, [r];\n}\n" ::"r"(bar), "r"(cta) : "memory");
+}
+// completion of all tcgen05.mma issued so far, to the barrier at this offset in both CTAs
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+                 : "memory");
+}
+
 // ---- thread-block clusters ------------------------------------------------------------------------------------------
 // barrier over all threads of the cluster, with release/acquire ordering of shared-memory writes
 __device__ __forceinline__ void cluster_sync_all() {

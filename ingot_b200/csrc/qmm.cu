@@ -52,23 +52,25 @@ int ta_step_bytes(int32_t fmt) { return fmt == kFmtAffine8 ? 64 : (fmt == kFmtTe
 typedef void (*TaKernel)(const TaMaps, const TaParams);
 
 // gate/up: the formats of experts and of dense FFNs
-template <int GROUPS>
+template <int GROUPS, bool PAIR>
 TaKernel ta_pick(int32_t fmt, int epi) {
     switch (fmt) {
-        case kFmtAffine4: return epi ? qmm_ta_kernel<kFmtAffine4, 1, GROUPS> : qmm_ta_kernel<kFmtAffine4, 0, GROUPS>;
-        case kFmtMxfp4: return epi ? qmm_ta_kernel<kFmtMxfp4, 1, GROUPS> : qmm_ta_kernel<kFmtMxfp4, 0, GROUPS>;
-        case kFmtAffine8: return epi ? qmm_ta_kernel<kFmtAffine8, 1, GROUPS> : qmm_ta_kernel<kFmtAffine8, 0, GROUPS>;
-        case kFmtAffine4G32: return epi ? qmm_ta_kernel<kFmtAffine4G32, 1, GROUPS> : qmm_ta_kernel<kFmtAffine4G32, 0, GROUPS>;
-        case kFmtTernary: return epi ? nullptr : qmm_ta_kernel<kFmtTernary, 0, GROUPS>;
+        case kFmtAffine4: return epi ? qmm_ta_kernel<kFmtAffine4, 1, GROUPS, PAIR> : qmm_ta_kernel<kFmtAffine4, 0, GROUPS, PAIR>;
+        case kFmtMxfp4: return epi ? qmm_ta_kernel<kFmtMxfp4, 1, GROUPS, PAIR> : qmm_ta_kernel<kFmtMxfp4, 0, GROUPS, PAIR>;
+        case kFmtAffine8: return epi ? qmm_ta_kernel<kFmtAffine8, 1, GROUPS, PAIR> : qmm_ta_kernel<kFmtAffine8, 0, GROUPS, PAIR>;
+        case kFmtAffine4G32: return epi ? qmm_ta_kernel<kFmtAffine4G32, 1, GROUPS, PAIR> : qmm_ta_kernel<kFmtAffine4G32, 0, GROUPS, PAIR>;
+        case kFmtTernary: return epi ? nullptr : qmm_ta_kernel<kFmtTernary, 0, GROUPS, PAIR>;
         default: return nullptr;
     }
 }
 
-// Tiling of a dense GEMM: token rows per tile (a multiple of 16, at most 192), K split of the tiles beyond the whole rounds.
+// Tiling of a dense GEMM: token rows per tile (a multiple of 16, at most 192), one CTA or a pair per tile, K split of the tiles beyond
+// the whole rounds.
 struct TaPlan {
     int rows, n_tiles, ustep, grid;
     TaSplit split;
-    bool low;  // two CTAs per SM
+    bool low;   // two CTAs per SM
+    bool pair;  // clusters of two CTAs on tiles of twice the features
 };
 int ta_xk(bool low, int rows) { return low ? (rows <= 32 ? 4 : 2) : (rows <= 128 ? 4 : 2); }  // K steps per copy of X
 int ta_ustep(int32_t fmt, int xk) { return std::max(128 / ta_step_bytes(fmt), xk); }  // whole stages of codes and of X
@@ -77,25 +79,29 @@ int ta_ustep(int32_t fmt, int xk) { return std::max(128 / ta_step_bytes(fmt), xk
 TaPlan ta_plan(int32_t fmt, int epi, int M, int N, int K, int sms, bool may_split) {
     TaPlan best = {};
     double best_cost = -1;
-    const int n_tiles = (N + (epi ? 63 : 127)) / (epi ? 64 : 128), ksteps = K / 64;
+    const int features = epi ? 64 : 128, ksteps = K / 64;
     for (int tiles = (M + kTaMaxRows - 1) / kTaMaxRows; tiles <= (M + 15) / 16; tiles++) {
-        TaPlan p;
-        p.rows = round_up((M + tiles - 1) / tiles, 16);
-        p.n_tiles = n_tiles;
-        const int total = (M + p.rows - 1) / p.rows * n_tiles;
-        // Two CTAs per SM for low tiles; with a tile per SM or less the one with four dequantiser groups (MXFP4 24576 x 2048 at 64
-        // rows 21.0 -> 18.5 us)
-        p.low = p.rows <= kTaLowRows && total > sms;
-        const int ctas = p.low ? 2 * sms : sms;
-        p.ustep = ta_ustep(fmt, ta_xk(p.low, p.rows));
-        p.split = may_split ? ta_split(total, ctas, ksteps, p.ustep, p.rows, p.low) : TaSplit{0, 0, 0};
-        const double step = ta_step_cycles(p.rows, p.low);
-        double cost = (double)((total - p.split.tiles + ctas - 1) / ctas) * ksteps * step;
-        if (p.split.tiles)
-            cost += (p.split.tiles * p.split.units + p.split.ctas - 1) / p.split.ctas * p.ustep * step + (double)ta_split_cycles(p.split, p.rows);
-        p.grid = total < ctas && p.split.tiles == 0 ? total : ctas;
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = p; }
-        if (p.rows <= 64) break;
+        const int rows = round_up((M + tiles - 1) / tiles, 16);
+        for (int pair = 0; pair < (sms % 2 == 0 ? 2 : 1); pair++) {
+            TaPlan p;
+            p.rows = rows;
+            p.pair = pair != 0;
+            p.n_tiles = (N + (features << pair) - 1) / (features << pair);
+            const int total = (M + rows - 1) / rows * p.n_tiles;
+            // Two CTAs per SM for low tiles; with a tile per SM or less the one with four dequantiser groups (MXFP4 24576 x 2048 at 64
+            // rows 21.0 -> 18.5 us)
+            p.low = !pair && rows <= kTaLowRows && total > sms;
+            const int ctas = pair ? sms / 2 : p.low ? 2 * sms : sms;
+            p.ustep = ta_ustep(fmt, ta_xk(p.low, rows));
+            p.split = may_split ? ta_split(total, ctas, ksteps, p.ustep, rows, p.low, p.pair) : TaSplit{0, 0, 0};
+            const double step = ta_step_cycles(rows, p.low, p.pair);
+            double cost = (double)((total - p.split.tiles + ctas - 1) / ctas) * ksteps * step + (pair ? 1500 : 0);  // (a pair's start)
+            if (p.split.tiles)
+                cost += (p.split.tiles * p.split.units + p.split.ctas - 1) / p.split.ctas * p.ustep * step + (double)ta_split_cycles(p.split, rows, p.pair);
+            p.grid = (total < ctas && p.split.tiles == 0 ? total : ctas) << pair;
+            if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = p; }
+        }
+        if (rows <= 64) break;
     }
     return best;
 }
@@ -105,9 +111,10 @@ TaPlan ta_plan(int32_t fmt, int epi, int M, int N, int K, int sms, bool may_spli
 int32_t qmm_init(iq_ctx* ctx) {
     for (int fmt = 0; fmt <= kFmtTernary; fmt++)
         for (int epi = 0; epi < 2; epi++) {
-            const TaKernel k = ta_pick<kTaGroups>(fmt, epi), low = ta_pick<kTaGroupsLow>(fmt, epi);
+            const TaKernel k = ta_pick<kTaGroups, false>(fmt, epi), pair = ta_pick<kTaGroups, true>(fmt, epi), low = ta_pick<kTaGroupsLow, false>(fmt, epi);
             if (k == nullptr) continue;
             cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k), cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemMax);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(pair), cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemMax);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(low), cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemLow);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmm_ta)");
         }
@@ -210,7 +217,7 @@ int32_t cached_rows16_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t r
 
 // The quantized formats: weights through tensor memory (csrc/qmm_ta.cuh). c.bn: the largest tile of the list (grouped).
 static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
-    if (ta_pick<kTaGroups>(c.fmt, c.epi) == nullptr) return fail(ctx, kErrNoKernel, "qmm: no kernel for format %d, epilogue %d", c.fmt, c.epi);
+    if (ta_pick<kTaGroups, false>(c.fmt, c.epi) == nullptr) return fail(ctx, kErrNoKernel, "qmm: no kernel for format %d, epilogue %d", c.fmt, c.epi);
     TaParams p;
     memset(&p, 0, sizeof(p));
     TaPlan plan = {};
@@ -219,12 +226,15 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     } else {
         plan.rows = c.bn;
         plan.low = plan.rows <= kTaLowRows;
+        plan.pair = plan.rows == kTaMaxRows && ctx->sms % 2 == 0;  // (tiles of 128: 1024 tokens of 128 experts 198 us alone, 200 in pairs)
         plan.grid = plan.low ? 2 * ctx->sms : ctx->sms;
         plan.ustep = ta_ustep(c.fmt, ta_xk(plan.low, plan.rows));
     }
     const int rows = plan.rows;
     const bool low = plan.low;
-    const TaKernel k = low ? ta_pick<kTaGroupsLow>(c.fmt, c.epi) : ta_pick<kTaGroups>(c.fmt, c.epi);
+    const int ctas = plan.pair ? 2 : 1;
+    const TaKernel k = low ? ta_pick<kTaGroupsLow, false>(c.fmt, c.epi) : plan.pair ? ta_pick<kTaGroups, true>(c.fmt, c.epi) : ta_pick<kTaGroups, false>(c.fmt, c.epi);
+    p.pair = plan.pair;
     p.ustep = plan.ustep;
     p.split = plan.split;
     p.part = c.split.part;
@@ -234,7 +244,7 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     p.xbox = c.tiles == nullptr || rows <= 16 ? rows : round_up(rows / 4, 16);
     p.nbox = rows / p.xbox;
     p.xk = ta_xk(low, rows);
-    p.x_stage = rows * 128 * p.xk;
+    p.x_stage = rows / ctas * 128 * p.xk;
     p.dcols = low ? kTaLowRows : (rows <= 128 ? 128 : kTaMaxRows);
     // stages: at least three of codes, then up to eight of X, then as many of codes as fit
     const int room = (low ? kTaSmemLow : kTaSmemMax) - kTaSmemFixed;
@@ -249,7 +259,7 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     TaMaps maps;
     int32_t r = kOk;
     for (int i = 0; i < p.nbox && r == kOk; i++)
-        r = make_map_ksteps(ctx, &maps.x[i], c.x16, (uint64_t)c.x_rows, (uint64_t)c.K / 64, (uint64_t)c.ldx * 2, p.xbox * (i + 1), p.xk);
+        r = make_map_ksteps(ctx, &maps.x[i], c.x16, (uint64_t)c.x_rows, (uint64_t)c.K / 64, (uint64_t)c.ldx * 2, p.xbox * (i + 1) / ctas, p.xk);
     const uint32_t wbox = c.epi ? 64 : 128;
     for (int i = 0; i <= c.epi && r == kOk; i++)
         r = make_map_2d(ctx, &maps.w[i], c.w[i], 0, row_bytes, (uint64_t)c.experts * c.N, row_bytes, 128, wbox, true);
@@ -281,14 +291,16 @@ static int32_t launch_qmm_ta(iq_ctx* ctx, cudaStream_t st, const QmmCall& c) {
     cfg.blockDim = dim3(ta_threads(low ? kTaGroupsLow : kTaGroups), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = plan.pair ? 2 : 1;
     r = check_cuda(ctx, cudaLaunchKernelEx(&cfg, k, maps, p), "qmm launch");
     if (r != kOk || p.split.tiles == 0) return r;
-    const int warps = plan.split.tiles * ((rows + 3) / 4) * 4, blocks = (warps + 7) / 8;
+    const int warps = plan.split.tiles * ((rows + 3) / 4) * 4 * ctas, blocks = (warps + 7) / 8;
     return check_cuda(ctx, launch_dependent(c.epi ? ta_sum_kernel<1> : ta_sum_kernel<0>, dim3(std::min(blocks, 8 * ctx->sms)), 256, 0, st, p),
                       "qmm sums launch");
 }
@@ -325,7 +337,7 @@ QmmSplit qmm_split(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K, void*
     QmmSplit r;
     if (fmt < 0 || fmt == kFmtAffine6 || fmt > kFmtTernary) return r;
     const TaPlan p = ta_plan(fmt, epi, M, N, K, ctx->sms, true);
-    r.bytes = round_up_sz(ta_split_bytes(p.split, p.rows), 256);
+    r.bytes = round_up_sz(ta_split_bytes(p.split, p.rows, p.pair), 256);
     if (r.bytes != 0 && bytes >= r.bytes && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0) r.part = static_cast<float*>(scratch);
     return r;
 }

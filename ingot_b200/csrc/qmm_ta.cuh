@@ -7,8 +7,8 @@
 // (tile stores 16, MMA reads of the tile 16 and of X 32, TMA writes of X 32, codes 8: 832 cycles at 128 B per cycle) for 512
 // cycles of MMA, and ran at that port's rate. tcgen05.mma takes its A operand from tensor memory: the dequantisers write
 // there with tcgen05.st, a thread per weight row and 64 weights at a time, and what is left for the port is X (written
-// and read once) and the packed codes. The MMA itself gains as well: a step of 64 inputs with N tokens takes 2 N + 40
-// cycles with A in tensor memory and 2 N + 172 with A in shared memory (measured, operands resident).
+// and read once) and the packed codes. A step of 64 inputs with N tokens is 2 N cycles of MMA, whatever else the SM does (measured with
+// operands resident, beside tcgen05.st, shared-memory loads and spinning warps).
 //
 // Tensor memory (512 columns): two accumulators of up to 192 columns and four A stages of 32 columns (64 fp16 inputs per
 // lane), or two of up to 128 columns and eight A stages. Two accumulators always: the epilogue of a tile runs under the
@@ -18,7 +18,7 @@
 //   warp 0       producer of X tiles: one tensor copy brings two or four K steps of the tile (128-byte swizzle). A step of its
 //                own per copy does not do: the wait, the expected bytes and the copy's issue are a chain of 500 cycles in one
 //                thread, whatever the box
-//   warp 1       allocates tensor memory, issues tcgen05.mma (one lane), commits stages and accumulators
+//   warp 1       allocates tensor memory, issues tcgen05.mma (one lane; in a pair the even CTA's), commits stages and accumulators
 //   warp 2       producer of the packed codes: a stage is 128 bytes of 128 weight rows (two to eight K steps), so that DRAM
 //                and L2 see whole lines; 128-byte swizzle, so that the dequantisers' row-wise 16-byte loads are free of bank
 //                conflicts
@@ -28,6 +28,15 @@
 // The gate/up form takes 64 gate rows and the matching 64 up rows as one tile of 128: lanes 0-15 of every warp's quadrant
 // hold gate rows, lanes 16-31 the same rows of up, so that the activation needs one shuffle per two tokens and
 // everything else is the plain form.
+// Pairs of CTAs (cta_group::2). One CTA's step of 176 tokens and more takes 500 to 530 cycles of the 2 N that the MMA needs, with A
+// and X always there: the issuing thread's loop runs beside sixteen warps that convert codes, and X goes through every SM's port
+// twice (written, then read) for 128 features. Two CTAs take 256 features: each holds half of the tile's tokens, the tensor cores
+// read both halves, one thread issues for both SMs, and every SM copies half as much X, which the clock feels as well (these
+// kernels run into the power limit: 2048 x 4096 x 14336 at 8 bits 1300 MHz with X copied, 1440 without). Copies of X of both CTAs
+// count on the even one's barrier, dequantisers and epilogue warps of the odd one arrive there, and commits go to both. 2048 x
+// 4096 x 14336 (8 bits, added) 228 -> 210 us, 4096 x 4096 x 7680 225 -> 202, FFN 4096 x 14336 of 1088 rows 338 -> 314 (sustained, at
+// the power limit: 284 -> 246 and 426 -> 368 with the K split below). Below some 150 rows one CTA's finer tiles win. On the way:
+// arrivals that release at cluster scope cost the dequantisers 10 to 25 %, reporting the odd CTA's X by a thread of its own 20 %.
 // Tiles of a list that hold up to 64 tokens (MoE decode and short prefills) leave the MMA idle: a step of 16 tokens is 72 cycles
 // of it, and the 400 cycles of the issuing thread and of its hand-overs are the time. Two CTAs per SM, each with two
 // dequantiser groups, half of the shared memory and 256 columns (two accumulators of 64, four A stages), run two such
@@ -91,6 +100,7 @@ struct TaParams {
     TaSplit split;           // dense
     float* part;             // its partial sums
     int32_t ustep;           // K steps per unit of the split
+    int32_t pair;            // pairs of CTAs: tiles, rounds and the split count pairs
     int32_t vec;             // how scales are read: 1 by asynchronous copies, 0 in pairs of bytes, -1 (MXFP4) byte by byte
     int32_t* status;
 };
@@ -109,18 +119,21 @@ struct TaMaps {
 // On one B200, us: 64 rows x 4096 x 14336 (8 bits) 72.7 -> 25.9, 128 x 7744 x 11520 (4 bits) 52.8 -> 36.6, 320 x 4096 x 14336
 // 65.5 -> 44.6, 4096 x 1024 x 7680 80.4 -> 72.8, 2048 x 4096 x 14336 (8 bits, added) 248 -> 239; dense FFN of 256 rows, 2048 x 7680 81 -> 65.
 constexpr int kTaSplitPieces = 8;    // pieces per tile at most (one more where a run begins in the tile before)
-// Cycles of a K step of tiles of `rows` tokens (measured: 440 up to 64 rows, where issue and hand-overs are the time, 0.65 more per row
-// beyond), and of a split: the sums' kernel, and the partial sums that are written and read at some 1900 bytes per cycle.
-inline int ta_step_cycles(int rows, bool low) { return (440 + (rows > 64 ? (rows - 64) * 13 / 20 : 0)) * (low ? 2 : 1); }
-inline long long ta_split_cycles(const TaSplit& s, int rows) { return 7000 + (long long)(s.ctas + s.tiles) * rows * 1024 / 1900; }
-inline TaSplit ta_split(int total, int ctas, int ksteps, int ustep, int rows, bool low) {
+// Cycles of a K step of tiles of `rows` tokens (fitted to dense calls of 64 to 4096 rows; `low`: two CTAs share the SM), and of a split:
+// the sums' kernel, and the partial sums that are written and read at some 1900 bytes per cycle.
+inline int ta_step_cycles(int rows, bool low, bool pair) {
+    const int over = rows > 64 ? rows - 64 : 0;
+    return pair ? 420 + over * 9 / 20 : low ? 880 + over * 2 : 400 + over;
+}
+inline long long ta_split_cycles(const TaSplit& s, int rows, bool pair) { return 7000 + (long long)(s.ctas + s.tiles) * rows * (pair ? 2048 : 1024) / 1900; }
+inline TaSplit ta_split(int total, int ctas, int ksteps, int ustep, int rows, bool low, bool pair) {
     TaSplit r;
     r.units = (ksteps + ustep - 1) / ustep;
     r.tiles = total < ctas ? total : total % ctas;
     r.ctas = r.tiles * kTaSplitPieces < ctas ? r.tiles * kTaSplitPieces : ctas;
     if (r.tiles * r.units < r.ctas) r.ctas = r.tiles * r.units;
     // the round saved, less the CTA's share of it, has to be longer than what the split costs
-    if (r.tiles == 0 || (long long)(r.ctas - r.tiles) * ksteps * ta_step_cycles(rows, low) <= ta_split_cycles(r, rows) * r.ctas) r.tiles = r.ctas = 0;
+    if (r.tiles == 0 || (long long)(r.ctas - r.tiles) * ksteps * ta_step_cycles(rows, low, pair) <= ta_split_cycles(r, rows, pair) * r.ctas) r.tiles = r.ctas = 0;
     return r;
 }
 // What a CTA does, worked out once and read from shared memory at every item (in registers it made the roles' loops spill): its
@@ -142,15 +155,25 @@ __host__ __device__ inline void ta_split_tile(const TaSplit& s, int t, int& c0, 
 }
 // floats of a slot for tiles of up to `rows` tokens; slots: one per CTA, one per split tile
 __host__ __device__ inline int ta_slot(int rows) { return 128 * ((rows + 15) & ~15); }
-inline size_t ta_split_bytes(const TaSplit& s, int rows) { return (size_t)(s.ctas + s.tiles) * ta_slot(rows) * 4; }
+inline size_t ta_split_bytes(const TaSplit& s, int rows, bool pair) { return (size_t)(s.ctas + s.tiles) * ta_slot(rows) * (pair ? 8 : 4); }
 
 // Shared-memory and instruction descriptors: K-major B tile with 128-byte swizzle (rows of 128 bytes, 8-row groups 1024
 // bytes apart; the low 14 bits take the address in units of 16 bytes), fp16 operands, fp32 accumulator, M = 128.
 constexpr uint64_t kTaDescHi = ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-__device__ __forceinline__ uint32_t ta_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
+__device__ __forceinline__ uint32_t ta_idesc(int n, int ctas) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((8u * ctas) << 24); }
 
 // D[128, N] (+)= A[128, 16] (tensor memory: lane = row, two inputs per column) * B[N, 16]^T (shared memory)
+// (PAIR: 256 rows, the upper 128 of A and D in the tensor memory of the pair's other CTA, half of B's rows in its shared memory)
+template <bool PAIR>
 __device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    if (PAIR) {
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+            ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc)
+            : "memory");
+        return;
+    }
     asm volatile(
         "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
@@ -322,11 +345,17 @@ __device__ __forceinline__ void ta_store(const TaParams& p, float (&v)[CW], int 
 }
 
 // EPI: 0 store, 1 gate + up + activation.
-template <int FMT, int EPI, int GROUPS>
+// PAIR: a cluster of two CTAs works on tiles of twice the features.
+template <int FMT, int EPI, int GROUPS, bool PAIR>
 __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 2) qmm_ta_kernel(const __grid_constant__ TaMaps maps, const TaParams p) {
     using F = TaFmt<FMT>;
     constexpr int KPS = F::KPS;
+    static_assert(!PAIR || GROUPS == kTaGroups, "a pair has its SMs to itself");
     constexpr uint32_t TCOLS = GROUPS == kTaGroups ? 512 : 256;
+    constexpr int CTAS = PAIR ? 2 : 1;
+    constexpr int RS = GROUPS == kTaGroups ? 2 : 1;  // A stages per hand-over to the issuer
+    const uint32_t rank = PAIR ? cluster_rank() : 0;  // the even CTA issues the MMAs
+    const int unit = (int)blockIdx.x / CTAS, units = (int)gridDim.x / CTAS;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t codes0 = smem_u32(smem), x0 = codes0 + p.nc * kTaCodeStage;  // codes, X, scales
@@ -351,12 +380,12 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             mbar_init(bar_xempty + 8 * i, 1);
         }
         for (int i = 0; i < 8; i++) {
-            mbar_init(bar_aready + 8 * i, 4);
+            mbar_init(bar_aready + 8 * i, 4 * RS * CTAS);
             mbar_init(bar_aempty + 8 * i, 1);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(bar_tfull + 8 * i, 1);
-            mbar_init(bar_tempty + 8 * i, 4);
+            mbar_init(bar_tempty + 8 * i, 4 * CTAS);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -364,8 +393,9 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         // the work list
         if (p.tiles != nullptr && !p.early) pdl_wait();
         constexpr int NROWS = EPI ? 64 : 128;
-        const int n_tiles = (p.N + NROWS - 1) / NROWS, m_tiles = p.tiles != nullptr ? (int)(*p.ntiles) : (p.M + p.tile_rows - 1) / p.tile_rows;
-        const int total = m_tiles * n_tiles, bid = (int)blockIdx.x;
+        const int n_tiles = (p.N + CTAS * NROWS - 1) / (CTAS * NROWS);
+        const int m_tiles = p.tiles != nullptr ? (int)(*p.ntiles) : (p.M + p.tile_rows - 1) / p.tile_rows;
+        const int total = m_tiles * n_tiles, bid = unit;
         const TaSplit& sp = p.split;
         sched->total = total; sched->n_tiles = n_tiles; sched->m_tiles = m_tiles; sched->split = sp.tiles;
         int np = 0;
@@ -383,12 +413,17 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         sched->np = np;
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TCOLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TCOLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TCOLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync_all();  // the other CTA's barriers exist
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     // The weights do not depend on the previous kernel of the stream, a tile list, the activations and y do. With dense tiling the
@@ -413,17 +448,17 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         if (i < np) {
             tile = sched->piece[i].tile; t.ks0 = sched->piece[i].ks0; t.ks1 = sched->piece[i].ks1;
         } else {
-            tile = sched->split + (int)blockIdx.x + (i - np) * (int)gridDim.x;
+            tile = sched->split + unit + (i - np) * units;
             t.ks0 = 0; t.ks1 = ksteps;
             if (tile >= sched->total) return false;
         }
         if (p.tiles != nullptr) {
             const Tile l = p.tiles[tile / n_tiles];
             t.expert = (int)l.expert - p.expert_lo; t.row0 = (int)l.start; t.rows = (int)l.count;
-            t.n0 = (tile % n_tiles) * NROWS;
+            t.n0 = ((tile % n_tiles) * CTAS + (int)rank) * NROWS;
         } else {
             t.expert = 0; t.row0 = (tile % m_tiles) * p.tile_rows; t.rows = min(p.tile_rows, p.M - t.row0);
-            t.n0 = (tile / m_tiles) * NROWS;
+            t.n0 = ((tile / m_tiles) * CTAS + (int)rank) * NROWS;
         }
         return true;
     };
@@ -439,10 +474,12 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                 const int bi = (t.rows - 1) / p.xbox;
                 const CUtensorMap* const map = &maps.x[bi];
                 const uint32_t bytes = (uint32_t)(p.xbox * (bi + 1) * p.xk * 128);
+                const int xrow = t.row0 + (PAIR ? (int)rank * (((t.rows + 15) & ~15) / 2) : 0);  // a pair's CTAs hold half of the MMA's tokens each
                 for (int ks = t.ks0; ks < t.ks1; ks += p.xk) {
                     if (!(ok = mbar_wait(bar_xempty + 8 * s, ph ^ 1, abort_flag))) break;
-                    mbar_arrive_expect_tx(bar_xfull + 8 * s, bytes);
-                    tma_load_3d(x0 + s * p.x_stage, map, bar_xfull + 8 * s, 0, t.row0, ks);
+                    if (rank == 0) mbar_arrive_expect_tx(bar_xfull + 8 * s, bytes);  // (of both halves)
+                    if (PAIR) tma_load_3d_pair(x0 + s * p.x_stage, map, bar_xfull + 8 * s, 0, xrow, ks);
+                    else tma_load_3d(x0 + s * p.x_stage, map, bar_xfull + 8 * s, 0, xrow, ks);
                     if (++s == p.nx) { s = 0; ph ^= 1; }
                 }
             }
@@ -529,11 +566,15 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        // Every barrier is asked one step ahead, before the MMAs of the current step are issued: three waits in a row per two
-        // steps, each a round trip of 100 cycles and more, cost 5 %. What is left, some 400 cycles of this one thread per step,
-        // is the bound of tiles with fewer than about 180 tokens (more state in the loop, such as answers asked two steps
-        // ahead or pairs of steps on one barrier, measured slower).
-        if (elect_one()) {
+        // The loop's time is its round trips to barriers (100 to 200 cycles each beside the dequantisers), not the MMAs' issue (some 15
+        // cycles each). So every barrier is asked one step ahead, behind the MMAs, and with four dequantiser groups two A stages are
+        // handed over on one barrier and back on their own: 64 x 14336 x 14336 (MXFP4) 46.7 -> 42.7 us, 192 x 4096 x 4096 19.9 -> 18.3
+        // (also handed back together, tiles of 192 rows were 3 % slower; two groups, which hold two such pairs in all, 5 to 10 %).
+        if (rank == 0 && elect_one()) {
+            auto commit = [&](uint32_t bar) {
+                if (PAIR) umma_commit_pair(bar);
+                else umma_commit(bar);
+            };
             int xs = 0, as = 0, acc = 0;
             uint32_t xph = 0, aph = 0, tph = 0;
             uint32_t a_hint = 0, x_hint = 0;
@@ -541,30 +582,42 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             bool ok = true;
             Item t;
             for (int i = 0; ok && item(i, t); i++) {
-                const uint32_t idesc = ta_idesc((t.rows + 15) & ~15);
+                const uint32_t idesc = ta_idesc((t.rows + 15) & ~15, CTAS);
                 if (!(ok = mbar_wait_hint(0, bar_tempty + 8 * acc, tph ^ 1, abort_flag))) break;
                 const uint32_t td = tmem + acc * p.dcols;
-                const uint32_t kunits = (uint32_t)(p.xbox * ((t.rows - 1) / p.xbox + 1) * 8);
-                for (int ks0 = t.ks0; ks0 < t.ks1 && ok; ks0 += p.xk) {
+                const uint32_t kunits = (uint32_t)(p.xbox * ((t.rows - 1) / p.xbox + 1) / CTAS * 8);
+                uint32_t more = 0;  // the tile's first MMA starts the sums
+                for (int left = t.ks1 - t.ks0; left > 0 && ok; left -= p.xk) {
                     if (!(ok = mbar_wait_hint(x_hint, bar_xfull + 8 * xs, xph, abort_flag))) break;
-                    const int ks1 = min(t.ks1, ks0 + p.xk);
                     uint32_t xdesc = xdesc0 + xs * ((uint32_t)p.x_stage >> 4);
                     const uint32_t xdone = bar_xempty + 8 * xs;
                     if (++xs == p.nx) { xs = 0; xph ^= 1; }
-                    for (int ks = ks0; ks < ks1; ks++, xdesc += kunits) {
-                        if (!(ok = mbar_wait_hint(a_hint, bar_aready + 8 * as, aph, abort_flag))) break;
+                    for (int j = min(left, p.xk); j > 0; j -= RS, xdesc += RS * kunits) {
+                        if (!(ok = mbar_wait_hint(a_hint, bar_aready + 8 / RS * as, aph, abort_flag))) break;
                         const uint32_t ta = tmem_a + as * 32, done = bar_aempty + 8 * as;
-                        if (++as == na) { as = 0; aph ^= 1; }
-                        a_hint = mbar_test(bar_aready + 8 * as, aph);
-                        if (ks + 1 == ks1) x_hint = mbar_test(bar_xfull + 8 * xs, xph);
                         tc_fence_after();
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, ks != t.ks0 || kk != 0 ? 1u : 0u);
-                        umma_commit(done);
+                        for (int kk = 0; kk < 4; kk++) {
+                            umma_f16_ta<PAIR>(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, more);
+                            more = 1;
+                        }
+                        commit(done);
+                        if (RS == 2) {
+                            if (j >= 2) {
+#pragma unroll
+                                for (int kk = 0; kk < 4; kk++)
+                                    umma_f16_ta<PAIR>(td, ta + 32 + 8 * kk, kTaDescHi | (uint64_t)(xdesc + kunits + 2 * kk), idesc, 1u);
+                            }
+                            commit(done + 8);
+                        }
+                        if (j <= RS) commit(xdone);
+                        as += RS;
+                        if (as == na) { as = 0; aph ^= 1; }
+                        a_hint = mbar_test(bar_aready + 8 / RS * as, aph);
+                        if (j <= RS) x_hint = mbar_test(bar_xfull + 8 * xs, xph);
                     }
-                    umma_commit(xdone);
                 }
-                if (ok) umma_commit(bar_tfull + 8 * acc);
+                if (ok) commit(bar_tfull + 8 * acc);
                 acc ^= 1;
                 if (acc == 0) tph ^= 1;
             }
@@ -614,24 +667,31 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                             sc = lds_u16(scales + 2 * (FMT == kFmtTernary ? j >> 1 : j));
                             if (F::BIAS) bi = lds_u16(scales + 128 * SPB + 2 * j);
                         }
-                        ok = __all_sync(0xffffffffu, a_hint || mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
-                        if (!ok) break;
-                        tc_fence_after();
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            uint32_t o[16];
+                        uint32_t o[2][16];
+                        auto convert = [&](int h) {
                             // groups of 32 (g32: 16 bits each; mxfp4: 8 bits each) have a scale per half
                             const uint32_t sch = FMT == kFmtAffine4G32 ? sc & 0xFFFFu : (FMT == kFmtMxfp4 ? sc & 0xFFu : sc);
                             ta_dequant32<FMT>(codes, (uint32_t)(j * (F::BPS / 16) + (FMT == kFmtTernary ? 0 : h * (F::BPS / 32))), h, sw, sch,
-                                              FMT == kFmtAffine4G32 ? bi & 0xFFFFu : bi, o);
-                            tmem_st16(my_a + as * 32 + h * 16, o);
+                                              FMT == kFmtAffine4G32 ? bi & 0xFFFFu : bi, o[h]);
                             if (FMT == kFmtAffine4G32) { sc >>= 16; bi >>= 16; }
                             if (FMT == kFmtMxfp4) sc >>= 8;
-                        }
+                        };
+                        // Converted before the wait where the registers allow it: a stage's turn-around is then a store, not a conversion
+                        if (RS == 2) { convert(0); convert(1); }
+                        ok = __all_sync(0xffffffffu, a_hint || mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (RS == 1) convert(0);
+                        tmem_st16(my_a + as * 32, o[0]);
+                        if (RS == 1) convert(1);
+                        tmem_st16(my_a + as * 32 + 16, o[1]);
                         tmem_st_wait();
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_aready + 8 * as);
+                        if (lane == 0) {
+                            if (PAIR && rank != 0) mbar_arrive_remote_done(bar_aready + 8 * (as / RS), 0);
+                            else mbar_arrive(bar_aready + 8 * (as / RS));
+                        }
                     }
                     if (!ok) break;
                 }
@@ -639,7 +699,17 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                 if (lane == 0) mbar_arrive(bar_cempty + 8 * cs);
                 if (++cs == p.nc) { cs = 0; cph ^= 1; }
             }
-            it0 += steps;
+            if (RS == 2 && (steps & 1)) {  // an odd number of steps: the second of the last two A stages holds nothing, but its group reports it
+                const uint32_t it = it0 + steps, as = it & (na - 1), aph = (it >> nash) & 1;
+                if (ok && (int)(it & (GROUPS - 1)) == grp) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
+                    if (ok && lane == 0) {
+                        if (PAIR && rank != 0) mbar_arrive_remote_done(bar_aready + 8 * (as / RS), 0);
+                        else mbar_arrive(bar_aready + 8 * (as / RS));
+                    }
+                }
+            }
+            it0 += (steps + RS - 1) & ~(RS - 1);
         }
     } else {
         // ================= epilogue (warps 4-7) =================
@@ -659,7 +729,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             const uint32_t td = tmem + acc * p.dcols + ((uint32_t)(32 * q) << 16);
             constexpr int CW = 16;  // token columns at a time
             const int slot = i < sched->np ? sched->piece[i].slot : -1;
-            float4* const part = reinterpret_cast<float4*>(p.part) + (size_t)slot * (ta_slot(p.tile_rows) / 4) + q * (ta_slot(p.tile_rows) / 16) + lane;
+            float4* const part = reinterpret_cast<float4*>(p.part) + ((size_t)slot * CTAS + rank) * (ta_slot(p.tile_rows) / 4) + q * (ta_slot(p.tile_rows) / 16) + lane;
             for (int c0 = 0; c0 < rows; c0 += CW) {
                 uint32_t r[CW];
                 tmem_ld16(td + c0, r);
@@ -678,7 +748,10 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+            if (lane == 0) {
+                if (PAIR && rank != 0) mbar_arrive_remote(bar_tempty + 8 * acc, 0);
+                else mbar_arrive(bar_tempty + 8 * acc);
+            }
             acc ^= 1;
             if (acc == 0) tph ^= 1;
         }
@@ -692,10 +765,12 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync_all();  // (the other CTA's MMAs read this one's memory, its arrivals go to this one's barriers)
     if (*abort_flag && threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, kErrTimeout);
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
     }
 }
 
@@ -710,9 +785,10 @@ __global__ void __launch_bounds__(256) ta_sum_kernel(const TaParams p) {
     const TaSplit& sp = p.split;
     const int cols = (p.tile_rows + 3) / 4, lane = threadIdx.x & 31;
     const int slot4 = ta_slot(p.tile_rows) / 4;
-    for (int w = blockIdx.x * 8 + (threadIdx.x >> 5); w < sp.tiles * cols * 4; w += gridDim.x * 8) {
-        const int q = w & 3, c4 = (w >> 2) % cols, t = (w >> 2) / cols;
-        const int row0 = (t % m_tiles) * p.tile_rows, rows = min(p.tile_rows, p.M - row0), n0 = (t / m_tiles) * NROWS;
+    const int ctas = p.pair ? 2 : 1, quarters = 4 * ctas;
+    for (int w = blockIdx.x * 8 + (threadIdx.x >> 5); w < sp.tiles * cols * quarters; w += gridDim.x * 8) {
+        const int q = w & 3, rank = (w % quarters) >> 2, c4 = w / quarters % cols, t = w / quarters / cols;
+        const int row0 = (t % m_tiles) * p.tile_rows, rows = min(p.tile_rows, p.M - row0), n0 = ((t / m_tiles) * ctas + rank) * NROWS;
         int a, b, slot0;
         ta_split_tile(sp, t, a, b, slot0);
         if (b - a == 1 || 4 * c4 >= rows) continue;
@@ -720,11 +796,11 @@ __global__ void __launch_bounds__(256) ta_sum_kernel(const TaParams p) {
         const bool n_ok = n < p.N;
         const float* eb = mi ? p.ebias[1] : p.ebias[0];
         const float bias = eb != nullptr && n_ok ? eb[n] : 0.f;
-        const float4* s = reinterpret_cast<const float4*>(p.part) + q * (slot4 / 4) + c4 * 32 + lane;
+        const float4* s = reinterpret_cast<const float4*>(p.part) + rank * slot4 + q * (slot4 / 4) + c4 * 32 + lane;
         float4 f[kTaSplitPieces + 2];  // (a run that starts inside the tile's neighbour makes one piece more)
 #pragma unroll
         for (int k = 0; k < kTaSplitPieces + 2; k++)
-            if (a + k < b) f[k] = s[(size_t)(k == 0 ? slot0 : a + k) * slot4];
+            if (a + k < b) f[k] = s[(size_t)(k == 0 ? slot0 : a + k) * ctas * slot4];
         float v[4] = {f[0].x, f[0].y, f[0].z, f[0].w};
 #pragma unroll
         for (int k = 1; k < kTaSplitPieces + 2; k++)

@@ -520,3 +520,13 @@ def test_router_tiled_float64_gemm(cuda_device, kind, E, D, T):
     assert np.array_equal(got[:, :E], logits) and not got[:, E:].any()
     inds, _ = qref.route(logits, K, sigmoid=kind == "sigmoid")
     assert np.array_equal(v["inds"].cpu().numpy().astype(np.uint32), inds)
+
+
+@pytest.mark.parametrize("fmt,act", [("affine", "silu"), ("mxfp4", "swiglu_oai")])
+@pytest.mark.parametrize("D,I,T", [(448, 576, 900), (192, 64, 3000)])
+def test_moe_tall_tiles_on_pairs(cuda_device, fmt, act, D, I, T):
+    """Tiles of up to 192 rows run on pairs of CTAs: widths that fill a pair's features in part, or only its first CTA's, tiles of a
+    few rows among full ones, odd numbers of K steps."""
+    rng = np.random.default_rng(91 + D + T)
+    layer, host = build_layer(rng, cuda_device, 32, 4, D, I, fmt=fmt, act=act, biases=fmt == "mxfp4", max_tokens=T)
+    check_layer(layer, host, synth.activations_np(rng, T, D), T, act)

@@ -234,3 +234,25 @@ def test_dense_ffn_split_along_k(cuda_device, rows, d, d_ff, act):
         h = (u + 1) * g / (1 + torch.exp(-1.702 * g))
     ref = h.to(torch.float16).double() @ w[1].T
     assert float((out - ref).abs().max() / ref.abs().max()) <= TOL
+
+
+@pytest.mark.parametrize("fmt,group", [("q4", 64), ("q8", 64), ("q4", 32), ("mxfp4", 32)])
+@pytest.mark.parametrize("M,N,K", [(4096, 2112, 832), (2048, 192, 1088), (1088, 14400, 320), (4096, 64, 64), (192, 9600, 2112)])
+def test_qmm_pairs_of_ctas(cuda_device, fmt, group, M, N, K):
+    """Tall calls run on pairs of CTAs with twice the features per tile: features that fill half a pair, one CTA of a pair or none of
+    its second one, token tiles whose halves differ, odd numbers of K steps; the same bits every time, and added onto a result."""
+    rng = np.random.default_rng(81 + M + N + K + group)
+    bits = 8 if fmt == "q8" else 4
+    m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, bits, cuda_device, group=group)
+    x = synth.activations_np(rng, M, K)
+    xt = x_tensor(x, cuda_device)
+    y = run_qmm(m, xt, M)
+    sel = np.unique(np.concatenate([np.sort(rng.choice(N, size=min(N, 64), replace=False)), np.arange(max(0, N - 16), N)]))
+    rows = np.unique(np.concatenate([np.sort(rng.choice(M, size=64, replace=False)), np.arange(M - 16, M)]))
+    ref = qref.matmul_t(x[rows], deq(tuple(h[:, sel] for h in host), bits, group=group))
+    got = y[torch.from_numpy(rows).to(cuda_device)][:, torch.from_numpy(sel).to(cuda_device)].cpu().numpy()
+    assert qref.max_rel(got, ref) <= TOL
+    assert bool(torch.isfinite(y).all())
+    for _ in range(3):
+        assert torch.equal(run_qmm(m, xt, M), y)
+    assert torch.equal(run_qmm(m, xt, M, accumulate=True, y=y.clone()), 2 * y)
