@@ -433,10 +433,8 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
                                 for (int c = 0; c < NS; c++) {
                                     const float v0 = (float)(d[i][c][0] * 256 + d[i][c][1]);
                                     const float v1 = (float)(d[i][c][2] * 256 + d[i][c][3]);
-                                    acc[i][c][0] = fmaf(v0, sc0 * xs[c].x, acc[i][c][0]);
-                                    acc[i][c][0] = fmaf(bi0, xs[c].y, acc[i][c][0]);
-                                    acc[i][c][1] = fmaf(v1, sc1 * xs[c].x, acc[i][c][1]);
-                                    acc[i][c][1] = fmaf(bi1, xs[c].y, acc[i][c][1]);
+                                    scaled_add2(acc[i][c][0], acc[i][c][1], v0, v1, sc0, sc1, xs[c].x, xs[c].x);
+                                    fma2(acc[i][c][0], acc[i][c][1], bi0, bi1, xs[c].y, xs[c].y);
                                 }
                             }
                         }
