@@ -199,7 +199,7 @@ __device__ __forceinline__ bool qi_consumer_barrier_or(int threads, bool pred) {
 // when known at compile time (the activation fragments of the warp's K slice then live in registers across all row
 // blocks), 0 when not.
 template <int FMT, int MS, int GW, bool TM = false>
-__global__ void __launch_bounds__(kQiMaxThreads, MS == 1 ? 2 : 1)
+__global__ void __launch_bounds__(kQiMaxThreads, 2)
     qmv_imma_kernel(const __grid_constant__ CUtensorMap wmap, const QiParams p) {
     constexpr bool W6 = FMT == kFmtAffine6;
     // W8: one code per operand byte, lane t of a quad owns inputs 16t..16t+15 of a group (8-bit codes as they are, 6-bit
