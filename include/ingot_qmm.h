@@ -127,7 +127,8 @@ int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_
  * x of dtype bf16/f32 is converted to fp16 into the workspace first; fp16 x is used in place. Where the tiles fill the GPU's SMs
  * badly, some are divided along k and their partial sums go through the workspace, behind the converted rows (round(rows * k * 2,
  * 256) bytes, none for fp16): iq_qmm_workspace_bytes asks for both, and a workspace that holds the converted rows only is
- * accepted as well (the same products, summed in another order). */
+ * accepted as well (the same products, summed in another order). The answer is enough for every call of up to `rows` rows of that
+ * x_dtype and never falls as rows grows, so that one buffer sized for the most rows serves all calls. */
 int32_t iq_qmm_workspace_bytes(iq_ctx* ctx, const iq_qlinear* m, int32_t rows, int32_t x_dtype, size_t* bytes);
 int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
                int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, void* workspace, size_t workspace_bytes);
@@ -146,6 +147,21 @@ int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_
  *     it — keep them on one stream or order them. Nothing in it has to be cleared between calls. */
 int32_t iq_qmm_noalloc(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m,
                        void* y, int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags);
+
+/* How iq_qmm (gate_up == 0) divides a call among the SMs of a GPU, and what the gate/up half of iq_dense_ffn does with the
+ * concatenated matrix m (gate_up != 0). Needs no GPU and no context, reads n, k, bits, group and mode of m only. No counterpart in the
+ * reference: for tests that have to know which path a shape takes, and for sizing. */
+typedef struct iq_qmm_tiling {
+    int32_t tile_rows;       /* token rows per tile */
+    int32_t tiles;           /* all tiles */
+    int32_t pair;            /* 1: a tile is two CTAs' work */
+    int32_t two_per_sm;      /* 1: two CTAs per SM */
+    int32_t split_tiles;     /* tiles divided along k (0: none), */
+    int32_t split_ctas;      /* and the CTAs (pairs) that share them */
+    size_t split_bytes;      /* partial sums of this call, */
+    size_t bytes_up_to_rows; /* and the most that a call of up to `rows` rows takes */
+} iq_qmm_tiling;
+int32_t iq_qmm_plan(const iq_qlinear* m, int32_t gate_up, int32_t rows, int32_t sms, iq_qmm_tiling* out);
 
 /* Rotated W8A8 prefill GEMM (lossy; an option of the serving path, not the default). Replaces DenseQ.encodeQmmI8(ctx, enc,
  * x:, y:, rows:, scratch:, accumulate:, halfOut:) (Sources/Ingot/Layers/Dense.swift:99-172) and w4_i8rot /
@@ -169,7 +185,7 @@ int32_t iq_qmm_w8a8(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, i
  * out[rows, d] (+)= down( act(gate x) * up x ) with gate|up concatenated by rows as one [2*d_ff, d] matrix (gate rows
  * first). Replaces DenseMLP.encode / encodePrefill (Sources/Ingot/Layers/Dense.swift:56-96) and dswiglu*
  * (Shaders/yy_model.metal:187-227). rows <= 16 takes the GEMV path, larger multiples of 64 the GEMM path. The workspace is
- * 16-byte aligned. */
+ * 16-byte aligned; as for iq_qmm, its size never falls as rows grows. */
 int32_t iq_dense_ffn_workspace_bytes(iq_ctx* ctx, const iq_qlinear* gate_up, const iq_qlinear* down, int32_t rows,
                                      int32_t x_dtype, size_t* bytes);
 int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* gate_up,

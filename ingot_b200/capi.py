@@ -33,13 +33,18 @@ SYMBOLS = [
     "iq_scales_div16_bf16", "iq_argmax_rows", "iq_topk64_scratch_bytes", "iq_topk64", "iq_embed_rows",
     "iq_ctx_set_wait_cycles", "iq_colsplit_create", "iq_colsplit_destroy", "iq_linear_colsplit_workspace_bytes",
     "iq_linear_colsplit", "iq_had_rows", "iq_embed_rows_ternary", "iq_qmm_w8a8_workspace_bytes", "iq_qmm_w8a8",
-    "iq_ep_index", "iq_moe_experts_indexed", "iq_ep_pack_push_tokens", "iq_ep_index_tokens",
+    "iq_qmm_plan", "iq_ep_index", "iq_moe_experts_indexed", "iq_ep_pack_push_tokens", "iq_ep_index_tokens",
 ]
 
 
 class QLinear(C.Structure):
     _fields_ = [("w", C.c_void_p), ("scales", C.c_void_p), ("biases", C.c_void_p), ("n", C.c_int32), ("k", C.c_int32),
                 ("bits", C.c_int32), ("group", C.c_int32), ("mode", C.c_int32), ("experts", C.c_int32)]
+
+
+class QmmTiling(C.Structure):
+    _fields_ = [("tile_rows", C.c_int32), ("tiles", C.c_int32), ("pair", C.c_int32), ("two_per_sm", C.c_int32),
+                ("split_tiles", C.c_int32), ("split_ctas", C.c_int32), ("split_bytes", C.c_size_t), ("bytes_up_to_rows", C.c_size_t)]
 
 
 class MoeDesc(C.Structure):
@@ -96,6 +101,8 @@ def lib() -> C.CDLL:
         l.iq_ctx_status.restype = i32
         l.iq_qmv.argtypes = [vp, vp, vp, i32, i64, C.POINTER(QLinear), vp, i32, i64, i32, u32, i32]
         l.iq_qmm_workspace_bytes.argtypes = [vp, C.POINTER(QLinear), i32, i32, C.POINTER(sz)]
+        l.iq_qmm_plan.argtypes = [C.POINTER(QLinear), i32, i32, i32, C.POINTER(QmmTiling)]
+        l.iq_qmm_plan.restype = i32
         l.iq_qmm.argtypes = [vp, vp, vp, i32, i64, C.POINTER(QLinear), vp, i32, i64, i32, u32, vp, sz]
         l.iq_dense_ffn_workspace_bytes.argtypes = [vp, C.POINTER(QLinear), C.POINTER(QLinear), i32, i32, C.POINTER(sz)]
         l.iq_dense_ffn.argtypes = [vp, vp, vp, i32, i64, C.POINTER(QLinear), C.POINTER(QLinear), i32, C.c_float, vp,
@@ -245,6 +252,15 @@ class Context:
             self.close()
         except Exception:
             pass
+
+
+def qmm_plan(n: int, k: int, bits: int, group: int, rows: int, mode: int = IQ_MODE_AFFINE, gate_up: bool = False, sms: int = 148) -> QmmTiling:
+    """How a prefill GEMM of this shape is divided (iq_qmm_plan); needs no GPU."""
+    out = QmmTiling()
+    st = lib().iq_qmm_plan(C.byref(QLinear(0, 0, 0, n, k, bits, group, mode, 1)), int(gate_up), rows, sms, C.byref(out))
+    if st != 0:
+        raise IngotError(st, lib().iq_strerror(st).decode())
+    return out
 
 
 _contexts = {}

@@ -137,6 +137,7 @@ struct QmmSplit {
     size_t bytes = 0;
 };
 QmmSplit qmm_split(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K, void* scratch, size_t bytes);
+size_t qmm_split_bound(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K);  // of any call of up to M rows: never falls as M grows
 size_t qmm_split_max_bytes(iq_ctx* ctx);  // of any dense GEMM
 int32_t launch_convert_x(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, void* out, int rows, int k);
 size_t qmm_convert_bytes(int rows, int k, int32_t x_dtype);

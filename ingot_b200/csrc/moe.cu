@@ -478,34 +478,43 @@ using namespace iq;
 namespace {
 // Scratch of the GEMM path: h fp16 | converted x | (ternary: gate|up fp32) | partial sums of the GEMMs' K splits
 struct FfnWs {
-    size_t convert, need, bytes;  // offset of the converted x; without the partial sums (their offset); with them
+    size_t convert, need;  // offset of the converted x; of the partial sums (the scratch without them)
+    bool fused;            // gate/up with the activation in its epilogue
 };
-FfnWs ffn_ws(iq_ctx* ctx, const iq_qlinear* gate_up, const iq_qlinear* down, int rows, int32_t x_dtype) {
+FfnWs ffn_ws(const iq_qlinear* gate_up, const iq_qlinear* down, int rows, int32_t x_dtype) {
     FfnWs w;
     const int32_t fmt = format_of(gate_up);
     const size_t d_ff = down->k;
     w.convert = round_up_sz((size_t)rows * d_ff * 2, 256);
     w.need = w.convert + round_up_sz(qmm_convert_bytes(rows, gate_up->k, x_dtype), 256);
-    const bool fused = fmt != kFmtTernary && fmt != kFmtAffine6;
-    if (!fused) w.need += round_up_sz((size_t)rows * 2 * d_ff * 4, 256);
-    w.bytes = w.need + std::max(qmm_split(ctx, fmt, fused, rows, fused ? (int)d_ff : gate_up->n, gate_up->k, nullptr, 0).bytes,
-                                qmm_split(ctx, format_of(down), 0, rows, down->n, down->k, nullptr, 0).bytes);
+    w.fused = fmt != kFmtTernary && fmt != kFmtAffine6;
+    if (!w.fused) w.need += round_up_sz((size_t)rows * 2 * d_ff * 4, 256);
     return w;
+}
+// ... of the GEMV path (up to 16 rows): h fp16 | x, then h, as block fixed point
+size_t ffn_small_ws(const iq_qlinear* gate_up, const iq_qlinear* down, int rows) {
+    const size_t d_ff = down->k;
+    return round_up_sz((size_t)rows * d_ff * 2, 256) + round_up_sz((size_t)rows * std::max(d_ff, (size_t)gate_up->k) / 2 * 7, 256);
+}
+int32_t ffn_chain_check(iq_ctx* ctx, const iq_qlinear* gate_up, const iq_qlinear* down) {
+    if (ctx == nullptr || gate_up == nullptr || down == nullptr) return kErrInvalidArg;
+    if (gate_up->n % 2 != 0 || gate_up->n / 2 != down->k || gate_up->k != down->n)
+        return fail(ctx, kErrInvalidArg, "dense_ffn: gate|up [%d, %d] and down [%d, %d] do not chain", gate_up->n,
+                    gate_up->k, down->n, down->k);
+    return kOk;
 }
 }  // namespace
 
 extern "C" int32_t iq_dense_ffn_workspace_bytes(iq_ctx* ctx, const iq_qlinear* gate_up, const iq_qlinear* down,
                                                 int32_t rows, int32_t x_dtype, size_t* bytes) {
-    if (ctx == nullptr || gate_up == nullptr || down == nullptr || bytes == nullptr) return kErrInvalidArg;
-    if (gate_up->n % 2 != 0 || gate_up->n / 2 != down->k || gate_up->k != down->n)
-        return fail(ctx, kErrInvalidArg, "dense_ffn: gate|up [%d, %d] and down [%d, %d] do not chain", gate_up->n,
-                    gate_up->k, down->n, down->k);
-    if (rows <= 16) {
-        const size_t d_ff = down->k;
-        *bytes = round_up_sz((size_t)rows * d_ff * 2, 256) +                                     // h fp16
-                 round_up_sz((size_t)rows * std::max(d_ff, (size_t)gate_up->k) / 2 * 7, 256);  // x, then h, as block fixed point
-    } else {
-        *bytes = ffn_ws(ctx, gate_up, down, rows, x_dtype).bytes;
+    const int32_t st = bytes == nullptr ? kErrInvalidArg : ffn_chain_check(ctx, gate_up, down);
+    if (st != kOk) return st;
+    // never less than a smaller call takes
+    *bytes = ffn_small_ws(gate_up, down, std::min(rows, 16));
+    if (rows > 16) {
+        const FfnWs w = ffn_ws(gate_up, down, rows, x_dtype);
+        *bytes = std::max(*bytes, w.need + std::max(qmm_split_bound(ctx, format_of(gate_up), w.fused, rows, w.fused ? down->k : gate_up->n, gate_up->k),
+                                                    qmm_split_bound(ctx, format_of(down), 0, rows, down->n, down->k)));
     }
     return kOk;
 }
@@ -514,14 +523,11 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
                                 const iq_qlinear* gate_up, const iq_qlinear* down, int32_t act, float act_limit, void* out,
                                 int32_t out_dtype, int64_t ldo, int32_t rows, uint32_t flags, void* workspace,
                                 size_t workspace_bytes) {
-    size_t need = 0;
-    int32_t st = iq_dense_ffn_workspace_bytes(ctx, gate_up, down, rows, x_dtype, &need);
+    int32_t st = ffn_chain_check(ctx, gate_up, down);
     if (st != kOk) return st;
-    FfnWs ws = {};
-    if (rows > 16) {
-        ws = ffn_ws(ctx, gate_up, down, rows, x_dtype);
-        need = ws.need;  // (a workspace without room for the K splits is good as well: every tile is one item then)
-    }
+    const FfnWs ws = ffn_ws(gate_up, down, rows, x_dtype);
+    // (a workspace without room for the K splits is good as well: every tile is one item then)
+    const size_t need = rows <= 16 ? ffn_small_ws(gate_up, down, rows) : ws.need;
     if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0)
         return fail(ctx, kErrWorkspace, "dense_ffn: workspace %zu < %zu (16-byte aligned)", workspace_bytes, need);
     if (act < IQ_ACT_SILU || act > IQ_ACT_RELU2) return fail(ctx, kErrUnsupported, "dense_ffn: activation %d", act);
@@ -570,11 +576,8 @@ extern "C" int32_t iq_dense_ffn(iq_ctx* ctx, void* stream, const void* x, int32_
         char* base = static_cast<char*>(workspace);
         const void* x16 = x;
         int64_t ld16 = ldx;
-        QmmSplit gu, dn;
-        if (workspace_bytes >= ws.bytes) {
-            gu = qmm_split(ctx, fmt, 1, rows, d_ff, gate_up->k, base + ws.need, ws.bytes - ws.need);
-            dn = qmm_split(ctx, format_of(down), 0, rows, down->n, down->k, base + ws.need, ws.bytes - ws.need);
-        }
+        const QmmSplit gu = qmm_split(ctx, fmt, 1, rows, d_ff, gate_up->k, base + ws.need, workspace_bytes - ws.need);
+        const QmmSplit dn = qmm_split(ctx, format_of(down), 0, rows, down->n, down->k, base + ws.need, workspace_bytes - ws.need);
         if (x_dtype != IQ_F16) {
             if (ldx < gate_up->k || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
                 return fail(ctx, kErrInvalidArg, "dense_ffn: x must be 16-byte aligned with ldx >= d and ldx %% 8 == 0");

@@ -106,6 +106,29 @@ TaPlan ta_plan(int32_t fmt, int epi, int M, int N, int K, int sms, bool may_spli
     return best;
 }
 
+// What the split of any call of up to M rows takes at most. The split of one call is no measure of a shorter one's (4096 x 14336:
+// 39 MiB of FFN scratch at 512 rows, 28 at 640), and a buffer sized for the most rows has to serve them all. Per height, more tiles mean more
+// slots until the split no longer pays, so the largest number of tiles for which it does is searched by halving.
+size_t ta_split_bound(int32_t fmt, int epi, int M, int N, int K, int sms) {
+    const int features = epi ? 64 : 128, ksteps = K / 64;
+    size_t most = 0;
+    for (int rows = 16; rows <= std::min(kTaMaxRows, round_up(M, 16)); rows += 16)
+        for (int kind = 0; kind < 3; kind++) {  // one CTA, a pair, two CTAs per SM
+            const bool pair = kind == 1, low = kind == 2;
+            if ((pair && sms % 2 != 0) || (low && rows > kTaLowRows)) continue;
+            const int ctas = pair ? sms / 2 : low ? 2 * sms : sms, ustep = ta_ustep(fmt, ta_xk(low, rows));
+            const int64_t total = (int64_t)((M + rows - 1) / rows) * ((N + (features << pair) - 1) / (features << pair));
+            int lo = 0, hi = (int)std::min<int64_t>(total, ctas - 1);  // tiles of the last round: the split pays for lo of them
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) / 2;
+                if (ta_split(mid, ctas, ksteps, ustep, rows, low, pair).tiles != 0) lo = mid;
+                else hi = mid - 1;
+            }
+            if (lo != 0) most = std::max(most, ta_split_bytes(ta_split(lo, ctas, ksteps, ustep, rows, low, pair), rows, pair));
+        }
+    return round_up_sz(most, 256);
+}
+
 }  // namespace
 
 int32_t qmm_init(iq_ctx* ctx) {
@@ -341,6 +364,9 @@ QmmSplit qmm_split(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K, void*
     if (r.bytes != 0 && bytes >= r.bytes && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0) r.part = static_cast<float*>(scratch);
     return r;
 }
+size_t qmm_split_bound(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K) {
+    return fmt < 0 || fmt == kFmtAffine6 || fmt > kFmtTernary ? 0 : ta_split_bound(fmt, epi, M, N, K, ctx->sms);
+}
 size_t qmm_split_max_bytes(iq_ctx* ctx) { return (size_t)2 * ctx->sms * ta_slot(kTaMaxRows) * 4; }  // (two CTAs per SM: slots of a third)
 size_t qmm_convert_bytes(int rows, int k, int32_t x_dtype) { return x_dtype == IQ_F16 ? 0 : round_up_sz((size_t)rows * k * 2, 256); }
 
@@ -350,7 +376,21 @@ extern "C" int32_t iq_qmm_workspace_bytes(iq_ctx* ctx, const iq_qlinear* m, int3
     if (ctx == nullptr || m == nullptr || bytes == nullptr || rows < 1) return kErrInvalidArg;
     // The MMA takes fp16 weights with fp16 activations only (a bf16 B operand beside an fp16 A operand is an illegal
     // instruction on sm_100a: kind::f16 wants both operands of one type), so bf16 and fp32 activations are converted
-    *bytes = qmm_convert_bytes(rows, m->k, x_dtype) + qmm_split(ctx, format_of(m), 0, rows, m->n, m->k, nullptr, 0).bytes;
+    *bytes = qmm_convert_bytes(rows, m->k, x_dtype) + qmm_split_bound(ctx, format_of(m), 0, rows, m->n, m->k);
+    return kOk;
+}
+
+extern "C" int32_t iq_qmm_plan(const iq_qlinear* m, int32_t gate_up, int32_t rows, int32_t sms, iq_qmm_tiling* out) {
+    if (m == nullptr || out == nullptr || rows < 1 || sms < 1 || m->n < 1 || m->k < 64 || (gate_up && m->n % 2 != 0)) return kErrInvalidArg;
+    const int32_t fmt = format_of(m);
+    if (fmt < 0 || fmt == kFmtAffine6 || (gate_up && fmt == kFmtTernary)) return kErrUnsupported;
+    const int n = gate_up ? m->n / 2 : m->n;
+    const TaPlan p = ta_plan(fmt, gate_up != 0, rows, n, m->k, sms, true);
+    out->tile_rows = p.rows; out->tiles = (rows + p.rows - 1) / p.rows * p.n_tiles;
+    out->pair = p.pair; out->two_per_sm = p.low;
+    out->split_tiles = p.split.tiles; out->split_ctas = p.split.ctas;
+    out->split_bytes = round_up_sz(ta_split_bytes(p.split, p.rows, p.pair), 256);
+    out->bytes_up_to_rows = ta_split_bound(fmt, gate_up != 0, rows, n, m->k, sms);
     return kOk;
 }
 

@@ -256,3 +256,32 @@ def test_qmm_pairs_of_ctas(cuda_device, fmt, group, M, N, K):
     for _ in range(3):
         assert torch.equal(run_qmm(m, xt, M), y)
     assert torch.equal(run_qmm(m, xt, M, accumulate=True, y=y.clone()), 2 * y)
+
+
+def test_dense_ffn_scratch_outlives_fewer_rows(cuda_device):
+    """Scratch sized by the largest call serves all smaller ones: a captured graph's addresses stay the module's own when fewer rows,
+    whose GEMMs divide along K in more pieces, follow."""
+    d, d_ff = 2048, 7680
+    rng = np.random.default_rng(73)
+    gu, _ = affine_case(rng, 2 * d_ff, d, 8, cuda_device)
+    dn, _ = affine_case(rng, d, d_ff, 8, cuda_device)
+    assert capi.qmm_plan(d, d_ff, 8, 64, 640).split_bytes < capi.qmm_plan(d, d_ff, 8, 64, 512).split_bytes
+    mlp = DenseMLP(gu, dn)
+    x = x_tensor(synth.activations_np(rng, 640, d), cuda_device)
+    want = torch.zeros(640, d, dtype=torch.float32, device=cuda_device)
+    mlp.encode(x, want, 640)
+    at = mlp._ws.data_ptr()
+    got = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        mlp.encode(x, got, 640)
+    for rows in (512, 320, 256, 64, 16, 3):
+        out = torch.zeros(rows, d, dtype=torch.float32, device=cuda_device)
+        mlp.encode(x[:rows], out, rows)
+        assert mlp._ws.data_ptr() == at
+        assert qref.max_rel(out.cpu().numpy(), want[:rows].cpu().numpy()) <= TOL
+    g.replay()
+    assert torch.equal(got, want)
+    for fmt in (torch.bfloat16, torch.float16):
+        assert dn.qmm_workspace_bytes(4096, fmt) >= max(dn.qmm_workspace_bytes(r, fmt) for r in range(64, 4096, 64))
