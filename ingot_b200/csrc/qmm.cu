@@ -93,7 +93,8 @@ TaPlan ta_plan(int32_t fmt, int epi, int M, int N, int K, int sms, bool may_spli
             p.low = !pair && rows <= kTaLowRows && total > sms;
             const int ctas = pair ? sms / 2 : p.low ? 2 * sms : sms;
             p.ustep = ta_ustep(fmt, ta_xk(p.low, rows));
-            p.split = may_split ? ta_split(total, ctas, ksteps, p.ustep, rows, p.low, p.pair) : TaSplit{0, 0, 0};
+            // (two CTAs per SM: never divided. Of 14,000 shapes asked none was, and the low kernel is faster without the code)
+            p.split = may_split && !p.low ? ta_split(total, ctas, ksteps, p.ustep, rows, p.pair) : TaSplit{0, 0, 0};
             const double step = ta_step_cycles(rows, p.low, p.pair);
             double cost = (double)((total - p.split.tiles + ctas - 1) / ctas) * ksteps * step + (pair ? 1500 : 0);  // (a pair's start)
             if (p.split.tiles)
@@ -113,18 +114,16 @@ size_t ta_split_bound(int32_t fmt, int epi, int M, int N, int K, int sms) {
     const int features = epi ? 64 : 128, ksteps = K / 64;
     size_t most = 0;
     for (int rows = 16; rows <= std::min(kTaMaxRows, round_up(M, 16)); rows += 16)
-        for (int kind = 0; kind < 3; kind++) {  // one CTA, a pair, two CTAs per SM
-            const bool pair = kind == 1, low = kind == 2;
-            if ((pair && sms % 2 != 0) || (low && rows > kTaLowRows)) continue;
-            const int ctas = pair ? sms / 2 : low ? 2 * sms : sms, ustep = ta_ustep(fmt, ta_xk(low, rows));
+        for (int pair = 0; pair < (sms % 2 == 0 ? 2 : 1); pair++) {
+            const int ctas = pair ? sms / 2 : sms, ustep = ta_ustep(fmt, ta_xk(false, rows));
             const int64_t total = (int64_t)((M + rows - 1) / rows) * ((N + (features << pair) - 1) / (features << pair));
             int lo = 0, hi = (int)std::min<int64_t>(total, ctas - 1);  // tiles of the last round: the split pays for lo of them
             while (lo < hi) {
                 const int mid = (lo + hi + 1) / 2;
-                if (ta_split(mid, ctas, ksteps, ustep, rows, low, pair).tiles != 0) lo = mid;
+                if (ta_split(mid, ctas, ksteps, ustep, rows, pair).tiles != 0) lo = mid;
                 else hi = mid - 1;
             }
-            if (lo != 0) most = std::max(most, ta_split_bytes(ta_split(lo, ctas, ksteps, ustep, rows, low, pair), rows, pair));
+            if (lo != 0) most = std::max(most, ta_split_bytes(ta_split(lo, ctas, ksteps, ustep, rows, pair), rows, pair));
         }
     return round_up_sz(most, 256);
 }

@@ -42,7 +42,11 @@
 // dequantiser groups, half of the shared memory and 256 columns (two accumulators of 64, four A stages), run two such
 // chains side by side: 32 experts of 2880 x 2880 (MXFP4) at 64 tokens, gate/up 102 -> 78 us (3.6 TB/s) and down 53 -> 45;
 // 128 experts of 2048 x 768 (4 bits) at 200 tokens 100 -> 90 and 51 -> 46. Three groups per CTA were slower (48 registers).
-// What bounds it now is issue slots: 70 % busy, two thirds of them the conversion of the codes.
+// What bounds it now is issue slots: 70 % busy, two thirds of them the conversion of the codes. With 64 registers a thread it takes the
+// plainer form of what it shares with the tall tiles (SPLIT below): tile numbers for work items, no K split, codes converted half a step at a
+// time, an issuer that asks its barriers ahead of the MMAs, a guard per stored column. With the tall tiles' forms the MoE block of 32
+// experts of 2880 x 2880 (MXFP4, 64 tokens) took 140.8 instead of 137.8 us, 128 of 3584 x 768 at 16 tokens 125 instead of 118, 512 of 3264 x 640
+// (4 bits, 64 tokens) 553 instead of 538. The other way round, one issuer loop for both cost 64-row dense calls 5 to 20 %.
 // Every wait is bounded: on a timeout the kernel writes a status word, all roles drain and tensor memory is released.
 //
 // Replaces qmm_t_nax3* (Shaders/qmm_nax_v3.metal:107-256) and, with a tile list, moe_gateup_swiglu2* / moe_down2*
@@ -126,14 +130,14 @@ inline int ta_step_cycles(int rows, bool low, bool pair) {
     return pair ? 420 + over * 9 / 20 : low ? 880 + over * 2 : 400 + over;
 }
 inline long long ta_split_cycles(const TaSplit& s, int rows, bool pair) { return 7000 + (long long)(s.ctas + s.tiles) * rows * (pair ? 2048 : 1024) / 1900; }
-inline TaSplit ta_split(int total, int ctas, int ksteps, int ustep, int rows, bool low, bool pair) {
+inline TaSplit ta_split(int total, int ctas, int ksteps, int ustep, int rows, bool pair) {
     TaSplit r;
     r.units = (ksteps + ustep - 1) / ustep;
     r.tiles = total < ctas ? total : total % ctas;
     r.ctas = r.tiles * kTaSplitPieces < ctas ? r.tiles * kTaSplitPieces : ctas;
     if (r.tiles * r.units < r.ctas) r.ctas = r.tiles * r.units;
     // the round saved, less the CTA's share of it, has to be longer than what the split costs
-    if (r.tiles == 0 || (long long)(r.ctas - r.tiles) * ksteps * ta_step_cycles(rows, low, pair) <= ta_split_cycles(r, rows, pair) * r.ctas) r.tiles = r.ctas = 0;
+    if (r.tiles == 0 || (long long)(r.ctas - r.tiles) * ksteps * ta_step_cycles(rows, false, pair) <= ta_split_cycles(r, rows, pair) * r.ctas) r.tiles = r.ctas = 0;
     return r;
 }
 // What a CTA does, worked out once and read from shared memory at every item (in registers it made the roles' loops spill): its
@@ -284,27 +288,33 @@ __device__ __forceinline__ void ta_dequant32(uint32_t codes, uint32_t unit, int 
     }
 }
 
-// What becomes of CW token columns of a tile: v[j] is feature n of token row0 + j (gate/up: lanes l and l + 16 hold gate and up of
-// feature n) with the expert's bias, j < live.
+// The activation of CW token columns of a tile: lanes l and l + 16 hold gate and up of one feature; the lower lane finishes token j, the
+// upper token j + 1.
+template <int CW>
+__device__ __forceinline__ void ta_gated(const TaParams& p, const float (&v)[CW], int mi, float (&g)[CW / 2]) {
+    float u[CW / 2];
+#pragma unroll
+    for (int j = 0; j < CW / 2; j++) {
+        const float other = __shfl_xor_sync(0xffffffffu, mi ? v[2 * j] : v[2 * j + 1], 16);
+        g[j] = mi ? other : v[2 * j];
+        u[j] = mi ? v[2 * j + 1] : other;
+    }
+    auto act = [&](auto tag) {
+#pragma unroll
+        for (int j = 0; j < CW / 2; j++) g[j] = glu<decltype(tag)::value>(g[j], u[j], p.limit);
+    };
+    if (p.act == kActSilu) act(std::integral_constant<int, kActSilu>{});
+    else if (p.act == kActSwigluOai) act(std::integral_constant<int, kActSwigluOai>{});
+    else if (p.act == kActGelu) act(std::integral_constant<int, kActGelu>{});
+    else act(std::integral_constant<int, kActRelu2>{});
+}
+
+// What becomes of CW token columns of a tile: v[j] is feature n of token row0 + j (gate/up: ta_gated) with the expert's bias, j < live.
 template <int EPI, int CW>
 __device__ __forceinline__ void ta_store(const TaParams& p, float (&v)[CW], int row0, int n, bool n_ok, int live, int mi) {
     if (EPI) {
-        // the lower lane finishes token j, the upper token j + 1
-        float g[CW / 2], u[CW / 2];
-#pragma unroll
-        for (int j = 0; j < CW / 2; j++) {
-            const float other = __shfl_xor_sync(0xffffffffu, mi ? v[2 * j] : v[2 * j + 1], 16);
-            g[j] = mi ? other : v[2 * j];
-            u[j] = mi ? v[2 * j + 1] : other;
-        }
-        auto act = [&](auto tag) {
-#pragma unroll
-            for (int j = 0; j < CW / 2; j++) g[j] = glu<decltype(tag)::value>(g[j], u[j], p.limit);
-        };
-        if (p.act == kActSilu) act(std::integral_constant<int, kActSilu>{});
-        else if (p.act == kActSwigluOai) act(std::integral_constant<int, kActSwigluOai>{});
-        else if (p.act == kActGelu) act(std::integral_constant<int, kActGelu>{});
-        else act(std::integral_constant<int, kActRelu2>{});
+        float g[CW / 2];
+        ta_gated(p, v, mi, g);
         if (!n_ok) return;
         __half* yp = reinterpret_cast<__half*>(p.y) + (size_t)(row0 + mi) * p.ldy + n;
         const size_t step = 2 * p.ldy;
@@ -344,6 +354,37 @@ __device__ __forceinline__ void ta_store(const TaParams& p, float (&v)[CW], int 
     }
 }
 
+// The same with a guard per column instead of stepped pointers, for the low tiles' kernel: it has 64 registers a thread, and few of its
+// sets of 16 columns are full.
+template <int EPI, int CW>
+__device__ __forceinline__ void ta_store_low(const TaParams& p, float (&v)[CW], int row0, int n, bool n_ok, int live, int mi) {
+    if (EPI) {
+        float g[CW / 2];
+        ta_gated(p, v, mi, g);
+        __half* yp = reinterpret_cast<__half*>(p.y) + (size_t)(row0 + mi) * p.ldy + n;
+#pragma unroll
+        for (int j = 0; j < CW / 2; j++)
+            if (n_ok && 2 * j + mi < live) yp[(size_t)(2 * j) * p.ldy] = __float2half_rn(g[j]);
+    } else {
+        const size_t o0 = (size_t)row0 * p.ldy + n;
+        auto store = [&](auto* y, auto load_f, auto round_f) {
+            if (p.accumulate) {  // all loads before the first store
+                float old[CW];
+#pragma unroll
+                for (int j = 0; j < CW; j++) old[j] = n_ok && j < live ? load_f(y[o0 + (size_t)j * p.ldy]) : 0.f;
+#pragma unroll
+                for (int j = 0; j < CW; j++) v[j] = old[j] + v[j];
+            }
+#pragma unroll
+            for (int j = 0; j < CW; j++)
+                if (n_ok && j < live) y[o0 + (size_t)j * p.ldy] = round_f(v[j]);
+        };
+        if (p.y_dtype == kF32) store(reinterpret_cast<float*>(p.y), [](float f) { return f; }, [](float f) { return f; });
+        else if (p.y_dtype == kF16) store(reinterpret_cast<__half*>(p.y), [](__half h) { return __half2float(h); }, [](float f) { return __float2half_rn(f); });
+        else store(reinterpret_cast<uint16_t*>(p.y), [](uint16_t u) { return bf16_bits_to_f32(u); }, [](float f) { return (uint16_t)f32_to_bf16_bits(f); });
+    }
+}
+
 // EPI: 0 store, 1 gate + up + activation.
 // PAIR: a cluster of two CTAs works on tiles of twice the features.
 template <int FMT, int EPI, int GROUPS, bool PAIR>
@@ -354,6 +395,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
     constexpr uint32_t TCOLS = GROUPS == kTaGroups ? 512 : 256;
     constexpr int CTAS = PAIR ? 2 : 1;
     constexpr int RS = GROUPS == kTaGroups ? 2 : 1;  // A stages per hand-over to the issuer
+    constexpr bool SPLIT = GROUPS == kTaGroups;      // (two CTAs per SM: tiles are never divided along K)
     const uint32_t rank = PAIR ? cluster_rank() : 0;  // the even CTA issues the MMAs
     const int unit = (int)blockIdx.x / CTAS, units = (int)gridDim.x / CTAS;
     extern __shared__ unsigned char smem_raw[];
@@ -390,7 +432,8 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
-        // the work list
+    }
+    if (SPLIT && threadIdx.x == 0) {  // the work list
         if (p.tiles != nullptr && !p.early) pdl_wait();
         constexpr int NROWS = EPI ? 64 : 128;
         const int n_tiles = (p.N + CTAS * NROWS - 1) / (CTAS * NROWS);
@@ -437,15 +480,26 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
 
     constexpr int NROWS = EPI ? 64 : 128;  // output features per tile
     const int ksteps = p.K / 64;
+    int n_all = 0, m_all = 0;
+    if (!SPLIT) {
+        n_all = (p.N + NROWS - 1) / NROWS;
+        m_all = p.tiles != nullptr ? (int)(*p.ntiles) : (p.M + p.tile_rows - 1) / p.tile_rows;
+    }
     const int na = p.dcols == 128 ? 8 : 4;
     const uint32_t tmem_a = tmem + 2 * p.dcols;
     struct Item {
         int ks0, ks1, expert, row0, rows, n0;
     };
+    // work items: the pieces and tiles of the schedule, 0 up; without one the tiles themselves
+    const int first = SPLIT ? 0 : unit, stride = SPLIT ? 1 : units;
     auto item = [&](int i, Item& t) -> bool {
         int tile;
-        const int np = sched->np, n_tiles = sched->n_tiles, m_tiles = sched->m_tiles;
-        if (i < np) {
+        const int np = SPLIT ? sched->np : 0, n_tiles = SPLIT ? sched->n_tiles : n_all, m_tiles = SPLIT ? sched->m_tiles : m_all;
+        if (!SPLIT) {
+            tile = i;
+            t.ks0 = 0; t.ks1 = ksteps;
+            if (tile >= n_all * m_all) return false;
+        } else if (i < np) {
             tile = sched->piece[i].tile; t.ks0 = sched->piece[i].ks0; t.ks1 = sched->piece[i].ks1;
         } else {
             tile = sched->split + unit + (i - np) * units;
@@ -470,7 +524,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             uint32_t ph = 0;
             bool ok = true;
             Item t;
-            for (int i = 0; ok && item(i, t); i++) {
+            for (int i = first; ok && item(i, t); i += stride) {
                 const int bi = (t.rows - 1) / p.xbox;
                 const CUtensorMap* const map = &maps.x[bi];
                 const uint32_t bytes = (uint32_t)(p.xbox * (bi + 1) * p.xk * 128);
@@ -491,7 +545,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             uint32_t ph = 0;
             bool ok = true;
             Item t;
-            for (int i = 0; ok && item(i, t); i++) {
+            for (int i = first; ok && item(i, t); i += stride) {
                 const int wrow = t.expert * p.N + t.n0;
                 for (int ch = t.ks0 / KPS; ch * KPS < t.ks1; ch++) {
                     if (!(ok = mbar_wait(bar_cempty + 8 * s, ph ^ 1, abort_flag))) break;
@@ -515,7 +569,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         uint32_t ph = 0;
         bool ok = true;
         Item t;
-        for (int it = 0; ok && item(it, t); it++) {
+        for (int it = first; ok && item(it, t); it += stride) {
             const char* src[4][NT];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
@@ -581,40 +635,62 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             const uint32_t xdesc0 = (x0 & 0x3FFFFu) >> 4;
             bool ok = true;
             Item t;
-            for (int i = 0; ok && item(i, t); i++) {
+            for (int i = first; ok && item(i, t); i += stride) {
                 const uint32_t idesc = ta_idesc((t.rows + 15) & ~15, CTAS);
                 if (!(ok = mbar_wait_hint(0, bar_tempty + 8 * acc, tph ^ 1, abort_flag))) break;
                 const uint32_t td = tmem + acc * p.dcols;
                 const uint32_t kunits = (uint32_t)(p.xbox * ((t.rows - 1) / p.xbox + 1) / CTAS * 8);
-                uint32_t more = 0;  // the tile's first MMA starts the sums
-                for (int left = t.ks1 - t.ks0; left > 0 && ok; left -= p.xk) {
-                    if (!(ok = mbar_wait_hint(x_hint, bar_xfull + 8 * xs, xph, abort_flag))) break;
-                    uint32_t xdesc = xdesc0 + xs * ((uint32_t)p.x_stage >> 4);
-                    const uint32_t xdone = bar_xempty + 8 * xs;
-                    if (++xs == p.nx) { xs = 0; xph ^= 1; }
-                    for (int j = min(left, p.xk); j > 0; j -= RS, xdesc += RS * kunits) {
-                        if (!(ok = mbar_wait_hint(a_hint, bar_aready + 8 / RS * as, aph, abort_flag))) break;
-                        const uint32_t ta = tmem_a + as * 32, done = bar_aempty + 8 * as;
-                        tc_fence_after();
+                if constexpr (!SPLIT) {
+                    // low tiles: the MMAs are over before answers asked behind them would come, so the barriers are asked ahead of them
+                    for (int ks0 = 0; ks0 < ksteps && ok; ks0 += p.xk) {
+                        if (!(ok = mbar_wait_hint(x_hint, bar_xfull + 8 * xs, xph, abort_flag))) break;
+                        const int ks1 = min(ksteps, ks0 + p.xk);
+                        uint32_t xdesc = xdesc0 + xs * ((uint32_t)p.x_stage >> 4);
+                        const uint32_t xdone = bar_xempty + 8 * xs;
+                        if (++xs == p.nx) { xs = 0; xph ^= 1; }
+                        for (int ks = ks0; ks < ks1; ks++, xdesc += kunits) {
+                            if (!(ok = mbar_wait_hint(a_hint, bar_aready + 8 * as, aph, abort_flag))) break;
+                            const uint32_t ta = tmem_a + as * 32, done = bar_aempty + 8 * as;
+                            if (++as == na) { as = 0; aph ^= 1; }
+                            a_hint = mbar_test(bar_aready + 8 * as, aph);
+                            if (ks + 1 == ks1) x_hint = mbar_test(bar_xfull + 8 * xs, xph);
+                            tc_fence_after();
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) {
-                            umma_f16_ta<PAIR>(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, more);
-                            more = 1;
+                            for (int kk = 0; kk < 4; kk++)
+                                umma_f16_ta<PAIR>(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, (ks | kk) ? 1u : 0u);
+                            commit(done);
                         }
-                        commit(done);
-                        if (RS == 2) {
+                        commit(xdone);
+                    }
+                } else {
+                    uint32_t more = 0;  // the tile's first MMA starts the sums
+                    for (int left = t.ks1 - t.ks0; left > 0 && ok; left -= p.xk) {
+                        if (!(ok = mbar_wait_hint(x_hint, bar_xfull + 8 * xs, xph, abort_flag))) break;
+                        uint32_t xdesc = xdesc0 + xs * ((uint32_t)p.x_stage >> 4);
+                        const uint32_t xdone = bar_xempty + 8 * xs;
+                        if (++xs == p.nx) { xs = 0; xph ^= 1; }
+                        for (int j = min(left, p.xk); j > 0; j -= 2, xdesc += 2 * kunits) {
+                            if (!(ok = mbar_wait_hint(a_hint, bar_aready + 4 * as, aph, abort_flag))) break;
+                            const uint32_t ta = tmem_a + as * 32, done = bar_aempty + 8 * as;
+                            tc_fence_after();
+#pragma unroll
+                            for (int kk = 0; kk < 4; kk++) {
+                                umma_f16_ta<PAIR>(td, ta + 8 * kk, kTaDescHi | (uint64_t)(xdesc + 2 * kk), idesc, more);
+                                more = 1;
+                            }
+                            commit(done);
                             if (j >= 2) {
 #pragma unroll
                                 for (int kk = 0; kk < 4; kk++)
                                     umma_f16_ta<PAIR>(td, ta + 32 + 8 * kk, kTaDescHi | (uint64_t)(xdesc + kunits + 2 * kk), idesc, 1u);
                             }
                             commit(done + 8);
+                            if (j <= 2) commit(xdone);
+                            as += 2;
+                            if (as == na) { as = 0; aph ^= 1; }
+                            a_hint = mbar_test(bar_aready + 4 * as, aph);
+                            if (j <= 2) x_hint = mbar_test(bar_xfull + 8 * xs, xph);
                         }
-                        if (j <= RS) commit(xdone);
-                        as += RS;
-                        if (as == na) { as = 0; aph ^= 1; }
-                        a_hint = mbar_test(bar_aready + 8 / RS * as, aph);
-                        if (j <= RS) x_hint = mbar_test(bar_xfull + 8 * xs, xph);
                     }
                 }
                 if (ok) commit(bar_tfull + 8 * acc);
@@ -640,7 +716,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         uint32_t cph = 0;
         bool ok = true;
         Item t;
-        for (int n = 0; ok && item(n, t); n++) {
+        for (int n = first; ok && item(n, t); n += stride) {
             const int steps = t.ks1 - t.ks0;  // (t.ks0 is the first step of a stage)
             for (int ch = 0; ch * KPS < steps; ch++) {
                 const int j0 = (grp - (int)it0 - ch * KPS) & (GROUPS - 1);  // this group's first step of the stage
@@ -667,24 +743,32 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                             sc = lds_u16(scales + 2 * (FMT == kFmtTernary ? j >> 1 : j));
                             if (F::BIAS) bi = lds_u16(scales + 128 * SPB + 2 * j);
                         }
-                        uint32_t o[2][16];
-                        auto convert = [&](int h) {
+                        auto convert = [&](int h, uint32_t (&o)[16]) {
                             // groups of 32 (g32: 16 bits each; mxfp4: 8 bits each) have a scale per half
                             const uint32_t sch = FMT == kFmtAffine4G32 ? sc & 0xFFFFu : (FMT == kFmtMxfp4 ? sc & 0xFFu : sc);
                             ta_dequant32<FMT>(codes, (uint32_t)(j * (F::BPS / 16) + (FMT == kFmtTernary ? 0 : h * (F::BPS / 32))), h, sw, sch,
-                                              FMT == kFmtAffine4G32 ? bi & 0xFFFFu : bi, o[h]);
+                                              FMT == kFmtAffine4G32 ? bi & 0xFFFFu : bi, o);
                             if (FMT == kFmtAffine4G32) { sc >>= 16; bi >>= 16; }
                             if (FMT == kFmtMxfp4) sc >>= 8;
                         };
-                        // Converted before the wait where the registers allow it: a stage's turn-around is then a store, not a conversion
-                        if (RS == 2) { convert(0); convert(1); }
+                        // Converted before the wait where the registers allow it (not with 64): a stage's turn-around is then a store, not a
+                        // conversion
+                        uint32_t early[SPLIT ? 2 : 1][16];
+                        if constexpr (SPLIT) { convert(0, early[0]); convert(1, early[1]); }
                         ok = __all_sync(0xffffffffu, a_hint || mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
                         if (!ok) break;
                         tc_fence_after();
-                        if (RS == 1) convert(0);
-                        tmem_st16(my_a + as * 32, o[0]);
-                        if (RS == 1) convert(1);
-                        tmem_st16(my_a + as * 32 + 16, o[1]);
+                        if constexpr (SPLIT) {
+                            tmem_st16(my_a + as * 32, early[0]);
+                            tmem_st16(my_a + as * 32 + 16, early[1]);
+                        } else {
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                uint32_t o[16];
+                                convert(h, o);
+                                tmem_st16(my_a + as * 32 + h * 16, o);
+                            }
+                        }
                         tmem_st_wait();
                         tc_fence_before();
                         __syncwarp();
@@ -719,7 +803,7 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
         int acc = 0;
         uint32_t tph = 0;
         Item t;
-        for (int i = 0; item(i, t); i++) {
+        for (int i = first; item(i, t); i += stride) {
             const int rows = t.rows, n = t.n0 + nl;
             const bool n_ok = n < p.N;
             const float* eb = mi ? p.ebias[1] : p.ebias[0];
@@ -728,13 +812,13 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
             tc_fence_after();
             const uint32_t td = tmem + acc * p.dcols + ((uint32_t)(32 * q) << 16);
             constexpr int CW = 16;  // token columns at a time
-            const int slot = i < sched->np ? sched->piece[i].slot : -1;
+            const int slot = SPLIT && i < sched->np ? sched->piece[i].slot : -1;
             float4* const part = reinterpret_cast<float4*>(p.part) + ((size_t)slot * CTAS + rank) * (ta_slot(p.tile_rows) / 4) + q * (ta_slot(p.tile_rows) / 16) + lane;
             for (int c0 = 0; c0 < rows; c0 += CW) {
                 uint32_t r[CW];
                 tmem_ld16(td + c0, r);
                 tmem_ld_wait();
-                if (slot >= 0) {  // a piece: [warp][four columns][lane], 16 bytes each
+                if (SPLIT && slot >= 0) {  // a piece: [warp][four columns][lane], 16 bytes each
 #pragma unroll
                     for (int j = 0; j < CW / 4; j++)
                         part[(c0 / 4 + j) * 32] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
@@ -744,7 +828,8 @@ __global__ void __launch_bounds__(ta_threads(GROUPS), GROUPS == kTaGroups ? 1 : 
                 float v[CW];
 #pragma unroll
                 for (int j = 0; j < CW; j++) v[j] = __uint_as_float(r[j]) + bias;
-                ta_store<EPI, CW>(p, v, t.row0 + c0, n, n_ok, rows - c0, mi);
+                if (SPLIT) ta_store<EPI, CW>(p, v, t.row0 + c0, n, n_ok, rows - c0, mi);
+                else ta_store_low<EPI, CW>(p, v, t.row0 + c0, n, n_ok, rows - c0, mi);
             }
             tc_fence_before();
             __syncwarp();
