@@ -55,10 +55,13 @@ struct TopkParams {
 //
 // Bound: latency (a row of 128,000 is 0.5 MB). Two kernels of 4096-logit parts, searching the 64th key two bits and one block-wide
 // barrier at a time, took 23 us for one row of 128,000, 34 for eight and 51 for sixteen; now 11.4, 11.5 and 21.
-// KEEP: the span stays in registers; where it is long, or more than eight rows want two blocks per SM (sixteen rows of 128,000
-// 23 -> 21 us), it is read again instead.
+// KEEP: the span stays in registers; where more than eight rows want two blocks per SM (sixteen rows of 128,000 23 -> 21 us), it is read
+// again instead. KPT = 0 (spans of more than 16 logits per thread): read again, eight logits a turn of a loop. Unrolled for 32 the
+// passes are some 50 KB of instructions, which a decode step's GEMV has driven out of the caches: behind the GEMV of a 151,936 x 2048 4-bit
+// head one row took 24.8 us of candidates, rolled 17.3 (four rows 31.5 -> 16.8, eight 78 -> 63 with the GEMV; 262,144: 32.5 -> 21.5). Spans of
+// up to 16 stay unrolled (131,072 with its GEMV 40.6 us, rolled 41.9).
 template <int KPT, bool KEEP>
-__global__ void __launch_bounds__(kTopThreads, KEEP ? 1 : 2) __cluster_dims__(kTopBlocks, 1, 1)
+__global__ void __launch_bounds__(kTopThreads, KEEP || KPT == 0 ? 1 : 2) __cluster_dims__(kTopBlocks, 1, 1)
     topk64_kernel(const __grid_constant__ TopkParams p) {
     __shared__ unsigned long long list[kTopList], group_max[128], bound_;
     __shared__ unsigned long long run[kTopBlocks][kTopK];  // the first block's: sorted candidates of every block
@@ -86,6 +89,17 @@ __global__ void __launch_bounds__(kTopThreads, KEEP ? 1 : 2) __cluster_dims__(kT
     }
     // every logit of the thread in order of id, eight loads at a time
     auto each = [&](auto f) {
+        if constexpr (KPT == 0) {
+#pragma unroll 1
+            for (int k0 = 0; k0 * kTopThreads < p.span; k0 += 8) {  // (read() ends at the span: its last turn may be short)
+                float v[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) v[k] = read(k0 + k);
+#pragma unroll
+                for (int k = 0; k < 8; k++) f(k0 + k, v[k]);
+            }
+            return;
+        }
 #pragma unroll
         for (int k0 = 0; k0 < KPT; k0 += 8) {
             float v[8];
@@ -334,7 +348,7 @@ extern "C" int32_t iq_topk64(iq_ctx* ctx, void* stream, const float* x, int64_t 
     }
     p.idx = idx; p.val = val; p.z = z;
     const int kpt = p.span / kTopThreads;
-    auto kernel = kpt <= 4 ? topk64_kernel<4, true> : kpt <= 8 ? topk64_kernel<8, true> : kpt > 16 ? topk64_kernel<32, false>
+    auto kernel = kpt <= 4 ? topk64_kernel<4, true> : kpt <= 8 ? topk64_kernel<8, true> : kpt > 16 ? topk64_kernel<0, false>
                   : rows <= 8 ? topk64_kernel<16, true> : topk64_kernel<16, false>;
     return check_cuda(ctx, launch_dependent(kernel, dim3(rows * kTopBlocks), kTopThreads, 0, reinterpret_cast<cudaStream_t>(stream), p), "topk64 launch");
 }

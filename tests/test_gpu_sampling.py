@@ -114,3 +114,13 @@ def test_candidates_of_orders_that_fill_the_list(cuda_device, V, rows, rest):
     x[:, (np.arange(V) % 1024) // 8 >= 63] = rest
     x[:, 1023] = -5.0  # (one small finite logit)
     check(x, [0.9])
+
+
+@pytest.mark.parametrize("V,rows", [(131072, 9), (131073, 1), (139265, 9), (196608, 2), (196609, 16), (262143, 3)])
+def test_candidates_where_the_passes_change(cuda_device, V, rows):
+    """Around the longest span whose passes are unrolled, and spans that end inside a turn of the rolled ones: random logits, rows that
+    are all equal (the list overflows and its bound is searched), and a best logit at the row's end."""
+    x = logits("random", V, rows, V)
+    x[0] = 1.5
+    x[-1, V - 1] = 99.0
+    check(x, [0.7])
