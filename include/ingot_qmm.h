@@ -137,7 +137,7 @@ int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_
  * ordinary Metal buffers made at construction). Meant for hosts where cudaMalloc is off limits at the call site: a
  * plugin inside an engine whose pool owns all device memory, a path that runs after the pool is sealed, a sandbox or
  * real-time loop with a "no allocation" rule. Same operation and results as iq_qmm, but the fp16 copy of bf16/fp32
- * activations goes to an array built into the library (8 MiB, and 40 MiB for partial sums, held by every GPU that loads it
+ * activations goes to an array built into the library (8 MiB, and 28 MiB for partial sums, held by every GPU that loads it
  * until the process exits) instead of a caller workspace. Limits and rules:
  *   - rows * k <= 4,194,304 (8 MiB of fp16); larger calls return IQ_ERR_WORKSPACE and should use iq_qmm;
  *   - the first call on a device looks up the array's device address (cudaGetSymbolAddress) with that device current;

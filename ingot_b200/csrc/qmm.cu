@@ -366,7 +366,7 @@ QmmSplit qmm_split(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K, void*
 size_t qmm_split_bound(iq_ctx* ctx, int32_t fmt, int epi, int M, int N, int K) {
     return fmt < 0 || fmt == kFmtAffine6 || fmt > kFmtTernary ? 0 : ta_split_bound(fmt, epi, M, N, K, ctx->sms);
 }
-size_t qmm_split_max_bytes(iq_ctx* ctx) { return (size_t)2 * ctx->sms * ta_slot(kTaMaxRows) * 4; }  // (two CTAs per SM: slots of a third)
+size_t qmm_split_max_bytes(iq_ctx* ctx) { return (size_t)2 * ctx->sms * ta_slot(kTaMaxRows) * 4; }
 size_t qmm_convert_bytes(int rows, int k, int32_t x_dtype) { return x_dtype == IQ_F16 ? 0 : round_up_sz((size_t)rows * k * 2, 256); }
 
 }  // namespace iq
@@ -466,7 +466,8 @@ extern "C" int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dt
 // caller to bring it. This variant brings its own: a fixed array that is part of the library image, so it exists on
 // every GPU that loads the library, from load until the process exits, and costs that GPU kNoAllocBytes + kNoAllocSplit of memory.
 constexpr size_t kNoAllocBytes = 8u << 20;   // 8 MiB: rows * k <= 4,194,304 activations (e.g. 1024 x 4096)
-constexpr size_t kNoAllocSplit = 40u << 20;  // partial sums of the K split: two slots of 192 tokens per SM (28 MiB on 148)
+constexpr size_t kNoAllocSplit = 28u << 20;  // partial sums of the K split: the most that any call on 148 SMs takes
+static_assert(kNoAllocSplit >= (size_t)2 * 148 * ta_slot(kTaMaxRows) * 4, "two slots of 192 tokens per SM");
 static __device__ __align__(256) unsigned char g_qmm_noalloc_scratch[kNoAllocBytes + kNoAllocSplit];
 
 namespace {
@@ -501,7 +502,7 @@ extern "C" int32_t iq_qmm_noalloc(iq_ctx* ctx, void* stream, const void* x, int3
         g_noalloc_ptr[dev].store(p, std::memory_order_release);  // two first callers store the same address
         scratch = p;
     }
-    // Every byte the GEMM reads from the scratch is written by this call's own conversion pass first, so nothing has
-    // to be cleared; what the previous call left behind is simply overwritten.
+    // Every byte that is read from the scratch is written by this call first (activations by the conversion pass, partial sums by the
+    // GEMM whose sums' kernel reads them), so nothing has to be cleared; what the previous call left behind is simply overwritten.
     return iq_qmm(ctx, stream, x, x_dtype, ldx, m, y, y_dtype, ldy, rows, flags, scratch, kNoAllocBytes + kNoAllocSplit);
 }

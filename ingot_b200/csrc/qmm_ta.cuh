@@ -158,7 +158,7 @@ __host__ __device__ inline void ta_split_tile(const TaSplit& s, int t, int& c0, 
     slot0 = c0 * all / s.ctas < ua ? s.ctas + t : c0;
 }
 // floats of a slot for tiles of up to `rows` tokens; slots: one per CTA, one per split tile
-__host__ __device__ inline int ta_slot(int rows) { return 128 * ((rows + 15) & ~15); }
+__host__ __device__ constexpr int ta_slot(int rows) { return 128 * ((rows + 15) & ~15); }
 inline size_t ta_split_bytes(const TaSplit& s, int rows, bool pair) { return (size_t)(s.ctas + s.tiles) * ta_slot(rows) * (pair ? 8 : 4); }
 
 // Shared-memory and instruction descriptors: K-major B tile with 128-byte swizzle (rows of 128 bytes, 8-row groups 1024

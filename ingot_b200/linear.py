@@ -233,7 +233,7 @@ class DenseQ:
                            stream: Optional[torch.cuda.Stream] = None):
         """The prefill GEMM for callers that may not allocate device memory (a plugin inside an engine that owns the
         memory pool, a sealed pool, a no-allocation rule): same results as `encode_qmm_f32`, with the fp16 copy of
-        bf16/fp32 activations (8 MiB) and the partial sums (40 MiB) kept in an array built into the library. rows * K must not exceed 4,194,304; calls
+        bf16/fp32 activations (8 MiB) and the partial sums (28 MiB) kept in an array built into the library. rows * K must not exceed 4,194,304; calls
         that may overlap on the GPU share that array and must be ordered on one stream; make the first call on a device
         outside any stream capture."""
         _need_cuda(x, y)

@@ -45,3 +45,21 @@ def test_noalloc_refuses_sizes_beyond_its_scratch(cuda_device):
     with pytest.raises(capi.IngotError) as e:
         m.encode_qmm_noalloc(x, y, M)
     assert e.value.status == -4 and "scratch" in str(e.value)
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 192, 14336), (192, 14336, 20992)])
+def test_noalloc_holds_the_partial_sums(cuda_device, M, N, K):
+    """Calls divided along K, the second with about the most partial sums that rows * k <= 4,194,304 allows: the bits of iq_qmm."""
+    plan = capi.qmm_plan(N, K, 4, 64, M, sms=torch.cuda.get_device_properties(0).multi_processor_count)
+    assert plan.split_tiles > 0 and plan.split_bytes + M * K * 2 <= (8 + 28) << 20
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(79)
+    m = synth.affine_cuda(gen, N, K, 4)
+    x = synth.activations_cuda(gen, M, K)
+    ws = torch.empty(m.qmm_workspace_bytes(M, x.dtype), dtype=torch.uint8, device=cuda_device)
+    want = torch.zeros(M, N, dtype=torch.float32, device=cuda_device)
+    m.encode_qmm_f32(x, want, M, workspace=ws)
+    got = torch.full_like(want, float("nan"))
+    m.encode_qmm_noalloc(x, got, M)
+    assert capi.context(0).device_status() == 0
+    assert torch.equal(got, want)
