@@ -359,12 +359,14 @@ def test_router_tensor_logits_of_96_experts(cuda_device):
 
 
 @pytest.mark.parametrize("gated", [True, False])
-@pytest.mark.parametrize("T", [1, 19, 300])
-def test_moe_shared_expert(cuda_device, T, gated):
+@pytest.mark.parametrize("T,D,IS", [(1, 256, 192), (19, 256, 192), (300, 256, 192), (50, 2048, 256), (100, 2048, 320)])
+def test_moe_shared_expert(cuda_device, T, D, IS, gated):
     """A shared expert of its own width beside the routed experts, with its 8-bit sigmoid gate or weight 1
-    (MoE.swift:140-154; KernelCaseMoE.swift:45-114): GEMV tiles for few tokens, the tcgen05 path for many."""
+    (MoE.swift:140-154; KernelCaseMoE.swift:45-114): GEMV tiles for few tokens, the tcgen05 path for many; at 2048 inputs its gate/up
+    tiles, of token rows that are no multiple of 16, are divided along K."""
     rng = np.random.default_rng(300 + T)
-    E, K, D, I, IS = 32, 4, 256, 128, 192
+    E, K, I = 32, 4, 128
+    assert D == 256 or capi.qmm_plan(2 * IS, D, 4, 64, T, gate_up=True).split_tiles > 0
     sg, su, sd = synth.affine_np(rng, IS, D, 4), synth.affine_np(rng, IS, D, 4), synth.affine_np(rng, D, IS, 4)
     gw = synth.affine_np(rng, 1, D, 8)
     mk = lambda t, bits: synth.dense_q_affine(t[0], t[1], t[2], bits, cuda_device)

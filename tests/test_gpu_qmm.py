@@ -187,12 +187,25 @@ def test_mxfp4_scales_at_any_address(cuda_device, K, by):
     assert capi.context(0).device_status() == 0
 
 
+def path_of(fmt, group, rows, n, k, gate_up=False):
+    """Which way the library takes: "pair" or "one" CTA per tile, "+split" where all tiles are divided along K, "+split+whole" where the
+    first ones are."""
+    p = capi.qmm_plan(2 * n if gate_up else n, k, 8 if fmt == "q8" else 4, group, rows, capi.IQ_MODE_MXFP4 if fmt == "mxfp4" else capi.IQ_MODE_AFFINE,
+                      gate_up, torch.cuda.get_device_properties(0).multi_processor_count)
+    return ("pair" if p.pair else "one") + ("" if p.split_tiles == 0 else "+split" if p.split_tiles == p.tiles else "+split+whole")
+
+
 @pytest.mark.parametrize("fmt,group", [("q4", 64), ("q8", 64), ("q4", 32), ("mxfp4", 32)])
-@pytest.mark.parametrize("M,N,K", [(64, 192, 14336), (64, 2112, 5824), (192, 128, 9216), (128, 7744, 2880), (320, 4096, 4160), (2048, 4096, 5120)])
-def test_qmm_split_along_k(cuda_device, fmt, group, M, N, K):
+@pytest.mark.parametrize("M,N,K,path", [
+    (64, 192, 14336, "one+split"), (64, 2112, 5824, "one+split"), (192, 128, 9216, "one+split"), (256, 9600, 1664, "one+split+whole"),
+    (320, 9600, 2112, "one+split+whole"), (704, 1216, 8256, "pair+split"), (704, 5056, 4160, "pair+split+whole"),
+    (64, 19456, 2112, "pair+split+whole"), (128, 7744, 2880, "one"), (320, 4096, 4160, "one"), (2048, 4096, 5120, "pair")])
+def test_qmm_split_along_k(cuda_device, fmt, group, M, N, K, path):
     """Tiles that fill no whole round are divided along K: one tile in eight pieces and more, runs that end inside a tile, an odd number
-    of stages, pieces before whole tiles. Against the oracle, against the call whose workspace has no room for the sums (every tile
-    in one piece), the same bits every time, and added onto a result."""
+    of stages, pieces before whole tiles, on one CTA and on pairs (a second CTA without features, a last token tile of another height,
+    odd numbers of K steps). Against the oracle, against the call whose workspace has no room for the sums (every tile in one
+    piece), the same bits every time, and added onto a result."""
+    assert path_of(fmt, group, M, N, K) == path
     rng = np.random.default_rng(71 + M + N + K + group)
     bits = 8 if fmt == "q8" else 4
     m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, bits, cuda_device, group=group)
@@ -204,31 +217,42 @@ def test_qmm_split_along_k(cuda_device, fmt, group, M, N, K):
     ref = qref.matmul_t(x, deq(some, bits, group=group))
     got = y[:, torch.from_numpy(sel).to(cuda_device)].cpu().numpy()
     assert qref.max_rel(got, ref) <= TOL
+    assert bool(torch.isfinite(y).all())
     whole = torch.zeros_like(y)
     m.encode_qmm_f32(xt, whole, M, workspace=torch.empty(M * K * 2, dtype=torch.uint8, device=cuda_device))
     # the same products in another order of sums: 14336 roundings of 2^-24, as a random walk, are 7e-6 of a sum's size
     assert float((y - whole).abs().max() / whole.abs().max()) <= 2e-5
+    assert ("split" in path) or torch.equal(y, whole)
     assert torch.equal(run_qmm(m, xt, M), y)
     y0 = torch.randn(M, N, device=cuda_device)
     assert torch.equal(run_qmm(m, xt, M, accumulate=True, y=y0.clone()), y0 + y)
     assert torch.equal(run_qmm(m, x_tensor(x, cuda_device, torch.float16), M, torch.float16), y.to(torch.float16))
 
 
-@pytest.mark.parametrize("act", ["silu", "swiglu_oai"])
-@pytest.mark.parametrize("rows,d,d_ff", [(64, 1216, 8768), (256, 2048, 7680), (320, 4160, 1088)])
-def test_dense_ffn_split_along_k(cuda_device, rows, d, d_ff, act):
-    """The gated epilogue on the sums of pieces, and the down projection's split, against a float64 product."""
+@pytest.mark.parametrize("fmt,group,act", [("q4", 64, "silu"), ("q4", 64, "swiglu_oai"), ("q8", 64, "silu"), ("q4", 32, "gelu"),
+                                           ("mxfp4", 32, "swiglu_oai")])
+@pytest.mark.parametrize("rows,d,d_ff,gate_up,down", [
+    (64, 1216, 8768, "one", "one+split"), (256, 2048, 7680, "one", "one+split"), (320, 4160, 1088, "one", "one"),
+    (64, 2112, 64, "one+split", "one"), (192, 2048, 256, "one+split", "one"), (704, 5120, 2880, "pair+split+whole", "one")])
+def test_dense_ffn_split_along_k(cuda_device, fmt, group, act, rows, d, d_ff, gate_up, down):
+    """The gated epilogue on the sums of pieces (on one CTA and on pairs, the last one with features for one of its CTAs), and the down
+    projection's split, against a float64 product."""
+    assert path_of(fmt, group, rows, d_ff, d, gate_up=True) == gate_up and path_of(fmt, group, rows, d, d_ff) == down
     rng = np.random.default_rng(72 + rows)
-    gu, hg = affine_case(rng, 2 * d_ff, d, 4, cuda_device)
-    dn, hd = affine_case(rng, d, d_ff, 4, cuda_device)
+    bits = 8 if fmt == "q8" else 4
+    mk = (lambda n, k: mxfp4_case(rng, n, k, cuda_device)) if fmt == "mxfp4" else (lambda n, k: affine_case(rng, n, k, bits, cuda_device, group=group))
+    gu, hg = mk(2 * d_ff, d)
+    dn, hd = mk(d, d_ff)
     x = x_tensor(synth.activations_np(rng, rows, d), cuda_device)
     out = torch.zeros(rows, d, dtype=torch.float32, device=cuda_device)
     DenseMLP(gu, dn, act).encode(x, out, rows)
     assert capi.context(0).device_status() == 0
-    w = [torch.from_numpy(deq(h, 4)).to(cuda_device).double() for h in (hg, hd)]
+    w = [torch.from_numpy(deq(h, bits, group=group)).to(cuda_device).double() for h in (hg, hd)]
     g, u = (x.double() @ w[0].T).split(d_ff, dim=1)
     if act == "silu":
         h = g / (1 + torch.exp(-g)) * u
+    elif act == "gelu":
+        h = torch.nn.functional.gelu(g, approximate="tanh") * u
     else:
         g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0)
         h = (u + 1) * g / (1 + torch.exp(-1.702 * g))
@@ -237,10 +261,14 @@ def test_dense_ffn_split_along_k(cuda_device, rows, d, d_ff, act):
 
 
 @pytest.mark.parametrize("fmt,group", [("q4", 64), ("q8", 64), ("q4", 32), ("mxfp4", 32)])
-@pytest.mark.parametrize("M,N,K", [(4096, 2112, 832), (2048, 192, 1088), (1088, 14400, 320), (4096, 64, 64), (192, 9600, 2112)])
-def test_qmm_pairs_of_ctas(cuda_device, fmt, group, M, N, K):
-    """Tall calls run on pairs of CTAs with twice the features per tile: features that fill half a pair, one CTA of a pair or none of
-    its second one, token tiles whose halves differ, odd numbers of K steps; the same bits every time, and added onto a result."""
+@pytest.mark.parametrize("M,N,K,path", [
+    (1472, 2112, 2112, "pair"), (576, 5056, 2112, "pair"), (1024, 2880, 2944, "pair"), (4096, 2880, 576, "pair"), (192, 9600, 2112, "pair"),
+    (4096, 2112, 832, "one"), (2048, 192, 1088, "one"), (1088, 14400, 320, "one"), (4096, 64, 64, "one")])
+def test_qmm_pairs_of_ctas(cuda_device, fmt, group, M, N, K, path):
+    """Tall calls run on pairs of CTAs with twice the features per tile: a last pair with features for half of its first CTA, for half of
+    its second one, token tiles whose halves differ and a last one of another height, odd numbers of K steps (and the same calls'
+    neighbours that run on single CTAs); the same bits every time, and added onto a result."""
+    assert path_of(fmt, group, M, N, K) == path
     rng = np.random.default_rng(81 + M + N + K + group)
     bits = 8 if fmt == "q8" else 4
     m, host = mxfp4_case(rng, N, K, cuda_device) if fmt == "mxfp4" else affine_case(rng, N, K, bits, cuda_device, group=group)

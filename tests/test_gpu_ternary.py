@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from ingot_b200 import capi, synth
-from ingot_b200.linear import VQMV
+from ingot_b200.linear import DenseQ, VQMV
 from oracle import qref
 from gpu_util import x_tensor
 
@@ -87,6 +87,35 @@ def test_ternary_prefill_gemm(cuda_device, M, N, K):
     ref = qref.matmul_t(qref.rotate_input(x, signs), wf)
     err = qref.max_rel(y.cpu().numpy(), ref)
     assert err <= TERN_TOL, err
+
+
+@pytest.mark.parametrize("M,N,K,path", [(64, 192, 9216, "one+split"), (256, 9600, 2048, "one+split+whole"), (704, 1216, 8320, "pair+split"),
+                                        (704, 5056, 4224, "pair+split+whole"), (1024, 2880, 2944, "pair")])
+def test_ternary_gemm_split_and_pairs(cuda_device, M, N, K, path):
+    """Tiles divided along K (units of eight K steps, one that K ends in) and pairs of CTAs (a last pair with features for one and a half
+    and for three quarters of a CTA, token tiles of different heights), on rows that are rotated already."""
+    p = capi.qmm_plan(N, K, 2, 128, M, sms=torch.cuda.get_device_properties(0).multi_processor_count)
+    assert path == ("pair" if p.pair else "one") + ("" if p.split_tiles == 0 else "+split" if p.split_tiles == p.tiles else "+split+whole")
+    rng = np.random.default_rng(M + N + K)
+    w, s, _ = synth.ternary_np(rng, N, K)
+    m, wf = DenseQ(torch.from_numpy(w.view(np.int32)).to(cuda_device), torch.from_numpy(s).to(cuda_device), None, N, K, 2, 128), qref.dequant_ternary(w, s)
+    x = half_activations(rng, M, K)
+    xt = x_tensor(x, cuda_device, torch.float16)
+    ws = torch.empty(max(m.qmm_workspace_bytes(M, torch.float16), 256), dtype=torch.uint8, device=cuda_device)
+    y, whole = (torch.zeros(M, N, dtype=torch.float32, device=cuda_device) for _ in range(2))
+    m.encode_qmm_f32(xt, y, M, workspace=ws)
+    m.encode_qmm_f32(xt, whole, M)
+    assert capi.context(0).device_status() == 0
+    sel = np.unique(np.concatenate([np.sort(rng.choice(N, size=64, replace=False)), np.arange(N - 16, N)]))
+    rows = np.unique(np.concatenate([np.sort(rng.choice(M, size=min(M, 128), replace=False)), np.arange(M - 16, M)]))
+    got = y[torch.from_numpy(rows).to(cuda_device)][:, torch.from_numpy(sel).to(cuda_device)].cpu().numpy()
+    assert qref.max_rel(got, qref.matmul_t(x[rows], wf[sel])) <= TERN_TOL
+    # the same products in another order of sums: 9216 roundings of 2^-24, as a random walk, are 6e-6 of a sum's size
+    assert bool(torch.isfinite(y).all()) and float((y - whole).abs().max() / whole.abs().max()) <= 2e-5
+    again = torch.zeros_like(y)
+    m.encode_qmm_f32(xt, again, M, workspace=ws)
+    torch.cuda.synchronize()
+    assert torch.equal(again, y)
 
 
 def test_ternary_unpacked_codes_bit_exact(cuda_device):
