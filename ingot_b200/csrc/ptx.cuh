@@ -156,8 +156,8 @@ __device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
     return r;
 }
 
-// Two fp32 operations per instruction, each rounded as fmaf and a product are (the grouped int8 kernel: MoE block of 64 tokens 124.1 ->
-// 121.0 us; no effect in the dense GEMVs): {a0, a1} += {v0, v1} * ({s0, s1} * {x0, x1}), and then
+// Two fp32 operations per instruction, each rounded as fmaf and a product are (the grouped int8 kernel, where its registers allow it; no
+// effect in the dense GEMVs): {a0, a1} += {v0, v1} * ({s0, s1} * {x0, x1}), and then
 // += {b0, b1} * {y0, y1}.
 __device__ __forceinline__ void scaled_add2(float& a0, float& a1, float v0, float v1, float s0, float s1, float x0, float x1) {
     asm("{\n.reg .b64 a, v, s, x;\nmov.b64 a, {%0, %1};\nmov.b64 v, {%2, %3};\nmov.b64 s, {%4, %5};\nmov.b64 x, {%6, %7};\n"

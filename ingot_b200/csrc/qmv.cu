@@ -402,10 +402,15 @@ typedef void (*QgKernel)(const CUtensorMap, const CUtensorMap, const QgParams);
 // gw4: each consumer warp's K slice is four groups, its activation fragments stay in registers
 template <int MODE, bool TM>
 QgKernel qg_pick_mt(bool gw4) {
-    return gw4 ? qmv_imma_grouped_kernel<MODE, TM, 4, 8> : qmv_imma_grouped_kernel<MODE, TM, 0, 8>;
+    constexpr bool TWO = MODE == kModeDown;
+    return gw4 ? qmv_imma_grouped_kernel<MODE, TM, 4, 8, TWO> : qmv_imma_grouped_kernel<MODE, TM, 0, 8, TWO>;
 }
-QgKernel qg_pick(int mode, bool tm, bool gw4, bool fx = false) {
-    if (fx) return qmv_imma_grouped_kernel<kModeGateUp, true, 4, 16>;
+// fx: the inputs of a gate/up that takes the rows as fixed point, or 0.
+// The two-wide fp32 form costs registers (gate/up spills 72 bytes instead of 60): it pays in the down projections and in gate/up of up
+// to 2048 inputs on sixteen warps. MoE block, us, plain / everywhere / as here: 128 experts of 2048 x 768 at 64 tokens 125.8 / 122.6 / 122.9,
+// 64 of 2048 x 1408 at 12 tokens 98.2 / 100.5 / 98.5, 128 of 4096 x 1536 at 12 tokens 193.5 / 198.4 / 191.5 and at 64 364.8 / 370.8 / 357.8.
+QgKernel qg_pick(int mode, bool tm, bool gw4, int fx = 0) {
+    if (fx) return fx <= 2048 ? qmv_imma_grouped_kernel<kModeGateUp, true, 4, 16, true> : qmv_imma_grouped_kernel<kModeGateUp, true, 4, 16, false>;
     if (mode == kModeGateUp) return tm ? qg_pick_mt<kModeGateUp, true>(gw4) : qg_pick_mt<kModeGateUp, false>(gw4);
     return tm ? qg_pick_mt<kModeDown, true>(gw4) : qg_pick_mt<kModeDown, false>(gw4);
 }
@@ -511,7 +516,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, gw4 && p.wk == kQgWarps, fx), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, gw4 && p.wk == kQgWarps, fx ? c.K : 0), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
 }
 
 int32_t gqmv_init(iq_ctx* ctx) {
@@ -526,8 +531,8 @@ int32_t gqmv_init(iq_ctx* ctx) {
         cudaError_t e = cudaFuncSetAttribute(qi[i], cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma)");
     }
-    {
-        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(kModeGateUp, true, true, true)),
+    for (int fx = 2048; fx <= 4096; fx += 2048) {
+        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(kModeGateUp, true, true, fx)),
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
     }

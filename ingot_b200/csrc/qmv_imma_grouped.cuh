@@ -76,7 +76,8 @@ struct QgParams {
 // of converting them per CTA and tile: the conversion's shared memory goes to the ring, its instructions away, and with
 // twice the warps per scheduler the latencies of a warp's chain (shared-memory loads, shuffles, MMAs, the hand-over) hide
 // behind one another: eight warps issued 0.43 instructions per cycle and scheduler.
-template <int MODE, bool TM, int GW, int NCW>
+// TWO: scales and biases by two-wide fp32 operations, three instructions for six, rounded alike (qg_pick).
+template <int MODE, bool TM, int GW, int NCW, bool TWO>
 __global__ void __launch_bounds__(qg_threads(NCW), 1)
     qmv_imma_grouped_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, const QgParams p) {
     constexpr int NW = MODE == kModeGateUp ? 2 : 1;
@@ -433,8 +434,15 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
                                 for (int c = 0; c < NS; c++) {
                                     const float v0 = (float)(d[i][c][0] * 256 + d[i][c][1]);
                                     const float v1 = (float)(d[i][c][2] * 256 + d[i][c][3]);
-                                    scaled_add2(acc[i][c][0], acc[i][c][1], v0, v1, sc0, sc1, xs[c].x, xs[c].x);
-                                    fma2(acc[i][c][0], acc[i][c][1], bi0, bi1, xs[c].y, xs[c].y);
+                                    if constexpr (TWO) {
+                                        scaled_add2(acc[i][c][0], acc[i][c][1], v0, v1, sc0, sc1, xs[c].x, xs[c].x);
+                                        fma2(acc[i][c][0], acc[i][c][1], bi0, bi1, xs[c].y, xs[c].y);
+                                    } else {
+                                        acc[i][c][0] = fmaf(v0, sc0 * xs[c].x, acc[i][c][0]);
+                                        acc[i][c][0] = fmaf(bi0, xs[c].y, acc[i][c][0]);
+                                        acc[i][c][1] = fmaf(v1, sc1 * xs[c].x, acc[i][c][1]);
+                                        acc[i][c][1] = fmaf(bi1, xs[c].y, acc[i][c][1]);
+                                    }
                                 }
                             }
                         }

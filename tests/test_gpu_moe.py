@@ -532,3 +532,13 @@ def test_moe_tall_tiles_on_pairs(cuda_device, fmt, act, D, I, T):
     rng = np.random.default_rng(91 + D + T)
     layer, host = build_layer(rng, cuda_device, 32, 4, D, I, fmt=fmt, act=act, biases=fmt == "mxfp4", max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, D), T, act)
+
+
+@pytest.mark.parametrize("D,I", [(1024, 320), (2048, 1408), (4096, 256)])
+@pytest.mark.parametrize("T", [5, 40])
+def test_moe_int8_experts_by_width(cuda_device, D, I, T):
+    """The int8 expert kernels with the rows as fixed point, whose scales go by two-wide or by plain fp32 operations depending on the
+    inputs: one set of rows per expert and two."""
+    rng = np.random.default_rng(95 + D + T)
+    layer, host = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
+    check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
