@@ -467,6 +467,7 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
         if (e >= p.E) taken |= 1u << j;
     }
     if (REFINE) {
+        if (WPT > 1) __syncthreads();  // all warps have the approximate logits before one stores an exact one over them
         // ---- which experts can still be among the k largest? Those within 2 eps of the k-th largest approximate value:
         // with |approx - exact| <= eps everywhere, at least k experts have an exact value >= kth - eps, so a true member of
         // the top k has exact >= kth - eps and approx >= kth - 2 eps. The exact values of these candidates decide.
