@@ -188,6 +188,7 @@ def graph_time_us(torch, fn, n_in_graph: int, reps: int = 20, dist=None, world: 
     the host's launch cost out of a microsecond-scale kernel's timing. With world > 1 every rank makes the same calls
     (kernels that meet at a barrier included) and the result is the maximum over the ranks."""
     s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())  # the operands are made there
     with torch.cuda.stream(s):
         for i in range(3):
             fn(i)
