@@ -128,7 +128,10 @@ int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_
  * badly, some are divided along k and their partial sums go through the workspace, behind the converted rows (round(rows * k * 2,
  * 256) bytes, none for fp16): iq_qmm_workspace_bytes asks for both, and a workspace that holds the converted rows only is
  * accepted as well (the same products, summed in another order). The answer is enough for every call of up to `rows` rows of that
- * x_dtype and never falls as rows grows, so that one buffer sized for the most rows serves all calls. */
+ * x_dtype and never falls as rows grows, so that one buffer sized for the most rows serves all calls. The workspace belongs to one
+ * call at a time, also with fp16 x: calls that may overlap on the GPU need one each. The fp32 sum of an element may be taken over k
+ * in another order when rows, n or the room in the workspace differ (each call gives the same bits every time): a row of a long chunk and
+ * the same row alone, or a column shard and the whole matrix, agree to the rounding of fp32 sums and not to the bit. */
 int32_t iq_qmm_workspace_bytes(iq_ctx* ctx, const iq_qlinear* m, int32_t rows, int32_t x_dtype, size_t* bytes);
 int32_t iq_qmm(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
                int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, void* workspace, size_t workspace_bytes);

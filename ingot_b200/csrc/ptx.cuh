@@ -199,6 +199,10 @@ __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
 
 // Programmatic dependent launch: let the next kernel in the stream start its independent prologue, and wait for the
 // previous kernel's results before touching anything it may have written. Both are no-ops without the launch attribute.
+// A kernel may let its successor start before it has waited for its own predecessor, and the successor may then read what neither
+// of the two writes: weights (codes, scales, biases) are read ahead of the wait by the GEMVs and the dense GEMM. So a kernel that writes
+// weights lets nothing start early (of this library's, the W8A8 conversions; anybody else's copy or kernel without the trigger is as good:
+// the first kernel behind it starts when it has ended, and all later ones after that).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

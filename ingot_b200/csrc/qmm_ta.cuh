@@ -35,7 +35,9 @@
 // kernels run into the power limit: 2048 x 4096 x 14336 at 8 bits 1300 MHz with X copied, 1440 without). Copies of X of both CTAs
 // count on the even one's barrier, dequantisers and epilogue warps of the odd one arrive there, and commits go to both. 2048 x
 // 4096 x 14336 (8 bits, added) 228 -> 210 us, 4096 x 4096 x 7680 225 -> 202, FFN 4096 x 14336 of 1088 rows 338 -> 314 (sustained, at
-// the power limit: 284 -> 246 and 426 -> 368 with the K split below). Below some 150 rows one CTA's finer tiles win. On the way:
+// the power limit: 284 -> 246 and 426 -> 368 with the K split below). Tiles below some 150 rows
+// mostly go to single CTAs, whose finer tiles fill the rounds better; the cost model takes pairs for them too where they save a round (64 rows
+// x 19456 x 4096 34.6 -> 28.3 us, K split included). On the way:
 // arrivals that release at cluster scope cost the dequantisers 10 to 25 %, reporting the odd CTA's X by a thread of its own 20 %.
 // Tiles of a list that hold up to 64 tokens (MoE decode and short prefills) leave the MMA idle: a step of 16 tokens is 72 cycles
 // of it, and the 400 cycles of the issuing thread and of its hand-overs are the time. Two CTAs per SM, each with two
@@ -164,6 +166,8 @@ inline size_t ta_split_bytes(const TaSplit& s, int rows, bool pair) { return (si
 // Shared-memory and instruction descriptors: K-major B tile with 128-byte swizzle (rows of 128 bytes, 8-row groups 1024
 // bytes apart; the low 14 bits take the address in units of 16 bytes), fp16 operands, fp32 accumulator, M = 128.
 constexpr uint64_t kTaDescHi = ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+// n: 16 to 256 in steps of 16, for M = 128 and for a pair's 256, whose CTAs then hold whole groups of eight rows each. (Steps of 32 on pairs,
+// which is all that CUTLASS's form with A in tensor memory offers, cost lists 0.3 to 1 %; tiles of all counts of rows are tested.)
 __device__ __forceinline__ uint32_t ta_idesc(int n, int ctas) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((8u * ctas) << 24); }
 
 // D[128, N] (+)= A[128, 16] (tensor memory: lane = row, two inputs per column) * B[N, 16]^T (shared memory)

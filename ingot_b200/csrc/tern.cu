@@ -51,7 +51,7 @@ __device__ __forceinline__ void fwht1024(float (&v)[4], float* sh, int tid) {
 __global__ void __launch_bounds__(256) had_rows_kernel(const void* __restrict__ x, int32_t x_dtype, int64_t ldx,
                                                       const float* __restrict__ signs, __half* __restrict__ y, int64_t ldy) {
     __shared__ __align__(16) float sh[1024];
-    pdl_launch_dependents();
+    pdl_launch_dependents();  // (ahead of the wait: the GEMV fetches codes and scales meanwhile; behind it 9216 x 5120, one row, 10.5 -> 11.0 us)
     const int tid = threadIdx.x, k0 = blockIdx.x * 1024;
     pdl_wait();
     float v[4];

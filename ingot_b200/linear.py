@@ -191,7 +191,8 @@ class DenseQ:
     def encode_qmm_f32(self, x: torch.Tensor, y: torch.Tensor, rows: int, accumulate: bool = False,
                        workspace: Optional[torch.Tensor] = None, stream: Optional[torch.cuda.Stream] = None):
         """Y[rows, N] (+)= X[rows, K] · Wᵀ on the tensor cores. y may be float32 (the reference's default), float16
-        (`halfOut`) or bfloat16. rows must be a multiple of 64 (Linear.swift:695)."""
+        (`halfOut`) or bfloat16. rows must be a multiple of 64 (Linear.swift:695). The workspace serves one call at a time; the order of an
+        element's fp32 sum over K depends on rows, N and whether the workspace has room for partial sums."""
         if not (x.is_cuda and y.is_cuda):
             _no_cpu()
         d = self._described()
