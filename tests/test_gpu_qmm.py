@@ -313,3 +313,28 @@ def test_dense_ffn_scratch_outlives_fewer_rows(cuda_device):
     assert torch.equal(got, want)
     for fmt in (torch.bfloat16, torch.float16):
         assert dn.qmm_workspace_bytes(4096, fmt) >= max(dn.qmm_workspace_bytes(r, fmt) for r in range(64, 4096, 64))
+
+
+@pytest.mark.parametrize("group", [64, 32])
+def test_qmm_affine4_weights_are_one_rounding_at_any_scale(cuda_device, group):
+    """Unit rows of x read the fp16 weights back: fma(q, s, b) rounded once, for scales just below and at 2^-4 (from where on the codes are
+    converted another way, for all 32 rows of a warp as soon as one of their scales is that large), tiny, large and negative ones."""
+    rng = np.random.default_rng(30 + group)
+    N, K, M = 256, 512, 64
+    w, _, _ = synth.affine_np(rng, N, K, 4, 1, group)
+    s = rng.uniform(0.001, 0.0624, size=(1, N, K // group)).astype(np.float32) * rng.choice([-1, 1], size=(1, N, K // group))
+    s[0, 32:64] = 2.0 ** rng.integers(-30, -5, size=(32, K // group))
+    s[0, 70, ::2] = 0.0625           # one row of a warp, every other group
+    s[0, 100:128] = rng.uniform(0.05, 300, size=(28, K // group))
+    s[0, 130, 1] = -0.0625
+    s[0, 131] = 0.06225586           # the largest below
+    s = synth.bf16_bits_to_f32(synth.to_bf16_bits(s.astype(np.float32)))
+    b = synth.bf16_bits_to_f32(synth.to_bf16_bits((-8 * s + rng.normal(0, 0.001, size=s.shape)).astype(np.float32)))
+    m = synth.dense_q_affine(w, synth.to_bf16_bits(s), synth.to_bf16_bits(b), 4, cuda_device, group)
+    q = np.stack([(w[0] >> (4 * j)) & 15 for j in range(8)], axis=-1).reshape(N, K).astype(np.float64)
+    want = (q * np.repeat(s[0], group, axis=1).astype(np.float64) + np.repeat(b[0], group, axis=1)).astype(np.float16)
+    for k0 in range(0, K, M):
+        x = torch.zeros(M, K, dtype=torch.float16, device=cuda_device)
+        x[torch.arange(M), k0 + torch.arange(M)] = 1
+        got = run_qmm(m, x, M).cpu().numpy()
+        assert np.array_equal(got.T, want[:, k0:k0 + M].astype(np.float32)), k0
