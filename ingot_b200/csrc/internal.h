@@ -83,7 +83,7 @@ int32_t make_map_rowblock(iq_ctx* ctx, CUtensorMap* map, const void* base, uint6
                           uint32_t box_rows);
 // The same through the context's cache, copied into *out; an error code (with the message recorded) when the encoding fails.
 int32_t cached_rowblock_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, int32_t box_rows, CUtensorMap* out);
-int32_t cached_rows16_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, CUtensorMap* out);
+int32_t cached_rows_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, int32_t box_rows, CUtensorMap* out);
 
 struct Tile;
 struct FixedRows;
@@ -182,5 +182,9 @@ int32_t w8a8_init(iq_ctx* ctx);
 int32_t gqmv_init(iq_ctx* ctx);
 int32_t qmm_init(iq_ctx* ctx);
 int32_t moe_init(iq_ctx* ctx);
+int32_t rows_init(iq_ctx* ctx);
+// A plain call of several rows of affine 4- or 8-bit weights on csrc/qmv_rows.cuh, with the ring kernel's sums over its wk K slices. 1: not for
+// this kernel.
+int32_t launch_qmv_rows(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, int wk);
 
 }  // namespace iq

@@ -221,17 +221,17 @@ int32_t cached_rowblock_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t
     return kOk;
 }
 
-// Blocks of 16 rows x 128 bytes with the 128-byte swizzle, of a matrix with any row pitch that is a multiple of 16 bytes.
-int32_t cached_rows16_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, CUtensorMap* out) {
+// Blocks of box_rows rows x 128 bytes with the 128-byte swizzle, of a matrix with any row pitch that is a multiple of 16 bytes.
+int32_t cached_rows_map(iq_ctx* ctx, const void* base, int64_t rows, int32_t row_bytes, int32_t box_rows, CUtensorMap* out) {
     std::lock_guard<std::mutex> hold(ctx->qmv_maps_lock);
     if (ctx->qmv_maps == nullptr) ctx->qmv_maps = new iq_ctx::QmvMap[iq_ctx::kQmvMaps];
     const uintptr_t key = reinterpret_cast<uintptr_t>(base);
-    iq_ctx::QmvMap& e = ctx->qmv_maps[((key >> 8) ^ (key >> 20) ^ (uintptr_t)rows) % iq_ctx::kQmvMaps];
-    if (e.base != base || e.rows != rows || e.row_bytes != row_bytes || e.box_rows != -16) {  // (negative: this kind of map)
+    iq_ctx::QmvMap& e = ctx->qmv_maps[((key >> 8) ^ (key >> 20) ^ (uintptr_t)rows ^ (uintptr_t)(box_rows - 16)) % iq_ctx::kQmvMaps];
+    if (e.base != base || e.rows != rows || e.row_bytes != row_bytes || e.box_rows != -box_rows) {  // (negative: this kind of map)
         e.base = nullptr;
-        const int32_t r = make_map_2d(ctx, &e.map, base, 0, (uint64_t)row_bytes, (uint64_t)rows, (uint64_t)row_bytes, 128, 16, true);
+        const int32_t r = make_map_2d(ctx, &e.map, base, 0, (uint64_t)row_bytes, (uint64_t)rows, (uint64_t)row_bytes, 128, (uint32_t)box_rows, true);
         if (r != kOk) return r;
-        e.base = base; e.rows = (int32_t)rows; e.row_bytes = row_bytes; e.box_rows = -16;
+        e.base = base; e.rows = (int32_t)rows; e.row_bytes = row_bytes; e.box_rows = -box_rows;
     }
     *out = e.map;
     return kOk;

@@ -204,6 +204,22 @@ QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms, bool wk8, b
                 if (fits(kQrShapes23[v], w)) { best.max_rows = qr_shape_rows(kQrShapes23[v]); break; }
     return best;
 }
+// Where csrc/qmv_rows.cuh takes a plain call over, one launch for any rows: by the rows that a launch here holds (max_rows: of 4-bit weights two above
+// some 8000 inputs, four above 7000, eight above 4000; of 8-bit ones four above 8000), and by whether the launches here share one conversion of the
+// activations (pre, the dense FFN's down projection). us here / there:
+// 4 bits, two rows a launch, 5 / 8 / 9 / 16 rows: 4096 x 14336 38.3 / 24.4, 53.7 / 27.1, 64.6 / 52.6, 106.3 / 63.3; 5120 x 13824 48.4 / 47.3, 67.1 / 51.3,
+//   81.6 / 56.5, 134.2 / 67.8; as the down projection of an FFN of 4096 / 14336 68.0 / 59.9, 80.0 / 64.4, 109.0 / 117.6, 155.3 / 137.1 for the whole FFN.
+//   Four: 2048 x 7680 at 9 / 13 / 16 rows 23.7 / 25.0, 32.8 / 28.4, 36.9 / 30.4 (FFN at 16 rows 44.9 / 51.1). Eight: 9216 x 5120 at 9 / 16 rows 25.7 / 22.5, 32.5 / 28.8.
+// 8 bits, four rows a launch: 4096 x 14336 at 5 / 8 / 16 rows 36.6 / 28.0, 43.1 / 30.1, 85.5 / 36.4, FFN 68.3 / 64.3, 70.0 / 67.1, 136.4 / 109.3.
+// Groups of 32, two rows a launch, 6 / 8 / 11 / 16 rows: 5120 x 13824 54.2 / 58.4, 72.0 / 62.4, 105.8 / 77.7, 144.0 / 85.5; FFN of 4096 / 14336 at 8 / 11 / 16
+//   rows 95.4 / 78.6, 141.9 / 149.9, 185.3 / 171.0.
+bool rows_kernel_pays(const GqmvCall& c, int nw, int max_rows, bool pre) {
+    if (nw != 1 || c.rows < 5) return false;
+    if (c.fmt == kFmtAffine8) return max_rows <= 4 && (c.N <= 16384 || c.rows > 12);  // (30000 x 12288 at 7 / 12 / 14 rows 153.8 / 157.2, 229.9 / 234.2, 302.9 / 249.3)
+    if (c.fmt == kFmtAffine4G32) return max_rows <= 2 && c.rows > 6 && (c.rows <= 8 || c.rows > (pre ? 13 : 10));
+    if (max_rows <= 2) return !pre || c.rows <= 8 || c.rows > 12;
+    return !pre && ((max_rows == 4 && c.rows > 12) || (max_rows == 8 && c.rows > 8 && c.N >= 8192));
+}
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk8 = false) {
     if (c.rows < 1 || c.rows > 16 || c.N % 16 != 0 || c.K % 64 != 0 || ctx->encode_tiled == nullptr) return 1;
@@ -222,10 +238,18 @@ int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk
     }
     const QrPlan plan = qr_plan(c.fmt, c.n_full > 0 ? c.n_full : c.N, c.K, nw, vec, ctx->sms, wk8, wide);
     if (plan.max_rows == 0 || plan.wk == 0) return 1;
+    // The activations: every CTA converts them, or one more kernel does it for all where that is shorter (a CTA takes about
+    // 1 us per 2000 units of eight inputs, the kernel 1.5 us)
+    const int units = c.rows * (c.K / 8);
+    const bool pre = c.scratch != nullptr && units > kQrPreUnits;
+    if (!wk8 && rows_kernel_pays(c, nw, plan.max_rows, pre)) {
+        const int32_t r = launch_qmv_rows(ctx, st, c, plan.wk);
+        if (r != 1) return r;
+    }
     const int row_bytes = c.fmt == kFmtAffine8 ? c.K : c.K / 2;
     QrMaps maps = {};
     for (int i = 0; i < nw; i++) {
-        const int32_t r = cached_rows16_map(ctx, c.w[i], c.N, row_bytes, &maps.w[i]);
+        const int32_t r = cached_rows_map(ctx, c.w[i], c.N, row_bytes, 16, &maps.w[i]);
         if (r != kOk) return r;
     }
     p.N = c.N; p.K = c.K;
@@ -236,10 +260,6 @@ int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk
     p.runs = wk8 ? 1 : 0;
     p.status = ctx->d_status;
     const size_t xes = c.x_dtype == kF32 ? 4 : 2, yes = c.y_dtype == kF32 ? 4 : 2;
-    // The activations: every CTA converts them, or one more kernel does it for all where that is shorter (a CTA takes about
-    // 1 us per 2000 units of eight inputs, the kernel 1.5 us)
-    const int units = c.rows * (c.K / 8);
-    const bool pre = c.scratch != nullptr && units > kQrPreUnits;
     const size_t rec = (size_t)G * qr_record(c.fmt == kFmtAffine4G32, wide ? kQr23 : kQr16);  // bytes of a row's digits
     if (pre) {
         unsigned char* digits = static_cast<unsigned char*>(c.scratch);

@@ -305,3 +305,25 @@ def test_qmv_mxfp4_row_invariance(cuda_device, N, K):
     for rows in (1, 5, 8, 9, 13):
         assert torch.equal(run(m, xt[:rows].contiguous(), rows), full[:rows]), rows
     assert torch.equal(run(m, xt[11:12].contiguous(), 1)[0], full[11])
+
+
+@pytest.mark.parametrize("bits,group", [(4, 64), (8, 64), (4, 32)])
+@pytest.mark.parametrize("N,K,rows", [(16, 64, 5), (128, 4096, 8), (144, 2048, 9), (1040, 2880, 6), (2064, 1088, 16), (4752, 2048, 7), (4784, 2048, 13),
+                                      (19008, 320, 5), (256, 14336, 16), (256, 14336, 8), (640, 16448, 12)])
+def test_qmv_rows_edges(cuda_device, bits, group, N, K, rows):
+    """Five rows and more (tcgen05): tiles of weight rows and columns of inputs that are not full, one to eight CTAs per tile, several tiles
+    per CTA, left-over blocks with K slices of their own (4784 rows of 2048 inputs), both heights; against the oracle, added to y, and every
+    row with the bits that it has alone."""
+    rng = np.random.default_rng(900 + bits + group + N + K + rows)
+    m, host = affine_case(rng, N, K, bits, cuda_device, group=group)
+    x = synth.activations_np(rng, rows, K)
+    xt = x_tensor(x, cuda_device)
+    y = run(m, xt, rows)
+    assert qref.max_rel(y.cpu().numpy(), qref.matmul_t(x, deq(host, bits, group=group))) <= TOL
+    for i in (0, rows // 2, rows - 1):
+        assert torch.equal(run(m, xt[i:i + 1].contiguous(), 1)[0], y[i]), i
+    y2 = y.clone()
+    VQMV.encode(xt, m, y2, rows, accumulate=True)
+    assert torch.equal(y2, y + y)
+    assert torch.equal(run(m, xt, rows, y_dtype=torch.float16), y.to(torch.float16))
+    assert capi.context(0).device_status() == 0
