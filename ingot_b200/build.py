@@ -20,7 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libingot_qmm.so")
 PYCALL = os.path.join(LIBDIR, "_iqcall.so")
-SOURCES = ["api.cu", "qmv.cu", "moe.cu", "qmm.cu", "rows.cu", "ep.cu", "colsplit.cu", "loader.cu", "sample.cu", "embed.cu", "tern.cu", "w8a8.cu"]
+SOURCES = ["api.cu", "qmv.cu", "moe.cu", "qmm.cu", "tile.cu", "rows.cu", "ep.cu", "colsplit.cu", "loader.cu", "sample.cu", "embed.cu", "tern.cu", "w8a8.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

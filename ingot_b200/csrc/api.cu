@@ -82,6 +82,7 @@ extern "C" int32_t iq_ctx_create(int32_t device, iq_ctx** out) {
     if (st == kOk) st = gqmv_init(ctx);
     if (st == kOk) st = qmm_init(ctx);
     if (st == kOk) st = moe_init(ctx);
+    if (st == kOk) st = tile_init(ctx);
     if (st == kOk) st = rows_init(ctx);
     if (st == kOk) st = w8a8_init(ctx);
     if (st != kOk) {

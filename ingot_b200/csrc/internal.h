@@ -119,7 +119,6 @@ struct GqmvCall {
     int32_t act = 0;  // gate/up mode: activation (kAct*)
     bool early = false;  // tiles: the list is complete when the launch's predecessor lets it start (a launch of the same kind did)
     void* scratch = nullptr;  // device memory of rows * K * 7 / 2 bytes that the call may use (256-byte aligned), or null
-    const FixedRows* fx = nullptr;  // grouped gate/up: the token rows as block fixed point, when the caller has them
 };
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
 // iq_qmv with scratch (see GqmvCall)
@@ -127,8 +126,6 @@ int32_t qmv_with_scratch(iq_ctx* ctx, void* stream, const void* x, int32_t x_dty
                          int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix, void* scratch);
 // Tiles of up to eight rows of affine 4-bit experts on the int8 kernel; 1: the shape does not fit it
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
-// Whether its gate/up form takes the token rows as fixed point (GqmvCall::fx) for K inputs; for others it converts them itself
-bool qmv_grouped_takes_fixed(const iq_ctx* ctx, int K);
 
 // Scratch of the GEMM's K split (csrc/qmm_ta.cuh). bytes: what the split of a dense GEMM takes (0: it is not split); part: null where
 // the scratch does not hold that.
@@ -176,12 +173,18 @@ struct QmmCall {
     QmmSplit split;   // quantized formats: scratch of the K split, or none
 };
 int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c);
+// A list of tiles of up to eight rows (c.bn) of affine 4-bit experts on csrc/qmv_tile.cuh, x as block fixed point (wide: three digits, gate/up only):
+// row row_map[position] / topk, or the position itself. Gate/up stores h as fp32. 1: not for this kernel.
+int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t max_tiles);
+// Rows as block fixed point, and as halves (copy, or null)
+int32_t launch_fixed_rows(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, int rows, int D, const FixedRows& fx, bool wide, __half* copy);
 int32_t launch_tern_qmv(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
                         int32_t y_dtype, int64_t ldy, int32_t rows, int32_t n, int32_t accumulate);
 int32_t w8a8_init(iq_ctx* ctx);
 int32_t gqmv_init(iq_ctx* ctx);
 int32_t qmm_init(iq_ctx* ctx);
 int32_t moe_init(iq_ctx* ctx);
+int32_t tile_init(iq_ctx* ctx);
 int32_t rows_init(iq_ctx* ctx);
 // A plain call of several rows of affine 4- or 8-bit weights on csrc/qmv_rows.cuh, with the ring kernel's sums over its wk K slices. 1: not for
 // this kernel.

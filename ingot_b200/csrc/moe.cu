@@ -36,9 +36,10 @@ struct MoeWs {
     Tile* tiles_a;
     Tile* tiles_b;
     __half* h;
+    float* h32;  // h before it is rounded (decode tiles)
     void* yd;
     __half* xs;  // activations in expert order, fp16 [P, d_model] (tensor-core path)
-    FixedRows fx, fh;  // the activations as block fixed point (up to kFixedTokens); h likewise (up to kSmallTokens)
+    FixedRows fx, fh;  // the activations as block fixed point and h likewise, as far as the int8 kernels go
     // shared expert (only when the layer has one): fp16 copy of x, h, output, per-token weight, tile list
     __half* s_x16;
     __half* s_h;
@@ -52,6 +53,17 @@ constexpr int kDecodeTileRows = 8;  // token rows per tile of the int8 expert ke
 constexpr int kRouterSmemMax = 200 * 1024;
 constexpr int kGroupChunkedMinPairs = 4096;  // from here on the permutation runs as a chunked counting sort
 constexpr int kFixedTokens = 512;  // up to here the counting kernel leaves the activations as fixed point for the int8 kernels
+// Affine experts run on the decode tiles (csrc/qmv_tile.cuh) while they see a few rows each on average; everything else, MXFP4 experts at any number of
+// rows, runs on the grouped GEMM. The tiles take the token rows as two digits (16 bits of a group's largest input) where their predecessor on
+// mma.sync did: 256 to 4096 inputs, a power of two, up to six rows per expert. Elsewhere the GEMM ran, which takes bf16 activations whole, and so do
+// three digits (23 bits): with a few input channels 100 times the rest, or one of every 64 300 times, two are 4.4e-4 to 4.9e-4 off the 64-bit result (24
+// tokens, 32 experts of 2880 x 768), the GEMM 3.0e-4, three 2.4e-4. MoE block, us, tiles / GEMM (eight, four, six and eight experts per token):
+//   128 experts of 2048 x 768, two digits    20 tokens 77 / 103, 64 97 / 128, 96 (6 rows) 115 / 135; three digits 112 (7 rows) 157 / 135
+//   32 of 4096 x 2048, two digits            20 tokens 118 / 153, 48 (6 rows) 140 / 170; three digits 64 (8 rows) 213 / 165
+//   64 of 3072 x 1408, three digits          8 tokens 106 / 112, 20 148 / 151, 40 (3.8 rows) 165 / 168, 64 (6 rows) 180 / 169
+//   128 of 2880 x 768, three digits          8 tokens 92 / 95, 20 131 / 147, 64 (4 rows) 174 / 183, 80 (5 rows) 198 / 191
+constexpr int kInt8RowsPerExpert = 6, kWideRowsPerExpert = 4;
+bool two_digit_inputs(const iq_moe* l) { return l->d.d_model >= 256 && l->d.d_model <= 4096 && (l->d.d_model & (l->d.d_model - 1)) == 0; }
 // Router products (tokens x experts x inputs) up to which a block takes eight tokens against a few experts in float64 (about
 // 0.35 us per million): beyond, the tensor cores with exact refinement (22 us at 27 to 400 million) where they apply, else the
 // tiled float64 GEMM. 128 experts x 2048 inputs, router and top-k: 128 tokens 22.8 -> 14.4 us, 200 tokens 22.5 -> 20.4, 400
@@ -87,11 +99,14 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     w.h = static_cast<__half*>(take(P * d.d_ff * 2));
     w.yd = take(P * d.d_model * (yd_dtype_of(l) == kF16 ? 2 : 4));
     w.xs = static_cast<__half*>(take(P * d.d_model * 2));
-    const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens, fixed = tokens < kFixedTokens ? tokens : kFixedTokens;
-    w.fx.digits = static_cast<unsigned char*>(take((fixed * 128 + few * 64) * (d.d_model / 64)));  // (few tokens: the wide form)
+    const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens;
+    const size_t pairs = l->fmt != kFmtAffine4 ? few * d.top_k : std::min(P, (size_t)d.expert_count * kInt8RowsPerExpert);
+    const size_t fixed = std::max(few, std::min((size_t)tokens, (size_t)d.expert_count * kInt8RowsPerExpert / d.top_k));
+    w.h32 = static_cast<float*>(take(l->fmt == kFmtAffine4 ? pairs * d.d_ff * 4 : 0));
+    w.fx.digits = static_cast<unsigned char*>(take(fixed * 192 * (d.d_model / 64)));  // (the wide form)
     w.fx.scale = static_cast<float2*>(take(fixed * (d.d_model / 64) * 8));
-    w.fh.digits = static_cast<unsigned char*>(take(few * d.top_k * (d.d_ff / 64) * 192));
-    w.fh.scale = static_cast<float2*>(take(few * d.top_k * (d.d_ff / 64) * 8));
+    w.fh.digits = static_cast<unsigned char*>(take(std::max(pairs * 128, few * d.top_k * 192) * (d.d_ff / 64)));
+    w.fh.scale = static_cast<float2*>(take(std::max(pairs, few * d.top_k) * (d.d_ff / 64) * 8));
     w.s_x16 = nullptr; w.s_h = nullptr; w.s_yd = nullptr; w.s_w = nullptr;
     if (d.shared != IQ_SHARED_NONE) {
         const size_t T = (size_t)tokens;
@@ -172,8 +187,7 @@ int32_t launch_route(iq_moe* l, cudaStream_t st, const float* logits, int ld, in
 // On the int8 kernels; 1: the shape does not fit them. Gate + up + activation of every tile: h[row, :] = half(act(x W_gate^T + b_g, x W_up^T + b_u)). Expert e's weights live
 // at local slot e - expert_lo: the offset is folded into the base pointers. row_map == nullptr: x rows are in place.
 int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, int64_t ldx, const uint32_t* row_map,
-                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, __half* h, int row_map_div = 0,
-                   const FixedRows* fx = nullptr) {
+                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, __half* h, int row_map_div) {
     const iq_moe_desc& d = l->d;
     const int64_t lo = d.expert_lo;
     GqmvCall c;
@@ -193,7 +207,7 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
     c.expert_lo = d.expert_lo; c.expert_count = d.expert_count;
     c.N = d.d_ff; c.K = d.d_model;
     c.x = x; c.x_dtype = x_dtype; c.ldx = ldx;
-    c.row_map = row_map; c.topk = row_map_div > 0 ? row_map_div : d.top_k;  // x row = row_map[sorted position] / divisor
+    c.row_map = row_map; c.topk = row_map_div;  // x row = row_map[sorted position] / divisor
     c.tiles = tiles; c.ntiles = ntiles; c.grid_tiles = max_tiles;
     c.rows = 0; c.max_rows = kDecodeTileRows;
     c.y = h; c.y_dtype = kF16; c.ldy = d.d_ff;
@@ -203,7 +217,6 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
     }
     c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
     c.act = d.act;
-    c.fx = fx;
     return launch_qmv_imma_grouped(l->ctx, cs, c);
 }
 
@@ -232,12 +245,12 @@ int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles,
     return launch_qmv_imma_grouped(l->ctx, cs, c);
 }
 
-// The affine experts run on the int8 kernels while they see up to six rows each on average; those need no dequantisation but
-// work through a tile four rows at a time. 128 experts of 2048 x 768, 8 of them per token, gate/up and down together: 64 tokens
-// (4 rows) 124 us against 139 on the grouped GEMM, 128 tokens (8 rows) 168 against 145. Everything else, MXFP4 experts
-// at any number of rows, runs on the grouped GEMM (MXFP4 at 4 tokens 132 -> 87 us for the layer, at 64 tokens 406 -> 145).
-constexpr int kInt8RowsPerExpert = 6;
-bool use_int8_path(const iq_moe* l, int64_t rows, int64_t expert_slots) { return l->fmt == kFmtAffine4 && rows <= expert_slots * kInt8RowsPerExpert; }
+bool use_int8_path(const iq_moe* l, int64_t rows) {
+    return l->fmt == kFmtAffine4 && rows <= (int64_t)l->d.expert_count * (two_digit_inputs(l) ? kInt8RowsPerExpert : kWideRowsPerExpert);
+}
+// The limit of the expert-parallel pieces, whose rows come as halves, on csrc/qmv_imma_grouped.cuh (128 experts of 2048 x 768, gate/up and down together: four
+// rows each 124 us against 139 on the grouped GEMM, eight 168 against 145)
+constexpr int kEpInt8RowsPerExpert = 6;
 // Token rows per tile of the grouped GEMM, by the average rows per expert. Up to 64 rows two CTAs share an SM (and 32 hold two
 // stages of activations more than 64); from 96 rows on every weight tile is dequantised less often at 192.
 int tensor_tile_rows(int64_t rows, int64_t expert_slots) {
@@ -281,6 +294,37 @@ int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows,
     c.early = early;
     c.split = split;
     return launch_qmm(l->ctx, cs, c);
+}
+
+// The same on tiles of up to eight rows, from block fixed point (csrc/qmv_tile.cuh): h as fp32, yd
+int32_t run_gateup_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, int max_tiles) {
+    const iq_moe_desc& d = l->d;
+    QmmCall c;
+    c.fmt = l->fmt; c.epi = 1; c.bn = kDecodeTileRows;
+    c.w[0] = d.gate.w; c.w[1] = d.up.w;
+    c.s[0] = d.gate.scales; c.s[1] = d.up.scales;
+    c.b[0] = d.gate.biases; c.b[1] = d.up.biases;
+    c.experts = d.expert_count; c.expert_lo = d.expert_lo;
+    c.N = d.d_ff; c.K = d.d_model;
+    c.tiles = w.tiles_a; c.ntiles = w.ntiles;
+    c.y = w.h32; c.y_dtype = kF32; c.ldy = d.d_ff;
+    c.ebias[0] = d.gate_bias; c.ebias[1] = d.up_bias;
+    c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
+    c.act = d.act;
+    return launch_qmv_tile(l->ctx, cs, c, w.fx, wide, w.row_map, d.top_k, max_tiles);
+}
+int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles, bool early) {
+    const iq_moe_desc& d = l->d;
+    QmmCall c;
+    c.fmt = l->fmt; c.epi = 0; c.bn = kDecodeTileRows;
+    c.w[0] = d.down.w; c.s[0] = d.down.scales; c.b[0] = d.down.biases;
+    c.experts = d.expert_count; c.expert_lo = d.expert_lo;
+    c.N = d.d_model; c.K = d.d_ff;
+    c.tiles = w.tiles_a; c.ntiles = w.ntiles;
+    c.y = w.yd; c.y_dtype = yd_dtype_of(l); c.ldy = d.d_model;
+    c.ebias[0] = d.down_bias;
+    c.early = early;
+    return launch_qmv_tile(l->ctx, cs, c, w.fh, false, nullptr, 1, max_tiles);
 }
 
 // ---- few tokens (csrc/moe_small.cuh) ----
@@ -773,9 +817,10 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     int32_t st;
 
     const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l);
-    const bool takes_fixed = l->fmt == kFmtAffine4 && qmv_grouped_takes_fixed(ctx, d.d_model);
+    const bool int8 = use_int8_path(l, P);
+    const bool wide = !two_digit_inputs(l);
     if (small) {
-        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, small_experts || takes_fixed, small_experts);
+        st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, small_experts || int8, small_experts || wide);
         if (st == kOk && small_experts)
             st = run_experts_small(l, cs, tokens, w, out, out_dtype, ldo, (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0);
         if (st != kOk) return st;
@@ -848,10 +893,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         st = launch_route(l, cs, w.logits, l->ld, tokens, w.inds, w.wts, fast_router ? x : nullptr, ldx);
         if (st != kOk) return st;
     }
-    const bool int8 = use_int8_path(l, P, d.expert_count);
     const int bn = tensor_tile_rows(P, d.expert_count);
-    // whole calls on the int8 kernels: the counting kernel leaves the activations as fixed point for the gate/up one, where that takes them
-    const bool fixed = int8 && takes_fixed && (pieces & IQ_PIECE_GATEUP) && (small || ((pieces & IQ_PIECE_GROUP) && tokens <= kFixedTokens && P < kGroupChunkedMinPairs));
+    // whole calls on the decode tiles: the counting kernel leaves the activations as fixed point
+    const bool fixed = int8 && (pieces & IQ_PIECE_GATEUP) && (small || ((pieces & IQ_PIECE_GROUP) && tokens <= kFixedTokens && P < kGroupChunkedMinPairs));
     if (pieces & IQ_PIECE_GROUP) {
         GroupParams gp;
         gp.inds = inds; gp.counts = w.counts; gp.offsets = w.offsets; gp.row_map = w.row_map; gp.pos = w.pos;
@@ -870,7 +914,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
             if (st == kOk) st = check_cuda(ctx, launch_dependent(moe_scan_kernel, dim3(1), 256, 0, cs, gp), "moe_scan launch");
             if (st == kOk) st = check_cuda(ctx, launch_dependent(moe_place_kernel, dim3(gp.chunks), 256, d.experts * 8 * 4, cs, gp), "moe_place launch");
         } else {
-            if (fixed) { gp.fx = w.fx; gp.x = x; gp.x_dtype = x_dtype; gp.ldx = ldx; gp.T = tokens; gp.D = d.d_model; }
+            if (fixed) { gp.fx = w.fx; gp.fx_wide = wide ? 1 : 0; gp.x = x; gp.x_dtype = x_dtype; gp.ldx = ldx; gp.T = tokens; gp.D = d.d_model; }
             st = check_cuda(ctx, launch_dependent(moe_count_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_count launch");
             if (st != kOk) return st;
             st = check_cuda(ctx, launch_dependent(moe_scatter_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_scatter launch");
@@ -882,8 +926,11 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     // which kernel made h: a down projection on the same one may start on the tile list and its weights before h is there
     bool after_int8 = false, after_gemm = false;
     if (pieces & IQ_PIECE_GATEUP) {
-        st = int8 ? run_gateup(l, cs, x, x_dtype, ldx, w.row_map, w.tiles_a, w.ntiles, max_tiles, w.h, 0, fixed ? &w.fx : nullptr) : 1;
+        st = int8 && !fixed ? launch_fixed_rows(ctx, cs, x, x_dtype, ldx, tokens, d.d_model, w.fx, wide, nullptr) : kOk;
+        if (st == kOk) st = int8 ? run_gateup_tile(l, cs, w, wide, max_tiles) : 1;
         after_int8 = st == kOk;
+        // h as halves (the view) and as fixed point for the down projection, from the sums' 32 bits
+        if (after_int8) st = launch_fixed_rows(ctx, cs, w.h32, kF32, d.d_ff, P, d.d_ff, w.fh, false, w.h);
         if (st == 1) {
             after_gemm = true;
             st = check_cuda(ctx, launch_dependent(moe_pack_tokens_kernel, dim3(tokens), 256, 0, cs, x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k),
@@ -893,7 +940,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st != kOk) return st;
     }
     if (pieces & IQ_PIECE_DOWN) {
-        st = int8 ? run_down(l, cs, w.h, w.tiles_a, w.ntiles, max_tiles, w.yd, yd_dtype_of(l), after_int8) : 1;
+        st = int8 && !after_gemm ? run_down_tile(l, cs, w, max_tiles, after_int8) : 1;
         if (st == 1) st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn, after_gemm);
         if (st != kOk) return st;
     }
@@ -1006,7 +1053,7 @@ int32_t moe_experts_impl(iq_moe* l, void* stream, const void* rows_f16, const ui
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
     const int64_t slots = (int64_t)sources * d.expert_count;
     // the row count is only known on the device: bounds come from the capacity, total_rows picks the kernels
-    const bool int8 = use_int8_path(l, total_rows, slots);
+    const bool int8 = l->fmt == kFmtAffine4 && total_rows <= slots * kEpInt8RowsPerExpert;
     const int bn = int8 ? 16 : tensor_tile_rows(total_rows, slots);  // (where a shape does not fit the int8 kernels the GEMM takes their tiles)
     ep_tiles_kernel<<<1, 512, 0, cs>>>(counts, sources, d.experts, d.expert_lo, d.expert_count, int8 ? kDecodeTileRows : bn,
                                        (uint32_t)region_rows, w.tiles, w.ntiles);

@@ -569,6 +569,7 @@ struct GroupParams {
     int32_t chunks;
     // the counting kernel also turns the activations into fixed point for the decode kernels (fx.digits null: it does not)
     FixedRows fx;
+    int32_t fx_wide;  // ... with three digits
     const void* x;
     int32_t x_dtype;
     int64_t ldx;
@@ -581,7 +582,10 @@ __global__ void __launch_bounds__(256) moe_count_kernel(const GroupParams p) {
     pdl_launch_dependents();
     pdl_wait();
     if (p.fx.digits != nullptr)
-        for (int t = blockIdx.x; t < p.T; t += gridDim.x) fixed_point_row<false>(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
+        for (int t = blockIdx.x; t < p.T; t += gridDim.x) {
+            if (p.fx_wide) fixed_point_row<true>(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
+            else fixed_point_row<false>(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
+        }
     uint32_t c = 0;
     for (int i = threadIdx.x; i < p.P; i += 256) c += p.inds[i] == e;
 #pragma unroll

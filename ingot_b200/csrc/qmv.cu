@@ -423,21 +423,14 @@ typedef void (*QgKernel)(const CUtensorMap, const CUtensorMap, const QgParams);
 template <int MODE, bool TM>
 QgKernel qg_pick_mt(bool gw4) {
     constexpr bool TWO = MODE == kModeDown;
-    return gw4 ? qmv_imma_grouped_kernel<MODE, TM, 4, 8, TWO> : qmv_imma_grouped_kernel<MODE, TM, 0, 8, TWO>;
+    return gw4 ? qmv_imma_grouped_kernel<MODE, TM, 4, TWO> : qmv_imma_grouped_kernel<MODE, TM, 0, TWO>;
 }
-// fx: the inputs of a gate/up that takes the rows as fixed point, or 0.
-// The two-wide fp32 form costs registers (gate/up spills 72 bytes instead of 60): it pays in the down projections and in gate/up of up
-// to 2048 inputs on sixteen warps. MoE block, us, plain / everywhere / as here: 128 experts of 2048 x 768 at 64 tokens 125.8 / 122.6 / 122.9,
-// 64 of 2048 x 1408 at 12 tokens 98.2 / 100.5 / 98.5, 128 of 4096 x 1536 at 12 tokens 193.5 / 198.4 / 191.5 and at 64 364.8 / 370.8 / 357.8.
-QgKernel qg_pick(int mode, bool tm, bool gw4, int fx = 0) {
-    if (fx) return fx <= 2048 ? qmv_imma_grouped_kernel<kModeGateUp, true, 4, 16, true> : qmv_imma_grouped_kernel<kModeGateUp, true, 4, 16, false>;
+// (the two-wide fp32 form costs registers: it pays in the down projections)
+QgKernel qg_pick(int mode, bool tm, bool gw4) {
     if (mode == kModeGateUp) return tm ? qg_pick_mt<kModeGateUp, true>(gw4) : qg_pick_mt<kModeGateUp, false>(gw4);
     return tm ? qg_pick_mt<kModeDown, true>(gw4) : qg_pick_mt<kModeDown, false>(gw4);
 }
 }  // namespace
-
-// Sixteen consumer warps: K slices of four groups that divide them (K = 256, 512, 1024, 2048, 4096)
-bool qmv_grouped_takes_fixed(const iq_ctx* ctx, int K) { return ctx->encode_tiled != nullptr && K % 256 == 0 && K <= 4096 && 16 % (K / 256) == 0; }
 
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
@@ -465,19 +458,15 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     p.srow_bytes = G * 2;
     p.xq_bytes = G * ms * 512;
     p.xsc_bytes = G * ms * 32;
-    // Sixteen consumer warps with the token rows as fixed point: gate/up tiles of eight rows
-    const bool fx = c.fx != nullptr && c.mode == kModeGateUp && tm && c.row_map != nullptr && qmv_grouped_takes_fixed(ctx, c.K);
-    const int kQgWarps = fx ? 16 : 8;
-    if (fx) { p.fx = *c.fx; p.xq_bytes = p.xsc_bytes = 0; }
     p.red_bytes = 2 * kQgWarps * nw * ms * 64 * 4;
     const int fixed = p.xq_bytes + p.xsc_bytes + p.red_bytes + 256 + (tm ? 1024 : 0);
     // K slices per block of rows: one slice of four groups per warp when K allows it (the activation
     // fragments then live in registers: 69 against 83 us on the 64-token layer); else four slices (32-row blocks: half as
     // many hand-overs per byte) when two stages of that size fit, else eight.
     int ctas = 1, nstages = 0;
-    const bool gw4 = fx || G == 4 * kQgWarps;
-    const int cand[4] = {fx ? G / 4 : (gw4 ? kQgWarps : kQgWarps / 2), kQgWarps, kQgWarps / 4, kQgWarps / 8};
-    for (int ci = 0; ci < (fx ? 1 : 4) && nstages < 2; ci++) {
+    const bool gw4 = G == 4 * kQgWarps;
+    const int cand[4] = {gw4 ? kQgWarps : kQgWarps / 2, kQgWarps, kQgWarps / 4, kQgWarps / 8};
+    for (int ci = 0; ci < 4 && nstages < 2; ci++) {
         const int wk = cand[ci];
         if (G % wk != 0 || (G / wk) % 4 != 0) continue;  // a warp's K slice: runs of four groups
         const int R = 16 * (kQgWarps / wk);
@@ -487,11 +476,6 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
         p.mat_bytes = round_up(R * p.row_pitch + 2 * R * p.srow_bytes, tm ? 1024 : 16);
         p.stage_bytes = nw * p.mat_bytes;
         nstages = (kQsSmemMax - fixed) / p.stage_bytes;
-    }
-    if (nstages < 2 && fx) {
-        GqmvCall without = c;
-        without.fx = nullptr;
-        return launch_qmv_imma_grouped(ctx, st, without);
     }
     if (nstages < 2) return 1;
     if (nstages > 8) nstages = 8;
@@ -528,7 +512,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)(items < slots ? items : slots), 1, 1);
-    cfg.blockDim = dim3(qg_threads(kQgWarps), 1, 1);
+    cfg.blockDim = dim3(kQgThreads, 1, 1);
     cfg.dynamicSmemBytes = fixed + nstages * p.stage_bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -536,7 +520,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, gw4 && p.wk == kQgWarps, fx ? c.K : 0), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, gw4 && p.wk == kQgWarps), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
 }
 
 int32_t gqmv_init(iq_ctx* ctx) {
@@ -550,11 +534,6 @@ int32_t gqmv_init(iq_ctx* ctx) {
     for (int i = 0; i < 14; i++) {
         cudaError_t e = cudaFuncSetAttribute(qi[i], cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma)");
-    }
-    for (int fx = 2048; fx <= 4096; fx += 2048) {
-        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(kModeGateUp, true, true, fx)),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
-        if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
     }
     for (int mode = kModeGateUp; mode <= kModeDown; mode++)
         for (int v = 0; v < 4; v++) {  // bulk or tensor copies; activations in registers or not

@@ -1,5 +1,6 @@
-// MoE decode on the int8 tensor-core path: the expert tiles' gate + up + activation and down projections for tiles of
-// up to eight routed rows (affine 4-bit experts). Same arithmetic as qmv_imma.cuh: codes enter m16n8k32 u8 x s8 MMAs
+// Decode of the expert-parallel pieces on the int8 tensor-core path: the expert tiles' gate + up + activation and down projections
+// for tiles of up to eight routed rows (affine 4-bit experts), which come and go as halves in the exchange's regions (whole
+// layers run on qmv_tile.cuh). Same arithmetic as qmv_imma.cuh: codes enter m16n8k32 u8 x s8 MMAs
 // unconverted, the tile's activation rows are converted once per tile to block fixed point (two signed 8-bit digits per
 // group of 64 inputs), per group y += s * 2^(e-15) * (256 * acc_hi + acc_lo) + b * sum(x); a row's bits do not depend on
 // the other rows of its tile.
@@ -19,18 +20,15 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "fixed_rows.cuh"
 #include "gqmv.cuh"
 #include "ptx.cuh"
 #include "qmv_imma.cuh"
 
 namespace iq {
 
-// epilogue warps: add the K slices, apply the activation, store (three beside sixteen consumers: twenty warps leave 96
-// registers a thread, twenty-one 80)
-constexpr int qg_epilogue_warps(int consumers) { return consumers == 16 ? 3 : 4; }
-// consumer warps (row blocks x K slices); one producer warp follows them, then the epilogue warps
-constexpr int qg_threads(int consumers) { return (consumers + 1 + qg_epilogue_warps(consumers)) * 32; }
+constexpr int kQgWarps = 8;          // consumer warps (row blocks x K slices); one producer warp follows them, then the epilogue warps,
+constexpr int kQgEpilogueWarps = 4;  // which add the K slices, apply the activation and store
+constexpr int kQgThreads = (kQgWarps + 1 + kQgEpilogueWarps) * 32;
 
 __device__ __forceinline__ void qg_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void qg_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
@@ -55,7 +53,6 @@ struct QgParams {
     float limit;
     int32_t act;
     int32_t early;               // the tile list is complete when this kernel starts
-    FixedRows fx;                // sixteen consumer warps: the token rows as block fixed point
     int32_t rgs, wk;             // row blocks of 16 per item x K slices = consumer warps
     int32_t NB;                  // items per tile
     int32_t row_bytes, row_pitch, srow_bytes;
@@ -72,20 +69,13 @@ struct QgParams {
 // GW: groups of 64 inputs per consumer warp when fixed at compile time (4), else 0. A warp's K slice does not change from
 // item to item, so with GW > 0 its activation fragments stay in registers between tile changes: read from shared
 // memory per item they are as many bytes as the codes themselves, and the kernel runs at the shared-memory port's rate.
-// NCW: consumer warps, 8 or 16. Sixteen (32-row items, gate/up with GW = 4) take the token rows as fixed point from fx instead
-// of converting them per CTA and tile: the conversion's shared memory goes to the ring, its instructions away, and with
-// twice the warps per scheduler the latencies of a warp's chain (shared-memory loads, shuffles, MMAs, the hand-over) hide
-// behind one another: eight warps issued 0.43 instructions per cycle and scheduler.
 // TWO: scales and biases by two-wide fp32 operations, three instructions for six, rounded alike (qg_pick).
-template <int MODE, bool TM, int GW, int NCW, bool TWO>
-__global__ void __launch_bounds__(qg_threads(NCW), 1)
+template <int MODE, bool TM, int GW, bool TWO>
+__global__ void __launch_bounds__(kQgThreads, 1)
     qmv_imma_grouped_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, const QgParams p) {
     constexpr int NW = MODE == kModeGateUp ? 2 : 1;
     constexpr int MS = 2;   // sets of four activation rows per tile
     constexpr int GB = 32;  // code bytes per group of 64 inputs (4-bit)
-    constexpr int kQgWarps = NCW;
-    constexpr bool FX = NCW == 16;
-    static_assert(!FX || (GW > 0 && TM && MODE == kModeGateUp), "sixteen consumer warps: the gate/up form with fragments in registers");
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char* xq = smem;                                            // [groups][MS][32 lanes] uint4: B fragments
     float2* xsc = reinterpret_cast<float2*>(smem + p.xq_bytes);          // [groups][MS * 4 rows] {2^(e-15), sum x}
@@ -100,7 +90,7 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NCT = kQgWarps * 32;     // consumer threads
-    constexpr int NET = qg_epilogue_warps(NCW) * 32;  // epilogue threads
+    constexpr int NET = kQgEpilogueWarps * 32;  // epilogue threads
     if (TM && tid == NCT) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map0) : "memory");
         if (NW == 2) asm volatile("prefetch.tensormap [%0];" ::"l"(&map1) : "memory");
@@ -260,29 +250,7 @@ __global__ void __launch_bounds__(qg_threads(NCW), 1)
         int s = 0, ti = lo / p.NB, blk = lo % p.NB;
         uint32_t ph = 0;
         for (int item = lo, it = 0; item < hi; item++, it++) {
-            if (FX && ti != cur_tile) {
-                // ---- this tile's fragments: digit g % 2 of row g / 2 of the set, scales of row t of the set ----------------
-                cur_tile = ti;
-                tile = p.tiles[ti];
-                M = min((int)tile.count, 4 * MS);
-                sets = (M + 3) >> 2;
-                const int G64 = p.K / 64;
-#pragma unroll
-                for (int c = 0; c < MS; c++) {
-                    const int m = 4 * c + (g >> 1), mt = 4 * c + t;
-                    const size_t rx = p.row_map[tile.start + min(m, M - 1)] / (uint32_t)p.topk;
-                    const size_t rt = p.row_map[tile.start + min(mt, M - 1)] / (uint32_t)p.topk;
-                    const unsigned char* xd = p.fx.digits + (rx * G64 + g0) * 128 + (g & 1) * 64 + t * 16;
-                    const float2* xs = p.fx.scale + rt * G64 + g0;
-#pragma unroll
-                    for (int q = 0; q < (GW > 0 ? GW : 1); q++) {
-                        xbr[q][c] = __ldg(reinterpret_cast<const uint4*>(xd + q * 128));
-                        if (m >= M) xbr[q][c] = make_uint4(0, 0, 0, 0);
-                        xsr[q][c] = __ldg(xs + q);
-                    }
-                }
-            }
-            if (!FX && ti != cur_tile) {
+            if (ti != cur_tile) {
                 // ---- this tile's activation rows -> block fixed point in B-fragment order (see qmv_imma.cuh) -----------
                 if (cur_tile >= 0) qi_consumer_barrier(NCT);
                 cur_tile = ti;

@@ -542,3 +542,34 @@ def test_moe_int8_experts_by_width(cuda_device, D, I, T):
     rng = np.random.default_rng(95 + D + T)
     layer, host = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
+
+
+@pytest.mark.parametrize("T", [4, 30, 34])
+@pytest.mark.parametrize("D,I", [(448, 192), (2880, 64), (320, 832), (1088, 320), (512, 448)])
+def test_moe_decode_tiles_edges(cuda_device, D, I, T):
+    """The decode tiles' kernel where a step of 256 inputs or a tile of weight rows is not full: seven, forty-five, five and seventeen groups
+    of inputs (scales of rows that are no multiple of eight bytes) as three digits and eight as two, output tiles of 64 of 128 rows, one group
+    of h; experts without rows, with one, with eight and with more (second tiles), biases; both sides of four rows per expert, where three
+    digits end."""
+    rng = np.random.default_rng(D + I + T)
+    E, K = 32, 4
+    layer, host = build_layer(rng, cuda_device, E, K, D, I, biases=True, max_tokens=T)
+    out = check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
+    assert np.isfinite(out.cpu().numpy()).all()
+
+
+def test_moe_decode_tiles_pieces_and_bits(cuda_device):
+    """Gate/up and down alone give the bits of the whole call (h as fixed point then comes from its halves), and a token's bits do not
+    depend on which row of its tiles it is."""
+    rng = np.random.default_rng(77)
+    T, D, I = 40, 512, 320
+    layer, _ = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
+    x = x_tensor(synth.activations_np(rng, T, D), cuda_device)
+    full, part, back = (torch.zeros(T, D, dtype=torch.float32, device=cuda_device) for _ in range(3))
+    layer.encode(x, full, T)
+    for piece in ("router", "route", "group", "gateup", "down", "combine"):
+        layer.encode(x, part, T, only=piece)
+    assert torch.equal(full, part)
+    layer.encode(x.flip(0).contiguous(), back, T)
+    assert torch.equal(back.flip(0), full)
+    assert capi.context(0).device_status() == 0
