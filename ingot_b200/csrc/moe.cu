@@ -52,7 +52,7 @@ struct MoeWs {
 constexpr int kDecodeTileRows = 8;  // token rows per tile of the int8 expert kernels
 constexpr int kRouterSmemMax = 200 * 1024;
 constexpr int kGroupChunkedMinPairs = 4096;  // from here on the permutation runs as a chunked counting sort
-constexpr int kFixedTokens = 512;  // up to here the counting kernel leaves the activations as fixed point for the int8 kernels
+constexpr int kFixedTokens = 512;  // up to here the grouping kernel leaves the activations as fixed point for the int8 kernels
 // Affine experts run on the decode tiles (csrc/qmv_tile.cuh) while they see a few rows each on average; everything else, MXFP4 experts at any number of
 // rows, runs on the grouped GEMM. The tiles take the token rows as two digits (16 bits of a group's largest input) where their predecessor on
 // mma.sync did: 256 to 4096 inputs, a power of two, up to six rows per expert. Elsewhere the GEMM ran, which takes bf16 activations whole, and so do
@@ -894,7 +894,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st != kOk) return st;
     }
     const int bn = tensor_tile_rows(P, d.expert_count);
-    // whole calls on the decode tiles: the counting kernel leaves the activations as fixed point
+    // whole calls on the decode tiles: the grouping kernel leaves the activations as fixed point
     const bool fixed = int8 && (pieces & IQ_PIECE_GATEUP) && (small || ((pieces & IQ_PIECE_GROUP) && tokens <= kFixedTokens && P < kGroupChunkedMinPairs));
     if (pieces & IQ_PIECE_GROUP) {
         GroupParams gp;
@@ -915,9 +915,7 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
             if (st == kOk) st = check_cuda(ctx, launch_dependent(moe_place_kernel, dim3(gp.chunks), 256, d.experts * 8 * 4, cs, gp), "moe_place launch");
         } else {
             if (fixed) { gp.fx = w.fx; gp.fx_wide = wide ? 1 : 0; gp.x = x; gp.x_dtype = x_dtype; gp.ldx = ldx; gp.T = tokens; gp.D = d.d_model; }
-            st = check_cuda(ctx, launch_dependent(moe_count_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_count launch");
-            if (st != kOk) return st;
-            st = check_cuda(ctx, launch_dependent(moe_scatter_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_scatter launch");
+            st = check_cuda(ctx, launch_dependent(moe_group_kernel, dim3(d.experts), 256, 0, cs, gp), "moe_group launch");
         }
         if (st == kOk) st = check_cuda(ctx, cudaGetLastError(), "moe_group launch");
         if (st != kOk) return st;

@@ -552,8 +552,8 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Token->expert permutation, deterministic: inside an expert the pairs keep ascending pair id.
-// count: one block per expert counts its pairs. scatter: one block per expert places them, writes the tile
-// descriptors for two tile heights and, in the last block, the totals.
+// One block per expert counts the pairs, places its own, writes the tile descriptors for two tile heights and, in the last block, the totals.
+constexpr int kGroupMaxExperts = 512;
 struct GroupParams {
     const uint32_t* inds;   // [P] expert of each pair
     uint32_t* counts;       // [E]
@@ -567,7 +567,7 @@ struct GroupParams {
     int32_t e_lo, e_hi;     // experts owned here (expert parallel); tiles are emitted only for these
     uint32_t* chunk_hist;   // [chunks, E] scratch of the chunked form (many pairs)
     int32_t chunks;
-    // the counting kernel also turns the activations into fixed point for the decode kernels (fx.digits null: it does not)
+    // the kernel also turns the activations into fixed point for the decode kernels (fx.digits null: it does not)
     FixedRows fx;
     int32_t fx_wide;  // ... with three digits
     const void* x;
@@ -576,40 +576,32 @@ struct GroupParams {
     int32_t T, D;
 };
 
-__global__ void __launch_bounds__(256) moe_count_kernel(const GroupParams p) {
-    __shared__ uint32_t wsum[8];
-    const uint32_t e = blockIdx.x;
+// A block per expert. Every block counts all pairs by itself (a few thousand at most) instead of waiting for a kernel that counts: one launch
+// less, 128 experts and 512 pairs 4.2 -> 2.7 us (32 pairs 3.5 -> 2.2).
+__global__ void __launch_bounds__(256) moe_group_kernel(const GroupParams p) {
+    __shared__ uint32_t sh[3][8];
+    __shared__ uint32_t base[4];
+    __shared__ uint32_t hist[kGroupMaxExperts];
     pdl_launch_dependents();
+    for (int i = threadIdx.x; i < p.E; i += 256) hist[i] = 0;
+    __syncthreads();
     pdl_wait();
+    for (int i = threadIdx.x; i < p.P; i += 256) {
+        const uint32_t x = p.inds[i];
+        if (x < (uint32_t)p.E) atomicAdd(&hist[x], 1u);
+    }
     if (p.fx.digits != nullptr)
         for (int t = blockIdx.x; t < p.T; t += gridDim.x) {
             if (p.fx_wide) fixed_point_row<true>(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
             else fixed_point_row<false>(p.x, p.x_dtype, (size_t)t * p.ldx, p.D, p.fx, t, threadIdx.x, 256);
         }
-    uint32_t c = 0;
-    for (int i = threadIdx.x; i < p.P; i += 256) c += p.inds[i] == e;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = c;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t s = 0;
-        for (int i = 0; i < 8; i++) s += wsum[i];
-        p.counts[e] = s;
-    }
-}
-
-__global__ void __launch_bounds__(256) moe_scatter_kernel(const GroupParams p) {
-    __shared__ uint32_t sh[3][8];
-    __shared__ uint32_t base[4];
-    pdl_launch_dependents();
-    pdl_wait();
     const uint32_t e = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // exclusive prefixes over the experts before this one: pairs, tiles of height a, tiles of height b
     uint32_t c0 = 0, ta = 0, tb = 0;
     for (int i = tid; i < (int)e; i += 256) {
-        const uint32_t c = p.counts[i];
+        const uint32_t c = hist[i];
         c0 += c;
         if (i >= p.e_lo && i < p.e_hi) {
             ta += (c + p.bm_a - 1) / p.bm_a;
@@ -631,8 +623,9 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const GroupParams p) {
     }
     __syncthreads();
     const uint32_t off = base[0], tile_a0 = base[1], tile_b0 = base[2];
-    const uint32_t cnt = p.counts[e];
+    const uint32_t cnt = hist[e];
     if (tid == 0) {
+        p.counts[e] = cnt;
         p.offsets[e] = off;
         if ((int)e == p.E - 1) {
             p.offsets[p.E] = off + cnt;
