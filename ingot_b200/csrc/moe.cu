@@ -355,9 +355,13 @@ bool use_route_small(const iq_moe* l, int tokens) {
     return tokens <= kSmallTokens && l->ext_inds == nullptr && d.expert_lo == 0 && d.expert_count == d.experts &&
            (int64_t)d.experts * d.d_model * tt <= (1 << 21) && route_small_smem(tt, d.d_model, d.experts) <= kRouteSmallSmemMax;
 }
-// The experts' kernels for few tokens: affine 4-bit weights, 16-byte aligned
-bool use_experts_small(const iq_moe* l) {
+// The experts' kernels for few tokens: affine 4-bit weights, 16-byte aligned; one token, or two and three of small experts. Beyond 24 million
+// weights (of one matrix, of every token's experts) the decode tiles take two and three, with three digits; below, the tiles leave the GPU
+// half empty. MoE block, us, here / tiles: 64 experts of 1536 x 512 at two tokens (12.6 million) 26.9 / 27.7, at three (18.9) 30.9 / 31.3, 64 of 2560 x
+// 1024 at two (21.0) 32.0 / 33.9, at three (31.5) 47.7 / 43.7, 128 of 2048 x 768 at two (25.2) 41.0 / 39.2, 128 of 2880 x 768 at two (35.4) 61.3 / 49.5
+bool use_experts_small(const iq_moe* l, int tokens) {
     const iq_moe_desc& d = l->d;
+    if (tokens > 1 && (int64_t)tokens * d.top_k * d.d_model * d.d_ff > 24000000) return false;
     uintptr_t a = 0;
     for (const iq_qlinear* m : {&d.gate, &d.up, &d.down})
         a |= reinterpret_cast<uintptr_t>(m->w) | (reinterpret_cast<uintptr_t>(m->scales) << 2) | (reinterpret_cast<uintptr_t>(m->biases) << 2);
@@ -816,9 +820,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     const float* wts = l->ext_wts ? l->ext_wts : w.wts;
     int32_t st;
 
-    const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l);
+    const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l, tokens);
     const bool int8 = use_int8_path(l, P);
-    const bool wide = !two_digit_inputs(l);
+    const bool wide = (small && !small_experts) || !two_digit_inputs(l);
     if (small) {
         st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, small_experts || int8, small_experts || wide);
         if (st == kOk && small_experts)

@@ -573,3 +573,13 @@ def test_moe_decode_tiles_pieces_and_bits(cuda_device):
     layer.encode(x.flip(0).contiguous(), back, T)
     assert torch.equal(back.flip(0), full)
     assert capi.context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("T", [1, 2, 3])
+@pytest.mark.parametrize("D,I,K", [(2048, 1472, 4), (2880, 704, 4)])
+def test_moe_two_and_three_tokens_by_size(cuda_device, D, I, K, T):
+    """One, two and three tokens on both sides of 24 million weights (two tokens 24.1 and 16.2, three 36 and 24.3), where the
+    decode tiles take over from the kernels for few tokens."""
+    rng = np.random.default_rng(D + I + T)
+    layer, host = build_layer(rng, cuda_device, 32, K, D, I, max_tokens=T)
+    check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
