@@ -102,7 +102,6 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens;
     const size_t pairs = l->fmt != kFmtAffine4 ? few * d.top_k : std::min(P, (size_t)d.expert_count * kInt8RowsPerExpert);
     const size_t fixed = std::max(few, std::min((size_t)tokens, (size_t)d.expert_count * kInt8RowsPerExpert / d.top_k));
-    w.h32 = static_cast<float*>(take(l->fmt == kFmtAffine4 ? pairs * d.d_ff * 4 : 0));
     w.fx.digits = static_cast<unsigned char*>(take(fixed * 192 * (d.d_model / 64)));  // (the wide form)
     w.fx.scale = static_cast<float2*>(take(fixed * (d.d_model / 64) * 8));
     w.fh.digits = static_cast<unsigned char*>(take(std::max(pairs * 128, few * d.top_k * 192) * (d.d_ff / 64)));
@@ -115,6 +114,8 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
         w.s_yd = take(T * d.d_model * 4);
         w.s_w = static_cast<float*>(take(T * 4));
     }
+    // (last: between the others it cost one token 0.1 of 25.5 us)
+    w.h32 = static_cast<float*>(take(l->fmt == kFmtAffine4 ? pairs * d.d_ff * 4 : 0));
     w.bytes = off;
     return w;
 }
