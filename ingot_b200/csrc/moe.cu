@@ -100,8 +100,9 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     w.yd = take(P * d.d_model * (yd_dtype_of(l) == kF16 ? 2 : 4));
     w.xs = static_cast<__half*>(take(P * d.d_model * 2));
     const size_t few = tokens < kSmallTokens ? tokens : kSmallTokens;
-    const size_t pairs = l->fmt != kFmtAffine4 ? few * d.top_k : std::min(P, (size_t)d.expert_count * kInt8RowsPerExpert);
-    const size_t fixed = std::max(few, std::min((size_t)tokens, (size_t)d.expert_count * kInt8RowsPerExpert / d.top_k));
+    // (of any format and number of owned experts: layers of one shape share a workspace)
+    const size_t pairs = std::min(P, (size_t)d.experts * kInt8RowsPerExpert);
+    const size_t fixed = std::max(few, std::min((size_t)tokens, (size_t)d.experts * kInt8RowsPerExpert / d.top_k));
     w.fx.digits = static_cast<unsigned char*>(take(fixed * 192 * (d.d_model / 64)));  // (the wide form)
     w.fx.scale = static_cast<float2*>(take(fixed * (d.d_model / 64) * 8));
     w.fh.digits = static_cast<unsigned char*>(take(std::max(pairs * 128, few * d.top_k * 192) * (d.d_ff / 64)));
@@ -115,7 +116,7 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
         w.s_w = static_cast<float*>(take(T * 4));
     }
     // (last: between the others it cost one token 0.1 of 25.5 us)
-    w.h32 = static_cast<float*>(take(l->fmt == kFmtAffine4 ? pairs * d.d_ff * 4 : 0));
+    w.h32 = static_cast<float*>(take(pairs * d.d_ff * 4));
     w.bytes = off;
     return w;
 }

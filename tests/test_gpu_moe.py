@@ -583,3 +583,21 @@ def test_moe_two_and_three_tokens_by_size(cuda_device, D, I, K, T):
     rng = np.random.default_rng(D + I + T)
     layer, host = build_layer(rng, cuda_device, 32, K, D, I, max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
+
+
+@pytest.mark.parametrize("T", [1, 5, 24, 300])
+def test_moe_layers_of_one_shape_share_a_workspace(cuda_device, T):
+    """Layers of one shape share their scratch: an affine layer, whose decode tiles need more than the rest, runs in the workspace of
+    an MXFP4 layer, and in that of one that owns a quarter of the experts, as in its own."""
+    rng = np.random.default_rng(61 + T)
+    E, K, D, I = 32, 4, 576, 1152
+    mx, _ = build_layer(rng, cuda_device, E, K, D, I, fmt="mxfp4", act="swiglu_oai", max_tokens=T)
+    part, _ = build_layer(rng, cuda_device, E, K, D, I, max_tokens=T, expert_lo=8, expert_count=8)
+    layer, _ = build_layer(rng, cuda_device, E, K, D, I, max_tokens=T)
+    x = x_tensor(synth.activations_np(rng, T, D), cuda_device)
+    own, shared = (torch.zeros(T, D, dtype=torch.float32, device=cuda_device) for _ in range(2))
+    layer.encode(x, own, T)
+    for other in (mx, part):
+        layer.share_scratch(other)
+        layer.encode(x, shared, T)
+        assert torch.equal(own, shared)
