@@ -165,6 +165,13 @@ __device__ __forceinline__ void scaled_add2(float& a0, float& a1, float v0, floa
         : "+f"(a0), "+f"(a1)
         : "f"(v0), "f"(v1), "f"(s0), "f"(s1), "f"(x0), "f"(x1));
 }
+// ... and {l0, l1} += {w0, w1} * that product, for a lower digit
+__device__ __forceinline__ void scaled_add2_low(float& a0, float& a1, float& l0, float& l1, float v0, float v1, float w0, float w1, float s, float x0, float x1) {
+    asm("{\n.reg .b64 a, l, v, w, s, x;\nmov.b64 a, {%0, %1};\nmov.b64 l, {%2, %3};\nmov.b64 v, {%4, %5};\nmov.b64 w, {%6, %7};\nmov.b64 s, {%8, %8};\n"
+        "mov.b64 x, {%9, %10};\nmul.rn.f32x2 s, s, x;\nfma.rn.f32x2 a, v, s, a;\nfma.rn.f32x2 l, w, s, l;\nmov.b64 {%0, %1}, a;\nmov.b64 {%2, %3}, l;\n}\n"
+        : "+f"(a0), "+f"(a1), "+f"(l0), "+f"(l1)
+        : "f"(v0), "f"(v1), "f"(w0), "f"(w1), "f"(s), "f"(x0), "f"(x1));
+}
 __device__ __forceinline__ void fma2(float& a0, float& a1, float b0, float b1, float y0, float y1) {
     asm("{\n.reg .b64 a, b, y;\nmov.b64 a, {%0, %1};\nmov.b64 b, {%2, %3};\nmov.b64 y, {%4, %5};\nfma.rn.f32x2 a, b, y, a;\nmov.b64 {%0, %1}, a;\n}\n"
         : "+f"(a0), "+f"(a1)

@@ -427,11 +427,14 @@ __global__ void __launch_bounds__(qt_threads(ND), 2) qmv_tile_kernel(const __gri
                             for (int j = 0; j < NP; j++) {
                                 const uint4 xv = lds128(xsb + (gs * (T / 2) + j) * 16);
                                 const float x0f = __uint_as_float(xv.x), x1f = __uint_as_float(xv.y);
-                                scaled_add2(acc[2 * j], acc[2 * j + 1], (float)(d[e][0][2 * j] * 256 + d[e][1][2 * j]), (float)(d[e][0][2 * j + 1] * 256 + d[e][1][2 * j + 1]), sc,
-                                            sc, x0f, x1f);
-                                fma2(acc[2 * j], acc[2 * j + 1], bi, bi, __uint_as_float(xv.z), __uint_as_float(xv.w));
+                                // The third digit's sum keeps the first ones' factor and is divided by 128 at the end: no products of its own (MoE block of 64
+                                // experts of 7168 x 2048 at 32 tokens 501 -> 475 us, 128 of 2880 x 768 152.7 -> 150.9)
+                                const float h0 = (float)(d[e][0][2 * j] * 256 + d[e][1][2 * j]), h1 = (float)(d[e][0][2 * j + 1] * 256 + d[e][1][2 * j + 1]);
                                 if constexpr (ND == 3)
-                                    scaled_add2(low[2 * j], low[2 * j + 1], (float)d[e][2][2 * j], (float)d[e][2][2 * j + 1], sc, sc, x0f * 0.0078125f, x1f * 0.0078125f);
+                                    scaled_add2_low(acc[2 * j], acc[2 * j + 1], low[2 * j], low[2 * j + 1], h0, h1, (float)d[e][2][2 * j], (float)d[e][2][2 * j + 1], sc, x0f, x1f);
+                                else
+                                    scaled_add2(acc[2 * j], acc[2 * j + 1], h0, h1, sc, sc, x0f, x1f);
+                                fma2(acc[2 * j], acc[2 * j + 1], bi, bi, __uint_as_float(xv.z), __uint_as_float(xv.w));
                             }
                         }
                     };
@@ -460,7 +463,7 @@ __global__ void __launch_bounds__(qt_threads(ND), 2) qmv_tile_kernel(const __gri
             if (!ok) break;
             // ---- the tile's outputs ----
 #pragma unroll
-            for (int j = 0; j < H; j++) acc[j] += ND == 3 ? low[ND == 3 ? j : 0] + bias : bias;
+            for (int j = 0; j < H; j++) acc[j] += ND == 3 ? fmaf(low[ND == 3 ? j : 0], 0.0078125f, bias) : bias;
             if (EPI) {
                 // lanes l and l + 16 hold gate and up of one feature: the lower lane finishes the even tokens, the upper one the odd ones
                 float* yp = reinterpret_cast<float*>(p.y) + (size_t)t.row0 * p.ldy + n;
