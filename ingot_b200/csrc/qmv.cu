@@ -205,20 +205,37 @@ QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms, bool wk8, b
     return best;
 }
 // Where csrc/qmv_rows.cuh takes a plain call over, one launch for any rows: by the rows that a launch here holds (max_rows: of 4-bit weights two above
-// some 8000 inputs, four above 7000, eight above 4000; of 8-bit ones four above 8000), and by whether the launches here share one conversion of the
-// activations (pre, the dense FFN's down projection). us here / there:
-// 4 bits, two rows a launch, 5 / 8 / 9 / 16 rows: 4096 x 14336 38.3 / 24.4, 53.7 / 27.1, 64.6 / 52.6, 106.3 / 63.3; 5120 x 13824 48.4 / 47.3, 67.1 / 51.3,
-//   81.6 / 56.5, 134.2 / 67.8; as the down projection of an FFN of 4096 / 14336 68.0 / 59.9, 80.0 / 64.4, 109.0 / 117.6, 155.3 / 137.1 for the whole FFN.
-//   Four: 2048 x 7680 at 9 / 13 / 16 rows 23.7 / 25.0, 32.8 / 28.4, 36.9 / 30.4 (FFN at 16 rows 44.9 / 51.1). Eight: 9216 x 5120 at 9 / 16 rows 25.7 / 22.5, 32.5 / 28.8.
-// 8 bits, four rows a launch: 4096 x 14336 at 5 / 8 / 16 rows 36.6 / 28.0, 43.1 / 30.1, 85.5 / 36.4, FFN 68.3 / 64.3, 70.0 / 67.1, 136.4 / 109.3.
-// Groups of 32, two rows a launch, 6 / 8 / 11 / 16 rows: 5120 x 13824 54.2 / 58.4, 72.0 / 62.4, 105.8 / 77.7, 144.0 / 85.5; FFN of 4096 / 14336 at 8 / 11 / 16
-//   rows 95.4 / 78.6, 141.9 / 149.9, 185.3 / 171.0.
+// some 11000 inputs, four above 7300, eight above 4100; of 8-bit ones four above 11000, eight above 5000), and by whether the launches here share one
+// conversion of the activations (pre, the dense FFN's down projection). us here / there:
+// 4 bits, two rows a launch, 5 / 8 / 9 / 16 rows: 4096 x 14336 38.3 / 21.7, 53.7 / 24.4, 64.6 / 45.7, 106.3 / 56.2; 5120 x 13824 48.4 / 43.9, 67.1 / 47.9,
+//   81.6 / 53.1, 134.2 / 64.7. Four: 4096 x 11008 28.9 / 19.1, 39.6 / 21.5, 48.0 / 24.1, 75 / 30.5; 2048 x 7680 15.0 / 13.8, 19.0 / 15.0, 24.1 / 17.3, 36.9 / 21.4.
+//   Eight: 4096 x 5504 at 5 / 8 / 9 / 16 rows 14.4 / 12.7, 17.6 / 14.1, 23.7 / 16.2, 34.5 / 19.6, 9216 x 5120 14.5 / 17.7, 16.5 / 19.9, 25.7 / 22.4, 32.5 / 28.7,
+//   2048 x 5120 at 8 / 9 / 14 11.1 / 14.9, 15.7 / 17.3, 19.1 / 19.8.
+// 8 bits, four rows a launch: 4096 x 14336 at 5 / 8 / 16 rows 36.6 / 28.0, 43.1 / 30.5, 85.5 / 36.6. Eight: 4096 x 11008 at 6 / 8 / 16 29.6 / 18.4, 34.1 / 19.4,
+//   66.5 / 31.1, 4096 x 8768 at 8 / 9 20.9 / 23.2, 32.7 / 25.8, 2048 x 5504 11.1 / 12.7, 16.0 / 14.7.
+// Groups of 32, two rows a launch, 6 / 8 / 9 / 16 rows: 5120 x 13824 54.4 / 56.6, 72.0 / 60.3, 88.2 / 70.4, 144 / 83.4. Four: 2048 x 7680 at 6 / 8 / 9 / 12 16.3 / 17.2,
+//   18.8 / 18.5, 24.2 / 22.4, 27.8 / 25.1, 4096 x 11008 at 8 / 9 / 12 40.8 / 26.8, 50.2 / 52.5, 60.4 / 58.3. Eight: 9216 x 5120 at 9 / 12 / 16 32.0 / 32.7, 37.2 / 35.0,
+//   46.3 / 36.9, 7168 x 5376 at 12 38.4 / 39.2, 2048 x 4160 at 14 18.8 / 21.2.
+// Many features are more than a wave of clusters: 12288 x 7680 at 5 / 8 rows 36.1 / 45.7, 43.5 / 50.1 (groups of 32 at 8 / 13 46.0 / 63.0, 84.1 / 99.1), 14336 x
+//   5504 at 9 / 13 42.7 / 46.2, 47.2 / 53.8. FFN with the down projection here / there: 4096 / 11008 at 9 / 16 rows 68.9 / 62.3, 87.9 / 73.5, 2048 / 7680 at 8 / 10 /
+//   13 / 16 26.4 / 28.1, 35.4 / 35.6, 41.8 / 38.4, 43.5 / 40.6.
 bool rows_kernel_pays(const GqmvCall& c, int nw, int max_rows, bool pre) {
     if (nw != 1 || c.rows < 5) return false;
-    if (c.fmt == kFmtAffine8) return max_rows <= 4 && (c.N <= 16384 || c.rows > 12);  // (30000 x 12288 at 7 / 12 / 14 rows 153.8 / 157.2, 229.9 / 234.2, 302.9 / 249.3)
-    if (c.fmt == kFmtAffine4G32) return max_rows <= 2 && c.rows > 6 && (c.rows <= 8 || c.rows > (pre ? 13 : 10));
+    if (c.fmt == kFmtAffine8) {
+        if (max_rows <= 4) return c.N <= 16384 || c.rows > 12;  // (30000 x 12288 at 7 / 12 / 14 rows 153.8 / 157.2, 229.9 / 234.2, 302.9 / 249.3)
+        return !pre && max_rows == 8 && c.N <= 4096 && (c.rows > 8 || (c.rows > 5 && c.K >= 9200));
+    }
+    if (c.fmt == kFmtAffine4G32) {
+        if (max_rows <= 2) return c.N <= 8192 && c.rows > 6 && (!pre || c.rows <= 8 || c.rows > 13);
+        if (pre || max_rows > 8) return false;
+        return max_rows <= 4 ? c.N <= 8192 && (c.rows > 11 || ((c.rows == 7 || c.rows == 8) && c.K >= 7500)) : c.N >= 4096 && c.N <= 9216 && c.rows > 12;
+    }
     if (max_rows <= 2) return !pre || c.rows <= 8 || c.rows > 12;
-    return !pre && ((max_rows == 4 && c.rows > 12) || (max_rows == 8 && c.rows > 8 && c.N >= 8192));
+    if (max_rows <= 4) {
+        if (pre) return c.N <= 4096 && (c.rows > 12 || (c.rows > 8 && c.K >= 9200));
+        return c.N <= 8192 || c.rows > 12;
+    }
+    return !pre && max_rows <= 8 && ((c.rows > 8 && c.N >= 4096 && c.N <= 9216) || (c.K >= 5500 && c.N <= 4096));
 }
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk8 = false) {

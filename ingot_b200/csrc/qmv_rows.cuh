@@ -4,10 +4,11 @@
 // has the same bits alone and among sixteen. That kernel holds the digits of all inputs in every CTA beside sixteen rings of weights: of
 // more than some 8000 inputs only two rows fit (8 bits: four), and sixteen rows are eight launches that each read the weights. Here a cluster
 // shares a tile of 128 weight rows, each CTA holding the digits of its K slices only, and one thread issues tcgen05.mma (kind::i8) for 128 weight
-// rows against all (digit, row) columns, so that sixteen rows are one launch: 4096 x 14336 (4 bits) at 8 rows 53.9 -> 27.7 us, at
-// 16 106.6 -> 63.0, 8 bits 85.6 -> 38.4; 1024 x 14336 at 16 rows 71.9 -> 20.3. Narrower inputs stay where they are: a step of 256 inputs takes
-// this machine 1000 to 2000 cycles whatever its rows (waits on barriers, loads from tensor memory and sums of one step follow one another in a warp), and
-// 14336 x 4096 at 8 rows took 29.0 us instead of 20.4.
+// rows against all (digit, row) columns, so that sixteen rows are one launch: 4096 x 14336 (4 bits) at 8 rows 53.9 -> 24.4 us, at
+// 16 106.6 -> 56.2, 4096 x 11008 at 12 58.6 -> 26.8, 8 bits 66.5 -> 31.1 at 16. How many clusters run at once is asked of the driver: thirty-three of four CTAs,
+// but fifteen of eight, since a cluster stays in one group of SMs (2048 x 7680 at 8 rows 20 us as sixteen clusters of eight, 15.0 of four). Narrower inputs
+// stay where they are: a step of 256 inputs takes this machine 1000 to 2000 cycles whatever its rows (waits on barriers, loads from tensor memory and sums
+// of one step follow one another in a warp), and 14336 x 4096 at 8 rows took 29.0 us instead of 20.4.
 //
 // Unit of work: a tile over all of K, or over the K slices of one CTA of a cluster. K is walked slice by slice as the ring kernel cuts it (every wk-th
 // column; a column is 128 bytes of a row's codes), so that every slice's sum is one accumulator's; the slices are added in their order

@@ -31,8 +31,9 @@ QwPlan qw_plan(const iq_ctx* ctx, int32_t fmt, int t, int N, int K, int wk) {
         const int js = (wk + s - 1) / s, xcols = std::min(ncol, js * ((ncol + wk - 1) / wk));
         const size_t most = 227 * 1024, fixed = kQwFixed + xcols * qw_x_bytes(ci, gpc, t, nd) + (s > 1 ? (size_t)js * t * 512 : 0);
         if (xcols >= kQwThreads || fixed + 3 * stage > most) continue;
-        // cycles: a CTA's start, its digits and its columns, some 1100 per 256 inputs (16 rows: 1500); clusters of eight do not fill every GPC
-        const int slots = ctx->sms * (s == 8 ? 7 : 8) / 8, waves = (tiles * s + slots - 1) / slots;
+        // cycles: a CTA's start, its digits and its columns, some 1100 per 256 inputs (16 rows: 1500); clusters at once: as the driver says (of
+        // eight CTAs the GPU holds fewer than 148 / 8, since a cluster stays in one group of SMs: 2048 x 5120 as 16 clusters of eight took two waves)
+        const int slots = s * ctx->rows_clusters[s == 8 ? 3 : s >> 1], waves = (tiles * s + slots - 1) / slots;
         const double col = (t == 8 ? 1100.0 : 1500.0) * ci / 256, dig = (double)xcols * ci / 256 * 18 * t;
         const double c = s == 1 ? 6000 + dig + waves * xcols * col : waves * (8000 + dig + xcols * col);
         if (best.cluster == 0 || c < cost) {
@@ -89,6 +90,26 @@ int32_t rows_init(iq_ctx* ctx) {
         const int32_t fmt = v < 2 ? kFmtAffine8 : v < 4 ? kFmtAffine4G32 : kFmtAffine4;
         cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qw_pick(fmt, v & 1 ? 16 : 8)), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_rows)");
+    }
+    // CTAs of a launch that the GPU holds at once, by the cluster's size 1, 2, 4, 8
+    for (int i = 0; i < 4; i++) {
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(ctx->sms / (1 << i) << i, 1, 1);
+        cfg.blockDim = dim3(kQwThreads, 1, 1);
+        cfg.dynamicSmemBytes = 227 * 1024;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 1 << i; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        cudaError_t e = cudaOccupancyMaxActiveClusters(&n, qw_pick(kFmtAffine4, 16), &cfg);
+        if (e != cudaSuccess) {  // (a guess does, the plans only have to be good)
+            cudaGetLastError();
+            n = ctx->sms * 7 / 8 >> i;
+        }
+        ctx->rows_clusters[i] = std::max(n, 1);
     }
     return kOk;
 }

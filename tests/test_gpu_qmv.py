@@ -327,3 +327,10 @@ def test_qmv_rows_edges(cuda_device, bits, group, N, K, rows):
     assert torch.equal(y2, y + y)
     assert torch.equal(run(m, xt, rows, y_dtype=torch.float16), y.to(torch.float16))
     assert capi.context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("bits,group", [(4, 64), (8, 64), (4, 32)])
+@pytest.mark.parametrize("N,K,rows", [(256, 7680, 5), (272, 7744, 8), (144, 5504, 9), (128, 9216, 6), (256, 11008, 12), (4112, 4672, 13)])
+def test_qmv_rows_by_width(cuda_device, bits, group, N, K, rows):
+    """The widths between the ring kernel's and the widest, on both sides of its limits of two, four and eight rows a launch: same demands."""
+    test_qmv_rows_edges(cuda_device, bits, group, N, K, rows)
