@@ -127,6 +127,8 @@ int32_t qmv_with_scratch(iq_ctx* ctx, void* stream, const void* x, int32_t x_dty
                          int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix, void* scratch);
 // Tiles of up to eight rows of affine 4-bit experts on the int8 kernel; 1: the shape does not fit it
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
+// The K slices that it cuts K inputs of nw matrices into, a multiple of four groups each, whose sums it adds in their order; 0: not for it
+int qmv_grouped_slices(int K, int nw);
 
 // Scratch of the GEMM's K split (csrc/qmm_ta.cuh). bytes: what the split of a dense GEMM takes (0: it is not split); part: null where
 // the scratch does not hold that.
@@ -175,10 +177,12 @@ struct QmmCall {
 };
 int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c);
 // A list of tiles of up to eight rows (c.bn) of affine 4-bit experts on csrc/qmv_tile.cuh, x as block fixed point (wide: three digits, gate/up only):
-// row row_map[position] / topk, or the position itself. Gate/up stores h as fp32. 1: not for this kernel.
-int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t max_tiles);
-// Rows as block fixed point, and as halves (copy, or null)
-int32_t launch_fixed_rows(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, int rows, int D, const FixedRows& fx, bool wide, __half* copy);
+// row row_map[position] / topk, or the position itself; slice: steps of 256 inputs with an accumulator of their own (two digits). Stores halves. 1: not for
+// this kernel.
+int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t slice,
+                        int32_t max_tiles);
+// Rows as block fixed point
+int32_t launch_fixed_rows(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, int rows, int D, const FixedRows& fx, bool wide);
 int32_t launch_tern_qmv(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
                         int32_t y_dtype, int64_t ldy, int32_t rows, int32_t n, int32_t accumulate);
 int32_t w8a8_init(iq_ctx* ctx);

@@ -36,7 +36,6 @@ struct MoeWs {
     Tile* tiles_a;
     Tile* tiles_b;
     __half* h;
-    float* h32;  // h before it is rounded (decode tiles)
     void* yd;
     __half* xs;  // activations in expert order, fp16 [P, d_model] (tensor-core path)
     FixedRows fx, fh;  // the activations as block fixed point and h likewise, as far as the int8 kernels go
@@ -115,8 +114,6 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
         w.s_yd = take(T * d.d_model * 4);
         w.s_w = static_cast<float*>(take(T * 4));
     }
-    // (last: between the others it cost one token 0.1 of 25.5 us)
-    w.h32 = static_cast<float*>(take(pairs * d.d_ff * 4));
     w.bytes = off;
     return w;
 }
@@ -298,7 +295,8 @@ int32_t run_down_tc(iq_moe* l, cudaStream_t cs, const __half* h, int64_t n_rows,
     return launch_qmm(l->ctx, cs, c);
 }
 
-// The same on tiles of up to eight rows, from block fixed point (csrc/qmv_tile.cuh): h as fp32, yd
+// The same on tiles of up to eight rows, from block fixed point (csrc/qmv_tile.cuh). Of two digits, the sums go over the grouped kernel's K slices: a
+// layer has the bits that iq_moe_experts gives for the same rows
 int32_t run_gateup_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, int max_tiles) {
     const iq_moe_desc& d = l->d;
     QmmCall c;
@@ -309,11 +307,15 @@ int32_t run_gateup_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, i
     c.experts = d.expert_count; c.expert_lo = d.expert_lo;
     c.N = d.d_ff; c.K = d.d_model;
     c.tiles = w.tiles_a; c.ntiles = w.ntiles;
-    c.y = w.h32; c.y_dtype = kF32; c.ldy = d.d_ff;
+    c.y = w.h; c.y_dtype = kF16; c.ldy = d.d_ff;
     c.ebias[0] = d.gate_bias; c.ebias[1] = d.up_bias;
     c.limit = d.act == IQ_ACT_SWIGLU_OAI ? d.act_limit : 0.f;
     c.act = d.act;
-    return launch_qmv_tile(l->ctx, cs, c, w.fx, wide, w.row_map, d.top_k, max_tiles);
+    return launch_qmv_tile(l->ctx, cs, c, w.fx, wide, w.row_map, d.top_k, 1, max_tiles);
+}
+int down_slice(int d_ff) {  // steps of 256 inputs; widths that the grouped kernel does not take: all of them
+    const int slices = qmv_grouped_slices(d_ff, 1);
+    return slices ? d_ff / 256 / slices : (d_ff + 255) / 256;
 }
 int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles, bool early) {
     const iq_moe_desc& d = l->d;
@@ -326,7 +328,7 @@ int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles,
     c.y = w.yd; c.y_dtype = yd_dtype_of(l); c.ldy = d.d_model;
     c.ebias[0] = d.down_bias;
     c.early = early;
-    return launch_qmv_tile(l->ctx, cs, c, w.fh, false, nullptr, 1, max_tiles);
+    return launch_qmv_tile(l->ctx, cs, c, w.fh, false, nullptr, 1, down_slice(d.d_ff), max_tiles);
 }
 
 // ---- few tokens (csrc/moe_small.cuh) ----
@@ -930,11 +932,10 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     // which kernel made h: a down projection on the same one may start on the tile list and its weights before h is there
     bool after_int8 = false, after_gemm = false;
     if (pieces & IQ_PIECE_GATEUP) {
-        st = int8 && !fixed ? launch_fixed_rows(ctx, cs, x, x_dtype, ldx, tokens, d.d_model, w.fx, wide, nullptr) : kOk;
+        st = int8 && !fixed ? launch_fixed_rows(ctx, cs, x, x_dtype, ldx, tokens, d.d_model, w.fx, wide) : kOk;
         if (st == kOk) st = int8 ? run_gateup_tile(l, cs, w, wide, max_tiles) : 1;
         after_int8 = st == kOk;
-        // h as halves (the view) and as fixed point for the down projection, from the sums' 32 bits
-        if (after_int8) st = launch_fixed_rows(ctx, cs, w.h32, kF32, d.d_ff, P, d.d_ff, w.fh, false, w.h);
+        if (after_int8) st = launch_fixed_rows(ctx, cs, w.h, kF16, d.d_ff, P, d.d_ff, w.fh, false);
         if (st == 1) {
             after_gemm = true;
             st = check_cuda(ctx, launch_dependent(moe_pack_tokens_kernel, dim3(tokens), 256, 0, cs, x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k),

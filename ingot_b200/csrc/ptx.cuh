@@ -165,6 +165,12 @@ __device__ __forceinline__ void scaled_add2(float& a0, float& a1, float v0, floa
         : "+f"(a0), "+f"(a1)
         : "f"(v0), "f"(v1), "f"(s0), "f"(s1), "f"(x0), "f"(x1));
 }
+// {a0, a1} = {v0, v1} * (s * {x0, x1}), rounded as scaled_add2 on zeros
+__device__ __forceinline__ void scaled_mul2(float& a0, float& a1, float v0, float v1, float s, float x0, float x1) {
+    asm("{\n.reg .b64 a, v, s, x;\nmov.b64 v, {%2, %3};\nmov.b64 s, {%4, %4};\nmov.b64 x, {%5, %6};\nmul.rn.f32x2 s, s, x;\nmul.rn.f32x2 a, v, s;\nmov.b64 {%0, %1}, a;\n}\n"
+        : "=f"(a0), "=f"(a1)
+        : "f"(v0), "f"(v1), "f"(s), "f"(x0), "f"(x1));
+}
 // ... and {l0, l1} += {w0, w1} * that product, for a lower digit
 __device__ __forceinline__ void scaled_add2_low(float& a0, float& a1, float& l0, float& l1, float v0, float v1, float w0, float w1, float s, float x0, float x1) {
     asm("{\n.reg .b64 a, l, v, w, s, x;\nmov.b64 a, {%0, %1};\nmov.b64 l, {%2, %3};\nmov.b64 v, {%4, %5};\nmov.b64 w, {%6, %7};\nmov.b64 s, {%8, %8};\n"

@@ -449,6 +449,47 @@ QgKernel qg_pick(int mode, bool tm, bool gw4) {
 }
 }  // namespace
 
+namespace {
+// How a call is cut. K slices per block of rows: one slice of four groups per warp when K allows it (the activation
+// fragments then live in registers: 69 against 83 us on the 64-token layer); else four slices (32-row blocks: half as
+// many hand-overs per byte) when two stages of that size fit, else eight.
+struct QgCut {
+    int wk, nstages;  // (fewer than two stages: the shape does not fit)
+    int row_pitch, srow_bytes, xq_bytes, xsc_bytes, red_bytes, fixed, mat_bytes;
+};
+QgCut qg_cut(int K, int nw, bool tm) {
+    constexpr int ms = 2;  // sets of four activation rows per tile
+    const int G = K / 64, row_bytes = K / 2;
+    QgCut c = {};
+    c.row_pitch = tm ? row_bytes : row_bytes + 32;
+    c.srow_bytes = G * 2;
+    c.xq_bytes = G * ms * 512;
+    c.xsc_bytes = G * ms * 32;
+    c.red_bytes = 2 * kQgWarps * nw * ms * 64 * 4;
+    c.fixed = c.xq_bytes + c.xsc_bytes + c.red_bytes + 256 + (tm ? 1024 : 0);
+    const bool gw4 = G == 4 * kQgWarps;
+    const int cand[4] = {gw4 ? kQgWarps : kQgWarps / 2, kQgWarps, kQgWarps / 4, kQgWarps / 8};
+    for (int ci = 0; ci < 4 && c.nstages < 2; ci++) {
+        const int wk = cand[ci];
+        if (G % wk != 0 || (G / wk) % 4 != 0) continue;  // a warp's K slice: runs of four groups
+        const int R = 16 * (kQgWarps / wk);
+        if ((R * c.srow_bytes) % 16 != 0) continue;
+        c.wk = wk;
+        c.mat_bytes = round_up(R * c.row_pitch + 2 * R * c.srow_bytes, tm ? 1024 : 16);
+        c.nstages = (kQsSmemMax - c.fixed) / (nw * c.mat_bytes);
+    }
+    return c;
+}
+// (tensor copies; without them no multiple of four groups is left)
+bool qg_tensor_copies(int K) { return K % 256 == 0 && K <= 65536; }
+}  // namespace
+
+int qmv_grouped_slices(int K, int nw) {
+    if (K % 64 != 0 || !qg_tensor_copies(K)) return 0;
+    const QgCut c = qg_cut(K, nw, true);
+    return c.nstages >= 2 ? c.wk : 0;
+}
+
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     if ((c.mode != kModeGateUp && c.mode != kModeDown) || c.tiles == nullptr || c.fmt != kFmtAffine4) return 1;
@@ -467,35 +508,17 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     // bulk copy per row measured 61.9 against 49.6 us on the fp16 tile kernels at 64 tokens; with tensor copies, 128-row
     // blocks and no K split (12 groups of 64 inputs do not divide into runs of four over more than one slice) it
     // measures 37.3 us (16 tokens: 23.9 against 30.6; 256 tokens: 79.8 against 121).
-    const bool tm = ctx->encode_tiled != nullptr && c.expert_count > 0 && p.row_bytes % 128 == 0 && p.row_bytes / 128 <= 256 &&
+    const bool tm = ctx->encode_tiled != nullptr && c.expert_count > 0 && qg_tensor_copies(c.K) &&
                     c.w_estride * 4 == (int64_t)c.N * p.row_bytes;
     if (c.K < 2048 && !tm) return 1;
-    constexpr int ms = 2;  // sets of four activation rows per tile
-    p.row_pitch = tm ? p.row_bytes : p.row_bytes + 32;
-    p.srow_bytes = G * 2;
-    p.xq_bytes = G * ms * 512;
-    p.xsc_bytes = G * ms * 32;
-    p.red_bytes = 2 * kQgWarps * nw * ms * 64 * 4;
-    const int fixed = p.xq_bytes + p.xsc_bytes + p.red_bytes + 256 + (tm ? 1024 : 0);
-    // K slices per block of rows: one slice of four groups per warp when K allows it (the activation
-    // fragments then live in registers: 69 against 83 us on the 64-token layer); else four slices (32-row blocks: half as
-    // many hand-overs per byte) when two stages of that size fit, else eight.
-    int ctas = 1, nstages = 0;
-    const bool gw4 = G == 4 * kQgWarps;
-    const int cand[4] = {gw4 ? kQgWarps : kQgWarps / 2, kQgWarps, kQgWarps / 4, kQgWarps / 8};
-    for (int ci = 0; ci < 4 && nstages < 2; ci++) {
-        const int wk = cand[ci];
-        if (G % wk != 0 || (G / wk) % 4 != 0) continue;  // a warp's K slice: runs of four groups
-        const int R = 16 * (kQgWarps / wk);
-        if ((R * p.srow_bytes) % 16 != 0) continue;
-        p.wk = wk; p.rgs = kQgWarps / wk;
-        p.NB = (c.N + R - 1) / R;
-        p.mat_bytes = round_up(R * p.row_pitch + 2 * R * p.srow_bytes, tm ? 1024 : 16);
-        p.stage_bytes = nw * p.mat_bytes;
-        nstages = (kQsSmemMax - fixed) / p.stage_bytes;
-    }
-    if (nstages < 2) return 1;
-    if (nstages > 8) nstages = 8;
+    const QgCut cut = qg_cut(c.K, nw, tm);
+    if (cut.nstages < 2) return 1;
+    const int nstages = cut.nstages < 8 ? cut.nstages : 8, R = 16 * (kQgWarps / cut.wk), fixed = cut.fixed;
+    p.row_pitch = cut.row_pitch; p.srow_bytes = cut.srow_bytes;
+    p.xq_bytes = cut.xq_bytes; p.xsc_bytes = cut.xsc_bytes; p.red_bytes = cut.red_bytes;
+    p.wk = cut.wk; p.rgs = kQgWarps / cut.wk;
+    p.NB = (c.N + R - 1) / R;
+    p.mat_bytes = cut.mat_bytes; p.stage_bytes = nw * cut.mat_bytes;
     p.nstages = nstages;
     for (int i = 0; i < 2; i++) {
         p.w[i] = reinterpret_cast<const unsigned char*>(c.w[i] ? c.w[i] : c.w[0]);
@@ -525,10 +548,9 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     p.act = c.act;
     p.status = ctx->d_status;
     const int64_t items = (int64_t)p.NB * c.grid_tiles;
-    const int64_t slots = (int64_t)ctx->sms * ctas;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(items < slots ? items : slots), 1, 1);
+    cfg.gridDim = dim3((unsigned)(items < ctx->sms ? items : ctx->sms), 1, 1);
     cfg.blockDim = dim3(kQgThreads, 1, 1);
     cfg.dynamicSmemBytes = fixed + nstages * p.stage_bytes;
     cfg.stream = st;
@@ -537,7 +559,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, gw4 && p.wk == kQgWarps), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, G == 4 * kQgWarps && p.wk == kQgWarps), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
 }
 
 int32_t gqmv_init(iq_ctx* ctx) {

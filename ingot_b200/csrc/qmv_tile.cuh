@@ -11,6 +11,10 @@
 // lane's own, and what is left are two streams of independent instructions: codes to bytes (16-byte shared-memory loads, masks,
 // tcgen05.st: 24 instructions per 32 rows and group) and sums to floats (tcgen05.ld, four instructions per pair of tokens).
 //
+// With two digits K is walked in the slices that the grouped kernel cuts it into, each with an accumulator of its own, and h is rounded to halves before the
+// down projection's digits are made, as there: a layer has the same bits whole and in expert-parallel pieces (sums in one accumulator and h's digits from
+// 32 bits had been 3.2e-4 away from them).
+//
 // A step is 256 inputs: four groups, 128 bytes of codes per row. Warp roles of one of two persistent CTAs per SM:
 //   warp 0      the tile's activation rows (digits, scales), gathered by asynchronous copies into the MMA's swizzled layout
 //   warp 1      allocates tensor memory, issues tcgen05.mma
@@ -57,10 +61,10 @@ struct QtParams {
     FixedRows x;
     const uint32_t* row_map;   // sorted position -> pair id (row of x = pair / topk); null: rows are in place
     int32_t topk;
+    int32_t slice;             // steps of 256 inputs whose sums are one accumulator's (two digits; gate/up: 1)
     const Tile* tiles;
     const uint32_t* ntiles;
-    void* y;
-    int32_t y_dtype;
+    __half* y;
     int64_t ldy;
     const float* ebias[2];
     float limit;
@@ -379,9 +383,10 @@ __global__ void __launch_bounds__(qt_threads(ND), 2) qmv_tile_kernel(const __gri
         bool ok = true;
         Item t;
         for (int i = first; ok && item(i, t); i += stride) {
-            float acc[H], low[ND == 3 ? H : 1];
+            float acc[H], low[ND == 3 ? H : 1], tot[ND == 2 ? H : 1];
 #pragma unroll
-            for (int j = 0; j < H; j++) acc[j] = low[ND == 3 ? j : 0] = 0.f;
+            for (int j = 0; j < H; j++) acc[j] = low[ND == 3 ? j : 0] = tot[ND == 2 ? j : 0] = 0.f;
+            int left = p.slice;
             const int n = t.n0 + nl, live = SG == 2 ? (t.rows - 2 * half + 3) >> 2 : (t.rows + 1) >> 1;  // pairs with a token
             const bool n_ok = n < p.N;
             const float* eb = mi ? p.ebias[1] : p.ebias[0];
@@ -397,44 +402,50 @@ __global__ void __launch_bounds__(qt_threads(ND), 2) qmv_tile_kernel(const __gri
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t td = my_d + ds * kDCols;
-                    // NP: the pairs of tokens that the tile has. FULL: a step of four groups (a branch at every second one only: across more of them the
-                    // registers do not suffice). The next group's sums are under way while one's are used; tensor memory is handed back
-                    // with the last ones in registers.
+                    // NP: the pairs of tokens that the tile has. FULL: a step of four groups. The next group's sums are under way while one's are used; tensor
+                    // memory is handed back with the last ones in registers. Two pairs at a time over the unit's groups: with all four at once the sums under
+                    // way, the slices' and the tile's take more than the 80 registers (MoE block of 128 experts 2048 x 768, 64 tokens: 105.2 us, 97.9 so).
                     auto body = [&](auto np_c, auto full_c) {
                         constexpr int NP = decltype(np_c)::value;
                         constexpr bool FULL = decltype(full_c)::value;
-                        int d[2][ND][H];
-                        auto fetch = [&](int g) {
+                        constexpr int PP = ND == 2 ? 2 : H / 2, NQ = (NP + PP - 1) / PP * UG;  // pairs per pass, loads
+                        int d[2][ND][2 * PP];
+                        auto fetch = [&](int q) {
 #pragma unroll
-                            for (int i = 0; i < ND; i++) qt_ld(td + g * NB + i * T, d[g & 1][i]);
+                            for (int i = 0; i < ND; i++) qt_ld(td + q % UG * NB + i * T + q / UG * 2 * PP, d[q & 1][i]);
                         };
                         fetch(0);
 #pragma unroll
-                        for (int g = 0; g < UG; g++) {
-                            const int e = g & 1, gs = u * UG + g;
+                        for (int q = 0; q < NQ; q++) {
+                            const int e = q & 1, g = q % UG, j0 = q / UG * PP, gs = u * UG + g;
                             qt_ld_wait(d[e][0], d[e][1]);
                             if (ND == 3) qt_ld_wait(d[e][0], d[e][ND - 1]);
-                            if (g + 1 < UG) fetch(g + 1);
-                            if (g + 1 == UG) {
+                            if (q + 1 < NQ) fetch(q + 1);
+                            if (q + 1 == NQ) {
                                 tc_fence_before();
                                 __syncwarp();
                                 if (lane == 0) mbar_arrive(bar_dempty + 8 * ds);
                             }
-                            if (FULL ? (g & 1) == 0 && t.row0 < 0 : gs >= ng) continue;  // (FULL: never)
+                            if (!FULL && gs >= ng) continue;
                             const uint32_t sw = gs < 2 ? scw.x : scw.y, bw = gs < 2 ? biw.x : biw.y;
                             const float sc = __uint_as_float(gs & 1 ? sw & 0xFFFF0000u : sw << 16), bi = __uint_as_float(gs & 1 ? bw & 0xFFFF0000u : bw << 16);
 #pragma unroll
-                            for (int j = 0; j < NP; j++) {
+                            for (int j = j0; j < NP && j < j0 + PP; j++) {
+                                const int c = 2 * (j - j0);
                                 const uint4 xv = lds128(xsb + (gs * (T / 2) + j) * 16);
                                 const float x0f = __uint_as_float(xv.x), x1f = __uint_as_float(xv.y);
                                 // The third digit's sum keeps the first ones' factor and is divided by 128 at the end: no products of its own (MoE block of 64
                                 // experts of 7168 x 2048 at 32 tokens 501 -> 475 us, 128 of 2880 x 768 152.7 -> 150.9)
-                                const float h0 = (float)(d[e][0][2 * j] * 256 + d[e][1][2 * j]), h1 = (float)(d[e][0][2 * j + 1] * 256 + d[e][1][2 * j + 1]);
+                                const float h0 = (float)(d[e][0][c] * 256 + d[e][1][c]), h1 = (float)(d[e][0][c + 1] * 256 + d[e][1][c + 1]);
                                 if constexpr (ND == 3)
-                                    scaled_add2_low(acc[2 * j], acc[2 * j + 1], low[2 * j], low[2 * j + 1], h0, h1, (float)d[e][2][2 * j], (float)d[e][2][2 * j + 1], sc, x0f, x1f);
+                                    scaled_add2_low(acc[2 * j], acc[2 * j + 1], low[2 * j], low[2 * j + 1], h0, h1, (float)d[e][2][c], (float)d[e][2][c + 1], sc, x0f, x1f);
+                                else if (EPI && g == 0)  // (the first one of a slice: no zeros)
+                                    scaled_mul2(acc[2 * j], acc[2 * j + 1], h0, h1, sc, x0f, x1f);
                                 else
                                     scaled_add2(acc[2 * j], acc[2 * j + 1], h0, h1, sc, sc, x0f, x1f);
                                 fma2(acc[2 * j], acc[2 * j + 1], bi, bi, __uint_as_float(xv.z), __uint_as_float(xv.w));
+                                if (EPI && ND == 2 && g == UG - 1)  // the slice (a step) is complete
+                                    fma2(tot[ND == 2 ? 2 * j : 0], tot[ND == 2 ? 2 * j + 1 : 0], acc[2 * j], acc[2 * j + 1], 1.f, 1.f);
                             }
                         }
                     };
@@ -459,30 +470,36 @@ __global__ void __launch_bounds__(qt_threads(ND), 2) qmv_tile_kernel(const __gri
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_empty + 8 * s);
                 if (++s == NST) { s = 0; ph ^= 1; }
+                if (ND == 2 && !EPI && --left == 0) {  // the slice is complete
+#pragma unroll
+                    for (int j = 0; j < H; j++) {
+                        tot[ND == 2 ? j : 0] += acc[j];
+                        acc[j] = 0.f;
+                    }
+                    left = p.slice;
+                }
             }
             if (!ok) break;
             // ---- the tile's outputs ----
 #pragma unroll
-            for (int j = 0; j < H; j++) acc[j] += ND == 3 ? fmaf(low[ND == 3 ? j : 0], 0.0078125f, bias) : bias;
+            for (int j = 0; j < H; j++) acc[j] = ND == 3 ? acc[j] + fmaf(low[ND == 3 ? j : 0], 0.0078125f, bias) : tot[ND == 2 ? j : 0] + bias;
             if (EPI) {
                 // lanes l and l + 16 hold gate and up of one feature: the lower lane finishes the even tokens, the upper one the odd ones
-                float* yp = reinterpret_cast<float*>(p.y) + (size_t)t.row0 * p.ldy + n;
+                __half* yp = p.y + (size_t)t.row0 * p.ldy + n;
 #pragma unroll
                 for (int j = 0; j < H / 2; j++) {
                     if (j >= live) break;
                     const float other = __shfl_xor_sync(0xffffffffu, mi ? acc[2 * j] : acc[2 * j + 1], 16);
                     const float g = mi ? other : acc[2 * j], up = mi ? acc[2 * j + 1] : other;
                     const int m = token(2 * j) + mi;
-                    if (n_ok && m < t.rows) yp[(size_t)m * p.ldy] = glu_rt(p.act, g, up, p.limit);
+                    if (n_ok && m < t.rows) yp[(size_t)m * p.ldy] = __float2half_rn(glu_rt(p.act, g, up, p.limit));
                 }
             } else if (n_ok) {
-                const size_t o = (size_t)t.row0 * p.ldy + n;
+                __half* yp = p.y + (size_t)t.row0 * p.ldy + n;
 #pragma unroll
                 for (int j = 0; j < H; j++) {
                     if (token(j) >= t.rows) break;
-                    if (p.y_dtype == kF32) reinterpret_cast<float*>(p.y)[o + (size_t)token(j) * p.ldy] = acc[j];
-                    else if (p.y_dtype == kF16) reinterpret_cast<__half*>(p.y)[o + (size_t)token(j) * p.ldy] = __float2half_rn(acc[j]);
-                    else reinterpret_cast<uint16_t*>(p.y)[o + (size_t)token(j) * p.ldy] = (uint16_t)f32_to_bf16_bits(acc[j]);
+                    yp[(size_t)token(j) * p.ldy] = __float2half_rn(acc[j]);
                 }
             }
         }
@@ -503,9 +520,9 @@ __global__ void __launch_bounds__(qt_threads(ND), 2) qmv_tile_kernel(const __gri
     }
 }
 
-// Rows as block fixed point, where no other kernel leaves them so, and as halves (copy, or null): grid-stride over the rows
+// Rows as block fixed point, where no other kernel leaves them so: grid-stride over the rows
 template <bool WIDE>
-__global__ void __launch_bounds__(256) fixed_rows_kernel(const void* x, int32_t x_dtype, int64_t ldx, int rows, int D, const FixedRows fx, __half* copy) {
+__global__ void __launch_bounds__(256) fixed_rows_kernel(const void* x, int32_t x_dtype, int64_t ldx, int rows, int D, const FixedRows fx) {
     pdl_wait();
     pdl_launch_dependents();
     const int units = D / 8, upad = (units + 31) / 32 * 32;
@@ -515,8 +532,6 @@ __global__ void __launch_bounds__(256) fixed_rows_kernel(const void* x, int32_t 
             const size_t o = (size_t)r * ldx + (live ? u : 0) * 8, g = (size_t)r * (D / 64) + (live ? u : 0) / 8;
             float v[8];
             load_x8(x, x_dtype, o, v);
-            if (copy != nullptr && live)
-                *reinterpret_cast<uint4*>(copy + (size_t)r * D + u * 8) = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
             fixed_point_unit<WIDE>(v, u & 7, live ? fx.digits + g * (WIDE ? 192 : 128) : nullptr, fx.scale + g);
         }
 }

@@ -8,13 +8,13 @@
 
 namespace iq {
 
-int32_t launch_fixed_rows(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, int rows, int D, const FixedRows& fx, bool wide, __half* copy) {
+int32_t launch_fixed_rows(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x_dtype, int64_t ldx, int rows, int D, const FixedRows& fx, bool wide) {
     return check_cuda(ctx, launch_dependent(wide ? fixed_rows_kernel<true> : fixed_rows_kernel<false>, dim3(std::min(rows, 8 * ctx->sms)), 256, 0, st, x, x_dtype, ldx,
-                                            rows, D, fx, copy), "fixed_rows launch");
+                                            rows, D, fx), "fixed_rows launch");
 }
 
-int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t max_tiles) {
-    if (c.fmt != kFmtAffine4 || c.tiles == nullptr || c.K % 64 != 0 || c.bn != kQtRows || c.accumulate || (c.epi && c.y_dtype != kF32) || (!c.epi && wide) ||
+int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t slice, int32_t max_tiles) {
+    if (c.fmt != kFmtAffine4 || c.tiles == nullptr || c.K % 64 != 0 || c.bn != kQtRows || c.accumulate || c.y_dtype != kF16 || (c.epi ? !wide && c.K % 256 != 0 : wide) ||
         ctx->encode_tiled == nullptr)
         return 1;
     QtParams p;
@@ -32,9 +32,9 @@ int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const Fi
     p.vec = c.K % 256 == 0 && (align & 7) == 0;
     p.expert_lo = c.expert_lo;
     p.N = c.N; p.K = c.K;
-    p.x = x; p.row_map = row_map; p.topk = topk;
+    p.x = x; p.row_map = row_map; p.topk = topk; p.slice = slice;
     p.tiles = c.tiles; p.ntiles = c.ntiles;
-    p.y = c.y; p.y_dtype = c.y_dtype; p.ldy = c.ldy;
+    p.y = static_cast<__half*>(c.y); p.ldy = c.ldy;
     p.limit = c.limit; p.act = c.act;
     p.early = c.early ? 1 : 0;
     p.status = ctx->d_status;

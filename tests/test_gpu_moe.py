@@ -601,3 +601,32 @@ def test_moe_layers_of_one_shape_share_a_workspace(cuda_device, T):
         layer.share_scratch(other)
         layer.encode(x, shared, T)
         assert torch.equal(own, shared)
+
+
+def block_in_pieces(layer, x, T):
+    """The block of one token batch as the expert-parallel pieces run it: rows out, the experts on them, rows back."""
+    dev, P = layer.device, T * layer.router.top_k
+    out = torch.zeros(T, layer.D, dtype=torch.float32, device=dev)
+    layer.encode(x, out, T, only=("router", "route", "group"))
+    off = layer.views(T)["offsets"]
+    counts = (off[1:] - off[:-1]).to(torch.int32).contiguous()
+    rows, yd = (torch.zeros(P, layer.D, dtype=torch.float16, device=dev) for _ in range(2))
+    layer.pack_rows(x, rows, T)
+    layer.experts(rows, P, counts, 1, yd, torch.empty(layer.experts_workspace_bytes(P, 1), dtype=torch.uint8, device=dev))
+    layer.combine_rows(yd, out, T)
+    return out
+
+
+@pytest.mark.parametrize("T", [4, 13, 44])
+@pytest.mark.parametrize("D,I", [(256, 4096), (512, 512), (512, 6144), (1024, 2048), (1024, 1280), (2048, 768), (2048, 1536), (2048, 256)])
+def test_moe_whole_layer_has_the_bits_of_its_pieces(cuda_device, D, I, T):
+    """Where the decode tiles and the expert-parallel pieces' kernel take the same rows as two digits (activations in half, h rounded to halves),
+    they give the same bits: one, two, four and eight K slices of h, tiles of one to eight rows and second tiles, expert biases."""
+    rng = np.random.default_rng(D + I + T)
+    layer, host = build_layer(rng, cuda_device, 32, 4, D, I, biases=True, max_tokens=T)
+    x = synth.activations_np(rng, T, D)
+    whole = check_layer(layer, host, x, T, "silu")
+    xt = x_tensor(x, cuda_device, torch.float16)
+    layer.encode(xt, whole, T)
+    assert torch.equal(block_in_pieces(layer, xt, T), whole)
+    assert capi.context(0).device_status() == 0
