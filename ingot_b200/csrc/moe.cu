@@ -317,7 +317,7 @@ int down_slice(int d_ff) {  // steps of 256 inputs; widths that the grouped kern
     const int slices = qmv_grouped_slices(d_ff, 1);
     return slices ? d_ff / 256 / slices : (d_ff + 255) / 256;
 }
-int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles, bool early) {
+int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles) {
     const iq_moe_desc& d = l->d;
     QmmCall c;
     c.fmt = l->fmt; c.epi = 0; c.bn = kDecodeTileRows;
@@ -327,7 +327,7 @@ int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles,
     c.tiles = w.tiles_a; c.ntiles = w.ntiles;
     c.y = w.yd; c.y_dtype = yd_dtype_of(l); c.ldy = d.d_model;
     c.ebias[0] = d.down_bias;
-    c.early = early;
+    c.early = true;
     return launch_qmv_tile(l->ctx, cs, c, w.fh, false, nullptr, 1, down_slice(d.d_ff), max_tiles);
 }
 
@@ -929,13 +929,10 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st != kOk) return st;
     }
     const int max_tiles = (int)std::min<int64_t>((int64_t)d.expert_count + P / kDecodeTileRows, P);
-    // which kernel made h: a down projection on the same one may start on the tile list and its weights before h is there
-    bool after_int8 = false, after_gemm = false;
+    bool after_gemm = false;  // h by the GEMM of this call: a down projection on it may start on the tile list and its weights before h is there
     if (pieces & IQ_PIECE_GATEUP) {
         st = int8 && !fixed ? launch_fixed_rows(ctx, cs, x, x_dtype, ldx, tokens, d.d_model, w.fx, wide) : kOk;
         if (st == kOk) st = int8 ? run_gateup_tile(l, cs, w, wide, max_tiles) : 1;
-        after_int8 = st == kOk;
-        if (after_int8) st = launch_fixed_rows(ctx, cs, w.h, kF16, d.d_ff, P, d.d_ff, w.fh, false);
         if (st == 1) {
             after_gemm = true;
             st = check_cuda(ctx, launch_dependent(moe_pack_tokens_kernel, dim3(tokens), 256, 0, cs, x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k),
@@ -945,7 +942,10 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
         if (st != kOk) return st;
     }
     if (pieces & IQ_PIECE_DOWN) {
-        st = int8 && !after_gemm ? run_down_tile(l, cs, w, max_tiles, after_int8) : 1;
+        // h's digits come from the halves that lie in the workspace, whichever call or caller left them there: the kernels for few tokens leave digits of
+        // another form in fh. The tiles may start before the digits are there: the kernel that makes them lets them, after its own wait.
+        st = int8 && !after_gemm ? launch_fixed_rows(ctx, cs, w.h, kF16, d.d_ff, P, d.d_ff, w.fh, false) : 1;
+        if (st == kOk) st = run_down_tile(l, cs, w, max_tiles);
         if (st == 1) st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn, after_gemm);
         if (st != kOk) return st;
     }

@@ -630,3 +630,22 @@ def test_moe_whole_layer_has_the_bits_of_its_pieces(cuda_device, D, I, T):
     layer.encode(xt, whole, T)
     assert torch.equal(block_in_pieces(layer, xt, T), whole)
     assert capi.context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 24, 120])
+@pytest.mark.parametrize("D,I", [(512, 256), (576, 192)])
+def test_moe_down_alone_takes_the_h_of_the_workspace(cuda_device, D, I, T):
+    """After a whole call on any of the paths (three kernels, decode tiles, GEMM) down and combine alone give its result again, and of an h that the
+    caller doubled twice that: every rounding scales with h, except of expert outputs below 2^-14, where halves lie 2^-24 apart (two such roundings, the
+    weights add up to one: 2^-23)."""
+    rng = np.random.default_rng(D + T)
+    layer, host = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
+    x = synth.activations_np(rng, T, D)
+    whole = check_layer(layer, host, x, T, "silu")
+    out = torch.zeros_like(whole)
+    layer.encode(x_tensor(x, cuda_device), out, T, only=("down", "combine"))
+    assert qref.max_rel(out.cpu().numpy(), whole.cpu().numpy()) <= TOL
+    layer.views(T)["h"].mul_(2)
+    twice = torch.zeros_like(whole)
+    layer.encode(x_tensor(x, cuda_device), twice, T, only=("down", "combine"))
+    assert (twice - 2 * out).abs().max().item() <= 2.0**-23 and twice.abs().max().item() > 0.1
