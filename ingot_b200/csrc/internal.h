@@ -176,7 +176,7 @@ struct QmmCall {
     QmmSplit split;   // quantized formats: scratch of the K split, or none
 };
 int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c);
-// A list of tiles of up to eight rows (c.bn) of affine 4-bit experts on csrc/qmv_tile.cuh, x as block fixed point (wide: three digits, gate/up only):
+// A list of tiles of up to eight rows (c.bn) of affine 4-bit experts on csrc/qmv_tile.cuh, x as block fixed point (wide: three digits):
 // row row_map[position] / topk, or the position itself; slice: steps of 256 inputs with an accumulator of their own (two digits). Stores halves. 1: not for
 // this kernel.
 int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t slice,

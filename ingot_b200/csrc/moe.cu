@@ -61,7 +61,13 @@ constexpr int kFixedTokens = 512;  // up to here the grouping kernel leaves the 
 //   32 of 4096 x 2048, two digits            20 tokens 118 / 153, 48 (6 rows) 140 / 170; three digits 64 (8 rows) 213 / 165
 //   64 of 3072 x 1408, three digits          8 tokens 106 / 112, 20 148 / 151, 40 (3.8 rows) 165 / 168, 64 (6 rows) 180 / 169
 //   128 of 2880 x 768, three digits          8 tokens 92 / 95, 20 131 / 147, 64 (4 rows) 174 / 183, 80 (5 rows) 198 / 191
+// Likewise h: as two digits in the widths that mma.sync took, as three (up to four rows per expert, two below 1024 features, then by the GEMM) in the others, where it has been whole
+// halves. With one feature of every 64 256 times the rest, that do not count in the outputs, two digits are 7e-3 off the 64-bit result, three as much as
+// the GEMM. h's three digits, tiles / GEMM: 64 of 2048 x 1408 at 4 tokens 55.1 / 58.9, 30 102.7 / 103.8, 45 (4.2 rows) 108.1 / 108.4, 64 (6) 121 / 116, 32 of
+// 2880 x 2880 at 16 153 / 159, 32 (4) 171 / 182, 256 of 1024 x 704 at 8 46.3 / 47.6, 64 (2) 96.6 / 94.9, 190 (5.9) 149 / 140,
+// 64 of 4096 x 704 at 16 (1.5) 95.0 / 97.2, 40 (3.8) 130 / 127.
 constexpr int kInt8RowsPerExpert = 6, kWideRowsPerExpert = 4;
+bool two_digit_h(const iq_moe* l) { return qmv_grouped_slices(l->d.d_ff, 1) > 0; }
 bool two_digit_inputs(const iq_moe* l) { return l->d.d_model >= 256 && l->d.d_model <= 4096 && (l->d.d_model & (l->d.d_model - 1)) == 0; }
 // Router products (tokens x experts x inputs) up to which a block takes eight tokens against a few experts in float64 (about
 // 0.35 us per million): beyond, the tensor cores with exact refinement (22 us at 27 to 400 million) where they apply, else the
@@ -104,7 +110,7 @@ MoeWs carve(const iq_moe* l, void* base, int tokens) {
     const size_t fixed = std::max(few, std::min((size_t)tokens, (size_t)d.experts * kInt8RowsPerExpert / d.top_k));
     w.fx.digits = static_cast<unsigned char*>(take(fixed * 192 * (d.d_model / 64)));  // (the wide form)
     w.fx.scale = static_cast<float2*>(take(fixed * (d.d_model / 64) * 8));
-    w.fh.digits = static_cast<unsigned char*>(take(std::max(pairs * 128, few * d.top_k * 192) * (d.d_ff / 64)));
+    w.fh.digits = static_cast<unsigned char*>(take(std::max(pairs, few * d.top_k) * 192 * (d.d_ff / 64)));
     w.fh.scale = static_cast<float2*>(take(std::max(pairs, few * d.top_k) * (d.d_ff / 64) * 8));
     w.s_x16 = nullptr; w.s_h = nullptr; w.s_yd = nullptr; w.s_w = nullptr;
     if (d.shared != IQ_SHARED_NONE) {
@@ -313,12 +319,9 @@ int32_t run_gateup_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, i
     c.act = d.act;
     return launch_qmv_tile(l->ctx, cs, c, w.fx, wide, w.row_map, d.top_k, 1, max_tiles);
 }
-int down_slice(int d_ff) {  // steps of 256 inputs; widths that the grouped kernel does not take: all of them
-    const int slices = qmv_grouped_slices(d_ff, 1);
-    return slices ? d_ff / 256 / slices : (d_ff + 255) / 256;
-}
-int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles) {
+int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, int max_tiles) {
     const iq_moe_desc& d = l->d;
+    const int slices = wide ? 1 : qmv_grouped_slices(d.d_ff, 1);
     QmmCall c;
     c.fmt = l->fmt; c.epi = 0; c.bn = kDecodeTileRows;
     c.w[0] = d.down.w; c.s[0] = d.down.scales; c.b[0] = d.down.biases;
@@ -328,7 +331,7 @@ int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, int max_tiles)
     c.y = w.yd; c.y_dtype = yd_dtype_of(l); c.ldy = d.d_model;
     c.ebias[0] = d.down_bias;
     c.early = true;
-    return launch_qmv_tile(l->ctx, cs, c, w.fh, false, nullptr, 1, down_slice(d.d_ff), max_tiles);
+    return launch_qmv_tile(l->ctx, cs, c, w.fh, wide, nullptr, 1, d.d_ff / 256 / slices, max_tiles);
 }
 
 // ---- few tokens (csrc/moe_small.cuh) ----
@@ -826,7 +829,8 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
 
     const bool small = pieces == IQ_PIECE_ALL && use_route_small(l, tokens), small_experts = small && use_experts_small(l, tokens);
     const bool int8 = use_int8_path(l, P);
-    const bool wide = (small && !small_experts) || !two_digit_inputs(l);
+    const bool few_on_tiles = small && !small_experts;  // (the kernels for few tokens take three digits of both)
+    const bool wide = few_on_tiles || !two_digit_inputs(l), wide_h = few_on_tiles || !two_digit_h(l);
     if (small) {
         st = run_route_small(l, cs, x, x_dtype, ldx, tokens, w, small_experts || int8, small_experts || wide);
         if (st == kOk && small_experts)
@@ -944,8 +948,9 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     if (pieces & IQ_PIECE_DOWN) {
         // h's digits come from the halves that lie in the workspace, whichever call or caller left them there: the kernels for few tokens leave digits of
         // another form in fh. The tiles may start before the digits are there: the kernel that makes them lets them, after its own wait.
-        st = int8 && !after_gemm ? launch_fixed_rows(ctx, cs, w.h, kF16, d.d_ff, P, d.d_ff, w.fh, false) : 1;
-        if (st == kOk) st = run_down_tile(l, cs, w, max_tiles);
+        const bool on_tiles = int8 && !after_gemm && (!wide_h || P <= (int64_t)d.expert_count * (d.d_ff < 1024 ? 2 : kWideRowsPerExpert));
+        st = on_tiles ? launch_fixed_rows(ctx, cs, w.h, kF16, d.d_ff, P, d.d_ff, w.fh, wide_h) : 1;
+        if (st == kOk) st = run_down_tile(l, cs, w, wide_h, max_tiles);
         if (st == 1) st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn, after_gemm);
         if (st != kOk) return st;
     }

@@ -13,8 +13,14 @@ int32_t launch_fixed_rows(iq_ctx* ctx, cudaStream_t st, const void* x, int32_t x
                                             rows, D, fx), "fixed_rows launch");
 }
 
+typedef void (*QtKernel)(const QtMaps, const QtParams);
+static QtKernel qt_pick(int epi, bool wide) {
+    if (epi) return wide ? qmv_tile_kernel<1, 3> : qmv_tile_kernel<1, 2>;
+    return wide ? qmv_tile_kernel<0, 3> : qmv_tile_kernel<0, 2>;
+}
+
 int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t slice, int32_t max_tiles) {
-    if (c.fmt != kFmtAffine4 || c.tiles == nullptr || c.K % 64 != 0 || c.bn != kQtRows || c.accumulate || c.y_dtype != kF16 || (c.epi ? !wide && c.K % 256 != 0 : wide) ||
+    if (c.fmt != kFmtAffine4 || c.tiles == nullptr || c.K % 64 != 0 || c.bn != kQtRows || c.accumulate || c.y_dtype != kF16 || (c.epi && !wide && c.K % 256 != 0) ||
         ctx->encode_tiled == nullptr)
         return 1;
     QtParams p;
@@ -40,16 +46,14 @@ int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const Fi
     p.status = ctx->d_status;
     const int nrows = c.epi ? 64 : 128;
     const int64_t items = (int64_t)max_tiles * ((c.N + nrows - 1) / nrows);
-    return check_cuda(ctx, launch_dependent(!c.epi ? qmv_tile_kernel<0, 2> : wide ? qmv_tile_kernel<1, 3> : qmv_tile_kernel<1, 2>,
+    return check_cuda(ctx, launch_dependent(qt_pick(c.epi, wide),
                                             dim3((unsigned)std::min<int64_t>(items, 2 * ctx->sms)), qt_threads(wide ? 3 : 2), qt_smem(wide ? 3 : 2), st, maps, p),
                       "qmv_tile launch");
 }
 
 int32_t tile_init(iq_ctx* ctx) {
-    const void* k[3] = {reinterpret_cast<const void*>(qmv_tile_kernel<0, 2>), reinterpret_cast<const void*>(qmv_tile_kernel<1, 2>),
-                        reinterpret_cast<const void*>(qmv_tile_kernel<1, 3>)};
-    for (int v = 0; v < 3; v++) {
-        cudaError_t e = cudaFuncSetAttribute(k[v], cudaFuncAttributeMaxDynamicSharedMemorySize, qt_smem(v == 2 ? 3 : 2));
+    for (int v = 0; v < 4; v++) {
+        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qt_pick(v & 1, v >= 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, qt_smem(v >= 2 ? 3 : 2));
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_tile)");
     }
     return kOk;

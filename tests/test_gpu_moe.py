@@ -649,3 +649,70 @@ def test_moe_down_alone_takes_the_h_of_the_workspace(cuda_device, D, I, T):
     twice = torch.zeros_like(whole)
     layer.encode(x_tensor(x, cuda_device), twice, T, only=("down", "combine"))
     assert (twice - 2 * out).abs().max().item() <= 2.0**-23 and twice.abs().max().item() > 0.1
+
+
+def outlier_layer(rng, device, E, K, D, I, max_tokens):
+    """Experts whose h has one feature of every 64 some 256 times the rest, which the down projection multiplies by zero: what counts are the others."""
+    g, u, d = synth.affine_np(rng, I, D, 4, E), synth.affine_np(rng, I, D, 4, E), synth.affine_np(rng, D, I, 4, E)
+    for t in u[1:]:
+        t[:, 5::64, :] += 8 << 7  # scales and biases of these rows times 2^8
+    sd = synth.bf16_bits_to_f32(d[1])
+    d = (d[0], d[1], synth.to_bf16_bits(-8 * sd))
+    d[0][:, :, 0::8] = (d[0][:, :, 0::8] & np.uint32(~(0xF << 20) & 0xFFFFFFFF)) | np.uint32(8 << 20)  # input 5 of a group: code 8, weight 0
+    mk = lambda t: synth.dense_q_affine(t[0], t[1], t[2], 4, device)
+    wr = synth.router_np(rng, E, D)
+    layer = MoELayer(RouterSpec(E, K), synth.bf16_values_tensor(wr, device), mk(g), mk(u), mk(d), max_tokens=max_tokens)
+    return layer, lambda e: tuple(qref.dequant_affine(t[0][e], t[1][e], t[2][e], 4).astype(np.float64) for t in (g, u, d))
+
+
+@pytest.mark.parametrize("D,I,T", [(512, 320, 24), (576, 192, 24), (1024, 1792, 12), (2048, 1536, 3)])
+def test_moe_decode_tiles_keep_h_beside_large_features(cuda_device, D, I, T):
+    """h beside features 256 times as large is as good as its halves are: widths that the tiles take as three digits, and three tokens of experts too
+    large for the kernels of few tokens. Against 64 bits; the bound is the error of h and the expert outputs rounded to halves, which both sides
+    have, and a tenth of it."""
+    rng = np.random.default_rng(D + I + T)
+    E, K = 32, 4
+    layer, weights = outlier_layer(rng, cuda_device, E, K, D, I, T)
+    x = synth.activations_np(rng, T, D)
+    out = torch.zeros(T, D, dtype=torch.float32, device=cuda_device)
+    layer.encode(x_tensor(x, cuda_device), out, T)
+    v = layer.views(T)
+    inds, wts = v["inds"].cpu().numpy(), v["wts"].cpu().numpy().astype(np.float64)
+    exact, halves, large, rest = np.zeros((T, D)), np.zeros((T, D)), 0.0, 0.0
+    for e in np.unique(inds):
+        gate, up, down = weights(int(e))
+        for t, k in zip(*np.nonzero(inds == e)):
+            a = gate @ x[t].astype(np.float64)
+            h = a / (1 + np.exp(-a)) * (up @ x[t].astype(np.float64))
+            large, rest = large + np.abs(h[5::64]).mean(), rest + np.abs(np.delete(h, np.s_[5::64])).mean()
+            exact[t] += wts[t, k] * (down @ h)
+            halves[t] += wts[t, k] * (down @ h.astype(np.float16).astype(np.float64)).astype(np.float16).astype(np.float64)
+    assert large > 100 * rest
+    rel = lambda y: np.linalg.norm(y - exact) / np.linalg.norm(exact)
+    assert rel(out.cpu().numpy()) <= 1.1 * rel(halves), (rel(out.cpu().numpy()), rel(halves))
+
+
+@pytest.mark.parametrize("D,I", [(512, 256), (512, 320), (576, 192)])
+def test_moe_decode_tiles_non_finite_and_overflowing_rows(cuda_device, D, I):
+    """A token with a NaN or an infinity comes out NaN, one whose h passes the range of halves non-finite where an expert's h does, and the other
+    tokens keep their bits: two and three digits of inputs and of h."""
+    rng = np.random.default_rng(D + I)
+    T = 24
+    layer, _ = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
+    x = x_tensor(synth.activations_np(rng, T, D), cuda_device)
+    clean, got = (torch.zeros(T, D, dtype=torch.float32, device=cuda_device) for _ in range(2))
+    layer.encode(x, clean, T)
+    inds, wts = layer.views(T)["inds"].clone(), layer.views(T)["wts"].clone()
+    layer.set_external_routing(inds, wts)  # (the router's logits of such a token are not the point)
+    layer.encode(x, got, T)
+    assert torch.equal(got, clean)
+    bad = x.clone()
+    bad[3, 70] = float("nan")
+    bad[9, 5] = float("inf")
+    bad[17] *= 2.0**13  # h is a product of two: 2^26 times as large
+    layer.encode(bad, got, T)
+    assert torch.isnan(got[3]).all() and torch.isnan(got[9]).all()
+    assert not torch.isfinite(got[17]).any()
+    keep = [t for t in range(T) if t not in (3, 9, 17)]
+    assert torch.equal(got[keep], clean[keep])
+    layer.set_external_routing(None, None)
