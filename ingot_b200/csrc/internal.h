@@ -105,7 +105,6 @@ struct GqmvCall {
     int32_t x_dtype = 0;
     int64_t ldx = 0;
     const uint32_t* row_map = nullptr;
-    int32_t topk = 1;
     const Tile* tiles = nullptr;
     const uint32_t* ntiles = nullptr;
     int32_t grid_tiles = 1;
@@ -118,7 +117,6 @@ struct GqmvCall {
     const float* ebias[2] = {nullptr, nullptr};
     float limit = 0.f;
     int32_t act = 0;  // gate/up mode: activation (kAct*)
-    bool early = false;  // tiles: the list is complete when the launch's predecessor lets it start (a launch of the same kind did)
     void* scratch = nullptr;  // device memory of rows * K * 7 / 2 bytes that the call may use (256-byte aligned), or null
 };
 int32_t launch_gqmv(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c);
@@ -165,7 +163,7 @@ struct QmmCall {
     int32_t w_rows = 0;  // plain formats: rows of w when fewer than N, the rest counts as zeros (0: N)
     const Tile* tiles = nullptr;
     const uint32_t* ntiles = nullptr;
-    bool early = false;  // see GqmvCall
+    bool early = false;  // tiles: the list is complete when the launch's predecessor lets it start (that one does so after its own wait)
     void* y = nullptr;
     int32_t y_dtype = 0;
     int64_t ldy = 0;
@@ -177,8 +175,7 @@ struct QmmCall {
 };
 int32_t launch_qmm(iq_ctx* ctx, cudaStream_t st, const QmmCall& c);
 // A list of tiles of up to eight rows (c.bn) of affine 4-bit experts on csrc/qmv_tile.cuh, x as block fixed point (wide: three digits):
-// row row_map[position] / topk, or the position itself; slice: steps of 256 inputs with an accumulator of their own (two digits). Stores halves. 1: not for
-// this kernel.
+// row row_map[position] / topk, or the position itself; slice: steps of 256 inputs with an accumulator of their own (two digits). Stores halves.
 int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t slice,
                         int32_t max_tiles);
 // Rows as block fixed point

@@ -192,7 +192,7 @@ int32_t launch_route(iq_moe* l, cudaStream_t st, const float* logits, int ld, in
 // On the int8 kernels; 1: the shape does not fit them. Gate + up + activation of every tile: h[row, :] = half(act(x W_gate^T + b_g, x W_up^T + b_u)). Expert e's weights live
 // at local slot e - expert_lo: the offset is folded into the base pointers. row_map == nullptr: x rows are in place.
 int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, int64_t ldx, const uint32_t* row_map,
-                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, __half* h, int row_map_div) {
+                   const Tile* tiles, const uint32_t* ntiles, int max_tiles, __half* h) {
     const iq_moe_desc& d = l->d;
     const int64_t lo = d.expert_lo;
     GqmvCall c;
@@ -212,7 +212,7 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
     c.expert_lo = d.expert_lo; c.expert_count = d.expert_count;
     c.N = d.d_ff; c.K = d.d_model;
     c.x = x; c.x_dtype = x_dtype; c.ldx = ldx;
-    c.row_map = row_map; c.topk = row_map_div;  // x row = row_map[sorted position] / divisor
+    c.row_map = row_map;
     c.tiles = tiles; c.ntiles = ntiles; c.grid_tiles = max_tiles;
     c.rows = 0; c.max_rows = kDecodeTileRows;
     c.y = h; c.y_dtype = kF16; c.ldy = d.d_ff;
@@ -227,7 +227,7 @@ int32_t run_gateup(iq_moe* l, cudaStream_t cs, const void* x, int32_t x_dtype, i
 
 // Likewise the down projection of every tile: yd[row, :] = h[row, :] W_down^T + b_d.
 int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles, const uint32_t* ntiles, int max_tiles, void* yd,
-                 int32_t yd_dtype, bool early = false) {
+                 int32_t yd_dtype) {
     const iq_moe_desc& d = l->d;
     const int64_t lo = d.expert_lo;
     GqmvCall c;
@@ -246,7 +246,6 @@ int32_t run_down(iq_moe* l, cudaStream_t cs, const __half* h, const Tile* tiles,
     c.rows = 0; c.max_rows = kDecodeTileRows;
     c.y = yd; c.y_dtype = yd_dtype; c.ldy = d.d_model;
     if (d.down_bias) c.ebias[0] = d.down_bias - lo * d.d_model;
-    c.early = early;
     return launch_qmv_imma_grouped(l->ctx, cs, c);
 }
 
@@ -321,7 +320,7 @@ int32_t run_gateup_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, i
 }
 int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, int max_tiles) {
     const iq_moe_desc& d = l->d;
-    const int slices = wide ? 1 : qmv_grouped_slices(d.d_ff, 1);
+    const int slice = wide ? 1 : d.d_ff / 256 / qmv_grouped_slices(d.d_ff, 1);  // (two digits: the widths that the grouped kernel takes)
     QmmCall c;
     c.fmt = l->fmt; c.epi = 0; c.bn = kDecodeTileRows;
     c.w[0] = d.down.w; c.s[0] = d.down.scales; c.b[0] = d.down.biases;
@@ -331,7 +330,7 @@ int32_t run_down_tile(iq_moe* l, cudaStream_t cs, const MoeWs& w, bool wide, int
     c.y = w.yd; c.y_dtype = yd_dtype_of(l); c.ldy = d.d_model;
     c.ebias[0] = d.down_bias;
     c.early = true;
-    return launch_qmv_tile(l->ctx, cs, c, w.fh, wide, nullptr, 1, d.d_ff / 256 / slices, max_tiles);
+    return launch_qmv_tile(l->ctx, cs, c, w.fh, wide, nullptr, 1, slice, max_tiles);
 }
 
 // ---- few tokens (csrc/moe_small.cuh) ----
@@ -935,9 +934,10 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     const int max_tiles = (int)std::min<int64_t>((int64_t)d.expert_count + P / kDecodeTileRows, P);
     bool after_gemm = false;  // h by the GEMM of this call: a down projection on it may start on the tile list and its weights before h is there
     if (pieces & IQ_PIECE_GATEUP) {
-        st = int8 && !fixed ? launch_fixed_rows(ctx, cs, x, x_dtype, ldx, tokens, d.d_model, w.fx, wide) : kOk;
-        if (st == kOk) st = int8 ? run_gateup_tile(l, cs, w, wide, max_tiles) : 1;
-        if (st == 1) {
+        if (int8) {
+            st = fixed ? kOk : launch_fixed_rows(ctx, cs, x, x_dtype, ldx, tokens, d.d_model, w.fx, wide);
+            if (st == kOk) st = run_gateup_tile(l, cs, w, wide, max_tiles);
+        } else {
             after_gemm = true;
             st = check_cuda(ctx, launch_dependent(moe_pack_tokens_kernel, dim3(tokens), 256, 0, cs, x, x_dtype, ldx, w.pos, w.xs, d.d_model, d.top_k),
                             "moe_pack_tokens launch");
@@ -948,10 +948,12 @@ extern "C" int32_t iq_moe_forward(iq_moe* l, void* stream, const void* x, int32_
     if (pieces & IQ_PIECE_DOWN) {
         // h's digits come from the halves that lie in the workspace, whichever call or caller left them there: the kernels for few tokens leave digits of
         // another form in fh. The tiles may start before the digits are there: the kernel that makes them lets them, after its own wait.
-        const bool on_tiles = int8 && !after_gemm && (!wide_h || P <= (int64_t)d.expert_count * (d.d_ff < 1024 ? 2 : kWideRowsPerExpert));
-        st = on_tiles ? launch_fixed_rows(ctx, cs, w.h, kF16, d.d_ff, P, d.d_ff, w.fh, wide_h) : 1;
-        if (st == kOk) st = run_down_tile(l, cs, w, wide_h, max_tiles);
-        if (st == 1) st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn, after_gemm);
+        if (int8 && (!wide_h || P <= (int64_t)d.expert_count * (d.d_ff < 1024 ? 2 : kWideRowsPerExpert))) {
+            st = launch_fixed_rows(ctx, cs, w.h, kF16, d.d_ff, P, d.d_ff, w.fh, wide_h);
+            if (st == kOk) st = run_down_tile(l, cs, w, wide_h, max_tiles);
+        } else {
+            st = run_down_tc(l, cs, w.h, P, w.tiles_b, w.ntiles + 1, w.yd, yd_dtype_of(l), bn, after_gemm);
+        }
         if (st != kOk) return st;
     }
     if (pieces & IQ_PIECE_COMBINE) {
@@ -1070,7 +1072,7 @@ int32_t moe_experts_impl(iq_moe* l, void* stream, const void* rows_f16, const ui
     int32_t st = check_cuda(ctx, cudaGetLastError(), "ep_tiles launch");
     if (st != kOk) return st;
     const int max_tiles = (int)std::min<int64_t>(max_rows / kDecodeTileRows + slots, max_rows);
-    st = int8 ? run_gateup(l, cs, rows_f16, kF16, d.d_model, row_index, w.tiles, w.ntiles, max_tiles, w.h, 1) : 1;
+    st = int8 ? run_gateup(l, cs, rows_f16, kF16, d.d_model, row_index, w.tiles, w.ntiles, max_tiles, w.h) : 1;
     if (st == 1) {
         const __half* rows = static_cast<const __half*>(rows_f16);
         if (row_index != nullptr) {

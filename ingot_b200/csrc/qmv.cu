@@ -434,39 +434,32 @@ int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     return kOk;
 }
 
-// ---- int8 tensor-core path for the MoE decode tiles (gate/up + activation, down; affine 4-bit experts) ---------------
+// ---- int8 tensor-core path of the expert-parallel pieces (gate/up + activation, down; affine 4-bit experts) ---------------
 typedef void (*QgKernel)(const CUtensorMap, const CUtensorMap, const QgParams);
 // gw4: each consumer warp's K slice is four groups, its activation fragments stay in registers
-template <int MODE, bool TM>
-QgKernel qg_pick_mt(bool gw4) {
-    constexpr bool TWO = MODE == kModeDown;
-    return gw4 ? qmv_imma_grouped_kernel<MODE, TM, 4, TWO> : qmv_imma_grouped_kernel<MODE, TM, 0, TWO>;
-}
 // (the two-wide fp32 form costs registers: it pays in the down projections)
-QgKernel qg_pick(int mode, bool tm, bool gw4) {
-    if (mode == kModeGateUp) return tm ? qg_pick_mt<kModeGateUp, true>(gw4) : qg_pick_mt<kModeGateUp, false>(gw4);
-    return tm ? qg_pick_mt<kModeDown, true>(gw4) : qg_pick_mt<kModeDown, false>(gw4);
+QgKernel qg_pick(int mode, bool gw4) {
+    if (mode == kModeGateUp) return gw4 ? qmv_imma_grouped_kernel<kModeGateUp, 4, false> : qmv_imma_grouped_kernel<kModeGateUp, 0, false>;
+    return gw4 ? qmv_imma_grouped_kernel<kModeDown, 4, true> : qmv_imma_grouped_kernel<kModeDown, 0, true>;
 }
-}  // namespace
 
-namespace {
 // How a call is cut. K slices per block of rows: one slice of four groups per warp when K allows it (the activation
 // fragments then live in registers: 69 against 83 us on the 64-token layer); else four slices (32-row blocks: half as
 // many hand-overs per byte) when two stages of that size fit, else eight.
 struct QgCut {
     int wk, nstages;  // (fewer than two stages: the shape does not fit)
-    int row_pitch, srow_bytes, xq_bytes, xsc_bytes, red_bytes, fixed, mat_bytes;
+    int srow_bytes, xq_bytes, xsc_bytes, red_bytes, fixed, mat_bytes;
 };
-QgCut qg_cut(int K, int nw, bool tm) {
+QgCut qg_cut(int K, int nw) {
     constexpr int ms = 2;  // sets of four activation rows per tile
     const int G = K / 64, row_bytes = K / 2;
     QgCut c = {};
-    c.row_pitch = tm ? row_bytes : row_bytes + 32;
+    if (K % 256 != 0 || K > 65536) return c;  // (tensor copies: whole columns of 128 bytes, up to 256 of them)
     c.srow_bytes = G * 2;
     c.xq_bytes = G * ms * 512;
     c.xsc_bytes = G * ms * 32;
     c.red_bytes = 2 * kQgWarps * nw * ms * 64 * 4;
-    c.fixed = c.xq_bytes + c.xsc_bytes + c.red_bytes + 256 + (tm ? 1024 : 0);
+    c.fixed = c.xq_bytes + c.xsc_bytes + c.red_bytes + 256 + 1024;
     const bool gw4 = G == 4 * kQgWarps;
     const int cand[4] = {gw4 ? kQgWarps : kQgWarps / 2, kQgWarps, kQgWarps / 4, kQgWarps / 8};
     for (int ci = 0; ci < 4 && c.nstages < 2; ci++) {
@@ -475,25 +468,22 @@ QgCut qg_cut(int K, int nw, bool tm) {
         const int R = 16 * (kQgWarps / wk);
         if ((R * c.srow_bytes) % 16 != 0) continue;
         c.wk = wk;
-        c.mat_bytes = round_up(R * c.row_pitch + 2 * R * c.srow_bytes, tm ? 1024 : 16);
+        c.mat_bytes = round_up(R * row_bytes + 2 * R * c.srow_bytes, 1024);
         c.nstages = (kQsSmemMax - c.fixed) / (nw * c.mat_bytes);
     }
     return c;
 }
-// (tensor copies; without them no multiple of four groups is left)
-bool qg_tensor_copies(int K) { return K % 256 == 0 && K <= 65536; }
 }  // namespace
 
 int qmv_grouped_slices(int K, int nw) {
-    if (K % 64 != 0 || !qg_tensor_copies(K)) return 0;
-    const QgCut c = qg_cut(K, nw, true);
+    const QgCut c = qg_cut(K, nw);
     return c.nstages >= 2 ? c.wk : 0;
 }
 
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     if ((c.mode != kModeGateUp && c.mode != kModeDown) || c.tiles == nullptr || c.fmt != kFmtAffine4) return 1;
-    if (c.K % 64 != 0 || c.N % 16 != 0 || c.max_rows > 8 || c.accumulate) return 1;
+    if (c.N % 16 != 0 || c.max_rows > 8 || c.accumulate || ctx->encode_tiled == nullptr) return 1;
     const int nw = c.mode == kModeGateUp ? 2 : 1;
     for (int i = 0; i < nw; i++)
         if ((reinterpret_cast<uintptr_t>(c.w[i]) & 15) || (reinterpret_cast<uintptr_t>(c.s[i]) & 15) ||
@@ -503,45 +493,30 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     QgParams p;
     memset(&p, 0, sizeof(p));
     p.row_bytes = c.K / 2;
-    // Tensor-copy staging: the stacked tensors must be known (which experts they hold) and dense, rows whole 128-byte
-    // columns. Short weight rows (the down projection's K = d_ff, 384 bytes) take this path only with tensor copies: one
-    // bulk copy per row measured 61.9 against 49.6 us on the fp16 tile kernels at 64 tokens; with tensor copies, 128-row
-    // blocks and no K split (12 groups of 64 inputs do not divide into runs of four over more than one slice) it
-    // measures 37.3 us (16 tokens: 23.9 against 30.6; 256 tokens: 79.8 against 121).
-    const bool tm = ctx->encode_tiled != nullptr && c.expert_count > 0 && qg_tensor_copies(c.K) &&
-                    c.w_estride * 4 == (int64_t)c.N * p.row_bytes;
-    if (c.K < 2048 && !tm) return 1;
-    const QgCut cut = qg_cut(c.K, nw, tm);
+    const QgCut cut = qg_cut(c.K, nw);
     if (cut.nstages < 2) return 1;
     const int nstages = cut.nstages < 8 ? cut.nstages : 8, R = 16 * (kQgWarps / cut.wk), fixed = cut.fixed;
-    p.row_pitch = cut.row_pitch; p.srow_bytes = cut.srow_bytes;
+    p.srow_bytes = cut.srow_bytes;
     p.xq_bytes = cut.xq_bytes; p.xsc_bytes = cut.xsc_bytes; p.red_bytes = cut.red_bytes;
     p.wk = cut.wk; p.rgs = kQgWarps / cut.wk;
     p.NB = (c.N + R - 1) / R;
     p.mat_bytes = cut.mat_bytes; p.stage_bytes = nw * cut.mat_bytes;
     p.nstages = nstages;
     for (int i = 0; i < 2; i++) {
-        p.w[i] = reinterpret_cast<const unsigned char*>(c.w[i] ? c.w[i] : c.w[0]);
         p.s[i] = reinterpret_cast<const unsigned char*>(c.s[i] ? c.s[i] : c.s[0]);
         p.b[i] = reinterpret_cast<const unsigned char*>(c.b[i] ? c.b[i] : c.b[0]);
         p.ebias[i] = c.ebias[i];
     }
-    p.w_ebytes = c.w_estride * 4;
     p.s_ebytes = c.s_estride * 2;
     p.expert_lo = c.expert_lo;
-    p.early = c.early ? 1 : 0;
     CUtensorMap wmaps[2] = {};
-    const CUtensorMap* maps[2] = {&wmaps[0], &wmaps[1]};
-    if (tm) {
-        for (int i = 0; i < nw; i++) {
-            const int32_t r = cached_rowblock_map(ctx, p.w[i] + (int64_t)c.expert_lo * p.w_ebytes, (int64_t)c.expert_count * c.N,
-                                                  p.row_bytes, 16 * p.rgs, &wmaps[i]);
-            if (r != kOk) return r;
-        }
+    for (int i = 0; i < nw; i++) {
+        const int32_t r = cached_rowblock_map(ctx, c.w[i] + (int64_t)c.expert_lo * c.w_estride, (int64_t)c.expert_count * c.N, p.row_bytes, 16 * p.rgs, &wmaps[i]);
+        if (r != kOk) return r;
     }
     p.N = c.N; p.K = c.K;
     p.x = c.x; p.x_dtype = c.x_dtype; p.ldx = c.ldx;
-    p.row_map = c.row_map; p.topk = c.topk;
+    p.row_map = c.row_map;
     p.tiles = c.tiles; p.ntiles = c.ntiles;
     p.y = c.y; p.y_dtype = c.y_dtype; p.ldy = c.ldy;
     p.limit = c.limit;
@@ -559,7 +534,7 @@ int32_t launch_qmv_imma_grouped(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, tm, G == 4 * kQgWarps && p.wk == kQgWarps), *maps[0], *maps[1], p), "qmv_imma_grouped launch");
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qg_pick(c.mode, G == 4 * kQgWarps && p.wk == kQgWarps), wmaps[0], wmaps[1], p), "qmv_imma_grouped launch");
 }
 
 int32_t gqmv_init(iq_ctx* ctx) {
@@ -575,8 +550,8 @@ int32_t gqmv_init(iq_ctx* ctx) {
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma)");
     }
     for (int mode = kModeGateUp; mode <= kModeDown; mode++)
-        for (int v = 0; v < 4; v++) {  // bulk or tensor copies; activations in registers or not
-            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(mode, v >= 2, v % 2 == 1)),
+        for (int v = 0; v < 2; v++) {  // activations in registers or not
+            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qg_pick(mode, v == 1)),
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kQsSmemMax);
             if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_imma_grouped)");
         }

@@ -34,16 +34,14 @@ __device__ __forceinline__ void qg_bar_sync(int id, int threads) { asm volatile(
 __device__ __forceinline__ void qg_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
 struct QgParams {
-    const unsigned char* w[2];
     const unsigned char* s[2];
     const unsigned char* b[2];
-    int64_t w_ebytes, s_ebytes;  // bytes between experts (codes; scales = biases)
+    int64_t s_ebytes;            // bytes between experts (scales = biases)
     int32_t N, K;
     const void* x;
     int32_t x_dtype;
     int64_t ldx;
-    const uint32_t* row_map;     // gate/up: sorted position -> pair id (token = pair / topk); null: rows are in place
-    int32_t topk;
+    const uint32_t* row_map;     // gate/up: sorted position -> row of x; null: rows are in place
     const Tile* tiles;
     const uint32_t* ntiles;
     void* y;
@@ -52,36 +50,34 @@ struct QgParams {
     const float* ebias[2];
     float limit;
     int32_t act;
-    int32_t early;               // the tile list is complete when this kernel starts
     int32_t rgs, wk;             // row blocks of 16 per item x K slices = consumer warps
     int32_t NB;                  // items per tile
-    int32_t row_bytes, row_pitch, srow_bytes;
+    int32_t row_bytes, srow_bytes;
     int32_t mat_bytes, stage_bytes, nstages;
-    int32_t expert_lo;           // tensor-copy staging: the first expert the stacked tensors (and the maps) hold
+    int32_t expert_lo;           // the first expert the stacked tensors (and the maps) hold
     int32_t xq_bytes, xsc_bytes, red_bytes;
     int32_t* status;
 };
 
 // MODE: kModeGateUp (two matrices, h = act(gate, up)) or kModeDown.
-// TM: a block of R rows of a matrix arrives as one swizzled tensor copy, laid out [128-byte column][row][128] (see
+// A block of R rows of a matrix arrives as one swizzled tensor copy, laid out [128-byte column][row][128] (see
 // qmv_imma.cuh), instead of one bulk copy per row: expert rows are 384 to 1024 bytes, and copies that short are bound by
 // their issue rate (one producer warp sustains about one per 60 ns), not by their bytes.
 // GW: groups of 64 inputs per consumer warp when fixed at compile time (4), else 0. A warp's K slice does not change from
 // item to item, so with GW > 0 its activation fragments stay in registers between tile changes: read from shared
 // memory per item they are as many bytes as the codes themselves, and the kernel runs at the shared-memory port's rate.
 // TWO: scales and biases by two-wide fp32 operations, three instructions for six, rounded alike (qg_pick).
-template <int MODE, bool TM, int GW, bool TWO>
+template <int MODE, int GW, bool TWO>
 __global__ void __launch_bounds__(kQgThreads, 1)
     qmv_imma_grouped_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, const QgParams p) {
     constexpr int NW = MODE == kModeGateUp ? 2 : 1;
     constexpr int MS = 2;   // sets of four activation rows per tile
-    constexpr int GB = 32;  // code bytes per group of 64 inputs (4-bit)
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char* xq = smem;                                            // [groups][MS][32 lanes] uint4: B fragments
     float2* xsc = reinterpret_cast<float2*>(smem + p.xq_bytes);          // [groups][MS * 4 rows] {2^(e-15), sum x}
     float* red = reinterpret_cast<float*>(smem + p.xq_bytes + p.xsc_bytes);  // [2][kQgWarps][NW * MS][32 lanes][2]
     unsigned char* stages = smem + p.xq_bytes + p.xsc_bytes + p.red_bytes;
-    if (TM) stages += (1024u - (smem_u32(stages) & 1023u)) & 1023u;  // the swizzle pattern is a function of the address
+    stages += (1024u - (smem_u32(stages) & 1023u)) & 1023u;  // the swizzle pattern is a function of the address
     uint64_t* bars = reinterpret_cast<uint64_t*>(stages + (size_t)p.nstages * p.stage_bytes);
     const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * p.nstages;
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * p.nstages);
@@ -91,7 +87,7 @@ __global__ void __launch_bounds__(kQgThreads, 1)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NCT = kQgWarps * 32;     // consumer threads
     constexpr int NET = kQgEpilogueWarps * 32;  // epilogue threads
-    if (TM && tid == NCT) {
+    if (tid == NCT) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map0) : "memory");
         if (NW == 2) asm volatile("prefetch.tensormap [%0];" ::"l"(&map1) : "memory");
     }
@@ -105,15 +101,13 @@ __global__ void __launch_bounds__(kQgThreads, 1)
         fence_async_smem();
     }
     __syncthreads();
-    // The tile list, the activations and y come from earlier kernels of the stream. A down projection behind this kernel's own
-    // gate/up (p.early) may read the list at once and stream weights: the gate/up lets its dependents start only after its
-    // own wait, so that the list is complete by then.
-    if (!p.early) pdl_wait();
+    // The tile list, the activations and y come from earlier kernels of the stream
+    pdl_wait();
     pdl_launch_dependents();
 
     const int R = 16 * p.rgs;
     const int G = p.K / 64;
-    const int codes_bytes = R * p.row_pitch;
+    const int codes_bytes = R * p.row_bytes;
     const int sc_bytes = R * p.srow_bytes;
     // This CTA's contiguous range of items. An item of a tile with more live row sets costs more (about 3 + sets in
     // units of issue slots), so the ranges are cut by cost, not by count: warp 0 adds up the tiles' costs (a lane per run
@@ -190,37 +184,19 @@ __global__ void __launch_bounds__(kQgThreads, 1)
             if (!ok) break;
             // (a tensor copy counts its whole box; rows past the block belong to the next expert or arrive as zeros)
             if (lane == 0)
-                mbar_arrive_expect_tx(bar_full + 8 * s, NW * ((TM ? R : rows) * p.row_bytes + 2 * rows * p.srow_bytes));
+                mbar_arrive_expect_tx(bar_full + 8 * s, NW * (R * p.row_bytes + 2 * rows * p.srow_bytes));
             __syncwarp();
             const uint32_t st = smem_u32(stages + (size_t)s * p.stage_bytes);
-            if (TM) {
-                // per matrix: one tensor copy of the codes, one bulk copy of the scales, one of the biases
-                if (lane < NW * 3) {
-                    const int i = lane / 3, q = lane % 3;
-                    const uint32_t dst = st + i * p.mat_bytes;
-                    if (q == 0) {
-                        tma_load_3d(dst, i == 0 ? &map0 : &map1, bar_full + 8 * s, 0,
-                                    (int)(expert - (uint32_t)p.expert_lo) * p.N + r0, 0);
-                    } else {
-                        const unsigned char* src = (q == 1 ? p.s[i] : p.b[i]) + expert * p.s_ebytes + (int64_t)r0 * p.srow_bytes;
-                        bulk_g2s(dst + codes_bytes + (q == 2 ? sc_bytes : 0), src, rows * p.srow_bytes, bar_full + 8 * s);
-                    }
-                }
-            } else {
-                // per matrix: one copy per row of codes (into padded rows), one for the scales, one for the biases
-                for (int j = lane; j < NW * (rows + 2); j += 32) {
-                    const int i = j / (rows + 2), q = j % (rows + 2);
-                    const uint32_t dst = st + i * p.mat_bytes;
-                    if (q < rows) {
-                        bulk_g2s(dst + q * p.row_pitch, p.w[i] + expert * p.w_ebytes + (int64_t)(r0 + q) * p.row_bytes, p.row_bytes,
-                                 bar_full + 8 * s);
-                    } else if (q == rows) {
-                        bulk_g2s(dst + codes_bytes, p.s[i] + expert * p.s_ebytes + (int64_t)r0 * p.srow_bytes, rows * p.srow_bytes,
-                                 bar_full + 8 * s);
-                    } else {
-                        bulk_g2s(dst + codes_bytes + sc_bytes, p.b[i] + expert * p.s_ebytes + (int64_t)r0 * p.srow_bytes,
-                                 rows * p.srow_bytes, bar_full + 8 * s);
-                    }
+            // per matrix: one tensor copy of the codes, one bulk copy of the scales, one of the biases
+            if (lane < NW * 3) {
+                const int i = lane / 3, q = lane % 3;
+                const uint32_t dst = st + i * p.mat_bytes;
+                if (q == 0) {
+                    tma_load_3d(dst, i == 0 ? &map0 : &map1, bar_full + 8 * s, 0,
+                                (int)(expert - (uint32_t)p.expert_lo) * p.N + r0, 0);
+                } else {
+                    const unsigned char* src = (q == 1 ? p.s[i] : p.b[i]) + expert * p.s_ebytes + (int64_t)r0 * p.srow_bytes;
+                    bulk_g2s(dst + codes_bytes + (q == 2 ? sc_bytes : 0), src, rows * p.srow_bytes, bar_full + 8 * s);
                 }
             }
             if (++s == p.nstages) { s = 0; ph ^= 1; }
@@ -236,7 +212,6 @@ __global__ void __launch_bounds__(kQgThreads, 1)
         }
     } else if (warp < kQgWarps) {
         // ================= consumers =================
-        if (p.early) pdl_wait();
         const int g = lane >> 2, t = lane & 3;
         const int rb = warp / p.wk, ks = warp % p.wk;
         const int gw = GW > 0 ? GW : G / p.wk, g0 = ks * gw;
@@ -267,8 +242,7 @@ __global__ void __launch_bounds__(kQgThreads, 1)
                 // the rows' places in x first (one round trip to memory for all of them), then the values, four units
                 // of eight inputs per thread in flight
                 if (tid < M) {
-                    srow[tid] = (MODE == kModeGateUp && p.row_map != nullptr) ? p.row_map[tile.start + tid] / (uint32_t)p.topk
-                                                                             : tile.start + (uint32_t)tid;
+                    srow[tid] = (MODE == kModeGateUp && p.row_map != nullptr) ? p.row_map[tile.start + tid] : tile.start + (uint32_t)tid;
                 }
                 qi_consumer_barrier(NCT);
                 const int units = G * 8 * M, upad = (units + 31) / 32 * 32;
@@ -368,12 +342,10 @@ __global__ void __launch_bounds__(kQgThreads, 1)
                             uint32_t a[NW][8];
 #pragma unroll
                             for (int i = 0; i < NW; i++) {
-                                // TM: column grp / 4 of the block, row rb * 16 + g, 16-byte piece ((grp % 4) * 2 + t / 2) ^ g
-                                const uint32_t wa0 = st + i * p.mat_bytes +
-                                                     (TM ? (grp >> 2) * (R * 128) + (rb * 16 + g) * 128 +
-                                                               (((((grp & 3) << 1) + (t >> 1)) ^ g) << 4) + ((t & 1) << 3)
-                                                         : (rb * 16 + g) * p.row_pitch + t * 8 + grp * GB);
-                                const uint32_t wa1 = wa0 + (TM ? 1024 : 8 * p.row_pitch);
+                                // column grp / 4 of the block, row rb * 16 + g, 16-byte piece ((grp % 4) * 2 + t / 2) ^ g
+                                const uint32_t wa0 = st + i * p.mat_bytes + (grp >> 2) * (R * 128) + (rb * 16 + g) * 128 +
+                                                     (((((grp & 3) << 1) + (t >> 1)) ^ g) << 4) + ((t & 1) << 3);
+                                const uint32_t wa1 = wa0 + 1024;
                                 const uint2 w0 = lds64_after(wa0, tok), w1 = lds64_after(wa1, tok);
                                 constexpr uint32_t MSK = 0x0F0F0F0Fu;
                                 a[i][0] = w0.x & MSK; a[i][1] = w1.x & MSK; a[i][2] = (w0.x >> 4) & MSK; a[i][3] = (w1.x >> 4) & MSK;
@@ -464,7 +436,6 @@ __global__ void __launch_bounds__(kQgThreads, 1)
         }
     } else {
         // ================= epilogue =================
-        if (p.early) pdl_wait();
         const int et = tid - (kQgWarps + 1) * 32;
         const int rsh = 31 - __clz(R);  // R is a power of two
         int ti = lo / p.NB, blk = lo % p.NB, cur_tile = -1, M = 0;

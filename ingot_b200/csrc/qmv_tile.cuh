@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(qt_threads(ND), 2) qmv_tile_kernel(const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // A down projection behind this kernel's own gate/up may read the tile list and the weights at once (p.early, see qmv_imma_grouped.cuh)
+    // With p.early (the kernel before this one lets its dependents start after its own wait) the tile list and the weights may be read at once
     const bool weights_only = warp == 2 || warp == 3 || warp >= 4 + 4 * SG;
     if (!p.early || !weights_only) pdl_wait();
     pdl_launch_dependents();

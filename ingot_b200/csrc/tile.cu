@@ -20,21 +20,19 @@ static QtKernel qt_pick(int epi, bool wide) {
 }
 
 int32_t launch_qmv_tile(iq_ctx* ctx, cudaStream_t st, const QmmCall& c, const FixedRows& x, bool wide, const uint32_t* row_map, int32_t topk, int32_t slice, int32_t max_tiles) {
-    if (c.fmt != kFmtAffine4 || c.tiles == nullptr || c.K % 64 != 0 || c.bn != kQtRows || c.accumulate || c.y_dtype != kF16 || (c.epi && !wide && c.K % 256 != 0) ||
-        ctx->encode_tiled == nullptr)
-        return 1;
+    if (c.fmt != kFmtAffine4 || c.tiles == nullptr || c.K % (wide ? 64 : 256) != 0 || c.bn != kQtRows || c.accumulate || c.y_dtype != kF16 || slice < 1)
+        return fail(ctx, kErrNoKernel, "moe: no decode tiles for format %d, %d inputs", c.fmt, c.K);
     QtParams p;
     memset(&p, 0, sizeof(p));
     QtMaps maps = {};
     uintptr_t align = 0;
     for (int i = 0; i <= c.epi; i++) {
-        if (reinterpret_cast<uintptr_t>(c.w[i]) & 15) return 1;
         align |= reinterpret_cast<uintptr_t>(c.s[i]) | reinterpret_cast<uintptr_t>(c.b[i]);
         p.s[i] = c.s[i]; p.b[i] = c.b[i]; p.ebias[i] = c.ebias[i];
         const int32_t r = cached_rows_map(ctx, c.w[i], (int64_t)c.experts * c.N, c.K / 2, c.epi ? 64 : 128, &maps.w[i]);
         if (r != kOk) return r;
     }
-    if (align & 1) return 1;
+    if (align & 1) return fail(ctx, kErrInvalidArg, "moe: scales and biases must be 2-byte aligned");
     p.vec = c.K % 256 == 0 && (align & 7) == 0;
     p.expert_lo = c.expert_lo;
     p.N = c.N; p.K = c.K;
