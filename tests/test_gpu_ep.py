@@ -32,10 +32,10 @@ def make_layers(rng, device, E, K, D, I, world, max_tokens):
     return layers, wr, (lambda e: (deq(g, e), deq(u, e), deq(d, e)))
 
 
-@pytest.mark.parametrize("world,T,region", [(2, 6, 0), (4, 37, 0), (2, 128, 0), (4, 37, 64), (2, 128, 300)])
-def test_ep_pieces_emulated_on_one_gpu(cuda_device, world, T, region):
+def run_pieces(cuda_device, world, T, region, D, I):
+    """A block of T tokens over `world` emulated ranks, the rows packed or in regions of their source, against the oracle."""
     rng = np.random.default_rng(world * 100 + T)
-    E, K, D, I = 32, 4, 256, 128
+    E, K = 32, 4
     layers, wr, weights = make_layers(rng, cuda_device, E, K, D, I, world, T)
     x = synth.activations_np(rng, T, D)
     slices = [ep.token_slice(r, world, T) for r in range(world)]
@@ -78,6 +78,19 @@ def test_ep_pieces_emulated_on_one_gpu(cuda_device, world, T, region):
     ref = qref.moe_ffn(x, inds, wts, weights)
     # the expert outputs cross the "wire" as fp32
     assert qref.max_rel(got, ref) <= TOL
+
+
+@pytest.mark.parametrize("world,T,region", [(2, 6, 0), (4, 37, 0), (2, 128, 0), (4, 37, 64), (2, 128, 300)])
+def test_ep_pieces_emulated_on_one_gpu(cuda_device, world, T, region):
+    run_pieces(cuda_device, world, T, region, 256, 128)
+
+
+@pytest.mark.parametrize("D,I", [(2048, 768), (1024, 2048), (512, 1536), (2112, 256), (2880, 768)])
+@pytest.mark.parametrize("world,T,region", [(2, 9, 0), (2, 60, 0), (4, 40, 64)])
+def test_ep_pieces_by_width(cuda_device, D, I, world, T, region):
+    """The forms of the pieces' kernel: gate/up and down with four groups per warp, one, two, four and eight K slices, one of the two by the GEMM (2112 and
+    2880 inputs); one to eight rows per tile and second tiles, rows packed and in regions."""
+    run_pieces(cuda_device, world, T, region, D, I)
 
 
 @pytest.mark.parametrize("world,T,yd_dtype,fused", [(2, 6, torch.float32, False), (4, 37, torch.float32, True),

@@ -482,7 +482,7 @@ def test_moe_mxfp4_scales_at_odd_addresses(cuda_device, T):
 @pytest.mark.parametrize("D,I", [(1536, 128), (3072, 64), (5120, 64), (768, 1536)])
 @pytest.mark.parametrize("T", [4, 40])
 def test_moe_decode_widths_that_are_no_power_of_two(cuda_device, D, I, T):
-    """Widths whose K slices do not divide the sixteen warps: the int8 kernels convert the token rows themselves, gate/up as down."""
+    """Inputs that are no power of two: the decode tiles take them as three digits, and h as two (1536 features) or three."""
     rng = np.random.default_rng(980 + D + T)
     layer, host = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
@@ -537,8 +537,7 @@ def test_moe_tall_tiles_on_pairs(cuda_device, fmt, act, D, I, T):
 @pytest.mark.parametrize("D,I", [(1024, 320), (2048, 1408), (4096, 256)])
 @pytest.mark.parametrize("T", [5, 40])
 def test_moe_int8_experts_by_width(cuda_device, D, I, T):
-    """The int8 expert kernels with the rows as fixed point, whose scales go by two-wide or by plain fp32 operations depending on the
-    inputs: one set of rows per expert and two."""
+    """The decode tiles with inputs as two digits, h as two (256 features) or three: up to four rows per expert and more."""
     rng = np.random.default_rng(95 + D + T)
     layer, host = build_layer(rng, cuda_device, 32, 4, D, I, max_tokens=T)
     check_layer(layer, host, synth.activations_np(rng, T, D), T, "silu")
