@@ -14,7 +14,7 @@
 struct iq_ctx {
     int device = 0;
     int sms = 0;
-    int rows_clusters[4] = {};  // clusters of 1, 2, 4 and 8 CTAs of csrc/qmv_rows.cuh that run at once
+    int rows_clusters[3] = {};  // clusters of two, four and eight CTAs of csrc/qmv_rows.cuh that run at once
     int smem_optin = 0;
     // cuTensorMapEncodeTiled, resolved through the runtime so that the library does not link libcuda directly
     void* encode_tiled = nullptr;

@@ -10,7 +10,8 @@
 // stay where they are: a step of 256 inputs takes this machine 1000 to 2000 cycles whatever its rows (waits on barriers, loads from tensor memory and sums
 // of one step follow one another in a warp), and 14336 x 4096 at 8 rows took 29.0 us instead of 20.4.
 //
-// Unit of work: a tile over all of K, or over the K slices of one CTA of a cluster. K is walked slice by slice as the ring kernel cuts it (every wk-th
+// Unit of work: a cluster of two to eight CTAs takes a tile, each its share of the K slices (the digits of all of K fit one CTA only where a cluster is
+// faster). K is walked slice by slice as the ring kernel cuts it (every wk-th
 // column; a column is 128 bytes of a row's codes), so that every slice's sum is one accumulator's; the slices are added in their order
 // at the end, through the cluster's shared memory. The activations' digits for the CTA's columns are made once, by the warps
 // that later finish the sums, while the first weights arrive, and stay in shared memory.
@@ -126,9 +127,9 @@ __global__ void __launch_bounds__(kQwThreads, 1) qmv_rows_kernel(const __grid_co
     const uint32_t xs0 = scales0 + NST * 2 * 128 * SPB;
     unsigned char* xd = smem + (size_t)NST * kQtCodes;
     float* xs = reinterpret_cast<float*>(smem + (size_t)(xs0 - codes0));
-    float* part = xs + (size_t)p.xcols * GPC * T * 2;         // [slice][token][128 lanes], clusters
-    const int rank = p.cluster > 1 ? (int)cluster_rank() : 0;
-    const int j0 = p.wk * rank / p.cluster, j1 = p.wk * (rank + 1) / p.cluster, jmax = p.cluster > 1 ? (p.wk + p.cluster - 1) / p.cluster : 0;
+    float* part = xs + (size_t)p.xcols * GPC * T * 2;         // [slice][token][128 lanes]
+    const int rank = (int)cluster_rank();
+    const int j0 = p.wk * rank / p.cluster, j1 = p.wk * (rank + 1) / p.cluster, jmax = (p.wk + p.cluster - 1) / p.cluster;
     uint64_t* bars = reinterpret_cast<uint64_t*>(part + (size_t)jmax * T * 128);
     const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kQwMaxStages, bar_aready = bar_empty + 8 * kQwMaxStages, bar_aempty = bar_aready + 32;
     const uint32_t bar_dfull = bar_aempty + 32, bar_dempty = bar_dfull + 16, bar_x = bar_dempty + 16;
@@ -178,23 +179,18 @@ __global__ void __launch_bounds__(kQwThreads, 1) qmv_rows_kernel(const __grid_co
     const int nloc = *ncols;
     pdl_launch_dependents();
 
-    const int ntile = (p.N + NROWS - 1) / NROWS;
-    const int first = (int)blockIdx.x / p.cluster, stride = (int)gridDim.x / p.cluster;
+    const int n0 = (int)blockIdx.x / p.cluster * NROWS;  // of the cluster's tile
 
     if (warp == 2) {
         // ================= packed codes =================
         if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
-            bool ok = true;
-            for (int tile = first; ok && tile < ntile; tile += stride) {
-                const int n0 = tile * NROWS;
-                for (int li = 0; li < nloc; li++) {
-                    if (!(ok = mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag))) break;
-                    mbar_arrive_expect_tx(bar_full + 8 * s, kQtCodes);
-                    tma_load_2d(codes0 + s * kQtCodes, &map, bar_full + 8 * s, (cols[li] & 0x7FFF) * 128, n0);
-                    if (++s == NST) { s = 0; ph ^= 1; }
-                }
+            for (int li = 0; li < nloc; li++) {
+                if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag)) break;
+                mbar_arrive_expect_tx(bar_full + 8 * s, kQtCodes);
+                tma_load_2d(codes0 + s * kQtCodes, &map, bar_full + 8 * s, (cols[li] & 0x7FFF) * 128, n0);
+                if (++s == NST) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 3) {
@@ -203,44 +199,42 @@ __global__ void __launch_bounds__(kQwThreads, 1) qmv_rows_kernel(const __grid_co
         int s = 0;
         uint32_t ph = 0;
         bool ok = true;
-        for (int tile = first; ok && tile < ntile; tile += stride) {
-            const char* src[4][2];
+        const char* src[4][2];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int n = min(tile * NROWS + i * 32 + lane, p.N - 1);
-                src[i][0] = static_cast<const char*>(p.s) + (size_t)n * pitch;
-                src[i][1] = static_cast<const char*>(p.b) + (size_t)n * pitch;
+        for (int i = 0; i < 4; i++) {
+            const int n = min(n0 + i * 32 + lane, p.N - 1);
+            src[i][0] = static_cast<const char*>(p.s) + (size_t)n * pitch;
+            src[i][1] = static_cast<const char*>(p.b) + (size_t)n * pitch;
+        }
+        for (int li = 0; li < nloc; li++) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag));
+            if (!ok) break;
+            const uint32_t dst = scales0 + s * (2 * 128 * SPB) + lane * SPB;
+            const int off = (cols[li] & 0x7FFF) * SPB, left = (int)pitch - off;
+            if (p.vec) {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int m = 0; m < 2; m++) cp_async_ca<SPB>(dst + (m * 128 + i * 32) * SPB, src[i][m] + off);
+                cp_async_arrive_noinc(bar_full + 8 * s);
+            } else {
+                uint32_t v[4][2][GPC];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int m = 0; m < 2; m++)
+#pragma unroll
+                        for (int e = 0; e < GPC; e++) v[i][m][e] = ldg_nc_u16(src[i][m] + off + min(2 * e, left - 2));
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int m = 0; m < 2; m++)
+#pragma unroll
+                        for (int e = 0; e < GPC / 2; e++)
+                            sts32(dst + (m * 128 + i * 32) * SPB + 4 * e, v[i][m][2 * e] | (v[i][m][2 * e + 1] << 16));
+                mbar_arrive(bar_full + 8 * s);
             }
-            for (int li = 0; li < nloc; li++) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag));
-                if (!ok) break;
-                const uint32_t dst = scales0 + s * (2 * 128 * SPB) + lane * SPB;
-                const int off = (cols[li] & 0x7FFF) * SPB, left = (int)pitch - off;
-                if (p.vec) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int m = 0; m < 2; m++) cp_async_ca<SPB>(dst + (m * 128 + i * 32) * SPB, src[i][m] + off);
-                    cp_async_arrive_noinc(bar_full + 8 * s);
-                } else {
-                    uint32_t v[4][2][GPC];
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int m = 0; m < 2; m++)
-#pragma unroll
-                            for (int e = 0; e < GPC; e++) v[i][m][e] = ldg_nc_u16(src[i][m] + off + min(2 * e, left - 2));
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int m = 0; m < 2; m++)
-#pragma unroll
-                            for (int e = 0; e < GPC / 2; e++)
-                                sts32(dst + (m * 128 + i * 32) * SPB + 4 * e, v[i][m][2 * e] | (v[i][m][2 * e + 1] << 16));
-                    mbar_arrive(bar_full + 8 * s);
-                }
-                if (++s == NST) { s = 0; ph ^= 1; }
-            }
+            if (++s == NST) { s = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
@@ -249,37 +243,35 @@ __global__ void __launch_bounds__(kQwThreads, 1) qmv_rows_kernel(const __grid_co
             uint32_t ph = 0, aph = 0, dph = 0;
             const uint32_t idesc = qt_idesc(NB), xdesc0 = (x0 & 0x3FFFFu) >> 4, cdesc0 = (codes0 & 0x3FFFFu) >> 4;
             bool ok = mbar_wait_hint(0, bar_x, 0, abort_flag);
-            for (int tile = first; ok && tile < ntile; tile += stride) {
-                for (int li = 0; li < nloc && ok; li++) {
-                    if (W8 && !(ok = mbar_wait_hint(0, bar_full + 8 * s, ph, abort_flag))) break;
+            for (int li = 0; li < nloc && ok; li++) {
+                if (W8 && !(ok = mbar_wait_hint(0, bar_full + 8 * s, ph, abort_flag))) break;
 #pragma unroll
-                    for (int u = 0; u < UPC; u++) {
-                        if (!W8 && !(ok = mbar_wait_hint(0, bar_aready + 8 * as, aph, abort_flag))) break;
-                        if (!(ok = mbar_wait_hint(0, bar_dempty + 8 * ds, dph ^ 1, abort_flag))) break;
-                        tc_fence_after();
-                        const uint32_t ta = tmem + as * AC, td = tmem + D0 + ds * DC;
+                for (int u = 0; u < UPC; u++) {
+                    if (!W8 && !(ok = mbar_wait_hint(0, bar_aready + 8 * as, aph, abort_flag))) break;
+                    if (!(ok = mbar_wait_hint(0, bar_dempty + 8 * ds, dph ^ 1, abort_flag))) break;
+                    tc_fence_after();
+                    const uint32_t ta = tmem + as * AC, td = tmem + D0 + ds * DC;
 #pragma unroll
-                        for (int g = 0; g < UG; g++) {
-                            const int k0 = (u * UG + g) * GS;  // of the column
-                            const uint32_t xdesc = xdesc0 + (li * (CI / 128) + k0 / 128) * (XT >> 4) + (k0 % 128) / 16;
+                    for (int g = 0; g < UG; g++) {
+                        const int k0 = (u * UG + g) * GS;  // of the column
+                        const uint32_t xdesc = xdesc0 + (li * (CI / 128) + k0 / 128) * (XT >> 4) + (k0 % 128) / 16;
 #pragma unroll
-                            for (int kk = 0; kk < KK; kk++) {
-                                const uint64_t bd = kQtDescHi | (uint64_t)(xdesc + 2 * kk);
-                                if (W8) umma_i8(td + g * NB, kQtDescHi | (uint64_t)(cdesc0 + s * (kQtCodes >> 4) + k0 / 16 + 2 * kk), bd, idesc, kk);
-                                else umma_i8_ta(td + g * NB, ta + g * (GS / 4) + kk * 8, bd, idesc, kk);
-                            }
+                        for (int kk = 0; kk < KK; kk++) {
+                            const uint64_t bd = kQtDescHi | (uint64_t)(xdesc + 2 * kk);
+                            if (W8) umma_i8(td + g * NB, kQtDescHi | (uint64_t)(cdesc0 + s * (kQtCodes >> 4) + k0 / 16 + 2 * kk), bd, idesc, kk);
+                            else umma_i8_ta(td + g * NB, ta + g * (GS / 4) + kk * 8, bd, idesc, kk);
                         }
-                        if (!W8) {
-                            umma_commit(bar_aempty + 8 * as);
-                            if (++as == NA) { as = 0; aph ^= 1; }
-                        }
-                        umma_commit(bar_dfull + 8 * ds);
-                        if (++ds == 2) { ds = 0; dph ^= 1; }
                     }
-                    if (!ok) break;
-                    umma_commit(bar_empty + 8 * s);
-                    if (++s == NST) { s = 0; ph ^= 1; }
+                    if (!W8) {
+                        umma_commit(bar_aempty + 8 * as);
+                        if (++as == NA) { as = 0; aph ^= 1; }
+                    }
+                    umma_commit(bar_dfull + 8 * ds);
+                    if (++ds == 2) { ds = 0; dph ^= 1; }
                 }
+                if (!ok) break;
+                umma_commit(bar_empty + 8 * s);
+                if (++s == NST) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp >= 12) {
@@ -292,46 +284,44 @@ __global__ void __launch_bounds__(kQwThreads, 1) qmv_rows_kernel(const __grid_co
             int s = 0, as = 0;
             uint32_t ph = 0, aph = 0, s_hint = 0, a_hint = 0;
             bool ok = true;
-            for (int tile = first; ok && tile < ntile; tile += stride) {
-                for (int li = 0; li < nloc; li++) {
-                    ok = __all_sync(0xffffffffu, s_hint || mbar_wait(bar_full + 8 * s, ph, abort_flag));
+            for (int li = 0; li < nloc; li++) {
+                ok = __all_sync(0xffffffffu, s_hint || mbar_wait(bar_full + 8 * s, ph, abort_flag));
+                if (!ok) break;
+                const uint32_t codes = codes0 + s * kQtCodes + row * 128;
+#pragma unroll
+                for (int u = 0; u < UPC; u++) {
+                    ok = __all_sync(0xffffffffu, a_hint || mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
                     if (!ok) break;
-                    const uint32_t codes = codes0 + s * kQtCodes + row * 128;
+                    tc_fence_after();
+                    constexpr int PC = UG * GS / 32;  // 16-byte pieces (32 codes) of a unit
 #pragma unroll
-                    for (int u = 0; u < UPC; u++) {
-                        ok = __all_sync(0xffffffffu, a_hint || mbar_wait(bar_aempty + 8 * as, aph ^ 1, abort_flag));
-                        if (!ok) break;
-                        tc_fence_after();
-                        constexpr int PC = UG * GS / 32;  // 16-byte pieces (32 codes) of a unit
+                    for (int i0 = 0; i0 < PC; i0 += 2) {
+                        uint4 v[2];
 #pragma unroll
-                        for (int i0 = 0; i0 < PC; i0 += 2) {
-                            uint4 v[2];
+                        for (int j = 0; j < 2; j++) v[j] = lds128(codes + (((uint32_t)(u * PC + i0 + j) ^ sw) << 4));
+                        const uint32_t w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
+                        uint32_t o[16];
+                        constexpr uint32_t MSK = 0x0F0F0F0Fu;
 #pragma unroll
-                            for (int j = 0; j < 2; j++) v[j] = lds128(codes + (((uint32_t)(u * PC + i0 + j) ^ sw) << 4));
-                            const uint32_t w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
-                            uint32_t o[16];
-                            constexpr uint32_t MSK = 0x0F0F0F0Fu;
-#pragma unroll
-                            for (int j = 0; j < 8; j++) {  // even inputs, odd inputs of eight
-                                o[2 * j] = w[j] & MSK;
-                                o[2 * j + 1] = (w[j] >> 4) & MSK;
-                            }
-                            qt_st16(my_a + as * AC + i0 * 8, o);
+                        for (int j = 0; j < 8; j++) {  // even inputs, odd inputs of eight
+                            o[2 * j] = w[j] & MSK;
+                            o[2 * j + 1] = (w[j] >> 4) & MSK;
                         }
-                        qt_st_wait();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) {
-                            mbar_arrive(bar_aready + 8 * as);
-                            if (u == UPC - 1) mbar_arrive(bar_empty + 8 * s);
-                        }
-                        if (++as == NA) { as = 0; aph ^= 1; }
-                        a_hint = mbar_test(bar_aempty + 8 * as, aph ^ 1);
+                        qt_st16(my_a + as * AC + i0 * 8, o);
                     }
-                    if (!ok) break;
-                    if (++s == NST) { s = 0; ph ^= 1; }
-                    s_hint = mbar_test(bar_full + 8 * s, ph);
+                    qt_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(bar_aready + 8 * as);
+                        if (u == UPC - 1) mbar_arrive(bar_empty + 8 * s);
+                    }
+                    if (++as == NA) { as = 0; aph ^= 1; }
+                    a_hint = mbar_test(bar_aempty + 8 * as, aph ^ 1);
                 }
+                if (!ok) break;
+                if (++s == NST) { s = 0; ph ^= 1; }
+                s_hint = mbar_test(bar_full + 8 * s, ph);
             }
         }
     } else if (warp >= 4) {
@@ -380,112 +370,98 @@ __global__ void __launch_bounds__(kQwThreads, 1) qmv_rows_kernel(const __grid_co
         int s = 0, ds = 0;
         uint32_t ph = 0, dph = 0, s_hint = 0, d_hint = 0;
         bool ok = true;
-        for (int tile = first; ok && tile < ntile; tile += stride) {
-            const int n = tile * NROWS + q * 32 + lane;
-            float acc[H], low[ND == 3 ? H : 1], tot[H];
+        float acc[H], low[ND == 3 ? H : 1];
 #pragma unroll
-            for (int j = 0; j < H; j++) acc[j] = tot[j] = 0.f;
+        for (int j = 0; j < H; j++) acc[j] = 0.f;
 #pragma unroll
-            for (int j = 0; j < (ND == 3 ? H : 1); j++) low[j] = 0.f;
-            int slice = 0;
-            for (int li = 0; li < nloc; li++) {
-                const int cw = cols[li], ng = min(GPC, G - (cw & 0x7FFF) * GPC);
-                ok = s_hint || mbar_wait(bar_full + 8 * s, ph, abort_flag);
-                const uint32_t sa = scales0 + s * (2 * 128 * SPB) + (q * 32 + lane) * SPB;
-                uint32_t scw[GPC / 2], biw[GPC / 2];
+        for (int j = 0; j < (ND == 3 ? H : 1); j++) low[j] = 0.f;
+        int slice = 0;
+        for (int li = 0; li < nloc; li++) {
+            const int cw = cols[li], ng = min(GPC, G - (cw & 0x7FFF) * GPC);
+            ok = s_hint || mbar_wait(bar_full + 8 * s, ph, abort_flag);
+            const uint32_t sa = scales0 + s * (2 * 128 * SPB) + (q * 32 + lane) * SPB;
+            uint32_t scw[GPC / 2], biw[GPC / 2];
 #pragma unroll
-                for (int b = 0; b < 2; b++) {
-                    uint32_t (&o)[GPC / 2] = b ? biw : scw;
-                    const uint32_t a = sa + b * 128 * SPB;
-                    if constexpr (GPC == 8) {
-                        const uint4 r = lds128(a);
-                        o[0] = r.x; o[1] = r.y; o[2] = r.z; o[3] = r.w;
-                    } else if constexpr (GPC == 4) {
-                        const uint2 r = lds64(a);
-                        o[0] = r.x; o[1] = r.y;
-                    } else {
-                        o[0] = lds32(a);
-                    }
-                }
-                const uint32_t xsb = xs0 + li * (GPC * T * 8) + half * (PAIRS * 16);
-#pragma unroll
-                for (int u = 0; u < UPC; u++) {
-                    ok = __all_sync(0xffffffffu, ok && (d_hint || mbar_wait(bar_dfull + 8 * ds, dph, abort_flag)));
-                    if (!ok) break;
-                    tc_fence_after();
-                    // a unit's sums in one go, tensor memory handed back before they are used, the next barriers asked (see qmv_tile.cuh)
-                    int d[UG][ND][H];
-                    if (live > 0) {
-                        const uint32_t td = my_d + ds * DC;
-#pragma unroll
-                        for (int g = 0; g < UG; g++)
-#pragma unroll
-                            for (int i = 0; i < ND; i++) qt_ld(td + g * NB + i * T, d[g][i]);
-#pragma unroll
-                        for (int g = 0; g < UG; g++)
-#pragma unroll
-                            for (int i = 0; i < ND; i++) qw_wait_ld(d[g][i]);
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_dempty + 8 * ds);
-                    if (++ds == 2) { ds = 0; dph ^= 1; }
-                    d_hint = mbar_test(bar_dfull + 8 * ds, dph);
-                    if (u == UPC - 1) s_hint = mbar_test(bar_full + 8 * (s + 1 == NST ? 0 : s + 1), s + 1 == NST ? ph ^ 1 : ph);
-                    auto body = [&](auto np_c, auto full_c) {  // FULL: no branches between the groups' operations
-                        constexpr int NP = decltype(np_c)::value;
-                        constexpr bool FULL = decltype(full_c)::value;
-#pragma unroll
-                        for (int g = 0; g < UG; g++) {
-                            const int gs = u * UG + g;
-                            if (FULL || gs < ng) {
-                                const float sc = __uint_as_float(gs & 1 ? scw[gs / 2] & 0xFFFF0000u : scw[gs / 2] << 16);
-                                const float bi = __uint_as_float(gs & 1 ? biw[gs / 2] & 0xFFFF0000u : biw[gs / 2] << 16);
-#pragma unroll
-                                for (int j = 0; j < NP; j++) {
-                                    const uint4 xv = lds128(xsb + (gs * (T / 2) + j) * 16);
-                                    const float x0f = __uint_as_float(xv.x), x1f = __uint_as_float(xv.y);
-                                    scaled_add2(acc[2 * j], acc[2 * j + 1], (float)(d[g][0][2 * j] * 256 + d[g][1][2 * j]),
-                                                (float)(d[g][0][2 * j + 1] * 256 + d[g][1][2 * j + 1]),
-                                                sc, sc, x0f, x1f);
-                                    fma2(acc[2 * j], acc[2 * j + 1], bi, bi, __uint_as_float(xv.z), __uint_as_float(xv.w));
-                                    if constexpr (ND == 3)
-                                        scaled_add2(low[2 * j], low[2 * j + 1], (float)d[g][ND - 1][2 * j], (float)d[g][ND - 1][2 * j + 1], sc, sc, x0f * 0.0078125f, x1f * 0.0078125f);
-                                }
-                            }
-                        }
-                    };
-                    if (live <= 0) continue;
-                    if (ng < GPC) body(std::integral_constant<int, PAIRS>{}, std::false_type{});
-                    else if (live >= PAIRS) body(std::integral_constant<int, PAIRS>{}, std::true_type{});
-                    else if (PAIRS == 4 && live == 3) body(std::integral_constant<int, PAIRS == 4 ? 3 : 1>{}, std::true_type{});
-                    else body(std::integral_constant<int, PAIRS == 4 ? 2 : 1>{}, std::true_type{});
-                }
-                if (!ok) break;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_empty + 8 * s);
-                if (++s == NST) { s = 0; ph ^= 1; }
-                if (cw & 0x8000) {  // the slice is complete
-#pragma unroll
-                    for (int j = 0; j < H; j++) {
-                        const float v = ND == 3 ? acc[j] + low[ND == 3 ? j : 0] : acc[j];
-                        if (p.cluster > 1) part[(size_t)(slice * T + 4 * (j >> 1) + 2 * half + (j & 1)) * 128 + q * 32 + lane] = v;
-                        else tot[j] += v;
-                        acc[j] = 0.f;
-                        if (ND == 3) low[ND == 3 ? j : 0] = 0.f;
-                    }
-                    slice++;
+            for (int b = 0; b < 2; b++) {
+                uint32_t (&o)[GPC / 2] = b ? biw : scw;
+                const uint32_t a = sa + b * 128 * SPB;
+                if constexpr (GPC == 8) {
+                    const uint4 r = lds128(a);
+                    o[0] = r.x; o[1] = r.y; o[2] = r.z; o[3] = r.w;
+                } else if constexpr (GPC == 4) {
+                    const uint2 r = lds64(a);
+                    o[0] = r.x; o[1] = r.y;
+                } else {
+                    o[0] = lds32(a);
                 }
             }
+            const uint32_t xsb = xs0 + li * (GPC * T * 8) + half * (PAIRS * 16);
+#pragma unroll
+            for (int u = 0; u < UPC; u++) {
+                ok = __all_sync(0xffffffffu, ok && (d_hint || mbar_wait(bar_dfull + 8 * ds, dph, abort_flag)));
+                if (!ok) break;
+                tc_fence_after();
+                // a unit's sums in one go, tensor memory handed back before they are used, the next barriers asked (see qmv_tile.cuh)
+                int d[UG][ND][H];
+                if (live > 0) {
+                    const uint32_t td = my_d + ds * DC;
+#pragma unroll
+                    for (int g = 0; g < UG; g++)
+#pragma unroll
+                        for (int i = 0; i < ND; i++) qt_ld(td + g * NB + i * T, d[g][i]);
+#pragma unroll
+                    for (int g = 0; g < UG; g++)
+#pragma unroll
+                        for (int i = 0; i < ND; i++) qw_wait_ld(d[g][i]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_dempty + 8 * ds);
+                if (++ds == 2) { ds = 0; dph ^= 1; }
+                d_hint = mbar_test(bar_dfull + 8 * ds, dph);
+                if (u == UPC - 1) s_hint = mbar_test(bar_full + 8 * (s + 1 == NST ? 0 : s + 1), s + 1 == NST ? ph ^ 1 : ph);
+                auto body = [&](auto np_c, auto full_c) {  // FULL: no branches between the groups' operations
+                    constexpr int NP = decltype(np_c)::value;
+                    constexpr bool FULL = decltype(full_c)::value;
+#pragma unroll
+                    for (int g = 0; g < UG; g++) {
+                        const int gs = u * UG + g;
+                        if (FULL || gs < ng) {
+                            const float sc = __uint_as_float(gs & 1 ? scw[gs / 2] & 0xFFFF0000u : scw[gs / 2] << 16);
+                            const float bi = __uint_as_float(gs & 1 ? biw[gs / 2] & 0xFFFF0000u : biw[gs / 2] << 16);
+#pragma unroll
+                            for (int j = 0; j < NP; j++) {
+                                const uint4 xv = lds128(xsb + (gs * (T / 2) + j) * 16);
+                                const float x0f = __uint_as_float(xv.x), x1f = __uint_as_float(xv.y);
+                                scaled_add2(acc[2 * j], acc[2 * j + 1], (float)(d[g][0][2 * j] * 256 + d[g][1][2 * j]),
+                                            (float)(d[g][0][2 * j + 1] * 256 + d[g][1][2 * j + 1]),
+                                            sc, sc, x0f, x1f);
+                                fma2(acc[2 * j], acc[2 * j + 1], bi, bi, __uint_as_float(xv.z), __uint_as_float(xv.w));
+                                if constexpr (ND == 3)
+                                    scaled_add2(low[2 * j], low[2 * j + 1], (float)d[g][ND - 1][2 * j], (float)d[g][ND - 1][2 * j + 1], sc, sc, x0f * 0.0078125f, x1f * 0.0078125f);
+                            }
+                        }
+                    }
+                };
+                if (live <= 0) continue;
+                if (ng < GPC) body(std::integral_constant<int, PAIRS>{}, std::false_type{});
+                else if (live >= PAIRS) body(std::integral_constant<int, PAIRS>{}, std::true_type{});
+                else if (PAIRS == 4 && live == 3) body(std::integral_constant<int, PAIRS == 4 ? 3 : 1>{}, std::true_type{});
+                else body(std::integral_constant<int, PAIRS == 4 ? 2 : 1>{}, std::true_type{});
+            }
             if (!ok) break;
-            if (p.cluster > 1) continue;  // (one tile per cluster: its outputs below)
-            // ---- the tile's outputs ----
-            if (n < p.N) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty + 8 * s);
+            if (++s == NST) { s = 0; ph ^= 1; }
+            if (cw & 0x8000) {  // the slice is complete
 #pragma unroll
                 for (int j = 0; j < H; j++) {
-                    const int m = 4 * (j >> 1) + 2 * half + (j & 1);
-                    if (m < p.M) qw_store(p, (size_t)m * p.ldy + n, tot[j]);
+                    const float v = ND == 3 ? acc[j] + low[ND == 3 ? j : 0] : acc[j];
+                    part[(size_t)(slice * T + 4 * (j >> 1) + 2 * half + (j & 1)) * 128 + q * 32 + lane] = v;
+                    acc[j] = 0.f;
+                    if (ND == 3) low[ND == 3 ? j : 0] = 0.f;
                 }
+                slice++;
             }
         }
     }
@@ -501,28 +477,26 @@ __global__ void __launch_bounds__(kQwThreads, 1) qmv_rows_kernel(const __grid_co
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
     }
-    if (p.cluster > 1) {
-        // ---- the slices meet: CTA r finishes rows r, r + cluster, ... of the activations ----
-        cluster_sync_all();
-        pdl_wait();
-        const int n0 = first * NROWS, mine = (p.M - rank + p.cluster - 1) / p.cluster;
-        const uint32_t part0 = smem_u32(part);
-        auto sum = [&](int m, int l) {
-            float v = 0.f;
-            for (int j = 0; j < p.wk; j++) {
-                const int r = ((j + 1) * p.cluster - 1) / p.wk;
-                v += ld_dsmem_f32(part0 + (((j - p.wk * r / p.cluster) * T + m) * 128 + l) * 4, (uint32_t)r);
-            }
-            return v;
-        };
-        if (*abort_flag == 0)
-            for (int o = threadIdx.x; o < mine * NROWS; o += kQwThreads) {
-                const int m = rank + o / NROWS * p.cluster, f = o % NROWS, n = n0 + f;
-                if (n >= p.N) continue;
-                qw_store(p, (size_t)m * p.ldy + n, sum(m, f));
-            }
-        cluster_sync_all();  // (the others read this CTA's slices)
-    }
+    // ---- the slices meet: CTA r finishes rows r, r + cluster, ... of the activations ----
+    cluster_sync_all();
+    pdl_wait();
+    const int mine = (p.M - rank + p.cluster - 1) / p.cluster;
+    const uint32_t part0 = smem_u32(part);
+    auto sum = [&](int m, int l) {
+        float v = 0.f;
+        for (int j = 0; j < p.wk; j++) {
+            const int r = ((j + 1) * p.cluster - 1) / p.wk;
+            v += ld_dsmem_f32(part0 + (((j - p.wk * r / p.cluster) * T + m) * 128 + l) * 4, (uint32_t)r);
+        }
+        return v;
+    };
+    if (*abort_flag == 0)
+        for (int o = threadIdx.x; o < mine * NROWS; o += kQwThreads) {
+            const int m = rank + o / NROWS * p.cluster, f = o % NROWS, n = n0 + f;
+            if (n >= p.N) continue;
+            qw_store(p, (size_t)m * p.ldy + n, sum(m, f));
+        }
+    cluster_sync_all();  // (the others read this CTA's slices)
     if (*abort_flag && threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, kErrTimeout);
 }
 

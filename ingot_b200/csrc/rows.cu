@@ -17,25 +17,25 @@ QwKernel qw_pick(int32_t fmt, int t) {
     return t == 8 ? qmv_rows_kernel<kFmtAffine4, 8> : qmv_rows_kernel<kFmtAffine4, 16>;
 }
 
-// How a call is cut: CTAs per tile (0: it does not fit), stages, columns of a CTA
+// How a call is cut: CTAs per tile (0: it does not fit), stages, columns of a CTA. at_once: clusters of two, four and eight CTAs that run at once
 struct QwPlan {
     int cluster, stages, xcols;
     size_t smem;
 };
-QwPlan qw_plan(const iq_ctx* ctx, int32_t fmt, int t, int N, int K, int wk) {
+QwPlan qw_plan(const int (&at_once)[3], int32_t fmt, int t, int N, int K, int wk) {
     const int ci = fmt == kFmtAffine8 ? 128 : 256, gpc = fmt == kFmtAffine8 ? 2 : fmt == kFmtAffine4G32 ? 8 : 4, nd = fmt == kFmtAffine8 ? 2 : 3;
     const int ncol = (K + ci - 1) / ci, tiles = (N + 127) / 128, stage = kQtCodes + 2 * 128 * 2 * gpc;
     QwPlan best = {0, 0, 0, 0};
     double cost = 0;
-    for (int s = 1; s <= 8 && s <= wk; s *= 2) {
+    for (int s = 2; s <= 8 && s <= wk; s *= 2) {
         const int js = (wk + s - 1) / s, xcols = std::min(ncol, js * ((ncol + wk - 1) / wk));
-        const size_t most = 227 * 1024, fixed = kQwFixed + xcols * qw_x_bytes(ci, gpc, t, nd) + (s > 1 ? (size_t)js * t * 512 : 0);
+        const size_t most = 227 * 1024, fixed = kQwFixed + xcols * qw_x_bytes(ci, gpc, t, nd) + (size_t)js * t * 512;
         if (xcols >= kQwThreads || fixed + 3 * stage > most) continue;
         // cycles: a CTA's start, its digits and its columns, some 1100 per 256 inputs (16 rows: 1500); clusters at once: as the driver says (of
         // eight CTAs the GPU holds fewer than 148 / 8, since a cluster stays in one group of SMs: 2048 x 5120 as 16 clusters of eight took two waves)
-        const int slots = s * ctx->rows_clusters[s == 8 ? 3 : s >> 1], waves = (tiles * s + slots - 1) / slots;
+        const int slots = at_once[s == 8 ? 2 : s == 4], waves = (tiles + slots - 1) / slots;
         const double col = (t == 8 ? 1100.0 : 1500.0) * ci / 256, dig = (double)xcols * ci / 256 * 18 * t;
-        const double c = s == 1 ? 6000 + dig + waves * xcols * col : waves * (8000 + dig + xcols * col);
+        const double c = waves * (8000 + dig + xcols * col);
         if (best.cluster == 0 || c < cost) {
             cost = c;
             best.cluster = s; best.stages = (int)std::min<size_t>(kQwMaxStages, (most - fixed) / stage); best.xcols = xcols;
@@ -50,7 +50,7 @@ int32_t launch_qmv_rows(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, int wk)
     if (c.rows < 1 || c.rows > 16 || ctx->encode_tiled == nullptr || c.mode != kModePlain) return 1;
     if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;
     const int t = c.rows <= 8 ? 8 : 16, row_bytes = c.fmt == kFmtAffine8 ? c.K : c.K / 2;
-    const QwPlan plan = qw_plan(ctx, c.fmt, t, c.N, c.K, wk);
+    const QwPlan plan = qw_plan(ctx->rows_clusters, c.fmt, t, c.N, c.K, wk);
     const uintptr_t align = reinterpret_cast<uintptr_t>(c.s[0]) | reinterpret_cast<uintptr_t>(c.b[0]);
     if (plan.cluster == 0 || (reinterpret_cast<uintptr_t>(c.w[0]) & 15) || (align & 1)) return 1;
     CUtensorMap map = {};
@@ -71,7 +71,7 @@ int32_t launch_qmv_rows(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, int wk)
     const int tiles = (c.N + 127) / 128;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(plan.cluster > 1 ? tiles * plan.cluster : std::min(tiles, ctx->sms), 1, 1);
+    cfg.gridDim = dim3(tiles * plan.cluster, 1, 1);
     cfg.blockDim = dim3(kQwThreads, 1, 1);
     cfg.dynamicSmemBytes = plan.smem;
     cfg.stream = st;
@@ -81,7 +81,7 @@ int32_t launch_qmv_rows(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, int wk)
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = plan.cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = plan.cluster > 1 ? 2 : 1;
+    cfg.numAttrs = 2;
     return check_cuda(ctx, cudaLaunchKernelEx(&cfg, qw_pick(c.fmt, t), map, p), "qmv_rows launch");
 }
 
@@ -91,8 +91,7 @@ int32_t rows_init(iq_ctx* ctx) {
         cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(qw_pick(fmt, v & 1 ? 16 : 8)), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return check_cuda(ctx, e, "cudaFuncSetAttribute(qmv_rows)");
     }
-    // CTAs of a launch that the GPU holds at once, by the cluster's size 1, 2, 4, 8
-    for (int i = 0; i < 4; i++) {
+    for (int i = 1; i < 4; i++) {
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3(ctx->sms / (1 << i) << i, 1, 1);
@@ -109,7 +108,7 @@ int32_t rows_init(iq_ctx* ctx) {
             cudaGetLastError();
             n = ctx->sms * 7 / 8 >> i;
         }
-        ctx->rows_clusters[i] = std::max(n, 1);
+        ctx->rows_clusters[i - 1] = std::max(n, 1);
     }
     return kOk;
 }
