@@ -119,6 +119,17 @@ int32_t iq_abi_version(void);
 int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m, void* y,
                int32_t y_dtype, int64_t ldy, int32_t rows, uint32_t flags, int32_t n_prefix);
 
+/* Whether iq_qmv takes a call over all features of m in one launch of clusters for all its rows (five to sixteen rows of wide 4- and 8-bit matrices,
+ * csrc/qmv_rows.cuh), and how that is divided. Needs no GPU and no context, reads n, k, bits, group and mode of m only and takes its tensors to be
+ * 16-byte aligned. sms, clusters_at_once: the GPU's SMs and how many clusters of two, four and eight CTAs of that kernel run at once (148 and 74, 33
+ * and 15 on B200). No counterpart in the reference: for tests that have to know which path a shape takes. */
+typedef struct iq_qmv_tiling {
+    int32_t cluster;  /* CTAs per tile of 128 features; 0: another kernel, the rest is 0 */
+    int32_t tiles;
+    int32_t slices;   /* pieces of k, each summed by one CTA */
+} iq_qmv_tiling;
+int32_t iq_qmv_plan(const iq_qlinear* m, int32_t rows, int32_t sms, const int32_t clusters_at_once[3], iq_qmv_tiling* out);
+
 /* ---- prefill GEMM --------------------------------------------------------------------------------------------------
  * Y[rows, n] (+)= X[rows, k] * W^T on the tcgen05 tensor cores (weights dequantised to fp16 and fp32 accumulation,
  * both in tensor memory). Replaces DenseQ.encodeQmmF32(ctx, enc, x:, xOffset:, y:, rows:, accumulate:, halfOut:)

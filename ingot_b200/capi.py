@@ -33,7 +33,7 @@ SYMBOLS = [
     "iq_scales_div16_bf16", "iq_argmax_rows", "iq_topk64_scratch_bytes", "iq_topk64", "iq_embed_rows",
     "iq_ctx_set_wait_cycles", "iq_colsplit_create", "iq_colsplit_destroy", "iq_linear_colsplit_workspace_bytes",
     "iq_linear_colsplit", "iq_had_rows", "iq_embed_rows_ternary", "iq_qmm_w8a8_workspace_bytes", "iq_qmm_w8a8",
-    "iq_qmm_plan", "iq_ep_index", "iq_moe_experts_indexed", "iq_ep_pack_push_tokens", "iq_ep_index_tokens",
+    "iq_qmm_plan", "iq_qmv_plan", "iq_ep_index", "iq_moe_experts_indexed", "iq_ep_pack_push_tokens", "iq_ep_index_tokens",
 ]
 
 
@@ -45,6 +45,10 @@ class QLinear(C.Structure):
 class QmmTiling(C.Structure):
     _fields_ = [("tile_rows", C.c_int32), ("tiles", C.c_int32), ("pair", C.c_int32), ("two_per_sm", C.c_int32),
                 ("split_tiles", C.c_int32), ("split_ctas", C.c_int32), ("split_bytes", C.c_size_t), ("bytes_up_to_rows", C.c_size_t)]
+
+
+class QmvTiling(C.Structure):
+    _fields_ = [("cluster", C.c_int32), ("tiles", C.c_int32), ("slices", C.c_int32)]
 
 
 class MoeDesc(C.Structure):
@@ -103,6 +107,8 @@ def lib() -> C.CDLL:
         l.iq_qmm_workspace_bytes.argtypes = [vp, C.POINTER(QLinear), i32, i32, C.POINTER(sz)]
         l.iq_qmm_plan.argtypes = [C.POINTER(QLinear), i32, i32, i32, C.POINTER(QmmTiling)]
         l.iq_qmm_plan.restype = i32
+        l.iq_qmv_plan.argtypes = [C.POINTER(QLinear), i32, i32, C.POINTER(i32), C.POINTER(QmvTiling)]
+        l.iq_qmv_plan.restype = i32
         l.iq_qmm.argtypes = [vp, vp, vp, i32, i64, C.POINTER(QLinear), vp, i32, i64, i32, u32, vp, sz]
         l.iq_dense_ffn_workspace_bytes.argtypes = [vp, C.POINTER(QLinear), C.POINTER(QLinear), i32, i32, C.POINTER(sz)]
         l.iq_dense_ffn.argtypes = [vp, vp, vp, i32, i64, C.POINTER(QLinear), C.POINTER(QLinear), i32, C.c_float, vp,
@@ -258,6 +264,15 @@ def qmm_plan(n: int, k: int, bits: int, group: int, rows: int, mode: int = IQ_MO
     """How a prefill GEMM of this shape is divided (iq_qmm_plan); needs no GPU."""
     out = QmmTiling()
     st = lib().iq_qmm_plan(C.byref(QLinear(0, 0, 0, n, k, bits, group, mode, 1)), int(gate_up), rows, sms, C.byref(out))
+    if st != 0:
+        raise IngotError(st, lib().iq_strerror(st).decode())
+    return out
+
+
+def qmv_plan(n: int, k: int, bits: int, group: int, rows: int, mode: int = IQ_MODE_AFFINE, sms: int = 148, at_once=(74, 33, 15)) -> QmvTiling:
+    """How a decode call of five rows and more is divided where the kernel of clusters takes it (iq_qmv_plan); needs no GPU."""
+    out = QmvTiling()
+    st = lib().iq_qmv_plan(C.byref(QLinear(0, 0, 0, n, k, bits, group, mode, 1)), rows, sms, (C.c_int32 * 3)(*at_once), C.byref(out))
     if st != 0:
         raise IngotError(st, lib().iq_strerror(st).decode())
     return out

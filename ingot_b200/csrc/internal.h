@@ -191,5 +191,7 @@ int32_t rows_init(iq_ctx* ctx);
 // A plain call of several rows of affine 4- or 8-bit weights on csrc/qmv_rows.cuh, with the ring kernel's sums over its wk K slices. 1: not for
 // this kernel.
 int32_t launch_qmv_rows(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, int wk);
+// CTAs per tile that it takes for such a call, 0: none
+int qmv_rows_cluster(const int (&at_once)[3], int32_t fmt, int rows, int N, int K, int wk);
 
 }  // namespace iq

@@ -310,33 +310,49 @@ int32_t launch_qmv_ring(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, bool wk
 }
 
 // ---- int8 tensor-core path (decode, up to four rows, affine codes) -----------------------------------------------
+// How it cuts K inputs of 4-, 6- or 8-bit codes; `fits`: two stages beside what eight rows need, whatever the row count of the call: a row must
+// see the same arithmetic alone and among sixteen.
+struct QiCut {
+    bool tm, pair, fits;
+    int row_bytes, row_pitch, stage_bytes;
+};
+constexpr int kQiConsumers = 8;  // warps (16 measured slower: 11.3 against 10.0 us on the 14336 x 4096 layer)
+// (+ 1024: the stages of the tensor copies start on a 1024-byte boundary)
+int qi_fixed_bytes(int K, bool tm, int ms) { return K / 64 * 544 * ms + 512 * ms * kQiConsumers + 256 + (tm ? 1024 : 0); }
+QiCut qi_cut(int32_t fmt, int K, bool tensor_copies) {
+    const bool w8 = fmt == kFmtAffine8, w6 = fmt == kFmtAffine6;
+    QiCut c;
+    c.row_bytes = w8 ? K : (w6 ? K / 4 * 3 : K / 2);
+    // 4-bit codes with rows of 1 KB (K = 2048): one swizzled tensor copy per block of 16 rows, no padding (the swizzle
+    // spreads the rows over the banks). Otherwise one bulk copy per row (4-bit) or per pair of rows (6- and 8-bit), padded apart by a quad's piece.
+    c.tm = fmt == kFmtAffine4 && c.row_bytes <= 1024 && tensor_copies;
+    c.pair = w8 || w6;  // two rows per bulk copy
+    c.row_pitch = c.tm ? c.row_bytes : (c.pair ? 2 : 1) * c.row_bytes + (w8 ? 64 : (w6 ? 48 : 32));
+    c.stage_bytes = (c.tm ? kQiRows * c.row_bytes : (c.pair ? kQiRows / 2 : kQiRows) * c.row_pitch) + 2 * kQiRows * (K / 64 * 2);
+    c.fits = K % 2048 == 0 && (kQsSmemMax - qi_fixed_bytes(K, c.tm, 2)) / c.stage_bytes >= 2;
+    return c;
+}
 // Returns kOk after a launch, 1 when the shape does not fit this path (the caller falls back), or an error.
 int32_t launch_qmv_imma(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c) {
     if (c.mode != kModePlain || c.rows > 16 || c.rows < 1) return 1;
     if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine8 && c.fmt != kFmtAffine6) return 1;
-    if (c.K % 2048 != 0 || c.N < kQiRows) return 1;
+    const QiCut cut = qi_cut(c.fmt, c.K, ctx->encode_tiled != nullptr);
+    if (!cut.fits || c.N < kQiRows) return 1;
     if ((reinterpret_cast<uintptr_t>(c.w[0]) & 15) || (reinterpret_cast<uintptr_t>(c.s[0]) & 15) ||
         (reinterpret_cast<uintptr_t>(c.b[0]) & 15))
         return 1;
-    const bool w8 = c.fmt == kFmtAffine8, w6 = c.fmt == kFmtAffine6;
+    const bool w8 = c.fmt == kFmtAffine8, w6 = c.fmt == kFmtAffine6, tm = cut.tm;
     const int G = c.K / 64;
     QiParams p;
     memset(&p, 0, sizeof(p));
-    p.row_bytes = w8 ? c.K : (w6 ? c.K / 4 * 3 : c.K / 2);
-    // 4-bit codes with rows of 1 KB (K = 2048): one swizzled tensor copy per block of 16 rows, no padding (the swizzle
-    // spreads the rows over the banks). Otherwise one bulk copy per row (4-bit) or per pair of rows (6- and 8-bit), padded apart by a quad's piece.
-    const bool tm = c.fmt == kFmtAffine4 && p.row_bytes <= 1024 && ctx->encode_tiled != nullptr;
-    p.pair = (w8 || w6) ? 1 : 0;  // two rows per bulk copy
-    p.row_pitch = tm ? p.row_bytes : (p.pair ? 2 : 1) * p.row_bytes + (w8 ? 64 : (w6 ? 48 : 32));
+    p.row_bytes = cut.row_bytes;
+    p.pair = cut.pair ? 1 : 0;
+    p.row_pitch = cut.row_pitch;
     p.srow_bytes = G * 2;
     p.srow_pitch = p.srow_bytes;
-    p.stage_bytes = (tm ? kQiRows * p.row_bytes : (p.pair ? kQiRows / 2 : kQiRows) * p.row_pitch) + 2 * kQiRows * p.srow_pitch;
-    // The path is chosen on what eight rows need, whatever the row count of this call: a row must see the same
-    // arithmetic alone and among sixteen.
-    const int ncw = 8;  // consumer warps (16 measured slower: 11.3 against 10.0 us on the 14336 x 4096 layer)
-    // (+ 1024: the stages of the tensor copies start on a 1024-byte boundary)
-    auto fixed_bytes = [&](int ms) { return G * 512 * ms + G * 32 * ms + 512 * ms * ncw + 256 + (tm ? 1024 : 0); };
-    if ((kQsSmemMax - fixed_bytes(2)) / p.stage_bytes < 2) return 1;
+    p.stage_bytes = cut.stage_bytes;
+    constexpr int ncw = kQiConsumers;
+    auto fixed_bytes = [&](int ms) { return qi_fixed_bytes(c.K, tm, ms); };
     p.w = reinterpret_cast<const unsigned char*>(c.w[0]);
     p.s = reinterpret_cast<const unsigned char*>(c.s[0]);
     p.b = reinterpret_cast<const unsigned char*>(c.b[0]);
@@ -703,6 +719,26 @@ int32_t iq::qmv_with_scratch(iq_ctx* ctx, void* stream, const void* x, int32_t x
     c.accumulate = (flags & IQ_FLAG_ACCUMULATE) ? 1 : 0;
     c.scratch = scratch;
     return launch_gqmv(ctx, reinterpret_cast<cudaStream_t>(stream), c);
+}
+
+extern "C" int32_t iq_qmv_plan(const iq_qlinear* m, int32_t rows, int32_t sms, const int32_t clusters_at_once[3], iq_qmv_tiling* out) {
+    if (m == nullptr || out == nullptr || clusters_at_once == nullptr || rows < 1 || rows > 16 || sms < 1 || m->n < 16 || m->n % 16 != 0 || m->k < 64 || m->k % 64 != 0)
+        return kErrInvalidArg;
+    const int at_once[3] = {clusters_at_once[0], clusters_at_once[1], clusters_at_once[2]};
+    for (int n : at_once)
+        if (n < 1) return kErrInvalidArg;
+    memset(out, 0, sizeof(*out));
+    GqmvCall c;
+    c.fmt = format_of(m); c.rows = rows; c.N = m->n; c.K = m->k;
+    if (c.fmt < 0) return kErrUnsupported;
+    if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return kOk;
+    if (c.fmt != kFmtAffine4G32 && qi_cut(c.fmt, c.K, true).fits) return kOk;
+    const bool vec = c.K / (c.fmt == kFmtAffine4G32 ? 32 : 64) % qr_groups(c.fmt) == 0;
+    const QrPlan plan = qr_plan(c.fmt, c.N, c.K, 1, vec, sms, false, c.fmt != kFmtAffine8);
+    if (plan.max_rows == 0 || plan.wk == 0 || !rows_kernel_pays(c, 1, plan.max_rows, false)) return kOk;
+    out->cluster = qmv_rows_cluster(at_once, c.fmt, rows, c.N, c.K, plan.wk);
+    if (out->cluster > 0) { out->tiles = (c.N + 127) / 128; out->slices = plan.wk; }
+    return kOk;
 }
 
 extern "C" int32_t iq_qmv(iq_ctx* ctx, void* stream, const void* x, int32_t x_dtype, int64_t ldx, const iq_qlinear* m,

@@ -46,6 +46,8 @@ QwPlan qw_plan(const int (&at_once)[3], int32_t fmt, int t, int N, int K, int wk
 }
 }  // namespace
 
+int qmv_rows_cluster(const int (&at_once)[3], int32_t fmt, int rows, int N, int K, int wk) { return qw_plan(at_once, fmt, rows <= 8 ? 8 : 16, N, K, wk).cluster; }
+
 int32_t launch_qmv_rows(iq_ctx* ctx, cudaStream_t st, const GqmvCall& c, int wk) {
     if (c.rows < 1 || c.rows > 16 || ctx->encode_tiled == nullptr || c.mode != kModePlain) return 1;
     if (c.fmt != kFmtAffine4 && c.fmt != kFmtAffine4G32 && c.fmt != kFmtAffine8) return 1;

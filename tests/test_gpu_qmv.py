@@ -311,9 +311,9 @@ def test_qmv_mxfp4_row_invariance(cuda_device, N, K):
 @pytest.mark.parametrize("N,K,rows", [(16, 64, 5), (128, 4096, 8), (144, 2048, 9), (1040, 2880, 6), (2064, 1088, 16), (4752, 2048, 7), (4784, 2048, 13),
                                       (19008, 320, 5), (256, 14336, 16), (256, 14336, 8), (640, 16448, 12)])
 def test_qmv_rows_edges(cuda_device, bits, group, N, K, rows):
-    """Five rows and more (tcgen05): tiles of weight rows and columns of inputs that are not full, one to eight CTAs per tile, several tiles
-    per CTA, left-over blocks with K slices of their own (4784 rows of 2048 inputs), both heights; against the oracle, added to y, and every
-    row with the bits that it has alone."""
+    """Five rows and more on whichever kernel takes the shape (staged, ring, clusters): tiles of weight rows and columns of inputs that are not full, left-over
+    blocks with K slices of their own (4784 rows of 2048 inputs), both heights; against the oracle, added to y, and every row with the bits that
+    it has alone."""
     rng = np.random.default_rng(900 + bits + group + N + K + rows)
     m, host = affine_case(rng, N, K, bits, cuda_device, group=group)
     x = synth.activations_np(rng, rows, K)
@@ -333,4 +333,19 @@ def test_qmv_rows_edges(cuda_device, bits, group, N, K, rows):
 @pytest.mark.parametrize("N,K,rows", [(256, 7680, 5), (272, 7744, 8), (144, 5504, 9), (128, 9216, 6), (256, 11008, 12), (4112, 4672, 13)])
 def test_qmv_rows_by_width(cuda_device, bits, group, N, K, rows):
     """The widths between the ring kernel's and the widest, on both sides of its limits of two, four and eight rows a launch: same demands."""
+    test_qmv_rows_edges(cuda_device, bits, group, N, K, rows)
+
+
+@pytest.mark.parametrize("bits,group,N,K,rows,cluster,waves,even", [
+    (4, 64, 5312, 7232, 5, 2, 1, True), (4, 64, 7712, 3648, 16, 2, 1, True), (4, 64, 2032, 5440, 16, 4, 1, True),
+    (4, 64, 5312, 6336, 9, 4, 2, True), (4, 64, 2032, 8576, 16, 8, 2, True), (4, 64, 5312, 13504, 5, 8, 3, True), (4, 64, 1040, 16448, 8, 8, 1, True),
+    (8, 64, 5312, 11264, 5, 2, 1, True), (8, 64, 12512, 17984, 5, 2, 2, True), (8, 64, 2480, 8576, 9, 4, 1, False), (8, 64, 2480, 9472, 8, 4, 1, False),
+    (8, 64, 16, 8576, 9, 8, 1, False), (8, 64, 464, 18880, 5, 8, 1, False), (8, 64, 2032, 17984, 9, 8, 2, False),
+    (4, 32, 5312, 4992, 16, 2, 1, True), (4, 32, 5312, 9920, 8, 2, 1, True), (4, 32, 2480, 9920, 16, 4, 1, True), (4, 32, 16, 19776, 8, 8, 1, False)])
+def test_qmv_rows_by_cluster(cuda_device, bits, group, N, K, rows, cluster, waves, even):
+    """The forms of the kernel of clusters: two, four and eight CTAs per tile, more clusters than the GPU holds at once, slices that the CTAs of a cluster
+    share evenly or not, both heights; same demands."""
+    at_once = {2: 74, 4: 33, 8: 15}
+    p = capi.qmv_plan(N, K, bits, group, rows, at_once=tuple(at_once.values()))
+    assert (p.cluster, -(-p.tiles // at_once[cluster]), p.slices % max(p.cluster, 1) == 0) == (cluster, waves, even)
     test_qmv_rows_edges(cuda_device, bits, group, N, K, rows)
