@@ -53,19 +53,20 @@ constexpr int kRouterSmemMax = 200 * 1024;
 constexpr int kGroupChunkedMinPairs = 4096;  // from here on the permutation runs as a chunked counting sort
 constexpr int kFixedTokens = 512;  // up to here the grouping kernel leaves the activations as fixed point for the int8 kernels
 // Affine experts run on the decode tiles (csrc/qmv_tile.cuh) while they see a few rows each on average; everything else, MXFP4 experts at any number of
-// rows, runs on the grouped GEMM. The tiles take the token rows as two digits (16 bits of a group's largest input) where their predecessor on
-// mma.sync did: 256 to 4096 inputs, a power of two, up to six rows per expert. Elsewhere the GEMM ran, which takes bf16 activations whole, and so do
-// three digits (23 bits): with a few input channels 100 times the rest, or one of every 64 300 times, two are 4.4e-4 to 4.9e-4 off the 64-bit result (24
-// tokens, 32 experts of 2880 x 768), the GEMM 3.0e-4, three 2.4e-4. MoE block, us, tiles / GEMM (eight, four, six and eight experts per token):
-//   128 experts of 2048 x 768, two digits    20 tokens 77 / 103, 64 97 / 128, 96 (6 rows) 115 / 135; three digits 112 (7 rows) 157 / 135
-//   32 of 4096 x 2048, two digits            20 tokens 118 / 153, 48 (6 rows) 140 / 170; three digits 64 (8 rows) 213 / 165
-//   64 of 3072 x 1408, three digits          8 tokens 106 / 112, 20 148 / 151, 40 (3.8 rows) 165 / 168, 64 (6 rows) 180 / 169
-//   128 of 2880 x 768, three digits          8 tokens 92 / 95, 20 131 / 147, 64 (4 rows) 174 / 183, 80 (5 rows) 198 / 191
-// Likewise h: as two digits in the widths that mma.sync took, as three (up to four rows per expert, two below 1024 features, then by the GEMM) in the others, where it has been whole
-// halves. With one feature of every 64 256 times the rest, that do not count in the outputs, two digits are 7e-3 off the 64-bit result, three as much as
-// the GEMM. h's three digits, tiles / GEMM: 64 of 2048 x 1408 at 4 tokens 55.1 / 58.9, 30 102.7 / 103.8, 45 (4.2 rows) 108.1 / 108.4, 64 (6) 121 / 116, 32 of
-// 2880 x 2880 at 16 153 / 159, 32 (4) 171 / 182, 256 of 1024 x 704 at 8 46.3 / 47.6, 64 (2) 96.6 / 94.9, 190 (5.9) 149 / 140,
-// 64 of 4096 x 704 at 16 (1.5) 95.0 / 97.2, 40 (3.8) 130 / 127.
+// rows, runs on the grouped GEMM. The tiles take the token rows as two digits (16 bits of a group's largest input), with the sums and so the bits of the
+// expert-parallel pieces' kernel, in the widths that this one takes and 4096: a power of two from 256, up to six rows per expert. In other widths the
+// pieces run on the GEMM, which takes bf16 activations whole, and so do three digits (23 bits): with a few input channels 100 times the rest, or one of
+// every 64 300 times, two are 4.3e-4 to 5.2e-4 off the 64-bit result (40 and 64 tokens of 2048 x 768), GEMM and three digits 3.0e-4 (24 tokens of 2880 x
+// 768). MoE block, us, tiles / GEMM (eight, four, six and eight experts per token):
+//   128 experts of 2048 x 768, two digits    20 tokens 77 / 102, 64 98 / 128, 96 (6 rows) 116 / 134, 112 (7 rows) 127 / 135
+//   32 of 4096 x 2048, two digits            20 tokens 117 / 152, 48 (6 rows) 142 / 168, 64 (8 rows) 168 / 165
+//   64 of 3072 x 1408, three digits          8 tokens 107 / 110, 20 149 / 150, 40 (3.8 rows) 166 / 168, 64 (6 rows) 183 / 169
+//   128 of 2880 x 768, three digits          8 tokens 89 / 94, 20 130 / 147, 64 (4 rows) 171 / 183, 80 (5 rows) 193 / 191
+// Likewise h: two digits in the widths that the pieces' kernel takes, three (up to four rows per expert, two below 1024 features, then the GEMM) in the
+// others, where it has been whole halves. With one feature of every 64 256 times the rest, that do not count in the outputs, two digits are 5e-3 to 7e-3
+// off the 64-bit result, three as much as the GEMM, 2.9e-4. h's three digits, tiles / GEMM: 64 of 2048 x 1408 at 4 tokens 55.1 / 58.9, 30 103 / 104,
+// 45 (4.2 rows) 108.1 / 108.4, 64 (6) 121 / 116, 32 of 2880 x 2880 at 16 153 / 159, 32 (4) 171 / 182, 256 of 1024 x 704 at 8 46.3 / 47.6, 64 (2) 96.6 / 94.9,
+// 190 (5.9) 149 / 140, 64 of 4096 x 704 at 16 (1.5) 95.0 / 97.2, 40 (3.8) 130 / 127.
 constexpr int kInt8RowsPerExpert = 6, kWideRowsPerExpert = 4;
 bool two_digit_h(const iq_moe* l) { return qmv_grouped_slices(l->d.d_ff, 1) > 0; }
 bool two_digit_inputs(const iq_moe* l) { return l->d.d_model >= 256 && l->d.d_model <= 4096 && (l->d.d_model & (l->d.d_model - 1)) == 0; }
@@ -363,8 +364,9 @@ bool use_route_small(const iq_moe* l, int tokens) {
 }
 // The experts' kernels for few tokens: affine 4-bit weights, 16-byte aligned; one token, or two and three of small experts. Beyond 24 million
 // weights (of one matrix, of every token's experts) the decode tiles take two and three, with three digits; below, the tiles leave the GPU
-// half empty. MoE block, us, here / tiles: 64 experts of 1536 x 512 at two tokens (12.6 million) 26.9 / 27.7, at three (18.9) 30.9 / 31.3, 64 of 2560 x
-// 1024 at two (21.0) 32.0 / 33.9, at three (31.5) 47.7 / 43.7, 128 of 2048 x 768 at two (25.2) 41.0 / 39.2, 128 of 2880 x 768 at two (35.4) 61.3 / 49.5
+// half empty. MoE block, us, here / tiles: 64 experts of 1536 x 512 at two and three tokens (12.6 and 18.9 million) 27.0 / 28.7, 30.5 / 32.1, 32 of 1024 x
+// 1792 (14.7, 22.0) 26.6 / 29.0, 36.9 / 34.8, 64 of 2880 x 704 (16.2, 24.3) 35.5 / 35.9, 44.1 / 40.0, 128 of 2048 x 768 at two (25.2) 40.9 / 39.9, 64 of
+// 2048 x 1408 (34.6) 44.8 / 43.8, 128 of 2880 x 768 (35.4) 61.9 / 50.3
 bool use_experts_small(const iq_moe* l, int tokens) {
     const iq_moe_desc& d = l->d;
     if (tokens > 1 && (int64_t)tokens * d.top_k * d.d_model * d.d_ff > 24000000) return false;

@@ -1,6 +1,6 @@
-// The MoE block for up to three tokens in three kernels, where a decode step of few tokens is a chain of latencies and not
-// of bytes (one token of the 128-expert layer reads 21 MB, 3 us, and took 59 us in eight kernels, 26 in three; three tokens
-// 52 us against 57. From four on, 67 against 61, the separate kernels, which stage the weights, win):
+// The MoE block for one token, and for two or three of small experts, in three kernels, where a decode step is a chain of latencies and not
+// of bytes (one token of the 128-expert layer reads 21 MB, 3 us, and took 59 us in eight kernels, 26 in three). Beyond 24 million weights of all
+// tokens' experts only the first of them runs here, then the decode tiles, which stage the weights (use_experts_small in moe.cu):
 //
 //   moe_route_small_kernel   router logits, top-k and the permutation in one cluster of eight blocks; also the activations as
 //                            block fixed point (the int8 kernels' operand, see qmv_imma.cuh), once per token
@@ -12,9 +12,9 @@
 // Each starts while its predecessor runs (programmatic dependent launch); the down kernel has its first weights on the way
 // before h exists. Affine 4-bit experts, all of them on this GPU. The results are those of the separate kernels: exact
 // float64 logits, sums in fixed orders. The activations and h are fixed point of 23 bits (three digits: the columns of an MMA are two
-// rows of (high, middle), (low, low), as in qmv_ring.cuh), which keeps bf16 activations whole as the fp16 kernels did that ran the
-// widths the staged kernels do not take: with 16 bits a layer of 2880 x 768 with input channels 100 times the rest was 8.5e-4 off
-// the 64-bit result instead of 4.9e-4.
+// rows of (high, middle), (low, low), as in qmv_ring.cuh), which keeps bf16 activations and halves of h whole as fp16 kernels do: with 16 bits a
+// layer of 2880 x 768 with input channels 100 times the rest was 8.5e-4 off the 64-bit result instead of 4.9e-4. The decode tiles take three digits
+// of both for two and three tokens too.
 #pragma once
 
 #include <type_traits>

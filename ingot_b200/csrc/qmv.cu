@@ -206,19 +206,20 @@ QrPlan qr_plan(int32_t fmt, int N, int K, int nw, bool vec, int sms, bool wk8, b
 }
 // Where csrc/qmv_rows.cuh takes a plain call over, one launch for any rows: by the rows that a launch here holds (max_rows: of 4-bit weights two above
 // some 11000 inputs, four above 7300, eight above 4100; of 8-bit ones four above 11000, eight above 5000), and by whether the launches here share one
-// conversion of the activations (pre, the dense FFN's down projection). us here / there:
-// 4 bits, two rows a launch, 5 / 8 / 9 / 16 rows: 4096 x 14336 38.3 / 21.7, 53.7 / 24.4, 64.6 / 45.7, 106.3 / 56.2; 5120 x 13824 48.4 / 43.9, 67.1 / 47.9,
-//   81.6 / 53.1, 134.2 / 64.7. Four: 4096 x 11008 28.9 / 19.1, 39.6 / 21.5, 48.0 / 24.1, 75 / 30.5; 2048 x 7680 15.0 / 13.8, 19.0 / 15.0, 24.1 / 17.3, 36.9 / 21.4.
-//   Eight: 4096 x 5504 at 5 / 8 / 9 / 16 rows 14.4 / 12.7, 17.6 / 14.1, 23.7 / 16.2, 34.5 / 19.6, 9216 x 5120 14.5 / 17.7, 16.5 / 19.9, 25.7 / 22.4, 32.5 / 28.7,
-//   2048 x 5120 at 8 / 9 / 14 11.1 / 14.9, 15.7 / 17.3, 19.1 / 19.8.
-// 8 bits, four rows a launch: 4096 x 14336 at 5 / 8 / 16 rows 36.6 / 28.0, 43.1 / 30.5, 85.5 / 36.6. Eight: 4096 x 11008 at 6 / 8 / 16 29.6 / 18.4, 34.1 / 19.4,
-//   66.5 / 31.1, 4096 x 8768 at 8 / 9 20.9 / 23.2, 32.7 / 25.8, 2048 x 5504 11.1 / 12.7, 16.0 / 14.7.
-// Groups of 32, two rows a launch, 6 / 8 / 9 / 16 rows: 5120 x 13824 54.4 / 56.6, 72.0 / 60.3, 88.2 / 70.4, 144 / 83.4. Four: 2048 x 7680 at 6 / 8 / 9 / 12 16.3 / 17.2,
-//   18.8 / 18.5, 24.2 / 22.4, 27.8 / 25.1, 4096 x 11008 at 8 / 9 / 12 40.8 / 26.8, 50.2 / 52.5, 60.4 / 58.3. Eight: 9216 x 5120 at 9 / 12 / 16 32.0 / 32.7, 37.2 / 35.0,
-//   46.3 / 36.9, 7168 x 5376 at 12 38.4 / 39.2, 2048 x 4160 at 14 18.8 / 21.2.
-// Many features are more than a wave of clusters: 12288 x 7680 at 5 / 8 rows 36.1 / 45.7, 43.5 / 50.1 (groups of 32 at 8 / 13 46.0 / 63.0, 84.1 / 99.1), 14336 x
-//   5504 at 9 / 13 42.7 / 46.2, 47.2 / 53.8. FFN with the down projection here / there: 4096 / 11008 at 9 / 16 rows 68.9 / 62.3, 87.9 / 73.5, 2048 / 7680 at 8 / 10 /
-//   13 / 16 26.4 / 28.1, 35.4 / 35.6, 41.8 / 38.4, 43.5 / 40.6.
+// conversion of the activations (pre, the dense FFN's down projection). us here / there, matrices of 300 MB in rotation:
+// 4 bits, two rows a launch, 5 / 8 / 9 / 16 rows: 4096 x 14336 38.2 / 24.2, 53.7 / 27.3, 64.6 / 51.1, 106 / 62.3; 5120 x 13824 48.3 / 46.1, 67.2 / 50.5, 81.7 /
+//   53.8, 134 / 65.1. Four: 4096 x 11008 30.3 / 20.3, 41.9 / 23.0, 51.0 / 24.2, 83.2 / 30.9; 2048 x 7680 15.1 / 12.8, 19.1 / 14.3, 24.4 / 16.3, 37.6 / 20.7.
+//   Eight: 4096 x 5504 14.4 / 11.8, 18.1 / 13.2, 24.6 / 15.1, 36.1 / 18.8; 9216 x 5120 14.7 / 18.3, 17.2 / 20.7, 25.8 / 22.2, 33.3 / 28.8; 2048 x 5120 at 8 / 9
+//   11.3 / 14.2, 16.0 / 16.2.
+// 8 bits, four rows a launch, 5 / 8 / 16 rows: 4096 x 14336 36.5 / 26.9, 43.0 / 28.9, 85.5 / 35.8. Eight: 4096 x 11008 at 6 / 8 / 16 29.8 / 18.1, 34.3 / 19.4,
+//   66.5 / 31.8, 4096 x 8768 at 8 / 9 22.2 / 25.6, 33.1 / 27.4, 2048 x 5504 11.6 / 12.5, 17.1 / 14.7.
+// Groups of 32, two rows a launch, 6 / 8 / 9 / 16 rows: 5120 x 13824 53.9 / 56.2, 71.9 / 60.2, 87.8 / 67.7, 144 / 80.8. Four: 2048 x 7680 at 6 / 8 / 12 16.6 / 16.3,
+//   19.2 / 17.6, 28.4 / 23.2, 4096 x 11008 at 8 / 9 / 12 42.7 / 28.3, 52.7 / 54.8, 63.8 / 60.6. Eight: 9216 x 5120 at 5 / 12 / 16 19.7 / 23.2, 37.4 / 33.4, 46.4 /
+//   36.3, 7168 x 5376 at 12 38.8 / 40.3.
+// Many features are more than a wave of clusters: 12288 x 7680 at 5 / 8 rows 36.1 / 44.4, 43.4 / 49.2 (groups of 32 at 8 / 12 45.5 / 60.5, 68.2 / 75.7), 14336 x
+//   5504 at 9 / 12 43.0 / 45.5, 47.9 / 50.0. FFN with the down projection here / there: 4096 / 11008 at 9 / 16 rows 68.5 / 61.2, 88.1 / 72.4, 2048 / 7680 at 8 / 9 /
+//   16 27.1 / 28.2, 36.9 / 35.9, 45.7 / 41.6. Over 350 calls the rule takes none that is slower there; it leaves some that would be faster (groups of 32 at
+//   five rows of 4096 x 14336 41.8 / 29.8 or nine of 8192 x 8768 69.2 / 63.6, 4 bits at five rows of 16384 x 10240 65.5 / 55.2).
 bool rows_kernel_pays(const GqmvCall& c, int nw, int max_rows, bool pre) {
     if (nw != 1 || c.rows < 5) return false;
     if (c.fmt == kFmtAffine8) {

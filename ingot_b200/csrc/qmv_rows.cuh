@@ -1,13 +1,13 @@
 // Decode linears of several rows and wide inputs on the 5th-generation tensor cores with integers (affine weights, 4 and 8 bits).
 //
 // The arithmetic, the digits and the order of the sums are those of the ring kernel (qmv_ring.cuh), which takes these shapes at fewer rows: a row
-// has the same bits alone and among sixteen. That kernel holds the digits of all inputs in every CTA beside sixteen rings of weights: of
-// more than some 8000 inputs only two rows fit (8 bits: four), and sixteen rows are eight launches that each read the weights. Here a cluster
+// has the same bits alone and among sixteen. That kernel holds the digits of all inputs in every CTA beside sixteen rings of weights: of wide inputs
+// few rows fit (rows_kernel_pays in qmv.cu: two of 11000 inputs), and sixteen rows are up to eight launches that each read the weights. Here a cluster
 // shares a tile of 128 weight rows, each CTA holding the digits of its K slices only, and one thread issues tcgen05.mma (kind::i8) for 128 weight
-// rows against all (digit, row) columns, so that sixteen rows are one launch: 4096 x 14336 (4 bits) at 8 rows 53.9 -> 24.4 us, at
-// 16 106.6 -> 56.2, 4096 x 11008 at 12 58.6 -> 26.8, 8 bits 66.5 -> 31.1 at 16. How many clusters run at once is asked of the driver: thirty-three of four CTAs,
-// but fifteen of eight, since a cluster stays in one group of SMs (2048 x 7680 at 8 rows 20 us as sixteen clusters of eight, 15.0 of four). Narrower inputs
-// stay where they are: a step of 256 inputs takes this machine 1000 to 2000 cycles whatever its rows (waits on barriers, loads from tensor memory and sums
+// rows against all (digit, row) columns, so that sixteen rows are one launch: 4096 x 14336 (4 bits) at 8 rows 53.7 -> 27.3 us, at
+// 16 106 -> 62.3, 4096 x 11008 at 12 62.5 -> 26.6, 8 bits 66.5 -> 31.8 at 16. How many clusters run at once is asked of the driver: thirty-three of four CTAs,
+// but fifteen of eight, since a cluster stays in one group of SMs (2048 x 7680 at 8 rows 20 us as sixteen clusters of eight, 14.3 of four). Inputs that the staged kernel takes
+// (2048, 4096, 8 bits 6144) stay there: a step of 256 inputs takes this machine 1000 to 2000 cycles whatever its rows (waits on barriers, loads from tensor memory and sums
 // of one step follow one another in a warp), and 14336 x 4096 at 8 rows took 29.0 us instead of 20.4.
 //
 // Unit of work: a cluster of two to eight CTAs takes a tile, each its share of the K slices (the digits of all of K fit one CTA only where a cluster is

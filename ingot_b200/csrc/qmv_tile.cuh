@@ -22,7 +22,8 @@
 //   warp 3      the rows' scales and biases
 //   4-7 (4-11)  sums to floats, a thread per weight row; at the end of a tile activation and stores
 //   the last 4  codes to bytes: A operand in tensor memory, a thread per weight row
-// Tensor memory (256 columns per CTA): the A operand and the sums, each twice, so that conversion, MMA and sums of three steps overlap.
+// Tensor memory (256 columns per CTA): the sums twice, the A operand in two slots of four groups (three digits: four of two), so that conversion, MMA and
+// sums of three steps overlap.
 // The gate/up form takes 64 gate rows and the matching 64 up rows (lanes 0-15 of a quadrant gate, lanes 16-31 up), as qmm_ta.cuh does.
 // Every wait is bounded: on a timeout the kernel writes a status word, all roles drain and tensor memory is released.
 //
@@ -48,7 +49,7 @@ constexpr int kQtXs = 4 * kQtRows * 8;              // [group][pair of tokens]{s
 constexpr int kQtScales = 2 * 128 * 8;              // scales and biases of the weight rows
 constexpr int qt_x_bytes(int nd) { return 2 * nd * kQtRows * 128; }  // digits of a step: [pair of groups][digit][token][128]
 constexpr int qt_stage(int nd) { return kQtCodes + qt_x_bytes(nd) + kQtScales + kQtXs; }
-// Four stages, 74 KB of codes under way per SM: a fifth would fit, but would take the L1 that serves a row's four pieces of a sector of scales
+// Four stages, 64 KB of codes per CTA. Beside two digits a fifth would fit, but would take the L1 that serves a row's four pieces of a sector of scales
 // (MoE of 128 experts 2048 x 768, 64 tokens: 106.9 us with five, 99.9 with four, 101.7 with three)
 constexpr int kQtStages = 4;
 constexpr int qt_smem(int nd) { return 1024 + kQtStages * qt_stage(nd) + 256; }  // alignment, stages, barriers
